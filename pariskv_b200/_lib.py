@@ -101,6 +101,22 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
+
+
+def native():
+    """The CPython binding of the library (``csrc_py/bind.cpp``), loaded once together with it.  The per-step entry
+    points go through it; what is called once in a while keeps the ctypes declarations below."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise RuntimeError(f"the native binding of {LIB_PATH} cannot be loaded ({e}): build it with "
+                               "`python -m pariskv_b200.build`") from e
+        _native = module
+    return _native
 
 
 def load():

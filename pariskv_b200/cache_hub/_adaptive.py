@@ -66,7 +66,7 @@ class AdaptiveKCache(_base_cache):
         st = self._layer_state[layer_idx]
         _, _, ex = ops.retrieve_ex(queries, self.srht_diagonal_signs, self._mag_centers, self.codebook_gpu[layer_idx],
                                    self.key_block_weight_gpu[layer_idx], self.key_4bit_packed_gpu[layer_idx],
-                                   self.cluster_key_counts_gpu[layer_idx], self._c_max, 0, kv_len=st[4:4 + self.batch_size],
+                                   self.cluster_key_counts_gpu[layer_idx], self._c_max, 0, kv_len=self._zone_len_dev[layer_idx],
                                    schedule=self._zone_schedule, want=("cand", "scores_f32", "query_avg"),
                                    scratch=self._retrieve_scratch)
         cand, cand_scores = ex["cand"], ex["scores_f32"]
@@ -107,6 +107,6 @@ class AdaptiveKCache(_base_cache):
         self.last_topk_indices = topk
         if fixed:
             return self._attend(queries, wk, wv, self.window_capacity, self._store_k[layer_idx], self._store_v[layer_idx],
-                                topk, n_sel=n_sel, n_window_dev=st[0:1], n_window_add=0)
+                                topk, n_sel=n_sel, n_window_dev=self._window_rows_dev[layer_idx], n_window_add=0)
         return self._attend(queries, wk, wv, n_win, self._store_k[layer_idx], self._store_v[layer_idx], topk,
                             n_sel=n_sel)

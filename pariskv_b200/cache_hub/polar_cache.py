@@ -117,6 +117,8 @@ class polar_cache(KV_Cache):
         self._win_vnorm = [torch.zeros(bs, H, cap_w, dtype=torch.float32, device=dev) for _ in range(layer_num)]
         # device-side positions per layer: [rows in the window, arrival counter, flushes, error flag, keys of sample 0..]
         self._layer_state = [torch.zeros(4 + bs, dtype=torch.int32, device=dev) for _ in range(layer_num)]
+        self._window_rows_dev = [t[0:1] for t in self._layer_state]      # views made once: a slice costs a microsecond
+        self._zone_len_dev = [t[4:4 + bs] for t in self._layer_state]
         # zone store: the K and V row of a key sit next to each other ([bs,H,cap,2,128]), so a selected key costs one
         # address translation of host memory instead of two; with zones of several GB per layer the row fetch of the
         # attention kernel ran 30 % faster on B200 this way.  unified_keys_cpu / unified_values_cpu are the two
@@ -161,6 +163,7 @@ class polar_cache(KV_Cache):
         # addresses never change, so decode steps captured in CUDA graphs stay valid however the zone grows.
         self._zone_schedule = _lib.zone_schedule(ZONE_BOUNDS, [r[0] for r in self._ratio_rows()],
                                                  [r[1] for r in self._ratio_rows()], TIER_RATIOS)
+        self._zone_schedule_addr = ctypes.addressof(self._zone_schedule)
         c_max = int(_lib.load().pk_zone_max_candidates(ctypes.byref(self._zone_schedule), max(self.zone_capacity, 1)))
         self._c_max = max(c_max, 1)
         rows = (bs * H, self.group_size) if self.per_query_head_retrieval else (bs, H)
@@ -381,7 +384,6 @@ class polar_cache(KV_Cache):
         queries = queries.contiguous()
         self._wait_offload(layer_idx)
         l = layer_idx
-        st = self._layer_state[l]
         wk, wv = self.unified_keys_gpu[l], self.unified_values_gpu[l]
         sk, sv = self._store_k[l], self._store_v[l]
         if self._full_regime(l):  # attend everything (eager only: the row count is a host number)
@@ -390,11 +392,13 @@ class polar_cache(KV_Cache):
                 raise RuntimeError("full attention over short sequences needs samples of equal length")
             if N <= 0:
                 return self._attend(queries, wk, wv, n_win)
-            if self._all_rows is None or self._all_rows.shape[-1] < N:
-                self._all_rows = torch.arange(self.zone_capacity, device=self.device).expand(
-                    self.batch_size, self.kv_head, -1).contiguous()
-            sel = self._all_rows[:, :, :N].contiguous() if N != self._all_rows.shape[-1] else self._all_rows
-            return self._attend(queries, wk, wv, n_win, sk, sv, sel)
+            # rows 0 .. N-1 of every head: a view of one index row, made again only when the zone has grown
+            if self._all_rows is None:
+                self._all_rows = torch.arange(self.zone_capacity, device=self.device).expand(self.batch_size, self.kv_head, -1)
+                self._all_rows_n = None
+            if self._all_rows_n is None or self._all_rows_n.shape[2] != N:
+                self._all_rows_n = self._all_rows[:, :, :N]
+            return self._attend(queries, wk, wv, n_win, sk, sv, self._all_rows_n)
         if self.per_query_head_retrieval:
             return self._compute_per_query_head(queries, l)
         # A caller whose queries are made BEFORE it calls decode_update_kv_cache (one kernel makes q and k) says so with
@@ -402,22 +406,25 @@ class polar_cache(KV_Cache):
         # collision kernel may prepare the query before it waits for the append (matters with dependent launch only).
         settled = self.queries_precede_append and self._appended_layer == l
         self._appended_layer = None
-        final, n_sel, _ = ops.retrieve_ex(queries, self.srht_diagonal_signs, self._mag_centers, self.codebook_gpu[l],
-                                          self.key_block_weight_gpu[l], self.key_4bit_packed_gpu[l],
-                                          self.cluster_key_counts_gpu[l], self._c_max, self.final_topk,
-                                          kv_len=st[4:4 + self.batch_size], schedule=self._zone_schedule,
-                                          scratch=self._retrieve_scratch, queries_settled=settled)
+        final, n_sel = _lib.native().retrieve_ex(
+            queries, self.srht_diagonal_signs, self._mag_centers, self.codebook_gpu[l], self.key_block_weight_gpu[l],
+            self.key_4bit_packed_gpu[l], self.cluster_key_counts_gpu[l], self._c_max, self.final_topk, None,
+            self._zone_len_dev[l], self._zone_schedule_addr, 0, None, None, 1, 0, None, None, None, None, None, None, None,
+            None, self._retrieve_scratch.buf, settled)
         self._remember_selection(final, n_sel, l)
         # window rows and zone rows per head are read on the device
         return self._attend(queries, wk, wv, self.window_capacity, sk, sv, final, n_sel=n_sel,
-                            n_window_dev=st[0:1], n_window_add=0)
+                            n_window_dev=self._window_rows_dev[l], n_window_add=0)
 
     def _remember_selection(self, final, n_sel, l):
         """last_topk_indices as the reference exposes it: [bs,H,K] with K = min(final_topk, candidates) when the
         samples agree on the zone length; with per-sample lengths the full rows plus last_n_sel."""
         self.last_n_sel = n_sel
-        if min(self.zone_len[l]) == max(self.zone_len[l]):
-            final = final[:, :, :self.retrieval_plan(self.zone_len[l][0])[2]]
+        z = self.zone_len[l]
+        if min(z) == max(z):
+            C = max(1, int(math.ceil(z[0] * self._get_adaptive_ratios(z[0])[0])))    # as in retrieval_plan
+            if C < self.final_topk:
+                final = final[:, :, :C]
         self.last_topk_indices = final
 
     def _compute_per_query_head(self, queries, l):
@@ -425,14 +432,13 @@ class polar_cache(KV_Cache):
         becomes a batch entry whose G "heads" all point at that KV head's keys (stride 0 over the group), and the
         same kernels run with a group size of one."""
         bs, H, G = self.batch_size, self.kv_head, self.group_size
-        st = self._layer_state[l]
 
         def per_group(t):   # [bs,H,...] -> [bs*H, G, ...], the group dimension with stride 0
             return t.view(bs * H, 1, *t.shape[2:]).expand(bs * H, G, *t.shape[2:])
 
         q = queries.view(bs, H, G, 128).reshape(bs * H, 1, G, 128)
         counts = per_group(self.cluster_key_counts_gpu[l]).contiguous()
-        kv_len = st[4:4 + bs].repeat_interleave(H)          # one entry per (batch, KV head)
+        kv_len = self._zone_len_dev[l].repeat_interleave(H)          # one entry per (batch, KV head)
         final, n_sel, _ = ops.retrieve_ex(q, self.srht_diagonal_signs, self._mag_centers, per_group(self.codebook_gpu[l]),
                                           per_group(self.key_block_weight_gpu[l]), per_group(self.key_4bit_packed_gpu[l]),
                                           counts, self._c_max, self.final_topk, kv_len=kv_len,
@@ -440,7 +446,7 @@ class polar_cache(KV_Cache):
         self._remember_selection(final.view(bs, H * G, -1), n_sel.view(bs, H * G), l)   # one row per query head
         wk, wv = per_group(self.unified_keys_gpu[l]), per_group(self.unified_values_gpu[l])
         sk, sv = per_group(self._store_k[l]), per_group(self._store_v[l])
-        out = self._attend(q, wk, wv, self.window_capacity, sk, sv, final, n_sel=n_sel, n_window_dev=st[0:1],
+        out = self._attend(q, wk, wv, self.window_capacity, sk, sv, final, n_sel=n_sel, n_window_dev=self._window_rows_dev[l],
                            n_window_add=0)
         return out.view(bs, 1, H * G, 128)
 

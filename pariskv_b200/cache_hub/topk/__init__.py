@@ -5,7 +5,7 @@ from types import SimpleNamespace
 
 import torch
 
-from ... import torch_ops  # noqa: F401  (registers torch.ops.pariskv.*)
+from ... import ops, torch_ops  # noqa: F401  (registers torch.ops.pariskv.*)
 
 
 def _topk_2d(input, k):
@@ -27,6 +27,8 @@ def bucket_topk(input: torch.Tensor, k: int) -> torch.Tensor:
     assert k > 0, f"k must be positive, got {k}"
     if input.dim() not in (2, 3):
         raise ValueError(f"input must be 2D or 3D, got {input.dim()}D")
+    if torch_ops.direct(input):
+        return ops.topk(input, k)
     return torch.ops.pariskv.topk(input, int(k))
 
 

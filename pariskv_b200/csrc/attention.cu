@@ -37,7 +37,8 @@ struct AttParams {
   int64_t cap_s;          // rows per (b,h) of the store
   int64_t s_b, s_h, s_l;  // store strides in elements (batch, head, row); K and V share them
   int kv_pair;            // the V row of a store key directly follows its K row: one 512-byte copy fetches both
-  const int64_t* sel;     // [bs*H][K]
+  const int64_t* sel;     // selected rows of (b,h) at sel[b*sel_b + h*sel_h + j]
+  int64_t sel_b, sel_h;
   const int32_t* n_sel;   // [bs*H] or null
   int64_t K, index_offset;
   int H, Hq, G, n_qgroups;
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
       if (r < n_window) {
         src = (is_v ? p.wv : p.wk) + b * p.w_b + h * p.w_h + r * p.w_l;
       } else {
-        const int64_t row = p.sel[bh * p.K + (r - n_window)] + p.index_offset;
+        const int64_t row = p.sel[b * p.sel_b + h * p.sel_h + (r - n_window)] + p.index_offset;
         ok = row >= 0 && row < p.cap_s;
         paired = p.kv_pair != 0;
         src = ((is_v && !paired) ? p.sv : p.sk) + b * p.s_b + h * p.s_h + (ok ? row : 0) * p.s_l;
@@ -538,8 +539,9 @@ extern "C" int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* wi
     p.s_b = store_k->shape[0] == 1 ? 0 : store_k->stride[0];
     p.s_h = store_k->shape[1] == 1 ? 0 : store_k->stride[1];
     p.s_l = store_k->shape[2] == 1 ? 128 : store_k->stride[2];
-    PK_REQUIRE(is_contig(selected) && selected->shape[0] == bs && selected->shape[1] == H,
-               "selected must be contiguous [bs,H,K]");
+    PK_REQUIRE(selected->shape[0] == bs && selected->shape[1] == H && (K <= 1 || selected->stride[2] == 1),
+               "selected must be [bs,H,K] with last stride 1");
+    p.sel_b = selected->stride[0], p.sel_h = selected->stride[1];
     p.sk = (const uint16_t*)store_k->data, p.sv = (const uint16_t*)store_v->data;
     p.kv_pair = (p.sv == p.sk + 128 && p.s_l >= 256) ? 1 : 0;
     p.cap_s = store_k->shape[2];

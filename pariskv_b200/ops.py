@@ -20,7 +20,9 @@ def workspace(device, nbytes, tag="default"):
     """A cached scratch buffer per (device, tag) for eager calls that do not bring their own.  It grows by
     replacement, so it must not grow while a CUDA graph is being captured (a graph captured earlier would keep
     the address of the buffer that was dropped): callers that capture pass a Scratch they own instead."""
-    key = (torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device(), tag)
+    if not isinstance(device, torch.device):
+        device = torch.device(device)
+    key = (device.index if device.index is not None else torch.cuda.current_device(), tag)
     buf = _WS.get(key)
     if buf is None or buf.numel() < nbytes:
         if torch.cuda.is_current_stream_capturing():
@@ -51,11 +53,11 @@ def _scratch(device, nbytes, tag, scratch):
 
 
 def retrieve_scratch_bytes(bs, H, N, C):
-    return int(L.load().pk_retrieve_workspace_bytes(int(bs), int(H), int(N), int(C)))
+    return L.native().retrieve_workspace_bytes(bs, H, N, C)
 
 
 def attention_scratch_bytes(bs, Hq, max_rows):
-    return int(L.load().pk_attention_workspace_bytes(int(bs), int(Hq), int(max_rows)))
+    return L.native().attention_workspace_bytes(bs, Hq, max_rows)
 
 
 def attention_status(scratch_or_buf, bs, Hq):
@@ -102,8 +104,7 @@ def encode_keys(keys, signs, codebook=None, block_weight=None, packed_4bit=None,
         codebook, block_weight, packed_4bit = alloc_key_metadata(bs, H, Lk, keys.device)
     if keys.numel() == 0:
         return codebook, block_weight, packed_4bit
-    d = [L.desc(t) for t in (keys, signs, codebook, block_weight, packed_4bit, cluster_counts)]
-    _call("pk_encode_keys", *[L.ref(x) for x in d], L.stream_ptr(keys.device))
+    L.native().encode_keys(keys, signs, codebook, block_weight, packed_4bit, cluster_counts)
     return codebook, block_weight, packed_4bit
 
 
@@ -120,43 +121,21 @@ def count_clusters(codebook, counts=None, accumulate=False):
 
 def query_prep(queries, kv_heads, signs, want_avg=False):
     """queries bf16 [bs,1,Hq,128] -> q_blocks [bs,H,16,8], q_norm [bs,H,1] (, query_avg [bs,H,128])."""
-    _require_cuda(queries, signs)
-    bs = queries.shape[0]
-    dev = queries.device
-    qb = torch.empty(bs, kv_heads, 16, 8, dtype=torch.bfloat16, device=dev)
-    qn = torch.empty(bs, kv_heads, 1, dtype=torch.bfloat16, device=dev)
-    qa = torch.empty(bs, kv_heads, 128, dtype=torch.bfloat16, device=dev) if want_avg else None
-    d = [L.desc(t) for t in (queries, signs, qb, qn, qa)]
-    _call("pk_query_prep", *[L.ref(x) for x in d], L.stream_ptr(dev))
-    return (qb, qn, qa) if want_avg else (qb, qn)
+    return L.native().query_prep(queries, int(kv_heads), signs, want_avg)
 
 
 def rank_clusters(q_blocks):
-    _require_cuda(q_blocks)
-    bs, H = q_blocks.shape[:2]
-    ids = torch.empty(bs, H, 16, 256, dtype=torch.int64, device=q_blocks.device)
-    dq, di = L.desc(q_blocks), L.desc(ids)
-    _call("pk_rank_clusters", L.ref(dq), L.ref(di), L.stream_ptr(q_blocks.device))
-    return ids
+    return L.native().rank_clusters(q_blocks)
 
 
 # --------------------------------------------------------------------------------------------------
 # collision
 # --------------------------------------------------------------------------------------------------
 def collision_fused(sorted_cluster_ids, cluster_key_counts, codebook, tier_counts, cache_cnt=None):
-    _require_cuda(sorted_cluster_ids, cluster_key_counts, codebook)
-    bs, H, B, N = codebook.shape
-    dev = codebook.device
-    if cache_cnt is None:
-        cache_cnt = torch.empty(bs, H, N, dtype=torch.int32, device=dev)
-    lib = L.load()
-    nb = lib.pk_collision_workspace_bytes(bs, H, B, sorted_cluster_ids.shape[-1])
-    ws = workspace(dev, nb, "collision")
-    tiers = L.i64_array(list(tier_counts))
-    d = [L.desc(t) for t in (sorted_cluster_ids, cluster_key_counts, codebook, cache_cnt)]
-    _call("pk_collision_fused", L.ref(d[0]), L.ref(d[1]), L.ref(d[2]), tiers, len(tier_counts), L.ref(d[3]),
-          ws.data_ptr(), ws.numel(), L.stream_ptr(dev))
-    return cache_cnt
+    _require_cuda(codebook)
+    bs, H, B, _ = codebook.shape
+    ws = workspace(codebook.device, bs * H * B * 256, "collision")   # pk_collision_workspace_bytes
+    return L.native().collision_fused(sorted_cluster_ids, cluster_key_counts, codebook, tier_counts, cache_cnt, ws)
 
 
 def collision_fused_static(sorted_cluster_ids, cluster_key_counts, codebook, tier_counts, cache_cnt):
@@ -195,38 +174,19 @@ def topk(x, k, order=0):
         x = x.to(torch.int32) if not x.dtype.is_floating_point else x.to(torch.float32)
     if x.stride(-1) != 1:
         x = x.contiguous()
-    lead = x.shape[:-1]
-    x2 = x.reshape(-1, x.shape[-1])
-    out = torch.empty(x2.shape[0], k, dtype=torch.int64, device=x.device)
-    dx, do = L.desc(x2), L.desc(out)
-    _call("pk_topk", L.ref(dx), int(k), L.ref(do), int(order), L.stream_ptr(x.device))
-    return out.view(*lead, k)
+    if x.dim() != 2 and not x.is_contiguous():
+        x = x.contiguous()
+    return L.native().topk(x, int(k), int(order))
 
 
 def final_topk(scores_f32, cand, K):
-    _require_cuda(scores_f32, cand)
-    bs, H, C = scores_f32.shape
-    out = torch.empty(bs, H, K, dtype=torch.int64, device=scores_f32.device)
-    d = [L.desc(t) for t in (scores_f32, cand, out)]
-    _call("pk_final_topk", L.ref(d[0]), L.ref(d[1]), int(K), L.ref(d[2]), L.stream_ptr(scores_f32.device))
-    return out
+    return L.native().final_topk(scores_f32, cand, int(K))
 
 
 def adaptive_topk(sl_logits, cand_scores, cand_scale, sl_vnorm, cand_indices, cand_vnorm, threshold, K_out,
                   value_norm=None, sink_size=0, min_k=0, max_k=0, adaptive_k=None, topk_indices=None):
-    _require_cuda(sl_logits, cand_scores, sl_vnorm, cand_indices)
-    bs, H = sl_logits.shape[:2]
-    dev = sl_logits.device
-    if adaptive_k is None:
-        adaptive_k = torch.empty(bs, H, dtype=torch.int64, device=dev)
-    if topk_indices is None:
-        topk_indices = torch.empty(bs, H, K_out, dtype=torch.int64, device=dev)
-    d = [L.desc(t) for t in (sl_logits, cand_scores, sl_vnorm, cand_indices, cand_vnorm, value_norm, adaptive_k,
-                             topk_indices)]
-    _call("pk_adaptive_topk", L.ref(d[0]), L.ref(d[1]), float(cand_scale), L.ref(d[2]), L.ref(d[3]), L.ref(d[4]),
-          L.ref(d[5]), int(sink_size), float(threshold), int(K_out), int(min_k), int(max_k), L.ref(d[6]),
-          L.ref(d[7]), L.stream_ptr(dev))
-    return adaptive_k, topk_indices
+    return L.native().adaptive_topk(sl_logits, cand_scores, float(cand_scale), sl_vnorm, cand_indices, cand_vnorm, value_norm,
+                                    int(sink_size), float(threshold), int(K_out), int(min_k), int(max_k), adaptive_k, topk_indices)
 
 
 # --------------------------------------------------------------------------------------------------
@@ -234,26 +194,17 @@ def adaptive_topk(sl_logits, cand_scores, cand_scale, sl_vnorm, cand_indices, ca
 # --------------------------------------------------------------------------------------------------
 def rerank(coarse_indices, key_4bit, key_block_weight, q_blocks, q_norm, mag_centers, approx_scores=None,
            scores_f32=None, v4b=None, want_f32=False):
-    _require_cuda(coarse_indices, key_4bit, key_block_weight, q_blocks, q_norm, mag_centers)
-    bs, H, C = coarse_indices.shape
-    dev = coarse_indices.device
-    if approx_scores is None:
-        approx_scores = torch.empty(bs, H, C, dtype=torch.bfloat16, device=dev)
     if scores_f32 is None and want_f32:
-        scores_f32 = torch.empty(bs, H, C, dtype=torch.float32, device=dev)
-    d = [L.desc(t) for t in (coarse_indices, key_4bit, key_block_weight, q_blocks, q_norm, mag_centers,
-                             approx_scores, scores_f32, v4b)]
-    _call("pk_rerank", *[L.ref(x) for x in d], L.stream_ptr(dev))
-    return approx_scores, scores_f32
+        scores_f32 = torch.empty(coarse_indices.shape, dtype=torch.float32, device=coarse_indices.device)
+    return L.native().rerank(coarse_indices, key_4bit, key_block_weight, q_blocks, q_norm, mag_centers, approx_scores,
+                             scores_f32, v4b), scores_f32
 
 
 # --------------------------------------------------------------------------------------------------
 # gather / attention
 # --------------------------------------------------------------------------------------------------
 def h2d_gather_kv(src_k, src_v, selected_indices, dst_k, dst_v):
-    _require_cuda(selected_indices, dst_k, dst_v)
-    d = [L.desc(t) for t in (src_k, src_v, selected_indices, dst_k, dst_v)]
-    _call("pk_h2d_gather_kv", *[L.ref(x) for x in d], L.stream_ptr(dst_k.device))
+    L.native().h2d_gather_kv(src_k, src_v, selected_indices, dst_k, dst_v)
 
 
 def h2d_gather_kv_packed(src_k, src_v, k_packed, v_packed, indices_packed, cu_seqlens_topk, cu_seqlens_k,
@@ -284,31 +235,23 @@ def append_encode(k_row, v_row, signs, window_k, window_v, win_codes, win_weight
                   block_weight, packed_4bit, value_norm, cluster_counts, store_kv, state, sink, interval):
     """One decode token into the cache: window row, key coding, and the flush of a full update buffer, all positions
     read from the device-side `state` words; see pk_append_encode."""
-    _require_cuda(k_row, v_row, window_k, window_v, state)
-    d = [L.desc(t) for t in (k_row, v_row, signs, window_k, window_v, win_codes, win_weight, win_4bit, win_vnorm, codebook,
-                             block_weight, packed_4bit, value_norm, cluster_counts, store_kv, state)]
-    _call("pk_append_encode", *[L.ref(x) for x in d], int(sink), int(interval), L.stream_ptr(window_k.device))
+    L.native().append_encode(k_row, v_row, signs, window_k, window_v, win_codes, win_weight, win_4bit, win_vnorm, codebook,
+                             block_weight, packed_4bit, value_norm, cluster_counts, store_kv, state, int(sink), int(interval))
 
 
 def sparse_attention(queries, window_k, window_v, n_window, store_k=None, store_v=None, selected=None, n_sel=None,
                      index_offset=0, scale=None, out=None, n_window_dev=None, n_window_add=0, lse=None, scratch=None):
     """Decode attention over window rows [0, n_window) plus the selected rows of the K/V store (device or
     pinned host memory); see pk_sparse_attention."""
-    _require_cuda(queries, window_k, window_v, selected)
+    _require_cuda(queries)
     bs, _, Hq, D = queries.shape
-    dev = queries.device
-    if out is None:
-        out = torch.empty_like(queries)
     if scale is None:
         scale = 1.0 / math.sqrt(D)
-    K = selected.shape[2] if selected is not None else 0
-    nb = L.load().pk_attention_workspace_bytes(bs, Hq, n_window + K)
-    ws = _scratch(dev, nb, "attention", scratch)
-    d = [L.desc(t) for t in (queries, window_k, window_v, store_k, store_v, selected, n_sel, out, n_window_dev, lse)]
-    _call("pk_sparse_attention", L.ref(d[0]), L.ref(d[1]), L.ref(d[2]), int(n_window), L.ref(d[8]), int(n_window_add),
-          L.ref(d[3]), L.ref(d[4]), L.ref(d[5]), L.ref(d[6]), int(index_offset), float(scale), L.ref(d[7]), L.ref(d[9]),
-          ws.data_ptr(), ws.numel(), L.stream_ptr(dev))
-    return out
+    N = L.native()
+    rows = n_window + (selected.shape[2] if selected is not None else 0)
+    ws = _scratch(queries.device, N.attention_workspace_bytes(bs, Hq, rows), "attention", scratch)
+    return N.sparse_attention(queries, window_k, window_v, int(n_window), n_window_dev, int(n_window_add), store_k, store_v,
+                              selected, n_sel, int(index_offset), float(scale), out, lse, ws)
 
 
 # --------------------------------------------------------------------------------------------------
@@ -367,43 +310,16 @@ def retrieve_ex(queries, signs, mag_centers, codebook, key_block_weight, key_4bi
         if name not in extras:
             shape, dt = shapes[name]
             extras[name] = torch.empty(*shape, dtype=dt, device=dev)
-    if phase != 1:
-        if final_indices is None and K > 0:
-            final_indices = torch.empty(bs, H, K, dtype=torch.int64, device=dev)
-        if n_sel is None and K > 0:
-            n_sel = torch.empty(bs, H, dtype=torch.int32, device=dev)
-        if n_cand is None:
-            n_cand = torch.empty(bs, H, dtype=torch.int32, device=dev)
+    if phase != 1 and n_cand is None:
+        n_cand = torch.empty(bs, H, dtype=torch.int32, device=dev)
     if phase == 1 and local_hist is None:
         local_hist = torch.empty(bs, H, 256, dtype=torch.int32, device=dev)
-    nb = retrieve_scratch_bytes(bs, H, N, row)
-    ws = _scratch(dev, nb, "retrieve", scratch)
-    a = L.PkRetrieveArgs()
-    keep = []
-
-    def put(field, t):
-        if t is not None:
-            d = L.desc(t)
-            keep.append(d)
-            setattr(a, field, L.ptr(d))
-
-    for field, t in (("queries", queries), ("signs", signs), ("mag_centers", mag_centers), ("codebook", codebook),
-                     ("key_block_weight", key_block_weight), ("key_4bit", key_4bit),
-                     ("cluster_key_counts", cluster_key_counts), ("kv_len", kv_len), ("local_hist", local_hist),
-                     ("shard_hist", shard_hist), ("final_indices", final_indices), ("n_sel", n_sel),
-                     ("cand", extras.get("cand")), ("n_cand", n_cand), ("scores_f32", extras.get("scores_f32")),
-                     ("q_blocks", extras.get("q_blocks")), ("q_norm", extras.get("q_norm")),
-                     ("query_avg", extras.get("query_avg"))):
-        put(field, t)
-    if tier_counts is not None:
-        tiers = L.i64_array(list(tier_counts))
-        a.tier_counts, a.n_tiers = tiers, len(tier_counts)
-    if schedule is not None:
-        a.schedule = ctypes.pointer(schedule)
-    a.phase, a.C, a.K, a.world, a.rank = int(phase), int(C), int(K), int(world), int(rank)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    a.queries_settled = 1 if queries_settled else 0
-    _call("pk_retrieve_ex", ctypes.byref(a), L.stream_ptr(dev))
+    ws = _scratch(dev, retrieve_scratch_bytes(bs, H, N, row), "retrieve", scratch)
+    final_indices, n_sel = L.native().retrieve_ex(
+        queries, signs, mag_centers, codebook, key_block_weight, key_4bit, cluster_key_counts, int(C), int(K), tier_counts, kv_len,
+        ctypes.addressof(schedule) if schedule is not None else 0, phase, local_hist, shard_hist, world, rank,
+        final_indices, n_sel, extras.get("cand"), n_cand, extras.get("scores_f32"), extras.get("q_blocks"),
+        extras.get("q_norm"), extras.get("query_avg"), ws, queries_settled)
     extras["n_cand"] = n_cand
     extras["local_hist"] = local_hist
     return final_indices, n_sel, extras
@@ -536,40 +452,21 @@ def qk_norm_rope(qkv, weight, cos, sin, eps=1e-6, out=None):
     """Per-head RMS-norm and rotate-half RoPE of the q and k heads of a fused q/k/v row in one launch.
     qkv bf16 [B, >= heads*128]; weight bf16 [heads,128]; cos / sin bf16 [1 or B,128] (sin = [-sin, sin]).
     Returns bf16 [B, heads, 128].  See pk_qk_norm_rope."""
-    _require_cuda(qkv, weight, cos, sin)
-    B, heads = qkv.shape[0], weight.shape[0]
-    if out is None:
-        out = torch.empty(B, heads, 128, dtype=torch.bfloat16, device=qkv.device)
-    d = [L.desc(t) for t in (qkv, weight, cos, sin, out)]
-    _call("pk_qk_norm_rope", *[L.ref(x) for x in d], float(eps), L.stream_ptr(qkv.device))
-    return out
+    return L.native().qk_norm_rope(qkv, weight, cos, sin, eps, out)
 
 
 def add_rmsnorm(a, residual, weight, eps=1e-6):
     """h = a + residual (residual may be None), x = RMS-norm(h) * weight, one launch.  Returns (h, x).
     See pk_add_rmsnorm."""
-    _require_cuda(a, weight)
-    h, x = torch.empty_like(a), torch.empty_like(a)
-    d = [L.desc(t) if t is not None else None for t in (a, residual, weight, h, x)]
-    _call("pk_add_rmsnorm", *[L.ref(t) if t is not None else None for t in d], float(eps), L.stream_ptr(a.device))
-    return h, x
+    return L.native().add_rmsnorm(a, residual, weight, eps)
 
 
 def silu_mul(gate_up):
     """silu(gate_up[:, :F]) * gate_up[:, F:], one launch.  See pk_silu_mul."""
-    _require_cuda(gate_up)
-    out = torch.empty(gate_up.shape[0], gate_up.shape[1] // 2, dtype=torch.bfloat16, device=gate_up.device)
-    d = [L.desc(gate_up), L.desc(out)]
-    _call("pk_silu_mul", L.ref(d[0]), L.ref(d[1]), L.stream_ptr(gate_up.device))
-    return out
+    return L.native().silu_mul(gate_up)
 
 
 def gemv(weight, x, gated=False):
     """x [1, I] @ weight[O, I]^T -> [1, O] (bf16, fp32 accumulation) for one token; gated: weight = [gate; up] stacked,
     result [1, O/2] = silu(gate x) * (up x).  See pk_gemv."""
-    _require_cuda(weight, x)
-    O = weight.shape[0]
-    out = torch.empty(1, O // 2 if gated else O, dtype=torch.bfloat16, device=x.device)
-    d = [L.desc(weight), L.desc(x), L.desc(out)]
-    _call("pk_gemv", L.ref(d[0]), L.ref(d[1]), L.ref(d[2]), int(bool(gated)), L.stream_ptr(x.device))
-    return out
+    return L.native().gemv(weight, x, gated)

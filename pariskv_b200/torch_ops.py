@@ -25,6 +25,14 @@ import torch
 
 from . import ops
 
+
+def direct(t) -> bool:
+    """Whether a mirror module may call `ops` itself instead of torch.ops.pariskv.*: a plain eager tensor, nothing
+    traced and no dispatch mode on.  The dispatcher and the Python kernel behind it cost about 10 us a call, more than
+    most of these operators take on the GPU."""
+    return type(t) is torch.Tensor and not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0
+
+
 _lib = torch.library.Library("pariskv", "DEF")
 _lib.define("collision(Tensor sorted_cluster_ids, Tensor topk_cluster_cnt, Tensor code_book) -> Tensor")
 _lib.define("collision_fused(Tensor sorted_cluster_ids, Tensor cluster_key_counts, Tensor codebook, int[] tier_counts) -> Tensor")
