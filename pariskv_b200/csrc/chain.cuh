@@ -1,0 +1,297 @@
+// Device pieces of the retrieval chain that its kernels share: register sort of the clusters of a subspace, query
+// rotation over one warp, 4-bit rerank of one candidate, block scan.
+#pragma once
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace pk {
+namespace {
+
+// byte k (0..3) of w, zero-extended: one PRMT
+__device__ __forceinline__ unsigned byte_of(uint32_t w, int k) { return __byte_perm(w, 0, 0x4440 | k); }
+
+// Sorts the 256 keys of a warp (8 per lane, element index e = 8 * lane + r) into DESCENDING order of e with a
+// bitonic network: exchanges at distance < 8 stay inside a lane, the others are xor shuffles.  Keys are distinct.
+// The merges run as loops over two small bodies: fully unrolled the network is 1500 instructions that every warp runs
+// once, and a kernel that starts with it waits for instruction fetches (a third of its stalls, measured).
+// A block that has to end ascending is sorted as complements, so every exchange inside a lane is one max and one min.
+__device__ __forceinline__ void lane_exchange(unsigned (&v)[8], int r, int l, bool up) {
+  const unsigned a = v[r], b = v[l], mx = max(a, b), mn = min(a, b);
+  v[r] = up ? mx : mn;
+  v[l] = up ? mn : mx;
+}
+__device__ __forceinline__ void warp_sort_desc_256(unsigned (&v)[8], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 4; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int r = 0; r < 8; r++)
+        if ((r ^ j) > r) lane_exchange(v, r, r ^ j, (r & k) == 0);
+#pragma unroll 1
+  for (int k = 8; k <= 256; k <<= 1) {
+    const unsigned flip = ((lane << 3) & k) ? 0xffffffffu : 0u;   // blocks with this bit set end ascending
+#pragma unroll
+    for (int r = 0; r < 8; r++) v[r] ^= flip;
+#pragma unroll 1
+    for (int lj = k >> 4; lj > 0; lj >>= 1) {
+      const bool take_max = (lane & lj) == 0;   // the lower element of a pair keeps the maximum
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const unsigned o = __shfl_xor_sync(0xffffffffu, v[r], lj);
+        v[r] = take_max ? max(v[r], o) : min(v[r], o);
+      }
+    }
+#pragma unroll
+    for (int j = 4; j > 0; j >>= 1)
+#pragma unroll
+      for (int r = 0; r < 8; r++)
+        if ((r ^ j) > r) lane_exchange(v, r, r ^ j, true);
+#pragma unroll
+    for (int r = 0; r < 8; r++) v[r] ^= flip;
+  }
+}
+
+// x: dims [4*lane, 4*lane+4) of the group-mean query (bf16 values as floats); sg: their SRHT signs.
+// Same pairwise trees and butterflies as rotate16, spread over 32 lanes.  Returns the bf16 norm.
+__device__ __forceinline__ float rotate4(float (&x)[4], const float (&sg)[4], int lane) {
+  float t0 = __fadd_rn(__fmul_rn(x[0], x[0]), __fmul_rn(x[1], x[1]));
+  float t1 = __fadd_rn(__fmul_rn(x[2], x[2]), __fmul_rn(x[3], x[3]));
+  float sum = __fadd_rn(t0, t1);
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, off));
+  const float n = bfround(__fsqrt_rn(sum));
+  const float den = fmaxf(n, bfround(1e-8f));
+#pragma unroll
+  for (int i = 0; i < 4; i++) x[i] = __fmul_rn(bfround(__fdiv_rn(x[i], den)), sg[i]);
+  {  // h = 1, 2 inside the lane
+    float a = x[0], b = x[1], c = x[2], d = x[3];
+    x[0] = __fadd_rn(a, b), x[1] = __fsub_rn(a, b), x[2] = __fadd_rn(c, d), x[3] = __fsub_rn(c, d);
+    a = x[0], b = x[1], c = x[2], d = x[3];
+    x[0] = __fadd_rn(a, c), x[2] = __fsub_rn(a, c), x[1] = __fadd_rn(b, d), x[3] = __fsub_rn(b, d);
+  }
+#pragma unroll
+  for (int bit = 1; bit < 32; bit <<= 1)  // h = 4 .. 64 across lanes
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float pv = __shfl_xor_sync(0xffffffffu, x[i], bit);
+      x[i] = (lane & bit) ? __fsub_rn(pv, x[i]) : __fadd_rn(x[i], pv);
+    }
+#pragma unroll
+  for (int i = 0; i < 4; i++) x[i] = bfround(__fmul_rn(x[i], 0.08838834764831845f));
+  return n;
+}
+
+// Ranks the 256 clusters of a subspace by (score descending, id ascending), the scores being the sums of +-q over the
+// bits of the cluster id: on return element e = 8 * lane + r of the order is cluster 255 - (key[r] & 255).
+// Register r of a lane starts with cluster c = 32 * r + lane: the first five terms of the score (bits 0..4 of c) are the
+// lane's, the last three (bits 5..7) the register's; the sum is taken in the order j = 0..7.
+__device__ __forceinline__ void rank_subspace(unsigned (&key)[8], const float* q8, int lane) {
+  float qv[8];
+#pragma unroll
+  for (int j = 0; j < 8; j++) qv[j] = q8[j];
+  float s5 = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 5; j++) s5 = __fadd_rn(s5, ((lane >> j) & 1) ? qv[j] : -qv[j]);
+#pragma unroll
+  for (int rr = 0; rr < 8; rr++) {
+    float sc = s5;
+#pragma unroll
+    for (int j = 5; j < 8; j++) sc = __fadd_rn(sc, ((rr >> (j - 5)) & 1) ? qv[j] : -qv[j]);
+    // order of (score descending, id ascending) as one unsigned compare; -0 counts as +0 like a float compare
+    unsigned bits = f2bf(sc);
+    if (bits == 0x8000u) bits = 0u;
+    const unsigned ord = (bits & 0x8000u) ? (~bits & 0xFFFFu) : (bits | 0x8000u);
+    key[rr] = (ord << 8) | (unsigned)(255 - (32 * rr + lane));
+  }
+  warp_sort_desc_256(key, lane);
+}
+
+// Sixteen times the sum over the 16 subspaces of a key of the tier count of its code.  lut: [16][128] bytes, entry c of a
+// subspace is nibble c >> 7 of byte c & 127: 128 bytes, one word per bank, so the 32 look-ups of a warp never conflict.
+// The integer ALU bounds this (half rate on sm_100a): eight of its instructions per four look-ups.  The four table
+// bytes are joined by multiply-adds, which run on the FMA pipe; c256 = 256 comes from a kernel argument, because
+// the compiler turns a multiplication by a known power of two into ALU shifts.
+__device__ __forceinline__ unsigned tier_sum16(uint4 cw, const uint8_t* lut, unsigned c256) {
+  const uint32_t w4[4] = {cw.x, cw.y, cw.z, cw.w};
+  unsigned acc = 0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const uint32_t w = w4[i], at = w & 0x7f7f7f7fu;
+    const uint8_t* t = lut + 4 * i * 128;
+    const unsigned b0 = t[byte_of(at, 0)], b1 = t[128 + byte_of(at, 1)], b2 = t[256 + byte_of(at, 2)], b3 = t[384 + byte_of(at, 3)];
+    const uint32_t v = ((b3 * c256 + b2) * c256 + b1) * c256 + b0;
+    uint32_t high;   // 0xff where the code is 128 or more: its nibble is the high one (the intrinsic drops the sign mode)
+    asm("prmt.b32 %0, %1, %2, 0xba98;" : "=r"(high) : "r"(w), "r"(0u));
+    // the wanted nibble of every byte in place, times 16 (low) or 1 (high)
+    acc = __dp4a(v & (high ^ 0x0f0f0f0fu), (high & 0x01010101u) | (~high & 0x10101010u), acc);
+  }
+  return acc;
+}
+
+__device__ __forceinline__ void unpack4(uint2 v, float* out) {
+  out[0] = __uint_as_float(v.x << 16), out[1] = __uint_as_float(v.x & 0xffff0000u);
+  out[2] = __uint_as_float(v.y << 16), out[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+
+struct RerankSmem {
+  float lev[16][32];  // lev[nibble][lane]
+  float q[128];
+};
+
+__device__ __forceinline__ void rerank_setup(RerankSmem& sm, const RerankArgs& a, int64_t bh, int tid, int nthreads) {
+  for (int i = tid; i < 16 * 32; i += nthreads) {
+    const int nib = i >> 5;
+    const float c = bf2f(a.centers[nib & 7]);
+    sm.lev[nib][i & 31] = (nib & 8) ? c : -c;
+  }
+  for (int i = tid; i < 128; i += nthreads) sm.q[i] = bf2f(a.q_blocks[bh * 128 + i]);
+}
+
+// FAST: key-major, 16-byte aligned records.  Returns the fp32 score of key `key`.
+template <bool FAST>
+__device__ __forceinline__ float rerank_one(const RerankSmem& sm, const RerankArgs& a, const uint8_t* k4,
+                                            const uint16_t* w, int64_t key, float qn, int lane, uint16_t* v4b_row,
+                                            int64_t v4b_sub_stride) {
+  uint32_t code[16];
+  uint32_t wt[8];
+  if (FAST) {
+    const uint4* cp = reinterpret_cast<const uint4*>(k4 + key * 64);
+    const uint4* wp = reinterpret_cast<const uint4*>(w + key * 16);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint4 v = __ldg(cp + i);
+      code[4 * i] = v.x, code[4 * i + 1] = v.y, code[4 * i + 2] = v.z, code[4 * i + 3] = v.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const uint4 v = __ldg(wp + i);
+      wt[4 * i] = v.x, wt[4 * i + 1] = v.y, wt[4 * i + 2] = v.z, wt[4 * i + 3] = v.w;
+    }
+  } else {
+#pragma unroll
+    for (int s = 0; s < 16; s++) {
+      const uint8_t* cp = k4 + s * a.k4_s + key * a.k4_l;
+      code[s] = (uint32_t)cp[0] | ((uint32_t)cp[1] << 8) | ((uint32_t)cp[2] << 16) | ((uint32_t)cp[3] << 24);
+    }
+#pragma unroll
+    for (int s = 0; s < 8; s++)
+      wt[s] = (uint32_t)w[(2 * s) * a.w_s + key * a.w_l] | ((uint32_t)w[(2 * s + 1) * a.w_s + key * a.w_l] << 16);
+  }
+  float acc = 0.0f;
+#pragma unroll
+  for (int s = 0; s < 16; s++) {
+    const float4 q0 = *reinterpret_cast<const float4*>(&sm.q[8 * s]);
+    const float4 q1 = *reinterpret_cast<const float4*>(&sm.q[8 * s + 4]);
+    const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    float dot = 0.0f;
+    float lv[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      lv[j] = sm.lev[(code[s] >> (4 * j)) & 0xFu][lane];
+      dot = __fmaf_rn(lv[j], qv[j], dot);
+    }
+    if (v4b_row) {
+      uint32_t o[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) o[j] = (uint32_t)f2bf(lv[2 * j]) | ((uint32_t)f2bf(lv[2 * j + 1]) << 16);
+      *reinterpret_cast<uint4*>(v4b_row + s * v4b_sub_stride) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    const float wf = __uint_as_float((s & 1) ? (wt[s >> 1] & 0xffff0000u) : (wt[s >> 1] << 16));
+    acc = __fmaf_rn(dot, wf, acc);
+  }
+  return __fmul_rn(acc, qn);
+}
+
+// The rerank of one candidate from key-major records, for kernels that rank many candidates per block.
+// Levels are looked up two at a time: entry v of lev2 holds the bf16 levels of the nibbles v & 15 and v >> 4, one copy
+// per lane (word v * 32 + lane: never a bank conflict), so a record costs 64 look-ups instead of 128.  Two subspaces
+// run side by side in packed fp32 multiply-adds; every subspace keeps its own chain over j, then
+// acc = fma(dot, w_b, acc) over b ascending, so the result has the bits of rerank_one.
+// Three instructions per dimension; c128 = 128 and c64k = 65536 come from kernel arguments, because multiplications by
+// known powers of two become shifts on the integer ALU (half rate), which is what bounds the loop.
+// Four lanes per candidate (whole sectors per load, the query in registers) measured 15 % slower: passing the sum from
+// lane to lane costs more instructions than the query's shared-memory reads.
+constexpr int LEV2_BYTES = 256 * 32 * 4;
+
+__device__ __forceinline__ void build_lev2(uint32_t* lev2, const uint16_t* __restrict__ centers, int tid, int nthreads) {
+  for (int v = tid >> 5; v < 256; v += nthreads >> 5) {
+    const uint32_t a = __ldg(centers + (v & 7)), b = __ldg(centers + ((v >> 4) & 7));
+    lev2[v * 32 + (tid & 31)] = ((v & 8) ? a : a ^ 0x8000u) | (((v & 0x80) ? b : b ^ 0x8000u) << 16);
+  }
+}
+// where dimension d of the query goes in the array rerank_pairs reads: for the subspaces 2p, 2p + 1 and the dimensions
+// 2i, 2i + 1 of a subspace, float4 p * 4 + i = (q[2p][2i], q[2p + 1][2i], q[2p][2i + 1], q[2p + 1][2i + 1])
+__device__ __forceinline__ int pair_slot(int d) {
+  const int sub = d >> 3, j = d & 7;
+  return ((sub >> 1) * 4 + (j >> 1)) * 4 + (j & 1) * 2 + (sub & 1);
+}
+__device__ __forceinline__ void load_record(uint4 (&rec)[6], const uint8_t* k4, const uint16_t* w, int64_t key) {
+  const uint4* cp = reinterpret_cast<const uint4*>(k4 + key * 64);
+  const uint4* wp = reinterpret_cast<const uint4*>(w + key * 16);
+#pragma unroll
+  for (int i = 0; i < 4; i++) rec[i] = __ldg(cp + i);
+  rec[4] = __ldg(wp), rec[5] = __ldg(wp + 1);
+}
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float rerank_pairs(const uint4 (&rec)[6], const uint32_t* lev2, const float4* q2, float qn, int lane,
+                                              unsigned c128, unsigned c64k) {
+  const uint32_t code[16] = {rec[0].x, rec[0].y, rec[0].z, rec[0].w, rec[1].x, rec[1].y, rec[1].z, rec[1].w,
+                             rec[2].x, rec[2].y, rec[2].z, rec[2].w, rec[3].x, rec[3].y, rec[3].z, rec[3].w};
+  const uint32_t wt[8] = {rec[4].x, rec[4].y, rec[4].z, rec[4].w, rec[5].x, rec[5].y, rec[5].z, rec[5].w};
+  const uint8_t* base = reinterpret_cast<const uint8_t*>(lev2) + lane * 4;
+  float acc = 0.0f;
+#pragma unroll
+  for (int p = 0; p < 8; p++) {
+    unsigned long long dot = 0ull;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float4 q = q2[p * 4 + i];
+      const uint32_t a = *reinterpret_cast<const uint32_t*>(base + byte_of(code[2 * p], i) * c128);
+      const uint32_t b = *reinterpret_cast<const uint32_t*>(base + byte_of(code[2 * p + 1], i) * c128);
+      dot = fma2(pack2(__uint_as_float(a * c64k), __uint_as_float(b * c64k)), pack2(q.x, q.y), dot);
+      dot = fma2(pack2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)), pack2(q.z, q.w), dot);
+    }
+    float d0, d1;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d0), "=f"(d1) : "l"(dot));
+    acc = __fmaf_rn(d0, __uint_as_float(wt[p] << 16), acc);
+    acc = __fmaf_rn(d1, __uint_as_float(wt[p] & 0xffff0000u), acc);
+  }
+  return __fmul_rn(acc, qn);
+}
+
+// Block-wide exclusive scan of a packed pair of counters; returns (exclusive prefix, block total).
+template <int NT>
+__device__ __forceinline__ unsigned long long block_scan_excl(unsigned long long mine, unsigned long long* s_scan,
+                                                              unsigned long long* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long sc = mine;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned long long o = __shfl_up_sync(0xffffffffu, sc, off);
+    if (lane >= off) sc += o;
+  }
+  if (lane == 31) s_scan[warp] = sc;
+  __syncthreads();
+  unsigned long long before = 0, tot = 0;
+#pragma unroll
+  for (int w = 0; w < NT / 32; w++) {
+    const unsigned long long v = s_scan[w];
+    if (w < warp) before += v;
+    tot += v;
+  }
+  *total = tot;
+  return before + sc - mine;
+}
+
+}  // namespace
+}  // namespace pk

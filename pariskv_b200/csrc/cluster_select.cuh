@@ -1,0 +1,341 @@
+// Exact top-K of a row that is spread over the CTAs of a thread-block cluster (each holds a contiguous slice):
+// first K of (value descending, position ascending), emitted in ascending position.
+//
+//   extremes of the row                      -> 256 linear value bins, about equally filled
+//   histogram of the bins, summed over ranks -> the bin of the K-th largest, this CTA's share above it and in it
+//   the elements of that bin, gathered by every CTA, cut once more into 64 sub-bins and ranked -> the exact threshold
+//   ordered emission of this CTA's elements at its offset.
+// Where more than SEL_TIES elements share the bin (flat rows, equal counts), further levels bin their ordered keys; if
+// that many are equal, the lowest positions win.  Three exchanges through distributed shared memory in the usual case.
+// What bounds it is their latency and three passes over the slice: 7 us for 13 K scores over 8 CTAs, where one CTA took 12.
+#pragma once
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace pk {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int SEL_THREADS = 512;
+constexpr int SEL_WARPS = SEL_THREADS / 32;
+constexpr int SEL_BINS = 256;
+constexpr int SEL_SUB = 64;
+constexpr int SEL_TIES = 1024;
+constexpr int SEL_REGION = 2 * SEL_TIES * 8;   // bytes of dynamic shared memory, at the same offset in every CTA
+
+struct F32Row {
+  static __device__ __forceinline__ float val(uint32_t u) { return __uint_as_float(u); }
+  static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key(__uint_as_float(u)); }
+  static __device__ __forceinline__ float from_key(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k); }
+};
+struct I32Row {
+  static __device__ __forceinline__ float val(uint32_t u) { return (float)(int32_t)u; }
+  static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key((int32_t)u); }
+  static __device__ __forceinline__ float from_key(uint32_t k) { return (float)(int32_t)(k ^ 0x80000000u); }
+};
+
+struct SelShared {               // static: what other CTAs of the cluster read, and small block-wide results
+  unsigned hist[2][SEL_BINS];    // local histograms, used alternately
+  unsigned kmin, kmax;           // extremes of the ordered keys of this slice
+  unsigned n_members;            // local elements of the threshold bin
+  unsigned thr_key, thr_pos;     // the last element taken from the threshold bin
+  unsigned lower_sel;            // elements taken from the threshold bin by lower ranks
+  unsigned res[5];               // threshold bin, elements above it, elements in it, the same two of lower ranks
+  unsigned range[2];
+  unsigned warp_a[SEL_WARPS], warp_b[SEL_WARPS];
+  unsigned sub[SEL_SUB], n_few;
+};
+
+template <int CS>
+__device__ __forceinline__ void sync_cluster(cg::cluster_group& cluster) {
+  if (CS == 1) __syncthreads();
+  else cluster.sync();
+}
+
+// Threshold of a histogram spread over the cluster: thread t sums bin t over the local histograms of all CTAs, a
+// block-wide suffix scan finds the highest bin with (elements in bins >= it) >= want; see SelShared::res.  Returns after
+// the result is visible to the block.
+template <int CS, int BINS>
+__device__ __forceinline__ void cluster_threshold(cg::cluster_group& cluster, SelShared& s, const unsigned* mine, unsigned rank,
+                                                  unsigned want) {
+  static_assert(BINS <= SEL_THREADS, "one bin per thread");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned tot = 0, pre = 0;
+  if (tid < BINS) {
+    if (CS == 1) {
+      tot = mine[tid];
+    } else {
+      unsigned v[CS];
+#pragma unroll
+      for (int r = 0; r < CS; r++) v[r] = cluster.map_shared_rank(mine, r)[tid];
+#pragma unroll
+      for (int r = 0; r < CS; r++) {
+        tot += v[r];
+        if ((unsigned)r < rank) pre += v[r];
+      }
+    }
+  }
+  unsigned suf = tot, psuf = pre;   // inclusive suffix over the lanes
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned o = __shfl_down_sync(0xffffffffu, suf, off), q = __shfl_down_sync(0xffffffffu, psuf, off);
+    if (lane + off < 32) suf += o, psuf += q;
+  }
+  if (lane == 0) s.warp_a[warp] = suf, s.warp_b[warp] = psuf;
+  __syncthreads();
+  for (int w = warp + 1; w < (BINS + 31) / 32; w++) suf += s.warp_a[w], psuf += s.warp_b[w];
+  const unsigned above = suf - tot;
+  if (tot && above < want && suf >= want)
+    s.res[0] = (unsigned)tid, s.res[1] = above, s.res[2] = tot, s.res[3] = psuf - pre, s.res[4] = pre;
+  __syncthreads();
+}
+
+// n: elements of this slice; at(i): raw 32 bits of element i; out_of(i): the 64-bit value to emit for it.
+// kmin / kmax: this thread's share of the extremes of the slice's ordered keys (~0 / 0 without any).
+// region: SEL_REGION bytes; words: 2 * words_cap words of this CTA's shared memory for ballots (longer slices are
+// evaluated again instead).  All CTAs of the cluster call this with the same K (>= 1, at most the row's length).
+// The caller must not leave before cluster.barrier_wait() if CS > 1: the closing arrive is done here.
+template <int CS, class V, class At, class OutOf>
+__device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelShared& s, unsigned* region, unsigned* words,
+                                               int words_cap, unsigned rank, int n, int K, int64_t* __restrict__ out, At at,
+                                               OutOf out_of, unsigned kmin, unsigned kmax) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto publish_range = [&]() {   // extremes over the cluster, to s.range; clears the histogram replicas
+    kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if (lane == 0) s.warp_a[warp] = kmin, s.warp_b[warp] = kmax;
+    __syncthreads();
+    if (warp == 0) {
+      const unsigned lo = __reduce_min_sync(0xffffffffu, s.warp_a[lane & (SEL_WARPS - 1)]);
+      const unsigned hi = __reduce_max_sync(0xffffffffu, s.warp_b[lane & (SEL_WARPS - 1)]);
+      if (lane == 0) s.kmin = lo, s.kmax = hi;
+    }
+    for (int i = tid; i < 4 * SEL_BINS; i += SEL_THREADS) region[i] = 0;
+    sync_cluster<CS>(cluster);
+    if (warp == 0) {
+      unsigned lo = 0xffffffffu, hi = 0u;
+      if (lane < CS) {
+        lo = CS == 1 ? s.kmin : *cluster.map_shared_rank(&s.kmin, lane);
+        hi = CS == 1 ? s.kmax : *cluster.map_shared_rank(&s.kmax, lane);
+      }
+      lo = __reduce_min_sync(0xffffffffu, lo), hi = __reduce_max_sync(0xffffffffu, hi);
+      if (lane == 0) s.range[0] = lo, s.range[1] = hi;
+    }
+    __syncthreads();
+  };
+  unsigned* my_hist = region + (lane & 3) * SEL_BINS;
+  auto publish_hist = [&](int buf) {
+    __syncthreads();
+    if (tid < SEL_BINS) s.hist[buf][tid] = region[tid] + region[SEL_BINS + tid] + region[2 * SEL_BINS + tid] + region[3 * SEL_BINS + tid];
+    sync_cluster<CS>(cluster);
+  };
+  // ---- level 0: linear value bins ----
+  publish_range();
+  const float vmin = V::from_key(s.range[0]);
+  float scale = (float)(SEL_BINS - 1) / (V::from_key(s.range[1]) - vmin);
+  if (!(scale > 0.0f) || !(scale < INFINITY)) scale = 0.0f;   // flat or non-finite: one bin, the key levels decide
+  auto bin0 = [&](uint32_t u) -> unsigned { return min((unsigned)(SEL_BINS - 1), (unsigned)((V::val(u) - vmin) * scale)); };
+#pragma unroll 4
+  for (int i = tid; i < n; i += SEL_THREADS) atomicAdd(&my_hist[bin0(at(i))], 1u);
+  publish_hist(1);
+  cluster_threshold<CS, SEL_BINS>(cluster, s, s.hist[1], rank, (unsigned)K);
+  const unsigned T0 = s.res[0];
+  unsigned rem = (unsigned)K - s.res[1], in_bin = s.res[2], pre_above = s.res[3], pre_in = s.res[4];
+  // ---- key levels: ordered keys of the members between their extremes ----
+  unsigned lo = 0u, hi = 0xffffffffu;
+  int buf = 0;
+  while (in_bin > (unsigned)SEL_TIES && lo != hi) {
+    kmin = 0xffffffffu, kmax = 0u;
+#pragma unroll 1
+    for (int i = tid; i < n; i += SEL_THREADS) {
+      const uint32_t u = at(i), k = V::key(u);
+      if (bin0(u) == T0 && k >= lo && k <= hi) kmin = min(kmin, k), kmax = max(kmax, k);
+    }
+    __syncthreads();   // s.res and the replicas have been read
+    publish_range();
+    const unsigned base = s.range[0], top = s.range[1];
+    if (base == top) {
+      lo = hi = base;
+      break;
+    }
+    const int shift = max(0, 24 - __clz(top - base));   // (top - base) >> shift < SEL_BINS
+#pragma unroll 1
+    for (int i = tid; i < n; i += SEL_THREADS) {
+      const uint32_t u = at(i), k = V::key(u);
+      if (bin0(u) == T0 && k >= base && k <= top) atomicAdd(&my_hist[(k - base) >> shift], 1u);
+    }
+    publish_hist(buf);
+    cluster_threshold<CS, SEL_BINS>(cluster, s, s.hist[buf], rank, rem);
+    lo = base + (s.res[0] << shift);
+    hi = min(lo + ((1u << shift) - 1u), top);
+    rem -= s.res[1], in_bin = s.res[2], pre_above += s.res[3], pre_in = s.res[4];
+    buf ^= 1;
+  }
+  const bool flat = in_bin > (unsigned)SEL_TIES;   // that many equal keys: the lowest positions win, rank by rank
+  const bool level0 = lo == 0u && hi == 0xffffffffu;
+
+  // ---- where every element stands: above the threshold bin, in it, below; ballots of 32 consecutive elements ----
+  const int wn = ((n + SEL_WARPS - 1) / SEL_WARPS + 31) / 32 * 32;   // a warp owns consecutive elements
+  const int i0 = min(n, warp * wn), i1 = min(n, i0 + wn);
+  auto standing = [&](int i, bool& above, bool& member) {
+    above = member = false;
+    if (i < i1) {
+      const uint32_t u = at(i);
+      const unsigned bn = bin0(u);
+      above = bn > T0, member = bn == T0;
+      if (!level0 && member) {
+        const unsigned k = V::key(u);
+        above = k > hi, member = k >= lo && k <= hi;
+      }
+    }
+  };
+  uint2* own = reinterpret_cast<uint2*>(region);   // this CTA's members: (key, rank and position)
+  uint2* all = own + SEL_TIES;                     // everybody's, in rank order
+  const bool kept = (n + 31) / 32 <= words_cap;
+  unsigned* above_w = words;
+  unsigned* member_w = words + words_cap;
+  __syncthreads();   // the histogram replicas under `own` have been read
+  if (tid == 0) s.n_members = 0, s.lower_sel = 0, s.n_few = 0;
+  if (tid < SEL_SUB) s.sub[tid] = 0;
+  __syncthreads();
+  if (kept || !flat) {
+#pragma unroll 1
+    for (int i = i0; i < i1; i += 32) {
+      bool above, member;
+      standing(i + lane, above, member);
+      const unsigned aw = __ballot_sync(0xffffffffu, above), mw = __ballot_sync(0xffffffffu, member);
+      if (kept && lane == 0) above_w[i >> 5] = aw, member_w[i >> 5] = mw;
+      if (!flat && mw) {
+        unsigned slot = 0;
+        if (lane == 0) slot = atomicAdd(&s.n_members, (unsigned)__popc(mw));
+        slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(mw & ((1u << lane) - 1u));
+        if (member && slot < (unsigned)SEL_TIES) own[slot] = make_uint2(V::key(at(i + lane)), (rank << 27) | (unsigned)(i + lane));
+      }
+    }
+  }
+  unsigned thr_key = 0u, thr_pos = 0xffffffffu, lower_sel = min(pre_in, rem);
+  if (!flat) {
+    sync_cluster<CS>(cluster);
+    unsigned before_me = 0, n_all = 0;
+    if (CS == 1) {
+      all = own, n_all = s.n_members;
+    } else {
+      const unsigned m = lane < CS ? *cluster.map_shared_rank(&s.n_members, lane) : 0u;
+      unsigned inc = m;
+#pragma unroll
+      for (int off = 1; off < CS; off <<= 1) {
+        const unsigned o = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += o;
+      }
+      n_all = min(__shfl_sync(0xffffffffu, inc, CS - 1), (unsigned)SEL_TIES);
+      before_me = __shfl_sync(0xffffffffu, inc - m, rank);
+      const unsigned off = __shfl_sync(0xffffffffu, inc - m, warp & (CS - 1)), c = __shfl_sync(0xffffffffu, m, warp & (CS - 1));
+      if (warp < CS) {   // warp w copies rank w's members
+        const uint2* src = cluster.map_shared_rank(own, warp);
+        for (unsigned i = lane; i < c && off + i < (unsigned)SEL_TIES; i += 32) all[off + i] = src[i];
+      }
+      __syncthreads();
+    }
+    // the members' place within the threshold bin: ranks have to be counted out only in the sub-bin of the last one taken
+    auto sub_of = [&](unsigned k) -> unsigned {
+      return level0 && scale > 0.0f
+                 ? min((unsigned)(SEL_SUB - 1), (unsigned)max(0.0f, ((V::from_key(k) - vmin) * scale - (float)T0) * (float)SEL_SUB))
+                 : 0u;
+    };
+    for (unsigned t = tid; t < n_all; t += SEL_THREADS) atomicAdd(&s.sub[sub_of(all[t].x)], 1u);
+    __syncthreads();
+    if (warp == 0) {   // lane l: sub-bins 2l, 2l + 1
+      const unsigned c0 = s.sub[2 * lane], c1 = s.sub[2 * lane + 1];
+      unsigned suf = c0 + c1;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned o = __shfl_down_sync(0xffffffffu, suf, off);
+        if (lane + off < 32) suf += o;
+      }
+      const unsigned above1 = suf - c0 - c1, above0 = above1 + c1;
+      if (above1 < rem && above0 >= rem) s.res[0] = 2 * lane + 1, s.res[1] = above1;
+      else if (above0 < rem && suf >= rem) s.res[0] = 2 * lane, s.res[1] = above0;
+    }
+    __syncthreads();
+    const unsigned S = s.res[0], need = rem - s.res[1];
+    uint2* few = all + (CS == 1 ? SEL_TIES : 0);   // the sub-bin's elements; bit 31 of the position: held by a lower rank
+    uint2 mine[SEL_TIES / SEL_THREADS];
+#pragma unroll
+    for (int j = 0; j < SEL_TIES / SEL_THREADS; j++) {
+      const unsigned t = tid + j * SEL_THREADS;
+      mine[j] = t < n_all ? all[t] : make_uint2(0u, 0u);
+    }
+    if (CS > 1) __syncthreads();   // `few` takes the place of `all`
+#pragma unroll
+    for (int j = 0; j < SEL_TIES / SEL_THREADS; j++) {
+      const unsigned t = tid + j * SEL_THREADS;
+      if (t < n_all) {
+        const unsigned ms = sub_of(mine[j].x);
+        if (ms == S) few[atomicAdd(&s.n_few, 1u)] = make_uint2(mine[j].x, mine[j].y | (t < before_me ? 0x80000000u : 0u));
+        else if (ms > S && t < before_me) atomicAdd(&s.lower_sel, 1u);
+      }
+    }
+    __syncthreads();
+    const unsigned n_few = s.n_few;
+#pragma unroll 1
+    for (unsigned t = tid; t < n_few; t += SEL_THREADS) {
+      const uint2 me = few[t];
+      const unsigned pos = me.y & 0x7fffffffu;
+      unsigned rk = 0;
+      for (unsigned j = 0; j < n_few; j++) {
+        const uint2 o = few[j];
+        rk += (o.x > me.x || (o.x == me.x && (o.y & 0x7fffffffu) < pos)) ? 1u : 0u;
+      }
+      if (rk < need && (me.y >> 31)) atomicAdd(&s.lower_sel, 1u);
+      if (rk + 1 == need) s.thr_key = me.x, s.thr_pos = pos;
+    }
+    __syncthreads();
+    thr_key = s.thr_key, thr_pos = s.thr_pos, lower_sel = s.lower_sel;
+  }
+  if (CS > 1) cluster.barrier_arrive();   // this CTA reads no other CTA's memory from here on
+
+  // ---- ordered emission ----
+  const unsigned room = flat && rem > lower_sel ? rem - lower_sel : 0u;   // flat bin: members this CTA may still take
+  auto words_of = [&](int i, unsigned& aw, unsigned& mw) {
+    if (kept) {
+      aw = above_w[i >> 5], mw = member_w[i >> 5];
+    } else {
+      bool above, member;
+      standing(i + lane, above, member);
+      aw = __ballot_sync(0xffffffffu, above), mw = __ballot_sync(0xffffffffu, member);
+    }
+    if (!flat && mw) {   // resolve the members
+      const unsigned k = ((mw >> lane) & 1u) ? V::key(at(i + lane)) : 0u;
+      const bool t = ((mw >> lane) & 1u) && (k > thr_key || (k == thr_key && ((rank << 27) | (unsigned)(i + lane)) <= thr_pos));
+      aw |= __ballot_sync(0xffffffffu, t);
+    }
+  };
+  unsigned n_take = 0, n_mem = 0;
+#pragma unroll 1
+  for (int i = i0; i < i1; i += 32) {
+    unsigned aw, mw;
+    words_of(i, aw, mw);
+    n_take += __popc(aw);
+    if (flat) n_mem += __popc(mw);
+  }
+  if (lane == 0) s.warp_a[warp] = n_take, s.warp_b[warp] = n_mem;
+  __syncthreads();
+  unsigned g = pre_above + lower_sel, e = 0;
+  for (int w = 0; w < warp; w++) g += s.warp_a[w], e += s.warp_b[w];
+  const unsigned lt = (1u << lane) - 1u;
+#pragma unroll 1
+  for (int i = i0; i < i1; i += 32) {
+    unsigned aw, mw;
+    words_of(i, aw, mw);
+    if (!flat) mw = 0;
+    const unsigned eb = e + __popc(mw & lt);
+    const unsigned pos = g + __popc(aw & lt) + min(eb, room);
+    const bool t = ((aw >> lane) & 1u) || (((mw >> lane) & 1u) && eb < room);
+    if (t && pos < (unsigned)K) out[pos] = out_of(i + lane);
+    g += __popc(aw), e += __popc(mw);
+  }
+}
+
+}  // namespace
+}  // namespace pk

@@ -6,6 +6,7 @@
 // every thread keeps 256 bytes in flight before it starts counting.
 #include <mutex>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 #include "rotate.cuh"
@@ -187,44 +188,6 @@ struct CollParams {
   float inv_g;
 };
 
-// byte k (0..3) of w, zero-extended: one PRMT
-__device__ __forceinline__ unsigned byte_of(uint32_t w, int k) { return __byte_perm(w, 0, 0x4440 | k); }
-
-// Sorts the 256 keys of a warp (8 per lane, element index e = 8 * lane + r) into DESCENDING order of e with a
-// bitonic network: exchanges at distance < 8 stay inside a lane, the others are xor shuffles.  Keys are distinct.
-__device__ __forceinline__ void warp_sort_desc_256(unsigned (&v)[8], int lane) {
-#pragma unroll
-  for (int k = 2; k <= 256; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      if (j >= 8) {
-        const int lj = j >> 3;
-        // block direction: "up" blocks end descending; the lower element of a pair keeps the maximum there
-        const bool up = ((lane << 3) & k) == 0;
-        const bool lower = (lane & lj) == 0;
-        const bool take_max = up == lower;
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-          const unsigned o = __shfl_xor_sync(0xffffffffu, v[r], lj);
-          v[r] = take_max ? max(v[r], o) : min(v[r], o);
-        }
-      } else {
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-          const int l = r ^ j;
-          if (l > r) {
-            const bool up = ((((lane << 3) | r) & k) == 0);
-            const unsigned a = v[r], b = v[l];
-            const unsigned mx = max(a, b), mn = min(a, b);
-            v[r] = up ? mx : mn;
-            v[l] = up ? mn : mx;
-          }
-        }
-      }
-    }
-  }
-}
-
 // The stand-alone op (tier table from global memory, int32 counts out), 256 threads.
 // LAYOUT 0: plane-major ([.., 16, N], key stride 1): a thread owns 16 consecutive keys.
 // LAYOUT 1: key-major ([.., N, 16], subspace stride 1): a warp owns 512 consecutive keys, lane-strided.
@@ -374,41 +337,6 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
 constexpr int CC_THREADS = 512;
 constexpr int CC_PASS = 8192;  // keys a block covers per pass: 16 warps x 512
 
-// x: dims [4*lane, 4*lane+4) of the group-mean query (bf16 values as floats); sg: their SRHT signs.
-// Same pairwise trees and butterflies as rotate16, spread over 32 lanes.  Returns the bf16 norm.
-__device__ __forceinline__ float rotate4(float (&x)[4], const float (&sg)[4], int lane) {
-  float t0 = __fadd_rn(__fmul_rn(x[0], x[0]), __fmul_rn(x[1], x[1]));
-  float t1 = __fadd_rn(__fmul_rn(x[2], x[2]), __fmul_rn(x[3], x[3]));
-  float sum = __fadd_rn(t0, t1);
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, off));
-  const float n = bfround(__fsqrt_rn(sum));
-  const float den = fmaxf(n, bfround(1e-8f));
-#pragma unroll
-  for (int i = 0; i < 4; i++) x[i] = __fmul_rn(bfround(__fdiv_rn(x[i], den)), sg[i]);
-  {  // h = 1, 2 inside the lane
-    float a = x[0], b = x[1], c = x[2], d = x[3];
-    x[0] = __fadd_rn(a, b), x[1] = __fsub_rn(a, b), x[2] = __fadd_rn(c, d), x[3] = __fsub_rn(c, d);
-    a = x[0], b = x[1], c = x[2], d = x[3];
-    x[0] = __fadd_rn(a, c), x[2] = __fsub_rn(a, c), x[1] = __fadd_rn(b, d), x[3] = __fsub_rn(b, d);
-  }
-#pragma unroll
-  for (int bit = 1; bit < 32; bit <<= 1)  // h = 4 .. 64 across lanes
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float pv = __shfl_xor_sync(0xffffffffu, x[i], bit);
-      x[i] = (lane & bit) ? __fsub_rn(pv, x[i]) : __fadd_rn(x[i], pv);
-    }
-#pragma unroll
-  for (int i = 0; i < 4; i++) x[i] = bfround(__fmul_rn(x[i], 0.08838834764831845f));
-  return n;
-}
-
-__device__ __forceinline__ void unpack4(uint2 v, float* out) {
-  out[0] = __uint_as_float(v.x << 16), out[1] = __uint_as_float(v.x & 0xffff0000u);
-  out[2] = __uint_as_float(v.y << 16), out[3] = __uint_as_float(v.y & 0xffff0000u);
-}
-
 template <int LAYOUT>
 __global__ void __launch_bounds__(CC_THREADS, 1) chain_collision_kernel(CollParams p) {
   __shared__ __align__(16) uint8_t s_lut[16 * 256];
@@ -444,28 +372,7 @@ __global__ void __launch_bounds__(CC_THREADS, 1) chain_collision_kernel(CollPara
       for (int i = 0; i < 4; i++) s_q[4 * lane + i] = qx[i];
     }
   };
-  auto rank_clusters = [&]() {   // after a barrier behind prepare_query()
-    // register r of a lane starts with cluster c = 32 * r + lane: the first five terms of the score (bits 0..4 of c)
-    // are the lane's, the last three (bits 5..7) the register's; the sum is taken in the order j = 0..7
-    float qv[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) qv[j] = s_q[warp * 8 + j];
-    float s5 = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 5; j++) s5 = __fadd_rn(s5, ((lane >> j) & 1) ? qv[j] : -qv[j]);
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) {
-      float sc = s5;
-#pragma unroll
-      for (int j = 5; j < 8; j++) sc = __fadd_rn(sc, ((rr >> (j - 5)) & 1) ? qv[j] : -qv[j]);
-      // order of (score descending, id ascending) as one unsigned compare; -0 counts as +0 like a float compare
-      unsigned bits = f2bf(sc);
-      if (bits == 0x8000u) bits = 0u;
-      const unsigned ord = (bits & 0x8000u) ? (~bits & 0xFFFFu) : (bits | 0x8000u);
-      key[rr] = (ord << 8) | (unsigned)(255 - (32 * rr + lane));
-    }
-    warp_sort_desc_256(key, lane);
-  };
+  auto rank_clusters = [&]() { rank_subspace(key, s_q + warp * 8, lane); };   // after a barrier behind prepare_query()
   const bool early = cq.early_query != 0;
   if (early) {
     prepare_query();

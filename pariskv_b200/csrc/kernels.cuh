@@ -94,6 +94,7 @@ struct RerankArgs {
   int H;
   int64_t C;
 };
+bool rerank_fast_layout(const RerankArgs& a);   // key-major, 16-byte aligned records
 int fill_rerank_args(RerankArgs* a, const pk_tensor* key_4bit, const pk_tensor* key_block_weight);
 int launch_rerank(const RerankArgs& a, int64_t bs_h, uint16_t* scores_bf16, float* scores_f32, uint16_t* v4b,
                   cudaStream_t st);
@@ -128,5 +129,11 @@ int64_t select_smem_bytes(int64_t chunk_keys, int64_t C, int64_t K);
 int64_t select_value_bins();     // words per (batch, head) of SelectArgs::val_hist
 int64_t select_final_max_row();  // longest score row whose final top-K the selection kernel finishes entirely in shared memory
 int launch_select_rerank(const RerankArgs& a, int64_t bs_h, const SelectArgs& s, cudaStream_t st);
+
+// retrieve_fused.cu: the whole chain in one launch, one cluster of `cs` CTAs per (batch, head)
+int fused_cluster_size(const pk_tensor* codebook, const RerankArgs& a, int64_t bs_h, int64_t N, int64_t C);
+// cand_out / scores_out: [bs*H][C] or null; ws_cand / ws_scores: the same arrays in the workspace
+int launch_fused_retrieve(int cs, const pk_tensor* codebook, const RerankArgs& a, const ChainQuery& cq, const SelectArgs& sa,
+                          int64_t* cand_out, float* scores_out, int64_t* ws_cand, float* ws_scores, cudaStream_t st);
 
 }  // namespace pk

@@ -6,6 +6,7 @@
 // in shared memory replicated once per lane (bank = lane), the query blocks are read as broadcasts.
 // fp32 order (shared with the CPU oracle): per subspace dot = fma chain over j ascending,
 // acc = fma(dot, w_b, acc) over b ascending, score = acc * ||q||.
+#include "chain.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -13,75 +14,6 @@ namespace pk {
 namespace {
 
 constexpr int RR_THREADS = 128;
-
-struct RerankSmem {
-  float lev[16][32];  // lev[nibble][lane]
-  float q[128];
-};
-
-__device__ __forceinline__ void rerank_setup(RerankSmem& sm, const RerankArgs& a, int64_t bh, int tid, int nthreads) {
-  for (int i = tid; i < 16 * 32; i += nthreads) {
-    const int nib = i >> 5;
-    const float c = bf2f(a.centers[nib & 7]);
-    sm.lev[nib][i & 31] = (nib & 8) ? c : -c;
-  }
-  for (int i = tid; i < 128; i += nthreads) sm.q[i] = bf2f(a.q_blocks[bh * 128 + i]);
-}
-
-// FAST: key-major, 16-byte aligned records.  Returns the fp32 score of key `key`.
-template <bool FAST>
-__device__ __forceinline__ float rerank_one(const RerankSmem& sm, const RerankArgs& a, const uint8_t* k4,
-                                            const uint16_t* w, int64_t key, float qn, int lane, uint16_t* v4b_row,
-                                            int64_t v4b_sub_stride) {
-  uint32_t code[16];
-  uint32_t wt[8];
-  if (FAST) {
-    const uint4* cp = reinterpret_cast<const uint4*>(k4 + key * 64);
-    const uint4* wp = reinterpret_cast<const uint4*>(w + key * 16);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint4 v = __ldg(cp + i);
-      code[4 * i] = v.x, code[4 * i + 1] = v.y, code[4 * i + 2] = v.z, code[4 * i + 3] = v.w;
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const uint4 v = __ldg(wp + i);
-      wt[4 * i] = v.x, wt[4 * i + 1] = v.y, wt[4 * i + 2] = v.z, wt[4 * i + 3] = v.w;
-    }
-  } else {
-#pragma unroll
-    for (int s = 0; s < 16; s++) {
-      const uint8_t* cp = k4 + s * a.k4_s + key * a.k4_l;
-      code[s] = (uint32_t)cp[0] | ((uint32_t)cp[1] << 8) | ((uint32_t)cp[2] << 16) | ((uint32_t)cp[3] << 24);
-    }
-#pragma unroll
-    for (int s = 0; s < 8; s++)
-      wt[s] = (uint32_t)w[(2 * s) * a.w_s + key * a.w_l] | ((uint32_t)w[(2 * s + 1) * a.w_s + key * a.w_l] << 16);
-  }
-  float acc = 0.0f;
-#pragma unroll
-  for (int s = 0; s < 16; s++) {
-    const float4 q0 = *reinterpret_cast<const float4*>(&sm.q[8 * s]);
-    const float4 q1 = *reinterpret_cast<const float4*>(&sm.q[8 * s + 4]);
-    const float qv[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-    float dot = 0.0f;
-    float lv[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      lv[j] = sm.lev[(code[s] >> (4 * j)) & 0xFu][lane];
-      dot = __fmaf_rn(lv[j], qv[j], dot);
-    }
-    if (v4b_row) {
-      uint32_t o[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) o[j] = (uint32_t)f2bf(lv[2 * j]) | ((uint32_t)f2bf(lv[2 * j + 1]) << 16);
-      *reinterpret_cast<uint4*>(v4b_row + s * v4b_sub_stride) = make_uint4(o[0], o[1], o[2], o[3]);
-    }
-    const float wf = __uint_as_float((s & 1) ? (wt[s >> 1] & 0xffff0000u) : (wt[s >> 1] << 16));
-    acc = __fmaf_rn(dot, wf, acc);
-  }
-  return __fmul_rn(acc, qn);
-}
 
 template <bool FAST>
 __global__ void __launch_bounds__(RR_THREADS) rerank_kernel(RerankArgs a, uint16_t* scores_bf16, float* scores_f32,
@@ -110,6 +42,7 @@ __global__ void __launch_bounds__(RR_THREADS) rerank_kernel(RerankArgs a, uint16
 // list comes out in ascending key order with no atomics and no second pass.  The block that finishes last for a
 // (batch, head) then selects the final top-K of that head's fp32 scores (an arrival counter per head; the scores
 // of the other blocks are read back from L2), so the chain needs no further launch.
+
 constexpr int SEL_THREADS = 512;  // the first 256 threads own the 256 count bins
 constexpr int FT_BINS = 4096;     // histogram bins of one radix pass of the final selection
 constexpr int FT_KEYS_MAX = 16384;  // scores kept in shared memory by the final selection (the rest is re-read from L2)
@@ -124,30 +57,6 @@ struct SelParams {
 // ---- final top-K of one (batch, head) by one block ------------------------------------------------------------------
 // Selected set = first K of (score descending, position ascending), emitted as cand[position] in ascending position
 // (positions are ascending key indices).  Two forms: rows that fit the shared-memory cache, and longer ones.
-
-// Block-wide exclusive scan of a packed pair of counters; returns (exclusive prefix, block total).
-template <int NT>
-__device__ __forceinline__ unsigned long long block_scan_excl(unsigned long long mine, unsigned long long* s_scan,
-                                                              unsigned long long* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long sc = mine;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const unsigned long long o = __shfl_up_sync(0xffffffffu, sc, off);
-    if (lane >= off) sc += o;
-  }
-  if (lane == 31) s_scan[warp] = sc;
-  __syncthreads();
-  unsigned long long before = 0, tot = 0;
-#pragma unroll
-  for (int w = 0; w < NT / 32; w++) {
-    const unsigned long long v = s_scan[w];
-    if (w < warp) before += v;
-    tot += v;
-  }
-  *total = tot;
-  return before + sc - mine;
-}
 
 // Threshold bin of hist[0..nb): the highest bin d with (elements in bins >= d) >= rem.  Result in res[0..2] =
 // (d, elements in higher bins, elements in d); every thread returns after the result is visible.
@@ -780,13 +689,13 @@ __global__ void __launch_bounds__(SEL_THREADS, FAST ? 2 : 1) select_rerank_kerne
   }
 }
 
+}  // namespace
+
 bool rerank_fast_layout(const RerankArgs& a) {
   return a.k4_s == 4 && a.k4_l == 64 && a.w_s == 1 && a.w_l == 16 && (reinterpret_cast<uintptr_t>(a.k4) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(a.w) & 15) == 0 && a.k4_b % 16 == 0 && a.k4_h % 16 == 0 && a.w_b % 8 == 0 &&
          a.w_h % 8 == 0;
 }
-
-}  // namespace
 
 int fill_rerank_args(RerankArgs* a, const pk_tensor* key_4bit, const pk_tensor* key_block_weight) {
   PK_CHECK_TENSOR(key_4bit, PK_U8, 5);

@@ -1,4 +1,5 @@
-// The whole retrieval chain of one decode step as one host call and two launches:
+// The whole retrieval chain of one decode step as one host call: one launch where the metadata is key-major and a
+// cluster of CTAs holds a head's zone on chip (retrieve_fused.cu), otherwise two launches:
 // (1) query preparation + cluster ranking + tier table + collision count (u8 counts + per-block histograms),
 // (2) candidate selection + 4-bit rerank + final top-K by the last block of every (batch, head).
 // All scratch comes from the caller.
@@ -176,8 +177,18 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
     cq.queries = (const uint16_t*)queries->data, cq.signs = (const uint16_t*)a.signs->data, cq.Hq = (int)Hq;
     cq.q_blocks = qb, cq.q_norm = qn, cq.query_avg = qa;
     cq.counts = (const int32_t*)counts_t->data;
-    cq.zero_words = counters;
     cq.early_query = a.queries_settled != 0;
+    const int cs = sharded ? 0 : fused_cluster_size(codebook, ra, bh, N, C);
+    if (cs) {
+      ra.q_blocks = nullptr, ra.q_norm = nullptr, ra.centers = (const uint16_t*)a.mag_centers->data, ra.C = row;
+      cq.q_blocks = a.q_blocks ? qb : nullptr, cq.q_norm = a.q_norm ? qn : nullptr;
+      sa.N = N, sa.C = row, sa.C_want = C, sa.K = K, sa.fill_tail = varlen;
+      sa.final_out = K > 0 ? (int64_t*)a.final_indices->data : nullptr;
+      sa.n_sel_out = n_sel, sa.n_cand_out = n_cand;
+      return launch_fused_retrieve(cs, codebook, ra, cq, sa, a.cand ? cd : nullptr, a.scores_f32 ? sc : nullptr,
+                                   (int64_t*)(ws + lay.cand), (float*)(ws + lay.scores), st);
+    }
+    cq.zero_words = counters;
     if (K > 0 && row > select_final_max_row() && (varlen || sharded || n_sel))
       cq.zero_area = (unsigned*)(ws + lay.vhist), cq.zero_area_words = (int)select_value_bins();
     if ((rc = launch_chain_collision(codebook, cq, counts, lay.u8_stride, hist, &mis, &chunk_keys, &n_chunks, st)))

@@ -1,0 +1,488 @@
+// The retrieval chain of one decode step as ONE launch: a thread-block cluster per (batch, KV head) takes the query to
+// the final top-K without leaving the chip.
+//
+// Every CTA of the cluster owns a contiguous slice of the zone's keys.  It prepares the query and the tier tables itself
+// (behind its first code loads), counts the collisions of its keys into shared memory, and from there on only histograms
+// and a few hundred scores cross the cluster (distributed shared memory):
+//   count histogram  -> threshold count, tie quota, this CTA's offset in the candidate list
+//   4-bit rerank of its own candidates, scores in shared memory
+//   final top-K over the cluster (cluster_select.cuh).
+//
+// Why this split: as two launches (count | select + rerank + final top-K by the last block of a head) the final stage ran
+// on one SM per head, 12 us of 48 at 128K keys, and counts and scores went through L2.  Time line of a CTA on B200
+// (8 heads x 131004 keys, 8 CTAs each): query and ranking 7 us, counting 16 K keys 9, threshold and list 2.7, rerank of
+// 1640 candidates 9.4, final selection 9.  Graph-replayed layer step, start -> now: 16 sequences of 16 - 32K keys
+// (one CTA per head, no exchange at all) 155 -> 123 us, 8 heads x 128K keys 70 -> 68, 10K keys 27 -> 20 for the chain.
+// What bounds it: the serial chain of exchanges for small zones, instruction issue (look-ups 85 instructions per key and
+// warp, rerank 420 per candidate and warp) for long ones; codes and records stream at under half of the HBM rate.
+#include "chain.cuh"
+#include "cluster_select.cuh"
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace pk {
+namespace {
+
+constexpr int FR_THREADS = SEL_THREADS;
+constexpr int FR_WARPS = FR_THREADS / 32;
+constexpr int FR_CBINS = 129;               // counts 0 .. 16 subspaces x 8 tiers
+constexpr int FR_LIST_MAX = 8192;           // candidates a CTA keeps in shared memory; more spill to the workspace
+constexpr int FR_SPAN_MAX = 40 * 1024;      // keys of a CTA: beyond it two launches over all SMs are faster
+constexpr int FR_REC = 112;                 // bytes between staged records (96 used): quarter-warp reads do not conflict
+constexpr int FR_STAGE = FR_WARPS * 32 * FR_REC;
+constexpr int FR_HIST_BYTES = FR_CBINS * 32 * 4;   // one replica per lane: a warp's atomics never collide on a bank
+constexpr int FR_WORDS = LEV2_BYTES / 8;    // ballots of the final selection, over the level table
+static_assert(FR_SPAN_MAX / 32 <= FR_WORDS, "one ballot per 32 candidates");
+static_assert(FR_HIST_BYTES >= 16 * 256 * 4 && FR_HIST_BYTES >= SEL_REGION, "the region serves three stages");
+
+struct FusedParams {
+  const uint8_t* codes;   // key-major records of 16 bytes; (b,h) at b*c_b + h*c_h
+  int64_t c_b, c_h;
+  RerankArgs a;
+  ChainQuery q;
+  int H, G;
+  float inv_g;
+  int64_t N;              // keys per head of the view (upper bound when q.n_dev is set)
+  int64_t C, C_want, K;   // row stride of the candidate arrays, candidates wanted (q.n_dev == null), final top-K
+  int fill_tail;
+  int span_cap, list_cap; // shared memory: keys and candidates per CTA
+  int64_t* cand_out;      // [bs*H][C] or null
+  float* scores_out;      // [bs*H][C] or null
+  unsigned c128, c256, c64k;   // 128, 256 and 65536 (see tier_sum16, rerank_pairs)
+  int64_t* ws_cand;       // the same arrays for what does not fit in shared memory (never null)
+  float* ws_scores;
+  int64_t* final_out;     // [bs*H][K]
+  int32_t* n_sel_out;
+  int32_t* n_cand_out;
+};
+
+template <int CS>
+__global__ void __launch_bounds__(FR_THREADS, 1) retrieve_fused_kernel(FusedParams p) {
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ __align__(16) unsigned char dyn[];
+  __shared__ SelShared s;
+  __shared__ unsigned s_tiers[9];
+  __shared__ float s_qnorm;
+  __shared__ __align__(16) float s_q[128];        // rotated query
+  __shared__ __align__(16) float4 s_q2[32];       // the same, the subspaces of a pair side by side (see rerank_pairs)
+  __shared__ __align__(16) uint8_t s_lut[16 * 128];
+  unsigned* region = reinterpret_cast<unsigned*>(dyn);
+  uint32_t* lev2 = reinterpret_cast<uint32_t*>(dyn + FR_HIST_BYTES);
+  uint8_t* cnt8 = dyn + FR_HIST_BYTES + LEV2_BYTES;
+  uint8_t* stage = cnt8 + (threadIdx.x >> 5) * (32 * FR_REC);   // the counts are done with when records are staged
+  int* ids = reinterpret_cast<int*>(cnt8 + max(p.span_cap, FR_STAGE));
+  float* sc = reinterpret_cast<float*>(ids + p.list_cap);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned rank = CS == 1 ? 0u : cluster.block_rank();
+  const int64_t bh = blockIdx.y;
+  const int b = (int)(bh / p.H), h = (int)(bh % p.H);
+  const ChainQuery& cq = p.q;
+  // ---- query: warp 0 averages, normalises and rotates it; then warp w ranks the clusters of subspace w (registers) ----
+  float qavg[4] = {0.0f, 0.0f, 0.0f, 0.0f}, qx[4] = {0.0f, 0.0f, 0.0f, 0.0f}, qn0 = 0.0f;
+  unsigned key[8];
+  auto prepare_query = [&]() {
+    if (warp == 0) {
+      const uint16_t* q = cq.queries + ((int64_t)b * cq.Hq + (int64_t)h * p.G) * 128 + 4 * lane;
+      float sg[4], acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      unpack4(__ldg(reinterpret_cast<const uint2*>(cq.signs + 4 * lane)), sg);
+      for (int g = 0; g < p.G; g++) {  // fp32 sum over the group, g ascending
+        float v[4];
+        unpack4(__ldg(reinterpret_cast<const uint2*>(q + g * 128)), v);
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[i] = __fadd_rn(acc[i], v[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) qx[i] = qavg[i] = bfround(__fmul_rn(acc[i], p.inv_g));
+      qn0 = rotate4(qx, sg, lane);
+#pragma unroll
+      for (int i = 0; i < 4; i++) s_q[4 * lane + i] = qx[i];
+      if (lane == 0) s_qnorm = qn0;
+    }
+  };
+  auto rank_clusters = [&]() { rank_subspace(key, s_q + warp * 8, lane); };
+  const bool early = cq.early_query != 0;
+  if (early) {
+    prepare_query();
+    __syncthreads();
+    rank_clusters();
+  }
+  pdl_wait();
+  pdl_trigger();
+  const int64_t N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
+  const int64_t C_want = cq.n_dev ? min((int64_t)zone_candidates(cq.sched, N), p.C) : p.C_want;
+  const int span = (int)(((N + CS - 1) / CS + 15) / 16 * 16);
+  const int64_t begin = (int64_t)rank * span;
+  const int n_keys = (int)max((int64_t)0, min((int64_t)span, N - begin));
+  const uint8_t* codes = p.codes + b * p.c_b + h * p.c_h + begin * 16;
+
+  // ---- code loads: a warp takes 128 consecutive keys (four per lane) every FR_WARPS * 128; two rounds are in flight,
+  // the first ones during the prologue ----
+  uint4 r0[4], r1[4];
+  constexpr int STEP = FR_WARPS * 128;
+  auto load_codes = [&](uint4 (&r)[4], int v0) {
+    if (n_keys > 0)
+#pragma unroll
+      for (int j = 0; j < 4; j++)   // past the end: the last key again, its count unused
+        r[j] = __ldg(reinterpret_cast<const uint4*>(codes) + min(v0 + 32 * j, n_keys - 1));
+  };
+  load_codes(r0, warp * 128 + lane);
+  load_codes(r1, warp * 128 + lane + STEP);
+  {
+    const int4* cp = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
+    const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1);   // cluster sizes of this warp's subspace
+    unsigned* my = region + warp * 256;
+    if (!early) prepare_query();
+    if (warp == 0 && rank == 0) {
+      if (cq.query_avg)
+        *reinterpret_cast<uint2*>(cq.query_avg + bh * 128 + 4 * lane) =
+            make_uint2((uint32_t)f2bf(qavg[0]) | ((uint32_t)f2bf(qavg[1]) << 16), (uint32_t)f2bf(qavg[2]) | ((uint32_t)f2bf(qavg[3]) << 16));
+      if (cq.q_blocks)
+        *reinterpret_cast<uint2*>(cq.q_blocks + bh * 128 + 4 * lane) =
+            make_uint2((uint32_t)f2bf(qx[0]) | ((uint32_t)f2bf(qx[1]) << 16), (uint32_t)f2bf(qx[2]) | ((uint32_t)f2bf(qx[3]) << 16));
+      if (cq.q_norm && lane == 0) cq.q_norm[bh] = f2bf(qn0);
+    }
+    if (tid == 32) {
+      if (cq.n_dev) {
+        unsigned t[8];
+        zone_tiers(cq.sched, (long long)N, t);
+        for (int i = 0; i < cq.sched.n_tiers; i++) s_tiers[i] = t[i];
+        s_tiers[8] = (unsigned)cq.sched.n_tiers;
+      } else {
+        for (int i = 0; i < cq.n_tiers; i++) s_tiers[i] = cq.tiers[i];
+        s_tiers[8] = (unsigned)cq.n_tiers;
+      }
+    }
+    *reinterpret_cast<int4*>(my + lane * 8) = c0;
+    *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
+    build_lev2(lev2, p.a.centers, tid, FR_THREADS);
+    __syncthreads();
+    if (!early) rank_clusters();
+    const int n_tiers = (int)s_tiers[8];
+    unsigned tier[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) tier[t] = t < n_tiers ? s_tiers[t] : 0u;
+    unsigned cnt[8], run = 0;
+#pragma unroll
+    for (int rr = 0; rr < 8; rr++) {
+      cnt[rr] = my[255u - (key[rr] & 255u)];
+      run += cnt[rr];
+    }
+    unsigned incl = run;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += o;
+    }
+    unsigned excl = incl - run;
+    __syncwarp();   // the sizes have been read: the same words take the tier counts, packed to nibbles below
+#pragma unroll
+    for (int rr = 0; rr < 8; rr++) {
+      unsigned wgt = 0;
+#pragma unroll
+      for (int t = 0; t < 8; t++) wgt += (excl < tier[t]) ? 1u : 0u;   // absent tiers are 0: never above a prefix sum
+      my[255u - (key[rr] & 255u)] = wgt;
+      excl += cnt[rr];
+    }
+    __syncwarp();
+    {  // entries i (low nibble) and i + 128 of byte i: four bytes per lane
+      const uint4 e0 = *reinterpret_cast<const uint4*>(my + lane * 4), e1 = *reinterpret_cast<const uint4*>(my + 128 + lane * 4);
+      const uint32_t w = (e0.x | (e1.x << 4)) | ((e0.y | (e1.y << 4)) << 8) | ((e0.z | (e1.z << 4)) << 16) | ((e0.w | (e1.w << 4)) << 24);
+      *reinterpret_cast<uint32_t*>(s_lut + warp * 128 + lane * 4) = w;
+    }
+    if (tid < 128) reinterpret_cast<float*>(s_q2)[pair_slot(tid)] = s_q[tid];
+    __syncthreads();   // the tables are complete and the staging area is free again
+    for (int i = tid; i < FR_CBINS * 32; i += FR_THREADS) region[i] = 0;
+    __syncthreads();
+  }
+  const float qn = s_qnorm;
+
+  // ---- collision counts of this CTA's keys ----
+  auto count_round = [&](uint4 (&r)[4], int v0) {   // counts four keys and puts the loads of the round after next in their place
+    unsigned c[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) c[j] = tier_sum16(r[j], s_lut, p.c256);
+    load_codes(r, v0 + 2 * STEP);
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (v0 + 32 * j < n_keys) {
+        cnt8[v0 + 32 * j] = (uint8_t)(c[j] >> 4);
+        atomicAdd(&region[c[j] * 2 + lane], 1u);   // c is a multiple of 16: word 32 per bin
+      }
+  };
+#pragma unroll 1
+  for (int v0 = warp * 128 + lane; v0 - lane < n_keys; v0 += 2 * STEP) {
+    count_round(r0, v0);
+    if (v0 - lane + STEP < n_keys) count_round(r1, v0 + STEP);
+  }
+  __syncthreads();
+  for (int bin = warp; bin < FR_CBINS; bin += FR_WARPS) {
+    const unsigned t = __reduce_add_sync(0xffffffffu, region[bin * 32 + lane]);
+    if (lane == 0) s.hist[0][bin] = t;
+  }
+  sync_cluster<CS>(cluster);
+  cluster_threshold<CS, FR_CBINS>(cluster, s, s.hist[0], rank, (unsigned)C_want);
+  const unsigned T = s.res[0], quota = (unsigned)C_want - s.res[1];
+  const unsigned gt_base = s.res[3], eq_base = s.res[4];
+  const int64_t C_here = min(C_want, p.C);
+
+  // ---- ordered candidate list of this CTA: counts above T, and ties at T while the quota lasts ----
+  const int64_t row_base = bh * p.C;
+  const int64_t out_pos = (int64_t)gt_base + min(eq_base, quota);
+  int n_list;
+  {
+    const int wspan = ((n_keys + FR_WARPS - 1) / FR_WARPS + 15) / 16 * 16;
+    const int k0 = min(n_keys, warp * wspan), k1 = min(n_keys, k0 + wspan);
+    const uint32_t add_gt = (127u - T) * 0x01010101u;           // T <= 128, counts <= 128: no carry between bytes
+    const uint32_t add_ge = T ? (128u - T) * 0x01010101u : 0u;
+    unsigned n_gt = 0, n_eq = 0;
+#pragma unroll 1
+    for (int k = k0 + 16 * lane; k < k1; k += 512) {   // 16 keys -> masks of counts above / at the threshold, kept in their place
+      unsigned gt = 0, eq = 0;
+      const uint4 v = *reinterpret_cast<const uint4*>(cnt8 + k);
+      const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const uint32_t g = T < 128u ? (w4[i] + add_gt) & 0x80808080u : 0u;
+        const uint32_t ge = T ? (w4[i] + add_ge) & 0x80808080u : 0x80808080u;
+        gt |= ((((g >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * i);
+        eq |= (((((ge & ~g) >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * i);
+      }
+      if (k1 - k < 16) gt &= (1u << (k1 - k)) - 1u, eq &= (1u << (k1 - k)) - 1u;
+      *reinterpret_cast<unsigned*>(cnt8 + k) = gt | (eq << 16);
+      n_gt += __popc(gt), n_eq += __popc(eq);
+    }
+    n_gt = __reduce_add_sync(0xffffffffu, n_gt), n_eq = __reduce_add_sync(0xffffffffu, n_eq);
+    if (lane == 0) s.warp_a[warp] = n_gt, s.warp_b[warp] = n_eq;
+    __syncthreads();
+    unsigned g = 0, e = eq_base, g_all = 0, e_all = eq_base;
+#pragma unroll
+    for (int w = 0; w < FR_WARPS; w++) {
+      const unsigned a = s.warp_a[w], c = s.warp_b[w];
+      if (w < warp) g += a, e += c;
+      g_all += a, e_all += c;
+    }
+    const unsigned eq_before = min(eq_base, quota);
+    n_list = (int)(g_all + min(e_all, quota) - eq_before);
+    n_list = (int)max((int64_t)0, min((int64_t)n_list, C_here - out_pos));   // a no-op with consistent histograms
+#pragma unroll 1
+    for (int k = k0; k < k1; k += 512) {
+      const unsigned m = k + 16 * lane < k1 ? *reinterpret_cast<const unsigned*>(cnt8 + k + 16 * lane) : 0u;
+      const unsigned gt = m & 0xffffu, eq = m >> 16;
+      const unsigned mine = ((unsigned)__popc(gt) << 16) | (unsigned)__popc(eq);
+      unsigned inc = mine;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned o = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += o;
+      }
+      const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
+      const unsigned eg = g + ((inc - mine) >> 16), ee = e + ((inc - mine) & 0xffffu);
+      const int room = (int)quota - (int)ee;   // ties this lane may still take
+      unsigned take = eq;
+      if (room < (int)__popc(eq))
+        for (int drop = (int)__popc(eq) - max(room, 0); drop > 0; drop--) take &= ~(1u << (31 - __clz(take)));
+      take |= gt;
+      int pos = (int)(eg + min(ee, quota) - eq_before);
+      const int kb = (int)begin + k + 16 * lane;
+      while (take) {
+        const int j = __ffs(take) - 1;
+        take &= take - 1;
+        if (pos < n_list) {
+          if (pos < p.list_cap) ids[pos] = kb + j;
+          else p.ws_cand[row_base + out_pos + pos] = kb + j;
+        }
+        pos++;
+      }
+      g += total >> 16, e += total & 0xffffu;
+    }
+  }
+  __syncthreads();
+
+  // ---- rerank ----
+  auto id_at = [&](int i) -> int { return i < p.list_cap ? ids[i] : (int)p.ws_cand[row_base + out_pos + i]; };
+  auto score_at = [&](int i) -> float { return i < p.list_cap ? sc[i] : p.ws_scores[row_base + out_pos + i]; };
+  unsigned kmin = 0xffffffffu, kmax = 0u;
+  {
+    const uint8_t* k4 = p.a.k4 + b * p.a.k4_b + h * p.a.k4_h;
+    const uint16_t* w = p.a.w + b * p.a.w_b + h * p.a.w_h;
+    // A warp takes 32 consecutive candidates per round: it loads their records with whole sectors per request (four lanes
+    // on the 64 bytes of codes, two on the 32 bytes of weights), turns them over its staging buffer to one record per lane,
+    // and has the loads of the next round in flight during the arithmetic.  One record per lane straight from memory
+    // touches 32 lines per request and is bound by the L1's tag look-ups, 6 per candidate.
+    constexpr int ROUND = FR_WARPS * 32;
+    uint4 in[6];
+    auto fetch = [&](int base) {   // out of range: the list's last candidate again
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        in[i] = __ldg(reinterpret_cast<const uint4*>(k4 + (int64_t)id_at(min(base + 8 * i + (lane >> 2), n_list - 1)) * 64) + (lane & 3));
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+        in[4 + i] = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)id_at(min(base + 16 * i + (lane >> 1), n_list - 1)) * 16) + (lane & 1));
+    };
+    if (warp * 32 < n_list) fetch(warp * 32);
+#pragma unroll 1
+    for (int base = warp * 32; base < n_list; base += ROUND) {
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; i++) *reinterpret_cast<uint4*>(stage + (8 * i + (lane >> 2)) * FR_REC + (lane & 3) * 16) = in[i];
+#pragma unroll
+      for (int i = 0; i < 2; i++) *reinterpret_cast<uint4*>(stage + (16 * i + (lane >> 1)) * FR_REC + 64 + (lane & 1) * 16) = in[4 + i];
+      __syncwarp();
+      if (base + ROUND < n_list) fetch(base + ROUND);
+      uint4 rec[6];
+#pragma unroll
+      for (int i = 0; i < 6; i++) rec[i] = *reinterpret_cast<const uint4*>(stage + lane * FR_REC + i * 16);
+      const float v = rerank_pairs(rec, lev2, s_q2, qn, lane, p.c128, p.c64k);
+      const int i = base + lane;
+      if (i < n_list) {
+        const int64_t at = row_base + out_pos + i;
+        if (i < p.list_cap) sc[i] = v;
+        else p.ws_scores[at] = v;
+        if (p.scores_out) p.scores_out[at] = v;
+        if (p.cand_out) p.cand_out[at] = id_at(i);
+        const unsigned u = ord_key(v);
+        kmin = min(kmin, u), kmax = max(kmax, u);
+      }
+    }
+    if (p.fill_tail && p.scores_out && p.cand_out)
+      for (int64_t i = C_here + (int64_t)rank * FR_THREADS + tid; i < p.C; i += CS * FR_THREADS) {
+        p.scores_out[row_base + i] = -INFINITY;
+        p.cand_out[row_base + i] = 0;
+      }
+  }
+  const int K_here = (int)min(p.K, C_here);
+  if (rank == 0 && tid == 0) {
+    if (p.n_cand_out) p.n_cand_out[bh] = (int32_t)C_here;
+    if (p.n_sel_out && p.K > 0) p.n_sel_out[bh] = K_here;
+  }
+  if (p.K <= 0) {
+    sync_cluster<CS>(cluster);   // shared memory must outlive the remote reads of the count histograms
+    return;
+  }
+
+  // ---- final top-K over the cluster ----
+  __syncthreads();   // the scores are complete; the level table and the histogram region are free
+  cluster_select<CS, F32Row>(
+      cluster, s, region, lev2, FR_WORDS, rank, n_list, K_here, p.final_out + bh * p.K,
+      [&](int i) -> uint32_t { return __float_as_uint(score_at(i)); }, [&](int i) -> int64_t { return id_at(i); }, kmin, kmax);
+  if (CS > 1) cluster.barrier_wait();   // shared memory must outlive the other CTAs' reads
+}
+
+// Largest clusters that fit the device at once, per cluster size 1, 2, 4, 8, 16 (0: the size cannot be launched).
+struct Capacity {
+  int active[5];
+};
+
+template <int CS>
+int active_clusters() {
+  auto kern = retrieve_fused_kernel<CS>;
+  const int smem = FR_HIST_BYTES + LEV2_BYTES + (FR_SPAN_MAX > FR_STAGE ? FR_SPAN_MAX : FR_STAGE) + 8 * FR_LIST_MAX;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return cudaGetLastError(), 0;
+  if (CS > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return cudaGetLastError(), 0;
+  if (CS == 1) return sm_count();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(CS, 64), cfg.blockDim = dim3(FR_THREADS), cfg.dynamicSmemBytes = (size_t)smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr, cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) return cudaGetLastError(), 0;
+  return n;
+}
+
+// Asked once per device: the answers and the shared-memory opt-ins belong to it.
+const Capacity* capacity() {
+  static Capacity cap[64];
+  static PerDevice asked;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  if (const unsigned long long bit = first_on_device(asked)) {
+    const Capacity c = {{active_clusters<1>(), active_clusters<2>(), active_clusters<4>(), active_clusters<8>(), active_clusters<16>()}};
+    cap[dev] = c;   // several threads may ask at the same time: they write the same numbers
+    mark_on_device(asked, bit);
+  }
+  return &cap[dev];
+}
+
+int span_of(int64_t N, int cs) { return (int)(((N + cs - 1) / cs + 15) / 16 * 16); }
+
+template <int CS>
+cudaError_t launch_cs(dim3 grid, size_t smem, cudaStream_t st, const FusedParams& p) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid, cfg.blockDim = dim3(FR_THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (CS > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = CS, attr[n].val.clusterDim.y = 1, attr[n].val.clusterDim.z = 1;
+    n++;
+  }
+  if (pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    n++;
+  }
+  cfg.attrs = attr, cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, retrieve_fused_kernel<CS>, p);
+}
+
+}  // namespace
+
+// CTAs per (batch, head), or 0 where the fused kernel does not apply: the codebook must be key-major, and a CTA's slice
+// of the zone at most FR_SPAN_MAX keys.
+// The size minimises waves x (fixed + share of the work): measured on B200, about 15 us of a CTA's time do not shrink with
+// its slice (query, ranking, exchanges), a key costs 0.5 ns and a candidate 3 - 6 ns of one SM (look-ups, rerank).
+int fused_cluster_size(const pk_tensor* codebook, const RerankArgs& a, int64_t bs_h, int64_t N, int64_t C) {
+  int layout = 0;
+  chain_layout(codebook, &layout);
+  if (layout != 1 || !rerank_fast_layout(a) || N >= (1ll << 30) || bs_h > 65535) return 0;
+  const Capacity* cap = capacity();
+  if (!cap) return 0;
+  int best = 0;
+  double best_us = 0.0;
+  for (int i = 0; i < 5; i++) {
+    const int cs = 1 << i;
+    if (cap->active[i] <= 0 || span_of(N, cs) > FR_SPAN_MAX) continue;
+    const double waves = (double)((bs_h + cap->active[i] - 1) / cap->active[i]);
+    const double us = waves * (15.0 + (0.0005 * (double)N + 0.0045 * (double)C) / cs);
+    if (!best || us < 0.98 * best_us) best = cs, best_us = us;
+  }
+  return best;
+}
+
+int launch_fused_retrieve(int cs, const pk_tensor* codebook, const RerankArgs& a, const ChainQuery& cq, const SelectArgs& sa,
+                          int64_t* cand_out, float* scores_out, int64_t* ws_cand, float* ws_scores, cudaStream_t st) {
+  const int64_t bs = codebook->shape[0], H = codebook->shape[1];
+  FusedParams p = {};
+  p.codes = (const uint8_t*)codebook->data, p.c_b = codebook->stride[0], p.c_h = codebook->stride[1];
+  p.a = a, p.q = cq, p.H = (int)H, p.G = cq.Hq / (int)H, p.inv_g = 1.0f / (float)p.G;
+  p.N = sa.N, p.C = sa.C, p.C_want = sa.C_want, p.K = sa.K, p.fill_tail = sa.fill_tail;
+  p.c128 = 128, p.c256 = 256, p.c64k = 65536;
+  p.cand_out = cand_out, p.scores_out = scores_out, p.ws_cand = ws_cand, p.ws_scores = ws_scores;
+  p.final_out = sa.final_out, p.n_sel_out = sa.n_sel_out, p.n_cand_out = sa.n_cand_out;
+  p.span_cap = span_of(sa.N, cs);
+  // twice an even share of the candidates: slices differ, and what does not fit goes through the workspace
+  int64_t list = (2 * sa.C / cs + 512 + 31) / 32 * 32;
+  if (list > p.span_cap + 32) list = (p.span_cap + 63) / 32 * 32;
+  p.list_cap = (int)(list < FR_LIST_MAX ? list : FR_LIST_MAX);
+  const size_t smem = (size_t)FR_HIST_BYTES + LEV2_BYTES + (p.span_cap > FR_STAGE ? p.span_cap : FR_STAGE) + 8 * (size_t)p.list_cap;
+  const dim3 grid((unsigned)cs, (unsigned)(bs * H));
+  StageTimer tm(ST_RETRIEVE, st);
+  cudaError_t e = cudaErrorInvalidValue;
+  switch (cs) {
+    case 1: e = launch_cs<1>(grid, smem, st, p); break;
+    case 2: e = launch_cs<2>(grid, smem, st, p); break;
+    case 4: e = launch_cs<4>(grid, smem, st, p); break;
+    case 8: e = launch_cs<8>(grid, smem, st, p); break;
+    case 16: e = launch_cs<16>(grid, smem, st, p); break;
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(PK_ERR_CUDA, "retrieve: %s", cudaGetErrorString(e));
+  }
+  return check_launch("retrieve");
+}
+
+}  // namespace pk
