@@ -92,6 +92,29 @@ int pk_encode_keys(const pk_tensor* keys, const pk_tensor* signs, const pk_tenso
                    const pk_tensor* block_weight, const pk_tensor* packed_4bit,
                    const pk_tensor* cluster_counts, void* stream);
 
+/* The whole prompt of one sample of a layer into the cache, one launch: key coding (as pk_encode_keys), cluster histogram,
+ * K/V rows to the window and to the store, value norms and the layer's position words.  Replaces the body of
+ * polar_cache.prefill_update_kv_cache (cache_hub/polar_cache.py:379-639) for one sample.
+ *   k / v          bf16 [P,H,128], last stride 1, rows 16-byte aligned
+ *   window_k/_v    bf16 [bs,H,cap_w,128]; win_codes / win_weight / win_4bit / win_vnorm: staging records, and codebook /
+ *   block_weight / packed_4bit / value_norm (or NULL): zone records of the layer, all as in pk_append_encode
+ *   cluster_counts i32 [bs,H,16,256] contiguous; row b is overwritten
+ *   rows           bf16 [H,n >= N,2,128], last two dims contiguous, device memory: where zone rows go (row b of the store,
+ *                  or a buffer that the caller copies to a host store: pk_copy_rows)
+ *   state          i32 [4 + bs]: state[0] = window rows, state[1..3] = 0, state[4 + b] = zone rows
+ * With N = max(0, P - sink - local): tokens [sink, sink + N) become zone rows 0 .. N - 1, the first `sink` and the last
+ * `local` tokens window rows (every token where N == 0; P must then fit the window). */
+int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const pk_tensor* signs, const pk_tensor* window_k,
+                      const pk_tensor* window_v, const pk_tensor* win_codes, const pk_tensor* win_weight,
+                      const pk_tensor* win_4bit, const pk_tensor* win_vnorm, const pk_tensor* codebook,
+                      const pk_tensor* block_weight, const pk_tensor* packed_4bit, const pk_tensor* value_norm,
+                      const pk_tensor* cluster_counts, const pk_tensor* rows, const pk_tensor* state, int64_t b,
+                      int64_t sink, int64_t local, void* stream);
+
+/* One 2-D copy: src [H,n,...] -> dst [H,n,...] of the same type and shape, everything behind the first dimension
+ * contiguous in both (a head's rows are one block, the blocks lie apart); device or pinned host memory on either side. */
+int pk_copy_rows(const pk_tensor* src, const pk_tensor* dst, void* stream);
+
 /* Histogram of codes per (batch, head, subspace): polar_cache._count_cluster_keys
  * (cache_hub/polar_cache.py:980-996).  counts i32 [bs,H,16,256] contiguous; accumulate != 0 adds
  * to the existing contents (as :774-775), 0 overwrites (as :600-601). */

@@ -59,6 +59,8 @@ SIGNATURES = {
     "pk_timing_read_graph": (_INT, [ctypes.POINTER(ctypes.c_double), _I64P, _INT]),
     "pk_timing_clear_graph": (_INT, []),
     "pk_encode_keys": (_INT, [TP, TP, TP, TP, TP, TP, _VP]),
+    "pk_prefill_sample": (_INT, [TP] * 16 + [_I64, _I64, _I64, _VP]),
+    "pk_copy_rows": (_INT, [TP, TP, _VP]),
     "pk_count_clusters": (_INT, [TP, TP, _INT, _VP]),
     "pk_query_prep": (_INT, [TP, TP, TP, TP, TP, _VP]),
     "pk_rank_clusters": (_INT, [TP, TP, _VP]),

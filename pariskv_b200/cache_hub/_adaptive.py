@@ -43,14 +43,6 @@ class AdaptiveKCache(_base_cache):
     def _zone_vnorm(self, layer):
         return self.value_norm_gpu[layer]
 
-    # ---- value norms of the prompt (decode rows are handled by the append kernel) -------------------------
-    def _prefill_sample(self, k, v, layer, b, vs):
-        super()._prefill_sample(k, v, layer, b, vs)
-        N = self.zone_len[layer][b]
-        if N > 0:
-            vn = torch.linalg.vector_norm(v[vs:].to(self.dtype).float(), dim=-1).transpose(0, 1)  # [H, P]
-            self.value_norm_gpu[layer][b, :, :N] = vn[:, self.sink_size:self.sink_size + N]
-
     # ---- decode attention ---------------------------------------------------------------------------------
     def compute(self, queries, layer_idx):
         queries = queries.contiguous()

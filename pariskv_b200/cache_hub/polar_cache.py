@@ -139,7 +139,8 @@ class polar_cache(KV_Cache):
         # first consumer of that layer's store (cache_hub/polar_cache.py:202-210, :617-639)
         self._copy_stream = torch.cuda.Stream(device=dev) if enable_offload else None
         self._offload_event = [None] * layer_num
-        self.BULK_OFFLOAD_ROWS = 4096
+        self.BULK_OFFLOAD_ROWS = 1024
+        self._staging, self._staging_turn = [[None, None], [None, None]], 0   # (buffer, event of the last copy out of it)
         self.codebook_gpu, self.key_block_weight_gpu, self.key_4bit_packed_gpu = [], [], []
         for _ in range(layer_num):
             cb, w, pk = ops.alloc_key_metadata(bs, H, self.zone_capacity, dev)
@@ -227,9 +228,7 @@ class polar_cache(KV_Cache):
                                  f"must all be at least sink + local = {self.steady_size} tokens long, or equally long")
             longest = max(seq_len - self._valid_start(b) for b in range(self.batch_size))
             self.current_seq_len[layer_idx] = longest
-            self.cpu_valid_end[layer_idx] = max(self.zone_len[layer_idx])
-            st = [self._window_len[layer_idx], 0, 0, 0] + list(self.zone_len[layer_idx])
-            self._layer_state[layer_idx].copy_(torch.tensor(st, dtype=torch.int32), non_blocking=False)
+            self.cpu_valid_end[layer_idx] = max(self.zone_len[layer_idx])   # (the kernels have set the device words)
             if layer_idx == self.layer_num - 1:
                 self.context += longest
         return key_states[:, vs:], value_states[:, vs:]
@@ -242,69 +241,69 @@ class polar_cache(KV_Cache):
 
     def _prefill_sample(self, k, v, layer, b, vs):
         """k, v: [seq_len, H, 128] of one sample; tokens before `vs` are padding."""
-        k = k[vs:].to(self.dtype)
-        v = v[vs:].to(self.dtype)
+        k, v = k[vs:].to(self.dtype), v[vs:].to(self.dtype)
+        if k.stride(2) != 1 or v.stride(2) != 1 or (k.data_ptr() | v.data_ptr()) & 15 or any(x & 7 for x in k.stride()[:2] + v.stride()[:2]):
+            k, v = k.contiguous(), v.contiguous()      # the kernel reads rows of 16-byte words
         P = k.shape[0]
-        sink, local = self.sink_size, self.local_size
-        wk, wv = self.unified_keys_gpu[layer], self.unified_values_gpu[layer]
         N = max(0, P - self.steady_size)
-        if N == 0:  # short prompt: everything stays in the window
-            n = min(P, self.window_capacity)
-            wk[b, :, :n] = k[:n].transpose(0, 1)
-            wv[b, :, :n] = v[:n].transpose(0, 1)
+        n = self.steady_size if N else min(P, self.window_capacity)
+        staged = N > 0 and self.enable_offload         # rows for the host store: gathered on the device, one copy for all heads
+        rows, slot = self._staging_rows(N) if staged else (self._store_kv[layer][b], None)
+        if P > 0:
+            _lib.native().prefill_sample(
+                k, v, self.srht_diagonal_signs, self.unified_keys_gpu[layer], self.unified_values_gpu[layer],
+                self._win_codes[layer], self._win_weight[layer], self._win_4bit[layer], self._win_vnorm[layer],
+                self.codebook_gpu[layer], self.key_block_weight_gpu[layer], self.key_4bit_packed_gpu[layer],
+                self._zone_vnorm(layer), self.cluster_key_counts_gpu[layer], rows if N else None, self._layer_state[layer], b,
+                self.sink_size, self.local_size)
         else:
-            n = self.steady_size
-            wk[b, :, :sink] = k[:sink].transpose(0, 1)
-            wv[b, :, :sink] = v[:sink].transpose(0, 1)
-            wk[b, :, sink:sink + local] = k[P - local:].transpose(0, 1)
-            wv[b, :, sink:sink + local] = v[P - local:].transpose(0, 1)
-            zk = k[sink:sink + N].transpose(0, 1)   # [H, N, 128] strided view, rows 16-byte aligned
-            zv = v[sink:sink + N].transpose(0, 1)
-            self._append_zone(layer, b, zk, zv, 0, N, reset_counts=True)
-        if N == 0:
             self.cluster_key_counts_gpu[layer][b].zero_()
-        self._stage_window_rows(layer, b, n)
+            self._layer_state[layer][:4].zero_()
+            self._layer_state[layer][4 + b] = 0
+        if staged:
+            self._offload_rows(layer, b, rows, N, slot)
         self._window_len[layer] = n
         self._sample_window[layer][b] = n
         self.zone_len[layer][b] = N
 
-    def _stage_window_rows(self, layer, b, n):
-        """Code the first n window rows of sample b into the staging arrays (the rows behind the sink will be flushed
-        later; their records must be ready) and record their value norms."""
-        if n <= 0:
-            return
-        wk, wv = self.unified_keys_gpu[layer], self.unified_values_gpu[layer]
-        view = lambda t: t[b:b + 1, :, :n].permute(0, 1, 3, 2)              # key-major storage, reference-shaped view
-        ops.encode_keys(wk[b:b + 1, :, :n], self.srht_diagonal_signs, view(self._win_codes[layer]),
-                        view(self._win_weight[layer]), self._win_4bit[layer][b:b + 1, :, :n].permute(0, 1, 3, 2, 4))
-        self._win_vnorm[layer][b, :, :n] = torch.linalg.vector_norm(wv[b, :, :n].float(), dim=-1)
+    STAGING_KEEP_BYTES = 64 << 20   # a staging buffer up to this size is kept for the next prompts
 
-    def _append_zone(self, layer, b, zk, zv, start, n, reset_counts=False):
-        """Code n keys ([H, n, 128]) of sample b into zone records [start, start+n) and copy K/V to the store."""
-        sl = slice(start, start + n)
-        counts = self.cluster_key_counts_gpu[layer][b:b + 1]
-        if reset_counts:
-            counts.zero_()
-        ops.encode_keys(zk.unsqueeze(0), self.srht_diagonal_signs,
-                        self.codebook_gpu[layer][b:b + 1, :, :, sl], self.key_block_weight_gpu[layer][b:b + 1, :, :, sl],
-                        self.key_4bit_packed_gpu[layer][b:b + 1, :, :, sl, :], cluster_counts=counts)
-        skv = self._store_kv[layer]
-        kv = torch.stack((zk, zv), dim=2)  # [H, n, 2, 128] on the device: K and V rows interleaved as the store holds them
-        if self._copy_stream is not None and n >= self.BULK_OFFLOAD_ROWS:
-            cur = torch.cuda.current_stream(kv.device)
-            self._wait_offload(layer)                 # an earlier bulk copy of this layer must stay ordered
-            self._copy_stream.wait_stream(cur)
-            with torch.cuda.stream(self._copy_stream):
-                for h in range(self.kv_head):
-                    skv[b, h, sl].copy_(kv[h], non_blocking=True)
-                ev = torch.cuda.Event()
-                ev.record(self._copy_stream)
-            kv.record_stream(self._copy_stream)       # keep the staging tensor alive until the copies have run
-            self._offload_event[layer] = ev
+    def _staging_rows(self, n):
+        """A device buffer [H,n,2,128] for rows on their way to the host store -> (buffer, slot of the kept pair or None).
+        Two kept buffers take turns, each reused when its last copy has left it; giving every prompt a fresh tensor makes
+        the allocator hold all of those whose copies are pending.  Larger buffers are allocated per prompt."""
+        numel = self.kv_head * n * 256
+        if numel * 2 > self.STAGING_KEEP_BYTES:
+            return torch.empty(self.kv_head, n, 2, 128, dtype=self.dtype, device=self.device), None
+        self._staging_turn ^= 1
+        slot = self._staging[self._staging_turn]
+        if slot[0] is None or slot[0].numel() < numel:
+            if slot[0] is not None:
+                slot[0].record_stream(self._copy_stream)
+            slot[0], slot[1] = torch.empty(numel, dtype=self.dtype, device=self.device), None
+        if slot[1] is not None:
+            torch.cuda.current_stream(self.device).wait_event(slot[1])
+        return slot[0][:numel].view(self.kv_head, n, 2, 128), slot
+
+    def _offload_rows(self, layer, b, rows, n, slot):
+        """Zone rows [0, n) of sample b to its host store: one copy, on the copy stream for all but short prompts."""
+        dst = self._store_kv[layer][b, :, :n]
+        if n < self.BULK_OFFLOAD_ROWS:
+            self._wait_offload(layer)                  # an earlier bulk copy of this layer must stay ordered
+            _lib.native().copy_rows(rows, dst)
+            if slot is not None:
+                slot[1] = None                         # the copy is ordered before later work of this stream
             return
-        self._wait_offload(layer)
-        for h in range(self.kv_head):  # contiguous per-head blocks: one async copy each, on the current stream
-            skv[b, h, sl].copy_(kv[h], non_blocking=True)
+        self._copy_stream.wait_stream(torch.cuda.current_stream(rows.device))
+        with torch.cuda.stream(self._copy_stream):
+            _lib.native().copy_rows(rows, dst)
+            ev = torch.cuda.Event()
+            ev.record(self._copy_stream)
+        self._offload_event[layer] = ev
+        if slot is not None:
+            slot[1] = ev
+        else:
+            rows.record_stream(self._copy_stream)      # keep the buffer alive until the copy has run
 
     def _wait_offload(self, layer):
         """Order the current stream after the layer's pending bulk offload, if any (no host block)."""

@@ -1,59 +1,13 @@
-// Key coding (SRHT normalise-rotate, sign code, 4-bit code, rerank weight), cluster histograms and
-// query preparation.  One key is handled by 8 lanes, 16 dimensions (two 8-dim subspaces) per lane:
-// the norm, the first four Hadamard stages and everything per subspace stay inside a lane; the last
-// three Hadamard stages and the norm tree cross lanes with xor shuffles.  Every fp32 operation is an
-// explicit round-to-nearest intrinsic in a fixed order, so results do not depend on the mapping.
+// Key coding (SRHT normalise-rotate, sign code, 4-bit code, rerank weight; keycode.cuh), prompt ingestion, cluster
+// histograms, query preparation and the append of a decode token.  One key is coded by 4 lanes, 32 dimensions (four
+// 8-dim subspaces) per lane.  Every fp32 operation rounds to nearest in a fixed order, so results do not depend on the
+// mapping.
 #include "common.cuh"
+#include "keycode.cuh"
 #include "rotate.cuh"
 
 namespace pk {
 namespace {
-
-__constant__ float c_thr[7] = {0.08447265625f, 0.169921875f, 0.2578125f, 0.349609375f,
-                               0.44921875f,    0.55859375f,  0.69140625f};
-__constant__ float c_cen[8] = {0.0419921875f, 0.126953125f, 0.212890625f, 0.302734375f,
-                               0.396484375f,  0.5f,         0.6171875f,   0.76171875f};
-
-// One 8-dim subspace of a rotated key: y = its 8 coordinates (bf16 values as floats), n = the key's bf16 norm.
-// -> 8-bit sign code, rerank weight, four bytes of (sign << 3 | level) nibbles.  The arithmetic of
-// polar_cache.batch_encode (cache_hub/polar_cache.py:950-976), every fp32 operation an explicit intrinsic.
-__device__ __forceinline__ void code_subspace(const float* y, float n, unsigned* code_out, uint16_t* wt_out,
-                                              uint32_t* packed_out) {
-  float t[8];
-  unsigned code = 0;
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    t[j] = __fmul_rn(y[j], y[j]);
-    if (y[j] >= 0.0f) code |= 1u << j;
-  }
-#pragma unroll
-  for (int w = 8; w > 1; w >>= 1)
-#pragma unroll
-    for (int i = 0; i < w / 2; i++) t[i] = __fadd_rn(t[2 * i], t[2 * i + 1]);
-  const float r = bfround(__fsqrt_rn(t[0]));
-  const float den = fmaxf(r, bfround(1e-8f));
-  unsigned nib[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const float au = fabsf(bfround(__fdiv_rn(y[j], den)));
-    unsigned lv = 0;
-#pragma unroll
-    for (int i = 0; i < 7; i++) lv += (c_thr[i] < au);
-    t[j] = bfround(__fmul_rn(c_cen[lv], au));
-    nib[j] = (((code >> j) & 1u) << 3) | lv;
-  }
-#pragma unroll
-  for (int w = 8; w > 1; w >>= 1)
-#pragma unroll
-    for (int i = 0; i < w / 2; i++) t[i] = __fadd_rn(t[2 * i], t[2 * i + 1]);
-  const float alpha = fmaxf(t[0], 1e-6f);
-  *code_out = code;
-  *wt_out = f2bf(__fmul_rn(__fdiv_rn(r, alpha), n));
-  uint32_t packed = 0;
-#pragma unroll
-  for (int i = 0; i < 4; i++) packed |= ((nib[2 * i + 1] << 4) | nib[2 * i]) << (8 * i);
-  *packed_out = packed;
-}
 
 struct EncodeParams {
   const uint16_t* keys;
@@ -70,62 +24,186 @@ struct EncodeParams {
   int64_t L, chunk;
 };
 
-__global__ void __launch_bounds__(128) encode_kernel(EncodeParams p) {
+constexpr int EN_THREADS = 256;
+constexpr int EN_KEYS = EN_THREADS / 4;   // keys per block and round
+
+__device__ __forceinline__ void load_key32(uint4 (&raw)[4], const uint16_t* row, int s) {
+#pragma unroll
+  for (int i = 0; i < 4; i++) raw[i] = __ldg(reinterpret_cast<const uint4*>(row + 32 * s) + i);
+}
+
+// KEY_MAJOR: records stored key by key ([..,L,16(,4)] contiguous over subspaces), so a lane's share of a record is one
+// store; otherwise any strides.
+template <bool KEY_MAJOR>
+__global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
   __shared__ int hist[16 * 256];
-  const int tid = threadIdx.x, s = tid & 7, grp = tid >> 3;
-  const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
+  const int tid = threadIdx.x, s = tid & 3, grp = tid >> 2;
+  const int bh = blockIdx.x, b = bh / p.H, h = bh % p.H;
   if (p.counts) {
-    for (int i = tid; i < 16 * 256; i += 128) hist[i] = 0;
+    for (int i = tid; i < 16 * 256; i += EN_THREADS) hist[i] = 0;
     __syncthreads();
   }
-  float sg[16];
-  {
-    const uint4* sp = reinterpret_cast<const uint4*>(p.signs + 16 * s);
-    unpack8(__ldg(sp), sg);
-    unpack8(__ldg(sp + 1), sg + 8);
-  }
-  const int64_t begin = (int64_t)blockIdx.x * p.chunk;
+  RotateLane rl;
+  make_rotate_lane(rl, p.signs, s);
+  const int64_t begin = (int64_t)blockIdx.y * p.chunk;
   const int64_t end = min(p.L, begin + p.chunk);
   const uint16_t* kbase = p.keys + b * p.k_b + h * p.k_h;
-  for (int64_t k0 = begin; k0 < end; k0 += 16) {  // uniform per block: shuffles need whole warps
+  uint4 raw[4], nxt[4];
+  load_key32(raw, kbase + min(begin + grp, end - 1) * p.k_l, s);
+  for (int64_t k0 = begin; k0 < end; k0 += EN_KEYS) {  // uniform per block: shuffles need whole warps
     const int64_t key = k0 + grp;
-    const bool valid = key < end;
-    float x[16];
-    if (valid) {
-      const uint4* kp = reinterpret_cast<const uint4*>(kbase + key * p.k_l + 16 * s);
-      unpack8(__ldg(kp), x);
-      unpack8(__ldg(kp + 1), x + 8);
+    load_key32(nxt, kbase + min(key + EN_KEYS, end - 1) * p.k_l, s);   // in flight during the arithmetic
+    const KeyCode kc = code_key(raw, rl);
+#pragma unroll
+    for (int i = 0; i < 4; i++) raw[i] = nxt[i];
+    if (key >= end) continue;
+    if (KEY_MAJOR) {
+      *reinterpret_cast<uint32_t*>(p.codes + b * p.c_b + h * p.c_h + key * 16 + 4 * s) = kc.codes;
+      *reinterpret_cast<uint2*>(p.w + b * p.w_b + h * p.w_h + key * 16 + 4 * s) = kc.weights;
+      *reinterpret_cast<uint4*>(p.pk + b * p.p_b + h * p.p_h + key * 64 + 16 * s) = kc.packed;
     } else {
+      const uint32_t pk4[4] = {kc.packed.x, kc.packed.y, kc.packed.z, kc.packed.w};
 #pragma unroll
-      for (int i = 0; i < 16; i++) x[i] = 0.0f;
-    }
-    const float n = rotate16(x, sg, s);
-    if (!valid) continue;
+      for (int i = 0; i < 4; i++) {
+        const int sub = 4 * s + i;
+        const uint32_t wt = i < 2 ? kc.weights.x : kc.weights.y;
+        p.codes[b * p.c_b + h * p.c_h + sub * p.c_s + key * p.c_l] = (uint8_t)(kc.codes >> (8 * i));
+        p.w[b * p.w_b + h * p.w_h + sub * p.w_s + key * p.w_l] = (uint16_t)((i & 1) ? wt >> 16 : wt);
+        uint8_t* pp = p.pk + b * p.p_b + h * p.p_h + sub * p.p_s + key * p.p_l;
+        if ((reinterpret_cast<uintptr_t>(pp) & 3) == 0) {
+          *reinterpret_cast<uint32_t*>(pp) = pk4[i];
+        } else {
 #pragma unroll
-    for (int half = 0; half < 2; half++) {
-      const int sub = 2 * s + half;
-      unsigned code;
-      uint16_t wt;
-      uint32_t packed;
-      code_subspace(x + 8 * half, n, &code, &wt, &packed);
-      p.codes[b * p.c_b + h * p.c_h + sub * p.c_s + key * p.c_l] = (uint8_t)code;
-      p.w[b * p.w_b + h * p.w_h + sub * p.w_s + key * p.w_l] = wt;
-      uint8_t* pp = p.pk + b * p.p_b + h * p.p_h + sub * p.p_s + key * p.p_l;
-      if ((reinterpret_cast<uintptr_t>(pp) & 3) == 0) {
-        *reinterpret_cast<uint32_t*>(pp) = packed;
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; i++) pp[i] = (uint8_t)(packed >> (8 * i));
+          for (int j = 0; j < 4; j++) pp[j] = (uint8_t)(pk4[i] >> (8 * j));
+        }
       }
-      if (p.counts) atomicAdd(&hist[sub * 256 + code], 1);
     }
+    if (p.counts)
+#pragma unroll
+      for (int i = 0; i < 4; i++) atomicAdd(&hist[(4 * s + i) * 256 + ((kc.codes >> (8 * i)) & 0xffu)], 1);
   }
   if (p.counts) {
     __syncthreads();
     int32_t* dst = p.counts + (int64_t)bh * 16 * 256;
-    for (int i = tid; i < 16 * 256; i += 128)
+    for (int i = tid; i < 16 * 256; i += EN_THREADS)
       if (hist[i]) atomicAdd(dst + i, hist[i]);
   }
+}
+
+// ---- a prompt into the cache, one launch per sample ---------------------------------------------------------------
+// Token t of the prompt is a window row (the first `sink` tokens and the last `local` ones; all of them where the prompt
+// is not longer than both together) or zone row t - sink.  Every row is read once: its K and V go to the window or to the
+// store (K row and V row of a key next to each other), its key is coded into the staging arrays or the zone records, ||v||
+// and the cluster histogram come with it.  Block (h, chunk): consecutive tokens of one head, the heads of a token range
+// side by side in the grid, since they are neighbours in memory.
+// What bounds it: issue slots of the coding (180 warp instructions per key, two thirds of the issue slots, the half-rate ALU 60 % busy), then HBM (1136 bytes per key).
+// 131072 tokens x 8 heads on B200: 2003 us as coding, interleaving and copy launches, 282 us as this one.  Rows by bulk
+// copies into shared memory took 450 (two 256-byte copies per row are too many for the copy engine), by cp.async three
+// rounds ahead no less than with the next round in registers.
+
+struct PrefillParams {
+  const uint16_t* k;        // [P][H][128] of one sample
+  const uint16_t* v;
+  int64_t k_l, k_h, v_l, v_h;
+  const uint16_t* signs;
+  uint16_t* wk;             // window rows of the sample: head h at h * w_h, rows 128 apart
+  uint16_t* wv;
+  int64_t w_h;
+  uint8_t* win_codes;       // staging records of the sample: [H][cap_w][16], [H][cap_w][16], [H][cap_w][64], [H][cap_w]
+  uint16_t* win_w;
+  uint8_t* win_pk;
+  float* win_vnorm;
+  uint8_t* z_codes;         // zone records of the sample: [H][cap_z][16], [H][cap_z][16], [H][cap_z][64], [H][cap_z] or null
+  uint16_t* z_w;
+  uint8_t* z_pk;
+  float* z_vnorm;
+  int32_t* counts;          // [H][16][256], zero at launch
+  uint16_t* store;          // [H][store_cap][2][128]
+  int32_t* state;           // the layer's words, or null (see pk_prefill_sample)
+  int64_t P, N, cap_z, store_cap, chunk;
+  int H, cap_w, sink, n_window, b;
+};
+
+__global__ void __launch_bounds__(EN_THREADS, 2) prefill_kernel(PrefillParams p) {
+  __shared__ int hist[16 * 256];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, s = tid & 3, grp = tid >> 2;
+  const int h = blockIdx.x;
+  for (int i = tid; i < 16 * 256; i += EN_THREADS) hist[i] = 0;
+  if (p.state && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) {
+    p.state[0] = p.n_window, p.state[1] = 0, p.state[2] = 0, p.state[3] = 0;
+    p.state[4 + p.b] = (int32_t)p.N;
+  }
+  __syncthreads();
+  RotateLane rl;
+  make_rotate_lane(rl, p.signs, s);
+  const int64_t begin = (int64_t)blockIdx.y * p.chunk, end = min(p.P, begin + p.chunk);
+  const uint16_t* kb = p.k + h * p.k_h;
+  const uint16_t* vb = p.v + h * p.v_h;
+  // V is only copied: a half warp takes a row (16 bytes per lane), a warp the rows 2i, 2i + 1 of its eight in step i
+  uint4 kr[4], kn[4], vr[4];
+  auto load_v = [&](int64_t t0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      vr[i] = __ldg(reinterpret_cast<const uint4*>(vb + min(t0 + warp * 8 + 2 * i + (lane >> 4), end - 1) * p.v_l) + (lane & 15));
+  };
+  load_key32(kr, kb + min(begin + grp, end - 1) * p.k_l, s);
+  load_v(begin);
+  for (int64_t t0 = begin; t0 < end; t0 += EN_KEYS) {
+    load_key32(kn, kb + min(t0 + EN_KEYS + grp, end - 1) * p.k_l, s);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int64_t t = t0 + warp * 8 + 2 * i + (lane >> 4), z = t - p.sink;
+      const bool zone = z >= 0 && z < p.N;
+      if (!zone || p.z_vnorm) {   // uniform over the half warp of a row
+        const uint32_t w[4] = {vr[i].x, vr[i].y, vr[i].z, vr[i].w};
+        float a = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; j++) a = fmaf(lo_f(w[j]), lo_f(w[j]), fmaf(hi_f(w[j]), hi_f(w[j]), a));
+        const unsigned mask = 0xffffu << (lane & 16);
+#pragma unroll
+        for (int off = 1; off < 16; off <<= 1) a += __shfl_xor_sync(mask, a, off);
+        if (t < end && (lane & 15) == 0) {
+          if (zone) p.z_vnorm[(int64_t)h * p.cap_z + z] = sqrtf(a);
+          else p.win_vnorm[(int64_t)h * p.cap_w + (z < p.N || p.N == 0 ? t : t - p.N)] = sqrtf(a);
+        }
+      }
+      if (t < end) {
+        if (zone) __stcs(reinterpret_cast<uint4*>(p.store + ((int64_t)h * p.store_cap + z) * 256 + 128) + (lane & 15), vr[i]);
+        else reinterpret_cast<uint4*>(p.wv + h * p.w_h + (z < p.N || p.N == 0 ? t : t - p.N) * 128)[lane & 15] = vr[i];
+      }
+    }
+    load_v(t0 + EN_KEYS);
+    const KeyCode kc = code_key(kr, rl);
+    const int64_t t = t0 + grp, z = t - p.sink;   // zone row, if 0 <= z < N; window row t or t - N otherwise
+    if (t < end) {
+      if (z >= 0 && z < p.N) {
+        uint4* st = reinterpret_cast<uint4*>(p.store + ((int64_t)h * p.store_cap + z) * 256) + 4 * s;
+#pragma unroll
+        for (int i = 0; i < 4; i++) st[i] = kr[i];
+        const int64_t rec = (int64_t)h * p.cap_z + z;
+        *reinterpret_cast<uint32_t*>(p.z_codes + rec * 16 + 4 * s) = kc.codes;
+        *reinterpret_cast<uint2*>(p.z_w + rec * 16 + 4 * s) = kc.weights;
+        *reinterpret_cast<uint4*>(p.z_pk + rec * 64 + 16 * s) = kc.packed;
+#pragma unroll
+        for (int i = 0; i < 4; i++) atomicAdd(&hist[(4 * s + i) * 256 + ((kc.codes >> (8 * i)) & 0xffu)], 1);
+      } else {
+        const int64_t wrow = z < p.N || p.N == 0 ? t : t - p.N;
+        uint4* wk = reinterpret_cast<uint4*>(p.wk + h * p.w_h + wrow * 128) + 4 * s;
+#pragma unroll
+        for (int i = 0; i < 4; i++) wk[i] = kr[i];
+        const int64_t rec = (int64_t)h * p.cap_w + wrow;
+        *reinterpret_cast<uint32_t*>(p.win_codes + rec * 16 + 4 * s) = kc.codes;
+        *reinterpret_cast<uint2*>(p.win_w + rec * 16 + 4 * s) = kc.weights;
+        *reinterpret_cast<uint4*>(p.win_pk + rec * 64 + 16 * s) = kc.packed;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) kr[i] = kn[i];
+  }
+  __syncthreads();
+  int32_t* dst = p.counts + (int64_t)h * 16 * 256;
+  for (int i = tid; i < 16 * 256; i += EN_THREADS)
+    if (hist[i]) atomicAdd(dst + i, hist[i]);
 }
 
 __global__ void __launch_bounds__(256) count_kernel(const uint8_t* codes, int64_t c_b, int64_t c_h,
@@ -224,42 +302,33 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
   float* wn = p.win_vnorm + bh * p.cap_w;
   const bool ok = pos >= 0 && pos < p.cap_w;
   if (tid < 32 && ok) {
-    const int s = lane & 7;
-    const uint4* kr = reinterpret_cast<const uint4*>(p.k_row + b * p.kr_b + h * p.kr_h);
+    const int s = lane & 3, l = lane & 15;
+    const uint16_t* kr = p.k_row + b * p.kr_b + h * p.kr_h;
     const uint4* vr = reinterpret_cast<const uint4*>(p.v_row + b * p.vr_b + h * p.vr_h);
     // the rows themselves: lanes 0-15 carry K, lanes 16-31 carry V
-    {
-      const int l = lane & 15;
-      const uint4 v = __ldg((lane < 16 ? kr : vr) + l);
-      reinterpret_cast<uint4*>((lane < 16 ? wk : wv) + (int64_t)pos * 128)[l] = v;
-    }
-    float x[16], sg[16], y[16];
-    unpack8(__ldg(kr + 2 * s), x);
-    unpack8(__ldg(kr + 2 * s + 1), x + 8);
-    unpack8(__ldg(reinterpret_cast<const uint4*>(p.signs) + 2 * s), sg);
-    unpack8(__ldg(reinterpret_cast<const uint4*>(p.signs) + 2 * s + 1), sg + 8);
-    unpack8(__ldg(vr + 2 * s), y);
-    unpack8(__ldg(vr + 2 * s + 1), y + 8);
+    const uint4 cp = __ldg((lane < 16 ? reinterpret_cast<const uint4*>(kr) : vr) + l);
+    uint4 raw[4];
+    load_key32(raw, kr, s);
+    RotateLane rl;
+    make_rotate_lane(rl, p.signs, s);
+    float y[8];
+    unpack8(__ldg(vr + l), y);
+    reinterpret_cast<uint4*>((lane < 16 ? wk : wv) + (int64_t)pos * 128)[l] = cp;
     // ||v||: fp32, pairwise tree over adjacent dimensions
 #pragma unroll
-    for (int i = 0; i < 16; i++) y[i] = __fmul_rn(y[i], y[i]);
+    for (int i = 0; i < 8; i++) y[i] = __fmul_rn(y[i], y[i]);
 #pragma unroll
-    for (int w = 16; w > 1; w >>= 1)
+    for (int w = 8; w > 1; w >>= 1)
 #pragma unroll
       for (int i = 0; i < w / 2; i++) y[i] = __fadd_rn(y[2 * i], y[2 * i + 1]);
     float vs = y[0];
 #pragma unroll
-    for (int off = 1; off < 8; off <<= 1) vs = __fadd_rn(vs, __shfl_xor_sync(FULL, vs, off));
-    const float n = rotate16(x, sg, s);
-    unsigned code[2];
-    uint16_t wt[2];
-    uint32_t packed[2];
-    code_subspace(x, n, &code[0], &wt[0], &packed[0]);
-    code_subspace(x + 8, n, &code[1], &wt[1], &packed[1]);
-    if (lane < 8) {
-      *reinterpret_cast<uint16_t*>(wc + (int64_t)pos * 16 + 2 * s) = (uint16_t)(code[0] | (code[1] << 8));
-      *reinterpret_cast<uint32_t*>(ww + (int64_t)pos * 16 + 2 * s) = (uint32_t)wt[0] | ((uint32_t)wt[1] << 16);
-      *reinterpret_cast<uint2*>(wp + (int64_t)pos * 64 + 8 * s) = make_uint2(packed[0], packed[1]);
+    for (int off = 1; off < 16; off <<= 1) vs = __fadd_rn(vs, __shfl_xor_sync(FULL, vs, off));
+    const KeyCode kc = code_key(raw, rl);   // (eight times the same: every group of four lanes)
+    if (lane < 4) {
+      *reinterpret_cast<uint32_t*>(wc + (int64_t)pos * 16 + 4 * s) = kc.codes;
+      *reinterpret_cast<uint2*>(ww + (int64_t)pos * 16 + 4 * s) = kc.weights;
+      *reinterpret_cast<uint4*>(wp + (int64_t)pos * 64 + 16 * s) = kc.packed;
       if (lane == 0) wn[pos] = __fsqrt_rn(vs);
     }
   }
@@ -331,6 +400,18 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
 
 }  // namespace
 
+// Keys per block: about eight blocks per SM over the whole launch (two waves of what is resident), whole rounds of 64 keys,
+// at most 4096 so that the blocks stay many; at least 64, so that clearing and adding a block's 16 KB histogram does not
+// outweigh the coding.
+static int64_t encode_chunk(int64_t L, int64_t heads) {
+  const int64_t target = (int64_t)sm_count() * 8;
+  int64_t chunk = ((L * heads + target - 1) / target + EN_KEYS - 1) / EN_KEYS * EN_KEYS;
+  if (chunk < 64) chunk = 64;
+  if (chunk > 4096) chunk = 4096;
+  while ((L + chunk - 1) / chunk > 65535) chunk *= 2;
+  return chunk;
+}
+
 // Host launchers shared with the fused retrieval entry point.
 int launch_query_prep(const uint16_t* queries, int bs, int Hq, int H, const uint16_t* signs,
                       uint16_t* q_blocks, uint16_t* q_norm, uint16_t* query_avg, cudaStream_t st) {
@@ -391,18 +472,162 @@ extern "C" int pk_encode_keys(const pk_tensor* keys, const pk_tensor* signs, con
   p.counts = cluster_counts ? (int32_t*)cluster_counts->data : nullptr;
   p.H = (int)H;
   p.L = L;
-  // chunk of keys per block: enough blocks to fill the machine, at most 2048 keys per block so the
-  // shared histogram is flushed by few blocks
-  int64_t target = (int64_t)sm_count() * 8;
-  int64_t chunk = (L * bs * H + target - 1) / target;
-  chunk = ((chunk + 15) / 16) * 16;
-  if (chunk < 16) chunk = 16;
-  if (chunk > 2048) chunk = 2048;
-  p.chunk = chunk;
-  dim3 grid((unsigned)((L + chunk - 1) / chunk), (unsigned)(bs * H));
+  p.chunk = encode_chunk(L, bs * H);
+  const bool key_major = p.c_s == 1 && p.c_l == 16 && p.w_s == 1 && p.w_l == 16 && p.p_s == 4 && p.p_l == 64 &&
+                         (reinterpret_cast<uintptr_t>(p.codes) & 3) == 0 && (reinterpret_cast<uintptr_t>(p.w) & 7) == 0 &&
+                         (reinterpret_cast<uintptr_t>(p.pk) & 15) == 0 && ((p.c_b | p.c_h | p.w_b | p.w_h) & 3) == 0 && ((p.p_b | p.p_h) & 15) == 0;
+  dim3 grid((unsigned)(bs * H), (unsigned)((L + p.chunk - 1) / p.chunk));
+  PK_REQUIRE(grid.y <= 65535, "too many keys for one call");
   StageTimer tm(ST_ENCODE, (cudaStream_t)stream);
-  encode_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(p);
+  if (key_major) encode_kernel<true><<<grid, EN_THREADS, 0, (cudaStream_t)stream>>>(p);
+  else encode_kernel<false><<<grid, EN_THREADS, 0, (cudaStream_t)stream>>>(p);
   return check_launch("encode_keys");
+}
+
+// The tensors of one cache layer that pk_append_encode and pk_prefill_sample share.
+struct CacheLayer {
+  int64_t bs, H, cap_w, cap_z, w_b, w_h;
+  float* z_vnorm;
+};
+static int check_cache_layer(CacheLayer* c, const pk_tensor* window_k, const pk_tensor* window_v, const pk_tensor* win_codes,
+                             const pk_tensor* win_weight, const pk_tensor* win_4bit, const pk_tensor* win_vnorm,
+                             const pk_tensor* codebook, const pk_tensor* block_weight, const pk_tensor* packed_4bit,
+                             const pk_tensor* value_norm, const pk_tensor* cluster_counts, const pk_tensor* state) {
+  PK_CHECK_TENSOR(window_k, PK_BF16, 4);
+  PK_CHECK_TENSOR(window_v, PK_BF16, 4);
+  PK_CHECK_TENSOR(win_codes, PK_U8, 4);
+  PK_CHECK_TENSOR(win_weight, PK_BF16, 4);
+  PK_CHECK_TENSOR(win_4bit, PK_U8, 5);
+  PK_CHECK_TENSOR(win_vnorm, PK_F32, 3);
+  PK_CHECK_TENSOR(codebook, PK_U8, 4);
+  PK_CHECK_TENSOR(block_weight, PK_BF16, 4);
+  PK_CHECK_TENSOR(packed_4bit, PK_U8, 5);
+  PK_CHECK_TENSOR(cluster_counts, PK_I32, 4);
+  PK_CHECK_TENSOR(state, PK_I32, 1);
+  const int64_t bs = window_k->shape[0], H = window_k->shape[1], cap_w = window_k->shape[2];
+  PK_REQUIRE(bs >= 1 && H >= 1 && bs * H < (1ll << 31), "window_k must be [bs,H,cap,128]");
+  PK_REQUIRE(window_k->shape[3] == 128 && window_k->stride[3] == 1 && window_k->stride[2] == 128 &&
+                 (reinterpret_cast<uintptr_t>(window_k->data) & 15) == 0 && (reinterpret_cast<uintptr_t>(window_v->data) & 15) == 0,
+             "window_k must be [bs,H,cap,128] with rows 128 elements apart, 16-byte aligned");
+  for (int i = 0; i < 4; i++)
+    PK_REQUIRE(window_v->shape[i] == window_k->shape[i] && (window_k->shape[i] == 1 || window_v->stride[i] == window_k->stride[i]),
+               "window_k and window_v must have the same shape and strides");
+  PK_REQUIRE(window_k->stride[0] % 8 == 0 && window_k->stride[1] % 8 == 0, "window strides must be multiples of 8 elements");
+  // staging arrays: contiguous, window-aligned
+  PK_REQUIRE(is_contig(win_codes) && win_codes->shape[0] == bs && win_codes->shape[1] == H && win_codes->shape[2] == cap_w &&
+                 win_codes->shape[3] == 16 && is_contig(win_weight) && numel(win_weight) == bs * H * cap_w * 16 &&
+                 is_contig(win_4bit) && numel(win_4bit) == bs * H * cap_w * 64 && is_contig(win_vnorm) &&
+                 numel(win_vnorm) == bs * H * cap_w,
+             "staging arrays must be contiguous [bs,H,cap,16] u8, [bs,H,cap,16] bf16, [bs,H,cap,16,4] u8, [bs,H,cap] f32");
+  for (const pk_tensor* t : {win_codes, win_weight, win_4bit})
+    PK_REQUIRE((reinterpret_cast<uintptr_t>(t->data) & 15) == 0, "staging arrays must be 16-byte aligned");
+  // zone records: logical [bs,H,16,cap_z(,4)], stored key-major and contiguous
+  const int64_t cap_z = codebook->shape[3];
+  PK_REQUIRE(codebook->shape[0] == bs && codebook->shape[1] == H && codebook->shape[2] == 16 && codebook->stride[2] == 1 &&
+                 codebook->stride[3] == 16 && codebook->stride[1] == cap_z * 16 && (bs == 1 || codebook->stride[0] == H * cap_z * 16),
+             "codebook must be the key-major [bs,H,16,cap] view of a contiguous [bs,H,cap,16] buffer");
+  PK_REQUIRE(block_weight->shape[3] == cap_z && block_weight->shape[2] == 16 && block_weight->stride[2] == 1 &&
+                 block_weight->stride[3] == 16 && block_weight->stride[1] == cap_z * 16 &&
+                 (bs == 1 || block_weight->stride[0] == H * cap_z * 16),
+             "block_weight must be the key-major [bs,H,16,cap] view of a contiguous [bs,H,cap,16] buffer");
+  PK_REQUIRE(packed_4bit->shape[3] == cap_z && packed_4bit->shape[2] == 16 && packed_4bit->shape[4] == 4 &&
+                 packed_4bit->stride[4] == 1 && packed_4bit->stride[2] == 4 && packed_4bit->stride[3] == 64 &&
+                 packed_4bit->stride[1] == cap_z * 64 && (bs == 1 || packed_4bit->stride[0] == H * cap_z * 64),
+             "packed_4bit must be the key-major [bs,H,16,cap,4] view of a contiguous [bs,H,cap,16,4] buffer");
+  for (const pk_tensor* t : {codebook, block_weight, packed_4bit})
+    PK_REQUIRE((reinterpret_cast<uintptr_t>(t->data) & 15) == 0, "zone records must be 16-byte aligned");
+  float* zv = nullptr;
+  if (value_norm) {
+    PK_CHECK_TENSOR(value_norm, PK_F32, 3);
+    PK_REQUIRE(is_contig(value_norm) && value_norm->shape[0] == bs && value_norm->shape[1] == H && value_norm->shape[2] == cap_z,
+               "value_norm must be contiguous [bs,H,cap] with the zone's capacity");
+    zv = (float*)value_norm->data;
+  }
+  PK_REQUIRE(is_contig(cluster_counts) && cluster_counts->shape[0] == bs && cluster_counts->shape[1] == H &&
+                 cluster_counts->shape[2] == 16 && cluster_counts->shape[3] == 256,
+             "cluster_counts must be contiguous [bs,H,16,256]");
+  PK_REQUIRE(state->stride[0] == 1 && state->shape[0] >= 4 + bs, "state must hold 4 + bs int32 words");
+  c->bs = bs, c->H = H, c->cap_w = cap_w, c->cap_z = cap_z, c->z_vnorm = zv;
+  c->w_b = bs == 1 ? 0 : window_k->stride[0], c->w_h = H == 1 ? 0 : window_k->stride[1];
+  return PK_OK;
+}
+
+extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const pk_tensor* signs, const pk_tensor* window_k,
+                                 const pk_tensor* window_v, const pk_tensor* win_codes, const pk_tensor* win_weight,
+                                 const pk_tensor* win_4bit, const pk_tensor* win_vnorm, const pk_tensor* codebook,
+                                 const pk_tensor* block_weight, const pk_tensor* packed_4bit, const pk_tensor* value_norm,
+                                 const pk_tensor* cluster_counts, const pk_tensor* rows, const pk_tensor* state, int64_t b,
+                                 int64_t sink, int64_t local, void* stream) {
+  PK_CHECK_TENSOR(k, PK_BF16, 3);
+  PK_CHECK_TENSOR(v, PK_BF16, 3);
+  PK_CHECK_TENSOR(signs, PK_BF16, 1);
+  PK_CHECK_TENSOR(cluster_counts, PK_I32, 4);
+  PK_CHECK_TENSOR(state, PK_I32, 1);
+  const int64_t P = k->shape[0], H = k->shape[1];
+  for (const pk_tensor* t : {k, v})
+    PK_REQUIRE(t->shape[0] == P && t->shape[1] == H && t->shape[2] == 128 && t->stride[2] == 1 &&
+                   (reinterpret_cast<uintptr_t>(t->data) & 15) == 0 && (P == 1 || t->stride[0] % 8 == 0) && (H == 1 || t->stride[1] % 8 == 0),
+               "k / v must be [P,H,128] with last stride 1 and 16-byte aligned rows");
+  PK_REQUIRE(signs->shape[0] == 128 && signs->stride[0] == 1 && (reinterpret_cast<uintptr_t>(signs->data) & 15) == 0,
+             "signs must be a 16-byte aligned [128]");
+  CacheLayer c;
+  int rc = check_cache_layer(&c, window_k, window_v, win_codes, win_weight, win_4bit, win_vnorm, codebook, block_weight,
+                             packed_4bit, value_norm, cluster_counts, state);
+  if (rc) return rc;
+  PK_REQUIRE(c.H == H && b >= 0 && b < c.bs, "k / v and the cache disagree on the heads, or sample %lld does not exist", (long long)b);
+  PK_REQUIRE(P >= 1 && sink >= 0 && local >= 0 && sink + local <= c.cap_w, "need at least one token and sink + local rows of window");
+  const int64_t N = P > sink + local ? P - sink - local : 0;
+  PK_REQUIRE(N > 0 || P <= c.cap_w, "a prompt without zone rows must fit the window");
+  PK_REQUIRE(N <= c.cap_z, "the zone records hold %lld keys, %lld needed", (long long)c.cap_z, (long long)N);
+  if (N > 0) {
+    PK_CHECK_TENSOR(rows, PK_BF16, 4);
+    PK_REQUIRE(rows->shape[0] == H && rows->shape[1] >= N && rows->shape[2] == 2 && rows->shape[3] == 128 && rows->stride[3] == 1 &&
+                   rows->stride[2] == 128 && rows->stride[1] == 256 && (H == 1 || rows->stride[0] % 256 == 0) &&
+                   (reinterpret_cast<uintptr_t>(rows->data) & 15) == 0,
+               "rows must be [H,n,2,128] with n >= %lld, a head's rows contiguous", (long long)N);
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  PrefillParams p = {};
+  p.k = (const uint16_t*)k->data, p.v = (const uint16_t*)v->data;
+  p.k_l = k->stride[0], p.k_h = k->stride[1], p.v_l = v->stride[0], p.v_h = v->stride[1];
+  p.signs = (const uint16_t*)signs->data;
+  p.wk = (uint16_t*)window_k->data + b * c.w_b, p.wv = (uint16_t*)window_v->data + b * c.w_b, p.w_h = c.w_h;
+  const int64_t wr = b * H * c.cap_w, zr = b * H * c.cap_z;
+  p.win_codes = (uint8_t*)win_codes->data + wr * 16, p.win_w = (uint16_t*)win_weight->data + wr * 16;
+  p.win_pk = (uint8_t*)win_4bit->data + wr * 64, p.win_vnorm = (float*)win_vnorm->data + wr;
+  p.z_codes = (uint8_t*)codebook->data + zr * 16, p.z_w = (uint16_t*)block_weight->data + zr * 16;
+  p.z_pk = (uint8_t*)packed_4bit->data + zr * 64, p.z_vnorm = c.z_vnorm ? c.z_vnorm + zr : nullptr;
+  p.counts = (int32_t*)cluster_counts->data + b * H * 16 * 256;
+  p.state = (int32_t*)state->data;
+  p.P = P, p.N = N, p.cap_z = c.cap_z;
+  if (N > 0) p.store = (uint16_t*)rows->data, p.store_cap = H == 1 ? rows->shape[1] : rows->stride[0] / 256;
+  p.H = (int)H, p.cap_w = (int)c.cap_w, p.sink = (int)sink, p.n_window = (int)(N > 0 ? sink + local : P), p.b = (int)b;
+  p.chunk = encode_chunk(P, H);
+  if (cudaMemsetAsync(p.counts, 0, (size_t)(H * 16 * 256 * 4), st) != cudaSuccess) return check_launch("prefill memset", 0);
+  StageTimer tm(ST_ENCODE, st);
+  prefill_kernel<<<dim3((unsigned)H, (unsigned)((P + p.chunk - 1) / p.chunk)), EN_THREADS, 0, st>>>(p);
+  return check_launch("prefill");
+}
+
+extern "C" int pk_copy_rows(const pk_tensor* src, const pk_tensor* dst, void* stream) {
+  PK_REQUIRE(src && dst && src->data && dst->data, "src / dst is null");
+  PK_REQUIRE(src->dtype == dst->dtype && src->ndim == dst->ndim && src->ndim >= 2, "src and dst must have the same type and shape");
+  int64_t inner = elem_size(src->dtype);
+  for (int i = src->ndim - 1; i >= 0; i--) {
+    PK_REQUIRE(src->shape[i] == dst->shape[i], "src and dst must have the same shape");
+    if (i == 0) break;
+    for (const pk_tensor* t : {src, dst})
+      PK_REQUIRE(t->shape[i] == 1 || t->stride[i] * elem_size(t->dtype) == inner, "everything behind the first dimension must be contiguous");
+    inner *= src->shape[i];
+  }
+  const int64_t H = src->shape[0];
+  if (H * inner == 0) return PK_OK;
+  const int64_t sp = H == 1 ? inner : src->stride[0] * elem_size(src->dtype), dp = H == 1 ? inner : dst->stride[0] * elem_size(dst->dtype);
+  PK_REQUIRE(sp >= inner && dp >= inner, "the blocks overlap");
+  if (cudaMemcpy2DAsync(dst->data, (size_t)dp, src->data, (size_t)sp, (size_t)inner, (size_t)H, cudaMemcpyDefault,
+                        (cudaStream_t)stream) != cudaSuccess)
+    return check_launch("copy_rows", 0);
+  return PK_OK;
 }
 
 extern "C" int pk_count_clusters(const pk_tensor* codebook, const pk_tensor* counts, int accumulate,
@@ -471,20 +696,13 @@ extern "C" int pk_append_encode(const pk_tensor* k_row, const pk_tensor* v_row, 
   PK_CHECK_TENSOR(k_row, PK_BF16, 4);
   PK_CHECK_TENSOR(v_row, PK_BF16, 4);
   PK_CHECK_TENSOR(signs, PK_BF16, 1);
-  PK_CHECK_TENSOR(window_k, PK_BF16, 4);
-  PK_CHECK_TENSOR(window_v, PK_BF16, 4);
-  PK_CHECK_TENSOR(win_codes, PK_U8, 4);
-  PK_CHECK_TENSOR(win_weight, PK_BF16, 4);
-  PK_CHECK_TENSOR(win_4bit, PK_U8, 5);
-  PK_CHECK_TENSOR(win_vnorm, PK_F32, 3);
-  PK_CHECK_TENSOR(codebook, PK_U8, 4);
-  PK_CHECK_TENSOR(block_weight, PK_BF16, 4);
-  PK_CHECK_TENSOR(packed_4bit, PK_U8, 5);
-  PK_CHECK_TENSOR(cluster_counts, PK_I32, 4);
   PK_CHECK_TENSOR(store_kv, PK_BF16, 5);
-  PK_CHECK_TENSOR(state, PK_I32, 1);
-  const int64_t bs = window_k->shape[0], H = window_k->shape[1], cap_w = window_k->shape[2];
-  PK_REQUIRE(bs >= 1 && H >= 1 && bs * H < (1ll << 31), "window_k must be [bs,H,cap,128]");
+  CacheLayer c;
+  int rc = check_cache_layer(&c, window_k, window_v, win_codes, win_weight, win_4bit, win_vnorm, codebook, block_weight,
+                             packed_4bit, value_norm, cluster_counts, state);
+  if (rc) return rc;
+  const int64_t bs = c.bs, H = c.H, cap_w = c.cap_w, cap_z = c.cap_z;
+  float* zv = c.z_vnorm;
   PK_REQUIRE(k_row->shape[0] == bs && k_row->shape[1] == 1 && k_row->shape[2] == H && k_row->shape[3] == 128 &&
                  k_row->stride[3] == 1 && v_row->shape[0] == bs && v_row->shape[1] == 1 && v_row->shape[2] == H &&
                  v_row->shape[3] == 128 && v_row->stride[3] == 1,
@@ -495,58 +713,17 @@ extern "C" int pk_append_encode(const pk_tensor* k_row, const pk_tensor* v_row, 
                "k_row / v_row rows must be 16-byte aligned");
   PK_REQUIRE(signs->shape[0] == 128 && signs->stride[0] == 1 && (reinterpret_cast<uintptr_t>(signs->data) & 15) == 0,
              "signs must be a 16-byte aligned [128]");
-  PK_REQUIRE(window_k->shape[3] == 128 && window_k->stride[3] == 1 && window_k->stride[2] == 128 &&
-                 (reinterpret_cast<uintptr_t>(window_k->data) & 15) == 0 && (reinterpret_cast<uintptr_t>(window_v->data) & 15) == 0,
-             "window_k must be [bs,H,cap,128] with rows 128 elements apart, 16-byte aligned");
-  for (int i = 0; i < 4; i++)
-    PK_REQUIRE(window_v->shape[i] == window_k->shape[i] && (window_k->shape[i] == 1 || window_v->stride[i] == window_k->stride[i]),
-               "window_k and window_v must have the same shape and strides");
-  PK_REQUIRE(window_k->stride[0] % 8 == 0 && window_k->stride[1] % 8 == 0, "window strides must be multiples of 8 elements");
   PK_REQUIRE(sink >= 0 && interval >= 1 && sink + interval <= cap_w, "need sink + interval <= window capacity");
-  // staging arrays: contiguous, window-aligned
-  PK_REQUIRE(is_contig(win_codes) && win_codes->shape[0] == bs && win_codes->shape[1] == H && win_codes->shape[2] == cap_w &&
-                 win_codes->shape[3] == 16 && is_contig(win_weight) && numel(win_weight) == bs * H * cap_w * 16 &&
-                 is_contig(win_4bit) && numel(win_4bit) == bs * H * cap_w * 64 && is_contig(win_vnorm) &&
-                 numel(win_vnorm) == bs * H * cap_w,
-             "staging arrays must be contiguous [bs,H,cap,16] u8, [bs,H,cap,16] bf16, [bs,H,cap,16,4] u8, [bs,H,cap] f32");
-  for (const pk_tensor* t : {win_codes, win_weight, win_4bit})
-    PK_REQUIRE((reinterpret_cast<uintptr_t>(t->data) & 15) == 0, "staging arrays must be 16-byte aligned");
-  // zone records: logical [bs,H,16,cap_z(,4)], stored key-major and contiguous
-  const int64_t cap_z = codebook->shape[3];
-  PK_REQUIRE(codebook->shape[0] == bs && codebook->shape[1] == H && codebook->shape[2] == 16 && codebook->stride[2] == 1 &&
-                 codebook->stride[3] == 16 && codebook->stride[1] == cap_z * 16 && (bs == 1 || codebook->stride[0] == H * cap_z * 16),
-             "codebook must be the key-major [bs,H,16,cap] view of a contiguous [bs,H,cap,16] buffer");
-  PK_REQUIRE(block_weight->shape[3] == cap_z && block_weight->shape[2] == 16 && block_weight->stride[2] == 1 &&
-                 block_weight->stride[3] == 16 && block_weight->stride[1] == cap_z * 16 &&
-                 (bs == 1 || block_weight->stride[0] == H * cap_z * 16),
-             "block_weight must be the key-major [bs,H,16,cap] view of a contiguous [bs,H,cap,16] buffer");
-  PK_REQUIRE(packed_4bit->shape[3] == cap_z && packed_4bit->shape[2] == 16 && packed_4bit->shape[4] == 4 &&
-                 packed_4bit->stride[4] == 1 && packed_4bit->stride[2] == 4 && packed_4bit->stride[3] == 64 &&
-                 packed_4bit->stride[1] == cap_z * 64 && (bs == 1 || packed_4bit->stride[0] == H * cap_z * 64),
-             "packed_4bit must be the key-major [bs,H,16,cap,4] view of a contiguous [bs,H,cap,16,4] buffer");
-  for (const pk_tensor* t : {codebook, block_weight, packed_4bit})
-    PK_REQUIRE((reinterpret_cast<uintptr_t>(t->data) & 15) == 0, "zone records must be 16-byte aligned");
-  float* zv = nullptr;
-  if (value_norm) {
-    PK_CHECK_TENSOR(value_norm, PK_F32, 3);
-    PK_REQUIRE(is_contig(value_norm) && value_norm->shape[0] == bs && value_norm->shape[1] == H && value_norm->shape[2] == cap_z,
-               "value_norm must be contiguous [bs,H,cap] with the zone's capacity");
-    zv = (float*)value_norm->data;
-  }
-  PK_REQUIRE(is_contig(cluster_counts) && cluster_counts->shape[0] == bs && cluster_counts->shape[1] == H &&
-                 cluster_counts->shape[2] == 16 && cluster_counts->shape[3] == 256,
-             "cluster_counts must be contiguous [bs,H,16,256]");
   PK_REQUIRE(is_contig(store_kv) && store_kv->shape[0] == bs && store_kv->shape[1] == H && store_kv->shape[3] == 2 &&
                  store_kv->shape[4] == 128 && (reinterpret_cast<uintptr_t>(store_kv->data) & 15) == 0,
              "store_kv must be contiguous, 16-byte aligned [bs,H,cap,2,128] (device or pinned host memory)");
-  PK_REQUIRE(state->stride[0] == 1 && state->shape[0] >= 4 + bs, "state must hold 4 + bs int32 words");
   AppendParams p;
   p.k_row = (const uint16_t*)k_row->data, p.v_row = (const uint16_t*)v_row->data;
   p.kr_b = k_row->shape[0] == 1 ? 0 : k_row->stride[0], p.kr_h = k_row->shape[2] == 1 ? 0 : k_row->stride[2];
   p.vr_b = v_row->shape[0] == 1 ? 0 : v_row->stride[0], p.vr_h = v_row->shape[2] == 1 ? 0 : v_row->stride[2];
   p.signs = (const uint16_t*)signs->data;
   p.wk = (uint16_t*)window_k->data, p.wv = (uint16_t*)window_v->data;
-  p.w_b = window_k->shape[0] == 1 ? 0 : window_k->stride[0], p.w_h = window_k->shape[1] == 1 ? 0 : window_k->stride[1];
+  p.w_b = c.w_b, p.w_h = c.w_h;
   p.win_codes = (uint8_t*)win_codes->data, p.win_w = (uint16_t*)win_weight->data, p.win_pk = (uint8_t*)win_4bit->data;
   p.win_vnorm = (float*)win_vnorm->data;
   p.z_codes = (uint8_t*)codebook->data, p.z_w = (uint16_t*)block_weight->data, p.z_pk = (uint8_t*)packed_4bit->data;

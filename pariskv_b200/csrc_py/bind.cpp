@@ -261,6 +261,40 @@ PyObject* py_retrieve(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PK_PY_END
 }
 
+// k, v, signs, window_k, window_v, win_codes, win_weight, win_4bit, win_vnorm, codebook, block_weight, packed_4bit,
+// value_norm, cluster_counts, rows, state, b, sink, local
+PyObject* py_prefill_sample(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (!arity(n, 19, "prefill_sample")) return nullptr;
+  PK_PY_BEGIN
+  Arg t[16];
+  for (int i = 0; i < 16; i++)
+    if (!take(a[i], &t[i], i == 12 || i == 14 ? ANY : CUDA)) return nullptr;
+  int64_t b, sink, local;
+  if (!to_i64(a[16], &b) || !to_i64(a[17], &sink) || !to_i64(a[18], &local)) return nullptr;
+  if (!t[0].t) return PyErr_SetString(PyExc_TypeError, "k is None"), nullptr;
+  void* st = stream_of(*t[0].t);
+  const int rc = without_gil([&] {
+    return pk_prefill_sample(t[0].p(), t[1].p(), t[2].p(), t[3].p(), t[4].p(), t[5].p(), t[6].p(), t[7].p(), t[8].p(), t[9].p(),
+                             t[10].p(), t[11].p(), t[12].p(), t[13].p(), t[14].p(), t[15].p(), b, sink, local, st);
+  });
+  if (rc) return raise(rc);
+  Py_RETURN_NONE;
+  PK_PY_END
+}
+
+// src (device), dst (device or pinned host)
+PyObject* py_copy_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (!arity(n, 2, "copy_rows")) return nullptr;
+  PK_PY_BEGIN
+  Arg src, dst;
+  if (!need(a[0], &src, CUDA) || !need(a[1], &dst, ANY)) return nullptr;
+  void* st = stream_of(*src.t);
+  const int rc = without_gil([&] { return pk_copy_rows(src.p(), dst.p(), st); });
+  if (rc) return raise(rc);
+  Py_RETURN_NONE;
+  PK_PY_END
+}
+
 // keys, signs, codebook, block_weight, packed_4bit, cluster_counts
 PyObject* py_encode_keys(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!arity(n, 6, "encode_keys")) return nullptr;
@@ -530,6 +564,8 @@ PyMethodDef methods[] = {
     PK_METHOD("append_encode", py_append_encode),
     PK_METHOD("sparse_attention", py_attention),
     PK_METHOD("retrieve_ex", py_retrieve),
+    PK_METHOD("prefill_sample", py_prefill_sample),
+    PK_METHOD("copy_rows", py_copy_rows),
     PK_METHOD("encode_keys", py_encode_keys),
     PK_METHOD("query_prep", py_query_prep),
     PK_METHOD("rank_clusters", py_rank_clusters),

@@ -1,0 +1,51 @@
+"""The one-launch prompt ingestion against the oracle: window rows, zone records, histogram, store rows, value norms and
+position words, at prompt lengths around the edges of the window and of a block's rounds."""
+import pytest
+import torch
+
+from conftest import bits_of
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("offload", [True, False])
+@pytest.mark.parametrize("P", [1, 20, 21, 51, 84, 85, 700, 4301])
+def test_prefill_matches_oracle(oracle, P, offload):
+    from pariskv_b200.cache_hub.polar_cache_adaptivek_varlen import polar_cache
+    H, sink, local, bs = 3, 4, 16, 2
+    cache = polar_cache(valid_start=[5, 5], layer_num=1, batch_size=bs, max_length=P + 5 + 32, num_key_value_heads=H,
+                        num_heads=2 * H, head_dim=128, dtype=torch.bfloat16, layer_mapping={"0": DEV}, max_new_length=32,
+                        sink_size=sink, local_size=local, final_topk=16, dynamic_update_interval=8, enable_offload=offload)
+    g = torch.Generator().manual_seed(P)
+    k = torch.randn(bs, P + 5, H, 128, generator=g)
+    k[..., [7, 37, 71, 101]] *= 8.0
+    k[:, 5, 0] = 0.0                                   # a zero key
+    k = (k * torch.exp(0.5 * torch.randn(bs, P + 5, H, 1, generator=g))).to(torch.bfloat16)
+    v = torch.randn(bs, P + 5, H, 128, generator=g).to(torch.bfloat16)
+    for _ in range(2):                                 # the second prompt overwrites the first one's histogram
+        cache.prefill_update_kv_cache(None, k.to(DEV), v.to(DEV), 0, 0)
+    cache.sync(0, 0)
+    torch.cuda.synchronize()
+    N = max(0, P - sink - local)
+    n_win = sink + local if N else P
+    assert cache._layer_state[0].tolist() == [n_win, 0, 0, 0] + [N] * bs
+    kt, vt = k[:, 5:].transpose(1, 2), v[:, 5:].transpose(1, 2)                       # [bs,H,P,128]
+    win = list(range(P)) if N == 0 else list(range(sink)) + list(range(P - local, P))
+    cb, w, pk = oracle.encode(kt.contiguous(), cache.srht_diagonal_signs.cpu())       # [bs,H,16,P(,4)]
+    assert torch.equal(cache.unified_keys_gpu[0][:, :, :n_win].cpu(), kt[:, :, win])
+    assert torch.equal(cache.unified_values_gpu[0][:, :, :n_win].cpu(), vt[:, :, win])
+    assert torch.equal(cache._win_codes[0][:, :, :n_win].cpu().permute(0, 1, 3, 2), cb[..., win])
+    assert torch.equal(bits_of(cache._win_weight[0][:, :, :n_win].cpu().permute(0, 1, 3, 2)), bits_of(w[..., win]))
+    assert torch.equal(cache._win_4bit[0][:, :, :n_win].cpu().permute(0, 1, 3, 2, 4), pk[..., win, :])
+    norm = vt.float().norm(dim=-1)
+    assert torch.allclose(cache._win_vnorm[0][:, :, :n_win].cpu(), norm[:, :, win], rtol=1e-5)
+    zone = slice(sink, sink + N)
+    assert torch.equal(cache.codebook_gpu[0][..., :N].cpu(), cb[..., zone])
+    assert torch.equal(bits_of(cache.key_block_weight_gpu[0][..., :N].cpu()), bits_of(w[..., zone]))
+    assert torch.equal(cache.key_4bit_packed_gpu[0][..., :N, :].cpu(), pk[..., zone, :])
+    assert torch.allclose(cache.value_norm_gpu[0][..., :N].cpu(), norm[..., zone], rtol=1e-5)
+    assert torch.equal(cache._store_k[0][:, :, :N].cpu(), kt[:, :, zone])
+    assert torch.equal(cache._store_v[0][:, :, :N].cpu(), vt[:, :, zone])
+    counts = oracle.cluster_counts(cb[..., zone].contiguous()) if N else torch.zeros(bs, H, 16, 256, dtype=torch.int32)
+    assert torch.equal(cache.cluster_key_counts_gpu[0].cpu(), counts)
