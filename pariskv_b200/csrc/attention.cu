@@ -5,8 +5,9 @@
 // live in pinned host memory.  The rows are cut into tiles of 64; a block takes one tile, or several consecutive
 // ones that it streams through two staging buffers, and stages a tile with TMA bulk copies (cp.async.bulk, one
 // 512-byte copy per selected key where its K and V rows are adjacent, completion counted on an mbarrier), so a whole
-// grid keeps megabytes outstanding on the host link.  16 groups of 8 lanes then run an online softmax over the staged
-// rows for the query heads that share the KV head (four at a time), and the block writes one partial (m, l, o) record.
+// grid keeps megabytes outstanding on the host link.  An online softmax over the staged rows runs on the tensor
+// cores for up to eight query heads per KV head (on 16 groups of 8 lanes, four heads at a time, for more), and the block
+// writes one partial (m, l, o) record per head.
 // The block that finishes last for a (batch, KV head) merges the partials and writes the output: one launch, no
 // second kernel, no waiting on other blocks.  Scores are kept in the log2 domain.
 #include "common.cuh"
@@ -17,7 +18,10 @@ namespace {
 
 constexpr int ATT_THREADS = 128;
 constexpr int ATT_TILE = 64;
-constexpr int ATT_GQ = 4;       // query heads per pass
+constexpr int ATT_GQ = 4;       // query heads per pass of the scalar form, and per step of the merge
+// Query heads per KV head that the tensor-core form takes in its one pass: the rows 0 .. 7 of its A operand.  Batch 8 of one
+// KV head with eight query heads, 2180 rows each: 45 us a launch with the scalar form (two passes), 20 with this one.
+constexpr int ATT_MQ = 8;
 constexpr int ATT_REC = 132;    // floats per partial: o[128], m, l, pad, pad
 constexpr int ATT_WAIT_LIMIT = 4000000;  // polls of the copy barrier before giving up
 // Elements (bf16) between two staged rows [K 128 | V 128 | pad].  The tensor-core form pads a row by 16 bytes, so that
@@ -87,8 +91,8 @@ __device__ __forceinline__ void mbar_arrive_expect(unsigned mb, unsigned bytes) 
 // loads, the partial record, the fence and the arrival - over its tiles and the grid is a single wave.
 //
 // MMA: the scores and the weighted sum of a tile run on the tensor cores (mma.sync m16n8k16, bf16 in, fp32 out) in the
-// arrangement of a flash-attention step with the query heads of the KV head as the 16 rows of the A operand (at most
-// eight are real): a warp takes 16 rows of the tile, S[head][row] = Q K^T is two n-tiles of eight k-steps, its C
+// arrangement of a flash-attention step with the query heads of the KV head as the 16 rows of the A operand (rows
+// 0 .. 7; rows 8 .. 15 are zero): a warp takes 16 rows of the tile, S[head][row] = Q K^T is two n-tiles of eight k-steps, its C
 // fragments ARE the A fragments of P for O[head][dim] += P V (sixteen n-tiles over the 128 dims), V^T comes from
 // ldmatrix.trans.  The probabilities are rounded to bf16 for the second product, as the reference's attention
 // library does.
@@ -97,10 +101,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   constexpr int RS = AttRow<MMA>::stride;  // elements per staged row
   extern __shared__ __align__(128) unsigned char dyn[];
   uint16_t* KVs = reinterpret_cast<uint16_t*>(dyn);                          // [2 buffers][64][RS]: K row, V row of a key
-  float* obuf = reinterpret_cast<float*>(dyn + 2 * ATT_TILE * RS);           // [16][4][128], over the SECOND buffer:
+  constexpr int PQ = MMA ? ATT_MQ : ATT_GQ;   // query heads of a pass
+  constexpr int PG = MMA ? ATT_THREADS / 32 : 16;   // groups of a block that hold partials of them
+  float* obuf = reinterpret_cast<float*>(dyn + 2 * ATT_TILE * RS);           // [PG][PQ][128], over the SECOND buffer:
                                                                              // used when that buffer is idle
   __shared__ __align__(8) unsigned long long mbar[2];
-  __shared__ float s_m[16][ATT_GQ], s_l[16][ATT_GQ];
+  __shared__ float s_m[PG][PQ], s_l[PG][PQ];
   __shared__ unsigned char s_valid[2][ATT_TILE];
   __shared__ int s_last;
   const int tid = threadIdx.x;
@@ -186,18 +192,20 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
     }
     return dead ? 0 : tile_rows(t_first + j);
   };
-  // Partial record of this block for up to ATT_GQ query heads from the groups' (m, l, o) in shared memory.
-  auto block_partial = [&](int qg, int n_heads, int n_grp) {
+  // Partial record of this block for up to PQ query heads from the groups' (m, l, o) in shared memory.
+  auto block_partial = [&](int qg, int n_heads) {
     for (int g = 0; g < n_heads; g++) {
       float M = -INFINITY;
-      for (int t = 0; t < n_grp; t++) M = fmaxf(M, s_m[t][g]);
+#pragma unroll 4
+      for (int t = 0; t < PG; t++) M = fmaxf(M, s_m[t][g]);
       float L = 0.0f, O = 0.0f;
-      for (int t = 0; t < n_grp; t++) {
+#pragma unroll 4
+      for (int t = 0; t < PG; t++) {
         const float f = (s_m[t][g] == -INFINITY) ? 0.0f : exp2f(s_m[t][g] - M);
         L += s_l[t][g] * f;
-        O += obuf[(t * ATT_GQ + g) * 128 + tid] * f;
+        O += obuf[(t * PQ + g) * 128 + tid] * f;
       }
-      float* rec = p.ws + (((int64_t)b * p.Hq + h * p.G + qg * ATT_GQ + g) * n_groups + blockIdx.x) * ATT_REC;
+      float* rec = p.ws + (((int64_t)b * p.Hq + h * p.G + qg * PQ + g) * n_groups + blockIdx.x) * ATT_REC;
       __stcg(rec + tid, O);
       if (tid == 0) {
         __stcg(rec + 128, M);
@@ -207,7 +215,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   };
 
   if constexpr (MMA) {
-    // ---- tensor-core form: one pass, at most ATT_GQ query heads per KV head ----
+    // ---- tensor-core form: one pass, at most ATT_MQ query heads per KV head ----
     const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const bool head_ok = g < p.G;
     uint32_t qa[8][2];  // A fragments of Q for the eight k-steps: rows g (a0, a2); rows g + 8 are zero (a1, a3)
@@ -300,19 +308,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
     // the four warps are the groups of the block-level merge
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-    if (g < ATT_GQ) {
+    if (head_ok) {
 #pragma unroll
-      for (int n = 0; n < 16; n++) {
-        obuf[(warp * ATT_GQ + g) * 128 + 8 * n + 2 * t] = oacc[n][0];
-        obuf[(warp * ATT_GQ + g) * 128 + 8 * n + 2 * t + 1] = oacc[n][1];
-      }
-      if (t == 0) {
-        s_m[warp][g] = head_ok ? m_run : -INFINITY;
-        s_l[warp][g] = head_ok ? l_run : 0.0f;
-      }
+      for (int n = 0; n < 16; n++)
+        *reinterpret_cast<float2*>(obuf + (warp * PQ + g) * 128 + 8 * n + 2 * t) = make_float2(oacc[n][0], oacc[n][1]);
+      if (t == 0) s_m[warp][g] = m_run, s_l[warp][g] = l_run;
     }
     __syncthreads();
-    block_partial(0, min(ATT_GQ, p.G), ATT_THREADS / 32);
+    block_partial(0, p.G);
   } else {
     const int s = tid & 7, grp = tid >> 3;
     for (int qg = 0; qg < p.n_qgroups; qg++) {  // more than one pass only for more than four query heads per KV head,
@@ -383,14 +386,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
 #pragma unroll
       for (int g = 0; g < ATT_GQ; g++) {
 #pragma unroll
-        for (int jj = 0; jj < 16; jj++) obuf[(grp * ATT_GQ + g) * 128 + 16 * s + jj] = o[g][jj];
+        for (int jj = 0; jj < 16; jj++) obuf[(grp * PQ + g) * 128 + 16 * s + jj] = o[g][jj];
         if (s == 0) {
           s_m[grp][g] = m[g];
           s_l[grp][g] = lsum[g];
         }
       }
       __syncthreads();
-      block_partial(qg, n_heads, 16);
+      block_partial(qg, n_heads);
       __syncthreads();  // obuf / s_m / s_l have been consumed before the next pass writes them
     }
   }
@@ -573,10 +576,11 @@ extern "C" int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* wi
   p.H = (int)H, p.Hq = (int)Hq, p.G = (int)(Hq / H);
   p.n_qgroups = (p.G + ATT_GQ - 1) / ATT_GQ;
   // Blocks per (batch, KV head): all the tiles when the launch is small (every copy of the launch outstanding at once),
-  // otherwise as many as give ONE wave of three blocks per SM, each streaming several tiles.  More than four query
-  // heads per KV head need the staged tile for several passes: one tile per block then.
+  // otherwise as many as give ONE wave of three blocks per SM, each streaming several tiles.  The scalar form needs
+  // the staged tile for several passes: one tile per block then.
   int64_t groups = n_tiles;
-  if (p.n_qgroups == 1) {
+  const bool mma = p.G <= ATT_MQ;   // at most ATT_MQ query heads per KV head: one pass on the tensor cores
+  if (mma) {
     const int64_t fit = (int64_t)sm_count() * 3 / (H * bs);
     groups = fit < 1 ? 1 : (fit < n_tiles ? fit : n_tiles);
   }
@@ -594,8 +598,6 @@ extern "C" int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* wi
     p.lse = (float*)lse->data;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  // at most ATT_GQ query heads per KV head: scores and weighted sum on the tensor cores; more: the scalar form in passes
-  const bool mma = p.G <= ATT_GQ;
   const int smem = 2 * ATT_TILE * (mma ? AttRow<true>::stride : AttRow<false>::stride) * 2;   // two staging buffers
   static PerDevice smem_attr[2];  // the opt-in to more than 48 KB of dynamic shared memory is per kernel and device
   if (const unsigned long long bit = first_on_device(smem_attr[mma])) {

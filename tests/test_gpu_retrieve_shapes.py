@@ -1,0 +1,65 @@
+"""The retrieval chain over the shapes its launch rule tells apart (clusters of 1 .. 16 blocks per head, and the launches
+over all SMs beyond), and attention at the group sizes where its form changes."""
+import pytest
+import torch
+
+from conftest import srht_signs, synth_keys, synth_queries
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+# (batch, heads, keys, candidates, K): one key; fewer keys than a cluster has blocks; odd slices; many heads (one block per
+# head); candidates crowded into one slice; every key a candidate; equal keys only (flat counts and scores); a long zone
+@pytest.mark.parametrize("bs,H,N,C,K,kind", [
+    (1, 1, 1, 1, 1, "plain"), (1, 3, 9, 5, 2, "plain"), (1, 8, 8191, 820, 100, "plain"), (2, 4, 20011, 4003, 2048, "plain"),
+    (5, 8, 3001, 700, 256, "plain"), (20, 8, 1500, 300, 64, "plain"), (1, 2, 30000, 9000, 1000, "crowded"),
+    (1, 2, 5000, 5000, 3000, "plain"), (1, 2, 9000, 4000, 1500, "equal"), (1, 1, 700001, 70001, 2048, "plain")])
+def test_retrieve_matches_oracle(oracle, bs, H, N, C, K, kind):
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(N + bs)
+    keys = synth_keys(g, bs, H, N)
+    if kind == "equal":
+        keys = keys[:, :, :1].expand(bs, H, N, 128).contiguous()
+    q = synth_queries(g, keys, 4)
+    if kind == "crowded":                    # a third of the zone points with the query: most candidates come from there
+        m = q.view(bs, 4 * H, 128).view(bs, H, 4, 128).float().mean(2, keepdim=True)
+        keys[:, :, 3000:13000] = (keys[:, :, 3000:13000].float() * 0.2 + m / m.norm(dim=-1, keepdim=True) * 8.0).to(torch.bfloat16)
+    signs = srht_signs()
+    _, cen = oracle.constants()
+    counts = torch.zeros(bs, H, 16, 256, dtype=torch.int32, device=DEV)
+    cb, w, pk = ops.encode_keys(keys.to(DEV), signs.to(DEV), cluster_counts=counts)
+    cb_o, w_o, pk_o = oracle.encode(keys, signs)
+    assert torch.equal(cb.cpu(), cb_o)
+    ref = oracle.retrieve(q, signs, cb_o, w_o, pk_o, oracle.cluster_counts(cb_o), cen, 0.25, C, K)
+    tiers = oracle.tier_counts(N, 0.25)
+    fin, ex = ops.retrieve(q.to(DEV), signs.to(DEV), cen.to(DEV), cb, w, pk, counts, tiers, C, K, want=("cand", "scores_f32"))
+    assert torch.equal(ex["cand"].cpu(), ref["cand"])
+    assert torch.equal(ex["scores_f32"].cpu(), ref["score32"])
+    assert torch.equal(fin.cpu(), ref["final"])
+    fin2, _ = ops.retrieve(q.to(DEV), signs.to(DEV), cen.to(DEV), cb, w, pk, counts, tiers, C, K)   # nothing but the result
+    assert torch.equal(fin2, fin)
+    _, ex2 = ops.retrieve(q.to(DEV), signs.to(DEV), cen.to(DEV), cb, w, pk, counts, tiers, C, 0, want=("cand", "scores_f32"))
+    assert torch.equal(ex2["cand"].cpu(), ref["cand"]) and torch.equal(ex2["scores_f32"].cpu(), ref["score32"])
+
+
+@pytest.mark.parametrize("group", [5, 8, 9])
+@pytest.mark.parametrize("n_window,K", [(1, 0), (63, 1), (64, 64), (70, 1000)])
+def test_attention_group_sizes(oracle, group, n_window, K):
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(group * 1000 + K)
+    bs, H, N = 2, 3, 1500
+    kv = torch.randn(bs, H, N, 2, 128, generator=g).to(torch.bfloat16)
+    q = (torch.randn(bs, 1, H * group, 128, generator=g) * 3).to(torch.bfloat16)
+    wk = torch.randn(bs, H, 256, 128, generator=g).to(torch.bfloat16)
+    wv = torch.randn(bs, H, 256, 128, generator=g).to(torch.bfloat16)
+    rk, rv, args = [wk[:, :, :n_window]], [wv[:, :, :n_window]], ()
+    if K:
+        sel = torch.stack([torch.stack([torch.randperm(N, generator=g)[:K].sort().values for _ in range(H)]) for _ in range(bs)])
+        dkv = kv.to(DEV)
+        args = (dkv[:, :, :, 0], dkv[:, :, :, 1], sel.to(DEV))
+        rk.append(oracle.gather(kv[:, :, :, 0].contiguous(), sel))
+        rv.append(oracle.gather(kv[:, :, :, 1].contiguous(), sel))
+    out = ops.sparse_attention(q.to(DEV), wk.to(DEV), wv.to(DEV), n_window, *args)
+    ref = oracle.attention(q, torch.cat(rk, 2), torch.cat(rv, 2))
+    assert (out.float().cpu() - ref).abs().max().item() <= 2e-2
