@@ -1,5 +1,5 @@
-// Device pieces of the retrieval chain that its kernels share: register sort of the clusters of a subspace, query
-// rotation over one warp, 4-bit rerank of one candidate, block scan.
+// Device pieces of the retrieval chain that its kernels share: query preparation, ranking of the clusters of a subspace,
+// tier tables and look-ups, the candidate list, the 4-bit rerank.
 #pragma once
 #include "common.cuh"
 #include "kernels.cuh"
@@ -129,6 +129,16 @@ __device__ __forceinline__ unsigned tier_sum16(uint4 cw, const uint8_t* lut, uns
   return acc;
 }
 
+// The tier counts of four codes of ONE subspace, one per byte; lut: its 128 bytes (see tier_sum16).
+__device__ __forceinline__ uint32_t tier_bytes(uint32_t w, const uint8_t* t, unsigned c256) {
+  const uint32_t at = w & 0x7f7f7f7fu;
+  const unsigned b0 = t[byte_of(at, 0)], b1 = t[byte_of(at, 1)], b2 = t[byte_of(at, 2)], b3 = t[byte_of(at, 3)];
+  const uint32_t v = ((b3 * c256 + b2) * c256 + b1) * c256 + b0;
+  uint32_t high;
+  asm("prmt.b32 %0, %1, %2, 0xba98;" : "=r"(high) : "r"(w), "r"(0u));
+  return (((v >> 4) & high) | (v & ~high)) & 0x0f0f0f0fu;
+}
+
 __device__ __forceinline__ void unpack4(uint2 v, float* out) {
   out[0] = __uint_as_float(v.x << 16), out[1] = __uint_as_float(v.x & 0xffff0000u);
   out[2] = __uint_as_float(v.y << 16), out[3] = __uint_as_float(v.y & 0xffff0000u);
@@ -226,13 +236,6 @@ __device__ __forceinline__ int pair_slot(int d) {
   const int sub = d >> 3, j = d & 7;
   return ((sub >> 1) * 4 + (j >> 1)) * 4 + (j & 1) * 2 + (sub & 1);
 }
-__device__ __forceinline__ void load_record(uint4 (&rec)[6], const uint8_t* k4, const uint16_t* w, int64_t key) {
-  const uint4* cp = reinterpret_cast<const uint4*>(k4 + key * 64);
-  const uint4* wp = reinterpret_cast<const uint4*>(w + key * 16);
-#pragma unroll
-  for (int i = 0; i < 4; i++) rec[i] = __ldg(cp + i);
-  rec[4] = __ldg(wp), rec[5] = __ldg(wp + 1);
-}
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -269,28 +272,201 @@ __device__ __forceinline__ float rerank_pairs(const uint4 (&rec)[6], const uint3
   return __fmul_rn(acc, qn);
 }
 
-// Block-wide exclusive scan of a packed pair of counters; returns (exclusive prefix, block total).
-template <int NT>
-__device__ __forceinline__ unsigned long long block_scan_excl(unsigned long long mine, unsigned long long* s_scan,
-                                                              unsigned long long* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long sc = mine;
+// ---- stages that the one-launch chain and its several-launch form share; blocks of CH_THREADS threads ------------------
+constexpr int CH_THREADS = 512;
+constexpr int CH_WARPS = CH_THREADS / 32;
+constexpr int CH_CBINS = 129;                      // counts 0 .. 16 subspaces x 8 tiers
+constexpr int CH_HIST_BYTES = CH_CBINS * 32 * 4;   // count histogram, one replica per lane: a warp's atomics never conflict
+constexpr int CH_REC = 112;                        // bytes between staged records (96 used): quarter-warp reads do not conflict
+constexpr int CH_STAGE = CH_WARPS * 32 * CH_REC;
+
+struct PreparedQuery {
+  float x[4], avg[4], n;   // warp 0: the lane's dimensions of the rotated and of the mean query, the norm
+};
+// Warp 0 averages the group's queries, normalises and rotates the mean into s_q.
+__device__ __forceinline__ void prepare_query(PreparedQuery& pq, const ChainQuery& cq, int b, int h, int G, float inv_g,
+                                              float* s_q, float* s_qnorm) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x >= 32) return;
+  const uint16_t* q = cq.queries + ((int64_t)b * cq.Hq + (int64_t)h * G) * 128 + 4 * lane;
+  float sg[4], acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  unpack4(__ldg(reinterpret_cast<const uint2*>(cq.signs + 4 * lane)), sg);
+  for (int g = 0; g < G; g++) {  // fp32 sum over the group, g ascending
+    float v[4];
+    unpack4(__ldg(reinterpret_cast<const uint2*>(q + g * 128)), v);
+#pragma unroll
+    for (int i = 0; i < 4; i++) acc[i] = __fadd_rn(acc[i], v[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) pq.x[i] = pq.avg[i] = bfround(__fmul_rn(acc[i], inv_g));
+  pq.n = rotate4(pq.x, sg, lane);
+#pragma unroll
+  for (int i = 0; i < 4; i++) s_q[4 * lane + i] = pq.x[i];
+  if (lane == 0) *s_qnorm = pq.n;
+}
+__device__ __forceinline__ void publish_query(const PreparedQuery& pq, const ChainQuery& cq, int64_t bh) {   // warp 0 of one block
+  const int lane = threadIdx.x & 31;
+  auto words = [](const float* v) {
+    return make_uint2((uint32_t)f2bf(v[0]) | ((uint32_t)f2bf(v[1]) << 16), (uint32_t)f2bf(v[2]) | ((uint32_t)f2bf(v[3]) << 16));
+  };
+  if (cq.query_avg) *reinterpret_cast<uint2*>(cq.query_avg + bh * 128 + 4 * lane) = words(pq.avg);
+  if (cq.q_blocks) *reinterpret_cast<uint2*>(cq.q_blocks + bh * 128 + 4 * lane) = words(pq.x);
+  if (cq.q_norm && lane == 0) cq.q_norm[bh] = f2bf(pq.n);
+}
+__device__ __forceinline__ void load_tiers(const ChainQuery& cq, long long N, unsigned* s_tiers) {   // one thread
+  if (cq.n_dev) {
+    unsigned t[8];
+    zone_tiers(cq.sched, N, t);
+    for (int i = 0; i < cq.sched.n_tiers; i++) s_tiers[i] = t[i];
+    s_tiers[8] = (unsigned)cq.sched.n_tiers;
+  } else {
+    for (int i = 0; i < cq.n_tiers; i++) s_tiers[i] = cq.tiers[i];
+    s_tiers[8] = (unsigned)cq.n_tiers;
+  }
+}
+// Tier table of one subspace by its warp.  sizes: 256 words with the cluster sizes (overwritten); key: the order made by
+// rank_subspace; lut: the subspace's 128 bytes (see tier_sum16).
+__device__ __forceinline__ void tier_table(const unsigned (&key)[8], unsigned* sizes, const unsigned* s_tiers, uint8_t* lut) {
+  const int lane = threadIdx.x & 31;
+  const int n_tiers = (int)s_tiers[8];
+  unsigned tier[8], cnt[8], run = 0;
+#pragma unroll
+  for (int t = 0; t < 8; t++) tier[t] = t < n_tiers ? s_tiers[t] : 0u;
+#pragma unroll
+  for (int rr = 0; rr < 8; rr++) {
+    cnt[rr] = sizes[255u - (key[rr] & 255u)];
+    run += cnt[rr];
+  }
+  unsigned incl = run;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const unsigned long long o = __shfl_up_sync(0xffffffffu, sc, off);
-    if (lane >= off) sc += o;
+    const unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += o;
   }
-  if (lane == 31) s_scan[warp] = sc;
-  __syncthreads();
-  unsigned long long before = 0, tot = 0;
+  unsigned excl = incl - run;
+  __syncwarp();   // the sizes have been read: the same words take the tier counts, packed to nibbles below
 #pragma unroll
-  for (int w = 0; w < NT / 32; w++) {
-    const unsigned long long v = s_scan[w];
-    if (w < warp) before += v;
-    tot += v;
+  for (int rr = 0; rr < 8; rr++) {
+    unsigned wgt = 0;
+#pragma unroll
+    for (int t = 0; t < 8; t++) wgt += (excl < tier[t]) ? 1u : 0u;   // absent tiers are 0: never above a prefix sum
+    sizes[255u - (key[rr] & 255u)] = wgt;
+    excl += cnt[rr];
   }
-  *total = tot;
-  return before + sc - mine;
+  __syncwarp();
+  // entries i (low nibble) and i + 128 of byte i: four bytes per lane
+  const uint4 e0 = *reinterpret_cast<const uint4*>(sizes + lane * 4), e1 = *reinterpret_cast<const uint4*>(sizes + 128 + lane * 4);
+  *reinterpret_cast<uint32_t*>(lut + lane * 4) =
+      (e0.x | (e1.x << 4)) | ((e0.y | (e1.y << 4)) << 8) | ((e0.z | (e1.z << 4)) << 16) | ((e0.w | (e1.w << 4)) << 24);
+}
+
+// Ordered candidate list of a block's n_keys counts (cnt8, overwritten; the first `skip` < 16 are not keys): those above T, and ties at T while the zone-wide
+// quota lasts, of which lower blocks have met eq_base.  put(position, offset of the key) for positions below `limit`;
+// returns the length of the list.  warp_a / warp_b: CH_WARPS words of scratch.
+template <class Put>
+__device__ __forceinline__ int list_candidates(uint8_t* cnt8, int n_keys, int skip, unsigned T, unsigned quota,
+                                               unsigned eq_base, int64_t limit, unsigned* warp_a, unsigned* warp_b, Put put) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wspan = ((n_keys + CH_WARPS - 1) / CH_WARPS + 15) / 16 * 16;
+  const int k0 = min(n_keys, warp * wspan), k1 = min(n_keys, k0 + wspan);
+  const uint32_t add_gt = (127u - T) * 0x01010101u;           // T <= 128, counts <= 128: no carry between bytes
+  const uint32_t add_ge = T ? (128u - T) * 0x01010101u : 0u;
+  unsigned n_gt = 0, n_eq = 0;
+#pragma unroll 1
+  for (int k = k0 + 16 * lane; k < k1; k += 512) {   // 16 keys -> masks of counts above / at the threshold, kept in their place
+    unsigned gt = 0, eq = 0;
+    const uint4 v = *reinterpret_cast<const uint4*>(cnt8 + k);
+    const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint32_t g = T < 128u ? (w4[i] + add_gt) & 0x80808080u : 0u;
+      const uint32_t ge = T ? (w4[i] + add_ge) & 0x80808080u : 0x80808080u;
+      gt |= ((((g >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * i);
+      eq |= (((((ge & ~g) >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * i);
+    }
+    if (k1 - k < 16) gt &= (1u << (k1 - k)) - 1u, eq &= (1u << (k1 - k)) - 1u;
+    if (k < skip) gt &= ~0u << skip, eq &= ~0u << skip;
+    *reinterpret_cast<unsigned*>(cnt8 + k) = gt | (eq << 16);
+    n_gt += __popc(gt), n_eq += __popc(eq);
+  }
+  n_gt = __reduce_add_sync(0xffffffffu, n_gt), n_eq = __reduce_add_sync(0xffffffffu, n_eq);
+  if (lane == 0) warp_a[warp] = n_gt, warp_b[warp] = n_eq;
+  __syncthreads();
+  unsigned g = 0, e = eq_base, g_all = 0, e_all = eq_base;
+#pragma unroll
+  for (int w = 0; w < CH_WARPS; w++) {
+    const unsigned a = warp_a[w], c = warp_b[w];
+    if (w < warp) g += a, e += c;
+    g_all += a, e_all += c;
+  }
+  const unsigned eq_before = min(eq_base, quota);
+  int n_list = (int)(g_all + min(e_all, quota) - eq_before);
+  n_list = (int)max((int64_t)0, min((int64_t)n_list, limit));   // a no-op with consistent histograms
+#pragma unroll 1
+  for (int k = k0; k < k1; k += 512) {
+    const unsigned m = k + 16 * lane < k1 ? *reinterpret_cast<const unsigned*>(cnt8 + k + 16 * lane) : 0u;
+    const unsigned gt = m & 0xffffu, eq = m >> 16;
+    const unsigned mine = ((unsigned)__popc(gt) << 16) | (unsigned)__popc(eq);
+    unsigned inc = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned o = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += o;
+    }
+    const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
+    const unsigned eg = g + ((inc - mine) >> 16), ee = e + ((inc - mine) & 0xffffu);
+    const int room = (int)quota - (int)ee;   // ties this lane may still take
+    unsigned take = eq;
+    if (room < (int)__popc(eq))
+      for (int drop = (int)__popc(eq) - max(room, 0); drop > 0; drop--) take &= ~(1u << (31 - __clz(take)));
+    take |= gt;
+    int pos = (int)(eg + min(ee, quota) - eq_before);
+    while (take) {
+      const int j = __ffs(take) - 1;
+      take &= take - 1;
+      if (pos < n_list) put(pos, k + 16 * lane + j);
+      pos++;
+    }
+    g += total >> 16, e += total & 0xffffu;
+  }
+  return n_list;
+}
+
+// 4-bit rerank of a list by one block, from key-major records: key_at(i) -> sink(i, key, score).
+// A warp takes 32 consecutive candidates per round: it loads their records with whole sectors per request (four lanes
+// on the 64 bytes of codes, two on the 32 bytes of weights), turns them over its staging buffer (32 * CH_REC bytes) to one
+// record per lane, and has the loads of the next round in flight during the arithmetic.
+template <class KeyAt, class Sink>
+__device__ __forceinline__ void rerank_list(int n_list, const uint8_t* k4, const uint16_t* w, uint8_t* stage, const uint32_t* lev2,
+                                            const float4* q2, float qn, unsigned c128, unsigned c64k, KeyAt key_at, Sink sink) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int ROUND = CH_WARPS * 32;
+  uint4 in[6];
+  auto fetch = [&](int base) {   // out of range: the list's last candidate again
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      in[i] = __ldg(reinterpret_cast<const uint4*>(k4 + (int64_t)key_at(min(base + 8 * i + (lane >> 2), n_list - 1)) * 64) + (lane & 3));
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      in[4 + i] = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)key_at(min(base + 16 * i + (lane >> 1), n_list - 1)) * 16) + (lane & 1));
+  };
+  if (warp * 32 < n_list) fetch(warp * 32);
+#pragma unroll 1
+  for (int base = warp * 32; base < n_list; base += ROUND) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; i++) *reinterpret_cast<uint4*>(stage + (8 * i + (lane >> 2)) * CH_REC + (lane & 3) * 16) = in[i];
+#pragma unroll
+    for (int i = 0; i < 2; i++) *reinterpret_cast<uint4*>(stage + (16 * i + (lane >> 1)) * CH_REC + 64 + (lane & 1) * 16) = in[4 + i];
+    __syncwarp();
+    if (base + ROUND < n_list) fetch(base + ROUND);
+    uint4 rec[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) rec[i] = *reinterpret_cast<const uint4*>(stage + lane * CH_REC + i * 16);
+    const float v = rerank_pairs(rec, lev2, q2, qn, lane, c128, c64k);
+    const int i = base + lane;
+    if (i < n_list) sink(i, key_at(i), v);
+  }
 }
 
 }  // namespace

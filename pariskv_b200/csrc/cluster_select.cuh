@@ -26,11 +26,13 @@ constexpr int SEL_TIES = 1024;
 constexpr int SEL_REGION = 2 * SEL_TIES * 8;   // bytes of dynamic shared memory, at the same offset in every CTA
 
 struct F32Row {
+  static constexpr bool whole = false;
   static __device__ __forceinline__ float val(uint32_t u) { return __uint_as_float(u); }
   static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key(__uint_as_float(u)); }
   static __device__ __forceinline__ float from_key(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k); }
 };
 struct I32Row {
+  static constexpr bool whole = true;
   static __device__ __forceinline__ float val(uint32_t u) { return (float)(int32_t)u; }
   static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key((int32_t)u); }
   static __device__ __forceinline__ float from_key(uint32_t k) { return (float)(int32_t)(k ^ 0x80000000u); }
@@ -172,27 +174,24 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     rem -= s.res[1], in_bin = s.res[2], pre_above += s.res[3], pre_in = s.res[4];
     buf ^= 1;
   }
-  const bool flat = in_bin > (unsigned)SEL_TIES;   // that many equal keys: the lowest positions win, rank by rank
   const bool level0 = lo == 0u && hi == 0xffffffffu;
+  // the threshold bin holds equal keys only: the lowest positions win, rank by rank (whole numbers in a small range have a
+  // bin each)
+  const bool flat = in_bin > (unsigned)SEL_TIES || (level0 && V::whole && s.range[1] - s.range[0] < (unsigned)SEL_BINS);
 
-  // ---- where every element stands: above the threshold bin, in it, below; ballots of 32 consecutive elements ----
-  const int wn = ((n + SEL_WARPS - 1) / SEL_WARPS + 31) / 32 * 32;   // a warp owns consecutive elements
-  const int i0 = min(n, warp * wn), i1 = min(n, i0 + wn);
-  auto standing = [&](int i, bool& above, bool& member) {
-    above = member = false;
-    if (i < i1) {
-      const uint32_t u = at(i);
-      const unsigned bn = bin0(u);
-      above = bn > T0, member = bn == T0;
-      if (!level0 && member) {
-        const unsigned k = V::key(u);
-        above = k > hi, member = k >= lo && k <= hi;
-      }
+  // ---- where every element stands: above the threshold bin, in it, below; one bit per element ----
+  auto standing = [&](uint32_t u, bool& above, bool& member) {
+    const unsigned bn = bin0(u);
+    above = bn > T0, member = bn == T0;
+    if (!level0 && member) {
+      const unsigned k = V::key(u);
+      above = k > hi, member = k >= lo && k <= hi;
     }
   };
   uint2* own = reinterpret_cast<uint2*>(region);   // this CTA's members: (key, rank and position)
   uint2* all = own + SEL_TIES;                     // everybody's, in rank order
-  const bool kept = (n + 31) / 32 <= words_cap;
+  const int n_words = (n + 31) / 32;
+  const bool kept = n_words <= words_cap;          // otherwise the words are made window by window, after the threshold
   unsigned* above_w = words;
   unsigned* member_w = words + words_cap;
   __syncthreads();   // the histogram replicas under `own` have been read
@@ -200,17 +199,19 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   if (tid < SEL_SUB) s.sub[tid] = 0;
   __syncthreads();
   if (kept || !flat) {
-#pragma unroll 1
-    for (int i = i0; i < i1; i += 32) {
-      bool above, member;
-      standing(i + lane, above, member);
+#pragma unroll 2
+    for (int w = warp; w < n_words; w += SEL_WARPS) {   // a warp takes every 16th group of 32 elements
+      const int i = w * 32 + lane;
+      bool above = false, member = false;
+      const uint32_t u = at(min(i, n - 1));
+      if (i < n) standing(u, above, member);
       const unsigned aw = __ballot_sync(0xffffffffu, above), mw = __ballot_sync(0xffffffffu, member);
-      if (kept && lane == 0) above_w[i >> 5] = aw, member_w[i >> 5] = mw;
+      if (kept && lane == 0) above_w[w] = aw, member_w[w] = flat ? mw : 0u;
       if (!flat && mw) {
         unsigned slot = 0;
         if (lane == 0) slot = atomicAdd(&s.n_members, (unsigned)__popc(mw));
         slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(mw & ((1u << lane) - 1u));
-        if (member && slot < (unsigned)SEL_TIES) own[slot] = make_uint2(V::key(at(i + lane)), (rank << 27) | (unsigned)(i + lane));
+        if (member && slot < (unsigned)SEL_TIES) own[slot] = make_uint2(V::key(u), (rank << 27) | (unsigned)i);
       }
     }
   }
@@ -279,61 +280,90 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     __syncthreads();
     const unsigned n_few = s.n_few;
 #pragma unroll 1
-    for (unsigned t = tid; t < n_few; t += SEL_THREADS) {
+    for (unsigned t = warp; t < n_few; t += SEL_WARPS) {   // a warp ranks an element
       const uint2 me = few[t];
       const unsigned pos = me.y & 0x7fffffffu;
       unsigned rk = 0;
-      for (unsigned j = 0; j < n_few; j++) {
+      for (unsigned j = lane; j < n_few; j += 32) {
         const uint2 o = few[j];
         rk += (o.x > me.x || (o.x == me.x && (o.y & 0x7fffffffu) < pos)) ? 1u : 0u;
       }
-      if (rk < need && (me.y >> 31)) atomicAdd(&s.lower_sel, 1u);
-      if (rk + 1 == need) s.thr_key = me.x, s.thr_pos = pos;
+      rk = __reduce_add_sync(0xffffffffu, rk);
+      if (lane == 0) {
+        if (rk < need && (me.y >> 31)) atomicAdd(&s.lower_sel, 1u);
+        if (rk + 1 == need) s.thr_key = me.x, s.thr_pos = pos;
+      }
     }
     __syncthreads();
     thr_key = s.thr_key, thr_pos = s.thr_pos, lower_sel = s.lower_sel;
   }
   if (CS > 1) cluster.barrier_arrive();   // this CTA reads no other CTA's memory from here on
 
-  // ---- ordered emission ----
-  const unsigned room = flat && rem > lower_sel ? rem - lower_sel : 0u;   // flat bin: members this CTA may still take
-  auto words_of = [&](int i, unsigned& aw, unsigned& mw) {
-    if (kept) {
-      aw = above_w[i >> 5], mw = member_w[i >> 5];
-    } else {
-      bool above, member;
-      standing(i + lane, above, member);
-      aw = __ballot_sync(0xffffffffu, above), mw = __ballot_sync(0xffffffffu, member);
+  // ---- ordered emission: a lane owns a word of 32 elements ----
+  auto taken = [&](unsigned k, unsigned pos) -> bool { return k > thr_key || (k == thr_key && pos <= thr_pos); };
+  if (kept && !flat) {   // members that are taken join the elements above
+    const unsigned m = min(s.n_members, (unsigned)SEL_TIES);
+    for (unsigned t = tid; t < m; t += SEL_THREADS) {
+      const uint2 me = own[t];
+      const unsigned i = me.y & 0x07ffffffu;
+      if (taken(me.x, me.y)) atomicOr(&above_w[i >> 5], 1u << (i & 31));
     }
-    if (!flat && mw) {   // resolve the members
-      const unsigned k = ((mw >> lane) & 1u) ? V::key(at(i + lane)) : 0u;
-      const bool t = ((mw >> lane) & 1u) && (k > thr_key || (k == thr_key && ((rank << 27) | (unsigned)(i + lane)) <= thr_pos));
-      aw |= __ballot_sync(0xffffffffu, t);
-    }
-  };
-  unsigned n_take = 0, n_mem = 0;
-#pragma unroll 1
-  for (int i = i0; i < i1; i += 32) {
-    unsigned aw, mw;
-    words_of(i, aw, mw);
-    n_take += __popc(aw);
-    if (flat) n_mem += __popc(mw);
   }
-  if (lane == 0) s.warp_a[warp] = n_take, s.warp_b[warp] = n_mem;
-  __syncthreads();
-  unsigned g = pre_above + lower_sel, e = 0;
-  for (int w = 0; w < warp; w++) g += s.warp_a[w], e += s.warp_b[w];
-  const unsigned lt = (1u << lane) - 1u;
-#pragma unroll 1
-  for (int i = i0; i < i1; i += 32) {
-    unsigned aw, mw;
-    words_of(i, aw, mw);
-    if (!flat) mw = 0;
-    const unsigned eb = e + __popc(mw & lt);
-    const unsigned pos = g + __popc(aw & lt) + min(eb, room);
-    const bool t = ((aw >> lane) & 1u) || (((mw >> lane) & 1u) && eb < room);
-    if (t && pos < (unsigned)K) out[pos] = out_of(i + lane);
-    g += __popc(aw), e += __popc(mw);
+  const unsigned room = flat && rem > lower_sel ? rem - lower_sel : 0u;   // flat bin: members this CTA may still take
+  unsigned g = pre_above + lower_sel, e = 0;   // entries of the final list, and members, before the window
+  for (int w0 = 0; w0 < n_words; w0 += words_cap) {
+    const int nw = min(n_words - w0, words_cap);
+    if (!kept) {
+      __syncthreads();   // the words of the window before have been read
+      for (int w = warp; w < nw; w += SEL_WARPS) {
+        const int i = (w0 + w) * 32 + lane;
+        bool above = false, member = false;
+        const uint32_t u = at(min(i, n - 1));
+        if (i < n) standing(u, above, member);
+        above = above || (!flat && member && taken(V::key(u), (rank << 27) | (unsigned)i));
+        const unsigned aw = __ballot_sync(0xffffffffu, above), mw = __ballot_sync(0xffffffffu, member);
+        if (lane == 0) above_w[w] = aw, member_w[w] = flat ? mw : 0u;
+      }
+    }
+    __syncthreads();
+    const int per = (nw + SEL_WARPS - 1) / SEL_WARPS;   // a warp's consecutive words
+    const int a0 = min(nw, warp * per), a1 = min(nw, a0 + per);
+    unsigned na = 0, nm = 0;
+    for (int w = a0 + lane; w < a1; w += 32) na += __popc(above_w[w]), nm += __popc(member_w[w]);
+    na = __reduce_add_sync(0xffffffffu, na), nm = __reduce_add_sync(0xffffffffu, nm);
+    if (lane == 0) s.warp_a[warp] = na, s.warp_b[warp] = nm;
+    __syncthreads();
+    unsigned gw = g, ew = e;
+    for (int w = 0; w < SEL_WARPS; w++) {
+      const unsigned x = s.warp_a[w], y = s.warp_b[w];
+      if (w < warp) gw += x, ew += y;
+      g += x, e += y;
+    }
+    for (int wb = a0; wb < a1; wb += 32) {
+      const int w = wb + lane;
+      unsigned aw = w < a1 ? above_w[w] : 0u, mw = w < a1 ? member_w[w] : 0u;
+      const unsigned long long mine = ((unsigned long long)__popc(aw) << 32) | (unsigned)__popc(mw);
+      unsigned long long inc = mine;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += o;
+      }
+      const unsigned long long total = __shfl_sync(0xffffffffu, inc, 31);
+      unsigned eb = ew + (unsigned)(inc - mine);
+      unsigned pos = gw + (unsigned)((inc - mine) >> 32) + min(eb, room);
+      if (eb >= room) mw = 0;
+      for (unsigned bits = aw | mw; bits; bits &= bits - 1) {
+        const int j = __ffs(bits) - 1;
+        if ((mw >> j) & 1u) {
+          if (eb >= room) continue;
+          eb++;
+        }
+        if (pos < (unsigned)K) out[pos] = out_of((w0 + w) * 32 + j);
+        pos++;
+      }
+      gw += (unsigned)(total >> 32), ew += (unsigned)total;
+    }
   }
 }
 

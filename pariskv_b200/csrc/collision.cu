@@ -173,39 +173,37 @@ __global__ void __launch_bounds__(256) rank_kernel(RankParams p) {
 struct CollParams {
   const uint8_t* codes;          // element (b,h,s,k) at codes[b*c_b + h*c_h + s*c_s + k*c_l]
   int64_t c_b, c_h, c_s, c_l;
-  const uint32_t* lut;           // [bs*H][B][64] words = 256 byte entries per subspace (FUSED == false)
-  int32_t* out_i32;              // [bs*H][N]            (OUT_U8 == false)
-  uint8_t* out_u8;               // [bs*H][u8_stride], indexed by virtual key (OUT_U8 == true)
-  uint32_t* chunk_hist;          // [bs*H][n_chunks][256] (OUT_U8 == true)
+  const uint32_t* lut;           // [bs*H][B][64] words = 256 byte entries per subspace (stand-alone op)
+  int32_t* out_i32;              // [bs*H][N]            (stand-alone op)
+  uint8_t* out_u8;               // [bs*H][u8_stride], indexed by virtual key (chain kernel)
+  uint32_t* chunk_hist;          // [bs*H][n_chunks][256] (chain kernel)
   int64_t u8_stride;
   int H, B;
   int64_t N;                     // keys per head
   int mis;                       // virtual key v = key + mis; loads are 16-byte aligned in v
   int64_t chunk_keys;            // virtual keys per block
   int64_t n_hist;                // histogram rows per (batch, head) of chunk_hist (chain kernel)
-  ChainQuery q;                  // FUSED == true: the table is built in the block from the query
+  ChainQuery q;                  // chain kernel: the table is built in the block from the query
   int G;
   float inv_g;
+  unsigned c256;                 // 256 (see tier_sum16)
 };
 
 // The stand-alone op (tier table from global memory, int32 counts out), 256 threads.
 // LAYOUT 0: plane-major ([.., 16, N], key stride 1): a thread owns 16 consecutive keys.
 // LAYOUT 1: key-major ([.., N, 16], subspace stride 1): a warp owns 512 consecutive keys, lane-strided.
 // LAYOUT 2: any strides, any B <= 32: a thread owns one key at a time.
-template <int LAYOUT, bool OUT_U8>
+template <int LAYOUT>
 __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
   __shared__ __align__(16) uint8_t s_lut[32 * 256];
-  __shared__ __align__(16) unsigned hist[8 * 256];  // eight replicas (lane & 7) cut same-bin collisions inside a warp
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
-  unsigned* my_hist = hist + ((lane & 7) << 8);
   const int64_t N = p.N;
   const int64_t Nv = N + p.mis;
   const int64_t v_begin = (int64_t)blockIdx.x * p.chunk_keys;
   const int64_t v_end = min(Nv, v_begin + p.chunk_keys);
   const uint8_t* base = p.codes + b * p.c_b + h * p.c_h - p.mis * p.c_l;
-  int32_t* out32 = OUT_U8 ? nullptr : p.out_i32 + (int64_t)bh * p.N;
-  uint8_t* out8 = OUT_U8 ? p.out_u8 + (int64_t)bh * p.u8_stride : nullptr;
+  int32_t* out32 = p.out_i32 + (int64_t)bh * p.N;
 
   // the first batch of code loads is issued before the table is staged, so both latencies overlap
   uint4 r[16];
@@ -222,8 +220,6 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
     for (int s = 0; s < 16; s++)
       r[s] = (v0 < v_end) ? __ldg(reinterpret_cast<const uint4*>(base + s * p.c_s + v0)) : make_uint4(0, 0, 0, 0);
   }
-  if (OUT_U8)
-    for (int i = tid; i < 8 * 256; i += 256) hist[i] = 0;
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.lut + (int64_t)bh * p.B * 64);
     uint4* dst = reinterpret_cast<uint4*>(s_lut);
@@ -250,15 +246,7 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
         for (int s = 0; s < 16; s++) r[s] = __ldg(reinterpret_cast<const uint4*>(base + s * p.c_s + vn));
       }
       const int64_t key0 = v0 - p.mis;
-      if (OUT_U8) {
-        uint32_t pk4[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-          pk4[k >> 2] |= (uint32_t)cnt[k] << (8 * (k & 3));
-          if (live && key0 + k >= 0 && key0 + k < N) atomicAdd(&my_hist[cnt[k]], 1u);
-        }
-        if (live) *reinterpret_cast<uint4*>(out8 + v0) = make_uint4(pk4[0], pk4[1], pk4[2], pk4[3]);
-      } else if (live) {
+      if (live) {
         if (key0 >= 0 && key0 + 16 <= N && ((reinterpret_cast<uintptr_t>(out32 + key0) & 15) == 0)) {
 #pragma unroll
           for (int q = 0; q < 4; q++)
@@ -294,12 +282,7 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
       for (int j = 0; j < 16; j++) {
         const int64_t v = w0 + 32 * j + lane;
         if (v < v_end) {
-          if (OUT_U8) {
-            out8[v] = (uint8_t)cnt[j];
-            atomicAdd(&my_hist[cnt[j]], 1u);
-          } else {
-            out32[v] = cnt[j];
-          }
+          out32[v] = cnt[j];
         }
       }
     }
@@ -309,272 +292,131 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
       if (key < 0) continue;
       int cnt = 0;
       for (int s = 0; s < p.B; s++) cnt += s_lut[s * 256 + base[s * p.c_s + v * p.c_l]];
-      if (OUT_U8) {
-        out8[v] = (uint8_t)cnt;
-        atomicAdd(&my_hist[cnt], 1u);
-      } else {
-        out32[key] = cnt;
-      }
+      out32[key] = cnt;
     }
-  }
-  if (OUT_U8) {
-    __syncthreads();
-    unsigned t = 0;
-#pragma unroll
-    for (int r = 0; r < 8; r++) t += hist[r * 256 + tid];
-    p.chunk_hist[((int64_t)bh * gridDim.x + blockIdx.x) * 256 + tid] = t;
   }
 }
 
-// ---- the collision kernel of the decode chain -------------------------------------------------------------------
-// 512 threads, one block per SM.  While its first code loads are in flight every block builds the tier table itself:
-// warp 0 prepares the query (group mean, normalise, rotate: 4 dimensions per lane, the arithmetic and the fixed
-// operation order of rotate16 / query_prep_kernel), then warp w ranks the 256 clusters of subspace w by (score
-// descending, id ascending) with a register bitonic sort, takes the exclusive prefix sum of the cluster sizes in
-// that order and writes, per cluster, the number of tiers whose threshold the prefix is below.  Output: one u8 count
-// per virtual key and 256-bin histograms of the counts, one per `hist_keys` keys (two per block when the block covers
-// its chunk in one pass), from which the selection kernel derives thresholds and output offsets.
-constexpr int CC_THREADS = 512;
-constexpr int CC_PASS = 8192;  // keys a block covers per pass: 16 warps x 512
-
+// ---- the collision kernel of the chain's several-launch form ---------------------------------------------------------
+// One block per SM.  While its first code loads are in flight every block builds the tier tables itself (query, ranking,
+// prefix sums; chain.cuh), then counts its keys: one u8 per virtual key and one histogram row per block, from which
+// the selection kernel derives thresholds and output offsets.
+// What bounds it: 7 us of prologue, then the half-rate integer ALU, 28 cycles per 32 keys and SM.  8 heads x 1M keys on B200:
+// 64 us with byte tables (bank conflicts), COLL_NOW now; the codes alone take 20 at the copy rate.
+// LAYOUT 1: key-major records; 0: plane-major ([.., 16, N], a thread owns 16 consecutive keys); 2: any strides.
 template <int LAYOUT>
-__global__ void __launch_bounds__(CC_THREADS, 1) chain_collision_kernel(CollParams p) {
-  __shared__ __align__(16) uint8_t s_lut[16 * 256];
-  // prologue: cluster sizes, 256 words per warp; afterwards: two histograms (one per half of a single-pass chunk) of
-  // eight replicas each (lane & 7 picks the replica, which cuts same-bin collisions inside a warp)
-  __shared__ __align__(16) unsigned hist[16 * 256];
-  __shared__ float s_q[128];
+__global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
+  __shared__ __align__(16) uint8_t s_lut[16 * 128];
+  __shared__ __align__(16) unsigned region[CH_HIST_BYTES / 4];   // cluster sizes, then the count histogram
+  __shared__ __align__(16) float s_q[128];
+  __shared__ float s_qnorm;
   __shared__ unsigned s_tiers[9];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
   const ChainQuery& cq = p.q;
-  // ---- query part of the prologue: warp 0 averages, normalises and rotates the query; then every warp scores the 256
-  // clusters of its subspace and sorts them (registers only).  It reads nothing but the queries and the signs, so where
-  // the caller vouches that those were complete before the PREVIOUS kernel on the stream started (cq.early_query: e.g.
-  // the append launch sits in between), it runs before the wait for that kernel, under its tail.
-  float qx[4] = {0.0f, 0.0f, 0.0f, 0.0f}, qavg[4] = {0.0f, 0.0f, 0.0f, 0.0f}, qn = 0.0f;
+  PreparedQuery pq;
   unsigned key[8];
-  auto prepare_query = [&]() {
-    if (warp == 0) {
-      const uint16_t* q = cq.queries + ((int64_t)b * cq.Hq + (int64_t)h * p.G) * 128 + 4 * lane;
-      float sg[4], acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      unpack4(__ldg(reinterpret_cast<const uint2*>(cq.signs + 4 * lane)), sg);
-      for (int g = 0; g < p.G; g++) {  // fp32 sum over the group, g ascending
-        float v[4];
-        unpack4(__ldg(reinterpret_cast<const uint2*>(q + g * 128)), v);
-#pragma unroll
-        for (int i = 0; i < 4; i++) acc[i] = __fadd_rn(acc[i], v[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; i++) qx[i] = qavg[i] = bfround(__fmul_rn(acc[i], p.inv_g));
-      qn = rotate4(qx, sg, lane);
-#pragma unroll
-      for (int i = 0; i < 4; i++) s_q[4 * lane + i] = qx[i];
-    }
-  };
-  auto rank_clusters = [&]() { rank_subspace(key, s_q + warp * 8, lane); };   // after a barrier behind prepare_query()
   const bool early = cq.early_query != 0;
-  if (early) {
-    prepare_query();
+  if (early) {   // the queries were complete before the kernel before this one started
+    prepare_query(pq, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     __syncthreads();
-    rank_clusters();
+    rank_subspace(key, s_q + warp * 8, lane);
   }
   if (cq.n_dev) pdl_wait();  // the zone length may have been written by the kernel just before this one
   const int64_t N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
   const int64_t Nv = N + p.mis;
   const int64_t v_begin = (int64_t)blockIdx.x * p.chunk_keys;
-  // every block clears its slice of the next kernel's value histogram, also a block beyond a short zone; a write, so
-  // it comes after the wait for the kernels before this one
-  auto clear_slice = [&]() {
-    if (!cq.zero_area) return;
-    const int per = (cq.zero_area_words + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int lo = (int)blockIdx.x * per, hi = min(cq.zero_area_words, lo + per);
-    for (int i = lo + tid; i < hi; i += CC_THREADS) cq.zero_area[(int64_t)bh * cq.zero_area_words + i] = 0u;
-  };
-  if (v_begin >= Nv) {  // beyond this sample's zone (whole block, before any barrier)
+  if (v_begin >= Nv) {  // beyond this sample's zone (whole block, before any barrier but the early one)
     pdl_wait();
     pdl_trigger();
-    clear_slice();
     return;
   }
-  const int64_t v_end = min(Nv, v_begin + p.chunk_keys);
-  const uint8_t* base = p.codes + b * p.c_b + h * p.c_h - p.mis * p.c_l;
-  uint8_t* out8 = p.out_u8 + (int64_t)bh * p.u8_stride;
-  const int pass_keys = (int)min(p.chunk_keys, (int64_t)CC_PASS);
-  const int tile = pass_keys >> 4;  // keys per warp and pass (LAYOUT 1), a multiple of 32
-  const int kpl = tile >> 5;        // keys per lane and pass, 1..16
-  const bool publish = blockIdx.x == 0;
-
-  // the first batch of code loads is issued before anything else, so their latency overlaps the prologue
-  uint4 r[16];
+  const int n_keys = (int)(min(Nv, v_begin + p.chunk_keys) - v_begin);   // virtual keys of this block
+  const uint8_t* base = p.codes + b * p.c_b + h * p.c_h + (v_begin - p.mis) * p.c_l;
+  uint8_t* out8 = p.out_u8 + (int64_t)bh * p.u8_stride + v_begin;
+  // the first code loads are issued before the tables are built
+  constexpr int STEP = CH_WARPS * 128;   // LAYOUT 1: a warp takes 128 consecutive keys (four per lane) of every STEP
+  uint4 r0[4], r1[4];
+  auto load_codes = [&](uint4 (&r)[4], int v0) {
+#pragma unroll
+    for (int j = 0; j < 4; j++)   // past the end: the last key again, its count unused
+      r[j] = __ldg(reinterpret_cast<const uint4*>(base) + min(v0 + 32 * j, n_keys - 1));
+  };
   if (LAYOUT == 1) {
-    const int64_t w0 = v_begin + (int64_t)tile * warp;
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-      const int64_t v = w0 + 32 * j + lane;
-      r[j] = (j < kpl && v < v_end) ? __ldg(reinterpret_cast<const uint4*>(base + v * 16)) : make_uint4(0, 0, 0, 0);
-    }
-  } else if (LAYOUT == 0) {
-    const int64_t v0 = v_begin + 16 * (int64_t)tid;
-#pragma unroll
-    for (int s = 0; s < 16; s++)
-      r[s] = (16 * tid < pass_keys && v0 < v_end) ? __ldg(reinterpret_cast<const uint4*>(base + s * p.c_s + v0))
-                                                   : make_uint4(0, 0, 0, 0);
+    load_codes(r0, warp * 128 + lane);
+    load_codes(r1, warp * 128 + lane + STEP);
   }
-  pdl_wait();     // the code loads above do not depend on the kernel before this one; the query below does
+  pdl_wait();
   pdl_trigger();
-  clear_slice();
-
-  // ---- prologue: query, cluster ranking, tier table ----
   {
-    const int sub = warp;
-    unsigned* my = hist + warp * 256;
-    // cluster sizes of this warp's subspace: 8 consecutive clusters per lane
-    const int4* cp = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + sub) * 256 + lane * 8);
-    const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1);
-    if (!early) prepare_query();
-    if (warp == 0 && publish) {
-      if (cq.query_avg)
-        *reinterpret_cast<uint2*>(cq.query_avg + (int64_t)bh * 128 + 4 * lane) =
-            make_uint2((uint32_t)f2bf(qavg[0]) | ((uint32_t)f2bf(qavg[1]) << 16),
-                       (uint32_t)f2bf(qavg[2]) | ((uint32_t)f2bf(qavg[3]) << 16));
-      *reinterpret_cast<uint2*>(cq.q_blocks + (int64_t)bh * 128 + 4 * lane) =
-          make_uint2((uint32_t)f2bf(qx[0]) | ((uint32_t)f2bf(qx[1]) << 16), (uint32_t)f2bf(qx[2]) | ((uint32_t)f2bf(qx[3]) << 16));
-      if (lane == 0) cq.q_norm[bh] = f2bf(qn);
-    }
-    if (tid == 32) {  // thresholds of this sample
-      if (cq.n_dev || cq.n_plan > 0) {
-        unsigned t[8];
-        zone_tiers(cq.sched, cq.n_dev ? (long long)N : cq.n_plan, t);
-        for (int i = 0; i < cq.sched.n_tiers; i++) s_tiers[i] = t[i];
-        s_tiers[8] = (unsigned)cq.sched.n_tiers;
-      } else {
-        for (int i = 0; i < cq.n_tiers; i++) s_tiers[i] = cq.tiers[i];
-        s_tiers[8] = (unsigned)cq.n_tiers;
-      }
-      if (publish && cq.zero_words) cq.zero_words[bh] = 0u;
-    }
+    const int4* cp = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
+    const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1);   // cluster sizes of this warp's subspace
+    unsigned* my = region + warp * 256;
+    if (!early) prepare_query(pq, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
+    if (warp == 0 && blockIdx.x == 0) publish_query(pq, cq, bh);
+    if (tid == 32) load_tiers(cq, cq.n_dev || cq.n_plan <= 0 ? (long long)N : cq.n_plan, s_tiers);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
     *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
     __syncthreads();
-    if (!early) rank_clusters();
-    const int n_tiers = (int)s_tiers[8];
-    unsigned tier[8];
-#pragma unroll
-    for (int t = 0; t < 8; t++) tier[t] = t < n_tiers ? s_tiers[t] : 0u;
-    unsigned cnt[8], run = 0;
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) {
-      cnt[rr] = my[255u - (key[rr] & 255u)];
-      run += cnt[rr];
-    }
-    unsigned incl = run;  // inclusive prefix over lanes
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += o;
-    }
-    unsigned excl = incl - run;
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) {
-      unsigned wgt = 0;
-#pragma unroll
-      for (int t = 0; t < 8; t++) wgt += (t < n_tiers && excl < tier[t]) ? 1u : 0u;
-      s_lut[sub * 256 + (255u - (key[rr] & 255u))] = (uint8_t)wgt;
-      excl += cnt[rr];
-    }
-    __syncthreads();  // the table is complete and the staging area is free again
-    for (int i = tid; i < 16 * 256; i += CC_THREADS) hist[i] = 0;
+    if (!early) rank_subspace(key, s_q + warp * 8, lane);
+    tier_table(key, my, s_tiers, s_lut + warp * 128);
+    __syncthreads();
+    for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
     __syncthreads();
   }
-
-  // a chunk covered in one pass gets two histograms (its halves), so the selection kernel can run two blocks on it
-  const bool split = p.chunk_keys <= CC_PASS;
-  const int64_t hist_keys = split ? (p.chunk_keys >> 1) : p.chunk_keys;
-  unsigned* hist_rep = hist + ((lane & 7) << 8);
-  if (LAYOUT == 0) {
-    for (int64_t t0 = v_begin; t0 < v_end; t0 += CC_PASS) {  // block-uniform trip count
-      const int64_t v0 = t0 + 16 * (int64_t)tid;
-      const bool live = 16 * tid < pass_keys && v0 < v_end;
-      int cnt[16];
+  if (LAYOUT == 1) {
+    auto count_round = [&](uint4 (&r)[4], int v0) {   // counts four keys and puts the loads of the round after next in their place
+      unsigned c[4];
 #pragma unroll
-      for (int k = 0; k < 16; k++) cnt[k] = 0;
+      for (int j = 0; j < 4; j++) c[j] = tier_sum16(r[j], s_lut, p.c256);
+      load_codes(r, v0 + 2 * STEP);
 #pragma unroll
-      for (int s = 0; s < 16; s++) {
-        const uint32_t w4[4] = {r[s].x, r[s].y, r[s].z, r[s].w};
-#pragma unroll
-        for (int k = 0; k < 16; k++) cnt[k] += s_lut[s * 256 + byte_of(w4[k >> 2], k & 3)];
-      }
-      const int64_t vn = v0 + CC_PASS;
-      if (16 * tid < pass_keys && vn < v_end) {
-#pragma unroll
-        for (int s = 0; s < 16; s++) r[s] = __ldg(reinterpret_cast<const uint4*>(base + s * p.c_s + vn));
-      }
-      if (live) {
-        const int64_t key0 = v0 - p.mis;
-        unsigned* hh = hist_rep + ((split && v0 - v_begin >= hist_keys) ? 8 * 256 : 0);
-        uint32_t pk4[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-          pk4[k >> 2] |= (uint32_t)cnt[k] << (8 * (k & 3));
-          if (key0 + k >= 0 && key0 + k < N) atomicAdd(&hh[cnt[k]], 1u);
+      for (int j = 0; j < 4; j++)
+        if (v0 + 32 * j < n_keys) {
+          out8[v0 + 32 * j] = (uint8_t)(c[j] >> 4);
+          atomicAdd(&region[c[j] * 2 + lane], 1u);   // c is a multiple of 16: word 32 per bin
         }
-        *reinterpret_cast<uint4*>(out8 + v0) = make_uint4(pk4[0], pk4[1], pk4[2], pk4[3]);
-      }
+    };
+#pragma unroll 1
+    for (int v0 = warp * 128 + lane; v0 - lane < n_keys; v0 += 2 * STEP) {
+      count_round(r0, v0);
+      if (v0 - lane + STEP < n_keys) count_round(r1, v0 + STEP);
     }
-  } else if (LAYOUT == 1) {
-    for (int64_t t0 = v_begin; t0 < v_end; t0 += CC_PASS) {
-      const int64_t w0 = t0 + (int64_t)tile * warp;
-      int cnt[16];
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        int c = 0;
-        if (j < kpl) {
-          const uint32_t w4[4] = {r[j].x, r[j].y, r[j].z, r[j].w};
-#pragma unroll
-          for (int s = 0; s < 16; s++) c += s_lut[s * 256 + byte_of(w4[s >> 2], s & 3)];
-        }
-        cnt[j] = c;
+  } else if (LAYOUT == 0) {
+    // 16 consecutive keys of a thread, one 16-byte load per subspace; four counts per word, added as bytes
+#pragma unroll 1
+    for (int v0 = 16 * tid; v0 < n_keys; v0 += 16 * CH_THREADS) {
+      uint32_t acc[4] = {0, 0, 0, 0};
+#pragma unroll 4
+      for (int s = 0; s < 16; s++) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(base + s * p.c_s + v0));
+        acc[0] += tier_bytes(w.x, s_lut + s * 128, p.c256), acc[1] += tier_bytes(w.y, s_lut + s * 128, p.c256);
+        acc[2] += tier_bytes(w.z, s_lut + s * 128, p.c256), acc[3] += tier_bytes(w.w, s_lut + s * 128, p.c256);
       }
-      const int64_t wn = w0 + CC_PASS;
-      if (wn < v_end) {
+      *reinterpret_cast<uint4*>(out8 + v0) = make_uint4(acc[0], acc[1], acc[2], acc[3]);
+      const int64_t key0 = v_begin + v0 - p.mis;
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-          const int64_t v = wn + 32 * j + lane;
-          r[j] = (j < kpl && v < v_end) ? __ldg(reinterpret_cast<const uint4*>(base + v * 16)) : make_uint4(0, 0, 0, 0);
-        }
-      }
-      unsigned* hh = hist_rep + ((split && w0 - v_begin >= hist_keys) ? 8 * 256 : 0);
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        const int64_t v = w0 + 32 * j + lane;
-        if (j < kpl && v < v_end) {
-          out8[v] = (uint8_t)cnt[j];
-          atomicAdd(&hh[cnt[j]], 1u);
-        }
-      }
+      for (int k = 0; k < 16; k++)
+        if (key0 + k >= 0 && key0 + k < N && v0 + k < n_keys)
+          atomicAdd(&region[byte_of(acc[k >> 2], k & 3) * 32 + lane], 1u);
     }
   } else {
-    for (int64_t v = v_begin + tid; v < v_end; v += CC_THREADS) {
-      const int64_t key = v - p.mis;
-      if (key < 0) continue;
-      int cnt = 0;
-      for (int s = 0; s < 16; s++) cnt += s_lut[s * 256 + base[s * p.c_s + v * p.c_l]];
+    for (int v = tid; v < n_keys; v += CH_THREADS) {
+      if (v_begin + v - p.mis < 0) continue;
+      unsigned cnt = 0;
+      for (int s = 0; s < 16; s++) {
+        const unsigned c = base[s * p.c_s + v * p.c_l];
+        cnt += (s_lut[s * 128 + (c & 127u)] >> (c >> 7 << 2)) & 15u;
+      }
       out8[v] = (uint8_t)cnt;
-      atomicAdd(&hist_rep[((split && v - v_begin >= hist_keys) ? 8 * 256 : 0) + cnt], 1u);
+      atomicAdd(&region[cnt * 32 + lane], 1u);
     }
   }
   __syncthreads();
-  {
-    const int half = tid >> 8, bin = tid & 255;
-    if (half == 0 || split) {
-      unsigned t = 0;
-#pragma unroll
-      for (int rep = 0; rep < 8; rep++) t += hist[(half * 8 + rep) * 256 + bin];
-      const int64_t row = split ? 2 * (int64_t)blockIdx.x + half : (int64_t)blockIdx.x;
-      if (row < p.n_hist)  // the second half of the last block may lie beyond the zone: it has no row
-        p.chunk_hist[((int64_t)bh * p.n_hist + row) * 256 + bin] = t;
-    }
+  uint32_t* row = p.chunk_hist + ((int64_t)bh * p.n_hist + blockIdx.x) * 256;
+  for (int bin = warp; bin < 256; bin += CH_WARPS) {
+    const unsigned t = bin < CH_CBINS ? __reduce_add_sync(0xffffffffu, region[bin * 32 + lane]) : 0u;
+    if (lane == 0) row[bin] = t;
   }
 }
 
@@ -654,23 +496,17 @@ int launch_rank(const uint16_t* queries, const uint16_t* signs, int Hq, int H, u
   return check_launch("rank_clusters");
 }
 
-// Launch geometry of the chain's collision kernel: about one block per SM over the whole grid.  A block covers
-// chunk_keys virtual keys: a multiple of 512 up to 8192 (one pass), else a multiple of 8192 up to 32768 (the selection
-// kernel keeps one int per key of a histogram row in shared memory).
-void chain_geometry(int64_t bs_h, int64_t Nv, int64_t* chunk_keys, int64_t* hist_keys, int64_t* n_hist) {
+// Launch geometry of the several-launch chain: about one block per SM over the whole grid, one histogram row each; both
+// the collision and the selection kernel take chunk_keys virtual keys per block, a multiple of 512.  At least 2048, because
+// every block of the selection kernel reads all rows of its head; at most what that kernel holds in shared memory.
+void chain_geometry(int64_t bs_h, int64_t Nv, int64_t* chunk_keys, int64_t* n_hist) {
   int64_t target = (int64_t)sm_count() / (bs_h > 0 ? bs_h : 1);
   if (target < 1) target = 1;
-  int64_t chunk = (Nv + target - 1) / target;
-  if (chunk < 2048) chunk = 2048;  // every block of the selection kernel reads all histogram rows: keep them few
-  if (chunk <= CC_PASS) {
-    chunk = (chunk + 511) / 512 * 512;
-  } else {
-    chunk = (chunk + CC_PASS - 1) / CC_PASS * CC_PASS;
-    if (chunk > 32768) chunk = 32768;
-  }
+  int64_t chunk = ((Nv + target - 1) / target + 511) / 512 * 512;
+  if (chunk < 2048) chunk = 2048;
+  if (chunk > CHAIN_CHUNK_MAX) chunk = CHAIN_CHUNK_MAX;
   *chunk_keys = chunk;
-  *hist_keys = chunk <= CC_PASS ? chunk / 2 : chunk;
-  *n_hist = (Nv + *hist_keys - 1) / *hist_keys;
+  *n_hist = (Nv + chunk - 1) / chunk;
 }
 
 // The stand-alone op: streams the codes of N keys per (batch, head) and writes int32 counts; table from `lut`.
@@ -696,17 +532,15 @@ int launch_collision(const pk_tensor* codebook, const uint32_t* lut, int32_t* ou
   const int64_t n_chunks = (Nv + p.chunk_keys - 1) / p.chunk_keys;
   dim3 grid((unsigned)n_chunks, (unsigned)(bs * H));
   StageTimer tm(ST_COLLISION, st);
-  if (layout == 0) collision_kernel<0, false><<<grid, 256, 0, st>>>(p);
-  else if (layout == 1) collision_kernel<1, false><<<grid, 256, 0, st>>>(p);
-  else collision_kernel<2, false><<<grid, 256, 0, st>>>(p);
+  if (layout == 0) collision_kernel<0><<<grid, 256, 0, st>>>(p);
+  else if (layout == 1) collision_kernel<1><<<grid, 256, 0, st>>>(p);
+  else collision_kernel<2><<<grid, 256, 0, st>>>(p);
   return check_launch("collision");
 }
 
-// The decode chain: query preparation, cluster ranking, tier table and the count in one kernel; compact output
-// (u8 per virtual key + 256-bin histograms, one per hist_keys keys).
+// First launch of the several-launch chain: u8 counts per virtual key and one 256-bin histogram row per chunk_keys keys.
 int launch_chain_collision(const pk_tensor* codebook, const ChainQuery& cq, uint8_t* counts_u8, int64_t u8_stride,
-                           uint32_t* chunk_hist, int* mis_out, int64_t* hist_keys_out, int64_t* n_hist_out,
-                           cudaStream_t st) {
+                           uint32_t* chunk_hist, int* mis_out, int64_t* chunk_keys_out, int64_t* n_hist_out, cudaStream_t st) {
   const int64_t bs = codebook->shape[0], H = codebook->shape[1], B = codebook->shape[2], N = codebook->shape[3];
   if (B != 16) return fail(PK_ERR_ARG, "the fused chain supports 16 subspaces");
   CollParams p = {};
@@ -719,19 +553,16 @@ int launch_chain_collision(const pk_tensor* codebook, const ChainQuery& cq, uint
   p.q = cq;
   p.G = H > 0 ? cq.Hq / (int)H : 1;
   p.inv_g = 1.0f / (float)p.G;
+  p.c256 = 256;
   int layout = 2;
-  p.mis = chain_layout(codebook, &layout);
-  int64_t hist_keys = 0;
-  chain_geometry(bs * H, N + p.mis, &p.chunk_keys, &hist_keys, &p.n_hist);
-  const int64_t n_blocks = (N + p.mis + p.chunk_keys - 1) / p.chunk_keys;
-  if (mis_out) *mis_out = p.mis;
-  if (hist_keys_out) *hist_keys_out = hist_keys;
-  if (n_hist_out) *n_hist_out = p.n_hist;
-  dim3 grid((unsigned)n_blocks, (unsigned)(bs * H));
+  *mis_out = p.mis = chain_layout(codebook, &layout);
+  chain_geometry(bs * H, N + p.mis, &p.chunk_keys, &p.n_hist);
+  *chunk_keys_out = p.chunk_keys, *n_hist_out = p.n_hist;
+  dim3 grid((unsigned)p.n_hist, (unsigned)(bs * H));
   StageTimer tm(ST_COLLISION, st);
-  if (layout == 0) launch_chain(chain_collision_kernel<0>, grid, dim3(CC_THREADS), 0, st, p);
-  else if (layout == 1) launch_chain(chain_collision_kernel<1>, grid, dim3(CC_THREADS), 0, st, p);
-  else launch_chain(chain_collision_kernel<2>, grid, dim3(CC_THREADS), 0, st, p);
+  if (layout == 0) launch_chain(collide_kernel<0>, grid, dim3(CH_THREADS), 0, st, p);
+  else if (layout == 1) launch_chain(collide_kernel<1>, grid, dim3(CH_THREADS), 0, st, p);
+  else launch_chain(collide_kernel<2>, grid, dim3(CH_THREADS), 0, st, p);
   return check_launch("chain collision");
 }
 

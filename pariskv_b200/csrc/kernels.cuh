@@ -58,28 +58,23 @@ struct ChainQuery {
   const int32_t* n_dev;       // [bs] searchable keys per sample (device), or null: all N keys of the view
   pk_zone_schedule sched;     // thresholds = zone_tiers(sched, n_dev[b]) when n_dev is set
   long long n_plan;           // > 0: thresholds from this zone length instead (a shard of a longer zone)
-  unsigned* zero_words;       // [bs*H] words set to zero here (arrival counters of the selection kernel), or null
   int early_query;            // the queries were complete before the previous kernel on the stream started
-  unsigned* zero_area;        // [bs*H][zero_area_words] set to zero here (the selection kernel's value histogram), or null
-  int zero_area_words;
 };
 int launch_collision(const pk_tensor* codebook, const uint32_t* lut, int32_t* out_i32, cudaStream_t st);
 int chain_layout(const pk_tensor* codebook, int* layout);
-void chain_geometry(int64_t bs_h, int64_t Nv, int64_t* chunk_keys, int64_t* hist_keys, int64_t* n_hist);
+constexpr int64_t CHAIN_CHUNK_MAX = 64 * 1024;   // keys per block of the several-launch chain
+void chain_geometry(int64_t bs_h, int64_t Nv, int64_t* chunk_keys, int64_t* n_hist);
 int launch_chain_collision(const pk_tensor* codebook, const ChainQuery& cq, uint8_t* counts_u8, int64_t u8_stride,
-                           uint32_t* chunk_hist, int* mis_out, int64_t* hist_keys_out, int64_t* n_hist_out,
+                           uint32_t* chunk_hist, int* mis_out, int64_t* chunk_keys_out, int64_t* n_hist_out,
                            cudaStream_t st);
 // local_hist[bh][bin] = sum over chunks of chunk_hist[bh][chunk][bin]
 int launch_hist_reduce(const uint32_t* chunk_hist, int64_t bs_h, int64_t n_chunks, int64_t chunk_keys, int mis, int H,
                        int64_t N, const int32_t* n_dev, uint32_t* local_hist, cudaStream_t st);
 
-// topk.cu: exact top-k of rows of 32-bit values; out[row][i] = map ? map[row*map_stride + pos] : pos
-// With `scratch` (topk_scratch_bytes(rows, L, k) bytes, 256-byte aligned; 0 = not needed) rows longer than 16384
-// elements are selected in two passes of the one-CTA kernel instead of the cluster kernel.
-int64_t topk_scratch_bytes(int64_t rows, int64_t L, int64_t k);
-int launch_topk(const void* in, bool is_float, int64_t rows, int64_t row_stride, int64_t L, int64_t k,
-                int64_t* out, const int64_t* map, int64_t map_stride, int order, cudaStream_t st, int stage,
-                void* scratch = nullptr, int64_t scratch_bytes = 0);
+// topk.cu: exact top-k of rows of 32-bit values; out[row][i] = map ? map[row*map_stride + pos] : pos.  n_dev: valid elements
+// of every row, read on the device (null: L); n_out: [rows] min(k, valid elements), or null.
+int launch_topk(const void* in, bool is_float, int64_t rows, int64_t row_stride, int64_t L, int64_t k, const int32_t* n_dev,
+                int64_t* out, int32_t* n_out, const int64_t* map, int64_t map_stride, int order, cudaStream_t st, int stage);
 
 // rerank.cu
 struct RerankArgs {
@@ -99,8 +94,7 @@ int fill_rerank_args(RerankArgs* a, const pk_tensor* key_4bit, const pk_tensor* 
 int launch_rerank(const RerankArgs& a, int64_t bs_h, uint16_t* scores_bf16, float* scores_f32, uint16_t* v4b,
                   cudaStream_t st);
 
-// Candidate selection from u8 counts + per-block histograms, the rerank of the selected keys and the final top-K
-// (by the block that finishes last for a (batch, head)) in one kernel.
+// Candidate selection from u8 counts + per-block histograms and the rerank of the selected keys in one kernel.
 struct SelectArgs {
   const uint8_t* counts_u8;      // [bs*H][u8_stride] virtual keys
   int64_t u8_stride;
@@ -110,24 +104,18 @@ struct SelectArgs {
   int64_t N;                     // keys per head of the view (upper bound when n_dev is set)
   int64_t C;                     // row stride (and capacity) of cand_out / scores_f32
   int64_t C_want;                // candidates wanted per head over the whole zone, all shards together (n_dev == null)
-  int64_t K;                     // final top-K; 0 = stop after the rerank
+  int64_t K;                     // final top-K (one-launch chain); 0 = stop after the rerank
   int fill_tail;                 // rows may be longer than the candidate list: the tail gets (score -inf, key 0)
-  unsigned* val_hist;            // [bs*H][select_value_bins()] zero at launch, or null: histogram of the scores' top
-                                 // key bits, filled while the scores are computed; long rows select their top-K from it
   const int32_t* n_dev;          // [bs] searchable keys per sample, or null
   pk_zone_schedule sched;        // candidates = zone_candidates(sched, n_dev[b]) when n_dev is set
   const uint32_t* shard_hist;    // [world][bs*H][256] histograms of every shard (exact sequence-sharded selection)
   int world, rank;
   int64_t* cand_out;             // [bs*H][C]
   float* scores_f32;             // [bs*H][C]
-  int64_t* final_out;            // [bs*H][K] ascending key index (K > 0)
+  int64_t* final_out;            // [bs*H][K] ascending key index (one-launch chain, K > 0)
   int32_t* n_sel_out;            // [bs*H] or null: entries of final_out that are valid = min(K, candidates)
   int32_t* n_cand_out;           // [bs*H] or null: candidates of this (batch, head)
-  unsigned* counters;            // [bs*H] arrival counters, zero at launch (K > 0)
 };
-int64_t select_smem_bytes(int64_t chunk_keys, int64_t C, int64_t K);
-int64_t select_value_bins();     // words per (batch, head) of SelectArgs::val_hist
-int64_t select_final_max_row();  // longest score row whose final top-K the selection kernel finishes entirely in shared memory
 int launch_select_rerank(const RerankArgs& a, int64_t bs_h, const SelectArgs& s, cudaStream_t st);
 
 // retrieve_fused.cu: the whole chain in one launch, one cluster of `cs` CTAs per (batch, head)

@@ -1,7 +1,7 @@
 // The whole retrieval chain of one decode step as one host call: one launch where the metadata is key-major and a
-// cluster of CTAs holds a head's zone on chip (retrieve_fused.cu), otherwise two launches:
+// cluster of CTAs holds a head's zone on chip (retrieve_fused.cu), otherwise three, each over all SMs:
 // (1) query preparation + cluster ranking + tier table + collision count (u8 counts + per-block histograms),
-// (2) candidate selection + 4-bit rerank + final top-K by the last block of every (batch, head).
+// (2) candidate selection + 4-bit rerank, (3) final top-K over a cluster per (batch, head).
 // All scratch comes from the caller.
 #include "common.cuh"
 #include "kernels.cuh"
@@ -12,7 +12,7 @@ namespace {
 inline int64_t align256(int64_t x) { return (x + 255) / 256 * 256; }
 
 struct RetrieveLayout {
-  int64_t q_blocks, q_norm, counters, counts, hist, scores, cand, vhist, topk, topk_bytes, total;
+  int64_t q_blocks, q_norm, n_cand, counts, hist, scores, cand, total;
   int64_t u8_stride, n_chunks_max;
 };
 
@@ -21,24 +21,19 @@ RetrieveLayout make_layout(int64_t bs, int64_t H, int64_t N, int64_t C) {
   const int64_t bh = bs * H;
   l.u8_stride = (N + 15 + 15) / 16 * 16 + 16;
   // an upper bound on the blocks per (batch, head) that grows with N, so that scratch sized for a zone's capacity
-  // serves every shorter zone: the launcher aims at one block per SM (two histogram rows each) and caps a block at
-  // 32768 keys
+  // serves every shorter zone: the launcher aims at one block per SM and caps the keys of a block
   int64_t target = (int64_t)sm_count() / (bh > 0 ? bh : 1);
   if (target < 1) target = 1;
-  const int64_t by_cap = (N + 15 + 32767) / 32768;
-  l.n_chunks_max = (2 * target > by_cap ? 2 * target : by_cap) + 2;
+  const int64_t by_cap = (N + 15 + CHAIN_CHUNK_MAX - 1) / CHAIN_CHUNK_MAX;
+  l.n_chunks_max = (target > by_cap ? target : by_cap) + 1;
   int64_t off = 0;
   l.q_blocks = off, off += align256(bh * 128 * 2);
   l.q_norm = off, off += align256(bh * 2);
-  l.counters = off, off += align256(bh * 4);
+  l.n_cand = off, off += align256(bh * 4);
   l.counts = off, off += align256(bh * l.u8_stride);
   l.hist = off, off += align256(bh * l.n_chunks_max * 256 * 4);
   l.scores = off, off += align256(bh * C * 4);
   l.cand = off, off += align256(bh * C * 8);
-  // value histogram of the final selection: long rows only
-  l.vhist = off, off += C > select_final_max_row() ? align256(bh * select_value_bins() * 4) : 0;
-  l.topk_bytes = topk_scratch_bytes(bh, C, 2048);   // long rows only; the size does not depend on K
-  l.topk = off, off += align256(l.topk_bytes);
   l.total = off;
   return l;
 }
@@ -168,7 +163,6 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
   }
   uint8_t* counts = (uint8_t*)(ws + lay.counts);
   uint32_t* hist = (uint32_t*)(ws + lay.hist);
-  unsigned* counters = (unsigned*)(ws + lay.counters);
   // the launch geometry is a function of the view alone, so phase 2 finds what phase 1 left in the workspace;
   // chunk_keys / n_chunks: keys per histogram row and rows per (batch, head), the selection kernel's grid
   int mis = 0;
@@ -188,9 +182,6 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
       return launch_fused_retrieve(cs, codebook, ra, cq, sa, a.cand ? cd : nullptr, a.scores_f32 ? sc : nullptr,
                                    (int64_t*)(ws + lay.cand), (float*)(ws + lay.scores), st);
     }
-    cq.zero_words = counters;
-    if (K > 0 && row > select_final_max_row() && (varlen || sharded || n_sel))
-      cq.zero_area = (unsigned*)(ws + lay.vhist), cq.zero_area_words = (int)select_value_bins();
     if ((rc = launch_chain_collision(codebook, cq, counts, lay.u8_stride, hist, &mis, &chunk_keys, &n_chunks, st)))
       return rc;
     if (n_chunks > lay.n_chunks_max) return fail(PK_ERR_WORKSPACE, "internal: histogram workspace undersized");
@@ -204,12 +195,11 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
   } else {
     int layout = 0;
     mis = chain_layout(codebook, &layout);
-    int64_t block_keys = 0;
-    chain_geometry(bh, N + mis, &block_keys, &chunk_keys, &n_chunks);
+    chain_geometry(bh, N + mis, &chunk_keys, &n_chunks);
   }
   sa.counts_u8 = counts, sa.u8_stride = lay.u8_stride, sa.chunk_hist = hist;
   sa.n_chunks = n_chunks, sa.chunk_keys = chunk_keys, sa.mis = mis, sa.N = N;
-  sa.C = row, sa.C_want = C, sa.K = K;
+  sa.C = row, sa.C_want = C;
   if (a.phase == 2) {
     PK_CHECK_TENSOR(a.shard_hist, PK_I32, 4);
     PK_REQUIRE(a.world >= 1 && a.world <= 64 && a.rank >= 0 && a.rank < a.world, "rank / world out of range");
@@ -219,24 +209,14 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
     sa.shard_hist = (const uint32_t*)a.shard_hist->data, sa.world = a.world, sa.rank = a.rank;
   }
   sa.cand_out = cd, sa.scores_f32 = sc;
-  // Long score rows.  Full rows of a fixed length (no per-sample lengths, no shards): the final top-K runs as the
-  // two-pass selection over many blocks after the selection kernel (measured faster at 100 K scores per row than one
-  // block per head).  Rows whose length is only known on the device: every block of the selection kernel adds its
-  // scores to a histogram of their top key bits, which the collision kernel cleared (phase 2 finds it cleared by
-  // phase 1), and the last block of a (batch, head) selects from it - still one launch.
   sa.fill_tail = varlen;
-  const bool long_rows = K > 0 && row > select_final_max_row();
-  const bool separate_final = long_rows && !varlen && !sharded && !n_sel;
-  sa.val_hist = long_rows && !separate_final ? (unsigned*)(ws + lay.vhist) : nullptr;
-  if (separate_final) sa.K = 0;
-  sa.final_out = K > 0 ? (int64_t*)a.final_indices->data : nullptr;
-  sa.n_sel_out = n_sel, sa.n_cand_out = n_cand, sa.counters = counters;
+  sa.n_cand_out = n_cand ? n_cand : (int32_t*)(ws + lay.n_cand);
   ra.cand = nullptr;
   ra.q_blocks = qb, ra.q_norm = qn, ra.centers = (const uint16_t*)a.mag_centers->data;
   ra.C = row;
-  if ((rc = launch_select_rerank(ra, bh, sa, st)) || !separate_final) return rc;
-  return launch_topk(sc, true, bh, row, row, K, (int64_t*)a.final_indices->data, cd, row, 0, st, ST_FINAL_TOPK,
-                     lay.topk_bytes ? ws + lay.topk : nullptr, lay.topk_bytes);
+  if ((rc = launch_select_rerank(ra, bh, sa, st)) || K <= 0) return rc;
+  return launch_topk(sc, true, bh, row, row, K, sa.n_cand_out, (int64_t*)a.final_indices->data, n_sel, cd, row, 0, st,
+                     ST_FINAL_TOPK);
 }
 }  // namespace
 

@@ -23,17 +23,12 @@
 namespace pk {
 namespace {
 
-constexpr int FR_THREADS = SEL_THREADS;
-constexpr int FR_WARPS = FR_THREADS / 32;
-constexpr int FR_CBINS = 129;               // counts 0 .. 16 subspaces x 8 tiers
+static_assert(CH_THREADS == SEL_THREADS, "one block shape");
 constexpr int FR_LIST_MAX = 8192;           // candidates a CTA keeps in shared memory; more spill to the workspace
 constexpr int FR_SPAN_MAX = 40 * 1024;      // keys of a CTA: beyond it two launches over all SMs are faster
-constexpr int FR_REC = 112;                 // bytes between staged records (96 used): quarter-warp reads do not conflict
-constexpr int FR_STAGE = FR_WARPS * 32 * FR_REC;
-constexpr int FR_HIST_BYTES = FR_CBINS * 32 * 4;   // one replica per lane: a warp's atomics never collide on a bank
 constexpr int FR_WORDS = LEV2_BYTES / 8;    // ballots of the final selection, over the level table
 static_assert(FR_SPAN_MAX / 32 <= FR_WORDS, "one ballot per 32 candidates");
-static_assert(FR_HIST_BYTES >= 16 * 256 * 4 && FR_HIST_BYTES >= SEL_REGION, "the region serves three stages");
+static_assert(CH_HIST_BYTES >= 16 * 256 * 4 && CH_HIST_BYTES >= SEL_REGION, "the region serves three stages");
 
 struct FusedParams {
   const uint8_t* codes;   // key-major records of 16 bytes; (b,h) at b*c_b + h*c_h
@@ -57,7 +52,7 @@ struct FusedParams {
 };
 
 template <int CS>
-__global__ void __launch_bounds__(FR_THREADS, 1) retrieve_fused_kernel(FusedParams p) {
+__global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedParams p) {
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ SelShared s;
@@ -67,44 +62,23 @@ __global__ void __launch_bounds__(FR_THREADS, 1) retrieve_fused_kernel(FusedPara
   __shared__ __align__(16) float4 s_q2[32];       // the same, the subspaces of a pair side by side (see rerank_pairs)
   __shared__ __align__(16) uint8_t s_lut[16 * 128];
   unsigned* region = reinterpret_cast<unsigned*>(dyn);
-  uint32_t* lev2 = reinterpret_cast<uint32_t*>(dyn + FR_HIST_BYTES);
-  uint8_t* cnt8 = dyn + FR_HIST_BYTES + LEV2_BYTES;
-  uint8_t* stage = cnt8 + (threadIdx.x >> 5) * (32 * FR_REC);   // the counts are done with when records are staged
-  int* ids = reinterpret_cast<int*>(cnt8 + max(p.span_cap, FR_STAGE));
+  uint32_t* lev2 = reinterpret_cast<uint32_t*>(dyn + CH_HIST_BYTES);
+  uint8_t* cnt8 = dyn + CH_HIST_BYTES + LEV2_BYTES;
+  uint8_t* stage = cnt8 + (threadIdx.x >> 5) * (32 * CH_REC);   // the counts are done with when records are staged
+  int* ids = reinterpret_cast<int*>(cnt8 + max(p.span_cap, CH_STAGE));
   float* sc = reinterpret_cast<float*>(ids + p.list_cap);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned rank = CS == 1 ? 0u : cluster.block_rank();
   const int64_t bh = blockIdx.y;
   const int b = (int)(bh / p.H), h = (int)(bh % p.H);
   const ChainQuery& cq = p.q;
-  // ---- query: warp 0 averages, normalises and rotates it; then warp w ranks the clusters of subspace w (registers) ----
-  float qavg[4] = {0.0f, 0.0f, 0.0f, 0.0f}, qx[4] = {0.0f, 0.0f, 0.0f, 0.0f}, qn0 = 0.0f;
+  PreparedQuery pq;
   unsigned key[8];
-  auto prepare_query = [&]() {
-    if (warp == 0) {
-      const uint16_t* q = cq.queries + ((int64_t)b * cq.Hq + (int64_t)h * p.G) * 128 + 4 * lane;
-      float sg[4], acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      unpack4(__ldg(reinterpret_cast<const uint2*>(cq.signs + 4 * lane)), sg);
-      for (int g = 0; g < p.G; g++) {  // fp32 sum over the group, g ascending
-        float v[4];
-        unpack4(__ldg(reinterpret_cast<const uint2*>(q + g * 128)), v);
-#pragma unroll
-        for (int i = 0; i < 4; i++) acc[i] = __fadd_rn(acc[i], v[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; i++) qx[i] = qavg[i] = bfround(__fmul_rn(acc[i], p.inv_g));
-      qn0 = rotate4(qx, sg, lane);
-#pragma unroll
-      for (int i = 0; i < 4; i++) s_q[4 * lane + i] = qx[i];
-      if (lane == 0) s_qnorm = qn0;
-    }
-  };
-  auto rank_clusters = [&]() { rank_subspace(key, s_q + warp * 8, lane); };
   const bool early = cq.early_query != 0;
-  if (early) {
-    prepare_query();
+  if (early) {   // the queries were complete before the kernel before this one started
+    prepare_query(pq, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     __syncthreads();
-    rank_clusters();
+    rank_subspace(key, s_q + warp * 8, lane);
   }
   pdl_wait();
   pdl_trigger();
@@ -115,10 +89,10 @@ __global__ void __launch_bounds__(FR_THREADS, 1) retrieve_fused_kernel(FusedPara
   const int n_keys = (int)max((int64_t)0, min((int64_t)span, N - begin));
   const uint8_t* codes = p.codes + b * p.c_b + h * p.c_h + begin * 16;
 
-  // ---- code loads: a warp takes 128 consecutive keys (four per lane) every FR_WARPS * 128; two rounds are in flight,
+  // ---- code loads: a warp takes 128 consecutive keys (four per lane) every CH_WARPS * 128; two rounds are in flight,
   // the first ones during the prologue ----
   uint4 r0[4], r1[4];
-  constexpr int STEP = FR_WARPS * 128;
+  constexpr int STEP = CH_WARPS * 128;
   auto load_codes = [&](uint4 (&r)[4], int v0) {
     if (n_keys > 0)
 #pragma unroll
@@ -131,67 +105,18 @@ __global__ void __launch_bounds__(FR_THREADS, 1) retrieve_fused_kernel(FusedPara
     const int4* cp = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
     const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1);   // cluster sizes of this warp's subspace
     unsigned* my = region + warp * 256;
-    if (!early) prepare_query();
-    if (warp == 0 && rank == 0) {
-      if (cq.query_avg)
-        *reinterpret_cast<uint2*>(cq.query_avg + bh * 128 + 4 * lane) =
-            make_uint2((uint32_t)f2bf(qavg[0]) | ((uint32_t)f2bf(qavg[1]) << 16), (uint32_t)f2bf(qavg[2]) | ((uint32_t)f2bf(qavg[3]) << 16));
-      if (cq.q_blocks)
-        *reinterpret_cast<uint2*>(cq.q_blocks + bh * 128 + 4 * lane) =
-            make_uint2((uint32_t)f2bf(qx[0]) | ((uint32_t)f2bf(qx[1]) << 16), (uint32_t)f2bf(qx[2]) | ((uint32_t)f2bf(qx[3]) << 16));
-      if (cq.q_norm && lane == 0) cq.q_norm[bh] = f2bf(qn0);
-    }
-    if (tid == 32) {
-      if (cq.n_dev) {
-        unsigned t[8];
-        zone_tiers(cq.sched, (long long)N, t);
-        for (int i = 0; i < cq.sched.n_tiers; i++) s_tiers[i] = t[i];
-        s_tiers[8] = (unsigned)cq.sched.n_tiers;
-      } else {
-        for (int i = 0; i < cq.n_tiers; i++) s_tiers[i] = cq.tiers[i];
-        s_tiers[8] = (unsigned)cq.n_tiers;
-      }
-    }
+    if (!early) prepare_query(pq, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
+    if (warp == 0 && rank == 0) publish_query(pq, cq, bh);
+    if (tid == 32) load_tiers(cq, (long long)N, s_tiers);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
     *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
-    build_lev2(lev2, p.a.centers, tid, FR_THREADS);
+    build_lev2(lev2, p.a.centers, tid, CH_THREADS);
     __syncthreads();
-    if (!early) rank_clusters();
-    const int n_tiers = (int)s_tiers[8];
-    unsigned tier[8];
-#pragma unroll
-    for (int t = 0; t < 8; t++) tier[t] = t < n_tiers ? s_tiers[t] : 0u;
-    unsigned cnt[8], run = 0;
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) {
-      cnt[rr] = my[255u - (key[rr] & 255u)];
-      run += cnt[rr];
-    }
-    unsigned incl = run;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += o;
-    }
-    unsigned excl = incl - run;
-    __syncwarp();   // the sizes have been read: the same words take the tier counts, packed to nibbles below
-#pragma unroll
-    for (int rr = 0; rr < 8; rr++) {
-      unsigned wgt = 0;
-#pragma unroll
-      for (int t = 0; t < 8; t++) wgt += (excl < tier[t]) ? 1u : 0u;   // absent tiers are 0: never above a prefix sum
-      my[255u - (key[rr] & 255u)] = wgt;
-      excl += cnt[rr];
-    }
-    __syncwarp();
-    {  // entries i (low nibble) and i + 128 of byte i: four bytes per lane
-      const uint4 e0 = *reinterpret_cast<const uint4*>(my + lane * 4), e1 = *reinterpret_cast<const uint4*>(my + 128 + lane * 4);
-      const uint32_t w = (e0.x | (e1.x << 4)) | ((e0.y | (e1.y << 4)) << 8) | ((e0.z | (e1.z << 4)) << 16) | ((e0.w | (e1.w << 4)) << 24);
-      *reinterpret_cast<uint32_t*>(s_lut + warp * 128 + lane * 4) = w;
-    }
+    if (!early) rank_subspace(key, s_q + warp * 8, lane);
+    tier_table(key, my, s_tiers, s_lut + warp * 128);
     if (tid < 128) reinterpret_cast<float*>(s_q2)[pair_slot(tid)] = s_q[tid];
     __syncthreads();   // the tables are complete and the staging area is free again
-    for (int i = tid; i < FR_CBINS * 32; i += FR_THREADS) region[i] = 0;
+    for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
     __syncthreads();
   }
   const float qn = s_qnorm;
@@ -215,12 +140,12 @@ __global__ void __launch_bounds__(FR_THREADS, 1) retrieve_fused_kernel(FusedPara
     if (v0 - lane + STEP < n_keys) count_round(r1, v0 + STEP);
   }
   __syncthreads();
-  for (int bin = warp; bin < FR_CBINS; bin += FR_WARPS) {
+  for (int bin = warp; bin < CH_CBINS; bin += CH_WARPS) {
     const unsigned t = __reduce_add_sync(0xffffffffu, region[bin * 32 + lane]);
     if (lane == 0) s.hist[0][bin] = t;
   }
   sync_cluster<CS>(cluster);
-  cluster_threshold<CS, FR_CBINS>(cluster, s, s.hist[0], rank, (unsigned)C_want);
+  cluster_threshold<CS, CH_CBINS>(cluster, s, s.hist[0], rank, (unsigned)C_want);
   const unsigned T = s.res[0], quota = (unsigned)C_want - s.res[1];
   const unsigned gt_base = s.res[3], eq_base = s.res[4];
   const int64_t C_here = min(C_want, p.C);
@@ -228,74 +153,10 @@ __global__ void __launch_bounds__(FR_THREADS, 1) retrieve_fused_kernel(FusedPara
   // ---- ordered candidate list of this CTA: counts above T, and ties at T while the quota lasts ----
   const int64_t row_base = bh * p.C;
   const int64_t out_pos = (int64_t)gt_base + min(eq_base, quota);
-  int n_list;
-  {
-    const int wspan = ((n_keys + FR_WARPS - 1) / FR_WARPS + 15) / 16 * 16;
-    const int k0 = min(n_keys, warp * wspan), k1 = min(n_keys, k0 + wspan);
-    const uint32_t add_gt = (127u - T) * 0x01010101u;           // T <= 128, counts <= 128: no carry between bytes
-    const uint32_t add_ge = T ? (128u - T) * 0x01010101u : 0u;
-    unsigned n_gt = 0, n_eq = 0;
-#pragma unroll 1
-    for (int k = k0 + 16 * lane; k < k1; k += 512) {   // 16 keys -> masks of counts above / at the threshold, kept in their place
-      unsigned gt = 0, eq = 0;
-      const uint4 v = *reinterpret_cast<const uint4*>(cnt8 + k);
-      const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const uint32_t g = T < 128u ? (w4[i] + add_gt) & 0x80808080u : 0u;
-        const uint32_t ge = T ? (w4[i] + add_ge) & 0x80808080u : 0x80808080u;
-        gt |= ((((g >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * i);
-        eq |= (((((ge & ~g) >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * i);
-      }
-      if (k1 - k < 16) gt &= (1u << (k1 - k)) - 1u, eq &= (1u << (k1 - k)) - 1u;
-      *reinterpret_cast<unsigned*>(cnt8 + k) = gt | (eq << 16);
-      n_gt += __popc(gt), n_eq += __popc(eq);
-    }
-    n_gt = __reduce_add_sync(0xffffffffu, n_gt), n_eq = __reduce_add_sync(0xffffffffu, n_eq);
-    if (lane == 0) s.warp_a[warp] = n_gt, s.warp_b[warp] = n_eq;
-    __syncthreads();
-    unsigned g = 0, e = eq_base, g_all = 0, e_all = eq_base;
-#pragma unroll
-    for (int w = 0; w < FR_WARPS; w++) {
-      const unsigned a = s.warp_a[w], c = s.warp_b[w];
-      if (w < warp) g += a, e += c;
-      g_all += a, e_all += c;
-    }
-    const unsigned eq_before = min(eq_base, quota);
-    n_list = (int)(g_all + min(e_all, quota) - eq_before);
-    n_list = (int)max((int64_t)0, min((int64_t)n_list, C_here - out_pos));   // a no-op with consistent histograms
-#pragma unroll 1
-    for (int k = k0; k < k1; k += 512) {
-      const unsigned m = k + 16 * lane < k1 ? *reinterpret_cast<const unsigned*>(cnt8 + k + 16 * lane) : 0u;
-      const unsigned gt = m & 0xffffu, eq = m >> 16;
-      const unsigned mine = ((unsigned)__popc(gt) << 16) | (unsigned)__popc(eq);
-      unsigned inc = mine;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const unsigned o = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += o;
-      }
-      const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
-      const unsigned eg = g + ((inc - mine) >> 16), ee = e + ((inc - mine) & 0xffffu);
-      const int room = (int)quota - (int)ee;   // ties this lane may still take
-      unsigned take = eq;
-      if (room < (int)__popc(eq))
-        for (int drop = (int)__popc(eq) - max(room, 0); drop > 0; drop--) take &= ~(1u << (31 - __clz(take)));
-      take |= gt;
-      int pos = (int)(eg + min(ee, quota) - eq_before);
-      const int kb = (int)begin + k + 16 * lane;
-      while (take) {
-        const int j = __ffs(take) - 1;
-        take &= take - 1;
-        if (pos < n_list) {
-          if (pos < p.list_cap) ids[pos] = kb + j;
-          else p.ws_cand[row_base + out_pos + pos] = kb + j;
-        }
-        pos++;
-      }
-      g += total >> 16, e += total & 0xffffu;
-    }
-  }
+  const int n_list = list_candidates(cnt8, n_keys, 0, T, quota, eq_base, C_here - out_pos, s.warp_a, s.warp_b, [&](int pos, int off) {
+    if (pos < p.list_cap) ids[pos] = (int)begin + off;
+    else p.ws_cand[row_base + out_pos + pos] = begin + off;
+  });
   __syncthreads();
 
   // ---- rerank ----
@@ -305,47 +166,17 @@ __global__ void __launch_bounds__(FR_THREADS, 1) retrieve_fused_kernel(FusedPara
   {
     const uint8_t* k4 = p.a.k4 + b * p.a.k4_b + h * p.a.k4_h;
     const uint16_t* w = p.a.w + b * p.a.w_b + h * p.a.w_h;
-    // A warp takes 32 consecutive candidates per round: it loads their records with whole sectors per request (four lanes
-    // on the 64 bytes of codes, two on the 32 bytes of weights), turns them over its staging buffer to one record per lane,
-    // and has the loads of the next round in flight during the arithmetic.  One record per lane straight from memory
-    // touches 32 lines per request and is bound by the L1's tag look-ups, 6 per candidate.
-    constexpr int ROUND = FR_WARPS * 32;
-    uint4 in[6];
-    auto fetch = [&](int base) {   // out of range: the list's last candidate again
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-        in[i] = __ldg(reinterpret_cast<const uint4*>(k4 + (int64_t)id_at(min(base + 8 * i + (lane >> 2), n_list - 1)) * 64) + (lane & 3));
-#pragma unroll
-      for (int i = 0; i < 2; i++)
-        in[4 + i] = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)id_at(min(base + 16 * i + (lane >> 1), n_list - 1)) * 16) + (lane & 1));
-    };
-    if (warp * 32 < n_list) fetch(warp * 32);
-#pragma unroll 1
-    for (int base = warp * 32; base < n_list; base += ROUND) {
-      __syncwarp();
-#pragma unroll
-      for (int i = 0; i < 4; i++) *reinterpret_cast<uint4*>(stage + (8 * i + (lane >> 2)) * FR_REC + (lane & 3) * 16) = in[i];
-#pragma unroll
-      for (int i = 0; i < 2; i++) *reinterpret_cast<uint4*>(stage + (16 * i + (lane >> 1)) * FR_REC + 64 + (lane & 1) * 16) = in[4 + i];
-      __syncwarp();
-      if (base + ROUND < n_list) fetch(base + ROUND);
-      uint4 rec[6];
-#pragma unroll
-      for (int i = 0; i < 6; i++) rec[i] = *reinterpret_cast<const uint4*>(stage + lane * FR_REC + i * 16);
-      const float v = rerank_pairs(rec, lev2, s_q2, qn, lane, p.c128, p.c64k);
-      const int i = base + lane;
-      if (i < n_list) {
-        const int64_t at = row_base + out_pos + i;
-        if (i < p.list_cap) sc[i] = v;
-        else p.ws_scores[at] = v;
-        if (p.scores_out) p.scores_out[at] = v;
-        if (p.cand_out) p.cand_out[at] = id_at(i);
-        const unsigned u = ord_key(v);
-        kmin = min(kmin, u), kmax = max(kmax, u);
-      }
-    }
+    rerank_list(n_list, k4, w, stage, lev2, s_q2, qn, p.c128, p.c64k, id_at, [&](int i, int k, float v) {
+      const int64_t at = row_base + out_pos + i;
+      if (i < p.list_cap) sc[i] = v;
+      else p.ws_scores[at] = v;
+      if (p.scores_out) p.scores_out[at] = v;
+      if (p.cand_out) p.cand_out[at] = k;
+      const unsigned u = ord_key(v);
+      kmin = min(kmin, u), kmax = max(kmax, u);
+    });
     if (p.fill_tail && p.scores_out && p.cand_out)
-      for (int64_t i = C_here + (int64_t)rank * FR_THREADS + tid; i < p.C; i += CS * FR_THREADS) {
+      for (int64_t i = C_here + (int64_t)rank * CH_THREADS + tid; i < p.C; i += CS * CH_THREADS) {
         p.scores_out[row_base + i] = -INFINITY;
         p.cand_out[row_base + i] = 0;
       }
@@ -376,13 +207,13 @@ struct Capacity {
 template <int CS>
 int active_clusters() {
   auto kern = retrieve_fused_kernel<CS>;
-  const int smem = FR_HIST_BYTES + LEV2_BYTES + (FR_SPAN_MAX > FR_STAGE ? FR_SPAN_MAX : FR_STAGE) + 8 * FR_LIST_MAX;
+  const int smem = CH_HIST_BYTES + LEV2_BYTES + (FR_SPAN_MAX > CH_STAGE ? FR_SPAN_MAX : CH_STAGE) + 8 * FR_LIST_MAX;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return cudaGetLastError(), 0;
   if (CS > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
     return cudaGetLastError(), 0;
   if (CS == 1) return sm_count();
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CS, 64), cfg.blockDim = dim3(FR_THREADS), cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.gridDim = dim3(CS, 64), cfg.blockDim = dim3(CH_THREADS), cfg.dynamicSmemBytes = (size_t)smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = CS, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
@@ -411,7 +242,7 @@ int span_of(int64_t N, int cs) { return (int)(((N + cs - 1) / cs + 15) / 16 * 16
 template <int CS>
 cudaError_t launch_cs(dim3 grid, size_t smem, cudaStream_t st, const FusedParams& p) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid, cfg.blockDim = dim3(FR_THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+  cfg.gridDim = grid, cfg.blockDim = dim3(CH_THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st;
   cudaLaunchAttribute attr[2];
   int n = 0;
   if (CS > 1) {
@@ -467,7 +298,7 @@ int launch_fused_retrieve(int cs, const pk_tensor* codebook, const RerankArgs& a
   int64_t list = (2 * sa.C / cs + 512 + 31) / 32 * 32;
   if (list > p.span_cap + 32) list = (p.span_cap + 63) / 32 * 32;
   p.list_cap = (int)(list < FR_LIST_MAX ? list : FR_LIST_MAX);
-  const size_t smem = (size_t)FR_HIST_BYTES + LEV2_BYTES + (p.span_cap > FR_STAGE ? p.span_cap : FR_STAGE) + 8 * (size_t)p.list_cap;
+  const size_t smem = (size_t)CH_HIST_BYTES + LEV2_BYTES + (p.span_cap > CH_STAGE ? p.span_cap : CH_STAGE) + 8 * (size_t)p.list_cap;
   const dim3 grid((unsigned)cs, (unsigned)(bs * H));
   StageTimer tm(ST_RETRIEVE, st);
   cudaError_t e = cudaErrorInvalidValue;
