@@ -1481,10 +1481,11 @@ def main():
     N = cache.cpu_valid_end[0]
     tiers, C, Kf = cache.retrieval_plan(N)
     n_rows = cfg["sink"] + cfg["local"] + cfg["interval"] // 2 + Kf
-    alg = {  # algorithmic bytes per launch (one layer, this rank's KV heads): codes + counts; candidates (selection,
-        # rerank and final top-K are one launch); rows
-        "collision": 20 * N * H,
-        "select_rerank": (4 * N + 8 * C + 106 * C + 10 * C + 8 * Kf) * H,
+    alg = {  # algorithmic bytes per launch (one layer, this rank's KV heads): the whole chain in one launch (codes and
+        # candidate records in, indices out) or, for the longest zones, codes + counts | candidates; rows
+        "retrieve": (16 * N + 96 * C + 8 * Kf) * H,
+        "collision": 17 * N * H,
+        "select_rerank": (N + 8 * C + 96 * C + 4 * C) * H,
         "attention": n_rows * 512 * H,
     }
     stages_out = {}
@@ -1496,16 +1497,17 @@ def main():
             ent["achieved_gbs"] = round(alg[name] / (us * 1e-6) / 1e9, 1)
         stages_out[name] = ent
     retrieval_us = sum(stages_out.get(s, {}).get("avg_us", 0.0) for s in
-                       ("query_prep", "rank_table", "collision", "select_rerank", "final_topk"))
+                       ("query_prep", "rank_table", "collision", "select_rerank", "final_topk", "retrieve"))
     stages_eager_us = {name: round(tot_ms * 1e3 / cnt, 3) for name, (tot_ms, cnt) in stage_eager.items()}
-    coll = stages_out.get("collision", {})
-    roofline = {"kernel": "chain_collision_kernel (query preparation + cluster ranking + weighted multi-tier collision count)",
+    chain = "retrieve" if "retrieve" in stages_out else "collision"
+    coll = stages_out.get(chain, {})
+    roofline = {"kernel": ("retrieve_fused_kernel (query preparation, collision count, candidate selection, rerank, final top-K)"
+                           if chain == "retrieve" else
+                           "collide_kernel (query preparation + cluster ranking + weighted multi-tier collision count)"),
                 "bound": "hbm",
                 "achieved": coll.get("achieved_gbs"), "peak": peak, "unit": "GB/s",
                 "frac": round(coll["achieved_gbs"] / peak, 4) if coll else None, "peak_kind": f"of {peak_kind}",
-                # DRAM bytes of one launch from the ncu capture summarised under profiles/ (16.19 B per key and head
-                # at N = 131004), scaled linearly to this run's N
-                "traffic": int(round(16.19 * N * H)), "algorithmic_bytes_per_launch": alg["collision"],
+                "algorithmic_bytes_per_launch": alg[chain],
                 # for context: the nominal HBM3e figure (the fraction that counts is the one of the measured peak)
                 "frac_of_nominal_8000_gbs": round(coll["achieved_gbs"] / 8000.0, 4) if coll else None}
     att = stages_out.get("attention", {})

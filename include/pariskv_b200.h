@@ -311,9 +311,10 @@ int pk_append_encode(const pk_tensor* k_row, const pk_tensor* v_row, const pk_te
 /* ---- the whole retrieval chain in one call ------------------------------------------------------- */
 
 /* queries -> final top-K key indices for one layer and one decode step: the body of
- * polar_cache.collision_based_topk_batch (cache_hub/polar_cache.py:1126-1162, :1207-1304), as TWO launches:
- * (1) query preparation + cluster ranking + tier table + collision count, (2) candidate selection + 4-bit rerank +
- * final top-K.
+ * polar_cache.collision_based_topk_batch (cache_hub/polar_cache.py:1126-1162, :1207-1304).
+ * Key-major views of up to 16 x 40K keys run it as ONE launch (a thread-block cluster per (batch, head)).  Everything
+ * else takes (1) query preparation + cluster ranking + tier table + collision count, (2) candidate selection + 4-bit
+ * rerank, and (3) the final top-K, a launch each.
  *   codebook / key_block_weight / key_4bit: views of the N searchable keys (as pk_collision_fused /
  *   pk_rerank); cluster_key_counts i32 [bs,H,16,256]; tier_counts host array (1..8 thresholds);
  *   C candidates, K final; final_indices i64 [bs,H,K] ascending key index.  K = 0 stops after the rerank

@@ -11,8 +11,8 @@ model runtime written for the reference decodes through it unchanged.  The body 
   zone-relative position, so record 0 is 16-byte aligned and a rerank candidate is two contiguous records.
   ``codebook_gpu / key_block_weight_gpu / key_4bit_packed_gpu`` expose them in the reference's logical
   shapes through permuted views.
-* One decode step of one layer is four launches: ``ops.append_encode`` (row append, key coding, flush),
-  ``ops.retrieve_ex`` (two launches) and ``ops.sparse_attention``.  No host synchronisation, no concatenation.
+* One decode step of one layer is three launches: ``ops.append_encode`` (row append, key coding, flush),
+  ``ops.retrieve_ex`` (one; three for the longest zones) and ``ops.sparse_attention``.  No host synchronisation, no concatenation.
 * Every position lives in device words (``_layer_state``: rows in the window, searchable keys per sample), read
   by the kernels themselves; the host keeps a mirror for its own decisions.  Launch arguments therefore never
   change: ONE captured CUDA graph serves the whole generation, flushes included.

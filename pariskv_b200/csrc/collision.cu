@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
 // prefix sums; chain.cuh), then counts its keys: one u8 per virtual key and one histogram row per block, from which
 // the selection kernel derives thresholds and output offsets.
 // What bounds it: 7 us of prologue, then the half-rate integer ALU, 28 cycles per 32 keys and SM.  8 heads x 1M keys on B200:
-// 64 us with byte tables (bank conflicts), COLL_NOW now; the codes alone take 20 at the copy rate.
+// 64 us with byte tables (bank conflicts), 35 now; the codes alone take 20 at the copy rate.
 // LAYOUT 1: key-major records; 0: plane-major ([.., 16, N], a thread owns 16 consecutive keys); 2: any strides.
 template <int LAYOUT>
 __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {

@@ -42,8 +42,8 @@ __global__ void __launch_bounds__(RR_THREADS) rerank_kernel(RerankArgs a, uint16
 // give every block the global threshold count, the tie quota and its own output offset, so the candidate
 // list comes out in ascending key order with no atomics and no second pass.
 // What bounds it: the rerank's arithmetic (chain.cuh) and the latency of histogram rows, counts and records before it.  With
-// the final top-K by the last block of a head inside it (one SM per head), 8 heads x 1M keys took 129 us on B200; SEL_NOW
-// here plus TOPK_C for the final top-K as a cluster launch.
+// the final top-K by the last block of a head inside it (one SM per head), 8 heads x 1M keys took 129 us on B200; 50
+// here plus 19 for the final top-K as a cluster launch.
 struct SelParams {
   SelectArgs s;
   int list_cap;            // candidates whose keys fit in shared memory; the others are read back from cand_out

@@ -25,7 +25,7 @@ namespace {
 
 static_assert(CH_THREADS == SEL_THREADS, "one block shape");
 constexpr int FR_LIST_MAX = 8192;           // candidates a CTA keeps in shared memory; more spill to the workspace
-constexpr int FR_SPAN_MAX = 40 * 1024;      // keys of a CTA: beyond it two launches over all SMs are faster
+constexpr int FR_SPAN_MAX = 40 * 1024;      // keys of a CTA: beyond it three launches over all SMs are faster
 constexpr int FR_WORDS = LEV2_BYTES / 8;    // ballots of the final selection, over the level table
 static_assert(FR_SPAN_MAX / 32 <= FR_WORDS, "one ballot per 32 candidates");
 static_assert(CH_HIST_BYTES >= 16 * 256 * 4 && CH_HIST_BYTES >= SEL_REGION, "the region serves three stages");

@@ -4,7 +4,7 @@
 // What bounds it: the latency of the selection's exchanges for rows of up to some 10 K elements, three to five passes over
 // a CTA's slice (shared memory where it fits) beyond.  On B200, us per launch before (a cluster kernel with five
 // bisected levels and per-thread spans; one CTA per row up to 16384 elements) -> now: 8 rows of 32768 counts, k 4096
-// 16.7 -> TOPK_A; 8 rows of 4096 scores, k 256 9.6 -> TOPK_B.
+// 16.7 -> 10.0; 8 rows of 4096 scores, k 256 9.6 -> 8.7.
 #include "cluster_select.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
