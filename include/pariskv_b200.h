@@ -207,6 +207,20 @@ int pk_adaptive_topk(const pk_tensor* sl_logits, const pk_tensor* cand_scores, f
                      float threshold, int64_t K_out, int64_t min_k, int64_t max_k,
                      const pk_tensor* adaptive_k, const pk_tensor* topk_indices, void* stream);
 
+/* The same selection for a decode step, with the window logits computed here and the scores taken as the rerank leaves
+ * them (cache_hub/polar_cache_adaptivek_varlen.py:1684-1812):
+ *   query_avg  bf16 [bs,H,128]; window_k bf16 [bs,H,>=S,128], rows contiguous and 16-byte aligned
+ *   n_window   i32 device word: window rows filled, rows beyond it get logit -inf; or NULL: all S
+ *   sl_logits  f32 [bs,H,S], OUTPUT: bf16(query_avg . row) * scale
+ *   cand_scores f32 [bs,H,C], ranked as bf16 values; logit = bf16(score) * scale
+ *   n_cand     i32 [bs,H] or NULL: candidates of a head, caps its result
+ *   n_sel      i32 [bs,H], OUTPUT: adaptive_k once more, as the attention takes it */
+int pk_adaptive_select(const pk_tensor* query_avg, const pk_tensor* window_k, const pk_tensor* n_window,
+                       const pk_tensor* sl_logits, const pk_tensor* cand_scores, const pk_tensor* n_cand, float scale,
+                       const pk_tensor* sl_vnorm, const pk_tensor* cand_indices, const pk_tensor* value_norm,
+                       float threshold, int64_t K_out, int64_t min_k, int64_t max_k, const pk_tensor* adaptive_k,
+                       const pk_tensor* topk_indices, const pk_tensor* n_sel, void* stream);
+
 /* ---- (d) rerank ------------------------------------------------------------------------------ */
 
 /* 4-bit RaBitQ rerank: module rerank.partial_rerank of cache_hub/rerank/rerank.cu:141-224

@@ -71,6 +71,7 @@ SIGNATURES = {
     "pk_collision_fused_static": (_INT, [TP, TP, TP, _I64P, _INT, TP, _VP]),
     "pk_topk": (_INT, [TP, _I64, TP, _INT, _VP]),
     "pk_final_topk": (_INT, [TP, TP, _I64, TP, _VP]),
+    "pk_adaptive_select": (_INT, [TP, TP, TP, TP, TP, TP, _F32, TP, TP, TP, _F32, _I64, _I64, _I64, TP, TP, TP, _VP]),
     "pk_adaptive_topk": (_INT, [TP, TP, _F32, TP, TP, TP, TP, _I64, _F32, _I64, _I64, _I64, TP, TP, _VP]),
     "pk_rerank": (_INT, [TP, TP, TP, TP, TP, TP, TP, TP, TP, _VP]),
     "pk_h2d_gather_kv": (_INT, [TP, TP, TP, TP, TP, _VP]),

@@ -4,14 +4,14 @@ Both variants keep all C rerank candidates, weight them by exp(logit - max) * ||
 rows, and attend the shortest benefit-ordered prefix that reaches a share `threshold` of the total benefit
 (reference: cache_hub/polar_cache_atten_value_indices_adaptive_k.py:1510-1589,
 cache_hub/polar_cache_adaptivek_varlen.py:1684-1812).  Here the selection is one kernel
-(ops.adaptive_topk), the value norms of the candidates are gathered inside it, and the attention kernel takes
-per-head row counts, so there is no host synchronisation, no index packing and no staging copy.
+(adaptive_select), which makes the window logits and gathers the value norms of the candidates itself, and the
+attention kernel takes per-head row counts, so there is no host synchronisation, no index packing and no staging copy.
 """
 import math
 
 import torch
 
-from .. import ops
+from .. import _lib, ops
 from .polar_cache import polar_cache as _base_cache
 
 
@@ -36,9 +36,15 @@ class AdaptiveKCache(_base_cache):
         self._sl_vnorm_cache = self._win_vnorm
         self.value_norm_gpu = [torch.zeros(bs, H, self.zone_capacity, dtype=torch.float32, device=dev)
                                for _ in range(self.layer_num)]
-        self.last_adaptive = None   # (adaptive_k, topk_indices, n_sel, sl_logits, cand, cand_scores) of the last compute
+        self._last_adaptive = None
         self.fixed_shapes = False   # True: capacity-shaped tensors on eager steps too (what a stream capture uses)
-        self._row_ids = torch.arange(self.window_capacity, device=dev, dtype=torch.int32)
+
+    @property
+    def last_adaptive(self):
+        """(adaptive_k, topk_indices, n_sel, sl_logits, cand, cand_scores) of the last compute, the scores as the bf16
+        values that were ranked."""
+        last = self._last_adaptive
+        return last and (*last[:5], last[5].to(torch.bfloat16))
 
     def _zone_vnorm(self, layer):
         return self.value_norm_gpu[layer]
@@ -55,7 +61,6 @@ class AdaptiveKCache(_base_cache):
         wk, wv = self.unified_keys_gpu[layer_idx], self.unified_values_gpu[layer_idx]
         # rows of the candidate lists are c_max long; a sample's own count follows from its zone length, read on the
         # device, and the rest of its row carries score -inf (no weight in the adaptive selection)
-        st = self._layer_state[layer_idx]
         _, _, ex = ops.retrieve_ex(queries, self.srht_diagonal_signs, self._mag_centers, self.codebook_gpu[layer_idx],
                                    self.key_block_weight_gpu[layer_idx], self.key_4bit_packed_gpu[layer_idx],
                                    self.cluster_key_counts_gpu[layer_idx], self._c_max, 0, kv_len=self._zone_len_dev[layer_idx],
@@ -74,28 +79,19 @@ class AdaptiveKCache(_base_cache):
         else:
             n_rows = n_win
             if equal:   # equal lengths: the lists as the reference shapes them, [bs,H,C]
-                cand, cand_scores = cand[:, :, :C].contiguous(), cand_scores[:, :, :C].contiguous()
-        cand_scores = cand_scores.to(torch.bfloat16)   # the reference ranks bf16 scores
-        # window logits: a small dense product, left to the library as the reference does
-        sl_logits = torch.einsum("bhd,bhkd->bhk", ex["query_avg"], wk[:, :, :n_rows]).to(torch.float32) * self._attn_scale
-        if fixed:
-            sl_logits = sl_logits.masked_fill(self._row_ids[:n_rows] >= st[0], float("-inf"))
+                cand, cand_scores = cand[:, :, :C], cand_scores[:, :, :C]
         K_out = min(self._max_k, C)
-        min_k = min(self._min_k, K_out)
-        adaptive_k, topk = ops.adaptive_topk(sl_logits.contiguous(), cand_scores, self._attn_scale,
-                                             self._sl_vnorm_cache[layer_idx][:, :, :n_rows], cand, None,
-                                             self.adaptive_topk_threshold, K_out,
-                                             value_norm=self.value_norm_gpu[layer_idx], sink_size=0,
-                                             min_k=max(1, min_k), max_k=max(1, K_out))
-        if fixed or not equal:   # rows longer than a sample's candidate list: its count caps what the head attends
-            adaptive_k = torch.minimum(adaptive_k, ex["n_cand"].to(adaptive_k.dtype))
-        if self._per_head:
-            n_sel = adaptive_k.to(torch.int32)
-        else:  # dense variant: every head attends the first max-over-heads rows of its own ranking
+        # rows longer than a sample's candidate list: its count caps what the head attends
+        capped = fixed or not equal
+        adaptive_k, topk, n_sel, sl_logits = _lib.native().adaptive_select(
+            ex["query_avg"], wk, self._window_rows_dev[layer_idx] if fixed else None, n_rows, cand_scores, ex["n_cand"] if capped else None,
+            self._attn_scale, self._sl_vnorm_cache[layer_idx][:, :, :n_rows], cand, self.value_norm_gpu[layer_idx],
+            self.adaptive_topk_threshold, K_out, max(1, min(self._min_k, K_out)), max(1, K_out))
+        if not self._per_head:  # dense variant: every head attends the first max-over-heads rows of its own ranking
             n_sel = adaptive_k.max().to(torch.int32).expand_as(adaptive_k).contiguous()
-            if fixed or not equal:
+            if capped:
                 n_sel = torch.minimum(n_sel, ex["n_cand"])
-        self.last_adaptive = (adaptive_k, topk, n_sel, sl_logits, cand, cand_scores)
+        self._last_adaptive = (adaptive_k, topk, n_sel, sl_logits, cand, cand_scores)
         self.last_topk_indices = topk
         if fixed:
             return self._attend(queries, wk, wv, self.window_capacity, self._store_k[layer_idx], self._store_v[layer_idx],

@@ -121,7 +121,8 @@ __device__ __forceinline__ uint32_t ord_key(float f) {
 __device__ __forceinline__ uint32_t ord_key(int32_t v) { return (uint32_t)v ^ 0x80000000u; }
 
 // exp for non-positive arguments with a fixed operation sequence (the CPU oracle runs the same
-// sequence, so both sides produce identical bits).
+// sequence, so both sides produce identical bits): Cody and Waite's two-part reduction by ln 2, then the Taylor polynomial
+// of degree 6.
 __device__ __forceinline__ float pinned_expf(float x) {
   if (x < -87.0f) return 0.0f;
   float n = rintf(__fmul_rn(x, 1.44269504088896341f));

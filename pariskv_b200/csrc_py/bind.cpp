@@ -442,6 +442,34 @@ PyObject* py_adaptive_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PK_PY_END
 }
 
+// query_avg, window_k, n_window or None, S, cand_scores, n_cand or None, scale, sl_vnorm, cand_indices, value_norm,
+// threshold, K_out, min_k, max_k -> (adaptive_k, topk_indices, n_sel, sl_logits)
+PyObject* py_adaptive_select(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (!arity(n, 14, "adaptive_select")) return nullptr;
+  PK_PY_BEGIN
+  Arg qa, wk, nw, sl, sc, nc, slv, ci, vn, ak, ti, ns;
+  at::Tensor oa, ot, os, ol;
+  double scale, thr;
+  int64_t S, K, lo, hi;
+  if (!need(a[0], &qa, CUDA) || !need(a[1], &wk, CUDA) || !take(a[2], &nw, CUDA) || !to_i64(a[3], &S) ||
+      !need(a[4], &sc, CUDA) || !take(a[5], &nc, CUDA) || !to_f64(a[6], &scale) || !need(a[7], &slv, CUDA) ||
+      !need(a[8], &ci, CUDA) || !need(a[9], &vn, CUDA) || !to_f64(a[10], &thr) || !to_i64(a[11], &K) ||
+      !to_i64(a[12], &lo) || !to_i64(a[13], &hi))
+    return nullptr;
+  const int64_t bs = qa.d.shape[0], H = qa.d.shape[1];
+  if (!output(Py_None, &ak, &oa, *qa.t, {bs, H}, at::kLong) || !output(Py_None, &ti, &ot, *qa.t, {bs, H, K}, at::kLong) ||
+      !output(Py_None, &ns, &os, *qa.t, {bs, H}, at::kInt) || !output(Py_None, &sl, &ol, *qa.t, {bs, H, S}, at::kFloat))
+    return nullptr;
+  void* st = stream_of(*qa.t);
+  const int rc = without_gil([&] {
+    return pk_adaptive_select(qa.p(), wk.p(), nw.p(), sl.p(), sc.p(), nc.p(), (float)scale, slv.p(), ci.p(), vn.p(), (float)thr, K,
+                              lo, hi, ak.p(), ti.p(), ns.p(), st);
+  });
+  if (rc) return raise(rc);
+  return Py_BuildValue("(NNNN)", give(Py_None, ak), give(Py_None, ti), give(Py_None, ns), give(Py_None, sl));
+  PK_PY_END
+}
+
 // coarse_indices, key_4bit, key_block_weight, q_blocks, q_norm, mag_centers, approx or None (made here), scores_f32,
 // v4b -> approx
 PyObject* py_rerank(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -573,6 +601,7 @@ PyMethodDef methods[] = {
     PK_METHOD("topk", py_topk),
     PK_METHOD("final_topk", py_final_topk),
     PK_METHOD("adaptive_topk", py_adaptive_topk),
+    PK_METHOD("adaptive_select", py_adaptive_select),
     PK_METHOD("rerank", py_rerank),
     PK_METHOD("h2d_gather_kv", py_h2d_gather_kv),
     PK_METHOD("qk_norm_rope", py_qk_norm_rope),
