@@ -72,8 +72,8 @@ int pk_timing_clear_graph(void);
  * dependent launch.  A kernel may then be scheduled while its predecessor on the stream still runs; it does only
  * what does not depend on earlier kernels (the collision kernel its first code loads, a projection its first weight
  * loads) and then waits for the predecessor to complete, and every kernel releases its successor only after its own
- * wait, so completion is transitive along the stream.  Off by default; with the decode step replayed as a CUDA graph
- * it measured +1.9 % tokens/s at the 128K configuration on B200. */
+ * wait, so completion is transitive along the stream.  On by default: eager decode steps of 10K-token contexts
+ * measured 207 -> 195 us on B200, and with the step replayed as a CUDA graph it is +1.9 % tokens/s at 128K. */
 int pk_set_pdl(int on);
 
 /* ---- (a) key coding ---------------------------------------------------------------------- */

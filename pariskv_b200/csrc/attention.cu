@@ -1,8 +1,8 @@
 // Split-K sparse decode attention with the UVA fetch of the selected rows fused in.
 //
-// Per (batch, KV head) the attended rows are the first n_window rows of the GPU window
-// ([sink | local | update buffer]) followed by the K selected rows of the big K/V store, which may
-// live in pinned host memory.  The rows are cut into tiles of 64; a block takes one tile, or several consecutive
+// Per (batch, KV head) the attended rows are the selected rows of the big K/V store, which may live in pinned host
+// memory, followed by the first n_window rows of the GPU window ([sink | local | update buffer]): with the selected
+// rows first, their indices can be loaded before the row counts are known.  The rows are cut into tiles of 64; a block takes one tile, or several consecutive
 // ones that it streams through two staging buffers, and stages a tile with TMA bulk copies (cp.async.bulk, one
 // 512-byte copy per selected key where its K and V rows are adjacent, completion counted on an mbarrier), so a whole
 // grid keeps megabytes outstanding on the host link.  An online softmax over the staged rows runs on the tensor
@@ -22,6 +22,7 @@ constexpr int ATT_GQ = 4;       // query heads per pass of the scalar form, and 
 // Query heads per KV head that the tensor-core form takes in its one pass: the rows 0 .. 7 of its A operand.  Batch 8 of one
 // KV head with eight query heads, 2180 rows each: 45 us a launch with the scalar form (two passes), 20 with this one.
 constexpr int ATT_MQ = 8;
+constexpr int ATT_MB = 5;       // records of a warp in flight together in the merge
 constexpr int ATT_REC = 132;    // floats per partial: o[128], m, l, pad, pad
 constexpr int ATT_WAIT_LIMIT = 4000000;  // polls of the copy barrier before giving up
 // Elements (bf16) between two staged rows [K 128 | V 128 | pad].  The tensor-core form pads a row by 16 bytes, so that
@@ -115,17 +116,24 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   const int n_groups = (int)gridDim.x, tpb = p.tiles_per_block;
   const int t_first = (int)blockIdx.x * tpb;
   const unsigned mb0 = (unsigned)__cvta_generic_to_shared(&mbar[0]);
-  pdl_wait();  // the selected indices and the per-head row counts come from the kernels before this one
-  const int64_t n_sel = p.n_sel ? min((int64_t)p.n_sel[bh], p.K) : p.K;
-  const int64_t n_window =
-      p.n_window_dev ? min(p.n_window, max((int64_t)0, (int64_t)p.n_window_dev[0] + p.n_window_add)) : p.n_window;
-  const int64_t n_rows = n_window + n_sel;
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0), "r"(ATT_THREADS) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0 + 8), "r"(ATT_THREADS) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  // index of this thread's row of tile t: loaded a tile ahead of the copy that needs it, the first with the row counts
+  auto index_of = [&](int t) -> int64_t {
+    const int64_t r = (int64_t)t * ATT_TILE + (tid >> 1);
+    return r < p.K ? p.sel[b * p.sel_b + h * p.sel_h + r] : 0;
+  };
+  pdl_wait();  // the selected indices and the per-head row counts come from the kernels before this one
+  pdl_trigger();
+  int64_t ahead = index_of(t_first);
+  const int64_t n_sel = p.n_sel ? min((int64_t)p.n_sel[bh], p.K) : p.K;
+  const int64_t n_window =
+      p.n_window_dev ? min(p.n_window, max((int64_t)0, (int64_t)p.n_window_dev[0] + p.n_window_add)) : p.n_window;
+  const int64_t n_rows = n_window + n_sel;
 
   // ---- stage a tile: thread t copies row t/2, K for even t and V for odd t; where the store keeps the V row of a
   // key right behind its K row, the even thread fetches both with one 512-byte copy (half as many requests on the
@@ -140,10 +148,10 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
     bool ok = i < tile_rows(t), paired = false;
     if (ok) {
       const int64_t r = (int64_t)t * ATT_TILE + i;
-      if (r < n_window) {
-        src = (is_v ? p.wv : p.wk) + b * p.w_b + h * p.w_h + r * p.w_l;
+      if (r >= n_sel) {
+        src = (is_v ? p.wv : p.wk) + b * p.w_b + h * p.w_h + (r - n_sel) * p.w_l;
       } else {
-        const int64_t row = p.sel[b * p.sel_b + h * p.sel_h + (r - n_window)] + p.index_offset;
+        const int64_t row = ahead + p.index_offset;
         ok = row >= 0 && row < p.cap_s;
         paired = p.kv_pair != 0;
         src = ((is_v && !paired) ? p.sv : p.sk) + b * p.s_b + h * p.s_h + (ok ? row : 0) * p.s_l;
@@ -171,6 +179,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
       }
       mbar_arrive(mb);
     }
+    ahead = index_of(t + 1);
   };
   issue(t_first, 0);
 
@@ -194,6 +203,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   };
   // Partial record of this block for up to PQ query heads from the groups' (m, l, o) in shared memory.
   auto block_partial = [&](int qg, int n_heads) {
+#pragma unroll 2
     for (int g = 0; g < n_heads; g++) {
       float M = -INFINITY;
 #pragma unroll 4
@@ -399,76 +409,80 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   }
 
   // ---- the block that arrives last for this (batch, KV head) merges all tiles ----
-  __threadfence();
   __syncthreads();
-  if (tid == 0) {
+  if (tid == 0) {   // one thread's fences order the whole block's records (the barriers carry them to and from it)
+    __threadfence();
     const unsigned prev = atomicAdd(p.counters + bh, 1u);
     s_last = prev + 1 == (unsigned)n_groups;
     if (s_last) p.counters[bh] = 0;  // ready for the next call on this stream
+    __threadfence();
   }
   __syncthreads();
   if (!s_last) return;
-  __threadfence();
-  // Up to ATT_GQ query heads are merged at a time.  Warp g takes head g: it reads the tiles' (m, l), reduces the
-  // maximum and the denominator with shuffles and leaves one scale factor per tile in shared memory; after ONE
-  // block barrier every thread sums its output dimension over the tiles for all of these heads, the loads of
-  // several tiles and heads in flight together (no serial chain of L2 round trips, no barrier per head).
-  float* s_f = obuf;                    // [ATT_GQ][1024] scale factor per tile (reuses the merge buffer)
-  __shared__ float s_L[ATT_GQ], s_M[ATT_GQ];
-  static_assert(ATT_THREADS == 32 * ATT_GQ, "one warp per query head of a group");
+  // Up to ATT_GQ query heads are merged at a time.  A warp takes every fourth record, a lane four dims of it; the
+  // records of ATT_MB steps are in flight together, (m, l) with the values, because nothing in this tail but their
+  // latency costs time: 36 records of four heads took 6.6 us with a pass for the scale factors and 16 single floats in
+  // flight per thread, 4.4 like this, and 3.7 as the 18 records of two tiles each.  The warps' sums meet in shared memory.
   const int warp = tid >> 5, lane = tid & 31;
+  static_assert(ATT_THREADS == 128, "one output dimension per thread, four record streams");
   for (int qg = 0; qg < p.n_qgroups; qg++) {
     const int n_heads = min(ATT_GQ, p.G - qg * ATT_GQ);
     const int64_t bq0 = (int64_t)b * p.Hq + h * p.G + qg * ATT_GQ;
-    if (qg) __syncthreads();            // the scale factors of the previous group have been consumed
-    if (warp < n_heads) {
-      const float* rec = p.ws + (bq0 + warp) * n_groups * ATT_REC;
-      float mloc = -INFINITY;
-      for (int64_t t = lane; t < n_groups; t += 32) {
-        const float mt = __ldcg(rec + t * ATT_REC + 128);
-        s_f[warp * 1024 + t] = mt;
-        mloc = fmaxf(mloc, mt);
-      }
+    float m[ATT_GQ], l[ATT_GQ];
+    float4 o[ATT_GQ];
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) mloc = fmaxf(mloc, __shfl_xor_sync(0xffffffffu, mloc, off));
-      float L = 0.0f;
-      for (int64_t t = lane; t < n_groups; t += 32) {
-        const float mt = s_f[warp * 1024 + t];
-        const float f = (mt == -INFINITY) ? 0.0f : exp2f(mt - mloc);
-        s_f[warp * 1024 + t] = f;
-        L += __ldcg(rec + t * ATT_REC + 129) * f;
-      }
+    for (int g = 0; g < ATT_GQ; g++) m[g] = -INFINITY, l[g] = 0.0f, o[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int t0 = warp; t0 < n_groups; t0 += 4 * ATT_MB) {
+      float4 v[ATT_MB][ATT_GQ];
+      float2 ml[ATT_MB][ATT_GQ];
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
-      if (lane == 0) s_L[warp] = L, s_M[warp] = mloc;
+      for (int i = 0; i < ATT_MB; i++)
+#pragma unroll
+        for (int g = 0; g < ATT_GQ; g++) {
+          const int t = t0 + 4 * i;
+          ml[i][g] = make_float2(-INFINITY, 0.0f), v[i][g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (t < n_groups && g < n_heads) {
+            const float* rec = p.ws + ((bq0 + g) * n_groups + t) * ATT_REC;
+            ml[i][g] = __ldcg(reinterpret_cast<const float2*>(rec + 128));
+            v[i][g] = __ldcg(reinterpret_cast<const float4*>(rec) + lane);
+          }
+        }
+#pragma unroll
+      for (int g = 0; g < ATT_GQ; g++) {
+        float mn = m[g];
+#pragma unroll
+        for (int i = 0; i < ATT_MB; i++) mn = fmaxf(mn, ml[i][g].x);
+        if (mn == -INFINITY) continue;   // no live row so far
+        const float c = exp2f(m[g] - mn);
+        m[g] = mn, l[g] *= c, o[g].x *= c, o[g].y *= c, o[g].z *= c, o[g].w *= c;
+#pragma unroll
+        for (int i = 0; i < ATT_MB; i++) {
+          const float f = exp2f(ml[i][g].x - mn);
+          l[g] += ml[i][g].y * f;
+          o[g].x += v[i][g].x * f, o[g].y += v[i][g].y * f, o[g].z += v[i][g].z * f, o[g].w += v[i][g].w * f;
+        }
+      }
+    }
+    if (qg) __syncthreads();            // the sums of the previous heads have been consumed
+#pragma unroll
+    for (int g = 0; g < ATT_GQ; g++) {
+      if (lane == 0) s_m[warp][g] = m[g], s_l[warp][g] = l[g];
+      reinterpret_cast<float4*>(obuf + (warp * ATT_GQ + g) * 128)[lane] = o[g];
     }
     __syncthreads();
-    float O[ATT_GQ];
-#pragma unroll
-    for (int g = 0; g < ATT_GQ; g++) O[g] = 0.0f;
-    const float* rec0 = p.ws + bq0 * n_groups * ATT_REC + tid;
-    int64_t t = 0;
-    for (; t + 4 <= n_groups; t += 4) {
-      float v[ATT_GQ][4];
-#pragma unroll
-      for (int g = 0; g < ATT_GQ; g++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) v[g][i] = g < n_heads ? __ldcg(rec0 + (g * n_groups + t + i) * ATT_REC) : 0.0f;
-#pragma unroll
-      for (int g = 0; g < ATT_GQ; g++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) O[g] += v[g][i] * s_f[g * 1024 + t + i];
-    }
-    for (; t < n_groups; t++)
-#pragma unroll
-      for (int g = 0; g < ATT_GQ; g++)
-        if (g < n_heads) O[g] += __ldcg(rec0 + (g * n_groups + t) * ATT_REC) * s_f[g * 1024 + t];
 #pragma unroll
     for (int g = 0; g < ATT_GQ; g++) {
       if (g >= n_heads) continue;
-      const float L = s_L[g];
-      p.out[(bq0 + g) * 128 + tid] = f2bf(L > 0.0f ? O[g] / L : 0.0f);
-      if (p.lse && tid == 0) p.lse[bq0 + g] = L > 0.0f ? s_M[g] + log2f(L) : -INFINITY;
+      const float M = fmaxf(fmaxf(s_m[0][g], s_m[1][g]), fmaxf(s_m[2][g], s_m[3][g]));
+      float L = 0.0f, O = 0.0f;
+#pragma unroll
+      for (int w = 0; w < 4; w++) {
+        const float f = s_m[w][g] == -INFINITY ? 0.0f : exp2f(s_m[w][g] - M);
+        L += s_l[w][g] * f;
+        O += obuf[(w * ATT_GQ + g) * 128 + tid] * f;
+      }
+      p.out[(bq0 + g) * 128 + tid] = f2bf(L > 0.0f ? O / L : 0.0f);
+      if (p.lse && tid == 0) p.lse[bq0 + g] = L > 0.0f ? M + log2f(L) : -INFINITY;
     }
   }
 }
@@ -575,14 +589,15 @@ extern "C" int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* wi
   p.K = K, p.index_offset = index_offset;
   p.H = (int)H, p.Hq = (int)Hq, p.G = (int)(Hq / H);
   p.n_qgroups = (p.G + ATT_GQ - 1) / ATT_GQ;
-  // Blocks per (batch, KV head): all the tiles when the launch is small (every copy of the launch outstanding at once),
+  // Blocks per (batch, KV head): one per two tiles when the launch is small (a block copies two tiles at once, so every
+  // copy of the launch is outstanding; a block per tile would only double the records that the merge reads),
   // otherwise as many as give ONE wave of three blocks per SM, each streaming several tiles.  The scalar form needs
   // the staged tile for several passes: one tile per block then.
   int64_t groups = n_tiles;
   const bool mma = p.G <= ATT_MQ;   // at most ATT_MQ query heads per KV head: one pass on the tensor cores
   if (mma) {
-    const int64_t fit = (int64_t)sm_count() * 3 / (H * bs);
-    groups = fit < 1 ? 1 : (fit < n_tiles ? fit : n_tiles);
+    const int64_t fit = (int64_t)sm_count() * 3 / (H * bs), pairs = (n_tiles + 1) / 2;
+    groups = fit < 1 ? 1 : (fit < pairs ? fit : pairs);
   }
   p.tiles_per_block = (int)((n_tiles + groups - 1) / groups);
   groups = (n_tiles + p.tiles_per_block - 1) / p.tiles_per_block;

@@ -75,7 +75,7 @@ StageTimer::~StageTimer() {
     (cap_ ? g_graph_spans : g_spans).push_back({stage_, a_, b});
 }
 
-static std::atomic<int> g_pdl{0};  // off unless asked for: measured neutral when the step is replayed as a graph
+static std::atomic<int> g_pdl{1};
 bool pdl_enabled() { return g_pdl.load(std::memory_order_relaxed) != 0; }
 
 static std::mutex g_dev_mu;
