@@ -10,45 +10,37 @@ namespace {
 // byte k (0..3) of w, zero-extended: one PRMT
 __device__ __forceinline__ unsigned byte_of(uint32_t w, int k) { return __byte_perm(w, 0, 0x4440 | k); }
 
-// Sorts the 256 keys of a warp (8 per lane, element index e = 8 * lane + r) into DESCENDING order of e with a
-// bitonic network: exchanges at distance < 8 stay inside a lane, the others are xor shuffles.  Keys are distinct.
-// The merges run as loops over two small bodies: fully unrolled the network is 1500 instructions that every warp runs
+// Sorts the 128 keys of a warp (4 per lane, element index e = 4 * lane + r) into DESCENDING order of e with a
+// bitonic network: exchanges at distance < 4 stay inside a lane, the others are xor shuffles.  Keys are distinct.
+// The merges run as loops over two small bodies: fully unrolled the network is long code that every warp runs
 // once, and a kernel that starts with it waits for instruction fetches (a third of its stalls, measured).
 // A block that has to end ascending is sorted as complements, so every exchange inside a lane is one max and one min.
-__device__ __forceinline__ void lane_exchange(unsigned (&v)[8], int r, int l, bool up) {
+__device__ __forceinline__ void lane_exchange(unsigned (&v)[4], int r, int l, bool up) {
   const unsigned a = v[r], b = v[l], mx = max(a, b), mn = min(a, b);
   v[r] = up ? mx : mn;
   v[l] = up ? mn : mx;
 }
-__device__ __forceinline__ void warp_sort_desc_256(unsigned (&v)[8], int lane) {
-#pragma unroll
-  for (int k = 2; k <= 4; k <<= 1)
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1)
-#pragma unroll
-      for (int r = 0; r < 8; r++)
-        if ((r ^ j) > r) lane_exchange(v, r, r ^ j, (r & k) == 0);
+__device__ __forceinline__ void warp_sort_desc_128(unsigned (&v)[4], int lane) {
+  lane_exchange(v, 0, 1, true);
+  lane_exchange(v, 2, 3, false);
 #pragma unroll 1
-  for (int k = 8; k <= 256; k <<= 1) {
-    const unsigned flip = ((lane << 3) & k) ? 0xffffffffu : 0u;   // blocks with this bit set end ascending
+  for (int k = 4; k <= 128; k <<= 1) {
+    const unsigned flip = ((lane << 2) & k) ? 0xffffffffu : 0u;   // blocks with this bit set end ascending
 #pragma unroll
-    for (int r = 0; r < 8; r++) v[r] ^= flip;
+    for (int r = 0; r < 4; r++) v[r] ^= flip;
 #pragma unroll 1
-    for (int lj = k >> 4; lj > 0; lj >>= 1) {
+    for (int lj = k >> 3; lj > 0; lj >>= 1) {
       const bool take_max = (lane & lj) == 0;   // the lower element of a pair keeps the maximum
 #pragma unroll
-      for (int r = 0; r < 8; r++) {
+      for (int r = 0; r < 4; r++) {
         const unsigned o = __shfl_xor_sync(0xffffffffu, v[r], lj);
         v[r] = take_max ? max(v[r], o) : min(v[r], o);
       }
     }
+    lane_exchange(v, 0, 2, true), lane_exchange(v, 1, 3, true);
+    lane_exchange(v, 0, 1, true), lane_exchange(v, 2, 3, true);
 #pragma unroll
-    for (int j = 4; j > 0; j >>= 1)
-#pragma unroll
-      for (int r = 0; r < 8; r++)
-        if ((r ^ j) > r) lane_exchange(v, r, r ^ j, true);
-#pragma unroll
-    for (int r = 0; r < 8; r++) v[r] ^= flip;
+    for (int r = 0; r < 4; r++) v[r] ^= flip;
   }
 }
 
@@ -83,10 +75,14 @@ __device__ __forceinline__ float rotate4(float (&x)[4], const float (&sg)[4], in
 }
 
 // Ranks the 256 clusters of a subspace by (score descending, id ascending), the scores being the sums of +-q over the
-// bits of the cluster id: on return element e = 8 * lane + r of the order is cluster 255 - (key[r] & 255).
+// bits of the cluster id.  The complement of an id has exactly the negated score, so the order is its own mirror image:
+// with a cluster at position e its complement is at position 255 - e, ties included (equal scores are ascending in the ids,
+// their negatives in the complements read backwards; of the scores that are zero the ids below 128 come first).  Only the
+// first 128 positions are sorted, one cluster of every pair: that of the positive score, or the lower id.  On return
+// position e = 4 * lane + r is cluster 255 - (key[r] & 255), position 255 - e cluster key[r] & 255.
 // Register r of a lane starts with cluster c = 32 * r + lane: the first five terms of the score (bits 0..4 of c) are the
-// lane's, the last three (bits 5..7) the register's; the sum is taken in the order j = 0..7.
-__device__ __forceinline__ void rank_subspace(unsigned (&key)[8], const float* q8, int lane) {
+// lane's, the next two the register's, bit 7 is clear; the sum is taken in the order j = 0..7.
+__device__ __forceinline__ void rank_subspace(unsigned (&key)[4], const float* q8, int lane) {
   float qv[8];
 #pragma unroll
   for (int j = 0; j < 8; j++) qv[j] = q8[j];
@@ -94,17 +90,15 @@ __device__ __forceinline__ void rank_subspace(unsigned (&key)[8], const float* q
 #pragma unroll
   for (int j = 0; j < 5; j++) s5 = __fadd_rn(s5, ((lane >> j) & 1) ? qv[j] : -qv[j]);
 #pragma unroll
-  for (int rr = 0; rr < 8; rr++) {
+  for (int rr = 0; rr < 4; rr++) {
     float sc = s5;
 #pragma unroll
-    for (int j = 5; j < 8; j++) sc = __fadd_rn(sc, ((rr >> (j - 5)) & 1) ? qv[j] : -qv[j]);
-    // order of (score descending, id ascending) as one unsigned compare; -0 counts as +0 like a float compare
-    unsigned bits = f2bf(sc);
-    if (bits == 0x8000u) bits = 0u;
-    const unsigned ord = (bits & 0x8000u) ? (~bits & 0xFFFFu) : (bits | 0x8000u);
-    key[rr] = (ord << 8) | (unsigned)(255 - (32 * rr + lane));
+    for (int j = 5; j < 7; j++) sc = __fadd_rn(sc, ((rr >> (j - 5)) & 1) ? qv[j] : -qv[j]);
+    const unsigned bits = f2bf(__fadd_rn(sc, -qv[7])), mag = bits & 0x7fffu;   // a zero of either sign counts as positive
+    const unsigned c = 32 * rr + lane, id = (bits & 0x8000u) && mag ? 255u - c : c;
+    key[rr] = (mag << 8) | (255u - id);
   }
-  warp_sort_desc_256(key, lane);
+  warp_sort_desc_128(key, lane);
 }
 
 // Sixteen times the sum over the 16 subspaces of a key of the tier count of its code.  lut: [16][128] bytes, entry c of a
@@ -283,19 +277,37 @@ constexpr int CH_STAGE = CH_WARPS * 32 * CH_REC;
 struct PreparedQuery {
   float x[4], avg[4], n;   // warp 0: the lane's dimensions of the rotated and of the mean query, the norm
 };
+// What warp 0 reads for it, issued ahead of everything that waits: eight queries of the group, the signs.
+struct QueryLoads {
+  uint2 raw[8], signs;
+};
+__device__ __forceinline__ void load_queries(QueryLoads& ql, const ChainQuery& cq, int b, int h, int G, int g0) {
+  const uint16_t* q = cq.queries + ((int64_t)b * cq.Hq + (int64_t)h * G) * 128 + 4 * (threadIdx.x & 31);
+#pragma unroll
+  for (int k = 0; k < 8; k++) ql.raw[k] = __ldg(reinterpret_cast<const uint2*>(q + min(g0 + k, G - 1) * 128));
+}
+__device__ __forceinline__ void load_query(QueryLoads& ql, const ChainQuery& cq, int b, int h, int G) {
+  if (threadIdx.x >= 32) return;
+  load_queries(ql, cq, b, h, G, 0);
+  ql.signs = __ldg(reinterpret_cast<const uint2*>(cq.signs + 4 * threadIdx.x));
+}
 // Warp 0 averages the group's queries, normalises and rotates the mean into s_q.
-__device__ __forceinline__ void prepare_query(PreparedQuery& pq, const ChainQuery& cq, int b, int h, int G, float inv_g,
-                                              float* s_q, float* s_qnorm) {
+__device__ __forceinline__ void prepare_query(PreparedQuery& pq, QueryLoads& ql, const ChainQuery& cq, int b, int h, int G,
+                                              float inv_g, float* s_q, float* s_qnorm) {
   const int lane = threadIdx.x & 31;
   if (threadIdx.x >= 32) return;
-  const uint16_t* q = cq.queries + ((int64_t)b * cq.Hq + (int64_t)h * G) * 128 + 4 * lane;
   float sg[4], acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  unpack4(__ldg(reinterpret_cast<const uint2*>(cq.signs + 4 * lane)), sg);
-  for (int g = 0; g < G; g++) {  // fp32 sum over the group, g ascending
-    float v[4];
-    unpack4(__ldg(reinterpret_cast<const uint2*>(q + g * 128)), v);
+  unpack4(ql.signs, sg);
+  for (int g0 = 0; g0 < G; g0 += 8) {  // fp32 sum over the group, g ascending
+    if (g0) load_queries(ql, cq, b, h, G, g0);
 #pragma unroll
-    for (int i = 0; i < 4; i++) acc[i] = __fadd_rn(acc[i], v[i]);
+    for (int k = 0; k < 8; k++) {
+      if (g0 + k >= G) break;
+      float v[4];
+      unpack4(ql.raw[k], v);
+#pragma unroll
+      for (int i = 0; i < 4; i++) acc[i] = __fadd_rn(acc[i], v[i]);
+    }
   }
 #pragma unroll
   for (int i = 0; i < 4; i++) pq.x[i] = pq.avg[i] = bfround(__fmul_rn(acc[i], inv_g));
@@ -326,32 +338,37 @@ __device__ __forceinline__ void load_tiers(const ChainQuery& cq, long long N, un
 }
 // Tier table of one subspace by its warp.  sizes: 256 words with the cluster sizes (overwritten); key: the order made by
 // rank_subspace; lut: the subspace's 128 bytes (see tier_sum16).
-__device__ __forceinline__ void tier_table(const unsigned (&key)[8], unsigned* sizes, const unsigned* s_tiers, uint8_t* lut) {
+__device__ __forceinline__ void tier_table(const unsigned (&key)[4], unsigned* sizes, const unsigned* s_tiers, uint8_t* lut) {
   const int lane = threadIdx.x & 31;
   const int n_tiers = (int)s_tiers[8];
-  unsigned tier[8], cnt[8], run = 0;
+  unsigned tier[8], front[4], back[4], n_front = 0, n_back = 0;
 #pragma unroll
   for (int t = 0; t < 8; t++) tier[t] = t < n_tiers ? s_tiers[t] : 0u;
 #pragma unroll
-  for (int rr = 0; rr < 8; rr++) {
-    cnt[rr] = sizes[255u - (key[rr] & 255u)];
-    run += cnt[rr];
+  for (int r = 0; r < 4; r++) {   // sizes at positions e and 255 - e
+    const unsigned id = key[r] & 255u;
+    front[r] = sizes[255u - id], back[r] = sizes[id];
+    n_front += front[r], n_back += back[r];
   }
-  unsigned incl = run;
+  unsigned inc_f = n_front, inc_b = n_back;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const unsigned o = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += o;
+    const unsigned f = __shfl_up_sync(0xffffffffu, inc_f, off), g = __shfl_up_sync(0xffffffffu, inc_b, off);
+    if (lane >= off) inc_f += f, inc_b += g;
   }
-  unsigned excl = incl - run;
+  // keys before position e, and up to position 255 - e
+  unsigned before = inc_f - n_front;
+  unsigned upto = __shfl_sync(0xffffffffu, inc_f, 31) + __shfl_sync(0xffffffffu, inc_b, 31) - (inc_b - n_back);
   __syncwarp();   // the sizes have been read: the same words take the tier counts, packed to nibbles below
 #pragma unroll
-  for (int rr = 0; rr < 8; rr++) {
-    unsigned wgt = 0;
+  for (int r = 0; r < 4; r++) {
+    const unsigned id = key[r] & 255u;
+    unsigned wf = 0, wb = 0;
+    upto -= back[r];   // keys before position 255 - e
 #pragma unroll
-    for (int t = 0; t < 8; t++) wgt += (excl < tier[t]) ? 1u : 0u;   // absent tiers are 0: never above a prefix sum
-    sizes[255u - (key[rr] & 255u)] = wgt;
-    excl += cnt[rr];
+    for (int t = 0; t < 8; t++) wf += (before < tier[t]) ? 1u : 0u, wb += (upto < tier[t]) ? 1u : 0u;   // absent tiers are 0: never above a prefix sum
+    sizes[255u - id] = wf, sizes[id] = wb;
+    before += front[r];
   }
   __syncwarp();
   // entries i (low nibble) and i + 128 of byte i: four bytes per lane
@@ -360,9 +377,9 @@ __device__ __forceinline__ void tier_table(const unsigned (&key)[8], unsigned* s
       (e0.x | (e1.x << 4)) | ((e0.y | (e1.y << 4)) << 8) | ((e0.z | (e1.z << 4)) << 16) | ((e0.w | (e1.w << 4)) << 24);
 }
 
-// Ordered candidate list of a block's n_keys counts (cnt8, overwritten; the first `skip` < 16 are not keys): those above T, and ties at T while the zone-wide
-// quota lasts, of which lower blocks have met eq_base.  put(position, offset of the key) for positions below `limit`;
-// returns the length of the list.  warp_a / warp_b: CH_WARPS words of scratch.
+// Ordered candidate list of a block's n_keys counts (cnt8, overwritten; the first `skip` < 16 are not keys): those above
+// T, and ties at T while the zone-wide quota lasts, of which lower blocks have met eq_base.  put(position, offset of the
+// key) for positions below `limit`; returns the length of the list.  warp_a / warp_b: CH_WARPS words of scratch.
 template <class Put>
 __device__ __forceinline__ int list_candidates(uint8_t* cnt8, int n_keys, int skip, unsigned T, unsigned quota,
                                                unsigned eq_base, int64_t limit, unsigned* warp_a, unsigned* warp_b, Put put) {

@@ -11,6 +11,8 @@
 #pragma once
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace pk {
@@ -49,6 +51,19 @@ struct SelShared {               // static: what other CTAs of the cluster read,
   unsigned warp_a[SEL_WARPS], warp_b[SEL_WARPS];
   unsigned sub[SEL_SUB], n_few;
 };
+
+// Cluster sizes that kernels are built for.  A cluster lies within one GPC; with a CTA per SM 148 / 74 / 45 / 33 / 26 /
+// 22 / 15 / 11 / 7 of these sizes are resident at once on B200, and no size above 10 does better than 7.
+constexpr int CLUSTER_SIZES[] = {1, 2, 3, 4, 5, 6, 8, 10, 16};
+constexpr int N_CLUSTER_SIZES = sizeof(CLUSTER_SIZES) / sizeof(int);
+// f(integral_constant<int, cs>) for a size of the table.
+template <int I = 0, class F>
+void with_cluster_size(int cs, F&& f) {
+  if constexpr (I < N_CLUSTER_SIZES) {
+    if (CLUSTER_SIZES[I] == cs) f(std::integral_constant<int, CLUSTER_SIZES[I]>());
+    else with_cluster_size<I + 1>(cs, f);
+  }
+}
 
 template <int CS>
 __device__ __forceinline__ void sync_cluster(cg::cluster_group& cluster) {
@@ -231,7 +246,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       }
       n_all = min(__shfl_sync(0xffffffffu, inc, CS - 1), (unsigned)SEL_TIES);
       before_me = __shfl_sync(0xffffffffu, inc - m, rank);
-      const unsigned off = __shfl_sync(0xffffffffu, inc - m, warp & (CS - 1)), c = __shfl_sync(0xffffffffu, m, warp & (CS - 1));
+      const unsigned off = __shfl_sync(0xffffffffu, inc - m, warp), c = __shfl_sync(0xffffffffu, m, warp);
       if (warp < CS) {   // warp w copies rank w's members
         const uint2* src = cluster.map_shared_rank(own, warp);
         for (unsigned i = lane; i < c && off + i < (unsigned)SEL_TIES; i += 32) all[off + i] = src[i];

@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
 template <int LAYOUT>
 __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
   __shared__ __align__(16) uint8_t s_lut[16 * 128];
-  __shared__ __align__(16) unsigned region[CH_HIST_BYTES / 4];   // cluster sizes, then the count histogram
+  __shared__ __align__(16) unsigned region[CH_HIST_BYTES / 4];   // count histogram
+  __shared__ __align__(16) unsigned s_sizes[16 * 256];           // cluster sizes, then tier counts
   __shared__ __align__(16) float s_q[128];
   __shared__ float s_qnorm;
   __shared__ unsigned s_tiers[9];
@@ -315,10 +316,12 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
   const int bh = blockIdx.y, b = bh / p.H, h = bh % p.H;
   const ChainQuery& cq = p.q;
   PreparedQuery pq;
-  unsigned key[8];
+  QueryLoads ql;
+  unsigned key[4];
   const bool early = cq.early_query != 0;
   if (early) {   // the queries were complete before the kernel before this one started
-    prepare_query(pq, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
+    load_query(ql, cq, b, h, p.G);
+    prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     __syncthreads();
     rank_subspace(key, s_q + warp * 8, lane);
   }
@@ -348,20 +351,20 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
   }
   pdl_wait();
   pdl_trigger();
+  if (!early) load_query(ql, cq, b, h, p.G);
   {
     const int4* cp = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
     const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1);   // cluster sizes of this warp's subspace
-    unsigned* my = region + warp * 256;
-    if (!early) prepare_query(pq, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
+    unsigned* my = s_sizes + warp * 256;
+    if (!early) prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     if (warp == 0 && blockIdx.x == 0) publish_query(pq, cq, bh);
     if (tid == 32) load_tiers(cq, cq.n_dev || cq.n_plan <= 0 ? (long long)N : cq.n_plan, s_tiers);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
     *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
+    for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
     __syncthreads();
     if (!early) rank_subspace(key, s_q + warp * 8, lane);
     tier_table(key, my, s_tiers, s_lut + warp * 128);
-    __syncthreads();
-    for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
     __syncthreads();
   }
   if (LAYOUT == 1) {

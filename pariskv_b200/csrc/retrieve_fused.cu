@@ -10,9 +10,10 @@
 //
 // Why this split: as two launches (count | select + rerank + final top-K by the last block of a head) the final stage ran
 // on one SM per head, 12 us of 48 at 128K keys, and counts and scores went through L2.  Time line of a CTA on B200
-// (8 heads x 131004 keys, 8 CTAs each): query and ranking 7 us, counting 16 K keys 9, threshold and list 2.7, rerank of
-// 1640 candidates 9.4, final selection 9.  Graph-replayed layer step, start -> now: 16 sequences of 16 - 32K keys
-// (one CTA per head, no exchange at all) 155 -> 123 us, 8 heads x 128K keys 70 -> 68, 10K keys 27 -> 20 for the chain.
+// (8 heads x 131004 keys, 10 CTAs each): query and ranking 6 us, counting 13 K keys 7.4, threshold and list 2.8, rerank
+// of 1310 candidates 8.2, final selection 8.6: 33 us (39 with 8 CTAs, all 256 clusters sorted, and one load waiting for
+// the other in the prologue).  Graph-replayed layer step, two launches -> one: 16 sequences of 16 - 32K keys
+// (one CTA per head, no exchange at all) 155 -> 116 us, 8 heads x 128K keys 70 -> 60, 10K keys 27 -> 19 for the chain.
 // What bounds it: the serial chain of exchanges for small zones, instruction issue (look-ups 85 instructions per key and
 // warp, rerank 420 per candidate and warp) for long ones; codes and records stream at under half of the HBM rate.
 #include "chain.cuh"
@@ -28,7 +29,7 @@ constexpr int FR_LIST_MAX = 8192;           // candidates a CTA keeps in shared 
 constexpr int FR_SPAN_MAX = 40 * 1024;      // keys of a CTA: beyond it three launches over all SMs are faster
 constexpr int FR_WORDS = LEV2_BYTES / 8;    // ballots of the final selection, over the level table
 static_assert(FR_SPAN_MAX / 32 <= FR_WORDS, "one ballot per 32 candidates");
-static_assert(CH_HIST_BYTES >= 16 * 256 * 4 && CH_HIST_BYTES >= SEL_REGION, "the region serves three stages");
+static_assert(CH_HIST_BYTES >= SEL_REGION && CH_STAGE >= 16 * 256 * 4, "areas that serve two stages");
 
 struct FusedParams {
   const uint8_t* codes;   // key-major records of 16 bytes; (b,h) at b*c_b + h*c_h
@@ -73,15 +74,25 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   const int b = (int)(bh / p.H), h = (int)(bh % p.H);
   const ChainQuery& cq = p.q;
   PreparedQuery pq;
-  unsigned key[8];
+  QueryLoads ql;
+  unsigned key[4];
+  // before the wait: what no kernel of the chain writes
+  build_lev2(lev2, p.a.centers, tid, CH_THREADS);
+  for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
   const bool early = cq.early_query != 0;
   if (early) {   // the queries were complete before the kernel before this one started
-    prepare_query(pq, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
+    load_query(ql, cq, b, h, p.G);
+    prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     __syncthreads();
     rank_subspace(key, s_q + warp * 8, lane);
   }
   pdl_wait();
   pdl_trigger();
+  // a word written by the kernel before this one takes over a microsecond to arrive: the queries, the cluster sizes and
+  // the zone length are asked for together
+  if (!early) load_query(ql, cq, b, h, p.G);
+  const int4* sizes = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
+  const int4 c0 = __ldg(sizes), c1 = __ldg(sizes + 1);   // of this warp's subspace
   const int64_t N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
   const int64_t C_want = cq.n_dev ? min((int64_t)zone_candidates(cq.sched, N), p.C) : p.C_want;
   const int span = (int)(((N + CS - 1) / CS + 15) / 16 * 16);
@@ -102,22 +113,17 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   load_codes(r0, warp * 128 + lane);
   load_codes(r1, warp * 128 + lane + STEP);
   {
-    const int4* cp = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
-    const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1);   // cluster sizes of this warp's subspace
-    unsigned* my = region + warp * 256;
-    if (!early) prepare_query(pq, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
+    unsigned* my = reinterpret_cast<unsigned*>(cnt8) + warp * 256;   // the counts are not there yet
+    if (!early) prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     if (warp == 0 && rank == 0) publish_query(pq, cq, bh);
     if (tid == 32) load_tiers(cq, (long long)N, s_tiers);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
     *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
-    build_lev2(lev2, p.a.centers, tid, CH_THREADS);
     __syncthreads();
     if (!early) rank_subspace(key, s_q + warp * 8, lane);
     tier_table(key, my, s_tiers, s_lut + warp * 128);
     if (tid < 128) reinterpret_cast<float*>(s_q2)[pair_slot(tid)] = s_q[tid];
-    __syncthreads();   // the tables are complete and the staging area is free again
-    for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
-    __syncthreads();
+    __syncthreads();   // the tables are complete, the sizes are done with
   }
   const float qn = s_qnorm;
 
@@ -199,9 +205,9 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   if (CS > 1) cluster.barrier_wait();   // shared memory must outlive the other CTAs' reads
 }
 
-// Largest clusters that fit the device at once, per cluster size 1, 2, 4, 8, 16 (0: the size cannot be launched).
+// Clusters that fit the device at once, per size in CLUSTER_SIZES (0: the size cannot be launched).
 struct Capacity {
-  int active[5];
+  int active[N_CLUSTER_SIZES];
 };
 
 template <int CS>
@@ -230,8 +236,8 @@ const Capacity* capacity() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   if (const unsigned long long bit = first_on_device(asked)) {
-    const Capacity c = {{active_clusters<1>(), active_clusters<2>(), active_clusters<4>(), active_clusters<8>(), active_clusters<16>()}};
-    cap[dev] = c;   // several threads may ask at the same time: they write the same numbers
+    for (int i = 0; i < N_CLUSTER_SIZES; i++)   // several threads may ask at the same time: they write the same numbers
+      with_cluster_size(CLUSTER_SIZES[i], [&](auto cs) { cap[dev].active[i] = active_clusters<cs.value>(); });
     mark_on_device(asked, bit);
   }
   return &cap[dev];
@@ -273,8 +279,8 @@ int fused_cluster_size(const pk_tensor* codebook, const RerankArgs& a, int64_t b
   if (!cap) return 0;
   int best = 0;
   double best_us = 0.0;
-  for (int i = 0; i < 5; i++) {
-    const int cs = 1 << i;
+  for (int i = 0; i < N_CLUSTER_SIZES; i++) {
+    const int cs = CLUSTER_SIZES[i];
     if (cap->active[i] <= 0 || span_of(N, cs) > FR_SPAN_MAX) continue;
     const double waves = (double)((bs_h + cap->active[i] - 1) / cap->active[i]);
     const double us = waves * (15.0 + (0.0005 * (double)N + 0.0045 * (double)C) / cs);
@@ -302,13 +308,7 @@ int launch_fused_retrieve(int cs, const pk_tensor* codebook, const RerankArgs& a
   const dim3 grid((unsigned)cs, (unsigned)(bs * H));
   StageTimer tm(ST_RETRIEVE, st);
   cudaError_t e = cudaErrorInvalidValue;
-  switch (cs) {
-    case 1: e = launch_cs<1>(grid, smem, st, p); break;
-    case 2: e = launch_cs<2>(grid, smem, st, p); break;
-    case 4: e = launch_cs<4>(grid, smem, st, p); break;
-    case 8: e = launch_cs<8>(grid, smem, st, p); break;
-    case 16: e = launch_cs<16>(grid, smem, st, p); break;
-  }
+  with_cluster_size(cs, [&](auto c) { e = launch_cs<c.value>(grid, smem, st, p); });
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(PK_ERR_CUDA, "retrieve: %s", cudaGetErrorString(e));

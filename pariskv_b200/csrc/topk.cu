@@ -93,7 +93,7 @@ int topk_active() {   // clusters that fit the device at once; also opts in to t
   return n;
 }
 struct TopkCapacity {
-  int active[5];   // cluster sizes 1, 2, 4, 8, 16
+  int active[N_CLUSTER_SIZES];
 };
 template <class Row>
 const TopkCapacity* topk_capacity() {
@@ -102,9 +102,8 @@ const TopkCapacity* topk_capacity() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   if (const unsigned long long bit = first_on_device(asked)) {
-    const TopkCapacity c = {{topk_active<1, Row>(), topk_active<2, Row>(), topk_active<4, Row>(), topk_active<8, Row>(),
-                             topk_active<16, Row>()}};
-    cap[dev] = c;   // several threads may ask at the same time: they write the same numbers
+    for (int i = 0; i < N_CLUSTER_SIZES; i++)   // several threads may ask at the same time: they write the same numbers
+      with_cluster_size(CLUSTER_SIZES[i], [&](auto cs) { cap[dev].active[i] = topk_active<cs.value, Row>(); });
     mark_on_device(asked, bit);
   }
   return &cap[dev];
@@ -136,8 +135,9 @@ int launch_rows(TopkParams p, int64_t rows, cudaStream_t st) {
   if (!cap) return fail(PK_ERR_CUDA, "topk: cannot identify the device");
   // CTAs per row: as many as are resident at once with at least 512 elements each (less does not pay for the exchanges);
   // a CTA numbers its elements with 27 bits
-  int best = 0, cs = 1;
-  for (int i = 0; i < 5; i++, cs <<= 1) {
+  int best = 0;
+  for (int i = 0; i < N_CLUSTER_SIZES; i++) {
+    const int cs = CLUSTER_SIZES[i];
     if (cap->active[i] <= 0) continue;
     const bool fits = rows <= cap->active[i] && p.L >= 512LL * cs;
     if (best == 0 || fits || (p.L + best - 1) / best >= (1LL << 27)) best = cs;
@@ -154,13 +154,7 @@ int launch_rows(TopkParams p, int64_t rows, cudaStream_t st) {
     if (q.n_dev) q.n_dev += r0;
     if (q.n_out) q.n_out += r0;
     cudaError_t e = cudaErrorInvalidValue;
-    switch (best) {
-      case 1: e = launch_topk_cs<1, Row>(nr, smem, st, q); break;
-      case 2: e = launch_topk_cs<2, Row>(nr, smem, st, q); break;
-      case 4: e = launch_topk_cs<4, Row>(nr, smem, st, q); break;
-      case 8: e = launch_topk_cs<8, Row>(nr, smem, st, q); break;
-      case 16: e = launch_topk_cs<16, Row>(nr, smem, st, q); break;
-    }
+    with_cluster_size(best, [&](auto c) { e = launch_topk_cs<c.value, Row>(nr, smem, st, q); });
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(PK_ERR_CUDA, "topk: %s", cudaGetErrorString(e));
