@@ -16,13 +16,11 @@
 namespace pk {
 namespace {
 
-constexpr int ATT_THREADS = 128;
-constexpr int ATT_TILE = 64;
+constexpr int ATT_TILE = 64;    // rows of a tile of the streaming form
 constexpr int ATT_GQ = 4;       // query heads per pass of the scalar form, and per step of the merge
 // Query heads per KV head that the tensor-core form takes in its one pass: the rows 0 .. 7 of its A operand.  Batch 8 of one
 // KV head with eight query heads, 2180 rows each: 45 us a launch with the scalar form (two passes), 20 with this one.
 constexpr int ATT_MQ = 8;
-constexpr int ATT_MB = 5;       // records of a warp in flight together in the merge
 constexpr int ATT_REC = 132;    // floats per partial: o[128], m, l, pad, pad
 constexpr int ATT_WAIT_LIMIT = 4000000;  // polls of the copy barrier before giving up
 // Elements (bf16) between two staged rows [K 128 | V 128 | pad].  The tensor-core form pads a row by 16 bytes, so that
@@ -97,18 +95,24 @@ __device__ __forceinline__ void mbar_arrive_expect(unsigned mb, unsigned bytes) 
 // fragments ARE the A fragments of P for O[head][dim] += P V (sixteen n-tiles over the 128 dims), V^T comes from
 // ldmatrix.trans.  The probabilities are rounded to bf16 for the second product, as the reference's attention
 // library does.
-template <bool MMA>
-__global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttParams p) {
+//
+// WARPS: a warp takes 16 rows of a tile.  Four: the streaming form.  Eight: launches that are one tile of 128 rows per
+// SM at most; there only latency counts: the same number of records, but one tile instead of two in a row, and twice the
+// warps to merge them.  8 heads of 2180 rows in HBM: 9.8 -> 9.3 us alone and 61 -> 58 us for the layer step in a graph;
+// batch 8 of one KV head with eight query heads 60 -> 53 us for the step.
+template <bool MMA, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attention_kernel(AttParams p) {
+  constexpr int THREADS = 32 * WARPS, TILE = 16 * WARPS, NBUF = WARPS > 4 ? 1 : 2;   // one buffer: one tile per block
   constexpr int RS = AttRow<MMA>::stride;  // elements per staged row
   extern __shared__ __align__(128) unsigned char dyn[];
   uint16_t* KVs = reinterpret_cast<uint16_t*>(dyn);                          // [2 buffers][64][RS]: K row, V row of a key
   constexpr int PQ = MMA ? ATT_MQ : ATT_GQ;   // query heads of a pass
-  constexpr int PG = MMA ? ATT_THREADS / 32 : 16;   // groups of a block that hold partials of them
-  float* obuf = reinterpret_cast<float*>(dyn + 2 * ATT_TILE * RS);           // [PG][PQ][128], over the SECOND buffer:
+  constexpr int PG = MMA ? WARPS : 16;   // groups of a block that hold partials of them
+  float* obuf = reinterpret_cast<float*>(dyn + (NBUF - 1) * 2 * TILE * RS);  // [PG][PQ][128], over the LAST buffer:
                                                                              // used when that buffer is idle
   __shared__ __align__(8) unsigned long long mbar[2];
   __shared__ float s_m[PG][PQ], s_l[PG][PQ];
-  __shared__ unsigned char s_valid[2][ATT_TILE];
+  __shared__ unsigned char s_valid[NBUF][TILE];
   __shared__ int s_last;
   const int tid = threadIdx.x;
   const int h = blockIdx.y, b = blockIdx.z;
@@ -117,14 +121,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   const int t_first = (int)blockIdx.x * tpb;
   const unsigned mb0 = (unsigned)__cvta_generic_to_shared(&mbar[0]);
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0), "r"(ATT_THREADS) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0 + 8), "r"(ATT_THREADS) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0), "r"(THREADS) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0 + 8), "r"(THREADS) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
   // index of this thread's row of tile t: loaded a tile ahead of the copy that needs it, the first with the row counts
   auto index_of = [&](int t) -> int64_t {
-    const int64_t r = (int64_t)t * ATT_TILE + (tid >> 1);
+    const int64_t r = (int64_t)t * TILE + (tid >> 1);
     return r < p.K ? p.sel[b * p.sel_b + h * p.sel_h + r] : 0;
   };
   pdl_wait();  // the selected indices and the per-head row counts come from the kernels before this one
@@ -139,7 +143,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   // key right behind its K row, the even thread fetches both with one 512-byte copy (half as many requests on the
   // host link).  Every thread arrives on the tile's barrier exactly once, the copying ones with their byte count ----
   auto tile_rows = [&](int t) -> int {
-    return (int)max((int64_t)0, min((int64_t)ATT_TILE, n_rows - (int64_t)t * ATT_TILE));
+    return (int)max((int64_t)0, min((int64_t)TILE, n_rows - (int64_t)t * TILE));
   };
   auto issue = [&](int t, int buf) {
     const int i = tid >> 1;
@@ -147,7 +151,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
     const uint16_t* src = nullptr;
     bool ok = i < tile_rows(t), paired = false;
     if (ok) {
-      const int64_t r = (int64_t)t * ATT_TILE + i;
+      const int64_t r = (int64_t)t * TILE + i;
       if (r >= n_sel) {
         src = (is_v ? p.wv : p.wk) + b * p.w_b + h * p.w_h + (r - n_sel) * p.w_l;
       } else {
@@ -161,7 +165,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
     const unsigned mb = mb0 + 8 * buf;
     if (ok && !(paired && is_v)) {
       const unsigned dst =
-          (unsigned)__cvta_generic_to_shared(KVs + buf * (ATT_TILE * RS) + i * RS + ((is_v && !paired) ? 128 : 0));
+          (unsigned)__cvta_generic_to_shared(KVs + buf * (TILE * RS) + i * RS + ((is_v && !paired) ? 128 : 0));
       mbar_arrive_expect(mb, paired ? 512u : 256u);
       if (paired)
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], 512, [%2];" ::"r"(dst),
@@ -173,7 +177,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
                      : "memory");
     } else {
       if (MMA && !ok) {  // a row without a copy is an operand of the matrix products all the same: make it zero
-        uint4* z = reinterpret_cast<uint4*>(KVs + buf * (ATT_TILE * RS) + i * RS + (is_v ? 128 : 0));
+        uint4* z = reinterpret_cast<uint4*>(KVs + buf * (TILE * RS) + i * RS + (is_v ? 128 : 0));
 #pragma unroll
         for (int k = 0; k < 16; k++) z[k] = make_uint4(0, 0, 0, 0);
       }
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   // as fatal.
   auto acquire = [&](int j) -> int {
     const int buf = j & 1;
-    if (j + 1 < tpb && !dead) issue(t_first + j + 1, buf ^ 1);
+    if (NBUF > 1 && j + 1 < tpb && !dead) issue(t_first + j + 1, buf ^ 1);
     if (!dead && !__syncthreads_and(mbar_wait(mb0 + 8 * buf, (unsigned)((j >> 1) & 1), ATT_WAIT_LIMIT))) {
       if (tid == 0) atomicExch(p.status, 1);
       mbar_wait(mb0 + 8 * buf, (unsigned)((j >> 1) & 1), ATT_WAIT_LIMIT);
@@ -203,8 +207,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   };
   // Partial record of this block for up to PQ query heads from the groups' (m, l, o) in shared memory.
   auto block_partial = [&](int qg, int n_heads) {
+    const int dim = tid & 127;
 #pragma unroll 2
-    for (int g = 0; g < n_heads; g++) {
+    for (int g = tid >> 7; g < n_heads; g += THREADS / 128) {
       float M = -INFINITY;
 #pragma unroll 4
       for (int t = 0; t < PG; t++) M = fmaxf(M, s_m[t][g]);
@@ -213,11 +218,11 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
       for (int t = 0; t < PG; t++) {
         const float f = (s_m[t][g] == -INFINITY) ? 0.0f : exp2f(s_m[t][g] - M);
         L += s_l[t][g] * f;
-        O += obuf[(t * PQ + g) * 128 + tid] * f;
+        O += obuf[(t * PQ + g) * 128 + dim] * f;
       }
       float* rec = p.ws + (((int64_t)b * p.Hq + h * p.G + qg * PQ + g) * n_groups + blockIdx.x) * ATT_REC;
-      __stcg(rec + tid, O);
-      if (tid == 0) {
+      __stcg(rec + dim, O);
+      if (dim == 0) {
         __stcg(rec + 128, M);
         __stcg(rec + 129, L);
       }
@@ -245,7 +250,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
     for (int j = 0; j < tpb; j++) {
       const int buf = j & 1;
       const int n_live = acquire(j);
-      const uint16_t* tile = KVs + buf * (ATT_TILE * RS);
+      const uint16_t* tile = KVs + buf * (TILE * RS);
       if (r0 < n_live) {  // warp-uniform
         // S[head][row] = Q K^T over the warp's 16 rows: two n-tiles of eight rows
         float sc[2][4];
@@ -355,8 +360,8 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
       for (int j = 0; j < tpb; j++) {
         const int buf = j & 1;
         const int n_live = qg == 0 ? acquire(j) : (dead ? 0 : tile_rows(t_first + j));
-        const uint16_t* tile = KVs + buf * (ATT_TILE * RS);
-        for (int i = grp; i < ATT_TILE; i += 16) {  // uniform trip count per warp: shuffles need all lanes
+        const uint16_t* tile = KVs + buf * (TILE * RS);
+        for (int i = grp; i < TILE; i += 16) {  // uniform trip count per warp: shuffles need all lanes
           const bool live = i < n_live && s_valid[buf][i];
           float kf[16], vf[16];
           if (live) {
@@ -419,12 +424,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
   }
   __syncthreads();
   if (!s_last) return;
-  // Up to ATT_GQ query heads are merged at a time.  A warp takes every fourth record, a lane four dims of it; the
-  // records of ATT_MB steps are in flight together, (m, l) with the values, because nothing in this tail but their
+  // Up to ATT_GQ query heads are merged at a time.  The warps take the records in turn, a lane four dims of each; the
+  // records of MB steps are in flight together, (m, l) with the values, because nothing in this tail but their
   // latency costs time: 36 records of four heads took 6.6 us with a pass for the scale factors and 16 single floats in
-  // flight per thread, 4.4 like this, and 3.7 as the 18 records of two tiles each.  The warps' sums meet in shared memory.
+  // flight per thread, 4.4 like this with four warps.  The warps' sums meet in shared memory.
+  constexpr int MB = WARPS > 4 || !MMA ? 3 : 5;
   const int warp = tid >> 5, lane = tid & 31;
-  static_assert(ATT_THREADS == 128, "one output dimension per thread, four record streams");
   for (int qg = 0; qg < p.n_qgroups; qg++) {
     const int n_heads = min(ATT_GQ, p.G - qg * ATT_GQ);
     const int64_t bq0 = (int64_t)b * p.Hq + h * p.G + qg * ATT_GQ;
@@ -432,14 +437,14 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
     float4 o[ATT_GQ];
 #pragma unroll
     for (int g = 0; g < ATT_GQ; g++) m[g] = -INFINITY, l[g] = 0.0f, o[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int t0 = warp; t0 < n_groups; t0 += 4 * ATT_MB) {
-      float4 v[ATT_MB][ATT_GQ];
-      float2 ml[ATT_MB][ATT_GQ];
+    for (int t0 = warp; t0 < n_groups; t0 += WARPS * MB) {
+      float4 v[MB][ATT_GQ];
+      float2 ml[MB][ATT_GQ];
 #pragma unroll
-      for (int i = 0; i < ATT_MB; i++)
+      for (int i = 0; i < MB; i++)
 #pragma unroll
         for (int g = 0; g < ATT_GQ; g++) {
-          const int t = t0 + 4 * i;
+          const int t = t0 + WARPS * i;
           ml[i][g] = make_float2(-INFINITY, 0.0f), v[i][g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           if (t < n_groups && g < n_heads) {
             const float* rec = p.ws + ((bq0 + g) * n_groups + t) * ATT_REC;
@@ -451,12 +456,12 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
       for (int g = 0; g < ATT_GQ; g++) {
         float mn = m[g];
 #pragma unroll
-        for (int i = 0; i < ATT_MB; i++) mn = fmaxf(mn, ml[i][g].x);
+        for (int i = 0; i < MB; i++) mn = fmaxf(mn, ml[i][g].x);
         if (mn == -INFINITY) continue;   // no live row so far
         const float c = exp2f(m[g] - mn);
         m[g] = mn, l[g] *= c, o[g].x *= c, o[g].y *= c, o[g].z *= c, o[g].w *= c;
 #pragma unroll
-        for (int i = 0; i < ATT_MB; i++) {
+        for (int i = 0; i < MB; i++) {
           const float f = exp2f(ml[i][g].x - mn);
           l[g] += ml[i][g].y * f;
           o[g].x += v[i][g].x * f, o[g].y += v[i][g].y * f, o[g].z += v[i][g].z * f, o[g].w += v[i][g].w * f;
@@ -470,21 +475,34 @@ __global__ void __launch_bounds__(ATT_THREADS, 3) sparse_attention_kernel(AttPar
       reinterpret_cast<float4*>(obuf + (warp * ATT_GQ + g) * 128)[lane] = o[g];
     }
     __syncthreads();
+    for (int g = tid >> 7; g < n_heads; g += THREADS / 128) {
+      float M = -INFINITY, L = 0.0f, O = 0.0f;
 #pragma unroll
-    for (int g = 0; g < ATT_GQ; g++) {
-      if (g >= n_heads) continue;
-      const float M = fmaxf(fmaxf(s_m[0][g], s_m[1][g]), fmaxf(s_m[2][g], s_m[3][g]));
-      float L = 0.0f, O = 0.0f;
+      for (int w = 0; w < WARPS; w++) M = fmaxf(M, s_m[w][g]);
 #pragma unroll
-      for (int w = 0; w < 4; w++) {
+      for (int w = 0; w < WARPS; w++) {
         const float f = s_m[w][g] == -INFINITY ? 0.0f : exp2f(s_m[w][g] - M);
         L += s_l[w][g] * f;
-        O += obuf[(w * ATT_GQ + g) * 128 + tid] * f;
+        O += obuf[(w * ATT_GQ + g) * 128 + (tid & 127)] * f;
       }
-      p.out[(bq0 + g) * 128 + tid] = f2bf(L > 0.0f ? O / L : 0.0f);
-      if (p.lse && tid == 0) p.lse[bq0 + g] = L > 0.0f ? M + log2f(L) : -INFINITY;
+      p.out[(bq0 + g) * 128 + (tid & 127)] = f2bf(L > 0.0f ? O / L : 0.0f);
+      if (p.lse && (tid & 127) == 0) p.lse[bq0 + g] = L > 0.0f ? M + log2f(L) : -INFINITY;
     }
   }
+}
+
+template <bool MMA, int WARPS>
+int launch_attention(const AttParams& p, dim3 grid, cudaStream_t st) {
+  const int smem = (WARPS > 4 ? 1 : 2) * 16 * WARPS * AttRow<MMA>::stride * 2;
+  static PerDevice smem_attr;   // the opt-in to more than 48 KB of dynamic shared memory is per kernel and device
+  if (const unsigned long long bit = first_on_device(smem_attr)) {
+    if (cudaFuncSetAttribute(sparse_attention_kernel<MMA, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return check_launch("sparse_attention smem");
+    mark_on_device(smem_attr, bit);
+  }
+  StageTimer tm(ST_ATTENTION, st);
+  launch_chain(sparse_attention_kernel<MMA, WARPS>, grid, dim3(32 * WARPS), (size_t)smem, st, p);
+  return check_launch("sparse_attention");
 }
 
 }  // namespace
@@ -589,18 +607,23 @@ extern "C" int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* wi
   p.K = K, p.index_offset = index_offset;
   p.H = (int)H, p.Hq = (int)Hq, p.G = (int)(Hq / H);
   p.n_qgroups = (p.G + ATT_GQ - 1) / ATT_GQ;
-  // Blocks per (batch, KV head): one per two tiles when the launch is small (a block copies two tiles at once, so every
-  // copy of the launch is outstanding; a block per tile would only double the records that the merge reads),
-  // otherwise as many as give ONE wave of three blocks per SM, each streaming several tiles.  The scalar form needs
-  // the staged tile for several passes: one tile per block then.
-  int64_t groups = n_tiles;
+  // Blocks per (batch, KV head): one per 128 rows when the whole launch is then a block per SM at most (every copy of the
+  // launch outstanding at once), otherwise one per two tiles of 64 rows - a block copies two at once - but no more than
+  // ONE wave of three blocks per SM, each streaming several tiles.  The scalar form needs the staged tile for several
+  // passes: one tile per block then.
   const bool mma = p.G <= ATT_MQ;   // at most ATT_MQ query heads per KV head: one pass on the tensor cores
-  if (mma) {
-    const int64_t fit = (int64_t)sm_count() * 3 / (H * bs), pairs = (n_tiles + 1) / 2;
-    groups = fit < 1 ? 1 : (fit < pairs ? fit : pairs);
+  const int64_t halves = (n_tiles + 1) / 2;
+  const bool wide = mma && halves * H * bs <= sm_count();
+  int64_t groups = n_tiles;
+  p.tiles_per_block = 1;
+  if (wide) {
+    groups = halves;
+  } else if (mma) {
+    const int64_t fit = (int64_t)sm_count() * 3 / (H * bs);
+    groups = fit < 1 ? 1 : (fit < halves ? fit : halves);
+    p.tiles_per_block = (int)((n_tiles + groups - 1) / groups);
+    groups = (n_tiles + p.tiles_per_block - 1) / p.tiles_per_block;
   }
-  p.tiles_per_block = (int)((n_tiles + groups - 1) / groups);
-  groups = (n_tiles + p.tiles_per_block - 1) / p.tiles_per_block;
   p.scale_log2 = scale * 1.4426950408889634f;
   PK_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15) == 0, "workspace must be 16-byte aligned");
   p.counters = (unsigned*)workspace;
@@ -613,17 +636,7 @@ extern "C" int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* wi
     p.lse = (float*)lse->data;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  const int smem = 2 * ATT_TILE * (mma ? AttRow<true>::stride : AttRow<false>::stride) * 2;   // two staging buffers
-  static PerDevice smem_attr[2];  // the opt-in to more than 48 KB of dynamic shared memory is per kernel and device
-  if (const unsigned long long bit = first_on_device(smem_attr[mma])) {
-    const cudaError_t e = mma ? cudaFuncSetAttribute(sparse_attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-                              : cudaFuncSetAttribute(sparse_attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return check_launch("sparse_attention smem");
-    mark_on_device(smem_attr[mma], bit);
-  }
-  dim3 grid((unsigned)groups, (unsigned)H, (unsigned)bs);
-  StageTimer tm(ST_ATTENTION, st);
-  if (mma) launch_chain(sparse_attention_kernel<true>, grid, dim3(ATT_THREADS), (size_t)smem, st, p);
-  else launch_chain(sparse_attention_kernel<false>, grid, dim3(ATT_THREADS), (size_t)smem, st, p);
-  return check_launch("sparse_attention");
+  const dim3 grid((unsigned)groups, (unsigned)H, (unsigned)bs);
+  if (wide) return launch_attention<true, 8>(p, grid, st);
+  return mma ? launch_attention<true, 4>(p, grid, st) : launch_attention<false, 4>(p, grid, st);
 }

@@ -224,30 +224,39 @@ __global__ void __launch_bounds__(256) count_kernel(const uint8_t* codes, int64_
     if (hist[i]) atomicAdd(dst + i, hist[i]);
 }
 
-__global__ void __launch_bounds__(32) query_prep_kernel(const uint16_t* queries, int Hq, int H, int G,
-                                                        float inv_g, const uint16_t* signs,
-                                                        uint16_t* q_blocks, uint16_t* q_norm,
-                                                        uint16_t* query_avg) {
-  const int lane = threadIdx.x, s = lane & 7;
+// One warp per (batch, KV head), four dims per lane.  What bounds it is the latency of its loads: those of eight queries go
+// out together (16 serial sums in 8 lanes before: 5.6 us for 8 heads of 4 queries on B200, 2.6 now).
+__global__ void __launch_bounds__(32) query_prep_kernel(const uint16_t* __restrict__ queries, int Hq, int H, int G, float inv_g,
+                                                        const uint16_t* __restrict__ signs, uint16_t* q_blocks,
+                                                        uint16_t* q_norm, uint16_t* query_avg) {
+  const int lane = threadIdx.x;
   const int bh = blockIdx.x, b = bh / H, h = bh % H;
-  const uint16_t* q = queries + ((int64_t)b * Hq + (int64_t)h * G) * 128 + 16 * s;
-  float x[16], sg[16];
+  const uint16_t* q = queries + ((int64_t)b * Hq + (int64_t)h * G) * 128 + 4 * lane;
+  float x[4], sg[4], acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-  for (int i = 0; i < 16; i++) {
-    float acc = 0.0f;
-    for (int g = 0; g < G; g++) acc = __fadd_rn(acc, bf2f(q[g * 128 + i]));
-    x[i] = bfround(__fmul_rn(acc, inv_g));
-    sg[i] = bf2f(signs[16 * s + i]);
+  for (int i = 0; i < 4; i++) sg[i] = bf2f(signs[4 * lane + i]);
+  for (int g0 = 0; g0 < G; g0 += 8) {   // fp32 sum over the group, g ascending
+    uint16_t raw[8][4];
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) raw[k][i] = q[min(g0 + k, G - 1) * 128 + i];
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        if (g0 + k < G) acc[i] = __fadd_rn(acc[i], bf2f(raw[k][i]));
   }
-  if (query_avg && lane < 8)
+  auto store = [&](uint16_t* out) {
 #pragma unroll
-    for (int i = 0; i < 16; i++) query_avg[(int64_t)bh * 128 + 16 * s + i] = f2bf(x[i]);
-  const float n = rotate16(x, sg, s);
-  if (lane < 8) {
+    for (int i = 0; i < 4; i++) out[(int64_t)bh * 128 + 4 * lane + i] = f2bf(x[i]);
+  };
 #pragma unroll
-    for (int i = 0; i < 16; i++) q_blocks[(int64_t)bh * 128 + 16 * s + i] = f2bf(x[i]);
-    if (lane == 0) q_norm[bh] = f2bf(n);
-  }
+  for (int i = 0; i < 4; i++) x[i] = bfround(__fmul_rn(acc[i], inv_g));
+  if (query_avg) store(query_avg);
+  const float n = rotate4(x, sg, lane);
+  store(q_blocks);
+  if (lane == 0) q_norm[bh] = f2bf(n);
 }
 
 // ---- append one decode token: window row, key coding, and the flush of a full update buffer, one launch ----------

@@ -63,3 +63,18 @@ def test_attention_group_sizes(oracle, group, n_window, K):
     out = ops.sparse_attention(q.to(DEV), wk.to(DEV), wv.to(DEV), n_window, *args)
     ref = oracle.attention(q, torch.cat(rk, 2), torch.cat(rv, 2))
     assert (out.float().cpu() - ref).abs().max().item() <= 2e-2
+
+
+@pytest.mark.parametrize("bs,H,n_window,K", [(1, 1, 127, 0), (1, 1, 128, 1), (1, 2, 1, 127), (2, 37, 100, 156), (2, 37, 100, 157)])
+def test_attention_tile_edges(oracle, bs, H, n_window, K):
+    """One tile of 128 rows per block up to a block per SM (2 x 37 heads of 256 rows on 148 SMs), tiles of 64 beyond."""
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(n_window + K)
+    k, v = (torch.randn(bs, H, 300, 128, generator=g).to(torch.bfloat16) for _ in range(2))
+    q = (torch.randn(bs, 1, 4 * H, 128, generator=g) * 3).to(torch.bfloat16)
+    wk, wv = (torch.randn(bs, H, n_window, 128, generator=g).to(torch.bfloat16) for _ in range(2))
+    sel = torch.stack([torch.stack([torch.randperm(300, generator=g)[:K] for _ in range(H)]) for _ in range(bs)])
+    args = (k.to(DEV), v.to(DEV), sel.to(DEV)) if K else ()
+    out = ops.sparse_attention(q.to(DEV), wk.to(DEV), wv.to(DEV), n_window, *args)
+    rk, rv = ([torch.cat([oracle.gather(k, sel), wk], 2), torch.cat([oracle.gather(v, sel), wv], 2)] if K else (wk, wv))
+    assert (out.float().cpu() - oracle.attention(q, rk, rv)).abs().max().item() <= 2e-2
