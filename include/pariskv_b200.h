@@ -68,12 +68,15 @@ int pk_timing_read(double* ms_per_stage, int64_t* spans_per_stage, int n_stages)
 int pk_timing_read_graph(double* ms_per_stage, int64_t* spans_per_stage, int n_stages);
 int pk_timing_clear_graph(void);
 
-/* Process-wide option, no counterpart in the reference: launch the kernels of this library with programmatic
- * dependent launch.  A kernel may then be scheduled while its predecessor on the stream still runs; it does only
- * what does not depend on earlier kernels (the collision kernel its first code loads, a projection its first weight
- * loads) and then waits for the predecessor to complete, and every kernel releases its successor only after its own
- * wait, so completion is transitive along the stream.  On by default: eager decode steps of 10K-token contexts
- * measured 207 -> 195 us on B200, and with the step replayed as a CUDA graph it is +1.9 % tokens/s at 128K. */
+/* Process-wide option, no counterpart in the reference.  The kernels of this library are launched with programmatic
+ * dependent launch: a kernel may be scheduled while its predecessor on the stream still runs, waits for that to complete
+ * before it touches global memory, and releases its successor only after its own wait, so completion is transitive
+ * along the stream and results do not depend on it (eager on B200: decode steps of 10K-token contexts 207 -> 181 us,
+ * a dense step of two layers 188 -> 157).
+ *   1   meant for a decode step captured as a CUDA graph: kernels also load before that wait what no launch of the step
+ *       writes (a projection its first weights, the chain its first codes): +1.9 % tokens/s at 128K
+ *   0   the default: no such early loads
+ *  -1   plain launches, each after its predecessor's end */
 int pk_set_pdl(int on);
 
 /* ---- (a) key coding ---------------------------------------------------------------------- */

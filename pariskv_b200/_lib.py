@@ -210,7 +210,7 @@ STAGES = ["query_prep", "rank_table", "collision", "select_rerank", "final_topk"
 
 
 def set_pdl(on: bool):
-    """Launch the kernels of a decode step with programmatic dependent launch (see pk_set_pdl)."""
+    """Let the dependently launched kernels of a decode step load ahead of their wait (see pk_set_pdl)."""
     check(load().pk_set_pdl(int(bool(on))))
 
 

@@ -31,6 +31,8 @@ __global__ void __launch_bounds__(256) lut_from_sorted_kernel(const IdT* __restr
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t blk = blockIdx.x;
   mask[tid] = 0;
+  pdl_wait();
+  pdl_trigger();
   long long id = -1;
   long long cnt = 0;
   if (tid < NC) {
@@ -203,6 +205,8 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
   const int64_t v_begin = (int64_t)blockIdx.x * p.chunk_keys;
   const int64_t v_end = min(Nv, v_begin + p.chunk_keys);
   const uint8_t* base = p.codes + b * p.c_b + h * p.c_h - p.mis * p.c_l;
+  pdl_wait();
+  pdl_trigger();
   int32_t* out32 = p.out_i32 + (int64_t)bh * p.N;
 
   // the first batch of code loads is issued before the table is staged, so both latencies overlap
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
     __syncthreads();
     rank_subspace(key, s_q + warp * 8, lane);
   }
-  if (cq.n_dev) pdl_wait();  // the zone length may have been written by the kernel just before this one
+  if (cq.n_dev || !cq.early_loads) pdl_wait();  // the zone length may have been written by the kernel just before this one
   const int64_t N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
   const int64_t Nv = N + p.mis;
   const int64_t v_begin = (int64_t)blockIdx.x * p.chunk_keys;
@@ -535,9 +539,9 @@ int launch_collision(const pk_tensor* codebook, const uint32_t* lut, int32_t* ou
   const int64_t n_chunks = (Nv + p.chunk_keys - 1) / p.chunk_keys;
   dim3 grid((unsigned)n_chunks, (unsigned)(bs * H));
   StageTimer tm(ST_COLLISION, st);
-  if (layout == 0) collision_kernel<0><<<grid, 256, 0, st>>>(p);
-  else if (layout == 1) collision_kernel<1><<<grid, 256, 0, st>>>(p);
-  else collision_kernel<2><<<grid, 256, 0, st>>>(p);
+  if (layout == 0) launch_chain(collision_kernel<0>, grid, dim3(256), 0, st, p);
+  else if (layout == 1) launch_chain(collision_kernel<1>, grid, dim3(256), 0, st, p);
+  else launch_chain(collision_kernel<2>, grid, dim3(256), 0, st, p);
   return check_launch("collision");
 }
 
@@ -678,11 +682,11 @@ extern "C" int pk_collision_fused(const pk_tensor* sorted_cluster_ids, const pk_
   {
     StageTimer tm(ST_RANK, st);
     if (sorted_cluster_ids->dtype == PK_I64)
-      lut_from_sorted_kernel<int64_t><<<nblk, 256, 0, st>>>((const int64_t*)sorted_cluster_ids->data,
-                                                            (const int32_t*)cluster_key_counts->data, (int)NC, tiers, lut);
+      launch_chain(lut_from_sorted_kernel<int64_t>, dim3(nblk), dim3(256), 0, st, (const int64_t*)sorted_cluster_ids->data,
+                   (const int32_t*)cluster_key_counts->data, (int)NC, tiers, lut);
     else
-      lut_from_sorted_kernel<int32_t><<<nblk, 256, 0, st>>>((const int32_t*)sorted_cluster_ids->data,
-                                                            (const int32_t*)cluster_key_counts->data, (int)NC, tiers, lut);
+      launch_chain(lut_from_sorted_kernel<int32_t>, dim3(nblk), dim3(256), 0, st, (const int32_t*)sorted_cluster_ids->data,
+                   (const int32_t*)cluster_key_counts->data, (int)NC, tiers, lut);
     rc = check_launch("collision table");
   }
   if (rc) return rc;

@@ -75,8 +75,9 @@ StageTimer::~StageTimer() {
     (cap_ ? g_graph_spans : g_spans).push_back({stage_, a_, b});
 }
 
-static std::atomic<int> g_pdl{1};
+static std::atomic<int> g_pdl{1};   // 0 off, 1 dependent launch, 2 the same with early loads
 bool pdl_enabled() { return g_pdl.load(std::memory_order_relaxed) != 0; }
+bool pdl_early() { return g_pdl.load(std::memory_order_relaxed) == 2; }
 
 static std::mutex g_dev_mu;
 unsigned long long first_on_device(PerDevice& p) {
@@ -110,7 +111,7 @@ const char* pk_last_error(void) { return pk::g_err; }
 int64_t pk_launch_count(void) { return pk::g_launches.load(std::memory_order_relaxed); }
 
 int pk_set_pdl(int on) {
-  pk::g_pdl.store(on ? 1 : 0, std::memory_order_relaxed);
+  pk::g_pdl.store(on > 0 ? 2 : on < 0 ? 0 : 1, std::memory_order_relaxed);
   return PK_OK;
 }
 

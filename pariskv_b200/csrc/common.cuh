@@ -70,10 +70,13 @@ inline int elem_size(int dtype) {
 // may be scheduled while its predecessor is still running, does the part of its prologue that does not read the
 // predecessor's output, and then blocks in pdl_wait() until the predecessor has completed and flushed.  Every
 // kernel signals pdl_trigger() only AFTER its own pdl_wait(), so completion is transitive along the chain.
-// Without the launch attribute both instructions do nothing.  The attribute is set unless pk_set_pdl(0).
+// Without the launch attribute both instructions do nothing.  The attribute is set unless pk_set_pdl(-1).
+// Only after pk_set_pdl(1) may a kernel load global memory before its wait (pdl_early(): weights, codes), and then only what
+// no launch of the running step writes: a caller who has not asked for it may have written those tensors a launch ago.
 // EVERY kernel launched through launch_chain() must call pdl_wait() before it reads or writes anything an earlier
 // kernel may touch: a kernel that skipped the wait would break the chain for its successors.
 bool pdl_enabled();
+bool pdl_early();
 
 // Per-device "done once" flags for settings that belong to a device (cudaFuncSetAttribute opt-ins): bit d is set
 // once the setting has been applied with device d current.  first_on_device() returns the bit to set, or 0 when

@@ -232,6 +232,8 @@ __global__ void __launch_bounds__(32) query_prep_kernel(const uint16_t* __restri
   const int lane = threadIdx.x;
   const int bh = blockIdx.x, b = bh / H, h = bh % H;
   const uint16_t* q = queries + ((int64_t)b * Hq + (int64_t)h * G) * 128 + 4 * lane;
+  pdl_wait();
+  pdl_trigger();
   float x[4], sg[4], acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int i = 0; i < 4; i++) sg[i] = bf2f(signs[4 * lane + i]);
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
   uint8_t* wp = p.win_pk + bh * p.cap_w * 64;
   float* wn = p.win_vnorm + bh * p.cap_w;
   const bool ok = pos >= 0 && pos < p.cap_w;
-  if (tid < 32 && ok) {
+  if (tid < 32) {   // the loads do not wait for the position
     const int s = lane & 3, l = lane & 15;
     const uint16_t* kr = p.k_row + b * p.kr_b + h * p.kr_h;
     const uint4* vr = reinterpret_cast<const uint4*>(p.v_row + b * p.vr_b + h * p.vr_h);
@@ -322,7 +324,7 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
     make_rotate_lane(rl, p.signs, s);
     float y[8];
     unpack8(__ldg(vr + l), y);
-    reinterpret_cast<uint4*>((lane < 16 ? wk : wv) + (int64_t)pos * 128)[l] = cp;
+    if (ok) reinterpret_cast<uint4*>((lane < 16 ? wk : wv) + (int64_t)pos * 128)[l] = cp;
     // ||v||: fp32, pairwise tree over adjacent dimensions
 #pragma unroll
     for (int i = 0; i < 8; i++) y[i] = __fmul_rn(y[i], y[i]);
@@ -334,7 +336,7 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
 #pragma unroll
     for (int off = 1; off < 16; off <<= 1) vs = __fadd_rn(vs, __shfl_xor_sync(FULL, vs, off));
     const KeyCode kc = code_key(raw, rl);   // (eight times the same: every group of four lanes)
-    if (lane < 4) {
+    if (ok && lane < 4) {
       *reinterpret_cast<uint32_t*>(wc + (int64_t)pos * 16 + 4 * s) = kc.codes;
       *reinterpret_cast<uint2*>(ww + (int64_t)pos * 16 + 4 * s) = kc.weights;
       *reinterpret_cast<uint4*>(wp + (int64_t)pos * 64 + 16 * s) = kc.packed;
@@ -388,9 +390,11 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
     }
   }
   // the block that arrives last advances the state (every block has read it by then)
-  __threadfence();
   __syncthreads();
-  if (tid == 0) s_last = atomicAdd(reinterpret_cast<unsigned*>(p.state + 1), 1u) + 1u == gridDim.x;
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(reinterpret_cast<unsigned*>(p.state + 1), 1u) + 1u == gridDim.x;
+  }
   __syncthreads();
   if (s_last && tid == 0) {
     if (!ok || (flush && !room)) {
@@ -426,8 +430,8 @@ int launch_query_prep(const uint16_t* queries, int bs, int Hq, int H, const uint
                       uint16_t* q_blocks, uint16_t* q_norm, uint16_t* query_avg, cudaStream_t st) {
   const int G = Hq / H;
   StageTimer tm(ST_QUERY_PREP, st);
-  query_prep_kernel<<<bs * H, 32, 0, st>>>(queries, Hq, H, G, 1.0f / (float)G, signs, q_blocks, q_norm,
-                                           query_avg);
+  launch_chain(query_prep_kernel, dim3(bs * H), dim3(32), 0, st, queries, Hq, H, G, 1.0f / (float)G, signs, q_blocks, q_norm,
+               query_avg);
   return check_launch("query_prep");
 }
 

@@ -27,6 +27,8 @@ __global__ void __launch_bounds__(256) h2d_gather_kernel(const uint4* __restrict
   const uint4* src = lane < 16 ? src_k : src_v;
   uint4* dst = lane < 16 ? dst_k : dst_v;
   const int l = lane & 15;
+  pdl_wait();
+  pdl_trigger();
   for (int64_t r = warp; r < total; r += n_warps) {
     const int64_t bh = r / K, j = r - bh * K;
     const int64_t row = __ldg(idx + r);
@@ -104,9 +106,9 @@ extern "C" int pk_h2d_gather_kv(const pk_tensor* src_k, const pk_tensor* src_v, 
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   StageTimer tm(ST_GATHER, (cudaStream_t)stream);
-  h2d_gather_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
-      (const uint4*)src_k->data, (const uint4*)src_v->data, (const int64_t*)selected_indices->data, (uint4*)dst_k->data,
-      (uint4*)dst_v->data, bs * H, N, dst_k->shape[2], K);
+  launch_chain(h2d_gather_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, (const uint4*)src_k->data,
+               (const uint4*)src_v->data, (const int64_t*)selected_indices->data, (uint4*)dst_k->data, (uint4*)dst_v->data,
+               bs * H, N, dst_k->shape[2], K);
   return check_launch("h2d_gather_kv");
 }
 

@@ -59,6 +59,7 @@ struct ChainQuery {
   pk_zone_schedule sched;     // thresholds = zone_tiers(sched, n_dev[b]) when n_dev is set
   long long n_plan;           // > 0: thresholds from this zone length instead (a shard of a longer zone)
   int early_query;            // the queries were complete before the previous kernel on the stream started
+  int early_loads;            // see pdl_early()
 };
 int launch_collision(const pk_tensor* codebook, const uint32_t* lut, int32_t* out_i32, cudaStream_t st);
 int chain_layout(const pk_tensor* codebook, int* layout);

@@ -23,6 +23,8 @@ __global__ void __launch_bounds__(RR_THREADS) rerank_kernel(RerankArgs a, uint16
   const int tid = threadIdx.x, lane = tid & 31;
   const int64_t bh = blockIdx.y;
   const int b = (int)(bh / a.H), h = (int)(bh % a.H);
+  pdl_wait();
+  pdl_trigger();
   rerank_setup(sm, a, bh, tid, RR_THREADS);
   __syncthreads();
   const float qn = bf2f(a.q_norm[bh]);
@@ -212,9 +214,9 @@ int launch_rerank(const RerankArgs& a, int64_t bs_h, uint16_t* scores_bf16, floa
   dim3 grid((unsigned)gx, (unsigned)bs_h);
   StageTimer tm(ST_RERANK, st);
   if (rerank_fast_layout(a))
-    rerank_kernel<true><<<grid, RR_THREADS, 0, st>>>(a, scores_bf16, scores_f32, v4b);
+    launch_chain(rerank_kernel<true>, grid, dim3(RR_THREADS), 0, st, a, scores_bf16, scores_f32, v4b);
   else
-    rerank_kernel<false><<<grid, RR_THREADS, 0, st>>>(a, scores_bf16, scores_f32, v4b);
+    launch_chain(rerank_kernel<false>, grid, dim3(RR_THREADS), 0, st, a, scores_bf16, scores_f32, v4b);
   return check_launch("rerank");
 }
 

@@ -171,7 +171,8 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
     cq.queries = (const uint16_t*)queries->data, cq.signs = (const uint16_t*)a.signs->data, cq.Hq = (int)Hq;
     cq.q_blocks = qb, cq.q_norm = qn, cq.query_avg = qa;
     cq.counts = (const int32_t*)counts_t->data;
-    cq.early_query = a.queries_settled != 0;
+    cq.early_loads = pdl_early();
+    cq.early_query = a.queries_settled != 0 && cq.early_loads;
     const int cs = sharded ? 0 : fused_cluster_size(codebook, ra, bh, N, C);
     if (cs) {
       ra.q_blocks = nullptr, ra.q_norm = nullptr, ra.centers = (const uint16_t*)a.mag_centers->data, ra.C = row;

@@ -76,9 +76,8 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   PreparedQuery pq;
   QueryLoads ql;
   unsigned key[4];
-  // before the wait: what no kernel of the chain writes
-  build_lev2(lev2, p.a.centers, tid, CH_THREADS);
   for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
+  if (cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
   const bool early = cq.early_query != 0;
   if (early) {   // the queries were complete before the kernel before this one started
     load_query(ql, cq, b, h, p.G);
@@ -115,6 +114,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   {
     unsigned* my = reinterpret_cast<unsigned*>(cnt8) + warp * 256;   // the counts are not there yet
     if (!early) prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
+    if (!cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
     if (warp == 0 && rank == 0) publish_query(pq, cq, bh);
     if (tid == 32) load_tiers(cq, (long long)N, s_tiers);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
