@@ -172,6 +172,7 @@ class polar_cache(KV_Cache):
         self._attn_rows_max = self.window_capacity + max(self.final_topk, self._max_selected_rows())
         self.queries_precede_append = False   # see compute(): set by callers that make q and k in one kernel
         self._appended_layer = None
+        self._softmax_scale = 1.0 / math.sqrt(self.head_dim)
         self._attn_scratch = ops.Scratch(dev, ops.attention_scratch_bytes(bs, num_heads, self._attn_rows_max))
 
     def _max_selected_rows(self):
@@ -183,12 +184,15 @@ class polar_cache(KV_Cache):
         """fp32 ||v|| of the zone rows, kept by the variants that rank candidates by it (None here)."""
         return None
 
-    def _attend(self, queries, wk, wv, n_win, *args, **kw):
-        """ops.sparse_attention on the cache's own scratch (the shared, growable one for an oversized eager call)."""
-        sel = args[2] if len(args) > 2 else kw.get("selected")
-        rows = n_win + (sel.shape[2] if sel is not None else 0)
-        scratch = self._attn_scratch if rows <= self._attn_rows_max else None
-        return ops.sparse_attention(queries, wk, wv, n_win, *args, scratch=scratch, **kw)
+    def _attend(self, queries, wk, wv, n_win, store_k=None, store_v=None, selected=None, n_sel=None, n_window_dev=None,
+                n_window_add=0):
+        """Sparse attention on the cache's own scratch (the shared, growable one for an oversized eager call)."""
+        rows = n_win + (selected.shape[2] if selected is not None else 0)
+        if rows > self._attn_rows_max:
+            return ops.sparse_attention(queries, wk, wv, n_win, store_k, store_v, selected, n_sel=n_sel,
+                                        n_window_dev=n_window_dev, n_window_add=n_window_add)
+        return _lib.native().sparse_attention(queries, wk, wv, n_win, n_window_dev, n_window_add, store_k, store_v, selected,
+                                              n_sel, 0, self._softmax_scale, None, None, self._attn_scratch.buf)
 
     def check_status(self):
         """Raise if a kernel reported a problem through its status word: an attention block whose row copies never
@@ -323,11 +327,11 @@ class polar_cache(KV_Cache):
         if self._window_len[l] + 1 == self.window_capacity and max(self.zone_len[l]) + self.dynamic_update_interval > self.zone_capacity:
             raise RuntimeError("zone store is full: construct the cache with a larger max_length / max_new_length")
         self._wait_offload(l)      # the flush writes store rows: stay ordered behind a pending bulk offload
-        ops.append_encode(key_states, value_states, self.srht_diagonal_signs, self.unified_keys_gpu[l],
-                          self.unified_values_gpu[l], self._win_codes[l], self._win_weight[l], self._win_4bit[l],
-                          self._win_vnorm[l], self.codebook_gpu[l], self.key_block_weight_gpu[l],
-                          self.key_4bit_packed_gpu[l], self._zone_vnorm(l), self.cluster_key_counts_gpu[l],
-                          self._store_kv[l], self._layer_state[l], self.sink_size, self.dynamic_update_interval)
+        _lib.native().append_encode(
+            key_states, value_states, self.srht_diagonal_signs, self.unified_keys_gpu[l], self.unified_values_gpu[l],
+            self._win_codes[l], self._win_weight[l], self._win_4bit[l], self._win_vnorm[l], self.codebook_gpu[l],
+            self.key_block_weight_gpu[l], self.key_4bit_packed_gpu[l], self._zone_vnorm(l), self.cluster_key_counts_gpu[l],
+            self._store_kv[l], self._layer_state[l], self.sink_size, self.dynamic_update_interval)
         self._mirror_append(l)
         self._appended_layer = l
         if l == 0:
