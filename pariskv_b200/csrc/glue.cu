@@ -211,8 +211,9 @@ extern "C" int pk_silu_mul(const pk_tensor* gate_up, const pk_tensor* out, void*
 // ---- matrix-vector products of a decode step (one token): y = W x, W bf16 [O, I] row-major, fp32 accumulation ------
 // HBM-bound: a warp takes two rows, every lane keeps sixteen 16-byte streaming loads in flight, x sits in shared memory.
 // What is lost to the copy rate is the start of each launch, about 4 us where nothing overlaps it: dependent launch takes a
-// dense step of two layers (770 MB of weights) from 189 to 158 us on B200, and telling the
-// compiler that two blocks share an SM to 151.  Reloading each register as soon as it is used (272 us) and smaller blocks for an even last wave (196 against 189) lost.
+// dense step of two layers (770 MB of weights) from 189 to 158 us on B200, and telling the compiler that two blocks share
+// an SM to 151.  Reloading each register as soon as it is used (272 us) and smaller blocks for an even last wave (196
+// against 189) lost.
 // GATED: the rows are (o, o + F) of a stacked [gate; up] matrix and the output is silu(gate) * up, rounded like the
 // separate launches would (bf16 after the product, after silu, after the multiply).
 namespace pk {

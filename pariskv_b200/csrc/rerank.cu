@@ -43,7 +43,9 @@ __global__ void __launch_bounds__(RR_THREADS) rerank_kernel(RerankArgs a, uint16
 // One block per (chunk of keys, batch*head), one block per SM.  The histogram rows written by the collision kernel
 // give every block the global threshold count, the tie quota and its own output offset, so the candidate
 // list comes out in ascending key order with no atomics and no second pass.
-// What bounds it: the rerank's arithmetic (chain.cuh) and the latency of histogram rows, counts and records before it.  With
+// What bounds it at 8 heads x 1M keys: HBM in units of 128 bytes.  A candidate's two records (64 and 32 bytes) cost 226 of
+// traffic, 203 MB for 840 K candidates, 4.1 TB/s over the launch and more without its first 10 us (histogram rows, counts,
+// list); issue slots are 49 % busy.  With
 // the final top-K by the last block of a head inside it (one SM per head), 8 heads x 1M keys took 129 us on B200; 50
 // here plus 19 for the final top-K as a cluster launch.
 struct SelParams {
@@ -67,9 +69,11 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t bh = blockIdx.y, chunk = blockIdx.x;
   const int b = (int)(bh / a.H), h = (int)(bh % a.H);
-  if (FAST) build_lev2(lev2, a.centers, tid, CH_THREADS);              // an input of the whole chain: not the last kernel's
+  // before the wait only where the collision kernel, which has waited itself, is the launch before this one
+  if (FAST && !p.shard_hist) build_lev2(lev2, a.centers, tid, CH_THREADS);
   pdl_wait();  // counts, histograms and query blocks come from the collision kernel
   pdl_trigger();
+  if (FAST && p.shard_hist) build_lev2(lev2, a.centers, tid, CH_THREADS);
   const int64_t N = p.n_dev ? min(max((int64_t)p.n_dev[b], (int64_t)1), p.N) : p.N;
   const int64_t Nv = N + p.mis;
   const int64_t v_begin = chunk * p.chunk_keys;
