@@ -1,7 +1,8 @@
 // Exact top-K of a row that is spread over the CTAs of a thread-block cluster (each holds a contiguous slice):
 // first K of (value descending, position ascending), emitted in ascending position.
 //
-//   extremes of the row                      -> 256 linear value bins, about equally filled
+//   extremes of the row                      -> 256 bins: linear in the value for floats, about equally filled; the top
+//                                               eight bits of (key - lowest key) for whole numbers, exact at any size
 //   histogram of the bins, summed over ranks -> the bin of the K-th largest, this CTA's share above it and in it
 //   the elements of that bin, gathered by every CTA, cut once more into 64 sub-bins and ranked -> the exact threshold
 //   ordered emission of this CTA's elements at its offset.
@@ -27,18 +28,40 @@ constexpr int SEL_SUB = 64;
 constexpr int SEL_TIES = 1024;
 constexpr int SEL_REGION = 2 * SEL_TIES * 8;   // bytes of dynamic shared memory, at the same offset in every CTA
 
+// Rows of a type: the ordered key of an element, and the level-0 bins between the extremes of the row's keys.  A bin is
+// monotone in the key; sub() cuts a bin into SEL_SUB parts, monotone as well; single(): a bin holds one value.
 struct F32Row {
-  static constexpr bool whole = false;
-  static __device__ __forceinline__ float val(uint32_t u) { return __uint_as_float(u); }
   static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key(__uint_as_float(u)); }
   static __device__ __forceinline__ float from_key(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k); }
+  struct Bins {
+    float vmin, scale;
+    __device__ __forceinline__ Bins(uint32_t kmin, uint32_t kmax) {
+      vmin = from_key(kmin);
+      scale = (float)(SEL_BINS - 1) / (from_key(kmax) - vmin);
+      if (!(scale > 0.0f) || !(scale < INFINITY)) scale = 0.0f;   // flat or non-finite: one bin, the key levels decide
+    }
+    __device__ __forceinline__ unsigned of(uint32_t u) const {
+      return min((unsigned)(SEL_BINS - 1), (unsigned)((__uint_as_float(u) - vmin) * scale));
+    }
+    __device__ __forceinline__ unsigned sub(uint32_t k, unsigned bin) const {
+      return scale > 0.0f ? min((unsigned)(SEL_SUB - 1), (unsigned)max(0.0f, ((from_key(k) - vmin) * scale - (float)bin) * (float)SEL_SUB)) : 0u;
+    }
+    __device__ __forceinline__ bool single() const { return false; }
+  };
 };
+// From the keys themselves: as floats, whole numbers above 2^24 would share a bin that single() takes for one value.
 struct I32Row {
-  static constexpr bool whole = true;
-  static __device__ __forceinline__ float val(uint32_t u) { return (float)(int32_t)u; }
   static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key((int32_t)u); }
-  static __device__ __forceinline__ float from_key(uint32_t k) { return (float)(int32_t)(k ^ 0x80000000u); }
+  struct Bins {
+    uint32_t kmin;
+    int shift;   // (kmax - kmin) >> shift < SEL_BINS
+    __device__ __forceinline__ Bins(uint32_t kmin_, uint32_t kmax) : kmin(kmin_) { shift = max(0, 24 - __clz(kmax - kmin)); }
+    __device__ __forceinline__ unsigned of(uint32_t u) const { return (key(u) - kmin) >> shift; }
+    __device__ __forceinline__ unsigned sub(uint32_t k, unsigned bin) const { return (k - kmin - (bin << shift)) >> max(0, shift - 6); }
+    __device__ __forceinline__ bool single() const { return shift == 0; }
+  };
 };
+static_assert(SEL_BINS == 256 && SEL_SUB == 64, "the shifts of I32Row::Bins");
 
 struct SelShared {               // static: what other CTAs of the cluster read, and small block-wide results
   unsigned hist[2][SEL_BINS];    // local histograms, used alternately
@@ -147,12 +170,10 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     if (tid < SEL_BINS) s.hist[buf][tid] = region[tid] + region[SEL_BINS + tid] + region[2 * SEL_BINS + tid] + region[3 * SEL_BINS + tid];
     sync_cluster<CS>(cluster);
   };
-  // ---- level 0: linear value bins ----
+  // ---- level 0: bins over the range of the row ----
   publish_range();
-  const float vmin = V::from_key(s.range[0]);
-  float scale = (float)(SEL_BINS - 1) / (V::from_key(s.range[1]) - vmin);
-  if (!(scale > 0.0f) || !(scale < INFINITY)) scale = 0.0f;   // flat or non-finite: one bin, the key levels decide
-  auto bin0 = [&](uint32_t u) -> unsigned { return min((unsigned)(SEL_BINS - 1), (unsigned)((V::val(u) - vmin) * scale)); };
+  const typename V::Bins bins(s.range[0], s.range[1]);
+  auto bin0 = [&](uint32_t u) -> unsigned { return bins.of(u); };
 #pragma unroll 4
   for (int i = tid; i < n; i += SEL_THREADS) atomicAdd(&my_hist[bin0(at(i))], 1u);
   publish_hist(1);
@@ -192,7 +213,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   const bool level0 = lo == 0u && hi == 0xffffffffu;
   // the threshold bin holds equal keys only: the lowest positions win, rank by rank (whole numbers in a small range have a
   // bin each)
-  const bool flat = in_bin > (unsigned)SEL_TIES || (level0 && V::whole && s.range[1] - s.range[0] < (unsigned)SEL_BINS);
+  const bool flat = in_bin > (unsigned)SEL_TIES || (level0 && bins.single());
 
   // ---- where every element stands: above the threshold bin, in it, below; one bit per element ----
   auto standing = [&](uint32_t u, bool& above, bool& member) {
@@ -254,11 +275,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       __syncthreads();
     }
     // the members' place within the threshold bin: ranks have to be counted out only in the sub-bin of the last one taken
-    auto sub_of = [&](unsigned k) -> unsigned {
-      return level0 && scale > 0.0f
-                 ? min((unsigned)(SEL_SUB - 1), (unsigned)max(0.0f, ((V::from_key(k) - vmin) * scale - (float)T0) * (float)SEL_SUB))
-                 : 0u;
-    };
+    auto sub_of = [&](unsigned k) -> unsigned { return level0 ? bins.sub(k, T0) : 0u; };
     for (unsigned t = tid; t < n_all; t += SEL_THREADS) atomicAdd(&s.sub[sub_of(all[t].x)], 1u);
     __syncthreads();
     if (warp == 0) {   // lane l: sub-bins 2l, 2l + 1

@@ -182,6 +182,19 @@ def test_topk_short_rows_tie_paths(ops, oracle, L, k, case):
     assert torch.equal(out.cpu(), oracle.topk(x, k))
 
 
+@pytest.mark.parametrize("L,k", [(3, 2), (100, 30), (5000, 1100), (40000, 4000)])
+@pytest.mark.parametrize("low", [0, (1 << 24) - 2, (1 << 25) + 1, -(1 << 25) - 7, -(1 << 31), (1 << 31) - 100000])
+def test_topk_whole_numbers_at_any_size(ops, oracle, L, k, low):
+    """int32 rows that 32-bit floats cannot hold, on both sides of 256 distinct values (a bin per value below), and rows from
+    end to end of the type."""
+    g = torch.Generator().manual_seed(L + k)
+    for span in (3, 256, 257, 100000, (1 << 32) - 1):
+        lo, hi = (low, min(low + span, 1 << 31)) if span < 1 << 31 else (-(1 << 31), 1 << 31)
+        x = torch.randint(lo, hi, (2, L), generator=g, dtype=torch.int64).to(torch.int32)
+        x[0, 0], x[0, -1] = hi - 1, lo
+        assert torch.equal(ops.topk(x.to(DEV), k).cpu(), oracle.topk(x, k)), span
+
+
 def test_topk_3d_strided_rows(ops, oracle):
     g = torch.Generator().manual_seed(5)
     x = torch.randint(0, 97, (2, 4, 3000), generator=g, dtype=torch.int32)
