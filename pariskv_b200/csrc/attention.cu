@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
       const uint32_t* qrow = reinterpret_cast<const uint32_t*>(p.q + ((int64_t)b * p.Hq + h * p.G + (head_ok ? g : 0)) * 128);
 #pragma unroll
       for (int k = 0; k < 8; k++) {
-        qa[k][0] = head_ok ? __ldg(qrow + 8 * k + t) : 0u;
-        qa[k][1] = head_ok ? __ldg(qrow + 8 * k + 4 + t) : 0u;
+        qa[k][0] = head_ok ? qrow[8 * k + t] : 0u;
+        qa[k][1] = head_ok ? qrow[8 * k + 4 + t] : 0u;
       }
     }
     float oacc[16][4];
@@ -342,8 +342,8 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
         if (g < n_heads) {
           const uint4* qp =
               reinterpret_cast<const uint4*>(p.q + ((int64_t)b * p.Hq + h * p.G + qg * ATT_GQ + g) * 128 + 16 * s);
-          unpack8f(__ldg(qp), qf[g]);
-          unpack8f(__ldg(qp + 1), qf[g] + 8);
+          unpack8f(qp[0], qf[g]);
+          unpack8f(qp[1], qf[g] + 8);
         } else {
 #pragma unroll
           for (int i = 0; i < 16; i++) qf[g][i] = 0.0f;

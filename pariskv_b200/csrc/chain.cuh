@@ -135,12 +135,12 @@ __device__ __forceinline__ float rerank_one(const RerankSmem& sm, const RerankAr
     const uint4* wp = reinterpret_cast<const uint4*>(w + key * 16);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      const uint4 v = __ldg(cp + i);
+      const uint4 v = cp[i];
       code[4 * i] = v.x, code[4 * i + 1] = v.y, code[4 * i + 2] = v.z, code[4 * i + 3] = v.w;
     }
 #pragma unroll
     for (int i = 0; i < 2; i++) {
-      const uint4 v = __ldg(wp + i);
+      const uint4 v = wp[i];
       wt[4 * i] = v.x, wt[4 * i + 1] = v.y, wt[4 * i + 2] = v.z, wt[4 * i + 3] = v.w;
     }
   } else {
@@ -189,9 +189,9 @@ __device__ __forceinline__ float rerank_one(const RerankSmem& sm, const RerankAr
 // lane to lane costs more instructions than the query's shared-memory reads.
 constexpr int LEV2_BYTES = 256 * 32 * 4;
 
-__device__ __forceinline__ void build_lev2(uint32_t* lev2, const uint16_t* __restrict__ centers, int tid, int nthreads) {
+__device__ __forceinline__ void build_lev2(uint32_t* lev2, const uint16_t* centers, int tid, int nthreads) {
   for (int v = tid >> 5; v < 256; v += nthreads >> 5) {
-    const uint32_t a = __ldg(centers + (v & 7)), b = __ldg(centers + ((v >> 4) & 7));
+    const uint32_t a = centers[v & 7], b = centers[(v >> 4) & 7];
     lev2[v * 32 + (tid & 31)] = ((v & 8) ? a : a ^ 0x8000u) | (((v & 0x80) ? b : b ^ 0x8000u) << 16);
   }
 }
@@ -255,12 +255,12 @@ struct QueryLoads {
 __device__ __forceinline__ void load_queries(QueryLoads& ql, const ChainQuery& cq, int b, int h, int G, int g0) {
   const uint16_t* q = cq.queries + ((int64_t)b * cq.Hq + (int64_t)h * G) * 128 + 4 * (threadIdx.x & 31);
 #pragma unroll
-  for (int k = 0; k < 8; k++) ql.raw[k] = __ldg(reinterpret_cast<const uint2*>(q + min(g0 + k, G - 1) * 128));
+  for (int k = 0; k < 8; k++) ql.raw[k] = *reinterpret_cast<const uint2*>(q + min(g0 + k, G - 1) * 128);
 }
 __device__ __forceinline__ void load_query(QueryLoads& ql, const ChainQuery& cq, int b, int h, int G) {
   if (threadIdx.x >= 32) return;
   load_queries(ql, cq, b, h, G, 0);
-  ql.signs = __ldg(reinterpret_cast<const uint2*>(cq.signs + 4 * threadIdx.x));
+  ql.signs = *reinterpret_cast<const uint2*>(cq.signs + 4 * threadIdx.x);
 }
 // Warp 0 averages the group's queries, normalises and rotates the mean into s_q.
 __device__ __forceinline__ void prepare_query(PreparedQuery& pq, QueryLoads& ql, const ChainQuery& cq, int b, int h, int G,
@@ -433,10 +433,10 @@ __device__ __forceinline__ void rerank_list(int n_list, const uint8_t* k4, const
   auto fetch = [&](int base) {   // out of range: the list's last candidate again
 #pragma unroll
     for (int i = 0; i < 4; i++)
-      in[i] = __ldg(reinterpret_cast<const uint4*>(k4 + (int64_t)key_at(min(base + 8 * i + (lane >> 2), n_list - 1)) * 64) + (lane & 3));
+      in[i] = reinterpret_cast<const uint4*>(k4 + (int64_t)key_at(min(base + 8 * i + (lane >> 2), n_list - 1)) * 64)[lane & 3];
 #pragma unroll
     for (int i = 0; i < 2; i++)
-      in[4 + i] = __ldg(reinterpret_cast<const uint4*>(w + (int64_t)key_at(min(base + 16 * i + (lane >> 1), n_list - 1)) * 16) + (lane & 1));
+      in[4 + i] = reinterpret_cast<const uint4*>(w + (int64_t)key_at(min(base + 16 * i + (lane >> 1), n_list - 1)) * 16)[lane & 1];
   };
   if (warp * 32 < n_list) fetch(warp * 32);
 #pragma unroll 1

@@ -23,9 +23,8 @@ struct Tiers {
 
 // From a given cluster order (the collision_fused op): one block per (batch, head, subspace).
 template <typename IdT>
-__global__ void __launch_bounds__(256) lut_from_sorted_kernel(const IdT* __restrict__ ids,
-                                                              const int32_t* __restrict__ counts, int NC,
-                                                              Tiers tiers, uint32_t* __restrict__ lut) {
+__global__ void __launch_bounds__(256) lut_from_sorted_kernel(const IdT* ids, const int32_t* counts, int NC, Tiers tiers,
+                                                              uint32_t* lut) {
   __shared__ long long warp_tot[8];
   __shared__ unsigned mask[256];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -94,21 +93,21 @@ __global__ void __launch_bounds__(256) rank_kernel(RankParams p) {
   const int sub = (int)(blk & 15);
   pdl_wait();     // first kernel of the chain: its inputs come from kernels outside the chain
   pdl_trigger();
-  const unsigned my_cnt = p.counts ? (unsigned)__ldg(p.counts + blk * 256 + c) : 0u;
+  const unsigned my_cnt = p.counts ? (unsigned)p.counts[blk * 256 + c] : 0u;
   if (p.queries) {
     if (c < 32) {
       const int s = c & 7;
       const int b = (int)(bh / p.H), h = (int)(bh % p.H);
       const uint16_t* q = p.queries + ((int64_t)b * p.Hq + (int64_t)h * p.G) * 128 + 16 * s;
       float x[16], sg[16], acc[16];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(p.signs + 16 * s)), sg);
-      unpack8(__ldg(reinterpret_cast<const uint4*>(p.signs + 16 * s) + 1), sg + 8);
+      unpack8(reinterpret_cast<const uint4*>(p.signs + 16 * s)[0], sg);
+      unpack8(reinterpret_cast<const uint4*>(p.signs + 16 * s)[1], sg + 8);
 #pragma unroll
       for (int i = 0; i < 16; i++) acc[i] = 0.0f;
       for (int g = 0; g < p.G; g++) {  // fp32 sum over the group, g ascending
         float v[16];
-        unpack8(__ldg(reinterpret_cast<const uint4*>(q + g * 128)), v);
-        unpack8(__ldg(reinterpret_cast<const uint4*>(q + g * 128) + 1), v + 8);
+        unpack8(reinterpret_cast<const uint4*>(q + g * 128)[0], v);
+        unpack8(reinterpret_cast<const uint4*>(q + g * 128)[1], v + 8);
 #pragma unroll
         for (int i = 0; i < 16; i++) acc[i] = __fadd_rn(acc[i], v[i]);
       }
@@ -216,18 +215,18 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
 #pragma unroll
     for (int j = 0; j < 16; j++) {
       const int64_t v = w0 + 32 * j + lane;
-      r[j] = (v < v_end) ? __ldg(reinterpret_cast<const uint4*>(base + v * 16)) : make_uint4(0, 0, 0, 0);
+      r[j] = (v < v_end) ? *reinterpret_cast<const uint4*>(base + v * 16) : make_uint4(0, 0, 0, 0);
     }
   } else if (LAYOUT == 0) {
     const int64_t v0 = v_begin + 16 * (int64_t)tid;
 #pragma unroll
     for (int s = 0; s < 16; s++)
-      r[s] = (v0 < v_end) ? __ldg(reinterpret_cast<const uint4*>(base + s * p.c_s + v0)) : make_uint4(0, 0, 0, 0);
+      r[s] = (v0 < v_end) ? *reinterpret_cast<const uint4*>(base + s * p.c_s + v0) : make_uint4(0, 0, 0, 0);
   }
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.lut + (int64_t)bh * p.B * 64);
     uint4* dst = reinterpret_cast<uint4*>(s_lut);
-    for (int i = tid; i < p.B * 16; i += 256) dst[i] = __ldg(src + i);
+    for (int i = tid; i < p.B * 16; i += 256) dst[i] = src[i];
   }
   __syncthreads();
 
@@ -247,7 +246,7 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
       const int64_t vn = v0 + 16 * 256;
       if (vn < v_end) {
 #pragma unroll
-        for (int s = 0; s < 16; s++) r[s] = __ldg(reinterpret_cast<const uint4*>(base + s * p.c_s + vn));
+        for (int s = 0; s < 16; s++) r[s] = *reinterpret_cast<const uint4*>(base + s * p.c_s + vn);
       }
       const int64_t key0 = v0 - p.mis;
       if (live) {
@@ -279,7 +278,7 @@ __global__ void __launch_bounds__(256, 2) collision_kernel(CollParams p) {
 #pragma unroll
         for (int j = 0; j < 16; j++) {
           const int64_t v = wn + 32 * j + lane;
-          r[j] = (v < v_end) ? __ldg(reinterpret_cast<const uint4*>(base + v * 16)) : make_uint4(0, 0, 0, 0);
+          r[j] = (v < v_end) ? *reinterpret_cast<const uint4*>(base + v * 16) : make_uint4(0, 0, 0, 0);
         }
       }
 #pragma unroll
@@ -347,7 +346,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
   auto load_codes = [&](uint4 (&r)[4], int v0) {
 #pragma unroll
     for (int j = 0; j < 4; j++)   // past the end: the last key again, its count unused
-      r[j] = __ldg(reinterpret_cast<const uint4*>(base) + min(v0 + 32 * j, n_keys - 1));
+      r[j] = reinterpret_cast<const uint4*>(base)[min(v0 + 32 * j, n_keys - 1)];
   };
   if (LAYOUT == 1) {
     load_codes(r0, warp * 128 + lane);
@@ -358,7 +357,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
   if (!early) load_query(ql, cq, b, h, p.G);
   {
     const int4* cp = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
-    const int4 c0 = __ldg(cp), c1 = __ldg(cp + 1);   // cluster sizes of this warp's subspace
+    const int4 c0 = cp[0], c1 = cp[1];   // cluster sizes of this warp's subspace
     unsigned* my = s_sizes + warp * 256;
     if (!early) prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     if (warp == 0 && blockIdx.x == 0) publish_query(pq, cq, bh);
@@ -396,7 +395,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
       uint32_t acc[4] = {0, 0, 0, 0};
 #pragma unroll 4
       for (int s = 0; s < 16; s++) {
-        const uint4 w = __ldg(reinterpret_cast<const uint4*>(base + s * p.c_s + v0));
+        const uint4 w = *reinterpret_cast<const uint4*>(base + s * p.c_s + v0);
         acc[0] += tier_bytes(w.x, s_lut + s * 128, p.c256), acc[1] += tier_bytes(w.y, s_lut + s * 128, p.c256);
         acc[2] += tier_bytes(w.z, s_lut + s * 128, p.c256), acc[3] += tier_bytes(w.w, s_lut + s * 128, p.c256);
       }
@@ -589,10 +588,9 @@ int chain_layout(const pk_tensor* codebook, int* layout) {
 
 namespace {
 // One block per (batch, head): bin `tid` summed over the chunks that hold keys of this sample.
-__global__ void __launch_bounds__(256) hist_reduce_kernel(const uint32_t* __restrict__ chunk_hist, int64_t n_chunks,
+__global__ void __launch_bounds__(256) hist_reduce_kernel(const uint32_t* chunk_hist, int64_t n_chunks,
                                                           int64_t chunk_keys, int mis, int H, int64_t N,
-                                                          const int32_t* __restrict__ n_dev,
-                                                          uint32_t* __restrict__ local_hist) {
+                                                          const int32_t* n_dev, uint32_t* local_hist) {
   const int64_t bh = blockIdx.x;
   const int tid = threadIdx.x;
   pdl_wait();
@@ -605,11 +603,11 @@ __global__ void __launch_bounds__(256) hist_reduce_kernel(const uint32_t* __rest
   for (; c + 8 <= live; c += 8) {
     unsigned v[8];
 #pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = __ldg(hp + (c + i) * 256);
+    for (int i = 0; i < 8; i++) v[i] = hp[(c + i) * 256];
 #pragma unroll
     for (int i = 0; i < 8; i++) t += v[i];
   }
-  for (; c < live; c++) t += __ldg(hp + c * 256);
+  for (; c < live; c++) t += hp[c * 256];
   local_hist[bh * 256 + tid] = t;
 }
 }  // namespace

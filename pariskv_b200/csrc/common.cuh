@@ -75,6 +75,9 @@ inline int elem_size(int dtype) {
 // no launch of the running step writes: a caller who has not asked for it may have written those tensors a launch ago.
 // EVERY kernel launched through launch_chain() must call pdl_wait() before it reads or writes anything an earlier
 // kernel may touch: a kernel that skipped the wait would break the chain for its successors.
+// Such a kernel is resident while its predecessor still writes, so nothing that it reads is read-only for its lifetime: it
+// uses plain loads, no __ldg and no __restrict__ on what it only reads (both become non-coherent loads, which need not see
+// those writes; the compiler may also move the latter's above the wait).
 bool pdl_enabled();
 bool pdl_early();
 

@@ -29,7 +29,7 @@ constexpr int EN_KEYS = EN_THREADS / 4;   // keys per block and round
 
 __device__ __forceinline__ void load_key32(uint4 (&raw)[4], const uint16_t* row, int s) {
 #pragma unroll
-  for (int i = 0; i < 4; i++) raw[i] = __ldg(reinterpret_cast<const uint4*>(row + 32 * s) + i);
+  for (int i = 0; i < 4; i++) raw[i] = reinterpret_cast<const uint4*>(row + 32 * s)[i];
 }
 
 // KEY_MAJOR: records stored key by key ([..,L,16(,4)] contiguous over subspaces), so a lane's share of a record is one
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(EN_THREADS, 2) prefill_kernel(PrefillParams p)
   auto load_v = [&](int64_t t0) {
 #pragma unroll
     for (int i = 0; i < 4; i++)
-      vr[i] = __ldg(reinterpret_cast<const uint4*>(vb + min(t0 + warp * 8 + 2 * i + (lane >> 4), end - 1) * p.v_l) + (lane & 15));
+      vr[i] = reinterpret_cast<const uint4*>(vb + min(t0 + warp * 8 + 2 * i + (lane >> 4), end - 1) * p.v_l)[lane & 15];
   };
   load_key32(kr, kb + min(begin + grp, end - 1) * p.k_l, s);
   load_v(begin);
@@ -226,8 +226,8 @@ __global__ void __launch_bounds__(256) count_kernel(const uint8_t* codes, int64_
 
 // One warp per (batch, KV head), four dims per lane.  What bounds it is the latency of its loads: those of eight queries go
 // out together (16 serial sums in 8 lanes before: 5.6 us for 8 heads of 4 queries on B200, 2.6 now).
-__global__ void __launch_bounds__(32) query_prep_kernel(const uint16_t* __restrict__ queries, int Hq, int H, int G, float inv_g,
-                                                        const uint16_t* __restrict__ signs, uint16_t* q_blocks,
+__global__ void __launch_bounds__(32) query_prep_kernel(const uint16_t* queries, int Hq, int H, int G, float inv_g,
+                                                        const uint16_t* signs, uint16_t* q_blocks,
                                                         uint16_t* q_norm, uint16_t* query_avg) {
   const int lane = threadIdx.x;
   const int bh = blockIdx.x, b = bh / H, h = bh % H;
@@ -317,13 +317,13 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
     const uint16_t* kr = p.k_row + b * p.kr_b + h * p.kr_h;
     const uint4* vr = reinterpret_cast<const uint4*>(p.v_row + b * p.vr_b + h * p.vr_h);
     // the rows themselves: lanes 0-15 carry K, lanes 16-31 carry V
-    const uint4 cp = __ldg((lane < 16 ? reinterpret_cast<const uint4*>(kr) : vr) + l);
+    const uint4 cp = (lane < 16 ? reinterpret_cast<const uint4*>(kr) : vr)[l];
     uint4 raw[4];
     load_key32(raw, kr, s);
     RotateLane rl;
     make_rotate_lane(rl, p.signs, s);
     float y[8];
-    unpack8(__ldg(vr + l), y);
+    unpack8(vr[l], y);
     if (ok) reinterpret_cast<uint4*>((lane < 16 ? wk : wv) + (int64_t)pos * 128)[l] = cp;
     // ||v||: fp32, pairwise tree over adjacent dimensions
 #pragma unroll

@@ -10,15 +10,14 @@ namespace {
 
 __device__ __forceinline__ uint4 ld_stream(const uint4* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
 }
 
-__global__ void __launch_bounds__(256) h2d_gather_kernel(const uint4* __restrict__ src_k, const uint4* __restrict__ src_v,
-                                                         const int64_t* __restrict__ idx, uint4* __restrict__ dst_k,
-                                                         uint4* __restrict__ dst_v, int64_t n_bh, int64_t src_len,
+__global__ void __launch_bounds__(256) h2d_gather_kernel(const uint4* src_k, const uint4* src_v, const int64_t* idx,
+                                                         uint4* dst_k, uint4* dst_v, int64_t n_bh, int64_t src_len,
                                                          int64_t dst_len, int64_t K) {
   const int lane = threadIdx.x & 31;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -31,7 +30,7 @@ __global__ void __launch_bounds__(256) h2d_gather_kernel(const uint4* __restrict
   pdl_trigger();
   for (int64_t r = warp; r < total; r += n_warps) {
     const int64_t bh = r / K, j = r - bh * K;
-    const int64_t row = __ldg(idx + r);
+    const int64_t row = idx[r];
     if (row < 0 || row >= src_len) continue;  // out-of-range index: row left untouched
     dst[(bh * dst_len + j) * 16 + l] = ld_stream(src + (bh * src_len + row) * 16 + l);
   }
@@ -51,7 +50,7 @@ __global__ void __launch_bounds__(256) h2d_gather_packed_kernel(
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t j = warp; j < n; j += n_warps) {
-    const int64_t row = __ldg(indices + in_base + j);
+    const int64_t row = indices[in_base + j];
     if (row < 0 || row >= src_len) continue;
     dst[(out_base + j) * 16 + l] = ld_stream(src + (vh * src_len + row) * 16 + l);
   }
@@ -70,7 +69,7 @@ __global__ void __launch_bounds__(32) append_kv_kernel(const uint4* __restrict__
   if (row < 0 || row >= cap) return;
   const uint4* src = lane < 16 ? k_row + b * k_b + h * k_h : v_row + b * v_b + h * v_h;
   uint4* dst = (lane < 16 ? wk : wv) + b * w_b + h * w_h + row * w_l;
-  dst[l] = __ldg(src + l);
+  dst[l] = src[l];
 }
 
 }  // namespace

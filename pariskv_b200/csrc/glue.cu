@@ -19,10 +19,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 // rotate-half partners (d xor 64) sit in lane L xor 16.
 //   y   = bf16( x * rsqrt(mean(x^2) + eps) * w[head] )
 //   out = bf16( y * cos + y[d xor 64] * sin )            (the sign of rotate-half is folded into sin by the caller)
-__global__ void __launch_bounds__(128) qk_norm_rope_kernel(const uint16_t* __restrict__ qkv, int64_t row_stride,
-                                                           const uint16_t* __restrict__ w, const uint16_t* __restrict__ cosv,
-                                                           const uint16_t* __restrict__ sinv, int64_t cs_stride,
-                                                           uint16_t* __restrict__ out, int heads, int64_t n_warps, float eps) {
+__global__ void __launch_bounds__(128) qk_norm_rope_kernel(const uint16_t* qkv, int64_t row_stride, const uint16_t* w,
+                                                           const uint16_t* cosv, const uint16_t* sinv, int64_t cs_stride, uint16_t* out, int heads, int64_t n_warps, float eps) {
   pdl_wait();
   pdl_trigger();
   const int64_t wid = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -31,11 +29,13 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kernel(const uint16_t* __res
   const int64_t b = wid / heads;
   const int hd = (int)(wid % heads);
   const uint2 raw = *reinterpret_cast<const uint2*>(qkv + b * row_stride + (int64_t)hd * 128 + 4 * lane);
+  const uint2 wr = *reinterpret_cast<const uint2*>(w + (int64_t)hd * 128 + 4 * lane);
+  const uint2 cr = *reinterpret_cast<const uint2*>(cosv + b * cs_stride + 4 * lane);
+  const uint2 sr = *reinterpret_cast<const uint2*>(sinv + b * cs_stride + 4 * lane);
   float x[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16),
                 __uint_as_float(raw.y & 0xffff0000u)};
   const float ss = warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
   const float rstd = rsqrtf(ss * (1.0f / 128.0f) + eps);
-  const uint2 wr = *reinterpret_cast<const uint2*>(w + (int64_t)hd * 128 + 4 * lane);
   const float wf[4] = {__uint_as_float(wr.x << 16), __uint_as_float(wr.x & 0xffff0000u), __uint_as_float(wr.y << 16),
                        __uint_as_float(wr.y & 0xffff0000u)};
   float y[4], yr[4];
@@ -43,8 +43,6 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kernel(const uint16_t* __res
   for (int i = 0; i < 4; i++) y[i] = bfround(x[i] * rstd * wf[i]);
 #pragma unroll
   for (int i = 0; i < 4; i++) yr[i] = __shfl_xor_sync(0xffffffffu, y[i], 16);
-  const uint2 cr = *reinterpret_cast<const uint2*>(cosv + b * cs_stride + 4 * lane);
-  const uint2 sr = *reinterpret_cast<const uint2*>(sinv + b * cs_stride + 4 * lane);
   const float cf[4] = {__uint_as_float(cr.x << 16), __uint_as_float(cr.x & 0xffff0000u), __uint_as_float(cr.y << 16),
                        __uint_as_float(cr.y & 0xffff0000u)};
   const float sf[4] = {__uint_as_float(sr.x << 16), __uint_as_float(sr.x & 0xffff0000u), __uint_as_float(sr.y << 16),
@@ -59,9 +57,8 @@ __global__ void __launch_bounds__(128) qk_norm_rope_kernel(const uint16_t* __res
 }
 
 // One block per row: h = bf16(a + r) (r optional), x = bf16( h * rsqrt(mean(h^2) + eps) * w ).
-__global__ void __launch_bounds__(512) add_rmsnorm_kernel(const uint16_t* __restrict__ a, const uint16_t* __restrict__ r,
-                                                          const uint16_t* __restrict__ w, uint16_t* __restrict__ h_out,
-                                                          uint16_t* __restrict__ x_out, int n, float eps) {
+__global__ void __launch_bounds__(512) add_rmsnorm_kernel(const uint16_t* a, const uint16_t* r, const uint16_t* w,
+                                                          uint16_t* h_out, uint16_t* x_out, int n, float eps) {
   pdl_wait();
   pdl_trigger();
   const int tid = threadIdx.x;
@@ -69,6 +66,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(const uint16_t* __rest
   __shared__ float s_part[16];
   __shared__ float s_rstd;
   float ss = 0.0f;
+  const uint4 w0 = tid * 8 < n ? *reinterpret_cast<const uint4*>(w + tid * 8) : make_uint4(0, 0, 0, 0);   // under the reduction
   for (int i = tid * 8; i < n; i += 512 * 8) {
     const uint4 av = *reinterpret_cast<const uint4*>(a + base + i);
     const uint4 rv = r ? *reinterpret_cast<const uint4*>(r + base + i) : make_uint4(0, 0, 0, 0);
@@ -96,7 +94,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(const uint16_t* __rest
   const float rstd = s_rstd;
   for (int i = tid * 8; i < n; i += 512 * 8) {   // every thread re-reads the values it wrote itself
     const uint4 hv = *reinterpret_cast<const uint4*>(h_out + base + i);
-    const uint4 wv = *reinterpret_cast<const uint4*>(w + i);
+    const uint4 wv = i == tid * 8 ? w0 : *reinterpret_cast<const uint4*>(w + i);
     const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w}, ww[4] = {wv.x, wv.y, wv.z, wv.w};
     uint32_t ow[4];
 #pragma unroll
@@ -110,7 +108,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(const uint16_t* __rest
 }
 
 // out[row][i] = bf16( bf16(silu(g[row][i])) * u[row][i] ), g = gu[row][0:F], u = gu[row][F:2F]
-__global__ void __launch_bounds__(256) silu_mul_kernel(const uint16_t* __restrict__ gu, uint16_t* __restrict__ out, int F) {
+__global__ void __launch_bounds__(256) silu_mul_kernel(const uint16_t* gu, uint16_t* out, int F) {
   pdl_wait();
   pdl_trigger();
   const int64_t row = blockIdx.y;
@@ -211,9 +209,9 @@ extern "C" int pk_silu_mul(const pk_tensor* gate_up, const pk_tensor* out, void*
 // ---- matrix-vector products of a decode step (one token): y = W x, W bf16 [O, I] row-major, fp32 accumulation ------
 // HBM-bound: a warp takes two rows, every lane keeps sixteen 16-byte streaming loads in flight, x sits in shared memory.
 // What is lost to the copy rate is the start of each launch, about 4 us where nothing overlaps it: dependent launch takes a
-// dense step of two layers (770 MB of weights) from 189 to 158 us on B200, and telling the compiler that two blocks share
-// an SM to 151.  Reloading each register as soon as it is used (272 us) and smaller blocks for an even last wave (196
-// against 189) lost.
+// dense step of two layers (770 MB of weights) from 189 to 158 us on B200, telling the compiler that two blocks share an SM
+// to 151, and x four loads at a time to 148.  Reloading each register as soon as it is used (272 us) and smaller blocks for
+// an even last wave (196 against 189) lost.
 // GATED: the rows are (o, o + F) of a stacked [gate; up] matrix and the output is silu(gate) * up, rounded like the
 // separate launches would (bf16 after the product, after silu, after the multiply).
 namespace pk {
@@ -230,8 +228,7 @@ constexpr int GV_THREADS = 256;
 constexpr int GV_UNROLL = 8;
 
 template <bool GATED>
-__global__ void __launch_bounds__(GV_THREADS, 2) gemv_kernel(const uint16_t* __restrict__ W, const uint16_t* __restrict__ x,
-                                                          uint16_t* __restrict__ out, int O, int I, int F, bool early) {
+__global__ void __launch_bounds__(GV_THREADS, 2) gemv_kernel(const uint16_t* W, const uint16_t* x, uint16_t* out, int O, int I, int F, bool early) {
   extern __shared__ __align__(16) unsigned char gv_smem[];
   uint4* xs = reinterpret_cast<uint4*>(gv_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -258,7 +255,14 @@ __global__ void __launch_bounds__(GV_THREADS, 2) gemv_kernel(const uint16_t* __r
   load_batch(lane);
   pdl_wait();
   pdl_trigger();
-  for (int c = tid; c < nchunk; c += GV_THREADS) xs[c] = __ldg(reinterpret_cast<const uint4*>(x) + c);
+  for (int c0 = tid; c0 < nchunk; c0 += 4 * GV_THREADS) {   // four loads in flight per thread
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = reinterpret_cast<const uint4*>(x)[min(c0 + u * GV_THREADS, nchunk - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (c0 + u * GV_THREADS < nchunk) xs[c0 + u * GV_THREADS] = v[u];
+  }
   __syncthreads();
   if (!live) return;
   float acc0 = 0.0f, acc1 = 0.0f;

@@ -107,6 +107,7 @@ struct SelectArgs {
   int64_t C_want;                // candidates wanted per head over the whole zone, all shards together (n_dev == null)
   int64_t K;                     // final top-K (one-launch chain); 0 = stop after the rerank
   int fill_tail;                 // rows may be longer than the candidate list: the tail gets (score -inf, key 0)
+  int early_loads;               // see pdl_early()
   const int32_t* n_dev;          // [bs] searchable keys per sample, or null
   pk_zone_schedule sched;        // candidates = zone_candidates(sched, n_dev[b]) when n_dev is set
   const uint32_t* shard_hist;    // [world][bs*H][256] histograms of every shard (exact sequence-sharded selection)

@@ -93,10 +93,10 @@ struct RotateLane {
   uint32_t flip[16];
   f32x2 side[2];
 };
-__device__ __forceinline__ void make_rotate_lane(RotateLane& rl, const uint16_t* __restrict__ signs, int s) {
+__device__ __forceinline__ void make_rotate_lane(RotateLane& rl, const uint16_t* signs, int s) {
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(signs + 32 * s) + i);
+    const uint4 a = reinterpret_cast<const uint4*>(signs + 32 * s)[i];
     rl.flip[4 * i] = a.x & 0x80008000u, rl.flip[4 * i + 1] = a.y & 0x80008000u;
     rl.flip[4 * i + 2] = a.z & 0x80008000u, rl.flip[4 * i + 3] = a.w & 0x80008000u;
   }

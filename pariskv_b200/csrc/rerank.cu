@@ -69,11 +69,10 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t bh = blockIdx.y, chunk = blockIdx.x;
   const int b = (int)(bh / a.H), h = (int)(bh % a.H);
-  // before the wait only where the collision kernel, which has waited itself, is the launch before this one
-  if (FAST && !p.shard_hist) build_lev2(lev2, a.centers, tid, CH_THREADS);
+  if (FAST && p.early_loads) build_lev2(lev2, a.centers, tid, CH_THREADS);
   pdl_wait();  // counts, histograms and query blocks come from the collision kernel
   pdl_trigger();
-  if (FAST && p.shard_hist) build_lev2(lev2, a.centers, tid, CH_THREADS);
+  if (FAST && !p.early_loads) build_lev2(lev2, a.centers, tid, CH_THREADS);
   const int64_t N = p.n_dev ? min(max((int64_t)p.n_dev[b], (int64_t)1), p.N) : p.N;
   const int64_t Nv = N + p.mis;
   const int64_t v_begin = chunk * p.chunk_keys;
@@ -126,7 +125,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
       g_tot = 0;
       const int64_t rows = (int64_t)gridDim.y;  // bs*H
       for (int r = 0; r < p.world; r++) {
-        const unsigned v = __ldg(p.shard_hist + ((int64_t)r * rows + bh) * 256 + tid);
+        const unsigned v = p.shard_hist[((int64_t)r * rows + bh) * 256 + tid];
         g_tot += v;
         if (r < p.rank) g_before += v;
       }

@@ -211,6 +211,7 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
   }
   sa.cand_out = cd, sa.scores_f32 = sc;
   sa.fill_tail = varlen;
+  sa.early_loads = pdl_early();
   sa.n_cand_out = n_cand ? n_cand : (int32_t*)(ws + lay.n_cand);
   ra.cand = nullptr;
   ra.q_blocks = qb, ra.q_norm = qn, ra.centers = (const uint16_t*)a.mag_centers->data;

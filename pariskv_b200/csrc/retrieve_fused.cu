@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   // the zone length are asked for together
   if (!early) load_query(ql, cq, b, h, p.G);
   const int4* sizes = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
-  const int4 c0 = __ldg(sizes), c1 = __ldg(sizes + 1);   // of this warp's subspace
+  const int4 c0 = sizes[0], c1 = sizes[1];   // of this warp's subspace
   const int64_t N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
   const int64_t C_want = cq.n_dev ? min((int64_t)zone_candidates(cq.sched, N), p.C) : p.C_want;
   const int span = (int)(((N + CS - 1) / CS + 15) / 16 * 16);
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
     if (n_keys > 0)
 #pragma unroll
       for (int j = 0; j < 4; j++)   // past the end: the last key again, its count unused
-        r[j] = __ldg(reinterpret_cast<const uint4*>(codes) + min(v0 + 32 * j, n_keys - 1));
+        r[j] = reinterpret_cast<const uint4*>(codes)[min(v0 + 32 * j, n_keys - 1)];
   };
   load_codes(r0, warp * 128 + lane);
   load_codes(r1, warp * 128 + lane + STEP);

@@ -8,11 +8,11 @@
 namespace pk {
 
 // Position of `key` in the ascending row a[0..n): first element >= key.
-__device__ __forceinline__ int lower_bound_i64(const int64_t* __restrict__ a, int n, int64_t key) {
+__device__ __forceinline__ int lower_bound_i64(const int64_t* a, int n, int64_t key) {
   int lo = 0, hi = n;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (__ldg(a + mid) < key) lo = mid + 1; else hi = mid;
+    if (a[mid] < key) lo = mid + 1; else hi = mid;
   }
   return lo;
 }
@@ -254,12 +254,9 @@ constexpr int TP_THREADS = 512;
 constexpr int TP_WORDS_MAX = 8;   // words per thread: rows of up to 8192 bf16
 constexpr int TP_WORLD_MAX = 16;
 
-__global__ void __launch_bounds__(TP_THREADS) tp_allreduce_kernel(const unsigned* __restrict__ partial,
-                                                                  const unsigned* __restrict__ residual,
-                                                                  unsigned* __restrict__ out, int n32, PeerSet peers,
+__global__ void __launch_bounds__(TP_THREADS) tp_allreduce_kernel(const unsigned* partial, const unsigned* residual, unsigned* out, int n32, PeerSet peers,
                                                                   int64_t gather_off, int64_t area_bytes, int rank, int world,
-                                                                  PeerCtl* ctl, const unsigned* __restrict__ norm_w,
-                                                                  unsigned* __restrict__ normed, float eps, int gather_only) {
+                                                                  PeerCtl* ctl, const unsigned* norm_w, unsigned* normed, float eps, int gather_only) {
   const int tid = threadIdx.x;
   __shared__ unsigned s_epoch;
   __shared__ float s_part[TP_THREADS / 32];

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
   for (int base = tid; base < n; base += 8 * SEL_THREADS) {   // eight loads in flight per thread
     uint32_t u[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) u[j] = __ldg(in + min(base + j * SEL_THREADS, n - 1));
+    for (int j = 0; j < 8; j++) u[j] = in[min(base + j * SEL_THREADS, n - 1)];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       const int i = base + j * SEL_THREADS;
@@ -64,13 +64,13 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
     }
   }
   const int64_t* map = p.map ? p.map + row * p.map_stride + begin : nullptr;
-  auto out_of = [&](int i) -> int64_t { return map ? __ldg(map + i) : begin + i; };
+  auto out_of = [&](int i) -> int64_t { return map ? map[i] : begin + i; };
   if (cached)
     cluster_select<CS, Row>(cluster, s, region, words, TK_WORDS, rank, n, K, p.out + row * p.k,
                             [&](int i) -> uint32_t { return cache[i]; }, out_of, kmin, kmax);
   else
     cluster_select<CS, Row>(cluster, s, region, words, TK_WORDS, rank, n, K, p.out + row * p.k,
-                            [&](int i) -> uint32_t { return __ldg(in + i); }, out_of, kmin, kmax);
+                            [&](int i) -> uint32_t { return in[i]; }, out_of, kmin, kmax);
   if (CS > 1) cluster.barrier_wait();   // shared memory must outlive the other CTAs' reads
 }
 
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(1024) sort_by_value_kernel(const uint32_t* in,
     unsigned long long v = 0;
     if (i < k) {
       const int64_t idx = o[i];
-      v = ((unsigned long long)(is_float ? F32Row::key(__ldg(row + idx)) : I32Row::key(__ldg(row + idx))) << 32) | (0xffffffffu - (unsigned)idx);
+      v = ((unsigned long long)(is_float ? F32Row::key(row[idx]) : I32Row::key(row[idx])) << 32) | (0xffffffffu - (unsigned)idx);
     }
     sk[i] = v;
   }
