@@ -282,7 +282,8 @@ int pk_gather_kv_out_cpu(const pk_tensor* src, const pk_tensor* index, const pk_
  *             merged exactly: out = sum_r out_r * 2^(lse_r - LSE), LSE = log2 sum_r 2^lse_r
  *   workspace >= pk_attention_workspace_bytes(bs,Hq,n_window+K) bytes, device, 16-byte aligned.  Its first
  *             256-byte-rounded header (arrival counters and a status word) must be ZERO before the first
- *             call; every call leaves it zero again.  The status word (int at index bs*Hq) becomes 1 if a
+ *             call; every call leaves it zero again.  Its size follows from bs*Hq, so a workspace that has
+ *             served another bs*Hq has to be cleared before.  The status word (int at index bs*Hq) becomes 1 if a
  *             block gave up waiting for its copies (the output of that head is then not written). */
 int64_t pk_attention_workspace_bytes(int64_t bs, int64_t Hq, int64_t max_rows);
 int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* window_k, const pk_tensor* window_v,

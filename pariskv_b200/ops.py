@@ -249,7 +249,9 @@ def sparse_attention(queries, window_k, window_v, n_window, store_k=None, store_
         scale = 1.0 / math.sqrt(D)
     N = L.native()
     rows = n_window + (selected.shape[2] if selected is not None else 0)
-    ws = _scratch(queries.device, N.attention_workspace_bytes(bs, Hq, rows), "attention", scratch)
+    # the arrival counters lie in a header whose size follows from bs * Hq: calls with headers of another size would find the
+    # partial records of this one in their counters, so each size has its shared buffer
+    ws = _scratch(queries.device, N.attention_workspace_bytes(bs, Hq, rows), f"attention {(bs * Hq + 64) // 64}", scratch)
     return N.sparse_attention(queries, window_k, window_v, int(n_window), n_window_dev, int(n_window_add), store_k, store_v,
                               selected, n_sel, int(index_offset), float(scale), out, lse, ws)
 

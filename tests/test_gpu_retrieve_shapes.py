@@ -78,3 +78,16 @@ def test_attention_tile_edges(oracle, bs, H, n_window, K):
     out = ops.sparse_attention(q.to(DEV), wk.to(DEV), wv.to(DEV), n_window, *args)
     rk, rv = ([torch.cat([oracle.gather(k, sel), wk], 2), torch.cat([oracle.gather(v, sel), wv], 2)] if K else (wk, wv))
     assert (out.float().cpu() - oracle.attention(q, rk, rv)).abs().max().item() <= 2e-2
+
+
+def test_attention_shared_scratch_serves_any_batch():
+    """Calls without their own scratch, few heads first and then many: the arrival counters of the second lie where the
+    partial records of the first may have been."""
+    from pariskv_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(3)
+    for bs, H in ((1, 1), (10, 8), (1, 4), (3, 30), (40, 8), (1, 1)):
+        k, v = (torch.randn(bs, H, 150, 128, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+        q = torch.randn(bs, 1, 2 * H, 128, generator=g, device=DEV).to(torch.bfloat16)
+        s = torch.einsum("bhgd,bhnd->bhgn", q.view(bs, H, 2, 128).double(), k.double()) / 128 ** 0.5
+        ref = torch.einsum("bhgn,bhnd->bhgd", torch.softmax(s, -1), v.double()).reshape(q.shape)
+        assert (ops.sparse_attention(q, k, v, 150).double() - ref).abs().max().item() <= 2e-2, (bs, H)
