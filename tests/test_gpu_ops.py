@@ -420,6 +420,31 @@ def test_sparse_attention_interleaved_store(ops, where):
         ops.sparse_attention(q, wk, wv, 16, kv[:, :, :, 0], vals.to(DEV), sel)
 
 
+@pytest.mark.parametrize("bs,H", [(1, 4), (10, 8)])   # a tile of 128 rows per block; several tiles of 64 in a row
+@pytest.mark.parametrize("group", [1, 4, 5, 8, 9])
+def test_sparse_attention_keeps_32_bits(ops, group, bs, H):
+    """Probabilities and sums are held in 32 bits for every group size: hardly an output differs from the 64-bit result
+    rounded to bf16.  An error e of the result before its rounding changes the rounding of a share of 2 |e| / ulp of the
+    outputs.  Sums in 32 bits: |e| below 2^-18 of the absolute products' sum, which is some three times the result over rows
+    of random sign, so 2 * 3 * 2^-18 / 2^-8 = 0.6 % at the very most (measured: below 0.1 %).  Probabilities rounded to
+    bf16 change 7.8 % of these outputs."""
+    g = torch.Generator(device=DEV).manual_seed(group * 100 + bs)
+    n = 90
+    k = torch.randn(bs, H, n, 128, generator=g, device=DEV).to(torch.bfloat16)
+    v = torch.randn(bs, H, n, 128, generator=g, device=DEV).to(torch.bfloat16)
+    q = torch.randn(bs, 1, H * group, 128, generator=g, device=DEV).to(torch.bfloat16)
+    out = ops.sparse_attention(q, k, v, n)
+    s = torch.einsum("bhgd,bhnd->bhgn", q.view(bs, H, group, 128).double(), k.double()) / math.sqrt(128.0)
+    ref = torch.einsum("bhgn,bhnd->bhgd", torch.softmax(s, -1), v.double()).reshape(out.shape)
+    assert (out != ref.to(torch.bfloat16)).double().mean().item() <= 0.006
+    # an infinite value stays one: no product of the split probabilities turns it into something that is not a number
+    v[0, 0, 17, 5] = float("inf")
+    out = ops.sparse_attention(q, k, v, n)
+    hit = torch.zeros_like(out, dtype=torch.bool)
+    hit[0, 0, :group, 5] = True
+    assert torch.equal(torch.isposinf(out), hit) and not torch.isnan(out).any()
+
+
 # ---- glue kernels of the sequence-sharded form (against the torch formulation used by the gloo tests) ----
 def test_shard_pack_unpack_owned_merge(ops):
     from pariskv_b200 import dist as pkd
