@@ -275,9 +275,11 @@ class polar_cache(KV_Cache):
     def _staging_rows(self, n):
         """A device buffer [H,n,2,128] for rows on their way to the host store -> (buffer, slot of the kept pair or None).
         Two kept buffers take turns, each reused when its last copy has left it; giving every prompt a fresh tensor makes
-        the allocator hold all of those whose copies are pending.  Larger buffers are allocated per prompt."""
+        the allocator hold all of those whose copies are pending.  Larger buffers are allocated per prompt, and so are those
+        of short prompts: their copies run on the caller's stream, where the allocator keeps the order, and no event tells
+        another stream when they are done."""
         numel = self.kv_head * n * 256
-        if numel * 2 > self.STAGING_KEEP_BYTES:
+        if numel * 2 > self.STAGING_KEEP_BYTES or n < self.BULK_OFFLOAD_ROWS:
             return torch.empty(self.kv_head, n, 2, 128, dtype=self.dtype, device=self.device), None
         self._staging_turn ^= 1
         slot = self._staging[self._staging_turn]
@@ -295,8 +297,6 @@ class polar_cache(KV_Cache):
         if n < self.BULK_OFFLOAD_ROWS:
             self._wait_offload(layer)                  # an earlier bulk copy of this layer must stay ordered
             _lib.native().copy_rows(rows, dst)
-            if slot is not None:
-                slot[1] = None                         # the copy is ordered before later work of this stream
             return
         self._copy_stream.wait_stream(torch.cuda.current_stream(rows.device))
         with torch.cuda.stream(self._copy_stream):

@@ -49,3 +49,25 @@ def test_prefill_matches_oracle(oracle, P, offload):
     assert torch.equal(cache._store_v[0][:, :, :N].cpu(), vt[:, :, zone])
     counts = oracle.cluster_counts(cb[..., zone].contiguous()) if N else torch.zeros(bs, H, 16, 256, dtype=torch.int32)
     assert torch.equal(cache.cluster_key_counts_gpu[0].cpu(), counts)
+
+
+def test_short_prompts_on_several_streams_share_no_buffer():
+    """Prompts whose rows are copied on the caller's own stream: another stream may fill the next layer at the same time, so
+    their staging rows come from the allocator, not from the cache's pair of buffers."""
+    from pariskv_b200.cache_hub.polar_cache import polar_cache
+    n, H, layers = 600, 2, 4
+    cache = polar_cache(valid_start=0, layer_num=layers, batch_size=1, max_length=n + 64, num_key_value_heads=H, num_heads=4 * H,
+                        head_dim=128, dtype=torch.bfloat16, layer_mapping={str(i): DEV for i in range(layers)}, max_new_length=64,
+                        sink_size=4, local_size=16, final_topk=64, dynamic_update_interval=32, enable_offload=True)
+    g = torch.Generator(device=DEV).manual_seed(1)
+    kv = [[torch.randn(1, n, H, 128, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2)] for _ in range(layers)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for l in range(layers):
+        with torch.cuda.stream(streams[l & 1]):
+            cache.prefill_update_kv_cache(None, kv[l][0], kv[l][1], l, 0)
+    torch.cuda.synchronize()
+    assert all(buf is None for buf, _ in cache._staging)
+    for l in range(layers):
+        for rows, store in zip(kv[l], (cache.unified_keys_cpu[l], cache.unified_values_cpu[l])):
+            assert torch.equal(store[0, :, :n - 20], rows[0, 4:n - 16].transpose(0, 1).cpu())
