@@ -1232,7 +1232,8 @@ def main():
                          "(default) or through the library GEMM")
     ap.add_argument("--pdl", default="on", choices=["on", "off"],
                     help="programmatic dependent launch between the kernels of this library (a kernel's prologue, e.g. "
-                         "the first weight loads of a projection, runs under the tail of its predecessor)")
+                         "the first weight loads of a projection, runs under the tail of its predecessor); off: plain "
+                         "launches")
     ap.add_argument("--no-numa", action="store_true",
                     help="variant: do not place the pinned K/V store on the NUMA node of the GPU's host link")
     ap.add_argument("--dense", default="tp", choices=["tp", "replicated"],
@@ -1278,7 +1279,7 @@ def main():
     from pariskv_b200.build import build
     build()
     _lib.load()
-    _lib.set_pdl(args.pdl == "on")
+    _lib.set_pdl(True) if args.pdl == "on" else _lib.set_dependent_launch(False)
 
     def barrier():
         if world > 1:

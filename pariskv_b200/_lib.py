@@ -214,6 +214,12 @@ def set_pdl(on: bool):
     check(load().pk_set_pdl(int(bool(on))))
 
 
+def set_dependent_launch(on: bool):
+    """False: plain launches, each kernel after its predecessor's end.  True: dependent launch without early loads, which is
+    how the library starts (see pk_set_pdl)."""
+    check(load().pk_set_pdl(0 if on else -1))
+
+
 def timing_enable(on: bool):
     check(load().pk_timing_enable(int(bool(on))))
 

@@ -21,6 +21,24 @@ def test_workload_config_names_the_sharding():
     assert "model" not in one and one["context"] == 131072 and one["topk"] == 2048
 
 
+def test_launch_modes_reach_the_library(monkeypatch):
+    """set_pdl chooses between early loads and none, set_dependent_launch(False) plain launches."""
+    from pariskv_b200 import _lib
+
+    class Recorder:
+        def __init__(self):
+            self.modes = []
+
+        def pk_set_pdl(self, mode):
+            self.modes.append(mode)
+            return 0
+
+    lib = Recorder()
+    monkeypatch.setattr(_lib, "load", lambda: lib)
+    _lib.set_pdl(True), _lib.set_pdl(False), _lib.set_dependent_launch(False), _lib.set_dependent_launch(True)
+    assert lib.modes == [1, 0, -1, 0]
+
+
 def test_bench_help_lists_every_mode():
     out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--help"], capture_output=True, text=True,
                          timeout=120)

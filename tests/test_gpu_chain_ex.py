@@ -180,9 +180,11 @@ def test_final_selection_with_ties_and_flat_scores(ops):
     assert float(ex["scores_f32"].max() - ex["scores_f32"].min()) == 0.0
 
 
-def test_early_query_preparation_gives_the_same_chain(ops, schedule):
+@pytest.mark.parametrize("launches", [1, 3])
+def test_early_query_preparation_gives_the_same_chain(ops, schedule, launches):
     """queries_settled only moves the query preparation and the cluster sort ahead of the kernel's dependency wait:
-    candidates, scores and final indices are bit-identical, with dependent launch on or off."""
+    candidates, scores and final indices are bit-identical with plain launches, dependent launch and early loads.  Codes
+    stored plane by plane take the chain of three launches."""
     from pariskv_b200 import _lib
     g = torch.Generator().manual_seed(404)
     lens = (33000, 12000)
@@ -196,13 +198,16 @@ def test_early_query_preparation_gives_the_same_chain(ops, schedule):
     for b, n in enumerate(lens):
         ops.encode_keys(keys[b:b + 1, :, :n].to(DEV), signs, cb[b:b + 1, :, :, :n], w[b:b + 1, :, :, :n],
                         pk[b:b + 1, :, :, :n, :], cluster_counts=counts[b:b + 1])
+    if launches == 3:
+        cb = cb.contiguous()
     kv_len = torch.tensor(lens, dtype=torch.int32, device=DEV)
     import ctypes
     Cmax = int(_lib.load().pk_zone_max_candidates(ctypes.byref(schedule), Nmax))
     outs = []
+    before = _lib.launch_count()
     try:
-        for pdl in (False, True):
-            _lib.set_pdl(pdl)
+        for launch in ("plain", "dependent", "early"):
+            _lib.set_dependent_launch(False) if launch == "plain" else _lib.set_pdl(launch == "early")
             for settled in (False, True):
                 fin, n_sel, ex = ops.retrieve_ex(q, signs, cen, cb, w, pk, counts, Cmax, 512, kv_len=kv_len,
                                                  schedule=schedule, want=("cand", "scores_f32", "q_blocks", "q_norm"),
@@ -211,6 +216,7 @@ def test_early_query_preparation_gives_the_same_chain(ops, schedule):
                              ex["q_blocks"].clone(), ex["q_norm"].clone()))
     finally:
         _lib.set_pdl(False)
+    assert _lib.launch_count() - before == 6 * launches
     for o in outs[1:]:
         for a, b in zip(outs[0], o):
             assert torch.equal(a, b)
