@@ -54,7 +54,7 @@ int64_t pk_launch_count(void);
 /* Optional instrumentation, no counterpart in the reference: when enabled, every kernel launch of the
  * decode path is bracketed by CUDA events on its own stream.  pk_timing_read waits for the recorded
  * events, sums elapsed milliseconds and launch counts per stage (stage ids: 0 query prep, 1 cluster
- * ranking/table, 2 collision, 3 select+rerank, 4 final top-k, 5 attention tiles, 6 attention merge,
+ * ranking/table, 2 collision, 3 select+rerank, 4 final top-k, 5 attention, 6 unused,
  * 7 encode, 8 stand-alone top-k, 9 stand-alone rerank, 10 UVA gather, 11 cluster histogram, 12 row append,
  * 13 decode glue, 14 tensor-parallel reduce, 15 shard pack / send, 16 shard receive / merge, 17 shard owned rows,
  * 18 shard count-histogram reduce, 19 matrix-vector product, 20 adaptive-k selection,

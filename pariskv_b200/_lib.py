@@ -204,7 +204,7 @@ def launch_count() -> int:
     return int(load().pk_launch_count())
 
 
-STAGES = ["query_prep", "rank_table", "collision", "select_rerank", "final_topk", "attention", "attention_merge",
+STAGES = ["query_prep", "rank_table", "collision", "select_rerank", "final_topk", "attention", "unused",
           "encode", "topk", "rerank", "uva_gather", "count_clusters", "append", "glue", "tp_reduce",
           "shard_send", "shard_recv", "shard_owned", "hist_reduce", "gemv", "adaptive_topk", "retrieve"]
 

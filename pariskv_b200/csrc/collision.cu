@@ -62,75 +62,16 @@ __global__ void __launch_bounds__(256) lut_from_sorted_kernel(const IdT* ids, co
   }
 }
 
-// From the query (the fused chain) and/or to produce the explicit order (rank_clusters op):
-// one block per (batch, head, subspace), thread c owns cluster c.
+// The explicit order of the clusters (rank_clusters op): one block per (batch, head, subspace), thread c owns cluster c.
 // score_c = bf16(sum_j +-q_j), fp32 sum j ascending; order: score descending, id ascending.
-// With `queries` set, warp 0 first does the query preparation itself (group mean, normalise, rotate),
-// so the fused chain needs no separate query kernel; the block of subspace 0 publishes q_blocks / q_norm
-// / query_avg for the later stages.
-struct RankParams {
-  const uint16_t* queries;   // [bs][Hq][128] or null
-  const uint16_t* signs;
-  int Hq, H, G;
-  float inv_g;
-  uint16_t* q_blocks;        // [bs*H][128]: input when queries == null, output otherwise
-  uint16_t* q_norm;          // [bs*H] output (queries != null)
-  uint16_t* query_avg;       // [bs*H][128] optional output
-  const int32_t* counts;     // [bs*H][16][256] or null
-  Tiers tiers;
-  uint32_t* lut;             // [bs*H][16][64] or null
-  int64_t* sorted_ids;       // [bs*H][16][256] or null
-};
-
-__global__ void __launch_bounds__(256) rank_kernel(RankParams p) {
-  // entry o: x = sortable key ((ordered bf16 score) << 8 | (255 - o)), y = keys in cluster o
-  __shared__ __align__(16) uint2 ent[256];
-  __shared__ unsigned nib[256];
+__global__ void __launch_bounds__(256) rank_kernel(const uint16_t* q_blocks, int64_t* sorted_ids) {
+  __shared__ __align__(16) unsigned keys[256];   // (ordered bf16 score) << 8 | (255 - id)
   __shared__ float s_q[8];
   const int c = threadIdx.x;
   const int64_t blk = blockIdx.x;  // (b*H + h)*16 + subspace
-  const int64_t bh = blk >> 4;
-  const int sub = (int)(blk & 15);
-  pdl_wait();     // first kernel of the chain: its inputs come from kernels outside the chain
+  pdl_wait();
   pdl_trigger();
-  const unsigned my_cnt = p.counts ? (unsigned)p.counts[blk * 256 + c] : 0u;
-  if (p.queries) {
-    if (c < 32) {
-      const int s = c & 7;
-      const int b = (int)(bh / p.H), h = (int)(bh % p.H);
-      const uint16_t* q = p.queries + ((int64_t)b * p.Hq + (int64_t)h * p.G) * 128 + 16 * s;
-      float x[16], sg[16], acc[16];
-      unpack8(reinterpret_cast<const uint4*>(p.signs + 16 * s)[0], sg);
-      unpack8(reinterpret_cast<const uint4*>(p.signs + 16 * s)[1], sg + 8);
-#pragma unroll
-      for (int i = 0; i < 16; i++) acc[i] = 0.0f;
-      for (int g = 0; g < p.G; g++) {  // fp32 sum over the group, g ascending
-        float v[16];
-        unpack8(reinterpret_cast<const uint4*>(q + g * 128)[0], v);
-        unpack8(reinterpret_cast<const uint4*>(q + g * 128)[1], v + 8);
-#pragma unroll
-        for (int i = 0; i < 16; i++) acc[i] = __fadd_rn(acc[i], v[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < 16; i++) x[i] = bfround(__fmul_rn(acc[i], p.inv_g));
-      if (sub == 0 && p.query_avg && c < 8)
-#pragma unroll
-        for (int i = 0; i < 16; i++) p.query_avg[bh * 128 + 16 * s + i] = f2bf(x[i]);
-      const float n = rotate16(x, sg, s);
-      if (c < 8) {
-        if (sub == 0) {
-#pragma unroll
-          for (int i = 0; i < 16; i++) p.q_blocks[bh * 128 + 16 * s + i] = f2bf(x[i]);
-          if (c == 0) p.q_norm[bh] = f2bf(n);
-        }
-        if (s == (sub >> 1))
-#pragma unroll
-          for (int j = 0; j < 8; j++) s_q[j] = x[8 * (sub & 1) + j];
-      }
-    }
-  } else if (c < 8) {
-    s_q[c] = bf2f(p.q_blocks[blk * 8 + c]);
-  }
+  if (c < 8) s_q[c] = bf2f(q_blocks[blk * 8 + c]);
   __syncthreads();
   float s = 0.0f;
 #pragma unroll
@@ -143,30 +84,16 @@ __global__ void __launch_bounds__(256) rank_kernel(RankParams p) {
   if (bits == 0x8000u) bits = 0u;
   const unsigned ord = (bits & 0x8000u) ? (~bits & 0xFFFFu) : (bits | 0x8000u);
   const unsigned my_key = (ord << 8) | (unsigned)(255 - c);
-  ent[c] = make_uint2(my_key, my_cnt);
+  keys[c] = my_key;
   __syncthreads();
-  unsigned excl = 0, rank = 0;
-  const uint4* e4 = reinterpret_cast<const uint4*>(ent);
+  unsigned rank = 0;
+  const uint4* k4 = reinterpret_cast<const uint4*>(keys);
 #pragma unroll 16
-  for (int o = 0; o < 128; o++) {
-    const uint4 e = e4[o];  // two entries per 128-bit read (a broadcast: every thread reads the same word)
-    const bool b0 = e.x > my_key, b1 = e.z > my_key;
-    rank += (unsigned)b0 + (unsigned)b1;
-    excl += (b0 ? e.y : 0u) + (b1 ? e.w : 0u);
+  for (int o = 0; o < 64; o++) {
+    const uint4 k = k4[o];  // four keys per 128-bit read (a broadcast: every thread reads the same words)
+    rank += (unsigned)(k.x > my_key) + (unsigned)(k.y > my_key) + (unsigned)(k.z > my_key) + (unsigned)(k.w > my_key);
   }
-  if (p.sorted_ids) p.sorted_ids[blk * 256 + rank] = c;
-  if (p.lut) {
-    unsigned wgt = 0;
-    for (int t = 0; t < p.tiers.n; t++) wgt += ((long long)excl < p.tiers.t[t]);
-    nib[c] = wgt;
-    __syncthreads();
-    if (c < 64) {
-      uint32_t w = 0;
-#pragma unroll
-      for (int i = 0; i < 4; i++) w |= nib[c * 4 + i] << (8 * i);
-      p.lut[blk * 64 + c] = w;
-    }
-  }
+  sorted_ids[blk * 256 + rank] = c;
 }
 
 // ---- the streaming count --------------------------------------------------------------------------
@@ -361,7 +288,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
     unsigned* my = s_sizes + warp * 256;
     if (!early) prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     if (warp == 0 && blockIdx.x == 0) publish_query(pq, cq, bh);
-    if (tid == 32) load_tiers(cq, cq.n_dev || cq.n_plan <= 0 ? (long long)N : cq.n_plan, s_tiers);
+    if (tid == 32) load_tiers(cq, (long long)N, s_tiers);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
     *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
     for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
@@ -483,23 +410,8 @@ int64_t collision_chunk_keys(int64_t bs_h, int64_t Nv) {
   if (n_chunks < 1) n_chunks = 1;
   int64_t chunk = (Nv + n_chunks - 1) / n_chunks;
   chunk = ((chunk + 4095) / 4096) * 4096;
-  if (chunk > 32768) chunk = 32768;  // the selection kernel keeps one int per key of a chunk in shared memory
+  if (chunk > 32768) chunk = 32768;  // long rows: more blocks, so that the last wave is short
   return chunk;
-}
-
-int launch_rank(const uint16_t* queries, const uint16_t* signs, int Hq, int H, uint16_t* q_blocks, uint16_t* q_norm,
-                uint16_t* query_avg, const int32_t* counts, const int64_t* tier_counts, int n_tiers, int64_t bs_h,
-                uint32_t* lut, int64_t* sorted_ids, cudaStream_t st) {
-  RankParams p;
-  p.queries = queries, p.signs = signs, p.Hq = Hq, p.H = H, p.G = H > 0 ? Hq / H : 1;
-  p.inv_g = 1.0f / (float)p.G;
-  p.q_blocks = q_blocks, p.q_norm = q_norm, p.query_avg = query_avg, p.counts = counts;
-  p.tiers = make_tiers(tier_counts, n_tiers);
-  p.lut = lut, p.sorted_ids = sorted_ids;
-  StageTimer tm(ST_RANK, st);
-  if (launch_chain(rank_kernel, dim3((unsigned)(bs_h * 16)), dim3(256), 0, st, p) != cudaSuccess)
-    return check_launch("rank_clusters");
-  return check_launch("rank_clusters");
 }
 
 // Launch geometry of the several-launch chain: about one block per SM over the whole grid, one histogram row each; both
@@ -587,36 +499,30 @@ int chain_layout(const pk_tensor* codebook, int* layout) {
 }
 
 namespace {
-// One block per (batch, head): bin `tid` summed over the chunks that hold keys of this sample.
-__global__ void __launch_bounds__(256) hist_reduce_kernel(const uint32_t* chunk_hist, int64_t n_chunks,
-                                                          int64_t chunk_keys, int mis, int H, int64_t N,
-                                                          const int32_t* n_dev, uint32_t* local_hist) {
+// One block per (batch, head): bin `tid` summed over the chunks.
+__global__ void __launch_bounds__(256) hist_reduce_kernel(const uint32_t* chunk_hist, int64_t n_chunks, uint32_t* local_hist) {
   const int64_t bh = blockIdx.x;
   const int tid = threadIdx.x;
   pdl_wait();
   pdl_trigger();
-  const int64_t n = n_dev ? min(max((int64_t)n_dev[bh / H], (int64_t)1), N) : N;
-  const int64_t live = min(n_chunks, (n + mis + chunk_keys - 1) / chunk_keys);
   const uint32_t* hp = chunk_hist + bh * n_chunks * 256 + tid;
   unsigned t = 0;
   int64_t c = 0;
-  for (; c + 8 <= live; c += 8) {
+  for (; c + 8 <= n_chunks; c += 8) {
     unsigned v[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = hp[(c + i) * 256];
 #pragma unroll
     for (int i = 0; i < 8; i++) t += v[i];
   }
-  for (; c < live; c++) t += hp[c * 256];
+  for (; c < n_chunks; c++) t += hp[c * 256];
   local_hist[bh * 256 + tid] = t;
 }
 }  // namespace
 
-int launch_hist_reduce(const uint32_t* chunk_hist, int64_t bs_h, int64_t n_chunks, int64_t chunk_keys, int mis, int H,
-                       int64_t N, const int32_t* n_dev, uint32_t* local_hist, cudaStream_t st) {
+int launch_hist_reduce(const uint32_t* chunk_hist, int64_t bs_h, int64_t n_chunks, uint32_t* local_hist, cudaStream_t st) {
   StageTimer tm(ST_HIST_REDUCE, st);
-  launch_chain(hist_reduce_kernel, dim3((unsigned)bs_h), dim3(256), 0, st, chunk_hist, n_chunks, chunk_keys, mis, H, N,
-               n_dev, local_hist);
+  launch_chain(hist_reduce_kernel, dim3((unsigned)bs_h), dim3(256), 0, st, chunk_hist, n_chunks, local_hist);
   return check_launch("shard histogram");
 }
 
@@ -639,8 +545,10 @@ extern "C" int pk_rank_clusters(const pk_tensor* q_blocks, const pk_tensor* sort
                  sorted_ids->shape[2] == 16 && sorted_ids->shape[3] == 256,
              "sorted_ids must be contiguous [bs,H,16,256]");
   if (bs * H == 0) return PK_OK;
-  return launch_rank(nullptr, nullptr, 0, (int)H, (uint16_t*)q_blocks->data, nullptr, nullptr, nullptr, nullptr, 0, bs * H,
-                     nullptr, (int64_t*)sorted_ids->data, (cudaStream_t)stream);
+  StageTimer tm(ST_RANK, (cudaStream_t)stream);
+  launch_chain(rank_kernel, dim3((unsigned)(bs * H * 16)), dim3(256), 0, (cudaStream_t)stream, (const uint16_t*)q_blocks->data,
+               (int64_t*)sorted_ids->data);
+  return check_launch("rank_clusters");
 }
 
 extern "C" int pk_collision_fused(const pk_tensor* sorted_cluster_ids, const pk_tensor* cluster_key_counts,

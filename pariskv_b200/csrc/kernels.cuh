@@ -38,10 +38,6 @@ __host__ __device__ inline long long zone_candidates(const pk_zone_schedule& s, 
 
 // collision.cu
 int64_t collision_chunk_keys(int64_t bs_h, int64_t Nv);
-// queries != null: query preparation is done inside (q_blocks / q_norm / query_avg become outputs)
-int launch_rank(const uint16_t* queries, const uint16_t* signs, int Hq, int H, uint16_t* q_blocks, uint16_t* q_norm,
-                uint16_t* query_avg, const int32_t* counts, const int64_t* tier_counts, int n_tiers, int64_t bs_h,
-                uint32_t* lut, int64_t* sorted_ids, cudaStream_t st);
 
 // The query side of the fused chain: the collision kernel prepares the query, ranks the clusters of every subspace
 // and builds the tier table itself, in every block, while its first code loads are in flight.
@@ -57,7 +53,6 @@ struct ChainQuery {
   int n_tiers;
   const int32_t* n_dev;       // [bs] searchable keys per sample (device), or null: all N keys of the view
   pk_zone_schedule sched;     // thresholds = zone_tiers(sched, n_dev[b]) when n_dev is set
-  long long n_plan;           // > 0: thresholds from this zone length instead (a shard of a longer zone)
   int early_query;            // the queries were complete before the previous kernel on the stream started
   int early_loads;            // see pdl_early()
 };
@@ -69,8 +64,7 @@ int launch_chain_collision(const pk_tensor* codebook, const ChainQuery& cq, uint
                            uint32_t* chunk_hist, int* mis_out, int64_t* chunk_keys_out, int64_t* n_hist_out,
                            cudaStream_t st);
 // local_hist[bh][bin] = sum over chunks of chunk_hist[bh][chunk][bin]
-int launch_hist_reduce(const uint32_t* chunk_hist, int64_t bs_h, int64_t n_chunks, int64_t chunk_keys, int mis, int H,
-                       int64_t N, const int32_t* n_dev, uint32_t* local_hist, cudaStream_t st);
+int launch_hist_reduce(const uint32_t* chunk_hist, int64_t bs_h, int64_t n_chunks, uint32_t* local_hist, cudaStream_t st);
 
 // topk.cu: exact top-k of rows of 32-bit values; out[row][i] = map ? map[row*map_stride + pos] : pos.  n_dev: valid elements
 // of every row, read on the device (null: L); n_out: [rows] min(k, valid elements), or null.

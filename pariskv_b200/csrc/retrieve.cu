@@ -191,7 +191,7 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
       PK_REQUIRE(is_contig(a.local_hist) && a.local_hist->shape[0] == bs && a.local_hist->shape[1] == H &&
                      a.local_hist->shape[2] == 256,
                  "local_hist must be contiguous i32 [bs,H,256]");
-      return launch_hist_reduce(hist, bh, n_chunks, chunk_keys, mis, (int)H, N, nullptr, (uint32_t*)a.local_hist->data, st);
+      return launch_hist_reduce(hist, bh, n_chunks, (uint32_t*)a.local_hist->data, st);
     }
   } else {
     int layout = 0;
