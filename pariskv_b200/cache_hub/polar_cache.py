@@ -415,7 +415,7 @@ class polar_cache(KV_Cache):
             return self._compute_per_query_head(queries, l)
         # A caller whose queries are made BEFORE it calls decode_update_kv_cache (one kernel makes q and k) says so with
         # queries_precede_append: the append launch of this layer then sits between that kernel and this call, and the
-        # collision kernel may prepare the query before it waits for the append (matters with dependent launch only).
+        # chain may prepare the query before it waits for the append (matters with early loads only, see pk_set_pdl).
         settled = self.queries_precede_append and self._appended_layer == l
         self._appended_layer = None
         final, n_sel = _lib.native().retrieve_ex(

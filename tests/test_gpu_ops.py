@@ -160,8 +160,8 @@ def test_topk_exact(ops, oracle, L, k, kind):
 @pytest.mark.parametrize("case", ["all_equal", "two_values", "dense_ties_float", "negatives", "tiny_spread", "signed_zero"])
 @pytest.mark.parametrize("L,k", [(1500, 1), (5000, 2048), (13101, 2048), (16384, 16000), (16384, 16384)])
 def test_topk_short_rows_tie_paths(ops, oracle, L, k, case):
-    """Rows of at most 16384 elements take the one-CTA kernel: exercise its radix levels (values that agree in the top
-    12 / 24 bits), the threshold bin above and below its ranking capacity, and equal keys at the last bit."""
+    """The selection's levels: values that agree in the top 12 / 24 bits, the threshold bin above and below its ranking
+    capacity, and equal keys at the last bit."""
     g = torch.Generator().manual_seed(L * 7 + k)
     rows = 2
     if case == "all_equal":
@@ -376,7 +376,7 @@ def test_sparse_attention(ops, oracle, store, n_window, K, group):
         rows_v.append(oracle.gather(vals, sel + off))
     ref = oracle.attention(q, torch.cat(rows_k, 2), torch.cat(rows_v, 2))
     err = (out.float().cpu() - ref).abs().max().item()
-    assert err <= 2e-2, err  # tolerance stated by the task: bf16 output, max abs 2e-2
+    assert err <= 2e-2, err  # bf16 output: max abs 2e-2
 
 
 def test_sparse_attention_per_head_counts(ops, oracle):
