@@ -21,6 +21,6 @@ def load_kernel_module(path="collision.cu", name="update_cache_cnt", **_):
 def update_cache_cnt_cuda_interface(sorted_cluster_ids, cluster_key_counts, codebook, tier_counts) -> torch.Tensor:
     """sorted_cluster_ids i64|i32 [bs,H,B,NC], cluster_key_counts i32 [bs,H,B,NC], codebook u8 [bs,H,B,N] (any
     strides), tier_counts list[int] -> cache_cnt i32 [bs,H,N]."""
-    if torch_ops.direct(codebook):
+    if torch_ops.direct(sorted_cluster_ids, cluster_key_counts, codebook):
         return ops.collision_fused(sorted_cluster_ids, cluster_key_counts, codebook, [int(t) for t in tier_counts])
     return torch.ops.pariskv.collision_fused(sorted_cluster_ids, cluster_key_counts, codebook, [int(t) for t in tier_counts])

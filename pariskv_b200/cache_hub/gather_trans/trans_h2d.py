@@ -12,7 +12,7 @@ def h2d_gather_kv(src_k_caches, src_v_caches, selected_indices, dst_k_caches, ds
     assert src_k_caches.is_cpu and src_v_caches.is_cpu and src_k_caches.is_pinned() and src_v_caches.is_pinned()
     assert dst_k_caches.is_cuda and dst_v_caches.is_cuda
     assert src_k_caches.dtype == src_v_caches.dtype == dst_k_caches.dtype == dst_v_caches.dtype == torch.bfloat16
-    if torch_ops.direct(selected_indices):
+    if torch_ops.direct(src_k_caches, src_v_caches, selected_indices, dst_k_caches, dst_v_caches):
         ops.h2d_gather_kv(src_k_caches, src_v_caches, selected_indices, dst_k_caches, dst_v_caches)
         return
     torch.ops.pariskv.gather_trans(src_k_caches, src_v_caches, selected_indices, dst_k_caches, dst_v_caches)

@@ -29,7 +29,7 @@ def partial_rerank_cuda(coarse_indices, key_4bit, key_block_weight, q_blocks, q_
     assert B == 16 and m == 8, "only B = 16, m = 8 is supported"
     bs, H, C = coarse_indices.shape
     if not want_v4b:
-        if torch_ops.direct(coarse_indices):
+        if torch_ops.direct(coarse_indices, key_4bit, key_block_weight, q_blocks, q_norm, mag_centers):
             return ops.rerank(coarse_indices, key_4bit, key_block_weight, q_blocks, q_norm, mag_centers)[0], None
         return torch.ops.pariskv.rerank(coarse_indices, key_4bit, key_block_weight, q_blocks, q_norm, mag_centers), None
     v4b = torch.empty(bs, H, B, C, m, dtype=torch.bfloat16, device=coarse_indices.device)

@@ -26,11 +26,15 @@ import torch
 from . import ops
 
 
-def direct(t) -> bool:
-    """Whether a mirror module may call `ops` itself instead of torch.ops.pariskv.*: a plain eager tensor, nothing
-    traced and no dispatch mode on.  The dispatcher and the Python kernel behind it cost about 10 us a call, more than
-    most of these operators take on the GPU."""
-    return type(t) is torch.Tensor and not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0
+def direct(*tensors) -> bool:
+    """Whether a mirror module may call `ops` itself instead of torch.ops.pariskv.*: plain eager tensors that need no
+    gradient, nothing compiled or traced, no function transform (vmap, functionalize, ...), dispatch or function mode
+    on.  The dispatcher and the Python kernel behind it cost about 10 us a call, more than most of these operators take
+    on the GPU; the questions asked here 1."""
+    C = torch._C
+    return (C._len_torch_dispatch_stack() == 0 and C._len_torch_function_stack() == 0 and
+            C._functorch.maybe_current_level() is None and not C._is_tracing() and not torch.compiler.is_compiling() and
+            all(type(t) is torch.Tensor and not t.requires_grad for t in tensors))
 
 
 _lib = torch.library.Library("pariskv", "DEF")

@@ -91,3 +91,22 @@ def test_attention_shared_scratch_serves_any_batch():
         s = torch.einsum("bhgd,bhnd->bhgn", q.view(bs, H, 2, 128).double(), k.double()) / 128 ** 0.5
         ref = torch.einsum("bhgn,bhnd->bhgd", torch.softmax(s, -1), v.double()).reshape(q.shape)
         assert (ops.sparse_attention(q, k, v, 150).double() - ref).abs().max().item() <= 2e-2, (bs, H)
+
+
+@pytest.mark.filterwarnings("ignore")
+def test_mirror_ops_under_transforms_and_tracing():
+    """The mirror modules call the library themselves on plain eager tensors only: function transforms, graph capture by
+    tracing and tensors that need gradients go through the dispatcher, which batches, records or refuses them."""
+    from pariskv_b200 import torch_ops
+    from pariskv_b200.cache_hub.topk import bucket_topk
+    x = torch.randint(0, 90, (3, 2, 500), dtype=torch.int32, device=DEV, generator=torch.Generator(DEV).manual_seed(1))
+    want = torch.stack([bucket_topk(r, 7) for r in x])
+
+    def f(r):
+        return bucket_topk(r, 7)
+    assert torch.equal(torch.vmap(f)(x), want)
+    assert torch.equal(torch.func.functionalize(f)(x[0]), want[0])
+    traced = torch.jit.trace(f, (x[0],), check_trace=False)
+    assert torch.equal(traced(x[1]), want[1])
+    assert torch_ops.direct(x) and not torch_ops.direct(x, torch.zeros(2, device=DEV, requires_grad=True))
+    assert not torch_ops.direct(torch.nn.Parameter(torch.zeros(2), requires_grad=False))
