@@ -8,8 +8,10 @@
 // The C ABI stays free of torch types; this module is one of its callers.
 #include <Python.h>
 
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -154,6 +156,28 @@ PyObject* oom_class() {
     PyErr_SetString(PyExc_RuntimeError, e.what());      \
     return nullptr;                                     \
   }
+
+// Whether the arguments are tensors that the dispatcher would take straight to the CUDA implementation: torch.Tensor or
+// Parameter, without gradient, conjugate or negative bit or a wrapper of a transform, and no transform, tracer, dispatch
+// or function mode active on this thread.
+PyObject* py_plain(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  using c10::DispatchKey;
+  static const c10::DispatchKeySet modes({DispatchKey::FuncTorchDynamicLayerFrontMode, DispatchKey::FuncTorchDynamicLayerBackMode,
+                                          DispatchKey::FuncTorchVmapMode, DispatchKey::VmapMode, DispatchKey::Functionalize,
+                                          DispatchKey::Tracer, DispatchKey::PreDispatch, DispatchKey::PythonDispatcher,
+                                          DispatchKey::Python, DispatchKey::PythonTLSSnapshot});
+  static const c10::DispatchKeySet wrappers({DispatchKey::Python, DispatchKey::PythonTLSSnapshot, DispatchKey::FuncTorchBatched,
+                                             DispatchKey::FuncTorchGradWrapper, DispatchKey::BatchedNestedTensor, DispatchKey::Batched,
+                                             DispatchKey::Functionalize, DispatchKey::Conjugate, DispatchKey::Negative,
+                                             DispatchKey::ZeroTensor});
+  if (c10::impl::tls_local_dispatch_key_set().included_.has_any(modes) || at::impl::torch_function_mode_enabled()) Py_RETURN_FALSE;
+  for (Py_ssize_t i = 0; i < n; i++) {
+    if (!THPVariable_CheckExact(a[i])) Py_RETURN_FALSE;
+    const at::Tensor& t = THPVariable_Unpack(a[i]);
+    if (t.requires_grad() || t.key_set().has_any(wrappers)) Py_RETURN_FALSE;
+  }
+  Py_RETURN_TRUE;
+}
 
 PyObject* py_append_encode(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!arity(n, 18, "append_encode")) return nullptr;
@@ -589,6 +613,7 @@ PyObject* py_retrieve_workspace_bytes(PyObject*, PyObject* const* a, Py_ssize_t 
 
 #define PK_METHOD(name, fn) {name, (PyCFunction)(void (*)(void))fn, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
+    PK_METHOD("plain", py_plain),
     PK_METHOD("append_encode", py_append_encode),
     PK_METHOD("sparse_attention", py_attention),
     PK_METHOD("retrieve_ex", py_retrieve),

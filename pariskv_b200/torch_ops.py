@@ -23,18 +23,15 @@ from typing import List, Tuple
 
 import torch
 
+from . import _lib as L
 from . import ops
 
 
 def direct(*tensors) -> bool:
-    """Whether a mirror module may call `ops` itself instead of torch.ops.pariskv.*: plain eager tensors that need no
-    gradient, nothing compiled or traced, no function transform (vmap, functionalize, ...), dispatch or function mode
-    on.  The dispatcher and the Python kernel behind it cost about 10 us a call, more than most of these operators take
-    on the GPU; the questions asked here 1."""
-    C = torch._C
-    return (C._len_torch_dispatch_stack() == 0 and C._len_torch_function_stack() == 0 and
-            C._functorch.maybe_current_level() is None and not C._is_tracing() and not torch.compiler.is_compiling() and
-            all(type(t) is torch.Tensor and not t.requires_grad for t in tensors))
+    """Whether a mirror module may call `ops` itself instead of torch.ops.pariskv.*: plain eager tensors, nothing compiled
+    or traced, no function transform or mode on (`plain` of the native binding).  The dispatcher and the Python kernel
+    behind it cost about 10 us a call, more than most of these operators take on the GPU."""
+    return not torch.compiler.is_compiling() and L.native().plain(*tensors)
 
 
 _lib = torch.library.Library("pariskv", "DEF")

@@ -109,4 +109,8 @@ def test_mirror_ops_under_transforms_and_tracing():
     traced = torch.jit.trace(f, (x[0],), check_trace=False)
     assert torch.equal(traced(x[1]), want[1])
     assert torch_ops.direct(x) and not torch_ops.direct(x, torch.zeros(2, device=DEV, requires_grad=True))
-    assert not torch_ops.direct(torch.nn.Parameter(torch.zeros(2), requires_grad=False))
+    assert not torch_ops.direct(x.as_subclass(type("Sub", (torch.Tensor,), {})))
+    neg = torch._neg_view(torch.randn(2, 500, device=DEV))
+    assert not torch_ops.direct(neg) and torch.equal(bucket_topk(neg, 7), bucket_topk(neg.clone(), 7))
+    with torch.device("cpu"):
+        assert not torch_ops.direct(x)
