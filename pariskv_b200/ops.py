@@ -239,6 +239,20 @@ def append_encode(k_row, v_row, signs, window_k, window_v, win_codes, win_weight
                              block_weight, packed_4bit, value_norm, cluster_counts, store_kv, state, int(sink), int(interval))
 
 
+_ATTENTION_HEADERS = 1 << 16   # bytes of the shared attention scratch that only ever hold headers
+
+
+def _shared_attention_scratch(device, heads, nbytes):
+    """The shared scratch for attention calls of any size.  The kernel's arrival counters lie in a header at the start of
+    its workspace, as long as `heads` (bs * Hq) asks for, and have to be zero between calls, while the partial records behind
+    them are left as they are.  So the header of every call ENDS at the same byte, and no call finds the records of another
+    in its counters; headers longer than that area have buffers of their own, one per length."""
+    header = (heads + 64) // 64 * 256
+    if header > _ATTENTION_HEADERS:
+        return workspace(device, nbytes, f"attention {header}")
+    return workspace(device, _ATTENTION_HEADERS + nbytes - header, "attention")[_ATTENTION_HEADERS - header:]
+
+
 def sparse_attention(queries, window_k, window_v, n_window, store_k=None, store_v=None, selected=None, n_sel=None,
                      index_offset=0, scale=None, out=None, n_window_dev=None, n_window_add=0, lse=None, scratch=None):
     """Decode attention over window rows [0, n_window) plus the selected rows of the K/V store (device or
@@ -249,9 +263,8 @@ def sparse_attention(queries, window_k, window_v, n_window, store_k=None, store_
         scale = 1.0 / math.sqrt(D)
     N = L.native()
     rows = n_window + (selected.shape[2] if selected is not None else 0)
-    # the arrival counters lie in a header whose size follows from bs * Hq: calls with headers of another size would find the
-    # partial records of this one in their counters, so each size has its shared buffer
-    ws = _scratch(queries.device, N.attention_workspace_bytes(bs, Hq, rows), f"attention {(bs * Hq + 64) // 64}", scratch)
+    nbytes = N.attention_workspace_bytes(bs, Hq, rows)
+    ws = scratch.take(nbytes, "attention") if scratch is not None else _shared_attention_scratch(queries.device, bs * Hq, nbytes)
     return N.sparse_attention(queries, window_k, window_v, int(n_window), n_window_dev, int(n_window_add), store_k, store_v,
                               selected, n_sel, int(index_offset), float(scale), out, lse, ws)
 

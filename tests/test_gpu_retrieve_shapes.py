@@ -85,7 +85,8 @@ def test_attention_shared_scratch_serves_any_batch():
     partial records of the first may have been."""
     from pariskv_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(3)
-    for bs, H in ((1, 1), (10, 8), (1, 4), (3, 30), (40, 8), (1, 1)):
+    assert ops.attention_scratch_bytes(7, 9, 64) - (7 * 9 + 64) // 64 * 256 == 7 * 9 * 132 * 4   # the header's length
+    for bs, H in ((1, 1), (10, 8), (1, 4), (3, 30), (40, 8), (1, 1), (1100, 8), (2, 3), (1024, 8), (1100, 8), (1, 1)):
         k, v = (torch.randn(bs, H, 150, 128, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
         q = torch.randn(bs, 1, 2 * H, 128, generator=g, device=DEV).to(torch.bfloat16)
         s = torch.einsum("bhgd,bhnd->bhgn", q.view(bs, H, 2, 128).double(), k.double()) / 128 ** 0.5
