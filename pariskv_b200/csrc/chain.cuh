@@ -131,8 +131,8 @@ __device__ __forceinline__ float rerank_one(const RerankSmem& sm, const RerankAr
   uint32_t code[16];
   uint32_t wt[8];
   if (FAST) {
-    const uint4* cp = reinterpret_cast<const uint4*>(k4 + key * 64);
-    const uint4* wp = reinterpret_cast<const uint4*>(w + key * 16);
+    const uint4* cp = reinterpret_cast<const uint4*>(k4 + key * a.k4_l);
+    const uint4* wp = reinterpret_cast<const uint4*>(w + key * a.w_l);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       const uint4 v = cp[i];
@@ -178,13 +178,14 @@ __device__ __forceinline__ float rerank_one(const RerankSmem& sm, const RerankAr
   return __fmul_rn(acc, qn);
 }
 
-// The rerank of one candidate from key-major records, for kernels that rank many candidates per block.
+// The rerank of one candidate from its key-major record, for kernels that rank many candidates per block.
 // Levels are looked up two at a time: entry v of lev2 holds the bf16 levels of the nibbles v & 15 and v >> 4, one copy
-// per lane (word v * 32 + lane: never a bank conflict), so a record costs 64 look-ups instead of 128.  Two subspaces
-// run side by side in packed fp32 multiply-adds; every subspace keeps its own chain over j, then
-// acc = fma(dot, w_b, acc) over b ascending, so the result has the bits of rerank_one.
-// Three instructions per dimension; c128 = 128 and c64k = 65536 come from kernel arguments, because multiplications by
-// known powers of two become shifts on the integer ALU (half rate), which is what bounds the loop.
+// per lane (word v * 32 + lane: never a bank conflict), so a record costs 64 look-ups instead of 128.  Levels and query are
+// bf16 and go into the fp32 multiply-adds as they are (fma.rn.f32.bf16: the exact product, one rounding), every subspace with
+// its own chain over j, then acc = fma(dot, w_b, acc) over b ascending, so the result has the bits of rerank_one.
+// c128 = 128 comes from a kernel argument, because a multiplication by a known power of two becomes a shift on the integer ALU
+// (half rate).  What bounds it: shared-memory wavefronts, 64 for the look-ups, 32 for the query, 24 for the record, some 30
+// for the fetch of the next.
 // Four lanes per candidate (whole sectors per load, the query in registers) measured 15 % slower: passing the sum from
 // lane to lane costs more instructions than the query's shared-memory reads.
 constexpr int LEV2_BYTES = 256 * 32 * 4;
@@ -195,44 +196,29 @@ __device__ __forceinline__ void build_lev2(uint32_t* lev2, const uint16_t* cente
     lev2[v * 32 + (tid & 31)] = ((v & 8) ? a : a ^ 0x8000u) | (((v & 0x80) ? b : b ^ 0x8000u) << 16);
   }
 }
-// where dimension d of the query goes in the array rerank_pairs reads: for the subspaces 2p, 2p + 1 and the dimensions
-// 2i, 2i + 1 of a subspace, float4 p * 4 + i = (q[2p][2i], q[2p + 1][2i], q[2p][2i + 1], q[2p + 1][2i + 1])
-__device__ __forceinline__ int pair_slot(int d) {
-  const int sub = d >> 3, j = d & 7;
-  return ((sub >> 1) * 4 + (j >> 1)) * 4 + (j & 1) * 2 + (sub & 1);
+// acc + a.lo * b.lo, then + a.hi * b.hi: bf16 factors, fp32 sums
+__device__ __forceinline__ float fma_bf16x2(uint32_t a, uint32_t b, float acc) {
+  asm("{\n\t.reg .b16 al, ah, bl, bh;\n\tmov.b32 {al, ah}, %1;\n\tmov.b32 {bl, bh}, %2;\n\t"
+      "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %0, ah, bh, %0;\n\t}"
+      : "+f"(acc)
+      : "r"(a), "r"(b));
+  return acc;
 }
-__device__ __forceinline__ unsigned long long pack2(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ float rerank_pairs(const uint4 (&rec)[6], const uint32_t* lev2, const float4* q2, float qn, int lane,
-                                              unsigned c128, unsigned c64k) {
+__device__ __forceinline__ float rerank_record(const uint4 (&rec)[6], const uint32_t* lev2, const uint4* q, float qn, int lane, unsigned c128) {
   const uint32_t code[16] = {rec[0].x, rec[0].y, rec[0].z, rec[0].w, rec[1].x, rec[1].y, rec[1].z, rec[1].w,
                              rec[2].x, rec[2].y, rec[2].z, rec[2].w, rec[3].x, rec[3].y, rec[3].z, rec[3].w};
   const uint32_t wt[8] = {rec[4].x, rec[4].y, rec[4].z, rec[4].w, rec[5].x, rec[5].y, rec[5].z, rec[5].w};
   const uint8_t* base = reinterpret_cast<const uint8_t*>(lev2) + lane * 4;
   float acc = 0.0f;
 #pragma unroll
-  for (int p = 0; p < 8; p++) {
-    unsigned long long dot = 0ull;
+  for (int s = 0; s < 16; s++) {
+    const uint4 qs = q[s];   // the eight dimensions of the subspace
+    const uint32_t qw[4] = {qs.x, qs.y, qs.z, qs.w};
+    float dot = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float4 q = q2[p * 4 + i];
-      const uint32_t a = *reinterpret_cast<const uint32_t*>(base + byte_of(code[2 * p], i) * c128);
-      const uint32_t b = *reinterpret_cast<const uint32_t*>(base + byte_of(code[2 * p + 1], i) * c128);
-      dot = fma2(pack2(__uint_as_float(a * c64k), __uint_as_float(b * c64k)), pack2(q.x, q.y), dot);
-      dot = fma2(pack2(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)), pack2(q.z, q.w), dot);
-    }
-    float d0, d1;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(d0), "=f"(d1) : "l"(dot));
-    acc = __fmaf_rn(d0, __uint_as_float(wt[p] << 16), acc);
-    acc = __fmaf_rn(d1, __uint_as_float(wt[p] & 0xffff0000u), acc);
+    for (int i = 0; i < 4; i++)
+      dot = fma_bf16x2(*reinterpret_cast<const uint32_t*>(base + byte_of(code[s], i) * c128), qw[i], dot);
+    acc = __fmaf_rn(dot, __uint_as_float((s & 1) ? (wt[s >> 1] & 0xffff0000u) : (wt[s >> 1] << 16)), acc);
   }
   return __fmul_rn(acc, qn);
 }
@@ -242,8 +228,10 @@ constexpr int CH_THREADS = 512;
 constexpr int CH_WARPS = CH_THREADS / 32;
 constexpr int CH_CBINS = 129;                      // counts 0 .. 16 subspaces x 8 tiers
 constexpr int CH_HIST_BYTES = CH_CBINS * 32 * 4;   // count histogram, one replica per lane: a warp's atomics never conflict
-constexpr int CH_REC = 112;                        // bytes between staged records (96 used): quarter-warp reads do not conflict
-constexpr int CH_STAGE = CH_WARPS * 32 * CH_REC;
+// A warp's 32 staged records: 96 bytes each, 16 more after every fourth.  Record r starts at unit 6 r + r / 4 of 16 bytes, so
+// the eight lanes of a quarter-warp read fall into eight different groups of four banks.
+constexpr int CH_STAGE_WARP = 16 * (6 * 32 + 8);
+constexpr int CH_STAGE = CH_WARPS * CH_STAGE_WARP;
 
 struct PreparedQuery {
   float x[4], avg[4], n;   // warp 0: the lane's dimensions of the rotated and of the mean query, the norm
@@ -420,38 +408,53 @@ __device__ __forceinline__ int list_candidates(uint8_t* cnt8, int n_keys, int sk
   return n_list;
 }
 
-// 4-bit rerank of a list by one block, from key-major records: key_at(i) -> sink(i, key, score).
-// A warp takes 32 consecutive candidates per round: it loads their records with whole sectors per request (four lanes
-// on the 64 bytes of codes, two on the 32 bytes of weights), turns them over its staging buffer (32 * CH_REC bytes) to one
-// record per lane, and has the loads of the next round in flight during the arithmetic.
+// 4-bit rerank of a list by one block, from key-major records: key_at(i) -> sink(i, key, score).  ids: the keys of the first
+// n_ids candidates in shared memory (all of them, or a multiple of 32); q: the rotated query, 128 bf16 in shared memory.
+// A warp takes 32 consecutive candidates per round.  The records of its next round are on their way to its staging buffer by
+// cp.async while it works on this one, which it has read into registers, one record per lane: 24 lanes fetch four records per
+// instruction, six 16-byte pieces each.
+// What bounds it: the wavefronts of rerank_record, 162 a round and SM, and HBM in units of 128 bytes (the records of a
+// candidate in two arrays are two).  128 blocks with 6000 candidates each on B200: 54 us with the records through registers
+// and packed fp32 products (264 wavefronts, 593 instructions a round), 33 like this (493 instructions).  16 sequences of
+// 16 - 32K keys 232.6 -> 219.5 us a step of two layers, adaptive budgets of 8 sequences 155.1 -> 147.1, 1M keys 135.0 -> 132.1.
+// A second buffer per warp, two candidates per lane and the TMA's four-row gather were no faster.
 template <class KeyAt, class Sink>
-__device__ __forceinline__ void rerank_list(int n_list, const uint8_t* k4, const uint16_t* w, uint8_t* stage, const uint32_t* lev2,
-                                            const float4* q2, float qn, unsigned c128, unsigned c64k, KeyAt key_at, Sink sink) {
+__device__ __forceinline__ void rerank_list(int n_list, const int* ids, int n_ids, const RerankArgs& a, const uint8_t* k4, const uint16_t* w,
+                                            uint8_t* stage, const uint32_t* lev2, const uint4* q, float qn, unsigned c128, KeyAt key_at,
+                                            Sink sink) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int ROUND = CH_WARPS * 32;
-  uint4 in[6];
-  auto fetch = [&](int base) {   // out of range: the list's last candidate again
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-      in[i] = reinterpret_cast<const uint4*>(k4 + (int64_t)key_at(min(base + 8 * i + (lane >> 2), n_list - 1)) * 64)[lane & 3];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-      in[4 + i] = reinterpret_cast<const uint4*>(w + (int64_t)key_at(min(base + 16 * i + (lane >> 1), n_list - 1)) * 16)[lane & 1];
+  const int sub = (lane * 43) >> 8, piece = lane - 6 * sub;   // lane / 6 and the rest
+  const uint8_t* src = piece < 4 ? k4 + 16 * piece : reinterpret_cast<const uint8_t*>(w) + 16 * (piece - 4);
+  const unsigned step = (unsigned)(piece < 4 ? a.k4_l : 2 * a.w_l);   // bytes from key to key
+  const unsigned dst = (unsigned)__cvta_generic_to_shared(stage) + 16 * lane;
+  const int n_whole = min(n_list, n_ids);
+  auto copy = [&](int i, int key) {   // records 4 i .. 4 i + 3 of the round
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 400 * i), "l"(src + (uint64_t)(unsigned)key * step) : "memory");
   };
-  if (warp * 32 < n_list) fetch(warp * 32);
+  auto fetch = [&](int base) {
+    if (base < n_list && lane < 24) {
+      if (base + 32 <= n_whole) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) copy(i, ids[base + 4 * i + sub]);
+      } else {   // past the end: the list's last candidate again
+#pragma unroll 1
+        for (int i = 0; i < 8; i++) copy(i, key_at(min(base + 4 * i + sub, n_list - 1)));
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(warp * 32);
 #pragma unroll 1
   for (int base = warp * 32; base < n_list; base += ROUND) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 4; i++) *reinterpret_cast<uint4*>(stage + (8 * i + (lane >> 2)) * CH_REC + (lane & 3) * 16) = in[i];
-#pragma unroll
-    for (int i = 0; i < 2; i++) *reinterpret_cast<uint4*>(stage + (16 * i + (lane >> 1)) * CH_REC + 64 + (lane & 1) * 16) = in[4 + i];
-    __syncwarp();
-    if (base + ROUND < n_list) fetch(base + ROUND);
     uint4 rec[6];
 #pragma unroll
-    for (int i = 0; i < 6; i++) rec[i] = *reinterpret_cast<const uint4*>(stage + lane * CH_REC + i * 16);
-    const float v = rerank_pairs(rec, lev2, q2, qn, lane, c128, c64k);
+    for (int i = 0; i < 6; i++) rec[i] = *reinterpret_cast<const uint4*>(stage + (6 * lane + (lane >> 2) + i) * 16);
+    __syncwarp();
+    fetch(base + ROUND);
+    const float v = rerank_record(rec, lev2, q, qn, lane, c128);
     const int i = base + lane;
     if (i < n_list) sink(i, key_at(i), v);
   }

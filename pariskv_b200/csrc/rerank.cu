@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(RR_THREADS) rerank_kernel(RerankArgs a, uint16
 struct SelParams {
   SelectArgs s;
   int list_cap;            // candidates whose keys fit in shared memory; the others are read back from cand_out
-  unsigned c128, c64k;     // 128 and 65536 (see rerank_pairs)
+  unsigned c128;           // 128 (see rerank_record)
 };
 
 template <bool FAST>
@@ -60,12 +60,12 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
   const SelectArgs& p = pp.s;
   uint32_t* lev2 = reinterpret_cast<uint32_t*>(dyn);                  // FAST: pair levels; otherwise RerankSmem
   uint8_t* cnt8 = dyn + LEV2_BYTES;
-  uint8_t* stage = cnt8 + (threadIdx.x >> 5) * (32 * CH_REC);          // the counts are done with when records are staged
+  uint8_t* stage = cnt8 + (threadIdx.x >> 5) * CH_STAGE_WARP;        // the counts are done with when records are staged
   int* ids = reinterpret_cast<int*>(cnt8 + max((int)p.chunk_keys, CH_STAGE));
   __shared__ unsigned tot[2][CH_CBINS + 3], pre[2][CH_CBINS + 3];
   __shared__ unsigned s_warp[CH_WARPS], s_pwarp[CH_WARPS];
   __shared__ unsigned s_res[6];   // threshold, quota, keys above it before this block, ties before it, candidates of this shard
-  __shared__ __align__(16) float4 s_q2[32];
+  __shared__ __align__(16) uint4 s_qb[16];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t bh = blockIdx.y, chunk = blockIdx.x;
   const int b = (int)(bh / a.H), h = (int)(bh % a.H);
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
   if (!FAST) {
     rerank_setup(*reinterpret_cast<RerankSmem*>(dyn), a, bh, tid, CH_THREADS);
   } else if (tid < 128) {
-    reinterpret_cast<float*>(s_q2)[pair_slot(tid)] = bf2f(a.q_blocks[bh * 128 + tid]);
+    reinterpret_cast<uint16_t*>(s_qb)[tid] = a.q_blocks[bh * 128 + tid];
   }
   // Bin totals over the rows: the block's two halves take alternate rows, eight loads in flight per thread.  Bins 0 .. 128
   // are the only ones: the halves' threads 0 .. 128.
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
   const uint16_t* w = a.w + b * a.w_b + h * a.w_h;
   float* scores = p.scores_f32 + row_base + out_pos;
   if (FAST) {
-    rerank_list(n_list, k4, w, stage, lev2, s_q2, qn, pp.c128, pp.c64k, key_at, [&](int i, int, float v) { scores[i] = v; });
+    rerank_list(n_list, ids, pp.list_cap, a, k4, w, stage, lev2, s_qb, qn, pp.c128, key_at, [&](int i, int, float v) { scores[i] = v; });
   } else {
     for (int i = tid; i < n_list; i += CH_THREADS)
       scores[i] = rerank_one<false>(*reinterpret_cast<RerankSmem*>(dyn), a, k4, w, key_at(i), qn, lane, nullptr, 0);
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
 }  // namespace
 
 bool rerank_fast_layout(const RerankArgs& a) {
-  return a.k4_s == 4 && a.k4_l == 64 && a.w_s == 1 && a.w_l == 16 && (reinterpret_cast<uintptr_t>(a.k4) & 15) == 0 &&
+  return a.k4_s == 4 && a.k4_l >= 0 && a.k4_l < (1 << 30) && a.k4_l % 16 == 0 && a.w_s == 1 && a.w_l >= 0 && a.w_l < (1 << 30) && a.w_l % 8 == 0 && (reinterpret_cast<uintptr_t>(a.k4) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(a.w) & 15) == 0 && a.k4_b % 16 == 0 && a.k4_h % 16 == 0 && a.w_b % 8 == 0 &&
          a.w_h % 8 == 0;
 }
@@ -226,10 +226,10 @@ int launch_rerank(const RerankArgs& a, int64_t bs_h, uint16_t* scores_bf16, floa
 int launch_select_rerank(const RerankArgs& a, int64_t bs_h, const SelectArgs& sa, cudaStream_t st) {
   SelParams p;
   p.s = sa;
-  p.c128 = 128, p.c64k = 65536;
+  p.c128 = 128;
   if (sa.C >= (1ll << 31) || sa.N >= (1ll << 31)) return fail(PK_ERR_ARG, "zone too long for the selection kernel");
   const int64_t body = sa.chunk_keys > CH_STAGE ? sa.chunk_keys : CH_STAGE;
-  int64_t list = (sa.C < sa.chunk_keys ? sa.C : sa.chunk_keys) + 32;
+  int64_t list = ((sa.C < sa.chunk_keys ? sa.C : sa.chunk_keys) + 31) / 32 * 32;
   if (list > SEL_LIST_MAX) list = SEL_LIST_MAX;
   p.list_cap = (int)list;
   const int smem = (int)(LEV2_BYTES + body + 4 * list);

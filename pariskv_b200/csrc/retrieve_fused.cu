@@ -44,7 +44,7 @@ struct FusedParams {
   int span_cap, list_cap; // shared memory: keys and candidates per CTA
   int64_t* cand_out;      // [bs*H][C] or null
   float* scores_out;      // [bs*H][C] or null
-  unsigned c128, c256, c64k;   // 128, 256 and 65536 (see tier_sum16, rerank_pairs)
+  unsigned c128, c256;    // 128 and 256 (see tier_sum16, rerank_record)
   int64_t* ws_cand;       // the same arrays for what does not fit in shared memory (never null)
   float* ws_scores;
   int64_t* final_out;     // [bs*H][K]
@@ -60,12 +60,12 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   __shared__ unsigned s_tiers[9];
   __shared__ float s_qnorm;
   __shared__ __align__(16) float s_q[128];        // rotated query
-  __shared__ __align__(16) float4 s_q2[32];       // the same, the subspaces of a pair side by side (see rerank_pairs)
+  __shared__ __align__(16) uint4 s_qb[16];        // the same, its bf16 values as such
   __shared__ __align__(16) uint8_t s_lut[16 * 128];
   unsigned* region = reinterpret_cast<unsigned*>(dyn);
   uint32_t* lev2 = reinterpret_cast<uint32_t*>(dyn + CH_HIST_BYTES);
   uint8_t* cnt8 = dyn + CH_HIST_BYTES + LEV2_BYTES;
-  uint8_t* stage = cnt8 + (threadIdx.x >> 5) * (32 * CH_REC);   // the counts are done with when records are staged
+  uint8_t* stage = cnt8 + (threadIdx.x >> 5) * CH_STAGE_WARP;   // the counts are done with when records are staged
   int* ids = reinterpret_cast<int*>(cnt8 + max(p.span_cap, CH_STAGE));
   float* sc = reinterpret_cast<float*>(ids + p.list_cap);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
     __syncthreads();
     if (!early) rank_subspace(key, s_q + warp * 8, lane);
     tier_table(key, my, s_tiers, s_lut + warp * 128);
-    if (tid < 128) reinterpret_cast<float*>(s_q2)[pair_slot(tid)] = s_q[tid];
+    if (tid < 128) reinterpret_cast<uint16_t*>(s_qb)[tid] = f2bf(s_q[tid]);
     __syncthreads();   // the tables are complete, the sizes are done with
   }
   const float qn = s_qnorm;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   {
     const uint8_t* k4 = p.a.k4 + b * p.a.k4_b + h * p.a.k4_h;
     const uint16_t* w = p.a.w + b * p.a.w_b + h * p.a.w_h;
-    rerank_list(n_list, k4, w, stage, lev2, s_q2, qn, p.c128, p.c64k, id_at, [&](int i, int k, float v) {
+    rerank_list(n_list, ids, p.list_cap, p.a, k4, w, stage, lev2, s_qb, qn, p.c128, id_at, [&](int i, int k, float v) {
       const int64_t at = row_base + out_pos + i;
       if (i < p.list_cap) sc[i] = v;
       else p.ws_scores[at] = v;
@@ -296,7 +296,7 @@ int launch_fused_retrieve(int cs, const pk_tensor* codebook, const RerankArgs& a
   p.codes = (const uint8_t*)codebook->data, p.c_b = codebook->stride[0], p.c_h = codebook->stride[1];
   p.a = a, p.q = cq, p.H = (int)H, p.G = cq.Hq / (int)H, p.inv_g = 1.0f / (float)p.G;
   p.N = sa.N, p.C = sa.C, p.C_want = sa.C_want, p.K = sa.K, p.fill_tail = sa.fill_tail;
-  p.c128 = 128, p.c256 = 256, p.c64k = 65536;
+  p.c128 = 128, p.c256 = 256;
   p.cand_out = cand_out, p.scores_out = scores_out, p.ws_cand = ws_cand, p.ws_scores = ws_scores;
   p.final_out = sa.final_out, p.n_sel_out = sa.n_sel_out, p.n_cand_out = sa.n_cand_out;
   p.span_cap = span_of(sa.N, cs);

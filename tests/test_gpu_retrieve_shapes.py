@@ -43,6 +43,45 @@ def test_retrieve_matches_oracle(oracle, bs, H, N, C, K, kind):
     assert torch.equal(ex2["cand"].cpu(), ref["cand"]) and torch.equal(ex2["scores_f32"].cpu(), ref["score32"])
 
 
+def _records(bs, H, N, size, first=0):
+    """Views of the 4-bit codes and the weights in records of `size` bytes, the first `first` records not used."""
+    rec = torch.zeros(bs, H, N + first, size, dtype=torch.uint8, device=DEV)[:, :, first:]
+    return rec.view(torch.bfloat16)[..., 32:48].permute(0, 1, 3, 2), rec[..., :64].unflatten(-1, (16, 4)).permute(0, 1, 3, 2, 4)
+
+
+# lists of less than, exactly and one more than the 32 candidates of a warp's round; odd rounds; one block and clusters; the
+# form in several launches
+@pytest.mark.parametrize("layout", ["arrays", "96", "112", "128", "128 from the fourth", "planes"])
+@pytest.mark.parametrize("bs,H,N,C", [(1, 1, 31, 31), (1, 1, 40, 32), (1, 2, 33, 33), (1, 2, 3001, 1029), (20, 8, 700, 130), (1, 1, 700001, 3001)])
+def test_rerank_of_any_record_layout(oracle, bs, H, N, C, layout):
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(N + C)
+    keys = synth_keys(g, bs, H, N)
+    q = synth_queries(g, keys, 4)
+    signs = srht_signs()
+    _, cen = oracle.constants()
+    counts = torch.zeros(bs, H, 16, 256, dtype=torch.int32, device=DEV)
+    cb = torch.zeros(bs, H, N, 16, dtype=torch.uint8, device=DEV).permute(0, 1, 3, 2)
+    if layout == "planes":
+        cb = cb.contiguous()
+        w, pk = torch.zeros(bs, H, 16, N, dtype=torch.bfloat16, device=DEV), torch.zeros(bs, H, 16, N, 4, dtype=torch.uint8, device=DEV)
+    elif layout == "arrays":
+        w = torch.zeros(bs, H, N, 16, dtype=torch.bfloat16, device=DEV).permute(0, 1, 3, 2)
+        pk = torch.zeros(bs, H, N, 16, 4, dtype=torch.uint8, device=DEV).permute(0, 1, 3, 2, 4)
+    else:
+        w, pk = _records(bs, H, N, int(layout.split()[0]), 4 if "from" in layout else 0)
+    ops.encode_keys(keys.to(DEV), signs.to(DEV), cb, w, pk, cluster_counts=counts)
+    cb_o, w_o, pk_o = oracle.encode(keys, signs)
+    assert torch.equal(cb.cpu(), cb_o) and torch.equal(w.cpu().float(), w_o.float()) and torch.equal(pk.cpu(), pk_o)
+    K = (C + 1) // 2
+    ref = oracle.retrieve(q, signs, cb_o, w_o, pk_o, oracle.cluster_counts(cb_o), cen, 0.25, C, K)
+    fin, ex = ops.retrieve(q.to(DEV), signs.to(DEV), cen.to(DEV), cb, w, pk, counts, oracle.tier_counts(N, 0.25), C, K,
+                           want=("cand", "scores_f32"))
+    assert torch.equal(ex["cand"].cpu(), ref["cand"])
+    assert torch.equal(ex["scores_f32"].cpu(), ref["score32"])
+    assert torch.equal(fin.cpu(), ref["final"])
+
+
 @pytest.mark.parametrize("group", [5, 8, 9])
 @pytest.mark.parametrize("n_window,K", [(1, 0), (63, 1), (64, 64), (70, 1000)])
 def test_attention_group_sizes(oracle, group, n_window, K):
