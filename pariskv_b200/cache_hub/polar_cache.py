@@ -8,7 +8,7 @@ model runtime written for the reference decodes through it unchanged.  The body 
   holds every older token: pinned host memory read through UVA when ``enable_offload`` is set, device
   memory otherwise.  Both modes run the same kernels.
 * Zone metadata (sign codes, 4-bit codes, rerank weights) is stored key-major and indexed by the
-  zone-relative position, so record 0 is 16-byte aligned and a rerank candidate is two contiguous records.
+  zone-relative position, so record 0 is 16-byte aligned and a rerank candidate is one 128-byte record.
   ``codebook_gpu / key_block_weight_gpu / key_4bit_packed_gpu`` expose them in the reference's logical
   shapes through permuted views.
 * One decode step of one layer is three launches: ``ops.append_encode`` (row append, key coding, flush),

@@ -32,8 +32,8 @@ __device__ __forceinline__ void load_key32(uint4 (&raw)[4], const uint16_t* row,
   for (int i = 0; i < 4; i++) raw[i] = reinterpret_cast<const uint4*>(row + 32 * s)[i];
 }
 
-// KEY_MAJOR: records stored key by key ([..,L,16(,4)] contiguous over subspaces), so a lane's share of a record is one
-// store; otherwise any strides.
+// KEY_MAJOR: records stored key by key (contiguous over subspaces), so a lane's share of a record is one store; otherwise
+// any strides.
 template <bool KEY_MAJOR>
 __global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
   __shared__ int hist[16 * 256];
@@ -59,8 +59,8 @@ __global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
     if (key >= end) continue;
     if (KEY_MAJOR) {
       *reinterpret_cast<uint32_t*>(p.codes + b * p.c_b + h * p.c_h + key * 16 + 4 * s) = kc.codes;
-      *reinterpret_cast<uint2*>(p.w + b * p.w_b + h * p.w_h + key * 16 + 4 * s) = kc.weights;
-      *reinterpret_cast<uint4*>(p.pk + b * p.p_b + h * p.p_h + key * 64 + 16 * s) = kc.packed;
+      *reinterpret_cast<uint2*>(p.w + b * p.w_b + h * p.w_h + key * p.w_l + 4 * s) = kc.weights;
+      *reinterpret_cast<uint4*>(p.pk + b * p.p_b + h * p.p_h + key * p.p_l + 16 * s) = kc.packed;
     } else {
       const uint32_t pk4[4] = {kc.packed.x, kc.packed.y, kc.packed.z, kc.packed.w};
 #pragma unroll
@@ -113,10 +113,11 @@ struct PrefillParams {
   uint16_t* win_w;
   uint8_t* win_pk;
   float* win_vnorm;
-  uint8_t* z_codes;         // zone records of the sample: [H][cap_z][16], [H][cap_z][16], [H][cap_z][64], [H][cap_z] or null
+  uint8_t* z_codes;         // zone records of the sample: [H][cap_z][16], [H][cap_z][16 of z_wl], [H][cap_z][64 of z_pl], [H][cap_z] or null
   uint16_t* z_w;
   uint8_t* z_pk;
   float* z_vnorm;
+  int64_t z_wl, z_pl;       // weights (elements) and 4-bit codes (bytes) from one key to the next
   int32_t* counts;          // [H][16][256], zero at launch
   uint16_t* store;          // [H][store_cap][2][128]
   int32_t* state;           // the layer's words, or null (see pk_prefill_sample)
@@ -182,8 +183,8 @@ __global__ void __launch_bounds__(EN_THREADS, 2) prefill_kernel(PrefillParams p)
         for (int i = 0; i < 4; i++) st[i] = kr[i];
         const int64_t rec = (int64_t)h * p.cap_z + z;
         *reinterpret_cast<uint32_t*>(p.z_codes + rec * 16 + 4 * s) = kc.codes;
-        *reinterpret_cast<uint2*>(p.z_w + rec * 16 + 4 * s) = kc.weights;
-        *reinterpret_cast<uint4*>(p.z_pk + rec * 64 + 16 * s) = kc.packed;
+        *reinterpret_cast<uint2*>(p.z_w + rec * p.z_wl + 4 * s) = kc.weights;
+        *reinterpret_cast<uint4*>(p.z_pk + rec * p.z_pl + 16 * s) = kc.packed;
 #pragma unroll
         for (int i = 0; i < 4; i++) atomicAdd(&hist[(4 * s + i) * 256 + ((kc.codes >> (8 * i)) & 0xffu)], 1);
       } else {
@@ -286,8 +287,9 @@ struct AppendParams {
   uint8_t* win_pk;                  // [bs*H][cap_w][64]
   float* win_vnorm;                 // [bs*H][cap_w]
   uint8_t* z_codes;                 // [bs*H][cap_z][16]   key-major zone records
-  uint16_t* z_w;                    // [bs*H][cap_z][16]
-  uint8_t* z_pk;                    // [bs*H][cap_z][64]
+  uint16_t* z_w;                    // [bs*H][cap_z][16 of z_wl]
+  uint8_t* z_pk;                    // [bs*H][cap_z][64 of z_pl]
+  int64_t z_wl, z_pl;               // weights (elements) and 4-bit codes (bytes) from one key to the next
   float* z_vnorm;                   // [bs*H][cap_z] or null
   int32_t* counts;                  // [bs*H][16][256]
   uint16_t* store;                  // [bs*H][cap_s][2][128]
@@ -353,11 +355,11 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
     const uint4* sp = reinterpret_cast<const uint4*>(wp + (int64_t)sink * 64);
     const uint4* sw = reinterpret_cast<const uint4*>(ww + (int64_t)sink * 16);
     uint4* zc = reinterpret_cast<uint4*>(p.z_codes + (bh * p.cap_z + N) * 16);
-    uint4* zp = reinterpret_cast<uint4*>(p.z_pk + (bh * p.cap_z + N) * 64);
-    uint4* zw = reinterpret_cast<uint4*>(p.z_w + (bh * p.cap_z + N) * 16);
+    uint8_t* zp = p.z_pk + (bh * p.cap_z + N) * p.z_pl;
+    uint16_t* zw = p.z_w + (bh * p.cap_z + N) * p.z_wl;
     for (int i = tid; i < I; i += 256) zc[i] = sc[i];
-    for (int i = tid; i < 4 * I; i += 256) zp[i] = sp[i];
-    for (int i = tid; i < 2 * I; i += 256) zw[i] = sw[i];
+    for (int i = tid; i < 4 * I; i += 256) reinterpret_cast<uint4*>(zp + (i >> 2) * p.z_pl)[i & 3] = sp[i];
+    for (int i = tid; i < 2 * I; i += 256) reinterpret_cast<uint4*>(zw + (i >> 1) * p.z_wl)[i & 1] = sw[i];
     if (p.z_vnorm)
       for (int i = tid; i < I; i += 256) p.z_vnorm[bh * p.cap_z + N + i] = wn[sink + i];
     uint4* st = reinterpret_cast<uint4*>(p.store + (bh * p.cap_s + N) * 256);
@@ -486,9 +488,9 @@ extern "C" int pk_encode_keys(const pk_tensor* keys, const pk_tensor* signs, con
   p.H = (int)H;
   p.L = L;
   p.chunk = encode_chunk(L, bs * H);
-  const bool key_major = p.c_s == 1 && p.c_l == 16 && p.w_s == 1 && p.w_l == 16 && p.p_s == 4 && p.p_l == 64 &&
-                         (reinterpret_cast<uintptr_t>(p.codes) & 3) == 0 && (reinterpret_cast<uintptr_t>(p.w) & 7) == 0 &&
-                         (reinterpret_cast<uintptr_t>(p.pk) & 15) == 0 && ((p.c_b | p.c_h | p.w_b | p.w_h) & 3) == 0 && ((p.p_b | p.p_h) & 15) == 0;
+  const bool key_major = p.c_s == 1 && p.c_l == 16 && p.w_s == 1 && p.p_s == 4 && (reinterpret_cast<uintptr_t>(p.codes) & 3) == 0 &&
+                         (reinterpret_cast<uintptr_t>(p.w) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.pk) & 15) == 0 &&
+                         ((p.c_b | p.c_h | p.w_b | p.w_h | p.w_l) & 3) == 0 && ((p.p_b | p.p_h | p.p_l) & 15) == 0;
   dim3 grid((unsigned)(bs * H), (unsigned)((L + p.chunk - 1) / p.chunk));
   PK_REQUIRE(grid.y <= 65535, "too many keys for one call");
   StageTimer tm(ST_ENCODE, (cudaStream_t)stream);
@@ -499,7 +501,7 @@ extern "C" int pk_encode_keys(const pk_tensor* keys, const pk_tensor* signs, con
 
 // The tensors of one cache layer that pk_append_encode and pk_prefill_sample share.
 struct CacheLayer {
-  int64_t bs, H, cap_w, cap_z, w_b, w_h;
+  int64_t bs, H, cap_w, cap_z, w_b, w_h, z_wl, z_pl;
   float* z_vnorm;
 };
 static int check_cache_layer(CacheLayer* c, const pk_tensor* window_k, const pk_tensor* window_v, const pk_tensor* win_codes,
@@ -539,14 +541,14 @@ static int check_cache_layer(CacheLayer* c, const pk_tensor* window_k, const pk_
   PK_REQUIRE(codebook->shape[0] == bs && codebook->shape[1] == H && codebook->shape[2] == 16 && codebook->stride[2] == 1 &&
                  codebook->stride[3] == 16 && codebook->stride[1] == cap_z * 16 && (bs == 1 || codebook->stride[0] == H * cap_z * 16),
              "codebook must be the key-major [bs,H,16,cap] view of a contiguous [bs,H,cap,16] buffer");
-  PK_REQUIRE(block_weight->shape[3] == cap_z && block_weight->shape[2] == 16 && block_weight->stride[2] == 1 &&
-                 block_weight->stride[3] == 16 && block_weight->stride[1] == cap_z * 16 &&
-                 (bs == 1 || block_weight->stride[0] == H * cap_z * 16),
-             "block_weight must be the key-major [bs,H,16,cap] view of a contiguous [bs,H,cap,16] buffer");
+  const int64_t wl = block_weight->stride[3], pl = packed_4bit->stride[3];   // from key to key; the heads follow each other
+  PK_REQUIRE(block_weight->shape[3] == cap_z && block_weight->shape[2] == 16 && block_weight->stride[2] == 1 && wl >= 16 &&
+                 wl % 8 == 0 && block_weight->stride[1] == cap_z * wl && (bs == 1 || block_weight->stride[0] == H * cap_z * wl),
+             "block_weight must be the key-major [bs,H,16,cap] view of [bs,H,cap] records of at least 16 elements, a multiple of 8");
   PK_REQUIRE(packed_4bit->shape[3] == cap_z && packed_4bit->shape[2] == 16 && packed_4bit->shape[4] == 4 &&
-                 packed_4bit->stride[4] == 1 && packed_4bit->stride[2] == 4 && packed_4bit->stride[3] == 64 &&
-                 packed_4bit->stride[1] == cap_z * 64 && (bs == 1 || packed_4bit->stride[0] == H * cap_z * 64),
-             "packed_4bit must be the key-major [bs,H,16,cap,4] view of a contiguous [bs,H,cap,16,4] buffer");
+                 packed_4bit->stride[4] == 1 && packed_4bit->stride[2] == 4 && pl >= 64 && pl % 16 == 0 &&
+                 packed_4bit->stride[1] == cap_z * pl && (bs == 1 || packed_4bit->stride[0] == H * cap_z * pl),
+             "packed_4bit must be the key-major [bs,H,16,cap,4] view of [bs,H,cap] records of at least 64 bytes, a multiple of 16");
   for (const pk_tensor* t : {codebook, block_weight, packed_4bit})
     PK_REQUIRE((reinterpret_cast<uintptr_t>(t->data) & 15) == 0, "zone records must be 16-byte aligned");
   float* zv = nullptr;
@@ -560,7 +562,7 @@ static int check_cache_layer(CacheLayer* c, const pk_tensor* window_k, const pk_
                  cluster_counts->shape[2] == 16 && cluster_counts->shape[3] == 256,
              "cluster_counts must be contiguous [bs,H,16,256]");
   PK_REQUIRE(state->stride[0] == 1 && state->shape[0] >= 4 + bs, "state must hold 4 + bs int32 words");
-  c->bs = bs, c->H = H, c->cap_w = cap_w, c->cap_z = cap_z, c->z_vnorm = zv;
+  c->bs = bs, c->H = H, c->cap_w = cap_w, c->cap_z = cap_z, c->z_vnorm = zv, c->z_wl = wl, c->z_pl = pl;
   c->w_b = bs == 1 ? 0 : window_k->stride[0], c->w_h = H == 1 ? 0 : window_k->stride[1];
   return PK_OK;
 }
@@ -608,8 +610,8 @@ extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const p
   const int64_t wr = b * H * c.cap_w, zr = b * H * c.cap_z;
   p.win_codes = (uint8_t*)win_codes->data + wr * 16, p.win_w = (uint16_t*)win_weight->data + wr * 16;
   p.win_pk = (uint8_t*)win_4bit->data + wr * 64, p.win_vnorm = (float*)win_vnorm->data + wr;
-  p.z_codes = (uint8_t*)codebook->data + zr * 16, p.z_w = (uint16_t*)block_weight->data + zr * 16;
-  p.z_pk = (uint8_t*)packed_4bit->data + zr * 64, p.z_vnorm = c.z_vnorm ? c.z_vnorm + zr : nullptr;
+  p.z_codes = (uint8_t*)codebook->data + zr * 16, p.z_w = (uint16_t*)block_weight->data + zr * c.z_wl;
+  p.z_pk = (uint8_t*)packed_4bit->data + zr * c.z_pl, p.z_wl = c.z_wl, p.z_pl = c.z_pl, p.z_vnorm = c.z_vnorm ? c.z_vnorm + zr : nullptr;
   p.counts = (int32_t*)cluster_counts->data + b * H * 16 * 256;
   p.state = (int32_t*)state->data;
   p.P = P, p.N = N, p.cap_z = c.cap_z;
@@ -740,7 +742,7 @@ extern "C" int pk_append_encode(const pk_tensor* k_row, const pk_tensor* v_row, 
   p.win_codes = (uint8_t*)win_codes->data, p.win_w = (uint16_t*)win_weight->data, p.win_pk = (uint8_t*)win_4bit->data;
   p.win_vnorm = (float*)win_vnorm->data;
   p.z_codes = (uint8_t*)codebook->data, p.z_w = (uint16_t*)block_weight->data, p.z_pk = (uint8_t*)packed_4bit->data;
-  p.z_vnorm = zv;
+  p.z_wl = c.z_wl, p.z_pl = c.z_pl, p.z_vnorm = zv;
   p.counts = (int32_t*)cluster_counts->data;
   p.store = (uint16_t*)store_kv->data;
   p.state = (int32_t*)state->data;
