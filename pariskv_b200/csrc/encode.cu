@@ -265,13 +265,13 @@ __global__ void __launch_bounds__(32) query_prep_kernel(const uint16_t* queries,
 // ---- append one decode token: window row, key coding, and the flush of a full update buffer, one launch ----------
 // Device-side state per layer (int32): [0] rows in the window, [1] arrival counter, [2] flushes done, [3] error flag,
 // [4 + b] searchable keys of sample b.  One block per (batch, KV head):
-//   * warp 0 writes the K and V row at window row `pos`, codes the key (the arithmetic of encode_kernel) and stores
-//     the codes, the rerank weights, the 4-bit codes and ||v|| in the window-aligned staging arrays, so every key is
-//     coded exactly once, when it arrives;
+//   * the K and V row go to window row `pos`, the key is coded (the arithmetic of encode_kernel) and its codes, the rerank
+//     weights, the 4-bit codes and ||v|| go to the window-aligned staging arrays, so every key is coded exactly once, when
+//     it arrives;
 //   * if that row filled the window, the oldest `interval` rows behind the sink are PUBLISHED: their staged records
 //     are copied to zone records [N, N + interval), their codes are added to the cluster histogram, their K/V rows go
 //     to the store (device or pinned host memory), and the rest of the window slides down;
-//   * the block that finishes last advances the state words.
+//   * the block that arrives last advances the state words.
 // Everything a later kernel needs (window length, zone length) is read from the state words, so the launch arguments
 // never change and one captured CUDA graph serves the whole generation, flushes included.
 struct AppendParams {
@@ -298,11 +298,58 @@ struct AppendParams {
   int64_t cap_z, cap_s;
 };
 
+// One key by a whole warp, four dimensions per lane: the same bits as code_key, which codes eight keys in the same time.  For
+// a single key the latency counts, and that of fetching the instructions: a fifth of code_key's.
+struct LaneCode {
+  uint32_t packed;   // the lane's four 4-bit codes
+  uint32_t code;     // even lanes: the sign code of subspace lane / 2
+  uint16_t weight;   // even lanes: its rerank weight
+};
+__device__ __forceinline__ LaneCode code_key_warp(uint2 raw, uint2 signs, int lane) {
+  float x[4] = {lo_f(raw.x), hi_f(raw.x), lo_f(raw.y), hi_f(raw.y)};
+  const float sg[4] = {lo_f(signs.x), hi_f(signs.x), lo_f(signs.y), hi_f(signs.y)};
+  const float n = rotate4(x, sg, lane);
+  float t[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) x[i] = __fadd_rn(x[i], 0.0f), t[i] = __fmul_rn(x[i], x[i]);   // -0 counts as non-negative
+  // adjacent pairwise tree over the eight dimensions of a subspace: two lanes
+  auto tree = [&](const float (&v)[4]) -> float {
+    const float s4 = __fadd_rn(__fadd_rn(v[0], v[1]), __fadd_rn(v[2], v[3]));
+    return __fadd_rn(s4, __shfl_xor_sync(FULL, s4, 1));
+  };
+  const float r = bfround(__fsqrt_rn(tree(t)));
+  const float ri = rcp_approx(fmaxf(r, bfround(1e-8f)));
+  uint32_t nib[2], p[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {   // dimensions 2 k, 2 k + 1 of the lane
+    const uint32_t au = bf16_2(__fmul_rn(x[2 * k], ri), __fmul_rn(x[2 * k + 1], ri)) & 0x7fff7fffu;
+    const uint32_t l = level_b2(au) & 0x00070007u;
+    p[k] = fma_b2(centre_b2(l), au, b2(0x8000));
+    const uint32_t v = l | (~bf16_2(x[2 * k], x[2 * k + 1]) >> 12 & 0x00080008u);   // sign | level
+    nib[k] = (v | (v >> 12)) & 0xffu;
+  }
+  const float pr[4] = {lo_f(p[0]), hi_f(p[0]), lo_f(p[1]), hi_f(p[1])};
+  const float al = fmaxf(tree(pr), 1e-6f);
+  LaneCode out;
+  out.packed = nib[0] | (nib[1] << 8);
+  uint32_t v = (out.packed >> 3) & 0x1111u;   // bit 3 of every nibble, gathered
+  v = (v | (v >> 3)) & 0x0303u;
+  v = (v | (v >> 6)) & 0xfu;
+  out.code = v | (__shfl_xor_sync(FULL, v, 1) << 4);
+  out.weight = f2bf(__fmul_rn(__fdiv_rn(r, al), n));
+  return out;
+}
+
+// What bounds it is the latency of dependent steps: the state words and the rows (one round trip), the coding, the stores.
+// Warp 0 codes the key, warp 1 copies the rows and takes ||v||.  The blocks arrive as soon as they have read the state words,
+// while the key is coded, not behind their writes: the new words are for the kernels that wait for all of this one.  On B200,
+// a step of four layers, against warp 0 doing everything with code_key and the arrival at the end: 10K keys in host memory
+// 178.3 -> 168.9 us, 128K keys 221.9 -> 212.4, a KV head of eight sequences 214.5 -> 208.0; two layers with adaptive budgets
+// of eight sequences 144.7 -> 136.0.
 __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t bh = blockIdx.x;
   const int b = (int)(bh / p.H), h = (int)(bh % p.H);
-  __shared__ int s_last;
   pdl_wait();     // the rows to append and the state words come from the kernels before this one
   pdl_trigger();
   const int pos = p.state[0];
@@ -313,21 +360,49 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
   uint16_t* ww = p.win_w + bh * p.cap_w * 16;
   uint8_t* wp = p.win_pk + bh * p.cap_w * 64;
   float* wn = p.win_vnorm + bh * p.cap_w;
-  const bool ok = pos >= 0 && pos < p.cap_w;
-  if (tid < 32) {   // the loads do not wait for the position
-    const int s = lane & 3, l = lane & 15;
-    const uint16_t* kr = p.k_row + b * p.kr_b + h * p.kr_h;
-    const uint4* vr = reinterpret_cast<const uint4*>(p.v_row + b * p.vr_b + h * p.vr_h);
-    // the rows themselves: lanes 0-15 carry K, lanes 16-31 carry V
-    const uint4 cp = (lane < 16 ? reinterpret_cast<const uint4*>(kr) : vr)[l];
-    uint4 raw[4];
-    load_key32(raw, kr, s);
-    RotateLane rl;
-    make_rotate_lane(rl, p.signs, s);
-    float y[8];
-    unpack8(vr[l], y);
-    if (ok) reinterpret_cast<uint4*>((lane < 16 ? wk : wv) + (int64_t)pos * 128)[l] = cp;
+  const uint16_t* kr = p.k_row + b * p.kr_b + h * p.kr_h;
+  const uint16_t* vr = p.v_row + b * p.vr_b + h * p.vr_h;
+  uint2 key, sg;
+  uint4 row;
+  if (warp == 0) {
+    key = reinterpret_cast<const uint2*>(kr)[lane], sg = reinterpret_cast<const uint2*>(p.signs)[lane];
+  } else if (warp == 1) {   // lanes 0-15 carry K, lanes 16-31 carry V
+    row = reinterpret_cast<const uint4*>(lane < 16 ? kr : vr)[lane & 15];
+  }
+  // every thread has its words when it passes (the vote uses them)
+  const bool ok = __syncthreads_and(pos >= 0 && pos < p.cap_w && N >= 0) != 0;
+  const int I = p.interval, sink = p.sink;
+  const bool flush = ok && pos + 1 == p.cap_w;
+  const bool room = N >= 0 && N + I <= p.cap_z && N + I <= p.cap_s;
+  if (tid == 64) {   // the block that arrives last advances the state: every block has read it
+    __threadfence();
+    if (atomicAdd(reinterpret_cast<unsigned*>(p.state + 1), 1u) + 1u == gridDim.x) {
+      if (!ok || (flush && !room)) {
+        p.state[3] = 1;   // window overrun or zone full: the host checks this word
+      } else if (flush) {
+        p.state[0] = p.cap_w - I;
+        p.state[2] += 1;
+        const int bs = (int)(gridDim.x / p.H);
+        for (int i = 0; i < bs; i++) p.state[4 + i] += I;
+      } else {
+        p.state[0] = pos + 1;
+      }
+      p.state[1] = 0;
+    }
+  }
+  if (warp == 0) {
+    const LaneCode kc = code_key_warp(key, sg, lane);
+    if (ok) {
+      reinterpret_cast<uint16_t*>(wp + (int64_t)pos * 64)[lane] = (uint16_t)kc.packed;
+      if (!(lane & 1)) {
+        wc[(int64_t)pos * 16 + (lane >> 1)] = (uint8_t)kc.code;
+        ww[(int64_t)pos * 16 + (lane >> 1)] = kc.weight;
+      }
+    }
+  } else if (warp == 1) {
     // ||v||: fp32, pairwise tree over adjacent dimensions
+    float y[8];
+    unpack8(row, y);
 #pragma unroll
     for (int i = 0; i < 8; i++) y[i] = __fmul_rn(y[i], y[i]);
 #pragma unroll
@@ -337,19 +412,13 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
     float vs = y[0];
 #pragma unroll
     for (int off = 1; off < 16; off <<= 1) vs = __fadd_rn(vs, __shfl_xor_sync(FULL, vs, off));
-    const KeyCode kc = code_key(raw, rl);   // (eight times the same: every group of four lanes)
-    if (ok && lane < 4) {
-      *reinterpret_cast<uint32_t*>(wc + (int64_t)pos * 16 + 4 * s) = kc.codes;
-      *reinterpret_cast<uint2*>(ww + (int64_t)pos * 16 + 4 * s) = kc.weights;
-      *reinterpret_cast<uint4*>(wp + (int64_t)pos * 64 + 16 * s) = kc.packed;
-      if (lane == 0) wn[pos] = __fsqrt_rn(vs);
+    if (ok) {
+      reinterpret_cast<uint4*>((lane < 16 ? wk : wv) + (int64_t)pos * 128)[lane & 15] = row;
+      if (lane == 16) wn[pos] = __fsqrt_rn(vs);
     }
   }
-  __syncthreads();
-  const int I = p.interval, sink = p.sink;
-  const bool flush = ok && pos + 1 == p.cap_w;
-  const bool room = N >= 0 && N + I <= p.cap_z && N + I <= p.cap_s;
   if (flush && room) {
+    __syncthreads();   // the new row and its records
     // publish rows [sink, sink + I): staged records -> zone records [N, N + I), K/V rows -> store, histogram
     const uint4* sc = reinterpret_cast<const uint4*>(wc + (int64_t)sink * 16);
     const uint4* sp = reinterpret_cast<const uint4*>(wp + (int64_t)sink * 64);
@@ -390,26 +459,6 @@ __global__ void __launch_bounds__(256) append_encode_kernel(AppendParams p) {
       for (int i = tid; i < rows; i += 256) wn[sink + r0 + i] = wn[sink + I + r0 + i];
       __syncthreads();
     }
-  }
-  // the block that arrives last advances the state (every block has read it by then)
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    s_last = atomicAdd(reinterpret_cast<unsigned*>(p.state + 1), 1u) + 1u == gridDim.x;
-  }
-  __syncthreads();
-  if (s_last && tid == 0) {
-    if (!ok || (flush && !room)) {
-      p.state[3] = 1;   // window overrun or zone full: the host checks this word
-    } else if (flush) {
-      p.state[0] = p.cap_w - I;
-      p.state[2] += 1;
-      const int bs = (int)(gridDim.x / p.H);
-      for (int i = 0; i < bs; i++) p.state[4 + i] += I;
-    } else {
-      p.state[0] = pos + 1;
-    }
-    p.state[1] = 0;
   }
 }
 

@@ -81,6 +81,19 @@ constexpr uint32_t LV_D51 = b2(0x3ec7), LV_D40 = b2(0x3ebb), LV_D20 = b2(0x3e32)
 // centres 0.0420 0.1270 0.2129 0.3027 0.3965 0.5 0.6172 0.7617 (bf16), low and high bytes of the eight
 constexpr uint32_t CEN_LO0 = 0x9b5a022cu, CEN_LO1 = 0x431e00cbu, CEN_HI0 = 0x3e3e3e3du, CEN_HI1 = 0x3f3f3f3eu;
 
+// levels of two magnitudes, in the low three bits of either half: 128 + level as bf16 has the level in the low bits of its pattern
+__device__ __forceinline__ uint32_t level_b2(uint32_t a) {
+  const uint32_t m1 = gt_b2(a, LV_T3);
+  const uint32_t m2 = gt_b2(a, fma_b2(m1, LV_D51, LV_T1));
+  const uint32_t m3 = gt_b2(a, fma_b2(m2, fma_b2(m1, LV_D64, LV_D20), fma_b2(m1, LV_D40, LV_T0)));
+  return fma_b2(m1, b2(0x4080), fma_b2(m2, b2(0x4000), fma_b2(m3, b2(0x3f80), b2(0x4300))));
+}
+// centres of two levels l.lo, l.hi < 8, by byte permutes
+__device__ __forceinline__ uint32_t centre_b2(uint32_t l) {
+  const uint32_t sel = l | (l >> 12);   // three bits per nibble
+  return __byte_perm(__byte_perm(CEN_LO0, CEN_LO1, sel), __byte_perm(CEN_HI0, CEN_HI1, sel), 0x5140);
+}
+
 struct KeyCode {
   uint32_t codes;    // sign codes of the lane's four subspaces, low byte first
   uint2 weights;     // their rerank weights, four bf16
@@ -213,12 +226,7 @@ __device__ __forceinline__ KeyCode code_key(const uint4 (&raw)[4], const RotateL
       for (int k = 0; k < 2; k++) {
         const int i = 2 * j + k;
         const uint32_t a = au[k] = bf16_2(mul_2(x[8 * g + i], ri)) & 0x7fff7fffu;
-        const uint32_t m1 = gt_b2(a, LV_T3);
-        const uint32_t m2 = gt_b2(a, fma_b2(m1, LV_D51, LV_T1));
-        const uint32_t m3 = gt_b2(a, fma_b2(m2, fma_b2(m1, LV_D64, LV_D20), fma_b2(m1, LV_D40, LV_T0)));
-        // 128 + level as bf16: the level is the low bits of its pattern
-        const uint32_t l = fma_b2(m1, b2(0x4080), fma_b2(m2, b2(0x4000), fma_b2(m3, b2(0x3f80), b2(0x4300))));
-        lv[k] = (l & 0x00070007u) | ((~y[i] >> 12) & 0x00080008u);   // sign | level nibbles
+        lv[k] = (level_b2(a) & 0x00070007u) | ((~y[i] >> 12) & 0x00080008u);   // sign | level nibbles
       }
       const uint32_t nib = lv[0] | (lv[1] << 8);
       u[j] = nib | (nib >> 4);

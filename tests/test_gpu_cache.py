@@ -496,3 +496,37 @@ def test_append_reports_a_full_zone_through_its_status_word():
     assert st.tolist()[3] == 1 and st.tolist()[4] == cache.zone_capacity
     with pytest.raises(RuntimeError, match="no room for a flush"):
         cache.check_status()
+
+
+def test_appended_key_has_the_bits_of_the_bulk_coder(oracle):
+    """The append codes a key on a whole warp, the prefill and encode_keys on four lanes: same records for ordinary keys and
+    for keys at the edges (zeros of both signs, one coordinate, equal coordinates, very large and very small norms)."""
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(11)
+    bs, H, n = 2, 3, 24
+    keys = synth_keys(g, bs, H, n).float()
+    keys[0, 0, 0] = 0.0
+    keys[0, 0, 1] = -0.0
+    keys[0, 1, 2] = 0.0
+    keys[0, 1, 2, 77] = -3.0
+    keys[0, 2, 3] = 1.5
+    keys[1, 0, 4] *= 1e15
+    keys[1, 1, 5] *= 1e-15
+    keys[1, 2, 6, 64:] = 0.0
+    keys = keys.to(torch.bfloat16)
+    V = torch.randn(bs, H, n, 128, generator=g).to(torch.bfloat16)
+    cache = _make_cache(30, 64, bs, H, 4 * H, 4, 8, 64, 16, False, layers=1)
+    first = synth_keys(g, bs, H, 12)
+    cache.prefill_update_kv_cache(None, *(first.transpose(1, 2).contiguous().to(DEV),) * 2, 0, 0)
+    for t in range(n):
+        cache.decode_update_kv_cache(keys[:, :, t:t + 1].transpose(1, 2).contiguous().to(DEV),
+                                     V[:, :, t:t + 1].transpose(1, 2).contiguous().to(DEV), 0)
+    cb, w, pk = ops.encode_keys(keys.to(DEV), cache.srht_diagonal_signs)
+    rows = slice(12, 12 + n)
+    assert torch.equal(cache._win_codes[0][:, :, rows].permute(0, 1, 3, 2), cb)
+    assert torch.equal(cache._win_weight[0][:, :, rows].permute(0, 1, 3, 2).float(), w.float())
+    assert torch.equal(cache._win_4bit[0][:, :, rows].permute(0, 1, 3, 2, 4), pk)
+    cb_o, w_o, pk_o = oracle.encode(keys, cache.srht_diagonal_signs.cpu())
+    assert torch.equal(cb.cpu(), cb_o) and torch.equal(w.cpu().float(), w_o.float()) and torch.equal(pk.cpu(), pk_o)
+    assert torch.equal(cache.unified_keys_gpu[0][:, :, rows].cpu(), keys) and torch.equal(cache.unified_values_gpu[0][:, :, rows].cpu(), V)
+    assert cache._layer_state[0].tolist()[:4] == [12 + n, 0, 0, 0]
