@@ -284,16 +284,10 @@ __device__ __forceinline__ void publish_query(const PreparedQuery& pq, const Cha
   if (cq.q_blocks) *reinterpret_cast<uint2*>(cq.q_blocks + bh * 128 + 4 * lane) = words(pq.x);
   if (cq.q_norm && lane == 0) cq.q_norm[bh] = f2bf(pq.n);
 }
-__device__ __forceinline__ void load_tiers(const ChainQuery& cq, long long N, unsigned* s_tiers) {   // one thread
-  if (cq.n_dev) {
-    unsigned t[8];
-    zone_tiers(cq.sched, N, t);
-    for (int i = 0; i < cq.sched.n_tiers; i++) s_tiers[i] = t[i];
-    s_tiers[8] = (unsigned)cq.sched.n_tiers;
-  } else {
-    for (int i = 0; i < cq.n_tiers; i++) s_tiers[i] = cq.tiers[i];
-    s_tiers[8] = (unsigned)cq.n_tiers;
-  }
+__device__ __forceinline__ void load_tiers(const ChainQuery& cq, long long N, unsigned* s_tiers, int t) {   // threads t = 0 .. 8
+  const int n = cq.n_dev ? cq.sched.n_tiers : cq.n_tiers;
+  if (t < n) s_tiers[t] = cq.n_dev ? zone_tier(cq.sched, N, t) : cq.tiers[t];
+  if (t == 8) s_tiers[8] = (unsigned)n;
 }
 // Tier table of one subspace by its warp.  sizes: 256 words with the cluster sizes (overwritten); key: the order made by
 // rank_subspace; lut: the subspace's 128 bytes (see tier_sum16).
@@ -409,7 +403,8 @@ __device__ __forceinline__ int list_candidates(uint8_t* cnt8, int n_keys, int sk
 }
 
 // 4-bit rerank of a list by one block, from key-major records: key_at(i) -> sink(i, key, score).  ids: the keys of the first
-// n_ids candidates in shared memory (all of them, or a multiple of 32); q: the rotated query, 128 bf16 in shared memory.
+// n_ids candidates in shared memory (all of them, or a multiple of 32); q: the rotated query, 128 bf16 in shared memory;
+// after_round(): called by whole warps behind each of their rounds.
 // A warp takes 32 consecutive candidates per round.  The records of its next round are on their way to its staging buffer by
 // cp.async while it works on this one, which it has read into registers, one record per lane: 24 lanes fetch four records per
 // instruction, six 16-byte pieces each.
@@ -418,10 +413,10 @@ __device__ __forceinline__ int list_candidates(uint8_t* cnt8, int n_keys, int sk
 // and packed fp32 products (264 wavefronts, 593 instructions a round), 33 like this (493 instructions).  16 sequences of
 // 16 - 32K keys 232.6 -> 219.5 us a step of two layers, adaptive budgets of 8 sequences 155.1 -> 147.1, 1M keys 135.0 -> 132.1.
 // A second buffer per warp, two candidates per lane and the TMA's four-row gather were no faster.
-template <class KeyAt, class Sink>
+template <class KeyAt, class Sink, class AfterRound>
 __device__ __forceinline__ void rerank_list(int n_list, const int* ids, int n_ids, const RerankArgs& a, const uint8_t* k4, const uint16_t* w,
                                             uint8_t* stage, const uint32_t* lev2, const uint4* q, float qn, unsigned c128, KeyAt key_at,
-                                            Sink sink) {
+                                            Sink sink, AfterRound after_round) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int ROUND = CH_WARPS * 32;
   const int sub = (lane * 43) >> 8, piece = lane - 6 * sub;   // lane / 6 and the rest
@@ -457,6 +452,8 @@ __device__ __forceinline__ void rerank_list(int n_list, const int* ids, int n_id
     const float v = rerank_record(rec, lev2, q, qn, lane, c128);
     const int i = base + lane;
     if (i < n_list) sink(i, key_at(i), v);
+    __syncwarp();
+    after_round();
   }
 }
 

@@ -5,10 +5,15 @@
 //                                               eight bits of (key - lowest key) for whole numbers, exact at any size
 //   histogram of the bins, summed over ranks -> the bin of the K-th largest, this CTA's share above it and in it
 //   the elements of that bin, gathered by every CTA, cut once more into 64 sub-bins and ranked -> the exact threshold
-//   ordered emission of this CTA's elements at its offset.
+//   ordered emission of this CTA's elements at its offset, a warp per 32 elements.
 // Where more than SEL_TIES elements share the bin (flat rows, equal counts), further levels bin their ordered keys; if
-// that many are equal, the lowest positions win.  Three exchanges through distributed shared memory in the usual case.
-// What bounds it is their latency and three passes over the slice: 7 us for 13 K scores over 8 CTAs, where one CTA took 12.
+// that many are equal, the lowest positions win.  Three exchanges in the usual case: what a CTA knows it WRITES into the
+// shared memory of all CTAs, then comes a cluster barrier, and everything is read at home.  (Reading from the others behind the
+// barrier adds a round trip over the cluster to each, two for the members, and a barrier before a CTA may leave.)  A caller
+// that makes the values itself can have the extremes exchanged while it still does (see `published`).
+// What bounds it is the latency of these steps and three passes over the slice.  On B200 the last stage of the chain takes 7.2
+// us with 1310 scores on each of 10 CTAs (9.7 with remote reads, the emission a word per lane and every rank counted in
+// sub-bins), 6.1 with 655 (9.5), 7 - 10 with some 5000 on one CTA (10 - 13).
 #pragma once
 #include <cooperative_groups.h>
 
@@ -26,7 +31,10 @@ constexpr int SEL_WARPS = SEL_THREADS / 32;
 constexpr int SEL_BINS = 256;
 constexpr int SEL_SUB = 64;
 constexpr int SEL_TIES = 1024;
-constexpr int SEL_REGION = 2 * SEL_TIES * 8;   // bytes of dynamic shared memory, at the same offset in every CTA
+constexpr int SEL_REGION = 2 * SEL_TIES * 8;   // bytes of dynamic shared memory
+// What the CTAs of a cluster write into each other, at the same offset of dynamic shared memory in every CTA and used by nothing
+// else: histograms [rank][SEL_BINS], extremes [rank][warp].
+__host__ __device__ constexpr int sel_inbox_bytes(int cs) { return cs * (SEL_BINS * 4 + SEL_WARPS * 8); }
 
 // Rows of a type: the ordered key of an element, and the level-0 bins between the extremes of the row's keys.  A bin is
 // monotone in the key; sub() cuts a bin into SEL_SUB parts, monotone as well; single(): a bin holds one value.
@@ -41,7 +49,7 @@ struct F32Row {
       if (!(scale > 0.0f) || !(scale < INFINITY)) scale = 0.0f;   // flat or non-finite: one bin, the key levels decide
     }
     __device__ __forceinline__ unsigned of(uint32_t u) const {
-      return min((unsigned)(SEL_BINS - 1), (unsigned)((__uint_as_float(u) - vmin) * scale));
+      return min((unsigned)(SEL_BINS - 1), __float2uint_rz((__uint_as_float(u) - vmin) * scale));   // (below vmin: 0)
     }
     __device__ __forceinline__ unsigned sub(uint32_t k, unsigned bin) const {
       return scale > 0.0f ? min((unsigned)(SEL_SUB - 1), (unsigned)max(0.0f, ((from_key(k) - vmin) * scale - (float)bin) * (float)SEL_SUB)) : 0u;
@@ -63,14 +71,11 @@ struct I32Row {
 };
 static_assert(SEL_BINS == 256 && SEL_SUB == 64, "the shifts of I32Row::Bins");
 
-struct SelShared {               // static: what other CTAs of the cluster read, and small block-wide results
-  unsigned hist[2][SEL_BINS];    // local histograms, used alternately
-  unsigned kmin, kmax;           // extremes of the ordered keys of this slice
+struct SelShared {               // static: small block-wide results
   unsigned n_members;            // local elements of the threshold bin
   unsigned thr_key, thr_pos;     // the last element taken from the threshold bin
   unsigned lower_sel;            // elements taken from the threshold bin by lower ranks
   unsigned res[5];               // threshold bin, elements above it, elements in it, the same two of lower ranks
-  unsigned range[2];
   unsigned warp_a[SEL_WARPS], warp_b[SEL_WARPS];
   unsigned sub[SEL_SUB], n_few;
 };
@@ -94,27 +99,39 @@ __device__ __forceinline__ void sync_cluster(cg::cluster_group& cluster) {
   else cluster.sync();
 }
 
-// Threshold of a histogram spread over the cluster: thread t sums bin t over the local histograms of all CTAs, a
-// block-wide suffix scan finds the highest bin with (elements in bins >= it) >= want; see SelShared::res.  Returns after
-// the result is visible to the block.
+// value -> *at in CTA r of the cluster, for all r: lane r of a warp (all lanes hold the value), or a thread for all CTAs
+template <int CS, class T>
+__device__ __forceinline__ void put_by_lanes(cg::cluster_group& cluster, T* at, T value, int lane) {
+  if (CS == 1) {
+    if (lane == 0) *at = value;
+  } else if (lane < CS) {
+    *cluster.map_shared_rank(at, lane) = value;
+  }
+}
+template <int CS, class T>
+__device__ __forceinline__ void put_everywhere(cg::cluster_group& cluster, T* at, T value) {
+  if (CS == 1) {
+    *at = value;
+  } else {
+#pragma unroll
+    for (int r = 0; r < CS; r++) *cluster.map_shared_rank(at, r) = value;
+  }
+}
+
+// Threshold of a histogram spread over the cluster, after the barrier that completes hists ([CS][SEL_BINS], one row per CTA):
+// thread t sums bin t, a block-wide suffix scan finds the highest bin with (elements in bins >= it) >= want; see
+// SelShared::res.  Returns after the result is visible to the block.
 template <int CS, int BINS>
-__device__ __forceinline__ void cluster_threshold(cg::cluster_group& cluster, SelShared& s, const unsigned* mine, unsigned rank,
-                                                  unsigned want) {
-  static_assert(BINS <= SEL_THREADS, "one bin per thread");
+__device__ __forceinline__ void cluster_threshold(SelShared& s, const unsigned* hists, unsigned rank, unsigned want) {
+  static_assert(BINS <= SEL_THREADS && BINS <= SEL_BINS, "one bin per thread");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned tot = 0, pre = 0;
   if (tid < BINS) {
-    if (CS == 1) {
-      tot = mine[tid];
-    } else {
-      unsigned v[CS];
 #pragma unroll
-      for (int r = 0; r < CS; r++) v[r] = cluster.map_shared_rank(mine, r)[tid];
-#pragma unroll
-      for (int r = 0; r < CS; r++) {
-        tot += v[r];
-        if ((unsigned)r < rank) pre += v[r];
-      }
+    for (int r = 0; r < CS; r++) {
+      const unsigned v = hists[r * SEL_BINS + tid];
+      tot += v;
+      if ((unsigned)r < rank) pre += v;
     }
   }
   unsigned suf = tot, psuf = pre;   // inclusive suffix over the lanes
@@ -125,64 +142,75 @@ __device__ __forceinline__ void cluster_threshold(cg::cluster_group& cluster, Se
   }
   if (lane == 0) s.warp_a[warp] = suf, s.warp_b[warp] = psuf;
   __syncthreads();
-  for (int w = warp + 1; w < (BINS + 31) / 32; w++) suf += s.warp_a[w], psuf += s.warp_b[w];
+  const bool later = lane > warp && lane < (BINS + 31) / 32;   // the sums of the warps behind this one
+  suf += __reduce_add_sync(0xffffffffu, later ? s.warp_a[lane] : 0u), psuf += __reduce_add_sync(0xffffffffu, later ? s.warp_b[lane] : 0u);
   const unsigned above = suf - tot;
   if (tot && above < want && suf >= want)
     s.res[0] = (unsigned)tid, s.res[1] = above, s.res[2] = tot, s.res[3] = psuf - pre, s.res[4] = pre;
   __syncthreads();
 }
 
+// A warp's extremes into the inboxes of all CTAs.
+template <int CS>
+__device__ __forceinline__ void publish_range(cg::cluster_group& cluster, unsigned* inbox, unsigned rank, unsigned kmin, unsigned kmax) {
+  uint2* extremes = reinterpret_cast<uint2*>(inbox + CS * SEL_BINS);
+  kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
+  put_by_lanes<CS>(cluster, extremes + rank * SEL_WARPS + (threadIdx.x >> 5), make_uint2(kmin, kmax), threadIdx.x & 31);
+}
+
 // n: elements of this slice; at(i): raw 32 bits of element i; out_of(i): the 64-bit value to emit for it.
-// kmin / kmax: this thread's share of the extremes of the slice's ordered keys (~0 / 0 without any).
-// region: SEL_REGION bytes; words: 2 * words_cap words of this CTA's shared memory for ballots (longer slices are
-// evaluated again instead).  All CTAs of the cluster call this with the same K (>= 1, at most the row's length).
-// The caller must not leave before cluster.barrier_wait() if CS > 1: the closing arrive is done here.
-template <int CS, class V, class At, class OutOf>
-__device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelShared& s, unsigned* region, unsigned* words,
-                                               int words_cap, unsigned rank, int n, int K, int64_t* __restrict__ out, At at,
-                                               OutOf out_of, unsigned kmin, unsigned kmax) {
+// kmin / kmax: this thread's share of the extremes of the slice's ordered keys (~0 / 0 without any).  published: every warp has
+// called publish_range() with the extremes of some of the slice's elements, and every thread has arrived at a cluster barrier
+// (CS > 1) behind it; the level-0 bins then lie between those extremes, elements outside fall into the first and the last one.
+// region: SEL_REGION bytes, inbox: sel_inbox_bytes(CS), at the same offsets in all CTAs; words: 2 * words_cap words of this
+// CTA's shared memory for ballots (longer slices are evaluated again instead).  All CTAs of the cluster call this with the same
+// K (>= 1, at most the row's length), after a cluster barrier, none of them still using its region for anything else.
+// LISTED: the elements are listed in shared memory before out_of() is asked for them, all at once: for values that have to be
+// fetched from global memory.
+template <int CS, class V, bool LISTED, class At, class OutOf>
+__device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelShared& s, unsigned* region, unsigned* inbox,
+                                               unsigned* words, int words_cap, unsigned rank, int n, int K, int64_t* __restrict__ out, At at,
+                                               OutOf out_of, unsigned kmin, unsigned kmax, bool published = false) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  auto publish_range = [&]() {   // extremes over the cluster, to s.range; clears the histogram replicas
-    kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
-    if (lane == 0) s.warp_a[warp] = kmin, s.warp_b[warp] = kmax;
-    __syncthreads();
-    if (warp == 0) {
-      const unsigned lo = __reduce_min_sync(0xffffffffu, s.warp_a[lane & (SEL_WARPS - 1)]);
-      const unsigned hi = __reduce_max_sync(0xffffffffu, s.warp_b[lane & (SEL_WARPS - 1)]);
-      if (lane == 0) s.kmin = lo, s.kmax = hi;
-    }
+  unsigned* hists = inbox;
+  uint2* extremes = reinterpret_cast<uint2*>(inbox + CS * SEL_BINS);
+  auto exchange_range = [&](bool published) {   // extremes over the cluster, to kmin and kmax of every thread; clears the histogram replicas
     for (int i = tid; i < 4 * SEL_BINS; i += SEL_THREADS) region[i] = 0;
-    sync_cluster<CS>(cluster);
-    if (warp == 0) {
-      unsigned lo = 0xffffffffu, hi = 0u;
-      if (lane < CS) {
-        lo = CS == 1 ? s.kmin : *cluster.map_shared_rank(&s.kmin, lane);
-        hi = CS == 1 ? s.kmax : *cluster.map_shared_rank(&s.kmax, lane);
-      }
-      lo = __reduce_min_sync(0xffffffffu, lo), hi = __reduce_max_sync(0xffffffffu, hi);
-      if (lane == 0) s.range[0] = lo, s.range[1] = hi;
+    if (published) {
+      if (CS > 1) cluster.barrier_wait();
+      __syncthreads();
+      kmin = 0xffffffffu, kmax = 0u;
+    } else {
+      publish_range<CS>(cluster, inbox, rank, kmin, kmax);
+      sync_cluster<CS>(cluster);
     }
-    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < (CS * SEL_WARPS + 31) / 32; i++) {
+      const uint2 e = extremes[min(i * 32 + lane, CS * SEL_WARPS - 1)];
+      kmin = min(kmin, e.x), kmax = max(kmax, e.y);
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
   };
   unsigned* my_hist = region + (lane & 3) * SEL_BINS;
-  auto publish_hist = [&](int buf) {
+  auto exchange_hist = [&]() {
     __syncthreads();
-    if (tid < SEL_BINS) s.hist[buf][tid] = region[tid] + region[SEL_BINS + tid] + region[2 * SEL_BINS + tid] + region[3 * SEL_BINS + tid];
+    if (tid < SEL_BINS)
+      put_everywhere<CS>(cluster, hists + rank * SEL_BINS + tid,
+                         region[tid] + region[SEL_BINS + tid] + region[2 * SEL_BINS + tid] + region[3 * SEL_BINS + tid]);
     sync_cluster<CS>(cluster);
   };
   // ---- level 0: bins over the range of the row ----
-  publish_range();
-  const typename V::Bins bins(s.range[0], s.range[1]);
+  exchange_range(published);
+  const typename V::Bins bins(kmin, kmax);
   auto bin0 = [&](uint32_t u) -> unsigned { return bins.of(u); };
 #pragma unroll 4
   for (int i = tid; i < n; i += SEL_THREADS) atomicAdd(&my_hist[bin0(at(i))], 1u);
-  publish_hist(1);
-  cluster_threshold<CS, SEL_BINS>(cluster, s, s.hist[1], rank, (unsigned)K);
+  exchange_hist();
+  cluster_threshold<CS, SEL_BINS>(s, hists, rank, (unsigned)K);
   const unsigned T0 = s.res[0];
   unsigned rem = (unsigned)K - s.res[1], in_bin = s.res[2], pre_above = s.res[3], pre_in = s.res[4];
   // ---- key levels: ordered keys of the members between their extremes ----
   unsigned lo = 0u, hi = 0xffffffffu;
-  int buf = 0;
   while (in_bin > (unsigned)SEL_TIES && lo != hi) {
     kmin = 0xffffffffu, kmax = 0u;
 #pragma unroll 1
@@ -191,8 +219,8 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       if (bin0(u) == T0 && k >= lo && k <= hi) kmin = min(kmin, k), kmax = max(kmax, k);
     }
     __syncthreads();   // s.res and the replicas have been read
-    publish_range();
-    const unsigned base = s.range[0], top = s.range[1];
+    exchange_range(false);
+    const unsigned base = kmin, top = kmax;
     if (base == top) {
       lo = hi = base;
       break;
@@ -203,12 +231,11 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       const uint32_t u = at(i), k = V::key(u);
       if (bin0(u) == T0 && k >= base && k <= top) atomicAdd(&my_hist[(k - base) >> shift], 1u);
     }
-    publish_hist(buf);
-    cluster_threshold<CS, SEL_BINS>(cluster, s, s.hist[buf], rank, rem);
+    exchange_hist();
+    cluster_threshold<CS, SEL_BINS>(s, hists, rank, rem);
     lo = base + (s.res[0] << shift);
     hi = min(lo + ((1u << shift) - 1u), top);
     rem -= s.res[1], in_bin = s.res[2], pre_above += s.res[3], pre_in = s.res[4];
-    buf ^= 1;
   }
   const bool level0 = lo == 0u && hi == 0xffffffffu;
   // the threshold bin holds equal keys only: the lowest positions win, rank by rank (whole numbers in a small range have a
@@ -224,13 +251,15 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       above = k > hi, member = k >= lo && k <= hi;
     }
   };
-  uint2* own = reinterpret_cast<uint2*>(region);   // this CTA's members: (key, rank and position)
-  uint2* all = own + SEL_TIES;                     // everybody's, in rank order
+  // The members of all CTAs, in rank order: (key, rank and position).  The histograms say how many the lower ranks have, so
+  // every CTA writes its own to their place in all of them.  (The histogram replicas there are done with in every CTA: the
+  // barrier of the last histogram lies behind.)
+  uint2* all = reinterpret_cast<uint2*>(region);
+  const uint2* own = all + pre_in;
   const int n_words = (n + 31) / 32;
   const bool kept = n_words <= words_cap;          // otherwise the words are made window by window, after the threshold
   unsigned* above_w = words;
   unsigned* member_w = words + words_cap;
-  __syncthreads();   // the histogram replicas under `own` have been read
   if (tid == 0) s.n_members = 0, s.lower_sel = 0, s.n_few = 0;
   if (tid < SEL_SUB) s.sub[tid] = 0;
   __syncthreads();
@@ -247,94 +276,81 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
         unsigned slot = 0;
         if (lane == 0) slot = atomicAdd(&s.n_members, (unsigned)__popc(mw));
         slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(mw & ((1u << lane) - 1u));
-        if (member && slot < (unsigned)SEL_TIES) own[slot] = make_uint2(V::key(u), (rank << 27) | (unsigned)i);
+        if (member && pre_in + slot < (unsigned)SEL_TIES) put_everywhere<CS>(cluster, all + pre_in + slot, make_uint2(V::key(u), (rank << 27) | (unsigned)i));
       }
     }
   }
   unsigned thr_key = 0u, thr_pos = 0xffffffffu, lower_sel = min(pre_in, rem);
   if (!flat) {
     sync_cluster<CS>(cluster);
-    unsigned before_me = 0, n_all = 0;
-    if (CS == 1) {
-      all = own, n_all = s.n_members;
-    } else {
-      const unsigned m = lane < CS ? *cluster.map_shared_rank(&s.n_members, lane) : 0u;
-      unsigned inc = m;
-#pragma unroll
-      for (int off = 1; off < CS; off <<= 1) {
-        const unsigned o = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += o;
+    const unsigned before_me = pre_in, n_all = min(in_bin, (unsigned)SEL_TIES);
+    if (n_all <= SEL_THREADS / 4) {   // four lanes rank a member
+      const unsigned t = tid >> 2;
+      const uint2 me = t < n_all ? all[t] : make_uint2(0u, 0u);
+      unsigned rk = 0;
+#pragma unroll 4
+      for (unsigned j = tid & 3; j < n_all; j += 4) {
+        const uint2 o = all[j];
+        rk += (o.x > me.x || (o.x == me.x && o.y < me.y)) ? 1u : 0u;
       }
-      n_all = min(__shfl_sync(0xffffffffu, inc, CS - 1), (unsigned)SEL_TIES);
-      before_me = __shfl_sync(0xffffffffu, inc - m, rank);
-      const unsigned off = __shfl_sync(0xffffffffu, inc - m, warp), c = __shfl_sync(0xffffffffu, m, warp);
-      if (warp < CS) {   // warp w copies rank w's members
-        const uint2* src = cluster.map_shared_rank(own, warp);
-        for (unsigned i = lane; i < c && off + i < (unsigned)SEL_TIES; i += 32) all[off + i] = src[i];
+      rk += __shfl_xor_sync(0xffffffffu, rk, 1);
+      rk += __shfl_xor_sync(0xffffffffu, rk, 2);
+      if (t < n_all && (tid & 3) == 0) {
+        if (rk < rem && t < before_me) atomicAdd(&s.lower_sel, 1u);
+        if (rk + 1 == rem) s.thr_key = me.x, s.thr_pos = me.y;
+      }
+    } else {
+      // the members' place within the threshold bin: ranks have to be counted out only in the sub-bin of the last one taken
+      auto sub_of = [&](unsigned k) -> unsigned { return level0 ? bins.sub(k, T0) : 0u; };
+      for (unsigned t = tid; t < n_all; t += SEL_THREADS) atomicAdd(&s.sub[sub_of(all[t].x)], 1u);
+      __syncthreads();
+      if (warp == 0) {   // lane l: sub-bins 2l, 2l + 1
+        const unsigned c0 = s.sub[2 * lane], c1 = s.sub[2 * lane + 1];
+        unsigned suf = c0 + c1;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const unsigned o = __shfl_down_sync(0xffffffffu, suf, off);
+          if (lane + off < 32) suf += o;
+        }
+        const unsigned above1 = suf - c0 - c1, above0 = above1 + c1;
+        if (above1 < rem && above0 >= rem) s.res[0] = 2 * lane + 1, s.res[1] = above1;
+        else if (above0 < rem && suf >= rem) s.res[0] = 2 * lane, s.res[1] = above0;
       }
       __syncthreads();
-    }
-    // the members' place within the threshold bin: ranks have to be counted out only in the sub-bin of the last one taken
-    auto sub_of = [&](unsigned k) -> unsigned { return level0 ? bins.sub(k, T0) : 0u; };
-    for (unsigned t = tid; t < n_all; t += SEL_THREADS) atomicAdd(&s.sub[sub_of(all[t].x)], 1u);
-    __syncthreads();
-    if (warp == 0) {   // lane l: sub-bins 2l, 2l + 1
-      const unsigned c0 = s.sub[2 * lane], c1 = s.sub[2 * lane + 1];
-      unsigned suf = c0 + c1;
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const unsigned o = __shfl_down_sync(0xffffffffu, suf, off);
-        if (lane + off < 32) suf += o;
-      }
-      const unsigned above1 = suf - c0 - c1, above0 = above1 + c1;
-      if (above1 < rem && above0 >= rem) s.res[0] = 2 * lane + 1, s.res[1] = above1;
-      else if (above0 < rem && suf >= rem) s.res[0] = 2 * lane, s.res[1] = above0;
-    }
-    __syncthreads();
-    const unsigned S = s.res[0], need = rem - s.res[1];
-    uint2* few = all + (CS == 1 ? SEL_TIES : 0);   // the sub-bin's elements; bit 31 of the position: held by a lower rank
-    uint2 mine[SEL_TIES / SEL_THREADS];
-#pragma unroll
-    for (int j = 0; j < SEL_TIES / SEL_THREADS; j++) {
-      const unsigned t = tid + j * SEL_THREADS;
-      mine[j] = t < n_all ? all[t] : make_uint2(0u, 0u);
-    }
-    if (CS > 1) __syncthreads();   // `few` takes the place of `all`
-#pragma unroll
-    for (int j = 0; j < SEL_TIES / SEL_THREADS; j++) {
-      const unsigned t = tid + j * SEL_THREADS;
-      if (t < n_all) {
-        const unsigned ms = sub_of(mine[j].x);
-        if (ms == S) few[atomicAdd(&s.n_few, 1u)] = make_uint2(mine[j].x, mine[j].y | (t < before_me ? 0x80000000u : 0u));
+      const unsigned S = s.res[0], need = rem - s.res[1];
+      uint2* few = all + SEL_TIES;   // the sub-bin's elements; bit 31 of the position: held by a lower rank
+      for (unsigned t = tid; t < n_all; t += SEL_THREADS) {
+        const uint2 m = all[t];
+        const unsigned ms = sub_of(m.x);
+        if (ms == S) few[atomicAdd(&s.n_few, 1u)] = make_uint2(m.x, m.y | (t < before_me ? 0x80000000u : 0u));
         else if (ms > S && t < before_me) atomicAdd(&s.lower_sel, 1u);
       }
-    }
-    __syncthreads();
-    const unsigned n_few = s.n_few;
+      __syncthreads();
+      const unsigned n_few = s.n_few;
 #pragma unroll 1
-    for (unsigned t = warp; t < n_few; t += SEL_WARPS) {   // a warp ranks an element
-      const uint2 me = few[t];
-      const unsigned pos = me.y & 0x7fffffffu;
-      unsigned rk = 0;
-      for (unsigned j = lane; j < n_few; j += 32) {
-        const uint2 o = few[j];
-        rk += (o.x > me.x || (o.x == me.x && (o.y & 0x7fffffffu) < pos)) ? 1u : 0u;
-      }
-      rk = __reduce_add_sync(0xffffffffu, rk);
-      if (lane == 0) {
-        if (rk < need && (me.y >> 31)) atomicAdd(&s.lower_sel, 1u);
-        if (rk + 1 == need) s.thr_key = me.x, s.thr_pos = pos;
+      for (unsigned t = warp; t < n_few; t += SEL_WARPS) {   // a warp ranks an element
+        const uint2 me = few[t];
+        const unsigned pos = me.y & 0x7fffffffu;
+        unsigned rk = 0;
+        for (unsigned j = lane; j < n_few; j += 32) {
+          const uint2 o = few[j];
+          rk += (o.x > me.x || (o.x == me.x && (o.y & 0x7fffffffu) < pos)) ? 1u : 0u;
+        }
+        rk = __reduce_add_sync(0xffffffffu, rk);
+        if (lane == 0) {
+          if (rk < need && (me.y >> 31)) atomicAdd(&s.lower_sel, 1u);
+          if (rk + 1 == need) s.thr_key = me.x, s.thr_pos = pos;
+        }
       }
     }
     __syncthreads();
     thr_key = s.thr_key, thr_pos = s.thr_pos, lower_sel = s.lower_sel;
   }
-  if (CS > 1) cluster.barrier_arrive();   // this CTA reads no other CTA's memory from here on
 
-  // ---- ordered emission: a lane owns a word of 32 elements ----
+  // ---- ordered emission: a warp takes a word of 32 elements at a time, a lane an element ----
   auto taken = [&](unsigned k, unsigned pos) -> bool { return k > thr_key || (k == thr_key && pos <= thr_pos); };
   if (kept && !flat) {   // members that are taken join the elements above
-    const unsigned m = min(s.n_members, (unsigned)SEL_TIES);
+    const unsigned m = min(s.n_members, (unsigned)SEL_TIES - min(pre_in, (unsigned)SEL_TIES));
     for (unsigned t = tid; t < m; t += SEL_THREADS) {
       const uint2 me = own[t];
       const unsigned i = me.y & 0x07ffffffu;
@@ -342,7 +358,10 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     }
   }
   const unsigned room = flat && rem > lower_sel ? rem - lower_sel : 0u;   // flat bin: members this CTA may still take
-  unsigned g = pre_above + lower_sel, e = 0;   // entries of the final list, and members, before the window
+  const unsigned pos0 = pre_above + lower_sel;
+  unsigned g = pos0, e = 0;   // entries of the final list, and members, before the window
+  int* list = reinterpret_cast<int*>(region);   // (the members are done with at the next barrier)
+  constexpr unsigned LIST = LISTED ? SEL_REGION / 4 : 0;
   for (int w0 = 0; w0 < n_words; w0 += words_cap) {
     const int nw = min(n_words - w0, words_cap);
     if (!kept) {
@@ -365,38 +384,47 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     na = __reduce_add_sync(0xffffffffu, na), nm = __reduce_add_sync(0xffffffffu, nm);
     if (lane == 0) s.warp_a[warp] = na, s.warp_b[warp] = nm;
     __syncthreads();
-    unsigned gw = g, ew = e;
-    for (int w = 0; w < SEL_WARPS; w++) {
-      const unsigned x = s.warp_a[w], y = s.warp_b[w];
-      if (w < warp) gw += x, ew += y;
-      g += x, e += y;
+    unsigned gw, ew;
+    {
+      const unsigned x = lane < SEL_WARPS ? s.warp_a[lane] : 0u, y = lane < SEL_WARPS ? s.warp_b[lane] : 0u;
+      gw = g + __reduce_add_sync(0xffffffffu, lane < warp ? x : 0u), ew = e + __reduce_add_sync(0xffffffffu, lane < warp ? y : 0u);
+      g += __reduce_add_sync(0xffffffffu, x), e += __reduce_add_sync(0xffffffffu, y);
     }
     for (int wb = a0; wb < a1; wb += 32) {
       const int w = wb + lane;
-      unsigned aw = w < a1 ? above_w[w] : 0u, mw = w < a1 ? member_w[w] : 0u;
-      const unsigned long long mine = ((unsigned long long)__popc(aw) << 32) | (unsigned)__popc(mw);
-      unsigned long long inc = mine;
+      const unsigned aw = w < a1 ? above_w[w] : 0u, mw = w < a1 ? member_w[w] : 0u;
+      const unsigned mine = ((unsigned)__popc(aw) << 16) | (unsigned)__popc(mw);   // at most 1024 of either in 32 words
+      unsigned inc = mine;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
-        const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, off);
+        const unsigned o = __shfl_up_sync(0xffffffffu, inc, off);
         if (lane >= off) inc += o;
       }
-      const unsigned long long total = __shfl_sync(0xffffffffu, inc, 31);
-      unsigned eb = ew + (unsigned)(inc - mine);
-      unsigned pos = gw + (unsigned)((inc - mine) >> 32) + min(eb, room);
-      if (eb >= room) mw = 0;
-      for (unsigned bits = aw | mw; bits; bits &= bits - 1) {
-        const int j = __ffs(bits) - 1;
-        if ((mw >> j) & 1u) {
-          if (eb >= room) continue;
-          eb++;
+      const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
+      const unsigned e0 = ew + ((inc - mine) & 0xffffu), g0 = gw + ((inc - mine) >> 16);   // before the lane's word
+#pragma unroll 4
+      for (int j = 0; j < min(32, a1 - wb); j++) {
+        const unsigned a = __shfl_sync(0xffffffffu, aw, j), below = (1u << lane) - 1u;
+        unsigned pos = __shfl_sync(0xffffffffu, g0, j) + __popc(a & below);
+        bool take = (a >> lane) & 1u;
+        if (flat) {
+          const unsigned m = __shfl_sync(0xffffffffu, mw, j), e = __shfl_sync(0xffffffffu, e0, j) + __popc(m & below);
+          take = take || (((m >> lane) & 1u) && e < room);
+          pos += min(e, room);
         }
-        if (pos < (unsigned)K) out[pos] = out_of((w0 + w) * 32 + j);
-        pos++;
+        if (take && pos < (unsigned)K) {
+          const int i = (w0 + wb + j) * 32 + lane;
+          if (pos - pos0 < LIST) list[pos - pos0] = i;
+          else out[pos] = out_of(i);
+        }
       }
-      gw += (unsigned)(total >> 32), ew += (unsigned)total;
+      gw += total >> 16, ew += total & 0xffffu;
     }
   }
+  if (!LISTED) return;
+  __syncthreads();
+  const unsigned last = min((unsigned)K, g + min(e, room)), n_list = last > pos0 ? min(last - pos0, LIST) : 0u;
+  for (unsigned t = tid; t < n_list; t += SEL_THREADS) out[pos0 + t] = out_of(list[t]);
 }
 
 }  // namespace

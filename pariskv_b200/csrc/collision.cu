@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
     unsigned* my = s_sizes + warp * 256;
     if (!early) prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     if (warp == 0 && blockIdx.x == 0) publish_query(pq, cq, bh);
-    if (tid == 32) load_tiers(cq, (long long)N, s_tiers);
+    if (tid >= 32 && tid < 41) load_tiers(cq, (long long)N, s_tiers, tid - 32);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
     *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
     for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;

@@ -21,14 +21,11 @@ __host__ __device__ inline int zone_row(const pk_zone_schedule& s, long long N) 
     if (N < s.bound[i]) row = i;
   return row;
 }
-__host__ __device__ inline void zone_tiers(const pk_zone_schedule& s, long long N, unsigned* tiers) {
-  const double base = (double)N * s.collision_ratio[zone_row(s, N)];
-  for (int t = 0; t < s.n_tiers; t++) {
-    double x = ceil(base * s.tier_ratio[t]);
-    if (!(x > 0.0)) x = 0.0;
-    if (x > 4294967295.0) x = 4294967295.0;
-    tiers[t] = (unsigned)x;
-  }
+__host__ __device__ inline unsigned zone_tier(const pk_zone_schedule& s, long long N, int t) {
+  double x = ceil((double)N * s.collision_ratio[zone_row(s, N)] * s.tier_ratio[t]);
+  if (!(x > 0.0)) x = 0.0;
+  if (x > 4294967295.0) x = 4294967295.0;
+  return (unsigned)x;
 }
 __host__ __device__ inline long long zone_candidates(const pk_zone_schedule& s, long long N) {
   const double x = ceil((double)N * s.candidate_ratio[zone_row(s, N)]);
@@ -52,7 +49,7 @@ struct ChainQuery {
   unsigned tiers[8];          // thresholds when n_dev == null
   int n_tiers;
   const int32_t* n_dev;       // [bs] searchable keys per sample (device), or null: all N keys of the view
-  pk_zone_schedule sched;     // thresholds = zone_tiers(sched, n_dev[b]) when n_dev is set
+  pk_zone_schedule sched;     // thresholds = zone_tier(sched, n_dev[b], t) when n_dev is set
   int early_query;            // the queries were complete before the previous kernel on the stream started
   int early_loads;            // see pdl_early()
 };

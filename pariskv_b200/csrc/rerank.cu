@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
   const uint16_t* w = a.w + b * a.w_b + h * a.w_h;
   float* scores = p.scores_f32 + row_base + out_pos;
   if (FAST) {
-    rerank_list(n_list, ids, pp.list_cap, a, k4, w, stage, lev2, s_qb, qn, pp.c128, key_at, [&](int i, int, float v) { scores[i] = v; });
+    rerank_list(n_list, ids, pp.list_cap, a, k4, w, stage, lev2, s_qb, qn, pp.c128, key_at, [&](int i, int, float v) { scores[i] = v; }, []() {});
   } else {
     for (int i = tid; i < n_list; i += CH_THREADS)
       scores[i] = rerank_one<false>(*reinterpret_cast<RerankSmem*>(dyn), a, k4, w, key_at(i), qn, lane, nullptr, 0);

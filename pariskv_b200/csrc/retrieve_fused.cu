@@ -10,9 +10,8 @@
 //
 // Why this split: as two launches (count | select + rerank + final top-K by the last block of a head) the final stage ran
 // on one SM per head, 12 us of 48 at 128K keys, and counts and scores went through L2.  Time line of a CTA on B200
-// (8 heads x 131004 keys, 10 CTAs each): query and ranking 6 us, counting 13 K keys 7.4, threshold and list 2.8, rerank
-// of 1310 candidates 8.2, final selection 8.6: 33 us (39 with 8 CTAs, all 256 clusters sorted, and one load waiting for
-// the other in the prologue).  Graph-replayed layer step, two launches -> one: 16 sequences of 16 - 32K keys
+// (8 heads x 131004 keys, 10 CTAs each; the query prepared before the wait): tables 3.1 us, counting 13 K keys 6.4, threshold
+// and list 4.0, rerank of 1310 candidates 6.1, final selection 7.2: 27 us.  Graph-replayed layer step, two launches -> one: 16 sequences of 16 - 32K keys
 // (one CTA per head, no exchange at all) 155 -> 116 us, 8 heads x 128K keys 70 -> 60, 10K keys 27 -> 19 for the chain.
 // What bounds it: the serial chain of exchanges for small zones, instruction issue (look-ups 85 instructions per key and
 // warp, rerank 420 per candidate and warp) for long ones; codes and records stream at under half of the HBM rate.
@@ -63,8 +62,9 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   __shared__ __align__(16) uint4 s_qb[16];        // the same, its bf16 values as such
   __shared__ __align__(16) uint8_t s_lut[16 * 128];
   unsigned* region = reinterpret_cast<unsigned*>(dyn);
-  uint32_t* lev2 = reinterpret_cast<uint32_t*>(dyn + CH_HIST_BYTES);
-  uint8_t* cnt8 = dyn + CH_HIST_BYTES + LEV2_BYTES;
+  unsigned* inbox = reinterpret_cast<unsigned*>(dyn + CH_HIST_BYTES);
+  uint32_t* lev2 = reinterpret_cast<uint32_t*>(dyn + CH_HIST_BYTES + sel_inbox_bytes(CS));
+  uint8_t* cnt8 = dyn + CH_HIST_BYTES + sel_inbox_bytes(CS) + LEV2_BYTES;
   uint8_t* stage = cnt8 + (threadIdx.x >> 5) * CH_STAGE_WARP;   // the counts are done with when records are staged
   int* ids = reinterpret_cast<int*>(cnt8 + max(p.span_cap, CH_STAGE));
   float* sc = reinterpret_cast<float*>(ids + p.list_cap);
@@ -78,6 +78,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   unsigned key[4];
   for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
   if (cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
+  if (CS > 1) cluster.barrier_arrive();   // a CTA has to run before the others may write into it
   const bool early = cq.early_query != 0;
   if (early) {   // the queries were complete before the kernel before this one started
     load_query(ql, cq, b, h, p.G);
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
     if (!early) prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
     if (!cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
     if (warp == 0 && rank == 0) publish_query(pq, cq, bh);
-    if (tid == 32) load_tiers(cq, (long long)N, s_tiers);
+    if (tid >= 32 && tid < 41) load_tiers(cq, (long long)N, s_tiers, tid - 32);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
     *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
     __syncthreads();
@@ -145,13 +146,16 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
     count_round(r0, v0);
     if (v0 - lane + STEP < n_keys) count_round(r1, v0 + STEP);
   }
+  if (CS > 1) cluster.barrier_wait();
   __syncthreads();
-  for (int bin = warp; bin < CH_CBINS; bin += CH_WARPS) {
+  for (int bin = warp; bin < CH_CBINS; bin += CH_WARPS) {   // bin totals, in the place of the first replicas
     const unsigned t = __reduce_add_sync(0xffffffffu, region[bin * 32 + lane]);
-    if (lane == 0) s.hist[0][bin] = t;
+    if (lane == 0) region[bin * 32] = t;
   }
+  __syncthreads();
+  if (tid < CH_CBINS) put_everywhere<CS>(cluster, inbox + rank * SEL_BINS + tid, region[tid * 32]);
   sync_cluster<CS>(cluster);
-  cluster_threshold<CS, CH_CBINS>(cluster, s, s.hist[0], rank, (unsigned)C_want);
+  cluster_threshold<CS, CH_CBINS>(s, inbox, rank, (unsigned)C_want);
   const unsigned T = s.res[0], quota = (unsigned)C_want - s.res[1];
   const unsigned gt_base = s.res[3], eq_base = s.res[4];
   const int64_t C_here = min(C_want, p.C);
@@ -169,6 +173,15 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   auto id_at = [&](int i) -> int { return i < p.list_cap ? ids[i] : (int)p.ws_cand[row_base + out_pos + i]; };
   auto score_at = [&](int i) -> float { return i < p.list_cap ? sc[i] : p.ws_scores[row_base + out_pos + i]; };
   unsigned kmin = 0xffffffffu, kmax = 0u;
+  // The bins of the final selection lie between the extremes of the scores of every warp's first round, so that their exchange
+  // passes under the other rounds.
+  bool published = p.K <= 0;
+  auto publish = [&]() {
+    if (published) return;
+    published = true;
+    publish_range<CS>(cluster, inbox, rank, kmin, kmax);
+    if (CS > 1) cluster.barrier_arrive();
+  };
   {
     const uint8_t* k4 = p.a.k4 + b * p.a.k4_b + h * p.a.k4_h;
     const uint16_t* w = p.a.w + b * p.a.w_b + h * p.a.w_h;
@@ -180,7 +193,8 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
       if (p.cand_out) p.cand_out[at] = k;
       const unsigned u = ord_key(v);
       kmin = min(kmin, u), kmax = max(kmax, u);
-    });
+    }, publish);
+    publish();   // warps without candidates
     if (p.fill_tail && p.scores_out && p.cand_out)
       for (int64_t i = C_here + (int64_t)rank * CH_THREADS + tid; i < p.C; i += CS * CH_THREADS) {
         p.scores_out[row_base + i] = -INFINITY;
@@ -192,17 +206,13 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
     if (p.n_cand_out) p.n_cand_out[bh] = (int32_t)C_here;
     if (p.n_sel_out && p.K > 0) p.n_sel_out[bh] = K_here;
   }
-  if (p.K <= 0) {
-    sync_cluster<CS>(cluster);   // shared memory must outlive the remote reads of the count histograms
-    return;
-  }
+  if (p.K <= 0) return;
 
   // ---- final top-K over the cluster ----
   __syncthreads();   // the scores are complete; the level table and the histogram region are free
-  cluster_select<CS, F32Row>(
-      cluster, s, region, lev2, FR_WORDS, rank, n_list, K_here, p.final_out + bh * p.K,
-      [&](int i) -> uint32_t { return __float_as_uint(score_at(i)); }, [&](int i) -> int64_t { return id_at(i); }, kmin, kmax);
-  if (CS > 1) cluster.barrier_wait();   // shared memory must outlive the other CTAs' reads
+  cluster_select<CS, F32Row, false>(
+      cluster, s, region, inbox, lev2, FR_WORDS, rank, n_list, K_here, p.final_out + bh * p.K,
+      [&](int i) -> uint32_t { return __float_as_uint(score_at(i)); }, [&](int i) -> int64_t { return id_at(i); }, kmin, kmax, true);
 }
 
 // Clusters that fit the device at once, per size in CLUSTER_SIZES (0: the size cannot be launched).
@@ -213,7 +223,7 @@ struct Capacity {
 template <int CS>
 int active_clusters() {
   auto kern = retrieve_fused_kernel<CS>;
-  const int smem = CH_HIST_BYTES + LEV2_BYTES + (FR_SPAN_MAX > CH_STAGE ? FR_SPAN_MAX : CH_STAGE) + 8 * FR_LIST_MAX;
+  const int smem = CH_HIST_BYTES + sel_inbox_bytes(CS) + LEV2_BYTES + (FR_SPAN_MAX > CH_STAGE ? FR_SPAN_MAX : CH_STAGE) + 8 * FR_LIST_MAX;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return cudaGetLastError(), 0;
   if (CS > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
     return cudaGetLastError(), 0;
@@ -304,7 +314,7 @@ int launch_fused_retrieve(int cs, const pk_tensor* codebook, const RerankArgs& a
   int64_t list = (2 * sa.C / cs + 512 + 31) / 32 * 32;
   if (list > p.span_cap + 32) list = (p.span_cap + 63) / 32 * 32;
   p.list_cap = (int)(list < FR_LIST_MAX ? list : FR_LIST_MAX);
-  const size_t smem = (size_t)CH_HIST_BYTES + LEV2_BYTES + (p.span_cap > CH_STAGE ? p.span_cap : CH_STAGE) + 8 * (size_t)p.list_cap;
+  const size_t smem = (size_t)CH_HIST_BYTES + sel_inbox_bytes(cs) + LEV2_BYTES + (p.span_cap > CH_STAGE ? p.span_cap : CH_STAGE) + 8 * (size_t)p.list_cap;
   const dim3 grid((unsigned)cs, (unsigned)(bs * H));
   StageTimer tm(ST_RETRIEVE, st);
   cudaError_t e = cudaErrorInvalidValue;

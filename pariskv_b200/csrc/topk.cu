@@ -4,7 +4,8 @@
 // What bounds it: the latency of the selection's exchanges for rows of up to some 10 K elements, three to five passes over
 // a CTA's slice (shared memory where it fits) beyond.  On B200, us per launch before (a cluster kernel with five
 // bisected levels and per-thread spans; one CTA per row up to 16384 elements) -> now: 8 rows of 32768 counts, k 4096
-// 16.7 -> 10.0; 8 rows of 4096 scores, k 256 9.6 -> 8.7.
+// 16.7 -> 10.0; 8 rows of 4096 scores, k 256 9.6 -> 8.7.  The operators' nine launches, two of them these: 68.1 -> 65.2 us with
+// the exchanges by remote stores.
 #include "cluster_select.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
@@ -14,7 +15,7 @@ namespace {
 
 constexpr int TK_WORDS = 1024;              // ballots kept per kind: slices of up to 32 K elements
 constexpr int TK_CACHE = 32 * TK_WORDS;     // elements of a slice kept in shared memory; longer ones are read again from L2
-constexpr int TK_FIXED = SEL_REGION + 2 * TK_WORDS * 4;
+__host__ __device__ constexpr int tk_fixed(int cs) { return SEL_REGION + 2 * TK_WORDS * 4 + sel_inbox_bytes(cs); }
 
 struct TopkParams {
   const uint32_t* in;
@@ -34,16 +35,21 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
   __shared__ SelShared s;
   unsigned* region = reinterpret_cast<unsigned*>(dyn);
   unsigned* words = region + SEL_REGION / 4;
-  uint32_t* cache = words + 2 * TK_WORDS;
+  unsigned* inbox = words + 2 * TK_WORDS;
+  uint32_t* cache = inbox + sel_inbox_bytes(CS) / 4;
   const int tid = threadIdx.x;
   const unsigned rank = CS == 1 ? 0u : cluster.block_rank();
   const int64_t row = blockIdx.y;
+  if (CS > 1) cluster.barrier_arrive();   // a CTA has to run before the others may write into it
   pdl_wait();
   pdl_trigger();
   const int64_t L = p.n_dev ? min((int64_t)max(p.n_dev[row], 0), p.L) : p.L;
   const int K = (int)min(p.k, L);
   if (p.n_out && rank == 0 && tid == 0) p.n_out[row] = K;
-  if (K <= 0) return;        // the same for all CTAs of the row
+  if (K <= 0) {   // the same for all CTAs of the row
+    if (CS > 1) cluster.barrier_wait();
+    return;
+  }
   const int64_t slice = ((L + CS - 1) / CS + 31) / 32 * 32, begin = min(L, (int64_t)rank * slice);
   const int n = (int)(min(L, begin + slice) - begin);
   const uint32_t* in = p.in + row * p.row_stride + begin;
@@ -63,21 +69,21 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
       }
     }
   }
+  if (CS > 1) cluster.barrier_wait();
   const int64_t* map = p.map ? p.map + row * p.map_stride + begin : nullptr;
   auto out_of = [&](int i) -> int64_t { return map ? map[i] : begin + i; };
   if (cached)
-    cluster_select<CS, Row>(cluster, s, region, words, TK_WORDS, rank, n, K, p.out + row * p.k,
+    cluster_select<CS, Row, true>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
                             [&](int i) -> uint32_t { return cache[i]; }, out_of, kmin, kmax);
   else
-    cluster_select<CS, Row>(cluster, s, region, words, TK_WORDS, rank, n, K, p.out + row * p.k,
+    cluster_select<CS, Row, true>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
                             [&](int i) -> uint32_t { return in[i]; }, out_of, kmin, kmax);
-  if (CS > 1) cluster.barrier_wait();   // shared memory must outlive the other CTAs' reads
 }
 
 template <int CS, class Row>
 int topk_active() {   // clusters that fit the device at once; also opts in to the shared memory
   auto kern = topk_kernel<CS, Row>;
-  const int smem = TK_FIXED + TK_CACHE * 4;
+  const int smem = tk_fixed(CS) + TK_CACHE * 4;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return cudaGetLastError(), 0;
   if (CS > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
     return cudaGetLastError(), 0;
@@ -145,7 +151,7 @@ int launch_rows(TopkParams p, int64_t rows, cudaStream_t st) {
   const int64_t slice = ((p.L + best - 1) / best + 31) / 32 * 32;
   if (slice >= (1LL << 27)) return fail(PK_ERR_ARG, "topk: row too long");
   p.cache = slice <= TK_CACHE ? (int)slice : 0;
-  const size_t smem = TK_FIXED + (size_t)p.cache * 4;
+  const size_t smem = tk_fixed(best) + (size_t)p.cache * 4;
   for (int64_t r0 = 0; r0 < rows; r0 += 65535) {   // grid.y limit
     TopkParams q = p;
     const int64_t nr = rows - r0 < 65535 ? rows - r0 : 65535;

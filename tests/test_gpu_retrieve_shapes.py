@@ -82,6 +82,36 @@ def test_rerank_of_any_record_layout(oracle, bs, H, N, C, layout):
     assert torch.equal(fin.cpu(), ref["final"])
 
 
+# The bins of the final selection lie between the extremes of every warp's first 32 candidates: with norms that rise along the
+# zone all that is selected lies beyond them, with falling ones nothing; one block per head and clusters
+@pytest.mark.parametrize("bs,H,N,K", [(20, 8, 1500, 300), (1, 8, 6000, 700), (1, 1, 9000, 1), (1, 2, 9000, 8999)])
+@pytest.mark.parametrize("step", [3.0, -3.0])
+def test_final_selection_beyond_the_first_rounds(oracle, bs, H, N, K, step):
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(N + K)
+    norm = torch.exp(torch.linspace(-step / 2, step / 2, N)).view(1, 1, N, 1)
+    keys = (synth_keys(g, bs, H, N).float() * norm).to(torch.bfloat16)
+    q = synth_queries(g, keys, 4)
+    signs = srht_signs()
+    _, cen = oracle.constants()
+    counts = torch.zeros(bs, H, 16, 256, dtype=torch.int32, device=DEV)
+    cb, w, pk = ops.encode_keys(keys.to(DEV), signs.to(DEV), cluster_counts=counts)
+    ref = oracle.retrieve(q, signs, cb.cpu(), w.cpu(), pk.cpu(), counts.cpu(), cen, 0.25, N, K)
+    fin, _ = ops.retrieve(q.to(DEV), signs.to(DEV), cen.to(DEV), cb, w, pk, counts, oracle.tier_counts(N, 0.25), N, K)
+    assert torch.equal(fin.cpu(), ref["final"])
+
+
+# more entries per block than it lists in shared memory (4096), and just as many
+@pytest.mark.parametrize("rows,L,K", [(1, 300000, 290000), (3, 100000, 65536), (200, 9000, 4097), (200, 9000, 4096)])
+def test_final_topk_of_long_lists(oracle, rows, L, K):
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(L + K)
+    scores = torch.randn(1, rows, L, generator=g)
+    cand = torch.randint(0, 1 << 40, (1, rows, L), generator=g)
+    at = torch.sort(torch.sort(scores, dim=-1, descending=True, stable=True).indices[..., :K], dim=-1).values
+    assert torch.equal(ops.final_topk(scores.to(DEV), cand.to(DEV), K).cpu(), torch.gather(cand, 2, at))
+
+
 @pytest.mark.parametrize("group", [5, 8, 9])
 @pytest.mark.parametrize("n_window,K", [(1, 0), (63, 1), (64, 64), (70, 1000)])
 def test_attention_group_sizes(oracle, group, n_window, K):
