@@ -2,14 +2,19 @@
 //
 // Per (batch, KV head) the attended rows are the selected rows of the big K/V store, which may live in pinned host
 // memory, followed by the first n_window rows of the GPU window ([sink | local | update buffer]): with the selected
-// rows first, their indices can be loaded before the row counts are known.  The rows are cut into tiles of 64; a block takes one tile, or several consecutive
-// ones that it streams through two staging buffers, and stages a tile with TMA bulk copies (cp.async.bulk, one
+// rows first, their indices can be loaded before the row counts are known.  The rows are cut into tiles of 64 or 128; a block
+// takes one tile, or several consecutive ones that it streams through its staging buffers, and stages a tile with TMA bulk copies (cp.async.bulk, one
 // 512-byte copy per selected key where its K and V rows are adjacent, completion counted on an mbarrier), so a whole
 // grid keeps megabytes outstanding on the host link.  An online softmax over the staged rows runs on the tensor
 // cores for up to eight query heads per KV head (on 16 groups of 8 lanes, four heads at a time, for more), and the block
-// writes one partial (m, l, o) record per head.
-// The block that finishes last for a (batch, KV head) merges the partials and writes the output: one launch, no
-// second kernel, no waiting on other blocks.  Scores are kept in the log2 domain.
+// has one partial (m, l, o) per head.
+// Where the blocks of a (batch, KV head) fit a thread-block cluster they merge their partials through distributed shared
+// memory, otherwise the block that finishes last merges them from records in the workspace and writes the output: one launch,
+// no second kernel, no waiting on blocks that may not be resident.  Scores are kept in the log2 domain.
+#include <cooperative_groups.h>
+
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -21,6 +26,9 @@ constexpr int ATT_GQ = 4;       // query heads per pass of the scalar form, and 
 // Query heads per KV head that the tensor-core form takes in its one pass: the rows 0 .. 7 of its A operand.  Batch 8 of one
 // KV head with eight query heads, 2180 rows each: 45 us a launch with the scalar form (two passes), 20 with this one.
 constexpr int ATT_MQ = 8;
+constexpr int ATT_HEAD_TILES = 5;  // tiles of 128 rows that a block of the cluster form takes at most (see head_tiles)
+constexpr int ATT_HEAD_BUFS = 3;   // tiles of 128 rows that a block of the cluster form has in flight: 198 KB
+constexpr int ATT_CLUSTER_MAX = 16;
 constexpr int ATT_CHAINS = 4;   // accumulators of a score's k-steps; eight spill in the streaming form and cost 1 % there
 constexpr int ATT_REC = 132;    // floats per partial: o[128], m, l, pad, pad
 constexpr int ATT_WAIT_LIMIT = 4000000;  // polls of the copy barrier before giving up
@@ -130,17 +138,29 @@ __device__ __forceinline__ void mbar_arrive_expect(unsigned mb, unsigned bytes) 
 // SM at most; there only latency counts: the same number of records, but one tile instead of two in a row, and twice the
 // warps to merge them.  8 heads of 2180 rows in HBM: 9.8 -> 9.3 us alone and 61 -> 58 us for the layer step in a graph;
 // batch 8 of one KV head with eight query heads 60 -> 53 us for the step.
-template <bool MMA, int WARPS>
+//
+// CLUSTER: the blocks of a head are a thread-block cluster.  Each has up to three of its tiles of 128 rows in flight, and the
+// blocks' partials meet through distributed shared memory: every block merges a share of the outputs.  What this saves is the
+// way over L2, 4.4 us from the last product to the end (partial record, fence, atomic, records back into one SM, all in a row;
+// 7.3 with eight query heads); 1.6 like this.  B200, a step: one KV head of eight sequences with eight query heads each, four
+// layers, 186.2 -> 176.8 us; 128K keys, four layers 203.2 -> 194.4; 10K keys in host memory, four layers 155.2 -> 144.3.
+template <bool MMA, int WARPS, bool CLUSTER>
 __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attention_kernel(AttParams p) {
-  constexpr int THREADS = 32 * WARPS, TILE = 16 * WARPS, NBUF = WARPS > 4 ? 1 : 2;   // one buffer: one tile per block
+  static_assert(!CLUSTER || (MMA && WARPS == 8), "the cluster form");
+  constexpr int THREADS = 32 * WARPS, TILE = 16 * WARPS;
+  constexpr int NBUF = CLUSTER ? ATT_HEAD_BUFS : WARPS > 4 ? 1 : 2;   // one buffer: one tile per block
   constexpr int RS = AttRow<MMA>::stride;  // elements per staged row
   extern __shared__ __align__(128) unsigned char dyn[];
   uint16_t* KVs = reinterpret_cast<uint16_t*>(dyn);                          // [2 buffers][64][RS]: K row, V row of a key
   constexpr int PQ = MMA ? ATT_MQ : ATT_GQ;   // query heads of a pass
   constexpr int PG = MMA ? WARPS : 16;   // groups of a block that hold partials of them
-  float* obuf = reinterpret_cast<float*>(dyn + (NBUF - 1) * 2 * TILE * RS);  // [PG][PQ][128], over the LAST buffer:
-                                                                             // used when that buffer is idle
-  __shared__ __align__(8) unsigned long long mbar[2];
+  // Floats between the partials of two heads: with 8 more than 128 the float2 stores of a half warp (four heads, four lanes of
+  // each) fall into all 32 banks, without them into eight.
+  constexpr int OS = MMA ? 136 : 128;
+  // [PG][PQ][OS], over the LAST buffer (CLUSTER: the first): used when that buffer is idle
+  float* obuf = reinterpret_cast<float*>(dyn + (CLUSTER ? 0 : NBUF - 1) * 2 * TILE * RS);
+  static_assert(PG * PQ * OS * 4 <= 2 * TILE * RS && WARPS * ATT_GQ * 128 * 4 <= 2 * TILE * RS, "partials fit a buffer");
+  __shared__ __align__(8) unsigned long long mbar[NBUF > 2 ? NBUF : 2];
   __shared__ float s_m[PG][PQ], s_l[PG][PQ];
   __shared__ unsigned char s_valid[NBUF][TILE];
   __shared__ int s_last;
@@ -151,8 +171,9 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
   const int t_first = (int)blockIdx.x * tpb;
   const unsigned mb0 = (unsigned)__cvta_generic_to_shared(&mbar[0]);
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0), "r"(THREADS) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0 + 8), "r"(THREADS) : "memory");
+#pragma unroll
+    for (int i = 0; i < (NBUF > 2 ? NBUF : 2); i++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb0 + 8 * i), "r"(THREADS) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -163,7 +184,10 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
   };
   pdl_wait();  // the selected indices and the per-head row counts come from the kernels before this one
   pdl_trigger();
-  int64_t ahead = index_of(t_first);
+  int64_t ahead = index_of(t_first), later[ATT_HEAD_BUFS - 1];
+  if (CLUSTER)
+#pragma unroll
+    for (int i = 0; i < ATT_HEAD_BUFS - 1; i++) later[i] = i + 1 < tpb ? index_of(t_first + i + 1) : 0;
   const int64_t n_sel = p.n_sel ? min((int64_t)p.n_sel[bh], p.K) : p.K;
   const int64_t n_window =
       p.n_window_dev ? min(p.n_window, max((int64_t)0, (int64_t)p.n_window_dev[0] + p.n_window_add)) : p.n_window;
@@ -213,9 +237,15 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
       }
       mbar_arrive(mb);
     }
-    ahead = index_of(t + 1);
+    if (!CLUSTER) ahead = index_of(t + 1);
   };
   issue(t_first, 0);
+  if (CLUSTER) {
+#pragma unroll
+    for (int i = 0; i < ATT_HEAD_BUFS - 1; i++)
+      if (i + 1 < tpb) ahead = later[i], issue(t_first + i + 1, i + 1);
+    if (ATT_HEAD_BUFS < tpb) ahead = index_of(t_first + ATT_HEAD_BUFS);
+  }
 
   bool dead = false;  // a copy barrier never completed: reported, the remaining tiles count as empty
   // Called by every thread once per tile j of the block: starts the copies of tile j + 1 (its buffer was released by
@@ -225,6 +255,14 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
   // its (batch, KV head), the merge runs and the counter returns to zero.  The host must treat a raised status word
   // as fatal.
   auto acquire = [&](int j) -> int {
+    if (CLUSTER) {
+      if (!dead && !__syncthreads_and(mbar_wait(mb0 + 8 * (j % ATT_HEAD_BUFS), (unsigned)(j / ATT_HEAD_BUFS & 1), ATT_WAIT_LIMIT))) {
+        if (tid == 0) atomicExch(p.status, 1);
+        for (int i = j; i < min(tpb, j + ATT_HEAD_BUFS); i++) mbar_wait(mb0 + 8 * (i % ATT_HEAD_BUFS), (unsigned)(i / ATT_HEAD_BUFS & 1), ATT_WAIT_LIMIT);
+        dead = true;
+      }
+      return dead ? 0 : tile_rows(t_first + j);
+    }
     const int buf = j & 1;
     if (NBUF > 1 && j + 1 < tpb && !dead) issue(t_first + j + 1, buf ^ 1);
     if (!dead && !__syncthreads_and(mbar_wait(mb0 + 8 * buf, (unsigned)((j >> 1) & 1), ATT_WAIT_LIMIT))) {
@@ -246,9 +284,9 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
       float L = 0.0f, O = 0.0f;
 #pragma unroll 4
       for (int t = 0; t < PG; t++) {
-        const float f = (s_m[t][g] == -INFINITY) ? 0.0f : exp2f(s_m[t][g] - M);
+        const float f = (s_m[t][g] == -INFINITY) ? 0.0f : exp2_neg(s_m[t][g] - M);
         L += s_l[t][g] * f;
-        O += obuf[(t * PQ + g) * 128 + dim] * f;
+        O += obuf[(t * PQ + g) * OS + dim] * f;
       }
       float* rec = p.ws + (((int64_t)b * p.Hq + h * p.G + qg * PQ + g) * n_groups + blockIdx.x) * ATT_REC;
       __stcg(rec + dim, O);
@@ -278,7 +316,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
     float m_run = -INFINITY, l_run = 0.0f;  // head g; l is this lane's share, summed over the four lanes at the end
     const int r0 = warp * 16;               // this warp's rows of every tile
     for (int j = 0; j < tpb; j++) {
-      const int buf = j & 1;
+      const int buf = CLUSTER ? j % ATT_HEAD_BUFS : j & 1;
       const int n_live = acquire(j);
       const uint16_t* tile = KVs + buf * (TILE * RS);
       if (r0 < n_live) {  // warp-uniform
@@ -357,6 +395,10 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
         }
       }
       __syncthreads();  // the tile has been consumed: its buffer may be refilled (after the last tile obuf is free)
+      if (CLUSTER && j + ATT_HEAD_BUFS < tpb && !dead) {
+        issue(t_first + j + ATT_HEAD_BUFS, buf);
+        ahead = index_of(t_first + j + ATT_HEAD_BUFS + 1);
+      }
     }
     // the four warps are the groups of the block-level merge
     l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
@@ -366,8 +408,76 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
     if (head_ok) {
 #pragma unroll
       for (int n = 0; n < 16; n++)
-        *reinterpret_cast<float2*>(obuf + (warp * PQ + g) * 128 + 8 * n + 2 * t) = make_float2(join(oacc[n][0], oacc[n][2]), join(oacc[n][1], oacc[n][3]));
+        *reinterpret_cast<float2*>(obuf + (warp * PQ + g) * OS + 8 * n + 2 * t) = make_float2(join(oacc[n][0], oacc[n][2]), join(oacc[n][1], oacc[n][3]));
       if (t == 0) s_m[warp][g] = m_run, s_l[warp][g] = l_run;
+    }
+    if constexpr (CLUSTER) {
+      // Unit u: dims 4 (u & 31) .. + 3 of head u >> 5.  The warps' partials become the block's, a thread per unit; behind the
+      // cluster barrier every block takes consecutive units, eight lanes a unit, each of them every eighth block's partial.
+      cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+      __shared__ __align__(16) float4 s_o[ATT_MQ * 32];
+      __shared__ float2 s_ml[ATT_MQ];
+      const int units = p.G * 32;
+      __syncthreads();
+      if (tid < units) {
+        const int hd = tid >> 5;
+        float M = -INFINITY, L = 0.0f;
+        float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) M = fmaxf(M, s_m[w][hd]);
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) {
+          const float f = s_m[w][hd] == -INFINITY ? 0.0f : exp2_neg(s_m[w][hd] - M);
+          const float4 v = reinterpret_cast<const float4*>(obuf + (w * PQ + hd) * OS)[lane];
+          L += s_l[w][hd] * f, o.x += v.x * f, o.y += v.y * f, o.z += v.z * f, o.w += v.w * f;
+        }
+        s_o[tid] = o;
+        if (lane == 0) s_ml[hd] = make_float2(M, L);
+      }
+      cluster.sync();
+      constexpr int MB = ATT_CLUSTER_MAX / 8;
+      const int per = (units + n_groups - 1) / n_groups, sub = lane & 7;
+      const int u1 = min(units, ((int)blockIdx.x + 1) * per);
+      for (int u0 = blockIdx.x * per; u0 < u1; u0 += THREADS / 8) {
+        const int u = u0 + (tid >> 3), hd = u < u1 ? u >> 5 : 0;
+        float2 ml[MB];
+        float4 v[MB];
+#pragma unroll
+        for (int i = 0; i < MB; i++) {
+          ml[i] = make_float2(-INFINITY, 0.0f), v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (u < u1 && sub + 8 * i < n_groups)
+            ml[i] = *cluster.map_shared_rank(&s_ml[hd], sub + 8 * i), v[i] = *cluster.map_shared_rank(&s_o[u], sub + 8 * i);
+        }
+        float m = -INFINITY, l = 0.0f;
+        float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < MB; i++) m = fmaxf(m, ml[i].x);
+#pragma unroll
+        for (int i = 0; i < MB; i++) {
+          const float f = ml[i].x == -INFINITY ? 0.0f : exp2_neg(ml[i].x - m);
+          l += ml[i].y * f, o.x += v[i].x * f, o.y += v[i].y * f, o.z += v[i].z * f, o.w += v[i].w * f;
+        }
+        float M = m;
+#pragma unroll
+        for (int off = 1; off < 8; off <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+        const float f = m == -INFINITY ? 0.0f : exp2_neg(m - M);
+        l *= f, o.x *= f, o.y *= f, o.z *= f, o.w *= f;
+#pragma unroll
+        for (int off = 1; off < 8; off <<= 1) {
+          l += __shfl_xor_sync(0xffffffffu, l, off);
+          o.x += __shfl_xor_sync(0xffffffffu, o.x, off), o.y += __shfl_xor_sync(0xffffffffu, o.y, off);
+          o.z += __shfl_xor_sync(0xffffffffu, o.z, off), o.w += __shfl_xor_sync(0xffffffffu, o.w, off);
+        }
+        if (u < u1 && sub == 0) {
+          const int64_t bq = (int64_t)b * p.Hq + h * p.G + hd;
+          const bool any = l > 0.0f;
+          *reinterpret_cast<uint2*>(p.out + bq * 128 + 4 * (u & 31)) =
+              any ? make_uint2(pack_bf16(o.x / l, o.y / l), pack_bf16(o.z / l, o.w / l)) : make_uint2(0u, 0u);
+          if (p.lse && (u & 31) == 0) p.lse[bq] = any ? M + log2f(l) : -INFINITY;
+        }
+      }
+      cluster.sync();   // shared memory must outlive the other blocks' reads
+      return;
     }
     __syncthreads();
     block_partial(0, p.G);
@@ -441,7 +551,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
 #pragma unroll
       for (int g = 0; g < ATT_GQ; g++) {
 #pragma unroll
-        for (int jj = 0; jj < 16; jj++) obuf[(grp * PQ + g) * 128 + 16 * s + jj] = o[g][jj];
+        for (int jj = 0; jj < 16; jj++) obuf[(grp * PQ + g) * OS + 16 * s + jj] = o[g][jj];
         if (s == 0) {
           s_m[grp][g] = m[g];
           s_l[grp][g] = lsum[g];
@@ -457,37 +567,37 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
   __syncthreads();
   if (tid == 0) {   // one thread's fences order the whole block's records (the barriers carry them to and from it)
     __threadfence();
-    const unsigned prev = atomicAdd(p.counters + bh, 1u);
-    s_last = prev + 1 == (unsigned)n_groups;
-    if (s_last) p.counters[bh] = 0;  // ready for the next call on this stream
+    s_last = atomicAdd(p.counters + bh, 1u) + 1u == (unsigned)n_groups;
     __threadfence();
   }
   __syncthreads();
   if (!s_last) return;
-  // Up to ATT_GQ query heads are merged at a time.  The warps take the records in turn, a lane four dims of each; the
-  // records of MB steps are in flight together, (m, l) with the values, because nothing in this tail but their
-  // latency costs time: 36 records of four heads took 6.6 us with a pass for the scale factors and 16 single floats in
-  // flight per thread, 4.4 like this with four warps.  The warps' sums meet in shared memory.
-  constexpr int MB = WARPS > 4 || !MMA ? 3 : 5;
+  if (tid == 0) p.counters[bh] = 0;  // ready for the next call on this stream (behind the fence: nobody waits for it)
+  // ATT_GQ query heads are merged by all warps, up to twice as many by half of the warps each.  The warps take the records in
+  // turn, a lane four dims of each; the records of MB steps are in flight together, (m, l) with the values, because nothing in
+  // this tail but their latency costs time: 36 records of four heads took 6.6 us with a pass for the scale factors and 16
+  // single floats in flight per thread, 4.4 like this with four warps.  The warps' sums meet in shared memory.
   const int warp = tid >> 5, lane = tid & 31;
-  for (int qg = 0; qg < p.n_qgroups; qg++) {
-    const int n_heads = min(ATT_GQ, p.G - qg * ATT_GQ);
-    const int64_t bq0 = (int64_t)b * p.Hq + h * p.G + qg * ATT_GQ;
+  auto merge = [&](auto n_parts, int q0) {
+    constexpr int parts = decltype(n_parts)::value, nw = WARPS / parts, MB = MMA && nw <= 4 ? 5 : 3;
+    const int n_heads = min(parts * ATT_GQ, p.G - q0);
+    const int first = warp / nw * ATT_GQ, mine = min(ATT_GQ, n_heads - first);   // this warp's heads
+    const int64_t bq0 = (int64_t)b * p.Hq + h * p.G + q0;
     float m[ATT_GQ], l[ATT_GQ];
     float4 o[ATT_GQ];
 #pragma unroll
     for (int g = 0; g < ATT_GQ; g++) m[g] = -INFINITY, l[g] = 0.0f, o[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int t0 = warp; t0 < n_groups; t0 += WARPS * MB) {
+    for (int t0 = warp % nw; t0 < n_groups; t0 += nw * MB) {
       float4 v[MB][ATT_GQ];
       float2 ml[MB][ATT_GQ];
 #pragma unroll
       for (int i = 0; i < MB; i++)
 #pragma unroll
         for (int g = 0; g < ATT_GQ; g++) {
-          const int t = t0 + WARPS * i;
+          const int t = t0 + nw * i;
           ml[i][g] = make_float2(-INFINITY, 0.0f), v[i][g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (t < n_groups && g < n_heads) {
-            const float* rec = p.ws + ((bq0 + g) * n_groups + t) * ATT_REC;
+          if (t < n_groups && g < mine) {
+            const float* rec = p.ws + ((bq0 + first + g) * n_groups + t) * ATT_REC;
             ml[i][g] = __ldcg(reinterpret_cast<const float2*>(rec + 128));
             v[i][g] = __ldcg(reinterpret_cast<const float4*>(rec) + lane);
           }
@@ -498,17 +608,17 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
 #pragma unroll
         for (int i = 0; i < MB; i++) mn = fmaxf(mn, ml[i][g].x);
         if (mn == -INFINITY) continue;   // no live row so far
-        const float c = exp2f(m[g] - mn);
+        const float c = exp2_neg(m[g] - mn);
         m[g] = mn, l[g] *= c, o[g].x *= c, o[g].y *= c, o[g].z *= c, o[g].w *= c;
 #pragma unroll
         for (int i = 0; i < MB; i++) {
-          const float f = exp2f(ml[i][g].x - mn);
+          const float f = exp2_neg(ml[i][g].x - mn);
           l[g] += ml[i][g].y * f;
           o[g].x += v[i][g].x * f, o[g].y += v[i][g].y * f, o[g].z += v[i][g].z * f, o[g].w += v[i][g].w * f;
         }
       }
     }
-    if (qg) __syncthreads();            // the sums of the previous heads have been consumed
+    if (q0) __syncthreads();            // the sums of the previous heads have been consumed
 #pragma unroll
     for (int g = 0; g < ATT_GQ; g++) {
       if (lane == 0) s_m[warp][g] = m[g], s_l[warp][g] = l[g];
@@ -516,18 +626,23 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
     }
     __syncthreads();
     for (int g = tid >> 7; g < n_heads; g += THREADS / 128) {
+      const int w0 = g / ATT_GQ * nw, gg = g % ATT_GQ;   // the warps that merged this head
       float M = -INFINITY, L = 0.0f, O = 0.0f;
 #pragma unroll
-      for (int w = 0; w < WARPS; w++) M = fmaxf(M, s_m[w][g]);
+      for (int w = 0; w < nw; w++) M = fmaxf(M, s_m[w0 + w][gg]);
 #pragma unroll
-      for (int w = 0; w < WARPS; w++) {
-        const float f = s_m[w][g] == -INFINITY ? 0.0f : exp2f(s_m[w][g] - M);
-        L += s_l[w][g] * f;
-        O += obuf[(w * ATT_GQ + g) * 128 + (tid & 127)] * f;
+      for (int w = 0; w < nw; w++) {
+        const float f = s_m[w0 + w][gg] == -INFINITY ? 0.0f : exp2_neg(s_m[w0 + w][gg] - M);
+        L += s_l[w0 + w][gg] * f;
+        O += obuf[((w0 + w) * ATT_GQ + gg) * 128 + (tid & 127)] * f;
       }
       p.out[(bq0 + g) * 128 + (tid & 127)] = f2bf(L > 0.0f ? O / L : 0.0f);
       if (p.lse && (tid & 127) == 0) p.lse[bq0 + g] = L > 0.0f ? M + log2f(L) : -INFINITY;
     }
+  };
+  for (int q0 = 0; q0 < p.G;) {
+    if (p.G - q0 > ATT_GQ) merge(std::integral_constant<int, 2>(), q0), q0 += 2 * ATT_GQ;
+    else merge(std::integral_constant<int, 1>(), q0), q0 += ATT_GQ;
   }
 }
 
@@ -536,12 +651,71 @@ int launch_attention(const AttParams& p, dim3 grid, cudaStream_t st) {
   const int smem = (WARPS > 4 ? 1 : 2) * 16 * WARPS * AttRow<MMA>::stride * 2;
   static PerDevice smem_attr;   // the opt-in to more than 48 KB of dynamic shared memory is per kernel and device
   if (const unsigned long long bit = first_on_device(smem_attr)) {
-    if (cudaFuncSetAttribute(sparse_attention_kernel<MMA, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (cudaFuncSetAttribute(sparse_attention_kernel<MMA, WARPS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
       return check_launch("sparse_attention smem");
     mark_on_device(smem_attr, bit);
   }
   StageTimer tm(ST_ATTENTION, st);
-  launch_chain(sparse_attention_kernel<MMA, WARPS>, grid, dim3(32 * WARPS), (size_t)smem, st, p);
+  launch_chain(sparse_attention_kernel<MMA, WARPS, false>, grid, dim3(32 * WARPS), (size_t)smem, st, p);
+  return check_launch("sparse_attention");
+}
+
+// ---- the cluster form ----
+int head_smem(int tiles) { return (tiles < ATT_HEAD_BUFS ? tiles : ATT_HEAD_BUFS) * 128 * AttRow<true>::stride * 2; }
+cudaLaunchConfig_t head_config(cudaLaunchAttribute* attr, dim3 grid, int tiles, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid, cfg.blockDim = dim3(256), cfg.dynamicSmemBytes = (size_t)head_smem(tiles), cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = grid.x, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr, cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cfg;
+}
+// Clusters of a size, with a number of tiles per block, that fit the device at once; asked once per device.
+struct HeadCapacity {
+  int active[ATT_HEAD_BUFS + 1][ATT_CLUSTER_MAX + 1];
+};
+const HeadCapacity* head_capacity() {
+  static HeadCapacity cap[64];
+  static PerDevice asked;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  if (const unsigned long long bit = first_on_device(asked)) {
+    auto kern = sparse_attention_kernel<true, 8, true>;
+    const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, head_smem(ATT_HEAD_BUFS)) == cudaSuccess &&
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    for (int tiles = 1; tiles <= ATT_HEAD_BUFS; tiles++)   // several threads may ask at the same time: they write the same numbers
+      for (int cs = 1; cs <= ATT_CLUSTER_MAX; cs++) {
+        cudaLaunchAttribute attr[2];
+        cudaLaunchConfig_t cfg = head_config(attr, dim3(cs, 64), tiles, nullptr);
+        cfg.numAttrs = 1;
+        int n = 0;
+        cap[dev].active[tiles][cs] = ok && cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess ? n : 0;
+      }
+    cudaGetLastError();
+    mark_on_device(asked, bit);
+  }
+  return &cap[dev];
+}
+// Tiles of 128 rows per block of the cluster form, or 0 where it does not apply: as few as make a cluster that is resident for
+// every head at once, at most ATT_HEAD_TILES.  On B200, us per launch of four query heads per KV head, the other forms -> this
+// one, at one to six tiles: 8 heads of 700 rows 7.4 -> 5.0; of 2244 rows 8 heads 7.7 -> 6.6, 16 heads 11.7 -> 8.6, 24 heads
+// 12.7 -> 11.1, 32 heads 14.3 -> 13.5, 40 heads 15.9 -> 16.2.  Beyond, three blocks of four warps per SM stream faster than one of eight.
+int head_tiles(int64_t n_halves, int64_t heads) {
+  const HeadCapacity* cap = head_capacity();
+  for (int64_t cs = n_halves < ATT_CLUSTER_MAX ? n_halves : ATT_CLUSTER_MAX; cap && cs >= 1; cs--) {
+    const int64_t tiles = (n_halves + cs - 1) / cs;
+    if (tiles > ATT_HEAD_TILES) break;
+    if (heads <= cap->active[tiles < ATT_HEAD_BUFS ? tiles : ATT_HEAD_BUFS][(n_halves + tiles - 1) / tiles]) return (int)tiles;
+  }
+  return 0;
+}
+int launch_head_attention(const AttParams& p, dim3 grid, cudaStream_t st) {
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = head_config(attr, grid, p.tiles_per_block, st);
+  StageTimer tm(ST_ATTENTION, st);
+  if (cudaLaunchKernelEx(&cfg, sparse_attention_kernel<true, 8, true>, p) != cudaSuccess) return check_launch("sparse_attention cluster", 0);
   return check_launch("sparse_attention");
 }
 
@@ -649,14 +823,19 @@ extern "C" int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* wi
   p.n_qgroups = (p.G + ATT_GQ - 1) / ATT_GQ;
   // Blocks per (batch, KV head): one per 128 rows when the whole launch is then a block per SM at most (every copy of the
   // launch outstanding at once), otherwise one per two tiles of 64 rows - a block copies two at once - but no more than
-  // ONE wave of three blocks per SM, each streaming several tiles.  The scalar form needs the staged tile for several
+  // ONE wave of three blocks per SM, each streaming several tiles.  Before either the cluster form is tried (see head_tiles).
+  // The scalar form needs the staged tile for several
   // passes: one tile per block then.
   const bool mma = p.G <= ATT_MQ;   // at most ATT_MQ query heads per KV head: one pass on the tensor cores
   const int64_t halves = (n_tiles + 1) / 2;
   const bool wide = mma && halves * H * bs <= sm_count();
   int64_t groups = n_tiles;
   p.tiles_per_block = 1;
-  if (wide) {
+  const int in_cluster = mma && (reinterpret_cast<uintptr_t>(out->data) & 7) == 0 ? head_tiles(halves, H * bs) : 0;   // (it stores four outputs at once)
+  if (in_cluster) {
+    p.tiles_per_block = in_cluster;
+    groups = (halves + in_cluster - 1) / in_cluster;
+  } else if (wide) {
     groups = halves;
   } else if (mma) {
     const int64_t fit = (int64_t)sm_count() * 3 / (H * bs);
@@ -677,6 +856,7 @@ extern "C" int pk_sparse_attention(const pk_tensor* queries, const pk_tensor* wi
   }
   cudaStream_t st = (cudaStream_t)stream;
   const dim3 grid((unsigned)groups, (unsigned)H, (unsigned)bs);
+  if (in_cluster) return launch_head_attention(p, grid, st);
   if (wide) return launch_attention<true, 8>(p, grid, st);
   return mma ? launch_attention<true, 4>(p, grid, st) : launch_attention<false, 4>(p, grid, st);
 }

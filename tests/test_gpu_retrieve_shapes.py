@@ -1,5 +1,7 @@
 """The retrieval chain over the shapes its launch rule tells apart (clusters of 1 .. 16 blocks per head, and the launches
 over all SMs beyond), and attention at the group sizes where its form changes."""
+import math
+
 import pytest
 import torch
 
@@ -132,6 +134,40 @@ def test_attention_group_sizes(oracle, group, n_window, K):
     out = ops.sparse_attention(q.to(DEV), wk.to(DEV), wv.to(DEV), n_window, *args)
     ref = oracle.attention(q, torch.cat(rk, 2), torch.cat(rv, 2))
     assert (out.float().cpu() - ref).abs().max().item() <= 2e-2
+
+
+# (heads, window, selected rows): clusters of 16 blocks with a tile each, of 9 with two, of 13 with three, of 6 with three; a
+# head over more blocks than a cluster has; last tiles of a row, and heads without any
+@pytest.mark.parametrize("H,n_window,K", [(1, 1, 2047), (8, 196, 2048), (4, 1, 4900), (16, 100, 2048), (2, 100, 6100), (8, 5, 2044), (3, 0, 900)])
+@pytest.mark.parametrize("group,offset", [(4, 0), (8, 0), (5, 2)])
+def test_attention_in_a_cluster(oracle, H, n_window, K, group, offset):
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(K + group)
+    kv = torch.randn(1, H, K + 50, 2, 128, generator=g).to(torch.bfloat16)
+    q = (torch.randn(1, 1, H * group, 128, generator=g) * 3).to(torch.bfloat16)
+    wk, wv = (torch.randn(1, H, max(n_window, 1), 128, generator=g).to(torch.bfloat16) for _ in range(2))
+    sel = torch.stack([torch.randperm(K + 50, generator=g)[:K] for _ in range(H)])[None]
+    n_sel = torch.randint(0, K + 1, (1, H), generator=g, dtype=torch.int32)
+    n_sel[0, 0], n_sel[0, -1] = K, 0 if H > 1 else K
+    dkv = kv.to(DEV)
+    buf = torch.zeros(H * group * 128 + offset, dtype=torch.bfloat16, device=DEV)   # an output that is not 8-byte aligned
+    out = buf[offset:].view(1, 1, H * group, 128)
+    lse = torch.empty(1, H * group, dtype=torch.float32, device=DEV)
+    ops.sparse_attention(q.to(DEV), wk.to(DEV) if n_window else None, wv.to(DEV) if n_window else None, n_window, dkv[:, :, :, 0], dkv[:, :, :, 1],
+                         sel.to(DEV), n_sel=n_sel.to(DEV), out=out, lse=lse)
+    for h in range(H):
+        n = int(n_sel[0, h])
+        k = torch.cat([kv[:, h:h + 1, sel[0, h, :n], 0], wk[:, h:h + 1, :n_window]], 2)
+        v = torch.cat([kv[:, h:h + 1, sel[0, h, :n], 1], wv[:, h:h + 1, :n_window]], 2)
+        mine = slice(h * group, (h + 1) * group)
+        if k.shape[2] == 0:
+            assert (out[:, :, mine] == 0).all() and (lse[:, mine] == -float("inf")).all()
+            continue
+        ref = oracle.attention(q[:, :, mine].contiguous(), k.contiguous(), v.contiguous())
+        assert (out[:, :, mine].float().cpu() - ref).abs().max().item() <= 2e-2
+        logits = torch.einsum("gd,nd->gn", q[0, 0, mine].double(), k[0, 0].double()) / 128 ** 0.5
+        want = torch.logsumexp(logits, 1) / math.log(2.0)
+        assert (lse[0, mine].double().cpu() - want).abs().max().item() <= 1e-4   # 32-bit sums of some thousand terms
 
 
 @pytest.mark.parametrize("bs,H,n_window,K", [(1, 1, 127, 0), (1, 1, 128, 1), (1, 2, 1, 127), (2, 37, 100, 156), (2, 37, 100, 157)])
