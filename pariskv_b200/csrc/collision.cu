@@ -258,13 +258,14 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
   if (cq.n_dev || !cq.early_loads) pdl_wait();  // the zone length may have been written by the kernel just before this one
   const int64_t N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
   const int64_t Nv = N + p.mis;
-  const int64_t v_begin = (int64_t)blockIdx.x * p.chunk_keys;
+  const int64_t chunk_keys = cq.n_dev ? chain_chunk(Nv, p.n_hist, p.chunk_keys) : p.chunk_keys;
+  const int64_t v_begin = (int64_t)blockIdx.x * chunk_keys;
   if (v_begin >= Nv) {  // beyond this sample's zone (whole block, before any barrier but the early one)
     pdl_wait();
     pdl_trigger();
     return;
   }
-  const int n_keys = (int)(min(Nv, v_begin + p.chunk_keys) - v_begin);   // virtual keys of this block
+  const int n_keys = (int)(min(Nv, v_begin + chunk_keys) - v_begin);   // virtual keys of this block
   const uint8_t* base = p.codes + b * p.c_b + h * p.c_h + (v_begin - p.mis) * p.c_l;
   uint8_t* out8 = p.out_u8 + (int64_t)bh * p.u8_stride + v_begin;
   // the first code loads are issued before the tables are built
@@ -415,13 +416,13 @@ int64_t collision_chunk_keys(int64_t bs_h, int64_t Nv) {
 }
 
 // Launch geometry of the several-launch chain: about one block per SM over the whole grid, one histogram row each; both
-// the collision and the selection kernel take chunk_keys virtual keys per block, a multiple of 512.  At least 2048, because
-// every block of the selection kernel reads all rows of its head; at most what that kernel holds in shared memory.
+// the collision and the selection kernel take chunk_keys virtual keys per block, a multiple of 512 (fewer where the zone's
+// length on the device asks for less, see chain_chunk); at most what the selection kernel holds in shared memory.
 void chain_geometry(int64_t bs_h, int64_t Nv, int64_t* chunk_keys, int64_t* n_hist) {
   int64_t target = (int64_t)sm_count() / (bs_h > 0 ? bs_h : 1);
   if (target < 1) target = 1;
   int64_t chunk = ((Nv + target - 1) / target + 511) / 512 * 512;
-  if (chunk < 2048) chunk = 2048;
+  if (chunk < CHAIN_CHUNK_MIN) chunk = CHAIN_CHUNK_MIN;
   if (chunk > CHAIN_CHUNK_MAX) chunk = CHAIN_CHUNK_MAX;
   *chunk_keys = chunk;
   *n_hist = (Nv + chunk - 1) / chunk;

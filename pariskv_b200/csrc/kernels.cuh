@@ -57,6 +57,14 @@ int launch_collision(const pk_tensor* codebook, const uint32_t* lut, int32_t* ou
 int chain_layout(const pk_tensor* codebook, int* layout);
 constexpr int64_t CHAIN_CHUNK_MAX = 64 * 1024;   // keys per block of the several-launch chain
 void chain_geometry(int64_t bs_h, int64_t Nv, int64_t* chunk_keys, int64_t* n_hist);
+constexpr int64_t CHAIN_CHUNK_MIN = 2048;        // every block of the selection reads the histogram rows of its whole head
+// Keys per block for a zone of Nv keys: the launch has blocks for the capacity of the zone; where the length comes from the
+// device, what the zone holds is spread over all of them.
+__host__ __device__ inline int64_t chain_chunk(int64_t Nv, int64_t n_blocks, int64_t at_most) {
+  const int64_t even = ((Nv + n_blocks - 1) / n_blocks + 511) / 512 * 512;
+  const int64_t c = even < CHAIN_CHUNK_MIN ? CHAIN_CHUNK_MIN : even;
+  return c < at_most ? c : at_most;
+}
 int launch_chain_collision(const pk_tensor* codebook, const ChainQuery& cq, uint8_t* counts_u8, int64_t u8_stride,
                            uint32_t* chunk_hist, int* mis_out, int64_t* chunk_keys_out, int64_t* n_hist_out,
                            cudaStream_t st);
@@ -112,7 +120,7 @@ struct SelectArgs {
 int launch_select_rerank(const RerankArgs& a, int64_t bs_h, const SelectArgs& s, cudaStream_t st);
 
 // retrieve_fused.cu: the whole chain in one launch, one cluster of `cs` CTAs per (batch, head)
-int fused_cluster_size(const pk_tensor* codebook, const RerankArgs& a, int64_t bs_h, int64_t N, int64_t C);
+int fused_cluster_size(const pk_tensor* codebook, const RerankArgs& a, int64_t bs_h, int64_t N, int64_t C, int64_t K);
 // cand_out / scores_out: [bs*H][C] or null; ws_cand / ws_scores: the same arrays in the workspace
 int launch_fused_retrieve(int cs, const pk_tensor* codebook, const RerankArgs& a, const ChainQuery& cq, const SelectArgs& sa,
                           int64_t* cand_out, float* scores_out, int64_t* ws_cand, float* ws_scores, cudaStream_t st);

@@ -75,10 +75,11 @@ __global__ void __launch_bounds__(CH_THREADS, 1) select_rerank_kernel(RerankArgs
   if (FAST && !p.early_loads) build_lev2(lev2, a.centers, tid, CH_THREADS);
   const int64_t N = p.n_dev ? min(max((int64_t)p.n_dev[b], (int64_t)1), p.N) : p.N;
   const int64_t Nv = N + p.mis;
-  const int64_t v_begin = chunk * p.chunk_keys;
+  const int64_t chunk_keys = p.n_dev ? chain_chunk(Nv, p.n_chunks, p.chunk_keys) : p.chunk_keys;   // as the collision kernel has it
+  const int64_t v_begin = chunk * chunk_keys;
   if (v_begin >= Nv) return;  // beyond this sample's zone (whole block, before any barrier)
-  const int n_keys = (int)(min(Nv, v_begin + p.chunk_keys) - v_begin);
-  const int64_t live_chunks = (Nv + p.chunk_keys - 1) / p.chunk_keys;
+  const int n_keys = (int)(min(Nv, v_begin + chunk_keys) - v_begin);
+  const int64_t live_chunks = (Nv + chunk_keys - 1) / chunk_keys;
   // candidates wanted over the whole zone (all shards together)
   const int64_t C_want = p.n_dev ? min((int64_t)zone_candidates(p.sched, N), p.C) : p.C_want;
   // this block's counts, straight into shared memory, under the latency of the histogram rows

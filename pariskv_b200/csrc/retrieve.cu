@@ -174,9 +174,8 @@ int retrieve_impl(const pk_retrieve_args& a, cudaStream_t st) {
     cq.early_loads = pdl_early();
     cq.early_query = a.queries_settled != 0 && cq.early_loads;
     // The form and its grid follow the capacity of the view, not the keys it holds: a captured launch serves every length.
-    // The price lies with caches that are nearly empty: two layers of 8 heads in a graph on B200, 10K / 50K / 200K keys in a
-    // cache for 1M 172 / 245 / 283 us a step, in one of their own size 88 / 98 / 137.
-    const int cs = sharded ? 0 : fused_cluster_size(codebook, ra, bh, N, C);
+    // The keys that are there are spread over all blocks of either form.
+    const int cs = sharded ? 0 : fused_cluster_size(codebook, ra, bh, N, C, K);
     if (cs) {
       ra.q_blocks = nullptr, ra.q_norm = nullptr, ra.centers = (const uint16_t*)a.mag_centers->data, ra.C = row;
       cq.q_blocks = a.q_blocks ? qb : nullptr, cq.q_norm = a.q_norm ? qn : nullptr;

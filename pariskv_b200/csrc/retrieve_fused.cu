@@ -277,26 +277,37 @@ cudaError_t launch_cs(dim3 grid, size_t smem, cudaStream_t st, const FusedParams
 
 }  // namespace
 
-// CTAs per (batch, head), or 0 where the fused kernel does not apply: the codebook must be key-major, and a CTA's slice
-// of the zone at most FR_SPAN_MAX keys.
-// The size minimises waves x (fixed + share of the work): measured on B200, about 15 us of a CTA's time do not shrink with
-// its slice (query, ranking, exchanges), a key costs 0.5 ns and a candidate 3 - 6 ns of one SM (look-ups, rerank).
-int fused_cluster_size(const pk_tensor* codebook, const RerankArgs& a, int64_t bs_h, int64_t N, int64_t C) {
+// CTAs per (batch, head), or 0 where the fused kernel does not apply (the codebook must be key-major, and a CTA's slice of the
+// zone at most FR_SPAN_MAX keys) or the several-launch form is faster.
+// Both forms are a fixed time and a share of the work; fitted on B200 to 1 .. 128 heads of 8 .. 400 K keys with 5 and 10 % of
+// candidates.  This one: waves x (16 us + 0.66 ns a key and 3.9 a candidate of a CTA's slice); without the final top-K 11 us,
+// 0.59 and 2.8.  The other: 22 us + 0.74 ns a key and 1.6 a candidate of an SM's share + 2.8 a candidate of a CTA's slice in the
+// top-k launch; without it 13 us.  It uses all SMs, so it wins where a cluster would leave most of them idle (one head) or the
+// heads are more than one wave.  us measured, this form | the other: 8 heads of 131K keys 30.0 | 31.4, of 200K 36.6 | 36.3, of
+// 400K 57.0 | 52.0; one head of 131K 25.7 | 26.4, of 400K 43.9 | 31.5; 16 heads of 262K 85.6 | 58.7; 128 heads of 33K 44.0 | 57.9;
+// without top-K 8 heads of 66K 15.8 | 16.0, of 131K 20.6 | 18.9, one head of 400K 29.8 | 18.2.  The other form has to win by 8 us
+// of a full zone: its further launches cost a program that calls eagerly, and is bound by its host, up to 5 (one layer of two heads,
+// adaptive budget, 91K keys 77.3 us a step with this form, 81.5 with the other), and a zone that is nearly empty 4 on the device.
+int fused_cluster_size(const pk_tensor* codebook, const RerankArgs& a, int64_t bs_h, int64_t N, int64_t C, int64_t K) {
   int layout = 0;
   chain_layout(codebook, &layout);
   if (layout != 1 || !rerank_fast_layout(a) || N >= (1ll << 30) || bs_h > 65535) return 0;
   const Capacity* cap = capacity();
   if (!cap) return 0;
-  int best = 0;
+  int best = 0, whole = 1;   // whole: the largest cluster that is resident for every head at once
   double best_us = 0.0;
+  const double fixed = K > 0 ? 16.0 : 11.0, work = (K > 0 ? 0.00066 : 0.00059) * (double)N + (K > 0 ? 0.0039 : 0.0028) * (double)C;
   for (int i = 0; i < N_CLUSTER_SIZES; i++) {
     const int cs = CLUSTER_SIZES[i];
+    if (bs_h <= cap->active[i]) whole = cs;
     if (cap->active[i] <= 0 || span_of(N, cs) > FR_SPAN_MAX) continue;
     const double waves = (double)((bs_h + cap->active[i] - 1) / cap->active[i]);
-    const double us = waves * (15.0 + (0.0005 * (double)N + 0.0045 * (double)C) / cs);
+    const double us = waves * (fixed + work / cs);
     if (!best || us < 0.98 * best_us) best = cs, best_us = us;
   }
-  return best;
+  const double spread = (0.00074 * (double)N + 0.0016 * (double)C) * (double)bs_h / sm_count();
+  const double other = K > 0 ? 22.0 + spread + 0.0028 * (double)C / whole : 13.0 + spread;
+  return !best || other + 8.0 < best_us ? 0 : best;
 }
 
 int launch_fused_retrieve(int cs, const pk_tensor* codebook, const RerankArgs& a, const ChainQuery& cq, const SelectArgs& sa,

@@ -87,6 +87,30 @@ def test_varlen_batch_equals_single_sequences_and_oracle(ops, oracle, schedule, 
         assert torch.equal(fin[b, :, :Kb].cpu(), ref["final"][0])
 
 
+@pytest.mark.parametrize("H,K", [(1, 256), (3, 0)])
+def test_short_zones_in_a_long_cache(ops, schedule, H, K):
+    """The several-launch form has blocks for the capacity and spreads what the zone holds over them: any length gives what a
+    view of just that length gives, which for the shorter ones is the one-launch form."""
+    import ctypes
+    from pariskv_b200 import _lib
+    g = torch.Generator().manual_seed(H)
+    cap = 700001
+    keys = torch.randn(1, H, cap, 128, generator=torch.Generator(DEV).manual_seed(H), device=DEV).to(torch.bfloat16)
+    q = synth_queries(g, keys[:, :, :1000].cpu(), 4).to(DEV)
+    signs, cen = srht_signs().to(DEV), torch.tensor([0.0420, 0.1266, 0.2130, 0.3025, 0.3973, 0.5001, 0.6169, 0.7633], dtype=torch.bfloat16, device=DEV)
+    cb, w, pk = ops.encode_keys(keys, signs)
+    Cmax = int(_lib.load().pk_zone_max_candidates(ctypes.byref(schedule), cap))
+    for n in (1, 15, 511, 2047, 2048, 2049, 30001, 140000, 303104, 303105, cap):
+        counts = ops.count_clusters(cb[..., :n])
+        fin, n_sel, ex = ops.retrieve_ex(q, signs, cen, cb, w, pk, counts, Cmax, K, kv_len=torch.tensor([n], dtype=torch.int32, device=DEV),
+                                         schedule=schedule, want=("cand", "scores_f32"))
+        tiers, C, _ = plan(n)
+        one, ex1 = ops.retrieve(q, signs, cen, cb[..., :n], w[..., :n], pk[..., :n, :], counts, tiers, C, min(K, C), want=("cand", "scores_f32"))
+        assert int(ex["n_cand"][0, 0]) == C
+        assert torch.equal(ex["cand"][:, :, :C], ex1["cand"]) and torch.equal(ex["scores_f32"][:, :, :C], ex1["scores_f32"])
+        assert K == 0 or torch.equal(fin[:, :, :min(K, C)], one)
+
+
 @pytest.mark.parametrize("N,K,world", [(40000, 512, 4), (9001, 256, 3), (131004, 2048, 8), (400000, 2048, 2),
                                        (300000, 1024, 3)])   # the last two: shard rows beyond the in-block final stage
 def test_sharded_phases_reproduce_single_gpu_selection(ops, oracle, N, K, world):
