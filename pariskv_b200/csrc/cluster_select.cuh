@@ -288,7 +288,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       const unsigned t = tid >> 2;
       const uint2 me = t < n_all ? all[t] : make_uint2(0u, 0u);
       unsigned rk = 0;
-#pragma unroll 4
+#pragma unroll 2
       for (unsigned j = tid & 3; j < n_all; j += 4) {
         const uint2 o = all[j];
         rk += (o.x > me.x || (o.x == me.x && o.y < me.y)) ? 1u : 0u;
@@ -402,7 +402,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       }
       const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
       const unsigned e0 = ew + ((inc - mine) & 0xffffu), g0 = gw + ((inc - mine) >> 16);   // before the lane's word
-#pragma unroll 4
+#pragma unroll 1
       for (int j = 0; j < min(32, a1 - wb); j++) {
         const unsigned a = __shfl_sync(0xffffffffu, aw, j), below = (1u << lane) - 1u;
         unsigned pos = __shfl_sync(0xffffffffu, g0, j) + __popc(a & below);

@@ -80,28 +80,21 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   if (cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
   if (CS > 1) cluster.barrier_arrive();   // a CTA has to run before the others may write into it
   const bool early = cq.early_query != 0;
-  if (early) {   // the queries were complete before the kernel before this one started
-    load_query(ql, cq, b, h, p.G);
-    prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
-    __syncthreads();
-    rank_subspace(key, s_q + warp * 8, lane);
+  // Both orders (queries before the wait or behind it) run through one copy of the preparation and the ranking: a CTA fetches its
+  // code as it goes, and with two copies of them and longer unrolls in the selection a step with 128K keys took 195.8 us against
+  // 191.9, one KV head of eight sequences 170.7 against 167.4.
+  if (!early) {
+    pdl_wait();
+    pdl_trigger();
   }
-  pdl_wait();
-  pdl_trigger();
-  // a word written by the kernel before this one takes over a microsecond to arrive: the queries, the cluster sizes and
-  // the zone length are asked for together
-  if (!early) load_query(ql, cq, b, h, p.G);
-  const int4* sizes = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
-  const int4 c0 = sizes[0], c1 = sizes[1];   // of this warp's subspace
-  const int64_t N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
-  const int64_t C_want = cq.n_dev ? min((int64_t)zone_candidates(cq.sched, N), p.C) : p.C_want;
-  const int span = (int)(((N + CS - 1) / CS + 15) / 16 * 16);
-  const int64_t begin = (int64_t)rank * span;
-  const int n_keys = (int)max((int64_t)0, min((int64_t)span, N - begin));
-  const uint8_t* codes = p.codes + b * p.c_b + h * p.c_h + begin * 16;
-
-  // ---- code loads: a warp takes 128 consecutive keys (four per lane) every CH_WARPS * 128; two rounds are in flight,
-  // the first ones during the prologue ----
+  load_query(ql, cq, b, h, p.G);
+  // A word written by the kernel before this one takes over a microsecond to arrive: the cluster sizes, the zone length and
+  // (where they may not be read earlier) the queries are asked for together.  Then the code loads: a warp takes 128
+  // consecutive keys (four per lane) every CH_WARPS * 128; two rounds are in flight, the first ones during the prologue.
+  int4 c0, c1;
+  int64_t N, begin;
+  int n_keys;
+  const uint8_t* codes;
   uint4 r0[4], r1[4];
   constexpr int STEP = CH_WARPS * 128;
   auto load_codes = [&](uint4 (&r)[4], int v0) {
@@ -110,18 +103,35 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
       for (int j = 0; j < 4; j++)   // past the end: the last key again, its count unused
         r[j] = reinterpret_cast<const uint4*>(codes)[min(v0 + 32 * j, n_keys - 1)];
   };
-  load_codes(r0, warp * 128 + lane);
-  load_codes(r1, warp * 128 + lane + STEP);
+  auto load_zone = [&]() {
+    const int4* sizes = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
+    c0 = sizes[0], c1 = sizes[1];   // of this warp's subspace
+    N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
+    const int span = (int)(((N + CS - 1) / CS + 15) / 16 * 16);
+    begin = (int64_t)rank * span;
+    n_keys = (int)max((int64_t)0, min((int64_t)span, N - begin));
+    codes = p.codes + b * p.c_b + h * p.c_h + begin * 16;
+    load_codes(r0, warp * 128 + lane);
+    load_codes(r1, warp * 128 + lane + STEP);
+  };
+  if (!early) load_zone();
+  prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
+  if (!cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
+  __syncthreads();
+  rank_subspace(key, s_q + warp * 8, lane);
+  if (early) {   // the queries were complete before the kernel before this one started
+    pdl_wait();
+    pdl_trigger();
+    load_zone();
+  }
+  const int64_t C_want = cq.n_dev ? min((int64_t)zone_candidates(cq.sched, N), p.C) : p.C_want;
   {
     unsigned* my = reinterpret_cast<unsigned*>(cnt8) + warp * 256;   // the counts are not there yet
-    if (!early) prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
-    if (!cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
     if (warp == 0 && rank == 0) publish_query(pq, cq, bh);
     if (tid >= 32 && tid < 41) load_tiers(cq, (long long)N, s_tiers, tid - 32);
     *reinterpret_cast<int4*>(my + lane * 8) = c0;
     *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
     __syncthreads();
-    if (!early) rank_subspace(key, s_q + warp * 8, lane);
     tier_table(key, my, s_tiers, s_lut + warp * 128);
     if (tid < 128) reinterpret_cast<uint16_t*>(s_qb)[tid] = f2bf(s_q[tid]);
     __syncthreads();   // the tables are complete, the sizes are done with
