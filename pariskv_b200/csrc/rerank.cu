@@ -43,11 +43,10 @@ __global__ void __launch_bounds__(RR_THREADS) rerank_kernel(RerankArgs a, uint16
 // One block per (chunk of keys, batch*head), one block per SM.  The histogram rows written by the collision kernel
 // give every block the global threshold count, the tie quota and its own output offset, so the candidate
 // list comes out in ascending key order with no atomics and no second pass.
-// What bounds it at 8 heads x 1M keys: HBM in units of 128 bytes.  A candidate's two records (64 and 32 bytes) cost 226 of
-// traffic, 203 MB for 840 K candidates, 4.1 TB/s over the launch and more without its first 10 us (histogram rows, counts,
-// list); issue slots are 49 % busy.  With
-// the final top-K by the last block of a head inside it (one SM per head), 8 heads x 1M keys took 129 us on B200; 50
-// here plus 19 for the final top-K as a cluster launch.
+// What bounds it at 8 heads x 1M keys, 33 us on B200: 4 for the threshold, 7 for the list (issue: some 190 instructions per 512
+// counts and warp), 20 for the rerank, 840 K candidates of which HBM reads 128 bytes each: 5.4 TB/s.  (50 us with codes and
+// weights in two arrays, 226 bytes a candidate, and the rerank through registers.)  With the final top-K by the last block of a
+// head inside it (one SM per head) 8 heads x 1M keys took 129 us where this and the top-k launch now take 52.
 struct SelParams {
   SelectArgs s;
   int list_cap;            // candidates whose keys fit in shared memory; the others are read back from cand_out

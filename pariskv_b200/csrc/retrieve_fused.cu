@@ -11,10 +11,11 @@
 // Why this split: as two launches (count | select + rerank + final top-K by the last block of a head) the final stage ran
 // on one SM per head, 12 us of 48 at 128K keys, and counts and scores went through L2.  Time line of a CTA on B200
 // (8 heads x 131004 keys, 10 CTAs each; the query prepared before the wait): tables 3.1 us, counting 13 K keys 6.4, threshold
-// and list 4.0, rerank of 1310 candidates 6.1, final selection 7.2: 27 us.  Graph-replayed layer step, two launches -> one: 16 sequences of 16 - 32K keys
-// (one CTA per head, no exchange at all) 155 -> 116 us, 8 heads x 128K keys 70 -> 60, 10K keys 27 -> 19 for the chain.
-// What bounds it: the serial chain of exchanges for small zones, instruction issue (look-ups 85 instructions per key and
-// warp, rerank 420 per candidate and warp) for long ones; codes and records stream at under half of the HBM rate.
+// and list 4.0, rerank of 1310 candidates 6.1, final selection 7.2: 27 us.  Graph-replayed layer step, two launches -> one: 16
+// sequences of 16 - 32K keys (one CTA per head, no exchange at all) 155 -> 116 us, 8 heads x 128K keys 70 -> 60, 10K keys 27 -> 19
+// for the chain.
+// What bounds it: the serial chain of exchanges for small zones; for long ones instruction issue in the counting (85
+// instructions per 32 keys, 28 cycles of an SM) and, with every SM at it, HBM in the rerank (16 sequences: 80 MB in 15 us).
 #include "chain.cuh"
 #include "cluster_select.cuh"
 #include "common.cuh"
