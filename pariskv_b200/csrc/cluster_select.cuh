@@ -234,7 +234,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     exchange_hist();
     cluster_threshold<CS, SEL_BINS>(s, hists, rank, rem);
     lo = base + (s.res[0] << shift);
-    hi = min(lo + ((1u << shift) - 1u), top);
+    hi = lo + min((1u << shift) - 1u, top - lo);   // the sum may not pass the highest key there is
     rem -= s.res[1], in_bin = s.res[2], pre_above += s.res[3], pre_in = s.res[4];
   }
   const bool level0 = lo == 0u && hi == 0xffffffffu;

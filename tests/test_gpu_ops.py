@@ -195,6 +195,22 @@ def test_topk_whole_numbers_at_any_size(ops, oracle, L, k, low):
         assert torch.equal(ops.topk(x.to(DEV), k).cpu(), oracle.topk(x, k)), span
 
 
+@pytest.mark.parametrize("k", [1, 2, 300, 3000])
+@pytest.mark.parametrize("kind", ["whole", "huge", "inf"])
+def test_topk_at_the_upper_end_of_the_type(ops, oracle, k, kind):
+    """Threshold bins that are cut further (over 1024 elements) and whose last part holds the highest values of the type: its
+    bounds do not wrap around."""
+    g = torch.Generator().manual_seed(k)
+    if kind == "whole":
+        x = torch.randint((1 << 31) - 3000, 1 << 31, (16, 5000), generator=g, dtype=torch.int64).to(torch.int32)
+        x[:, 0], x[:, 77] = -(1 << 31), (1 << 31) - 1
+    else:
+        x = torch.randn(16, 5000, generator=g)
+        x[:, 100:100 + min(k + 1, 2900)] = torch.finfo(torch.float32).max if kind == "huge" else float("inf")
+        x[:, -1] = -x[:, 100]
+    assert torch.equal(ops.topk(x.to(DEV), k).cpu(), oracle.topk(x, k))
+
+
 def test_topk_3d_strided_rows(ops, oracle):
     g = torch.Generator().manual_seed(5)
     x = torch.randint(0, 97, (2, 4, 3000), generator=g, dtype=torch.int32)
