@@ -121,7 +121,10 @@ __device__ __forceinline__ float bfround(float f) { return bf2f(f2bf(f)); }
 
 // Order-preserving map of fp32 / int32 to uint32 (larger value -> larger key).
 __device__ __forceinline__ uint32_t ord_key(float f) {
-  uint32_t u = __float_as_uint(f);
+  // The bits as the compiler cannot follow them: it makes -|f| of setting the sign bit of a float, and the GPU's negation gives one
+  // and the same pattern for everything that is not a number, which as a key is below all positive values.
+  uint32_t u;
+  asm("mov.b32 %0, %1;" : "=r"(u) : "f"(f));
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ __forceinline__ uint32_t ord_key(int32_t v) { return (uint32_t)v ^ 0x80000000u; }

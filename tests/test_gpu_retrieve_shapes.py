@@ -103,6 +103,34 @@ def test_final_selection_beyond_the_first_rounds(oracle, bs, H, N, K, step):
     assert torch.equal(fin.cpu(), ref["final"])
 
 
+# Scores that are not numbers or infinite (positions of the zone): a NaN ranks above infinity.  The weights as arrays of planes: the
+# form in several launches
+@pytest.mark.parametrize("bs,H,N", [(20, 8, 1500), (1, 8, 6000), (1, 1, 9000)])
+@pytest.mark.parametrize("nan,inf", [((3,), ()), ((3, 40), (5,)), ((), (3, 5))])
+def test_final_selection_with_scores_that_are_no_numbers(oracle, bs, H, N, nan, inf):
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(N)
+    keys = synth_keys(g, bs, H, N)
+    q = synth_queries(g, keys, 4)
+    signs = srht_signs()
+    _, cen = oracle.constants()
+    counts = torch.zeros(bs, H, 16, 256, dtype=torch.int32, device=DEV)
+    cb, w, pk = ops.encode_keys(keys.to(DEV), signs.to(DEV), cluster_counts=counts)
+    for n in nan:
+        w[:, :, 7, n] = float("nan")
+    for n in inf:
+        w[:, :, 7, n] = float("inf")   # of either sign in the score, as the key's code has it
+    args = (counts, oracle.tier_counts(N, 0.25), N)
+    forms = [(cb, w, pk), (cb.contiguous(), w.contiguous(), pk.contiguous())]
+    for K in (2, 300):
+        for form in forms:
+            fin, ex = ops.retrieve(q.to(DEV), signs.to(DEV), cen.to(DEV), *form, *args, K, want=("cand", "scores_f32"))
+            assert torch.equal(ex["scores_f32"].isnan().sum(-1).cpu(), torch.full((bs, H), len(nan)))
+            assert torch.equal(ex["cand"], torch.arange(N, device=DEV).expand(bs, H, N))
+            at = torch.sort(ex["scores_f32"], dim=-1, descending=True, stable=True).indices[..., :K].sort(dim=-1).values
+            assert torch.equal(fin, at)
+
+
 # more entries per block than it lists in shared memory (4096), and just as many
 @pytest.mark.parametrize("rows,L,K", [(1, 300000, 290000), (3, 100000, 65536), (200, 9000, 4097), (200, 9000, 4096)])
 def test_final_topk_of_long_lists(oracle, rows, L, K):
