@@ -41,18 +41,22 @@ __host__ __device__ constexpr int sel_inbox_bytes(int cs) { return cs * (SEL_BIN
 struct F32Row {
   static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key(__uint_as_float(u)); }
   static __device__ __forceinline__ float from_key(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k); }
+  // Counted down from the row's highest value: a NaN, which the conversion makes zero, then shares the highest bin with what lies
+  // above the range.  Its key is the highest there is where arithmetic made it; one with the sign bit set, the lowest key there
+  // is, has to lie within the range (which then has no scale).
   struct Bins {
-    float vmin, scale;
+    float vmax, scale;
     __device__ __forceinline__ Bins(uint32_t kmin, uint32_t kmax) {
-      vmin = from_key(kmin);
-      scale = (float)(SEL_BINS - 1) / (from_key(kmax) - vmin);
+      vmax = from_key(kmax);
+      scale = (float)(SEL_BINS - 1) / (vmax - from_key(kmin));
       if (!(scale > 0.0f) || !(scale < INFINITY)) scale = 0.0f;   // flat or non-finite: one bin, the key levels decide
     }
     __device__ __forceinline__ unsigned of(uint32_t u) const {
-      return min((unsigned)(SEL_BINS - 1), __float2uint_rz((__uint_as_float(u) - vmin) * scale));   // (below vmin: 0)
+      return SEL_BINS - 1 - min((unsigned)(SEL_BINS - 1), __float2uint_rz((vmax - __uint_as_float(u)) * scale));   // (above vmax: the last)
     }
     __device__ __forceinline__ unsigned sub(uint32_t k, unsigned bin) const {
-      return scale > 0.0f ? min((unsigned)(SEL_SUB - 1), (unsigned)max(0.0f, ((from_key(k) - vmin) * scale - (float)bin) * (float)SEL_SUB)) : 0u;
+      const float down = (vmax - from_key(k)) * scale - (float)(SEL_BINS - 1 - bin);   // of the bin, from its upper end
+      return SEL_SUB - 1 - min((unsigned)(SEL_SUB - 1), __float2uint_rz(down * (float)SEL_SUB));
     }
     __device__ __forceinline__ bool single() const { return false; }
   };

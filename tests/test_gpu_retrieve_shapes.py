@@ -103,11 +103,14 @@ def test_final_selection_beyond_the_first_rounds(oracle, bs, H, N, K, step):
     assert torch.equal(fin.cpu(), ref["final"])
 
 
-# Scores that are not numbers or infinite (positions of the zone): a NaN ranks above infinity.  The weights as arrays of planes: the
-# form in several launches
+# Scores that are not numbers or infinite (positions of the zone): a NaN ranks above infinity.  Positions from 512 on lie behind the
+# first round of every warp (of the first block of a cluster), whose extremes the bins lie between; with weights that are 64 times as
+# large there, most of what is selected lies above that range, as the NaN does.  The weights as arrays of planes: the form in several
+# launches
 @pytest.mark.parametrize("bs,H,N", [(20, 8, 1500), (1, 8, 6000), (1, 1, 9000)])
-@pytest.mark.parametrize("nan,inf", [((3,), ()), ((3, 40), (5,)), ((), (3, 5))])
-def test_final_selection_with_scores_that_are_no_numbers(oracle, bs, H, N, nan, inf):
+@pytest.mark.parametrize("nan,inf,rise", [((3,), (), False), ((3, 40), (5,), False), ((), (3, 5), False), ((550,), (), False),
+                                          ((3, 550), (560,), False), ((550, 555), (560,), False), ((550,), (), True)])
+def test_final_selection_with_scores_that_are_no_numbers(oracle, bs, H, N, nan, inf, rise):
     from pariskv_b200 import ops
     g = torch.Generator().manual_seed(N)
     keys = synth_keys(g, bs, H, N)
@@ -116,6 +119,8 @@ def test_final_selection_with_scores_that_are_no_numbers(oracle, bs, H, N, nan, 
     _, cen = oracle.constants()
     counts = torch.zeros(bs, H, 16, 256, dtype=torch.int32, device=DEV)
     cb, w, pk = ops.encode_keys(keys.to(DEV), signs.to(DEV), cluster_counts=counts)
+    if rise:
+        w[..., 512:] *= 64
     for n in nan:
         w[:, :, 7, n] = float("nan")
     for n in inf:
