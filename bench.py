@@ -1033,7 +1033,7 @@ def seqshard_mode(args, device, rank, world, local_rank):
     n_total = cfg["context"] - cfg["sink"] - cfg["local"]
     start, end = sequence_shard(n_total, rank, world)
     need_gb = 2 * Lyr * H * n_total * 256 / 1e9          # all ranks together: they share the host
-    if args.store == "hbm" or (args.store == "auto" and Lyr * H * (end - start) * 624 + (36 << 30) < 180e9):
+    if args.store == "hbm" or (args.store == "auto" and Lyr * H * (end - start) * SequenceShardedCache.bytes_per_key() + (36 << 30) < 180e9):
         need_gb = 2 * H * (end - start) * 256 * 2 / 1e9   # staging of one layer only
     try:
         import psutil

@@ -376,7 +376,7 @@ class SequenceShardedCache:
         if store not in ("host", "hbm", "auto"):
             raise ValueError("store must be 'host', 'hbm' or 'auto'")
         if store == "auto":   # keep the shard's K/V rows in HBM when they fit beside the codes, else pinned host memory
-            need = layer_num * num_kv_heads * (self._n_local[0] + self.growth) * (512 + 112)
+            need = layer_num * num_kv_heads * (self._n_local[0] + self.growth) * self.bytes_per_key()
             free, _ = torch.cuda.mem_get_info(device)
             store = "hbm" if need + (16 << 30) < free else "host"
         self.store = store
@@ -398,6 +398,12 @@ class SequenceShardedCache:
         c_cap = min(n_cap, max(1, int(math.ceil(n_all * candidate_ratio))))
         self._retrieve_scratch = ops.Scratch(device, ops.retrieve_scratch_bytes(1, num_kv_heads, n_cap, c_cap))
         self._attn_scratch = ops.Scratch(device, ops.attention_scratch_bytes(1, num_heads, cap + final_topk))
+
+    @staticmethod
+    def bytes_per_key():
+        """HBM of a key of a shard with its rows there: K and V row, codes, 4-bit codes and weights."""
+        from . import ops
+        return 512 + ops.key_metadata_bytes()
 
     # the names the single-GPU cache uses for the same quantities
     @property

@@ -101,6 +101,12 @@ def alloc_key_metadata(bs, H, cap, device):
     return cb.permute(0, 1, 3, 2), w.permute(0, 1, 3, 2), pk.permute(0, 1, 3, 2, 4)
 
 
+def key_metadata_bytes():
+    """Bytes that alloc_key_metadata takes per key: from one key to the next in its two arrays."""
+    cb, w, _ = alloc_key_metadata(1, 1, 1, "meta")
+    return cb.stride(3) + 2 * w.stride(3)
+
+
 def encode_keys(keys, signs, codebook=None, block_weight=None, packed_4bit=None, cluster_counts=None):
     """keys bf16 [bs,H,L,128] -> (codebook, block_weight, packed_4bit); see pk_encode_keys.
     When `cluster_counts` (i32 [bs,H,16,256]) is given, the code histogram of these keys is ADDED to it."""
