@@ -8,7 +8,7 @@ model runtime written for the reference decodes through it unchanged.  The body 
   holds every older token: pinned host memory read through UVA when ``enable_offload`` is set, device
   memory otherwise.  Both modes run the same kernels.
 * Zone metadata (sign codes, 4-bit codes, rerank weights) is stored key-major and indexed by the
-  zone-relative position, so record 0 is 16-byte aligned and a rerank candidate is one 128-byte record.
+  zone-relative position, so record 0 is 16-byte aligned and a rerank candidate is one record.
   ``codebook_gpu / key_block_weight_gpu / key_4bit_packed_gpu`` expose them in the reference's logical
   shapes through permuted views.
 * One decode step of one layer is three launches: ``ops.append_encode`` (row append, key coding, flush),
@@ -61,7 +61,8 @@ class polar_cache(KV_Cache):
                  cache_cluster_num: int = 0, num_gpus: int = 1, model_size: int = 0,
                  codebook_path: str = "./turboquant/codebooks/codebook_d128_m8_Kr1_Kw256_rabitq_sign.json",
                  final_topk: int = 100, dynamic_update_interval: int = 512, full_attention_threshold: int = 2000,
-                 enable_offload: bool = True, srht_sign_vector=None, per_query_head_retrieval: bool = False) -> None:
+                 enable_offload: bool = True, srht_sign_vector=None, per_query_head_retrieval: bool = False,
+                 key_record_bytes: int = 128) -> None:
         super().__init__(layer_num, batch_size, max_length, num_key_value_heads, num_heads, head_dim, dtype,
                          layer_mapping, num_gpus, model_size)
         if head_dim != 128:
@@ -82,6 +83,8 @@ class polar_cache(KV_Cache):
         # Option beyond the reference, which ranks keys by the MEAN of the query heads that share a KV head
         # (cache_hub/polar_cache.py:1026-1031): every query head retrieves its own top-k from its KV head's keys.
         self.per_query_head_retrieval = bool(per_query_head_retrieval)
+        # Option: 96 saves 32 bytes of HBM per key, 128 reads a candidate's record in one unit of it (ops.alloc_key_metadata)
+        self.key_record_bytes = int(key_record_bytes)
         self.polar_m, self.polar_K_r, self.polar_K_omega = 8, 1, 256
         if codebook_path and os.path.exists(codebook_path):
             with open(codebook_path) as f:
@@ -147,7 +150,7 @@ class polar_cache(KV_Cache):
         self._staging, self._staging_turn = [[None, None], [None, None]], 0   # (buffer, event of the last copy out of it)
         self.codebook_gpu, self.key_block_weight_gpu, self.key_4bit_packed_gpu = [], [], []
         for _ in range(layer_num):
-            cb, w, pk = ops.alloc_key_metadata(bs, H, self.zone_capacity, dev)
+            cb, w, pk = ops.alloc_key_metadata(bs, H, self.zone_capacity, dev, self.key_record_bytes)
             self.codebook_gpu.append(cb)
             self.key_block_weight_gpu.append(w)
             self.key_4bit_packed_gpu.append(pk)

@@ -342,12 +342,13 @@ class SequenceShardedCache:
 
     def __init__(self, layer_num, num_kv_heads, num_heads, n_total, sink_size, local_size, interval, final_topk,
                  device, rank, world, group=None, collision_ratio=0.2, candidate_ratio=0.1, srht_sign_vector=None,
-                 store="host", exchange="nccl", max_new_length=0):
+                 store="host", exchange="nccl", max_new_length=0, key_record_bytes=128):
         from .cache_hub.polar_cache import srht_signs
         self.layer_num, self.kv_head, self.num_heads = layer_num, num_kv_heads, num_heads
         self.sink_size, self.local_size, self.interval = sink_size, local_size, interval
         self.dynamic_update_interval = interval
         self.steady_size = sink_size + local_size
+        self.key_record_bytes = key_record_bytes
         self.final_topk, self.device, self.rank, self.world, self.group = final_topk, device, rank, world, group
         self.collision_ratio, self.candidate_ratio = collision_ratio, candidate_ratio
         self.start, end0 = sequence_shard(n_total, rank, world)
@@ -376,7 +377,7 @@ class SequenceShardedCache:
         if store not in ("host", "hbm", "auto"):
             raise ValueError("store must be 'host', 'hbm' or 'auto'")
         if store == "auto":   # keep the shard's K/V rows in HBM when they fit beside the codes, else pinned host memory
-            need = layer_num * num_kv_heads * (self._n_local[0] + self.growth) * self.bytes_per_key()
+            need = layer_num * num_kv_heads * (self._n_local[0] + self.growth) * self.bytes_per_key(key_record_bytes)
             free, _ = torch.cuda.mem_get_info(device)
             store = "hbm" if need + (16 << 30) < free else "host"
         self.store = store
@@ -400,10 +401,10 @@ class SequenceShardedCache:
         self._attn_scratch = ops.Scratch(device, ops.attention_scratch_bytes(1, num_heads, cap + final_topk))
 
     @staticmethod
-    def bytes_per_key():
+    def bytes_per_key(key_record_bytes=128):
         """HBM of a key of a shard with its rows there: K and V row, codes, 4-bit codes and weights."""
         from . import ops
-        return 512 + ops.key_metadata_bytes()
+        return 512 + ops.key_metadata_bytes(key_record_bytes)
 
     # the names the single-GPU cache uses for the same quantities
     @property
@@ -425,7 +426,7 @@ class SequenceShardedCache:
         n_local = shard_keys.shape[2]
         assert n_local == self._n_local[layer], "shard length differs from sequence_shard()"
         cap = max(n_local + self.growth, 1)
-        cb, w, pk = ops.alloc_key_metadata(1, self.kv_head, cap, self.device)
+        cb, w, pk = ops.alloc_key_metadata(1, self.kv_head, cap, self.device, self.key_record_bytes)
         counts = torch.zeros(1, self.kv_head, 16, 256, dtype=torch.int32, device=self.device)
         ops.encode_keys(shard_keys, self.signs, cb[:, :, :, :n_local], w[:, :, :, :n_local], pk[:, :, :, :n_local, :],
                         cluster_counts=counts)

@@ -86,24 +86,28 @@ def _require_cuda(*tensors):
 # --------------------------------------------------------------------------------------------------
 # key coding
 # --------------------------------------------------------------------------------------------------
-def alloc_key_metadata(bs, H, cap, device):
+def alloc_key_metadata(bs, H, cap, device, record_bytes=128):
     """Key-major metadata storage for `cap` keys per head, returned as reference-shaped views:
     (codebook u8 [bs,H,16,cap], block_weight bf16 [bs,H,16,cap], packed u8 [bs,H,16,cap,4]).
     The sign codes, which every search reads from end to end, are an array of their own.  What the rerank reads of a few keys
-    only lies in one 128-byte record per key: 64 bytes of 4-bit codes, 32 of weights, 32 unused.  HBM is read in units of 128
+    only lies in one record per key: 64 bytes of 4-bit codes, 32 of weights, of 128 bytes the rest unused.  HBM is read in units of 128
     bytes: with the two in arrays of their own a candidate costs two units, with 96-byte records one and a half.  On B200 arrays
     -> records: 1M keys 132.1 -> 119.4 us a step, 16 sequences of 16 - 32K keys 219.5 -> 210.7, adaptive budgets of 8 sequences
-    147.1 -> 144.7, 128K keys 226.3 -> 221.9; 32 bytes of memory more per key, 112 -> 144."""
+    147.1 -> 144.7, 128K keys 226.3 -> 221.9; 32 bytes of memory more per key, 112 -> 144.  record_bytes=96 leaves these away, where
+    memory counts for more: records of 128 -> 96 bytes, 1M keys 114.1 -> 118.8 us a step, adaptive budgets of 8 sequences 128.1 ->
+    131.1, 16 sequences of 16 - 32K keys 200.1 -> 199.0."""
+    if record_bytes < 96 or record_bytes % 16:
+        raise ValueError("records are of at least 96 bytes, a multiple of 16")
     cb = torch.zeros(bs, H, cap, 16, dtype=torch.uint8, device=device)
-    rec = torch.zeros(bs, H, cap, 128, dtype=torch.uint8, device=device)
+    rec = torch.zeros(bs, H, cap, record_bytes, dtype=torch.uint8, device=device)
     w = rec.view(torch.bfloat16)[..., 32:48]
     pk = rec[..., :64].view(bs, H, cap, 16, 4)
     return cb.permute(0, 1, 3, 2), w.permute(0, 1, 3, 2), pk.permute(0, 1, 3, 2, 4)
 
 
-def key_metadata_bytes():
+def key_metadata_bytes(record_bytes=128):
     """Bytes that alloc_key_metadata takes per key: from one key to the next in its two arrays."""
-    cb, w, _ = alloc_key_metadata(1, 1, 1, "meta")
+    cb, w, _ = alloc_key_metadata(1, 1, 1, "meta", record_bytes)
     return cb.stride(3) + 2 * w.stride(3)
 
 

@@ -199,15 +199,18 @@ def test_shard_candidate_plan_splits_ties_in_rank_order():
     assert [int(g[2]) for g in got] == [2, 2, 1]
 
 
-def test_auto_store_counts_the_metadata_as_it_is_allocated(monkeypatch):
+@pytest.mark.parametrize("record", [128, 96])
+def test_auto_store_counts_the_metadata_as_it_is_allocated(monkeypatch, record):
     """store="auto" keeps a shard's rows in HBM only where they and the key metadata, at the size that its allocator takes, leave
     the reserve of 16 GB."""
     from pariskv_b200 import dist as pkd, ops
-    parts = ops.alloc_key_metadata(1, 1, 64, "cpu")
+    parts = ops.alloc_key_metadata(1, 1, 64, "cpu", record)
     meta = sum({t.untyped_storage().data_ptr(): t.untyped_storage().nbytes() for t in parts}.values()) // 64
+    assert meta == 16 + record
     layers, H, N, interval = 32, 8, 1_000_000, 32
     need = layers * H * (N + interval) * (512 + meta) + (16 << 30)   # one rank: room for a flush
     for free, want in ((need + 1, "hbm"), (need, "host")):
         monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (free, 180 << 30))
-        cache = pkd.SequenceShardedCache(layers, H, 32, N, 4, 64, interval, 100, "cpu", 0, 1, store="auto", srht_sign_vector=srht_signs())
+        cache = pkd.SequenceShardedCache(layers, H, 32, N, 4, 64, interval, 100, "cpu", 0, 1, store="auto", srht_sign_vector=srht_signs(),
+                                         key_record_bytes=record)
         assert cache.store == want

@@ -85,6 +85,40 @@ def test_cache_decode_matches_state_machine(oracle, offload):
     assert torch.equal(cache.cluster_key_counts_gpu[0].cpu(), oracle.cluster_counts(cb))
 
 
+def test_cache_with_compact_key_records(oracle):
+    """Records of 96 bytes per key: the same steps as with the usual 128, across a flush."""
+    from pariskv_b200.cache_hub.polar_cache import polar_cache
+    bs, H, Hq, sink, local, I, topk, P = 2, 2, 8, 4, 16, 8, 32, 2100
+    caches = []
+    for record in (128, 96):
+        caches.append(polar_cache(
+            valid_start=[0] * bs, layer_num=1, batch_size=bs, max_length=P + 64, num_key_value_heads=H, num_heads=Hq, head_dim=128,
+            dtype=torch.bfloat16, layer_mapping={"0": DEV}, max_new_length=64, sink_size=sink, local_size=local, final_topk=topk,
+            dynamic_update_interval=I, enable_offload=False, key_record_bytes=record))
+        assert caches[-1].key_block_weight_gpu[0].stride(3) * 2 == record
+    g = torch.Generator().manual_seed(11)
+    k, v = (synth_keys(g, bs, P, H).to(DEV) for _ in range(2))
+    steps = [[synth_keys(g, bs, 1, H).to(DEV) for _ in range(2)] + [torch.randn(bs, 1, Hq, 128, generator=g).to(DEV, torch.bfloat16)]
+             for _ in range(I + 3)]
+    outs = []
+    for c in caches:
+        c.prefill_update_kv_cache(None, k, v, 0, 0)
+        outs.append([])
+        for nk, nv, q in steps:
+            c.decode_update_kv_cache(nk, nv, 0)
+            outs[-1] += [c.compute(q, 0), c.last_topk_indices]
+        c.check_status()
+        n = c.cpu_valid_end[0]
+        outs[-1] += [t[0][:, :, :, :n] for t in (c.codebook_gpu, c.key_block_weight_gpu, c.key_4bit_packed_gpu)]
+    assert n == P - sink - local + I
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+    with pytest.raises(ValueError):
+        polar_cache(valid_start=[0], layer_num=1, batch_size=1, max_length=P, num_key_value_heads=H, num_heads=Hq, head_dim=128,
+                    dtype=torch.bfloat16, layer_mapping={"0": DEV}, max_new_length=64, sink_size=sink, local_size=local,
+                    enable_offload=False, key_record_bytes=80)
+
+
 def test_cache_short_prompt_dense_path(oracle):
     g = torch.Generator().manual_seed(3)
     bs, H, Hq, sink, local, I, topk = 1, 2, 8, 4, 8, 4, 16
