@@ -77,7 +77,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&x);
 }
 
-// 2^x for x <= 0: the unit's own instruction, results below 2^-126 are zero
+// 2^x for x <= 0: the unit's own instruction, results below 2^-126 are zero.  For the rows of a warp of the tensor-core form only: the
+// partials are merged with exp2f, a factor below 2^-126 as it is, because a partial may hold an infinite value.
 __device__ __forceinline__ float exp2_neg(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
       float L = 0.0f, O = 0.0f;
 #pragma unroll 4
       for (int t = 0; t < PG; t++) {
-        const float f = (s_m[t][g] == -INFINITY) ? 0.0f : exp2_neg(s_m[t][g] - M);
+        const float f = (s_m[t][g] == -INFINITY) ? 0.0f : exp2f(s_m[t][g] - M);
         L += s_l[t][g] * f;
         O += obuf[(t * PQ + g) * OS + dim] * f;
       }
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
         for (int w = 0; w < WARPS; w++) M = fmaxf(M, s_m[w][hd]);
 #pragma unroll
         for (int w = 0; w < WARPS; w++) {
-          const float f = s_m[w][hd] == -INFINITY ? 0.0f : exp2_neg(s_m[w][hd] - M);
+          const float f = s_m[w][hd] == -INFINITY ? 0.0f : exp2f(s_m[w][hd] - M);
           const float4 v = reinterpret_cast<const float4*>(obuf + (w * PQ + hd) * OS)[lane];
           L += s_l[w][hd] * f, o.x += v.x * f, o.y += v.y * f, o.z += v.z * f, o.w += v.w * f;
         }
@@ -454,13 +455,13 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
         for (int i = 0; i < MB; i++) m = fmaxf(m, ml[i].x);
 #pragma unroll
         for (int i = 0; i < MB; i++) {
-          const float f = ml[i].x == -INFINITY ? 0.0f : exp2_neg(ml[i].x - m);
+          const float f = ml[i].x == -INFINITY ? 0.0f : exp2f(ml[i].x - m);
           l += ml[i].y * f, o.x += v[i].x * f, o.y += v[i].y * f, o.z += v[i].z * f, o.w += v[i].w * f;
         }
         float M = m;
 #pragma unroll
         for (int off = 1; off < 8; off <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
-        const float f = m == -INFINITY ? 0.0f : exp2_neg(m - M);
+        const float f = m == -INFINITY ? 0.0f : exp2f(m - M);
         l *= f, o.x *= f, o.y *= f, o.z *= f, o.w *= f;
 #pragma unroll
         for (int off = 1; off < 8; off <<= 1) {
@@ -608,11 +609,11 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
 #pragma unroll
         for (int i = 0; i < MB; i++) mn = fmaxf(mn, ml[i][g].x);
         if (mn == -INFINITY) continue;   // no live row so far
-        const float c = exp2_neg(m[g] - mn);
+        const float c = exp2f(m[g] - mn);
         m[g] = mn, l[g] *= c, o[g].x *= c, o[g].y *= c, o[g].z *= c, o[g].w *= c;
 #pragma unroll
         for (int i = 0; i < MB; i++) {
-          const float f = exp2_neg(ml[i][g].x - mn);
+          const float f = exp2f(ml[i][g].x - mn);
           l[g] += ml[i][g].y * f;
           o[g].x += v[i][g].x * f, o[g].y += v[i][g].y * f, o[g].z += v[i][g].z * f, o[g].w += v[i][g].w * f;
         }
@@ -632,7 +633,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
       for (int w = 0; w < nw; w++) M = fmaxf(M, s_m[w0 + w][gg]);
 #pragma unroll
       for (int w = 0; w < nw; w++) {
-        const float f = s_m[w0 + w][gg] == -INFINITY ? 0.0f : exp2_neg(s_m[w0 + w][gg] - M);
+        const float f = s_m[w0 + w][gg] == -INFINITY ? 0.0f : exp2f(s_m[w0 + w][gg] - M);
         L += s_l[w0 + w][gg] * f;
         O += obuf[((w0 + w) * ATT_GQ + gg) * 128 + (tid & 127)] * f;
       }

@@ -461,6 +461,28 @@ def test_sparse_attention_keeps_32_bits(ops, group, bs, H):
     assert torch.equal(torch.isposinf(out), hit) and not torch.isnan(out).any()
 
 
+@pytest.mark.parametrize("bs,H", [(1, 2), (20, 8)])   # blocks of a head in a cluster; two tiles of 64 in a row
+@pytest.mark.parametrize("group", [1, 4, 8, 9])       # (9: the scalar form)
+def test_sparse_attention_merges_partials_of_tiny_weight(ops, group, bs, H):
+    """Rows 2^-130.6 of the others' weight hold an infinite value, in the block of the others and in one of their own: the factor
+    that their partials are merged with is a subnormal number, not zero, so the output is infinite as in 64 bits."""
+    g = torch.Generator(device=DEV).manual_seed(group)
+    n = 256
+    k = torch.zeros(bs, H, n, 128, dtype=torch.bfloat16, device=DEV)
+    k[:, :, 16:, 0] = -32.0                                # q k / sqrt(128) = -90.5
+    q = torch.zeros(bs, 1, H * group, 128, dtype=torch.bfloat16, device=DEV)
+    q[..., 0] = 32.0
+    v = torch.randn(bs, H, n, 128, generator=g, device=DEV).to(torch.bfloat16)
+    v[:, :, 20, 5], v[:, :, 200, 6] = float("inf"), float("-inf")
+    out = ops.sparse_attention(q, k, v, n).view(bs, H, group, 128)
+    s = torch.einsum("bhgd,bhnd->bhgn", q.view(bs, H, group, 128).double(), k.double()) / math.sqrt(128.0)
+    ref = torch.einsum("bhgn,bhnd->bhgd", torch.softmax(s, -1), v.double())
+    assert torch.isposinf(ref[..., 5]).all() and torch.isneginf(ref[..., 6]).all()
+    assert torch.equal(torch.isposinf(out), torch.isposinf(ref)) and torch.equal(torch.isneginf(out), torch.isneginf(ref))
+    rest = torch.isfinite(ref)
+    assert (out.double()[rest] - ref[rest]).abs().max().item() <= 2e-2
+
+
 # ---- glue kernels of the sequence-sharded form (against the torch formulation used by the gloo tests) ----
 def test_shard_pack_unpack_owned_merge(ops):
     from pariskv_b200 import dist as pkd
