@@ -143,8 +143,9 @@ __device__ __forceinline__ void mbar_arrive_expect(unsigned mb, unsigned bytes) 
 // CLUSTER: the blocks of a head are a thread-block cluster.  Each has up to three of its tiles of 128 rows in flight, and the
 // blocks' partials meet through distributed shared memory: every block merges a share of the outputs.  What this saves is the
 // way over L2, 4.4 us from the last product to the end (partial record, fence, atomic, records back into one SM, all in a row;
-// 7.3 with eight query heads); 1.6 like this.  B200, a step: one KV head of eight sequences with eight query heads each, four
-// layers, 186.2 -> 176.8 us; 128K keys, four layers 203.2 -> 194.4; 10K keys in host memory, four layers 155.2 -> 144.3.
+// 7.3 with eight query heads); 1.6 like this.  B200, a step of four layers with this form switched off -> on, all else the
+// same: 10K keys in host memory 156.4 -> 145.1 us, 128K keys 198.4 -> 191.7, one KV head of eight sequences with eight query heads each
+// 182.5 -> 176.3.
 template <bool MMA, int WARPS, bool CLUSTER>
 __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attention_kernel(AttParams p) {
   static_assert(!CLUSTER || (MMA && WARPS == 8), "the cluster form");
