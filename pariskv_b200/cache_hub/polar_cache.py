@@ -208,7 +208,8 @@ class polar_cache(KV_Cache):
         ops.check_attention_status(self._attn_scratch, self.batch_size, self.num_heads)
         flags = torch.stack([s[3] for s in self._layer_state]).cpu()
         if int(flags.abs().sum()) != 0:
-            raise RuntimeError("append: a layer's window was overrun or its zone / store had no room for a flush "
+            raise RuntimeError("append: a layer's window was overrun or its zone / store had no room for a flush, or a prompt's "
+                               "rows never arrived "
                                f"(layers {[i for i, f in enumerate(flags.tolist()) if f]})")
 
     # ------------------------------------------------------------------------------------------------

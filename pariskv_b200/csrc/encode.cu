@@ -2,6 +2,9 @@
 // histograms, query preparation and the append of a decode token.  One key is coded by 4 lanes, 32 dimensions (four
 // 8-dim subspaces) per lane.  Every fp32 operation rounds to nearest in a fixed order, so results do not depend on the
 // mapping.
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include "common.cuh"
 #include "keycode.cuh"
 #include "rotate.cuh"
@@ -43,8 +46,11 @@ __global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
     for (int i = tid; i < 16 * 256; i += EN_THREADS) hist[i] = 0;
     __syncthreads();
   }
-  RotateLane rl;
-  make_rotate_lane(rl, p.signs, s);
+  const RotateLane rl(s);
+  uint4 mask[4];
+  load_key32(mask, p.signs, s);
+#pragma unroll
+  for (int i = 0; i < 4; i++) mask[i] = sign_mask(mask[i]);
   const int64_t begin = (int64_t)blockIdx.y * p.chunk;
   const int64_t end = min(p.L, begin + p.chunk);
   const uint16_t* kbase = p.keys + b * p.k_b + h * p.k_h;
@@ -53,7 +59,9 @@ __global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
   for (int64_t k0 = begin; k0 < end; k0 += EN_KEYS) {  // uniform per block: shuffles need whole warps
     const int64_t key = k0 + grp;
     load_key32(nxt, kbase + min(key + EN_KEYS, end - 1) * p.k_l, s);   // in flight during the arithmetic
-    const KeyCode kc = code_key(raw, rl);
+#pragma unroll
+    for (int i = 0; i < 4; i++) raw[i] = flip(raw[i], mask[i]);
+    const KeyCode kc = code_key<1>(raw, rl);
 #pragma unroll
     for (int i = 0; i < 4; i++) raw[i] = nxt[i];
     if (key >= end) continue;
@@ -94,14 +102,23 @@ __global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
 // Token t of the prompt is a window row (the first `sink` tokens and the last `local` ones; all of them where the prompt
 // is not longer than both together) or zone row t - sink.  Every row is read once: its K and V go to the window or to the
 // store (K row and V row of a key next to each other), its key is coded into the staging arrays or the zone records, ||v||
-// and the cluster histogram come with it.  Block (h, chunk): consecutive tokens of one head, the heads of a token range
-// side by side in the grid, since they are neighbours in memory.
-// What bounds it: issue slots of the coding (180 warp instructions per key, two thirds of the issue slots, the half-rate ALU 60 % busy), then HBM (1136 bytes per key).
-// 131072 tokens x 8 heads on B200: 2003 us as coding, interleaving and copy launches, 282 us as this one.  Rows by bulk
-// copies into shared memory took 450 (two 256-byte copies per row are too many for the copy engine), by cp.async three
-// rounds ahead no less than with the next round in registers.
-
+// and the cluster histogram come with it.  A head's tokens are cut into tiles of 96, the zone rows first and the window
+// rows behind them; a block takes consecutive tiles, the heads of a token range side by side in the grid, since they are
+// neighbours in memory.
+// Tiles of zone rows come by TMA into one of two stages of shared memory and go to the store from there, K and V, four
+// instructions of one thread each way; the warps only read the keys, lane l of a warp 32 dimensions (quarter l / 8) of its key
+// l % 8, so that with the copies' 128-byte swizzle the eight lanes of a quarter-warp read fall into eight different groups of
+// four banks.  Other tiles (window rows; every row where the tensors cannot be described to the TMA unit) are loaded and
+// stored row by row.
+// What bounds it: issue slots of the coding, 70 - 75 % of them taken (integer ALU 60 %, DRAM 67 - 80 %), with 24 warps per SM.
+// 131072 tokens x 8 heads on B200: 2003 us as coding, interleaving and copy launches; 271 as one launch that carried the rows
+// through registers, 126 of them, 16 warps per SM; 226 as this one: 5.3 TB/s of 1136 bytes per key.  A block's tiles are an even
+// share of one wave: two waves of half the size take 229.  (Single rows by bulk copies took 450: the copy engine takes a row
+// per instruction no faster than a tile.)
 struct PrefillParams {
+  CUtensorMap map_k, map_v; // [P][H][128] by 64 dimensions x 1 head x 96 tokens
+  CUtensorMap map_store;    // [H][N][256] by 64 x 96 rows x 1 head
+  int tma, heads_inner;     // the maps are there; the heads are the middle dimension of map_k and map_v, not the outer one
   const uint16_t* k;        // [P][H][128] of one sample
   const uint16_t* v;
   int64_t k_l, k_h, v_l, v_h;
@@ -120,90 +137,180 @@ struct PrefillParams {
   int64_t z_wl, z_pl;       // weights (elements) and 4-bit codes (bytes) from one key to the next
   int32_t* counts;          // [H][16][256], zero at launch
   uint16_t* store;          // [H][store_cap][2][128]
-  int32_t* state;           // the layer's words, or null (see pk_prefill_sample)
-  int64_t P, N, cap_z, store_cap, chunk;
+  int32_t* state;           // the layer's words
+  int64_t P, N, cap_z, store_cap;
+  int64_t zone_tiles, n_tiles, tiles_per_block;   // tiles of a head: those by TMA, all
   int H, cap_w, sink, n_window, b;
 };
 
-__global__ void __launch_bounds__(EN_THREADS, 2) prefill_kernel(PrefillParams p) {
-  __shared__ int hist[16 * 256];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, s = tid & 3, grp = tid >> 2;
+constexpr int PF_THREADS = 384, PF_WARPS = PF_THREADS / 32;
+constexpr int PF_TILE = 8 * PF_WARPS;             // tokens
+constexpr int PF_HALF = PF_TILE * 128;            // bytes of 64 dimensions of a tile's K or V rows
+constexpr int PF_STAGE = 4 * PF_HALF;             // K, V; two halves each
+constexpr int PF_HIST = 16 * 256 * 4;
+constexpr int PF_SMEM = 2 * PF_STAGE + PF_HIST + 256 + 32;
+constexpr int PF_WAIT_LIMIT = 4000000;            // polls of a barrier before giving up
+
+__device__ __forceinline__ bool pf_wait(unsigned mbar, unsigned parity) {
+  unsigned done = 0;
+  for (int it = 0; it < PF_WAIT_LIMIT && !done; it++)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+  return done != 0;
+}
+
+__global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_constant__ PrefillParams p) {
+  extern __shared__ __align__(1024) unsigned char pf_smem[];   // (no static shared memory: the stages start on 1024 bytes)
+  int* hist = reinterpret_cast<int*>(pf_smem + 2 * PF_STAGE);
+  uint32_t* masks = reinterpret_cast<uint32_t*>(pf_smem + 2 * PF_STAGE + PF_HIST);
+  const unsigned smem0 = (unsigned)__cvta_generic_to_shared(pf_smem);
+  const unsigned full0 = smem0 + 2 * PF_STAGE + PF_HIST + 256, empty0 = full0 + 16;   // one barrier per stage: filled, read by all warps
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, s = lane >> 3;
   const int h = blockIdx.x;
-  for (int i = tid; i < 16 * 256; i += EN_THREADS) hist[i] = 0;
-  if (p.state && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) {
+  const int64_t first = (int64_t)blockIdx.y * p.tiles_per_block;
+  const int n = (int)min(p.tiles_per_block, p.n_tiles - first);                       // tiles of this block
+  const int n_tma = (int)min((int64_t)n, max((int64_t)0, p.zone_tiles - first));      // the leading ones come by TMA
+  if (tid == 0)
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n\tmbarrier.init.shared::cta.b64 [%1], %2;" ::"r"(full0 + 8 * i), "r"(empty0 + 8 * i),
+                   "r"(PF_WARPS)
+                   : "memory");
+  if (tid == 0) asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  for (int i = tid; i < 16 * 256; i += PF_THREADS) hist[i] = 0;
+  if (tid < 64) masks[tid] = reinterpret_cast<const uint32_t*>(p.signs)[tid] & 0x80008000u;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) {
     p.state[0] = p.n_window, p.state[1] = 0, p.state[2] = 0, p.state[3] = 0;
     p.state[4 + p.b] = (int32_t)p.N;
   }
   __syncthreads();
-  RotateLane rl;
-  make_rotate_lane(rl, p.signs, s);
-  const int64_t begin = (int64_t)blockIdx.y * p.chunk, end = min(p.P, begin + p.chunk);
-  const uint16_t* kb = p.k + h * p.k_h;
-  const uint16_t* vb = p.v + h * p.v_h;
-  // V is only copied: a half warp takes a row (16 bytes per lane), a warp the rows 2i, 2i + 1 of its eight in step i
-  uint4 kr[4], kn[4], vr[4];
-  auto load_v = [&](int64_t t0) {
+  auto load_tile = [&](int j) {   // (thread 0)
+    const unsigned dst = smem0 + (j & 1) * PF_STAGE, bar = full0 + 8 * (j & 1);
+    const int t = (int)(p.sink + (first + j) * PF_TILE), c1 = p.heads_inner ? h : t, c2 = p.heads_inner ? t : h;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(PF_STAGE) : "memory");
 #pragma unroll
     for (int i = 0; i < 4; i++)
-      vr[i] = reinterpret_cast<const uint4*>(vb + min(t0 + warp * 8 + 2 * i + (lane >> 4), end - 1) * p.v_l)[lane & 15];
+      asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                       dst + i * PF_HALF),
+                   "l"(i < 2 ? &p.map_k : &p.map_v), "r"((i & 1) * 64), "r"(c1), "r"(c2), "r"(bar)
+                   : "memory");
   };
-  load_key32(kr, kb + min(begin + grp, end - 1) * p.k_l, s);
-  load_v(begin);
-  for (int64_t t0 = begin; t0 < end; t0 += EN_KEYS) {
-    load_key32(kn, kb + min(t0 + EN_KEYS + grp, end - 1) * p.k_l, s);
+  auto store_tile = [&](int j) {   // (thread 0)
+    const unsigned src = smem0 + (j & 1) * PF_STAGE;
+    const int z = (int)((first + j) * PF_TILE);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int64_t t = t0 + warp * 8 + 2 * i + (lane >> 4), z = t - p.sink;
-      const bool zone = z >= 0 && z < p.N;
-      if (!zone || p.z_vnorm) {   // uniform over the half warp of a row
-        const uint32_t w[4] = {vr[i].x, vr[i].y, vr[i].z, vr[i].w};
+    for (int i = 0; i < 4; i++)
+      asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(&p.map_store), "r"(i * 64), "r"(z),
+                   "r"(h), "r"(src + i * PF_HALF)
+                   : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  };
+  if (tid == 0) {
+    if (n_tma > 0) load_tile(0);
+    if (n_tma > 1) load_tile(1);
+  }
+  const RotateLane rl(s);
+  const uint16_t* kb = p.k + h * p.k_h;
+  const uint16_t* vb = p.v + h * p.v_h;
+  bool lost = false;
+#pragma unroll 1
+  for (int j = 0; j < n; j++) {
+    const int row = warp * 8 + (lane & 7);   // the lane's key in the tile
+    const unsigned stage = smem0 + (j & 1) * PF_STAGE;
+    uint4 key[4];
+    int64_t t;       // the lane's token; P: none
+    if (j < n_tma) {
+      lost = __any_sync(0xffffffffu, lost || !pf_wait(full0 + 8 * (j & 1), (unsigned)(j >> 1) & 1u));
+      if (lost) {    // a copy that never landed: reported, and once more waited for, since it writes into this block's memory
+        if (lane == 0) atomicExch(p.state + 3, 1);
+        for (int i = j; i < min(n_tma, j + 2); i++) pf_wait(full0 + 8 * (i & 1), (unsigned)(i >> 1) & 1u);
+        break;
+      }
+      if (tid == 0) store_tile(j);
+      t = p.sink + (first + j) * PF_TILE + row;
+      if (t >= p.sink + p.N) t = p.P;
+      const unsigned at = stage + (s >> 1) * PF_HALF + row * 128;
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(key[i].x), "=r"(key[i].y), "=r"(key[i].z), "=r"(key[i].w)
+                     : "r"(at + ((((s & 1) * 4 + i) ^ (lane & 7)) << 4)));
+    } else {
+      const int64_t q = (first + j - p.zone_tiles) * PF_TILE + row;   // counted without the rows that come by TMA
+      t = q < (p.tma ? p.n_window : p.P) ? (p.tma && q >= p.sink ? q + p.N : q) : p.P;
+#pragma unroll
+      for (int i = 0; i < 4; i++) key[i] = reinterpret_cast<const uint4*>(kb + min(t, p.P - 1) * p.k_l + 32 * s)[i];
+    }
+    const int64_t z = t - p.sink;   // zone row, if 0 <= z < N; window row t or t - N otherwise
+    const bool zone = z >= 0 && z < p.N;
+    const int64_t wrow = z < p.N || p.N == 0 ? t : t - p.N;
+    if (j >= n_tma && t < p.P) {
+      uint4* dst = reinterpret_cast<uint4*>(zone ? p.store + ((int64_t)h * p.store_cap + z) * 256 : p.wk + h * p.w_h + wrow * 128) + 4 * s;
+#pragma unroll
+      for (int i = 0; i < 4; i++) dst[i] = key[i];
+    }
+    // V: a half warp takes a row (16 bytes per lane), a warp the rows 2i, 2i + 1 of its eight in step i; those that TMA copies
+    // are looked at for their norms only
+    if (j >= n_tma || p.z_vnorm) {
+#pragma unroll 1
+      for (int i = 0; i < 4; i++) {
+        const int64_t tv = __shfl_sync(0xffffffffu, t, 2 * i + (lane >> 4)), zv = tv - p.sink;
+        const int64_t wv = zv < p.N || p.N == 0 ? tv : tv - p.N;
+        const bool in_zone = zv >= 0 && zv < p.N;
+        const int l = lane & 15;
+        uint4 raw;
+        if (j < n_tma) {
+          const int r = warp * 8 + 2 * i + (lane >> 4);
+          const unsigned at = stage + (2 + (l >> 3)) * PF_HALF + r * 128 + (((l & 7) ^ (r & 7)) << 4);
+          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(raw.x), "=r"(raw.y), "=r"(raw.z), "=r"(raw.w) : "r"(at));
+        } else {
+          raw = reinterpret_cast<const uint4*>(vb + min(tv, p.P - 1) * p.v_l)[l];
+          if (tv < p.P)
+            (reinterpret_cast<uint4*>(in_zone ? p.store + ((int64_t)h * p.store_cap + zv) * 256 + 128 : p.wv + h * p.w_h + wv * 128))[l] = raw;
+        }
+        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
         float a = 0.0f;
 #pragma unroll
-        for (int j = 0; j < 4; j++) a = fmaf(lo_f(w[j]), lo_f(w[j]), fmaf(hi_f(w[j]), hi_f(w[j]), a));
-        const unsigned mask = 0xffffu << (lane & 16);
+        for (int k = 0; k < 4; k++) a = fmaf(lo_f(w[k]), lo_f(w[k]), fmaf(hi_f(w[k]), hi_f(w[k]), a));
 #pragma unroll
-        for (int off = 1; off < 16; off <<= 1) a += __shfl_xor_sync(mask, a, off);
-        if (t < end && (lane & 15) == 0) {
-          if (zone) p.z_vnorm[(int64_t)h * p.cap_z + z] = sqrtf(a);
-          else p.win_vnorm[(int64_t)h * p.cap_w + (z < p.N || p.N == 0 ? t : t - p.N)] = sqrtf(a);
+        for (int off = 1; off < 16; off <<= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+        if (tv < p.P && l == 0) {
+          if (!in_zone) p.win_vnorm[(int64_t)h * p.cap_w + wv] = sqrtf(a);
+          else if (p.z_vnorm) p.z_vnorm[(int64_t)h * p.cap_z + zv] = sqrtf(a);
         }
       }
-      if (t < end) {
-        if (zone) __stcs(reinterpret_cast<uint4*>(p.store + ((int64_t)h * p.store_cap + z) * 256 + 128) + (lane & 15), vr[i]);
-        else reinterpret_cast<uint4*>(p.wv + h * p.w_h + (z < p.N || p.N == 0 ? t : t - p.N) * 128)[lane & 15] = vr[i];
-      }
     }
-    load_v(t0 + EN_KEYS);
-    const KeyCode kc = code_key(kr, rl);
-    const int64_t t = t0 + grp, z = t - p.sink;   // zone row, if 0 <= z < N; window row t or t - N otherwise
-    if (t < end) {
-      if (z >= 0 && z < p.N) {
-        uint4* st = reinterpret_cast<uint4*>(p.store + ((int64_t)h * p.store_cap + z) * 256) + 4 * s;
+    if (j < n_tma) {
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty0 + 8 * (j & 1)) : "memory");
+    }
 #pragma unroll
-        for (int i = 0; i < 4; i++) st[i] = kr[i];
-        const int64_t rec = (int64_t)h * p.cap_z + z;
-        *reinterpret_cast<uint32_t*>(p.z_codes + rec * 16 + 4 * s) = kc.codes;
-        *reinterpret_cast<uint2*>(p.z_w + rec * p.z_wl + 4 * s) = kc.weights;
-        *reinterpret_cast<uint4*>(p.z_pk + rec * p.z_pl + 16 * s) = kc.packed;
+    for (int i = 0; i < 4; i++) key[i] = flip(key[i], reinterpret_cast<const uint4*>(masks)[4 * s + i]);
+    const KeyCode kc = code_key<8>(key, rl);
+    if (t < p.P) {
+      const int64_t rec = zone ? (int64_t)h * p.cap_z + z : (int64_t)h * p.cap_w + wrow;
+      *reinterpret_cast<uint32_t*>((zone ? p.z_codes : p.win_codes) + rec * 16 + 4 * s) = kc.codes;
+      *reinterpret_cast<uint2*>((zone ? p.z_w + rec * p.z_wl : p.win_w + rec * 16) + 4 * s) = kc.weights;
+      *reinterpret_cast<uint4*>((zone ? p.z_pk + rec * p.z_pl : p.win_pk + rec * 64) + 16 * s) = kc.packed;
+      if (zone)
 #pragma unroll
         for (int i = 0; i < 4; i++) atomicAdd(&hist[(4 * s + i) * 256 + ((kc.codes >> (8 * i)) & 0xffu)], 1);
-      } else {
-        const int64_t wrow = z < p.N || p.N == 0 ? t : t - p.N;
-        uint4* wk = reinterpret_cast<uint4*>(p.wk + h * p.w_h + wrow * 128) + 4 * s;
-#pragma unroll
-        for (int i = 0; i < 4; i++) wk[i] = kr[i];
-        const int64_t rec = (int64_t)h * p.cap_w + wrow;
-        *reinterpret_cast<uint32_t*>(p.win_codes + rec * 16 + 4 * s) = kc.codes;
-        *reinterpret_cast<uint2*>(p.win_w + rec * 16 + 4 * s) = kc.weights;
-        *reinterpret_cast<uint4*>(p.win_pk + rec * 64 + 16 * s) = kc.packed;
-      }
     }
-#pragma unroll
-    for (int i = 0; i < 4; i++) kr[i] = kn[i];
+    if (tid == 0 && j + 2 < n_tma) {   // the stage goes to tile j + 2 once all warps have read it and the stores have
+      lost = !pf_wait(empty0 + 8 * (j & 1), (unsigned)(j >> 1) & 1u);
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      if (!lost) load_tile(j + 2);
+    }
   }
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   __syncthreads();
   int32_t* dst = p.counts + (int64_t)h * 16 * 256;
-  for (int i = tid; i < 16 * 256; i += EN_THREADS)
+  for (int i = tid; i < 16 * 256; i += PF_THREADS)
     if (hist[i]) atomicAdd(dst + i, hist[i]);
 }
 
@@ -548,6 +655,41 @@ extern "C" int pk_encode_keys(const pk_tensor* keys, const pk_tensor* signs, con
   return check_launch("encode_keys");
 }
 
+// ---- tensor maps of the prompt's copies ----
+// The driver's encoder, asked for once: through the runtime, so that the library does not link to the driver.
+static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+  static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+      return cudaGetLastError(), (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
+    return (PFN_cuTensorMapEncodeTiled_v12000)f;
+  }();
+  return fn;
+}
+// 64 elements x box1 x box2 of a bf16 tensor [d2][d1][inner] in device memory; strides in elements, a multiple of 8.
+static bool row_map(CUtensorMap* m, const void* base, int64_t inner, int64_t d1, int64_t s1, int64_t d2, int64_t s2, int box1, int box2) {
+  const auto encode = tensor_map_encoder();
+  cudaPointerAttributes at;
+  if (!encode || s1 <= 0 || s2 <= 0 || s1 >= (1ll << 38) || s2 >= (1ll << 38) || d1 >= (1ll << 31) || d2 >= (1ll << 31)) return false;
+  if (cudaPointerGetAttributes(&at, base) != cudaSuccess || at.type != cudaMemoryTypeDevice) return cudaGetLastError(), false;
+  const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)d1, (cuuint64_t)d2}, strides[2] = {(cuuint64_t)s1 * 2, (cuuint64_t)s2 * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)box1, (cuuint32_t)box2}, steps[3] = {1, 1, 1};
+  return encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// The maps of a prompt with zone rows; false: the kernel copies row by row.  K and V share the order of their dimensions.
+static bool prefill_maps(PrefillParams& p) {
+  const int64_t kh = p.H == 1 ? p.P * p.k_l : p.k_h, vh = p.H == 1 ? p.P * p.v_l : p.v_h;
+  p.heads_inner = p.H > 1 && kh < p.k_l;
+  if (p.heads_inner != (p.H > 1 && vh < p.v_l)) return false;
+  auto prompt = [&](CUtensorMap* m, const uint16_t* x, int64_t sl, int64_t sh) {
+    return p.heads_inner ? row_map(m, x, 128, p.H, sh, p.P, sl, 1, PF_TILE) : row_map(m, x, 128, p.P, sl, p.H, sh, PF_TILE, 1);
+  };
+  return prompt(&p.map_k, p.k, p.k_l, kh) && prompt(&p.map_v, p.v, p.v_l, vh) &&
+         row_map(&p.map_store, p.store, 256, p.N, 256, p.H, p.store_cap * 256, PF_TILE, 1);
+}
+
 // The tensors of one cache layer that pk_append_encode and pk_prefill_sample share.
 struct CacheLayer {
   int64_t bs, H, cap_w, cap_z, w_b, w_h, z_wl, z_pl;
@@ -666,10 +808,21 @@ extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const p
   p.P = P, p.N = N, p.cap_z = c.cap_z;
   if (N > 0) p.store = (uint16_t*)rows->data, p.store_cap = H == 1 ? rows->shape[1] : rows->stride[0] / 256;
   p.H = (int)H, p.cap_w = (int)c.cap_w, p.sink = (int)sink, p.n_window = (int)(N > 0 ? sink + local : P), p.b = (int)b;
-  p.chunk = encode_chunk(P, H);
+  p.tma = N > 0 && prefill_maps(p);
+  p.zone_tiles = p.tma ? (N + PF_TILE - 1) / PF_TILE : 0;
+  p.n_tiles = p.zone_tiles + ((p.tma ? p.n_window : P) + PF_TILE - 1) / PF_TILE;
+  // one wave of two blocks per SM, an even share of the tiles for each
+  const int64_t fit = 2 * (int64_t)sm_count() / H;
+  p.tiles_per_block = fit > 1 ? (p.n_tiles + fit - 1) / fit : p.n_tiles;
+  while ((p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block > 65535) p.tiles_per_block *= 2;
+  static PerDevice smem_attr;
+  if (const unsigned long long bit = first_on_device(smem_attr)) {
+    if (cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM) != cudaSuccess) return check_launch("prefill smem", 0);
+    mark_on_device(smem_attr, bit);
+  }
   if (cudaMemsetAsync(p.counts, 0, (size_t)(H * 16 * 256 * 4), st) != cudaSuccess) return check_launch("prefill memset", 0);
   StageTimer tm(ST_ENCODE, st);
-  prefill_kernel<<<dim3((unsigned)H, (unsigned)((P + p.chunk - 1) / p.chunk)), EN_THREADS, 0, st>>>(p);
+  prefill_kernel<<<dim3((unsigned)H, (unsigned)((p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block)), PF_THREADS, PF_SMEM, st>>>(p);
   return check_launch("prefill");
 }
 

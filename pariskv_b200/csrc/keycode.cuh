@@ -100,25 +100,24 @@ struct KeyCode {
   uint4 packed;      // their 4-bit codes
 };
 
-// What a lane needs besides the key: sign masks of its dimensions (bit 15 / 31 of word j: dimensions 2j, 2j + 1 are
+// What lane s of a key's four needs besides the key: sign masks of its dimensions (bits 15 and 31 of a word: the dimension is
 // negated) and which side of the two cross-lane butterflies it is on.
-struct RotateLane {
-  uint32_t flip[16];
-  f32x2 side[2];
-};
-__device__ __forceinline__ void make_rotate_lane(RotateLane& rl, const uint16_t* signs, int s) {
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint4 a = reinterpret_cast<const uint4*>(signs + 32 * s)[i];
-    rl.flip[4 * i] = a.x & 0x80008000u, rl.flip[4 * i + 1] = a.y & 0x80008000u;
-    rl.flip[4 * i + 2] = a.z & 0x80008000u, rl.flip[4 * i + 3] = a.w & 0x80008000u;
-  }
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const float f = ((s >> i) & 1) ? -1.0f : 1.0f;
-    rl.side[i] = pair(f, f);
-  }
+__device__ __forceinline__ uint4 sign_mask(uint4 signs) {
+  return make_uint4(signs.x & 0x80008000u, signs.y & 0x80008000u, signs.z & 0x80008000u, signs.w & 0x80008000u);
 }
+__device__ __forceinline__ uint4 flip(uint4 raw, uint4 mask) {
+  return make_uint4(raw.x ^ mask.x, raw.y ^ mask.y, raw.z ^ mask.z, raw.w ^ mask.w);
+}
+struct RotateLane {
+  f32x2 side[2];
+  __device__ __forceinline__ explicit RotateLane(int s) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const float f = ((s >> i) & 1) ? -1.0f : 1.0f;
+      side[i] = pair(f, f);
+    }
+  }
+};
 
 // adjacent pairwise tree over eight pairs, both halves at once
 __device__ __forceinline__ f32x2 tree8(const f32x2* t) {
@@ -135,15 +134,17 @@ __device__ __forceinline__ float sqrt_approx(float x) {   // within 2 last place
   return r;
 }
 
-// raw: the lane's 32 dimensions of the key (bf16); all 32 lanes of the warp take part (eight keys).
-__device__ __forceinline__ KeyCode code_key(const uint4 (&raw)[4], const RotateLane& rl) {
+// key: the lane's 32 dimensions of the key (bf16), their signs applied; all 32 lanes of the warp take part (eight keys).
+// Lanes that share a key are APART from each other.
+template <int APART>
+__device__ __forceinline__ KeyCode code_key(const uint4 (&key)[4], const RotateLane& rl) {
   uint32_t in[16];
 #pragma unroll
-  for (int i = 0; i < 4; i++) in[4 * i] = raw[i].x, in[4 * i + 1] = raw[i].y, in[4 * i + 2] = raw[i].z, in[4 * i + 3] = raw[i].w;
+  for (int i = 0; i < 4; i++) in[4 * i] = key[i].x, in[4 * i + 1] = key[i].y, in[4 * i + 2] = key[i].z, in[4 * i + 3] = key[i].w;
   f32x2 x[16], t[16];
 #pragma unroll
   for (int j = 0; j < 8; j++) {   // pair i = dimensions i, i + 16; the sign flips do not change the norm
-    const uint32_t a = in[j] ^ rl.flip[j], b = in[j + 8] ^ rl.flip[j + 8];
+    const uint32_t a = in[j], b = in[j + 8];
     x[2 * j] = pair(lo_f(a), lo_f(b));
     x[2 * j + 1] = pair(hi_f(a), hi_f(b));
   }
@@ -155,7 +156,7 @@ __device__ __forceinline__ KeyCode code_key(const uint4 (&raw)[4], const RotateL
     split(add_2(tree8(t), tree8(t + 8)), a, b);
     float sum = __fadd_rn(a, b);
 #pragma unroll
-    for (int off = 1; off < 4; off <<= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, off));
+    for (int off = 1; off < 4; off <<= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, off * APART));
     n = sqrt_approx(sum);
     if (near_boundary<8>(n)) n = __fsqrt_rn(sum);
     n = bfround(n);
@@ -192,7 +193,7 @@ __device__ __forceinline__ KeyCode code_key(const uint4 (&raw)[4], const RotateL
     for (int i = 0; i < 16; i++) {
       float a, b;
       split(x[i], a, b);
-      const f32x2 p = pair(__shfl_xor_sync(0xffffffffu, a, 1 << st), __shfl_xor_sync(0xffffffffu, b, 1 << st));
+      const f32x2 p = pair(__shfl_xor_sync(0xffffffffu, a, APART << st), __shfl_xor_sync(0xffffffffu, b, APART << st));
       x[i] = fma_2(x[i], rl.side[st], p);   // x + p on one side, p - x on the other
     }
   // per half of the pairs (i < 8: subspaces 0 and 2 of the lane, i >= 8: 1 and 3)

@@ -71,3 +71,55 @@ def test_short_prompts_on_several_streams_share_no_buffer():
     for l in range(layers):
         for rows, store in zip(kv[l], (cache.unified_keys_cpu[l], cache.unified_values_cpu[l])):
             assert torch.equal(store[0, :, :n - 20], rows[0, 4:n - 16].transpose(0, 1).cpu())
+
+
+def _prompt(g, layout, bs, P, H):
+    """[bs,P,H,128] with the given order in memory: tokens outermost, heads outermost, one head's rows for all heads, or K
+    one way and V the other."""
+    def rows(kind):
+        if kind == "heads":
+            return torch.randn(bs, H, P, 128, generator=g).to(torch.bfloat16).to(DEV).transpose(1, 2)
+        if kind == "expanded":
+            return torch.randn(bs, P, 1, 128, generator=g).to(torch.bfloat16).to(DEV).expand(bs, P, H, 128)
+        if kind == "slice":     # the K or V columns of a wider row, whose first column lies 16 bytes into it
+            wide = torch.randn(bs, P, (H + 1) * 128 + 8, generator=g).to(torch.bfloat16).to(DEV)
+            return wide[..., 8:8 + H * 128].unflatten(-1, (H, 128))
+        return torch.randn(bs, P, H, 128, generator=g).to(torch.bfloat16).to(DEV)
+    return [rows(kind) for kind in (("tokens", "heads") if layout == "mixed" else (layout, layout))]
+
+
+# Zone rows around the edges of a tile of 96, windows of one tile and of two, one tile per block and several (both stages in turn).
+@pytest.mark.parametrize("P,H,local,layout", [
+    (115, 3, 16, "tokens"), (116, 3, 16, "heads"), (117, 3, 16, "mixed"), (211, 2, 16, "slice"), (213, 2, 16, "expanded"),
+    (228, 1, 128, "tokens"), (229, 2, 128, "heads"), (95, 2, 91, "tokens"), (96, 2, 91, "tokens"), (5001, 8, 64, "expanded"),
+    (90001, 1, 64, "slice"), (12900, 5, 100, "heads"), (40000, 2, 64, "tokens")])
+def test_prefill_tiles_match_oracle(oracle, P, H, local, layout):
+    from pariskv_b200.cache_hub.polar_cache_adaptivek_varlen import polar_cache
+    sink, bs = 4, 1
+    g = torch.Generator().manual_seed(P)
+    k, v = _prompt(g, layout, bs, P, H)
+    cache = polar_cache(valid_start=0, layer_num=1, batch_size=bs, max_length=P + 32, num_key_value_heads=H, num_heads=H, head_dim=128,
+                        dtype=torch.bfloat16, layer_mapping={"0": DEV}, max_new_length=32, sink_size=sink, local_size=local,
+                        final_topk=16, dynamic_update_interval=8, enable_offload=False)
+    cache.prefill_update_kv_cache(None, k, v, 0, 0)
+    cache.check_status()
+    N = max(0, P - sink - local)
+    kt, vt = k.transpose(1, 2).cpu(), v.transpose(1, 2).cpu()
+    win = list(range(P)) if N == 0 else list(range(sink)) + list(range(P - local, P))
+    cb, w, pk = oracle.encode(kt.contiguous(), cache.srht_diagonal_signs.cpu())
+    n, zone, norm = len(win), slice(sink, sink + N), vt.float().norm(dim=-1)
+    for got, want in [(cache.unified_keys_gpu[0][:, :, :n], kt[:, :, win]), (cache.unified_values_gpu[0][:, :, :n], vt[:, :, win]),
+                      (cache._win_codes[0][:, :, :n].permute(0, 1, 3, 2), cb[..., win]),
+                      (cache._win_4bit[0][:, :, :n].permute(0, 1, 3, 2, 4), pk[..., win, :]),
+                      (cache.codebook_gpu[0][..., :N], cb[..., zone]), (cache.key_4bit_packed_gpu[0][..., :N, :], pk[..., zone, :]),
+                      (cache._store_k[0][:, :, :N], kt[:, :, zone]), (cache._store_v[0][:, :, :N], vt[:, :, zone])]:
+        assert torch.equal(got.cpu(), want)
+    assert torch.equal(bits_of(cache._win_weight[0][:, :, :n].cpu().permute(0, 1, 3, 2)), bits_of(w[..., win]))
+    assert torch.equal(bits_of(cache.key_block_weight_gpu[0][..., :N].cpu()), bits_of(w[..., zone]))
+    # sums of 128 squares in fp32, whatever the order: at most 127 roundings of 2^-24 each in the sum, half of it in the root
+    assert torch.allclose(cache._win_vnorm[0][:, :, :n].cpu(), norm[:, :, win], rtol=1e-5)
+    assert torch.allclose(cache.value_norm_gpu[0][..., :N].cpu(), norm[..., zone], rtol=1e-5)
+    counts = oracle.cluster_counts(cb[..., zone].contiguous()) if N else torch.zeros(bs, H, 16, 256, dtype=torch.int32)
+    assert torch.equal(cache.cluster_key_counts_gpu[0].cpu(), counts)
+    if N:   # rows behind the zone's end are untouched
+        assert not cache._store_kv[0][:, :, N:].any() and not cache.codebook_gpu[0][..., N:].any()
