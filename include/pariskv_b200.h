@@ -522,8 +522,8 @@ int pk_qk_norm_rope(const pk_tensor* qkv, const pk_tensor* weight, const pk_tens
 int pk_add_rmsnorm(const pk_tensor* a, const pk_tensor* residual, const pk_tensor* weight, const pk_tensor* h_out,
                    const pk_tensor* x_out, double eps, void* stream);
 int pk_silu_mul(const pk_tensor* gate_up, const pk_tensor* out, void* stream);
-/* pk_gemv: out[1,O] = x[1,I] * weight[O,I]^T (bf16, fp32 accumulation), one token; HBM-bound streaming kernel, two rows
- *   per warp.  gated != 0: weight is a stacked [gate; up] matrix of O = 2F rows and out[1,F] = silu(gate x) * (up x),
+/* pk_gemv: out[1,O] = x[1,I] * weight[O,I]^T (bf16, fp32 accumulation), one token; HBM-bound streaming kernel, an
+ *   even share of the rows per SM.  gated != 0: weight is a stacked [gate; up] matrix of O = 2F rows and out[1,F] = silu(gate x) * (up x),
  *   rounded like pk_silu_mul after a separate product.  I a multiple of 8, at most 24576. */
 int pk_gemv(const pk_tensor* weight, const pk_tensor* x, const pk_tensor* out, int gated, void* stream);
 

@@ -196,14 +196,6 @@ __device__ __forceinline__ void build_lev2(uint32_t* lev2, const uint16_t* cente
     lev2[v * 32 + (tid & 31)] = ((v & 8) ? a : a ^ 0x8000u) | (((v & 0x80) ? b : b ^ 0x8000u) << 16);
   }
 }
-// acc + a.lo * b.lo, then + a.hi * b.hi: bf16 factors, fp32 sums
-__device__ __forceinline__ float fma_bf16x2(uint32_t a, uint32_t b, float acc) {
-  asm("{\n\t.reg .b16 al, ah, bl, bh;\n\tmov.b32 {al, ah}, %1;\n\tmov.b32 {bl, bh}, %2;\n\t"
-      "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %0, ah, bh, %0;\n\t}"
-      : "+f"(acc)
-      : "r"(a), "r"(b));
-  return acc;
-}
 __device__ __forceinline__ float rerank_record(const uint4 (&rec)[6], const uint32_t* lev2, const uint4* q, float qn, int lane, unsigned c128) {
   const uint32_t code[16] = {rec[0].x, rec[0].y, rec[0].z, rec[0].w, rec[1].x, rec[1].y, rec[1].z, rec[1].w,
                              rec[2].x, rec[2].y, rec[2].z, rec[2].w, rec[3].x, rec[3].y, rec[3].z, rec[3].w};

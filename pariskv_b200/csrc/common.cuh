@@ -119,6 +119,15 @@ __device__ __forceinline__ uint16_t f2bf(float f) {
 }
 __device__ __forceinline__ float bfround(float f) { return bf2f(f2bf(f)); }
 
+// acc + a.lo * b.lo, then + a.hi * b.hi: bf16 factors, fp32 sums
+__device__ __forceinline__ float fma_bf16x2(uint32_t a, uint32_t b, float acc) {
+  asm("{\n\t.reg .b16 al, ah, bl, bh;\n\tmov.b32 {al, ah}, %1;\n\tmov.b32 {bl, bh}, %2;\n\t"
+      "fma.rn.f32.bf16 %0, al, bl, %0;\n\tfma.rn.f32.bf16 %0, ah, bh, %0;\n\t}"
+      : "+f"(acc)
+      : "r"(a), "r"(b));
+  return acc;
+}
+
 // Order-preserving map of fp32 / int32 to uint32 (larger value -> larger key).
 __device__ __forceinline__ uint32_t ord_key(float f) {
   // The bits as the compiler cannot follow them: it makes -|f| of setting the sign bit of a float, and the GPU's negation gives one

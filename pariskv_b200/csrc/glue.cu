@@ -4,6 +4,8 @@
 // model_hub/qwen.py:381 silu_and_mul, :405 and :429 rmsnorm, :482 the rotary embedding); they are here because a
 // decode step of 36 layers is launch-latency bound outside the host-link fetch, and every separate elementwise
 // launch between two cache calls costs as much as the collision count itself.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace pk {
@@ -67,6 +69,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(const uint16_t* a, con
   __shared__ float s_rstd;
   float ss = 0.0f;
   const uint4 w0 = tid * 8 < n ? *reinterpret_cast<const uint4*>(w + tid * 8) : make_uint4(0, 0, 0, 0);   // under the reduction
+  uint4 h0 = make_uint4(0, 0, 0, 0);
   for (int i = tid * 8; i < n; i += 512 * 8) {
     const uint4 av = *reinterpret_cast<const uint4*>(a + base + i);
     const uint4 rv = r ? *reinterpret_cast<const uint4*>(r + base + i) : make_uint4(0, 0, 0, 0);
@@ -80,7 +83,9 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(const uint16_t* a, con
       ss += fl * fl + fh * fh;
       ow[k] = (uint32_t)lo | ((uint32_t)hi << 16);
     }
-    *reinterpret_cast<uint4*>(h_out + base + i) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+    const uint4 hv = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+    if (i == tid * 8) h0 = hv;
+    *reinterpret_cast<uint4*>(h_out + base + i) = hv;
   }
   ss = warp_sum(ss);
   if ((tid & 31) == 0) s_part[tid >> 5] = ss;
@@ -92,8 +97,8 @@ __global__ void __launch_bounds__(512) add_rmsnorm_kernel(const uint16_t* a, con
   }
   __syncthreads();
   const float rstd = s_rstd;
-  for (int i = tid * 8; i < n; i += 512 * 8) {   // every thread re-reads the values it wrote itself
-    const uint4 hv = *reinterpret_cast<const uint4*>(h_out + base + i);
+  for (int i = tid * 8; i < n; i += 512 * 8) {   // of rows longer than 4096 a thread re-reads what it wrote itself
+    const uint4 hv = i == tid * 8 ? h0 : *reinterpret_cast<const uint4*>(h_out + base + i);
     const uint4 wv = i == tid * 8 ? w0 : *reinterpret_cast<const uint4*>(w + i);
     const uint32_t hw[4] = {hv.x, hv.y, hv.z, hv.w}, ww[4] = {wv.x, wv.y, wv.z, wv.w};
     uint32_t ow[4];
@@ -207,92 +212,159 @@ extern "C" int pk_silu_mul(const pk_tensor* gate_up, const pk_tensor* out, void*
 }
 
 // ---- matrix-vector products of a decode step (one token): y = W x, W bf16 [O, I] row-major, fp32 accumulation ------
-// HBM-bound: a warp takes two rows, every lane keeps sixteen 16-byte streaming loads in flight, x sits in shared memory.
-// What is lost to the copy rate is the start of each launch, about 4 us where nothing overlaps it: dependent launch takes a
-// dense step of two layers (770 MB of weights) from 189 to 158 us on B200, telling the compiler that two blocks share an SM
-// to 151, and x four loads at a time to 148.  Reloading each register as soon as it is used (272 us) and smaller blocks for
-// an even last wave (196 against 189) lost.
+// HBM-bound: the weights are read once.  A block per SM takes an even share of the rows, one range of memory; its warps share the
+// columns (GvSplit::k_warps of them; where rows are short several rows are taken side by side), so that a warp keeps its part
+// of x in registers for all rows, and every lane has two steps of weight loads in flight.
+// What is lost to the copy rate is the start of each launch: its blocks are there while the launch before it still runs, and ask
+// for the first 48 KB of their rows by one prefetch to L2 before they wait.  On B200, a dense pass of two layers: hidden 4096,
+// feed-forward 12288 (770 MB) 148.8 -> 143.1 us against two rows per warp, 256 threads and a grid of 1.2 to 5.2 waves (without
+// the prefetch 146.4; 16, 32, 64, 128 KB 145.1, 143.4, 143.7, 146.4); hidden 2944, 8008: 93.4 -> 83; 5120, 13824: 217 -> 194.5.
 // GATED: the rows are (o, o + F) of a stacked [gate; up] matrix and the output is silu(gate) * up, rounded like the
 // separate launches would (bf16 after the product, after silu, after the multiply).
 namespace pk {
 namespace {
 
-__device__ __forceinline__ void unpack8(const uint4 v, float* f) {
-  f[0] = __uint_as_float(v.x << 16), f[1] = __uint_as_float(v.x & 0xffff0000u);
-  f[2] = __uint_as_float(v.y << 16), f[3] = __uint_as_float(v.y & 0xffff0000u);
-  f[4] = __uint_as_float(v.z << 16), f[5] = __uint_as_float(v.z & 0xffff0000u);
-  f[6] = __uint_as_float(v.w << 16), f[7] = __uint_as_float(v.w & 0xffff0000u);
+constexpr int GV_THREADS = 512, GV_WARPS = GV_THREADS / 32;
+constexpr int GV_CHUNKS = 6;               // 16-byte pieces of a row that a lane takes at most
+constexpr int GV_PANEL = 128;              // rows whose partial sums are kept at a time
+constexpr unsigned GV_PREFETCH = 48 << 10; // bytes
+
+// How the columns are split: 1 << k_log warps over a row, `chunks` pieces for a lane.
+struct GvSplit {
+  int k_log, chunks;
+};
+// The split that leaves the fewest lanes without a piece, of those with as many warps on a row as possible.
+GvSplit gemv_split(int64_t I) {
+  const int64_t n = I / 8;
+  GvSplit best = {0, 0};
+  double used = 0.0;
+  for (int k_log = 4; k_log >= 0; k_log--) {
+    const int64_t per_warp = (n + (1 << k_log) - 1) >> k_log, chunks = (per_warp + 31) / 32;
+    const double u = (double)n / (double)((chunks * 32) << k_log);
+    if (chunks <= GV_CHUNKS && u > used + 0.02) best = {k_log, (int)chunks}, used = u;
+  }
+  return best;
 }
 
-constexpr int GV_THREADS = 256;
-constexpr int GV_UNROLL = 8;
-
-template <bool GATED>
-__global__ void __launch_bounds__(GV_THREADS, 2) gemv_kernel(const uint16_t* W, const uint16_t* x, uint16_t* out, int O, int I, int F, bool early) {
-  extern __shared__ __align__(16) unsigned char gv_smem[];
-  uint4* xs = reinterpret_cast<uint4*>(gv_smem);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nchunk = I >> 3;
-  const int n_pairs = GATED ? F : (O + 1) / 2;
-  const int p = blockIdx.x * (GV_THREADS / 32) + warp;
-  const bool live = p < n_pairs;
-  const int r0 = GATED ? p : 2 * p, r1 = GATED ? p + F : 2 * p + 1;
-  const bool has1 = live && r1 < O;
-  const uint4* w0 = reinterpret_cast<const uint4*>(W + (int64_t)(live ? r0 : 0) * I);
-  const uint4* w1 = reinterpret_cast<const uint4*>(W + (int64_t)(has1 ? r1 : (live ? r0 : 0)) * I);
-  // With early loads (the weights never change) the first batch is issued before the wait for the kernel that produces
-  // x: the stream of weights starts under the tail of that kernel.
-  uint4 a[GV_UNROLL], b[GV_UNROLL];
-  auto load_batch = [&](int c0) {
+// Sums of N (a power of two) values over the lanes of a warp; every lane gets that of value sum_of<N>(lane).
+template <int N>
+__device__ __forceinline__ float warp_sums(float (&v)[N], int lane) {
+  int off = 16;
 #pragma unroll
-    for (int u = 0; u < GV_UNROLL; u++) {
-      const int c = c0 + 32 * u;
-      a[u] = (live && c < nchunk) ? __ldcs(w0 + c) : make_uint4(0, 0, 0, 0);
-      b[u] = (live && c < nchunk) ? __ldcs(w1 + c) : make_uint4(0, 0, 0, 0);
+  for (int n = N / 2; n >= 1; n /= 2, off /= 2) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < n; i++) {
+      const float keep = up ? v[i + n] : v[i], give = up ? v[i] : v[i + n];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
     }
-  };
-  if (!early) pdl_wait();
-  load_batch(lane);
-  pdl_wait();
-  pdl_trigger();
-  for (int c0 = tid; c0 < nchunk; c0 += 4 * GV_THREADS) {   // four loads in flight per thread
-    uint4 v[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) v[u] = reinterpret_cast<const uint4*>(x)[min(c0 + u * GV_THREADS, nchunk - 1)];
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-      if (c0 + u * GV_THREADS < nchunk) xs[c0 + u * GV_THREADS] = v[u];
   }
-  __syncthreads();
-  if (!live) return;
-  float acc0 = 0.0f, acc1 = 0.0f;
-  for (int base = 0; base < nchunk; base += 32 * GV_UNROLL) {   // warp-uniform trip count
-    const int c0 = base + lane;
 #pragma unroll
-    for (int u = 0; u < GV_UNROLL; u++) {
-      const int c = c0 + 32 * u;
-      if (c < nchunk) {
-        float xf[8], af[8], bf[8];
-        unpack8(xs[c], xf);
-        unpack8(a[u], af);
-        unpack8(b[u], bf);
+  for (; off > 0; off /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+  return v[0];
+}
+template <int N>
+__device__ __forceinline__ int sum_of(int lane) { return lane * N / 32; }
+
+// CH: pieces of a row per lane
+template <bool GATED, int CH>
+__global__ void __launch_bounds__(GV_THREADS, 1) gemv_kernel(const uint16_t* W, const uint16_t* x, uint16_t* out, int n_out, int I, int k_log, bool early) {
+  constexpr int U = GATED ? 2 : 1;                                            // rows of W per output
+  constexpr int RB = CH * U >= 5 ? 1 : CH * U >= 3 ? 2 / U + (U == 2 && CH == 2) : 8 / (CH * U);   // outputs of a warp per step
+  constexpr int NV = RB * U;
+  static_assert(NV == 1 || NV == 2 || NV == 4 || NV == 8, "warp_sums");
+  __shared__ float part[GV_PANEL * U][GV_WARPS + 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int k_warps = 1 << k_log, kw = warp & (k_warps - 1), side = GV_WARPS >> k_log, group = warp >> k_log;
+  const int first = (int)((int64_t)n_out * blockIdx.x / gridDim.x), rows = (int)((int64_t)n_out * (blockIdx.x + 1) / gridDim.x) - first;
+  const int n = I >> 3, c0 = (int)((int64_t)n * kw >> k_log) + lane, c1 = (int)((int64_t)n * (kw + 1) >> k_log);
+  if (tid == 0) {   // what this block reads first, on its way to L2 while it waits (a hint: no value is taken before the wait)
+    const int64_t bytes = (int64_t)rows * I * 2;
+    const unsigned size = (unsigned)min(bytes, (int64_t)(GV_PREFETCH / U));
 #pragma unroll
-        for (int k = 0; k < 8; k++) acc0 = fmaf(af[k], xf[k], acc0), acc1 = fmaf(bf[k], xf[k], acc1);
+    for (int u = 0; u < U; u++)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(W + ((int64_t)first + (int64_t)u * n_out) * I), "r"(size) : "memory");
+  }
+  struct Step {
+    uint4 w[RB][U][CH];
+  };
+  auto load = [&](Step& s, int step) {   // outputs (step * RB + i) * side + group of the block
+#pragma unroll
+    for (int i = 0; i < RB; i++) {
+      const int r = (step * RB + i) * side + group;
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const uint4* row = reinterpret_cast<const uint4*>(W + ((int64_t)first + r + (int64_t)u * n_out) * I);
+#pragma unroll
+        for (int j = 0; j < CH; j++) s.w[i][u][j] = r < rows && c0 + 32 * j < c1 ? __ldcs(row + c0 + 32 * j) : make_uint4(0, 0, 0, 0);
       }
     }
-    if (base + 32 * GV_UNROLL < nchunk) load_batch(c0 + 32 * GV_UNROLL);
-  }
-  acc0 = warp_sum(acc0);
-  acc1 = warp_sum(acc1);
-  if (lane == 0) {
-    if (GATED) {
-      const float g = bfround(acc0), uu = bfround(acc1);
-      out[p] = f2bf(bfround(g / (1.0f + __expf(-g))) * uu);
-    } else {
-      out[r0] = f2bf(acc0);
-      if (has1) out[r1] = f2bf(acc1);
+  };
+  Step a, b;
+  if (!early) pdl_wait();
+  load(a, 0);
+  pdl_wait();
+  pdl_trigger();
+  uint4 xs[CH];
+#pragma unroll
+  for (int j = 0; j < CH; j++) xs[j] = c0 + 32 * j < c1 ? reinterpret_cast<const uint4*>(x)[c0 + 32 * j] : make_uint4(0, 0, 0, 0);
+  const int per_step = RB * side, steps = (rows + per_step - 1) / per_step, panel = GV_PANEL / per_step;
+  auto flush = [&](int p0, int p_rows) {   // the panel's outputs
+    __syncthreads();
+    if (tid < p_rows) {
+      float y[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        y[u] = 0.0f;
+        for (int k = 0; k < k_warps; k++) y[u] += part[tid * U + u][k];
+      }
+      if (GATED) {
+        const float g = bfround(y[0]), up = bfround(y[U - 1]);
+        out[first + p0 + tid] = f2bf(bfround(g / (1.0f + __expf(-g))) * up);
+      } else {
+        out[first + p0 + tid] = f2bf(y[0]);
+      }
+    }
+  };
+  auto use = [&](const Step& s, int step, int in_panel) {
+    float v[NV];
+#pragma unroll
+    for (int i = 0; i < RB; i++)
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        float acc = 0.0f;
+#pragma unroll
+        for (int j = 0; j < CH; j++) {
+          const uint4 w = s.w[i][u][j];
+          acc = fma_bf16x2(w.x, xs[j].x, acc), acc = fma_bf16x2(w.y, xs[j].y, acc);
+          acc = fma_bf16x2(w.z, xs[j].z, acc), acc = fma_bf16x2(w.w, xs[j].w, acc);
+        }
+        v[i * U + u] = acc;
+      }
+    const float sum = warp_sums(v, lane);
+    const int at = sum_of<NV>(lane), r = (in_panel * RB + at / U) * side + group;
+    if (lane % (32 / NV) == 0) part[r * U + at % U][kw] = sum;
+  };
+  int in_panel = 0, p0 = 0;
+  auto step_done = [&]() {
+    if (++in_panel == panel) {
+      flush(p0, min(panel * per_step, rows - p0));
+      __syncthreads();
+      in_panel = 0, p0 += panel * per_step;
+    }
+  };
+#pragma unroll 1
+  for (int step = 0; step < steps; step += 2) {
+    if (step + 1 < steps) load(b, step + 1);
+    use(a, step, in_panel);
+    step_done();
+    if (step + 1 < steps) {
+      if (step + 2 < steps) load(a, step + 2);
+      use(b, step + 1, in_panel);
+      step_done();
     }
   }
+  if (in_panel) flush(p0, rows - p0);
 }
 
 }  // namespace
@@ -309,15 +381,22 @@ extern "C" int pk_gemv(const pk_tensor* weight, const pk_tensor* x, const pk_ten
   PK_REQUIRE(gated ? (O % 2 == 0 && out->shape[1] == O / 2) : out->shape[1] == O,
              "out must have O columns (O/2 when gated, with O even)");
   PK_REQUIRE(aligned16(weight->data) && aligned16(x->data), "weight and x must be 16-byte aligned");
-  const int64_t pairs = gated ? O / 2 : (O + 1) / 2;
-  const unsigned grid = (unsigned)((pairs + GV_THREADS / 32 - 1) / (GV_THREADS / 32));
-  const size_t smem = (size_t)I * 2;
+  const GvSplit split = gemv_split(I);
+  const int64_t n_out = gated ? O / 2 : O;
+  const unsigned grid = (unsigned)(n_out < sm_count() ? n_out : sm_count());
   StageTimer timer(ST_GEMV, (cudaStream_t)stream);
-  if (gated)
-    launch_chain(gemv_kernel<true>, dim3(grid), dim3(GV_THREADS), smem, (cudaStream_t)stream, (const uint16_t*)weight->data,
-                 (const uint16_t*)x->data, (uint16_t*)out->data, (int)O, (int)I, (int)(O / 2), pdl_early());
-  else
-    launch_chain(gemv_kernel<false>, dim3(grid), dim3(GV_THREADS), smem, (cudaStream_t)stream, (const uint16_t*)weight->data,
-                 (const uint16_t*)x->data, (uint16_t*)out->data, (int)O, (int)I, 0, pdl_early());
+  auto launch = [&](auto chunks) {
+    constexpr int CH = decltype(chunks)::value;
+    launch_chain(gated ? gemv_kernel<true, CH> : gemv_kernel<false, CH>, dim3(grid), dim3(GV_THREADS), 0, (cudaStream_t)stream,
+                 (const uint16_t*)weight->data, (const uint16_t*)x->data, (uint16_t*)out->data, (int)n_out, (int)I, split.k_log, pdl_early());
+  };
+  switch (split.chunks) {
+    case 1: launch(std::integral_constant<int, 1>()); break;
+    case 2: launch(std::integral_constant<int, 2>()); break;
+    case 3: launch(std::integral_constant<int, 3>()); break;
+    case 4: launch(std::integral_constant<int, 4>()); break;
+    case 5: launch(std::integral_constant<int, 5>()); break;
+    default: launch(std::integral_constant<int, 6>());
+  }
   return check_launch("gemv");
 }

@@ -759,3 +759,28 @@ def test_gemv_against_fp32(ops, O, I):
         want = torch.nn.functional.silu(gu[:, :O // 2]).to(torch.bfloat16).float() * gu[:, O // 2:]
         assert act.shape == (1, O // 2)
         assert (act.float().cpu() - want).abs().max().item() <= 3e-2 * max(1.0, want.abs().max().item())
+
+
+# Every number of pieces per lane and several splits of the columns over the warps, rows that do not divide by the blocks, fewer
+# rows than blocks, and more than one panel of 128 rows per block (148 blocks on B200).
+@pytest.mark.parametrize("O,I", [(1, 8), (7, 256), (150, 264), (148 * 3 + 1, 1024), (600, 1280), (300, 12288), (290, 2048 + 16), (333, 9000), (444, 5120),
+                                 (298, 15000), (150, 24576), (148 * 2 * 131, 32), (148 * 300 + 7, 136)])
+def test_gemv_splits_against_fp64(ops, O, I):
+    """fp32 sums of I products and one rounding to bf16 (2^-8 of the value): the sums' error is below I * 2^-24 of the sum of
+    magnitudes whatever their order."""
+    g = torch.Generator().manual_seed(O + I)
+    W = (torch.randn(O, I, generator=g) * 0.05).to(torch.bfloat16)
+    x = torch.randn(1, I, generator=g).to(torch.bfloat16)
+    W[0, :] = 0.0
+    if O > 2:
+        W[O - 1] = 1.0
+    y = ops.gemv(W.to(DEV), x.to(DEV)).double().cpu()
+    ref, mag = x.double() @ W.double().t(), x.double().abs() @ W.double().abs().t()
+    assert ((y - ref).abs() <= 2.0 ** -8 * ref.abs() + I * 2.0 ** -24 * mag + 1e-30).all()
+    if O % 2 == 0:
+        act = ops.gemv(W.to(DEV), x.to(DEV), gated=True).double().cpu()
+        gate, up = ref[:, :O // 2], ref[:, O // 2:]
+        want = torch.nn.functional.silu(gate) * up
+        # two roundings of either factor (gate, silu(gate); up), one of the product; silu's slope is below 1.1
+        err = 2.0 ** -8 * (1.1 * gate.abs() * up.abs() + 3 * want.abs()) + I * 2.0 ** -22 * (mag[:, :O // 2] * up.abs() + mag[:, O // 2:] * gate.abs() + 1)
+        assert ((act - want).abs() <= err).all()
