@@ -191,7 +191,8 @@ __device__ __forceinline__ float rerank_one(const RerankSmem& sm, const RerankAr
 constexpr int LEV2_BYTES = 256 * 32 * 4;
 
 __device__ __forceinline__ void build_lev2(uint32_t* lev2, const uint16_t* centers, int tid, int nthreads) {
-  for (int v = tid >> 5; v < 256; v += nthreads >> 5) {
+  for (int v = tid >> 5; v < 256; v += nthreads >> 5) {   // (tid < 0: a warp that leaves it to the others)
+    if (tid < 0) break;
     const uint32_t a = centers[v & 7], b = centers[(v >> 4) & 7];
     lev2[v * 32 + (tid & 31)] = ((v & 8) ? a : a ^ 0x8000u) | (((v & 0x80) ? b : b ^ 0x8000u) << 16);
   }
@@ -281,9 +282,9 @@ __device__ __forceinline__ void load_tiers(const ChainQuery& cq, long long N, un
   if (t < n) s_tiers[t] = cq.n_dev ? zone_tier(cq.sched, N, t) : cq.tiers[t];
   if (t == 8) s_tiers[8] = (unsigned)n;
 }
-// Tier table of one subspace by its warp.  sizes: 256 words with the cluster sizes (overwritten); key: the order made by
-// rank_subspace; lut: the subspace's 128 bytes (see tier_sum16).
-__device__ __forceinline__ void tier_table(const unsigned (&key)[4], unsigned* sizes, const unsigned* s_tiers, uint8_t* lut) {
+// Tier table of one subspace by a warp: the lane's four of the 128 bytes (see tier_sum16).  sizes: 256 words with the cluster
+// sizes (overwritten); key: the order made by rank_subspace.
+__device__ __forceinline__ uint32_t tier_table(const unsigned (&key)[4], unsigned* sizes, const unsigned* s_tiers) {
   const int lane = threadIdx.x & 31;
   const int n_tiers = (int)s_tiers[8];
   unsigned tier[8], front[4], back[4], n_front = 0, n_back = 0;
@@ -318,8 +319,7 @@ __device__ __forceinline__ void tier_table(const unsigned (&key)[4], unsigned* s
   __syncwarp();
   // entries i (low nibble) and i + 128 of byte i: four bytes per lane
   const uint4 e0 = *reinterpret_cast<const uint4*>(sizes + lane * 4), e1 = *reinterpret_cast<const uint4*>(sizes + 128 + lane * 4);
-  *reinterpret_cast<uint32_t*>(lut + lane * 4) =
-      (e0.x | (e1.x << 4)) | ((e0.y | (e1.y << 4)) << 8) | ((e0.z | (e1.z << 4)) << 16) | ((e0.w | (e1.w << 4)) << 24);
+  return (e0.x | (e1.x << 4)) | ((e0.y | (e1.y << 4)) << 8) | ((e0.z | (e1.z << 4)) << 16) | ((e0.w | (e1.w << 4)) << 24);
 }
 
 // Ordered candidate list of a block's n_keys counts (cnt8, overwritten; the first `skip` < 16 are not keys): those above
@@ -331,21 +331,21 @@ __device__ __forceinline__ int list_candidates(uint8_t* cnt8, int n_keys, int sk
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wspan = ((n_keys + CH_WARPS - 1) / CH_WARPS + 15) / 16 * 16;
   const int k0 = min(n_keys, warp * wspan), k1 = min(n_keys, k0 + wspan);
-  const uint32_t add_gt = (127u - T) * 0x01010101u;           // T <= 128, counts <= 128: no carry between bytes
-  const uint32_t add_ge = T ? (128u - T) * 0x01010101u : 0u;
+  // the top bit of every byte: count above / not below T (T <= 128, counts <= 128: no carry between bytes)
+  const uint32_t add_gt = T < 128u ? (127u - T) * 0x01010101u : 0u, keep_gt = T < 128u ? 0x80808080u : 0u;
+  const uint32_t add_ge = T ? (128u - T) * 0x01010101u : 0u, all_ge = T ? 0u : 0x80808080u;
+  // the top bits of 16 bytes, in order: dot products place eight of them side by side, 128 times as large
+  auto gather = [](uint32_t a, uint32_t b, uint32_t c, uint32_t d) -> unsigned {
+    return (__dp4a(b, 0x80402010u, __dp4a(a, 0x08040201u, 0u)) >> 7) | (__dp4a(d, 0x80402010u, __dp4a(c, 0x08040201u, 0u)) << 1);
+  };
   unsigned n_gt = 0, n_eq = 0;
 #pragma unroll 1
   for (int k = k0 + 16 * lane; k < k1; k += 512) {   // 16 keys -> masks of counts above / at the threshold, kept in their place
-    unsigned gt = 0, eq = 0;
     const uint4 v = *reinterpret_cast<const uint4*>(cnt8 + k);
-    const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t g = T < 128u ? (w4[i] + add_gt) & 0x80808080u : 0u;
-      const uint32_t ge = T ? (w4[i] + add_ge) & 0x80808080u : 0x80808080u;
-      gt |= ((((g >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * i);
-      eq |= (((((ge & ~g) >> 7) * 0x01020408u) >> 24) & 0xfu) << (4 * i);
-    }
+    auto above = [&](uint32_t w) -> uint32_t { return (w + add_gt) & keep_gt; };
+    auto not_below = [&](uint32_t w) -> uint32_t { return ((w + add_ge) | all_ge) & 0x80808080u; };
+    unsigned gt = gather(above(v.x), above(v.y), above(v.z), above(v.w));
+    unsigned eq = gather(not_below(v.x), not_below(v.y), not_below(v.z), not_below(v.w)) & ~gt;
     if (k1 - k < 16) gt &= (1u << (k1 - k)) - 1u, eq &= (1u << (k1 - k)) - 1u;
     if (k < skip) gt &= ~0u << skip, eq &= ~0u << skip;
     *reinterpret_cast<unsigned*>(cnt8 + k) = gt | (eq << 16);

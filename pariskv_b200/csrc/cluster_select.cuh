@@ -1,8 +1,8 @@
 // Exact top-K of a row that is spread over the CTAs of a thread-block cluster (each holds a contiguous slice):
 // first K of (value descending, position ascending), emitted in ascending position.
 //
-//   extremes of the row                      -> 256 bins: linear in the value for floats, about equally filled; the top
-//                                               eight bits of (key - lowest key) for whole numbers, exact at any size
+//   extremes of the row                      -> 512 bins: linear in the value for floats, about equally filled; the top
+//                                               nine bits of (key - lowest key) for whole numbers, exact at any size
 //   histogram of the bins, summed over ranks -> the bin of the K-th largest, this CTA's share above it and in it
 //   the elements of that bin, gathered by every CTA, cut once more into 64 sub-bins and ranked -> the exact threshold
 //   ordered emission of this CTA's elements at its offset, a warp per 32 elements.
@@ -13,7 +13,9 @@
 // that makes the values itself can have the extremes exchanged while it still does (see `published`).
 // What bounds it is the latency of these steps and three passes over the slice.  On B200 the last stage of the chain takes 7.2
 // us with 1310 scores on each of 10 CTAs (9.7 with remote reads, the emission a word per lane and every rank counted in
-// sub-bins), 6.1 with 655 (9.5), 7 - 10 with some 5000 on one CTA (10 - 13).
+// sub-bins), 6.1 with 655 (9.5), 7 - 10 with some 5000 on one CTA (10 - 13), all with 256 bins of 32 bits.  512 bins halve the members
+// of the threshold bin and what ranking them takes (1.9 -> 1.5 us of the 7.2, with fewer than 129 a warp has four lanes for each);
+// as words of 32 bits their exchange would take as much longer (10 CTAs: 1.1 -> 1.6 us), as halves it does not.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -28,17 +30,19 @@ namespace cg = cooperative_groups;
 
 constexpr int SEL_THREADS = 512;
 constexpr int SEL_WARPS = SEL_THREADS / 32;
-constexpr int SEL_BINS = 256;
+constexpr int SEL_WORDS = 256;   // words of a histogram: 512 bins of 16 bits for slices below 65536 elements, 256 of 32 bits for longer ones
 constexpr int SEL_SUB = 64;
 constexpr int SEL_TIES = 1024;
 constexpr int SEL_REGION = 2 * SEL_TIES * 8;   // bytes of dynamic shared memory
 // What the CTAs of a cluster write into each other, at the same offset of dynamic shared memory in every CTA and used by nothing
-// else: histograms [rank][SEL_BINS], extremes [rank][warp].
-__host__ __device__ constexpr int sel_inbox_bytes(int cs) { return cs * (SEL_BINS * 4 + SEL_WARPS * 8); }
+// else: histograms [rank][SEL_WORDS], extremes [rank][warp].
+__host__ __device__ constexpr int sel_inbox_bytes(int cs) { return cs * (SEL_WORDS * 4 + SEL_WARPS * 8); }
 
 // Rows of a type: the ordered key of an element, and the level-0 bins between the extremes of the row's keys.  A bin is
 // monotone in the key; sub() cuts a bin into SEL_SUB parts, monotone as well; single(): a bin holds one value.
+template <int N_BINS>
 struct F32Row {
+  static constexpr int BINS = N_BINS;
   static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key(__uint_as_float(u)); }
   static __device__ __forceinline__ float from_key(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k); }
   // Counted down from the row's highest value: a NaN, which the conversion makes zero, then shares the highest bin with what lies
@@ -48,32 +52,34 @@ struct F32Row {
     float vmax, scale;
     __device__ __forceinline__ Bins(uint32_t kmin, uint32_t kmax) {
       vmax = from_key(kmax);
-      scale = (float)(SEL_BINS - 1) / (vmax - from_key(kmin));
+      scale = (float)(BINS - 1) / (vmax - from_key(kmin));
       if (!(scale > 0.0f) || !(scale < INFINITY)) scale = 0.0f;   // flat or non-finite: one bin, the key levels decide
     }
     __device__ __forceinline__ unsigned of(uint32_t u) const {
-      return SEL_BINS - 1 - min((unsigned)(SEL_BINS - 1), __float2uint_rz((vmax - __uint_as_float(u)) * scale));   // (above vmax: the last)
+      return BINS - 1 - min((unsigned)(BINS - 1), __float2uint_rz((vmax - __uint_as_float(u)) * scale));   // (above vmax: the last)
     }
     __device__ __forceinline__ unsigned sub(uint32_t k, unsigned bin) const {
-      const float down = (vmax - from_key(k)) * scale - (float)(SEL_BINS - 1 - bin);   // of the bin, from its upper end
+      const float down = (vmax - from_key(k)) * scale - (float)(BINS - 1 - bin);   // of the bin, from its upper end
       return SEL_SUB - 1 - min((unsigned)(SEL_SUB - 1), __float2uint_rz(down * (float)SEL_SUB));
     }
     __device__ __forceinline__ bool single() const { return false; }
   };
 };
 // From the keys themselves: as floats, whole numbers above 2^24 would share a bin that single() takes for one value.
+template <int N_BINS>
 struct I32Row {
+  static constexpr int BINS = N_BINS;
   static __device__ __forceinline__ uint32_t key(uint32_t u) { return ord_key((int32_t)u); }
   struct Bins {
     uint32_t kmin;
-    int shift;   // (kmax - kmin) >> shift < SEL_BINS
-    __device__ __forceinline__ Bins(uint32_t kmin_, uint32_t kmax) : kmin(kmin_) { shift = max(0, 24 - __clz(kmax - kmin)); }
+    int shift;   // (kmax - kmin) >> shift < BINS
+    __device__ __forceinline__ Bins(uint32_t kmin_, uint32_t kmax) : kmin(kmin_) { shift = max(0, (BINS == 512 ? 23 : 24) - __clz(kmax - kmin)); }
     __device__ __forceinline__ unsigned of(uint32_t u) const { return (key(u) - kmin) >> shift; }
     __device__ __forceinline__ unsigned sub(uint32_t k, unsigned bin) const { return (k - kmin - (bin << shift)) >> max(0, shift - 6); }
     __device__ __forceinline__ bool single() const { return shift == 0; }
   };
 };
-static_assert(SEL_BINS == 256 && SEL_SUB == 64, "the shifts of I32Row::Bins");
+static_assert(SEL_SUB == 64, "the shifts of I32Row::Bins");
 
 struct SelShared {               // static: small block-wide results
   unsigned n_members;            // local elements of the threshold bin
@@ -122,18 +128,19 @@ __device__ __forceinline__ void put_everywhere(cg::cluster_group& cluster, T* at
   }
 }
 
-// Threshold of a histogram spread over the cluster, after the barrier that completes hists ([CS][SEL_BINS], one row per CTA):
+// Threshold of a histogram spread over the cluster, after the barrier that completes hists ([CS][SEL_WORDS], one row per CTA;
+// two bins of 16 bits in a word where there are 512):
 // thread t sums bin t, a block-wide suffix scan finds the highest bin with (elements in bins >= it) >= want; see
 // SelShared::res.  Returns after the result is visible to the block.
 template <int CS, int BINS>
 __device__ __forceinline__ void cluster_threshold(SelShared& s, const unsigned* hists, unsigned rank, unsigned want) {
-  static_assert(BINS <= SEL_THREADS && BINS <= SEL_BINS, "one bin per thread");
+  static_assert(BINS <= SEL_THREADS && (BINS <= SEL_WORDS || BINS == 2 * SEL_WORDS), "one bin per thread");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned tot = 0, pre = 0;
   if (tid < BINS) {
 #pragma unroll
     for (int r = 0; r < CS; r++) {
-      const unsigned v = hists[r * SEL_BINS + tid];
+      const unsigned v = BINS <= SEL_WORDS ? hists[r * SEL_WORDS + tid] : (unsigned)reinterpret_cast<const uint16_t*>(hists + r * SEL_WORDS)[tid];
       tot += v;
       if ((unsigned)r < rank) pre += v;
     }
@@ -157,7 +164,7 @@ __device__ __forceinline__ void cluster_threshold(SelShared& s, const unsigned* 
 // A warp's extremes into the inboxes of all CTAs.
 template <int CS>
 __device__ __forceinline__ void publish_range(cg::cluster_group& cluster, unsigned* inbox, unsigned rank, unsigned kmin, unsigned kmax) {
-  uint2* extremes = reinterpret_cast<uint2*>(inbox + CS * SEL_BINS);
+  uint2* extremes = reinterpret_cast<uint2*>(inbox + CS * SEL_WORDS);
   kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
   put_by_lanes<CS>(cluster, extremes + rank * SEL_WARPS + (threadIdx.x >> 5), make_uint2(kmin, kmax), threadIdx.x & 31);
 }
@@ -166,6 +173,7 @@ __device__ __forceinline__ void publish_range(cg::cluster_group& cluster, unsign
 // kmin / kmax: this thread's share of the extremes of the slice's ordered keys (~0 / 0 without any).  published: every warp has
 // called publish_range() with the extremes of some of the slice's elements, and every thread has arrived at a cluster barrier
 // (CS > 1) behind it; the level-0 bins then lie between those extremes, elements outside fall into the first and the last one.
+// V::BINS: 512 where no CTA's slice has more than 65535 elements, otherwise 256.
 // region: SEL_REGION bytes, inbox: sel_inbox_bytes(CS), at the same offsets in all CTAs; words: 2 * words_cap words of this
 // CTA's shared memory for ballots (longer slices are evaluated again instead).  All CTAs of the cluster call this with the same
 // K (>= 1, at most the row's length), after a cluster barrier, none of them still using its region for anything else.
@@ -175,11 +183,13 @@ template <int CS, class V, bool LISTED, class At, class OutOf>
 __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelShared& s, unsigned* region, unsigned* inbox,
                                                unsigned* words, int words_cap, unsigned rank, int n, int K, int64_t* __restrict__ out, At at,
                                                OutOf out_of, unsigned kmin, unsigned kmax, bool published = false) {
+  constexpr int BINS = V::BINS;
+  static_assert(BINS == SEL_WORDS || BINS == 2 * SEL_WORDS, "one word or half a word per bin");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned* hists = inbox;
-  uint2* extremes = reinterpret_cast<uint2*>(inbox + CS * SEL_BINS);
+  uint2* extremes = reinterpret_cast<uint2*>(inbox + CS * SEL_WORDS);
   auto exchange_range = [&](bool published) {   // extremes over the cluster, to kmin and kmax of every thread; clears the histogram replicas
-    for (int i = tid; i < 4 * SEL_BINS; i += SEL_THREADS) region[i] = 0;
+    for (int i = tid; i < 4 * BINS; i += SEL_THREADS) region[i] = 0;
     if (published) {
       if (CS > 1) cluster.barrier_wait();
       __syncthreads();
@@ -195,12 +205,22 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     }
     kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
   };
-  unsigned* my_hist = region + (lane & 3) * SEL_BINS;
+  unsigned* my_hist = region + (lane & 3) * BINS;
   auto exchange_hist = [&]() {
     __syncthreads();
-    if (tid < SEL_BINS)
-      put_everywhere<CS>(cluster, hists + rank * SEL_BINS + tid,
-                         region[tid] + region[SEL_BINS + tid] + region[2 * SEL_BINS + tid] + region[3 * SEL_BINS + tid]);
+    if (tid < SEL_WORDS) {
+      unsigned word = 0;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {   // (16 bits a bin: the halves' sums stay below 65536)
+        if (BINS == SEL_WORDS) {
+          word += region[i * BINS + tid];
+        } else {
+          const uint2 v = reinterpret_cast<const uint2*>(region + i * BINS)[tid];
+          word += v.x | (v.y << 16);
+        }
+      }
+      put_everywhere<CS>(cluster, hists + rank * SEL_WORDS + tid, word);
+    }
     sync_cluster<CS>(cluster);
   };
   // ---- level 0: bins over the range of the row ----
@@ -210,7 +230,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
 #pragma unroll 4
   for (int i = tid; i < n; i += SEL_THREADS) atomicAdd(&my_hist[bin0(at(i))], 1u);
   exchange_hist();
-  cluster_threshold<CS, SEL_BINS>(s, hists, rank, (unsigned)K);
+  cluster_threshold<CS, BINS>(s, hists, rank, (unsigned)K);
   const unsigned T0 = s.res[0];
   unsigned rem = (unsigned)K - s.res[1], in_bin = s.res[2], pre_above = s.res[3], pre_in = s.res[4];
   // ---- key levels: ordered keys of the members between their extremes ----
@@ -229,14 +249,14 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       lo = hi = base;
       break;
     }
-    const int shift = max(0, 24 - __clz(top - base));   // (top - base) >> shift < SEL_BINS
+    const int shift = max(0, (BINS == 512 ? 23 : 24) - __clz(top - base));   // (top - base) >> shift < BINS
 #pragma unroll 1
     for (int i = tid; i < n; i += SEL_THREADS) {
       const uint32_t u = at(i), k = V::key(u);
       if (bin0(u) == T0 && k >= base && k <= top) atomicAdd(&my_hist[(k - base) >> shift], 1u);
     }
     exchange_hist();
-    cluster_threshold<CS, SEL_BINS>(s, hists, rank, rem);
+    cluster_threshold<CS, BINS>(s, hists, rank, rem);
     lo = base + (s.res[0] << shift);
     hi = lo + min((1u << shift) - 1u, top - lo);   // the sum may not pass the highest key there is
     rem -= s.res[1], in_bin = s.res[2], pre_above += s.res[3], pre_in = s.res[4];

@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) collide_kernel(CollParams p) {
     for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
     __syncthreads();
     if (!early) rank_subspace(key, s_q + warp * 8, lane);
-    tier_table(key, my, s_tiers, s_lut + warp * 128);
+    reinterpret_cast<uint32_t*>(s_lut + warp * 128)[lane] = tier_table(key, my, s_tiers);
     __syncthreads();
   }
   if (LAYOUT == 1) {

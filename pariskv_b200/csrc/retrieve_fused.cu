@@ -10,8 +10,8 @@
 //
 // Why this split: as two launches (count | select + rerank + final top-K by the last block of a head) the final stage ran
 // on one SM per head, 12 us of 48 at 128K keys, and counts and scores went through L2.  Time line of a CTA on B200
-// (8 heads x 131004 keys, 10 CTAs each; the query prepared before the wait): tables 3.1 us, counting 13 K keys 6.4, threshold
-// and list 4.0, rerank of 1310 candidates 6.1, final selection 7.2: 27 us.  Graph-replayed layer step, two launches -> one: 16
+// (8 heads x 131004 keys, 10 CTAs each; query and ranking, 2.4 us, before the wait): tables 1.9 us, counting 13 K keys 6.8, threshold
+// 1.5, list 2.2, rerank of 1310 candidates 5.9, final selection 6.7.  Graph-replayed layer step, two launches -> one: 16
 // sequences of 16 - 32K keys (one CTA per head, no exchange at all) 155 -> 116 us, 8 heads x 128K keys 70 -> 60, 10K keys 27 -> 19
 // for the chain.
 // What bounds it: the serial chain of exchanges for small zones; for long ones instruction issue in the counting (85
@@ -28,7 +28,7 @@ static_assert(CH_THREADS == SEL_THREADS, "one block shape");
 constexpr int FR_LIST_MAX = 8192;           // candidates a CTA keeps in shared memory; more spill to the workspace
 constexpr int FR_SPAN_MAX = 40 * 1024;      // keys of a CTA: beyond it three launches over all SMs are faster
 constexpr int FR_WORDS = LEV2_BYTES / 8;    // ballots of the final selection, over the level table
-static_assert(FR_SPAN_MAX / 32 <= FR_WORDS, "one ballot per 32 candidates");
+static_assert(FR_SPAN_MAX / 32 <= FR_WORDS && FR_SPAN_MAX < 65536, "one ballot per 32 candidates, 16 bits for a bin's count");
 static_assert(CH_HIST_BYTES >= SEL_REGION && CH_STAGE >= 16 * 256 * 4, "areas that serve two stages");
 
 struct FusedParams {
@@ -78,9 +78,10 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   QueryLoads ql;
   unsigned key[4];
   for (int i = tid; i < CH_CBINS * 32; i += CH_THREADS) region[i] = 0;
-  if (cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
-  if (CS > 1) cluster.barrier_arrive();   // a CTA has to run before the others may write into it
   const bool early = cq.early_query != 0;
+  // the level table is left to the warps that do not prepare the query
+  if (cq.early_loads) build_lev2(lev2, p.a.centers, tid - 32, CH_THREADS - 32);
+  if (CS > 1) cluster.barrier_arrive();   // a CTA has to run before the others may write into it
   // Both orders (queries before the wait or behind it) run through one copy of the preparation and the ranking: a CTA fetches its
   // code as it goes, and with two copies of them and longer unrolls in the selection a step with 128K keys took 195.8 us against
   // 191.9, one KV head of eight sequences 170.7 against 167.4.
@@ -92,7 +93,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   // A word written by the kernel before this one takes over a microsecond to arrive: the cluster sizes, the zone length and
   // (where they may not be read earlier) the queries are asked for together.  Then the code loads: a warp takes 128
   // consecutive keys (four per lane) every CH_WARPS * 128; two rounds are in flight, the first ones during the prologue.
-  int4 c0, c1;
+  int4 c0, c1;   // cluster sizes of this warp's subspace
   int64_t N, begin;
   int n_keys;
   const uint8_t* codes;
@@ -104,9 +105,21 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
       for (int j = 0; j < 4; j++)   // past the end: the last key again, its count unused
         r[j] = reinterpret_cast<const uint4*>(codes)[min(v0 + 32 * j, n_keys - 1)];
   };
+  // In a large cluster a CTA makes the tables of its share of the subspaces only, a warp each, and writes them into all CTAs:
+  // sixteen warps at the tier counts are bound by the integer ALU, and the exchange costs less than that (sort and tables of 10K
+  // keys on 10 CTAs 3.6 -> 2.7 us; on one or two CTAs there is nothing to gain).  With the level table left to the warps that do not
+  // prepare the query, a histogram that four threads a bin add up, and 512 bins in the selection, a step of four layers with
+  // 10K keys in host memory 140.6 -> 133.2 us, with 128K keys 188.5 -> 182.3, one KV head of eight sequences 168.3 -> 162.1; of two
+  // layers with 16 sequences of 16 - 32K keys 195.5 -> 190.8.  All pairs of clusters compared by all threads instead of the sort
+  // took 0.6 us longer: reads of shared memory.
+  constexpr bool SHARED_TABLES = CS >= 4;
+  const int sub = SHARED_TABLES ? (int)rank + CS * warp : warp;
+  const bool ranks = sub < 16;
   auto load_zone = [&]() {
-    const int4* sizes = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + warp) * 256 + lane * 8);
-    c0 = sizes[0], c1 = sizes[1];   // of this warp's subspace
+    if (ranks) {
+      const int4* sizes = reinterpret_cast<const int4*>(cq.counts + ((int64_t)bh * 16 + sub) * 256 + lane * 8);
+      c0 = sizes[0], c1 = sizes[1];
+    }
     N = cq.n_dev ? min(max((int64_t)cq.n_dev[b], (int64_t)1), p.N) : p.N;
     const int span = (int)(((N + CS - 1) / CS + 15) / 16 * 16);
     begin = (int64_t)rank * span;
@@ -117,9 +130,9 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   };
   if (!early) load_zone();
   prepare_query(pq, ql, cq, b, h, p.G, p.inv_g, s_q, &s_qnorm);
-  if (!cq.early_loads) build_lev2(lev2, p.a.centers, tid, CH_THREADS);
+  if (!cq.early_loads) build_lev2(lev2, p.a.centers, tid - 32, CH_THREADS - 32);
   __syncthreads();
-  rank_subspace(key, s_q + warp * 8, lane);
+  if (ranks) rank_subspace(key, s_q + sub * 8, lane);
   if (early) {   // the queries were complete before the kernel before this one started
     pdl_wait();
     pdl_trigger();
@@ -127,15 +140,26 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   }
   const int64_t C_want = cq.n_dev ? min((int64_t)zone_candidates(cq.sched, N), p.C) : p.C_want;
   {
-    unsigned* my = reinterpret_cast<unsigned*>(cnt8) + warp * 256;   // the counts are not there yet
     if (warp == 0 && rank == 0) publish_query(pq, cq, bh);
-    if (tid >= 32 && tid < 41) load_tiers(cq, (long long)N, s_tiers, tid - 32);
-    *reinterpret_cast<int4*>(my + lane * 8) = c0;
-    *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
-    __syncthreads();
-    tier_table(key, my, s_tiers, s_lut + warp * 128);
+    if (tid >= CH_THREADS - 32 && tid < CH_THREADS - 23) load_tiers(cq, (long long)N, s_tiers, tid - (CH_THREADS - 32));
     if (tid < 128) reinterpret_cast<uint16_t*>(s_qb)[tid] = f2bf(s_q[tid]);
-    __syncthreads();   // the tables are complete, the sizes are done with
+    unsigned* my = reinterpret_cast<unsigned*>(cnt8) + warp * 256;   // the counts are not there yet
+    if (ranks) {
+      *reinterpret_cast<int4*>(my + lane * 8) = c0;
+      *reinterpret_cast<int4*>(my + lane * 8 + 4) = c1;
+    }
+    __syncthreads();
+    uint32_t table = 0;
+    if (ranks) table = tier_table(key, my, s_tiers);
+    uint32_t* at = reinterpret_cast<uint32_t*>(s_lut + sub * 128) + lane;
+    if (SHARED_TABLES) {
+      cluster.barrier_wait();
+      if (ranks) put_everywhere<CS>(cluster, at, table);
+      cluster.sync();
+    } else {
+      *at = table;
+      __syncthreads();   // the tables are complete, the sizes are done with
+    }
   }
   const float qn = s_qnorm;
 
@@ -157,14 +181,27 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
     count_round(r0, v0);
     if (v0 - lane + STEP < n_keys) count_round(r1, v0 + STEP);
   }
-  if (CS > 1) cluster.barrier_wait();
+  if (CS > 1 && !SHARED_TABLES) cluster.barrier_wait();
   __syncthreads();
-  for (int bin = warp; bin < CH_CBINS; bin += CH_WARPS) {   // bin totals, in the place of the first replicas
-    const unsigned t = __reduce_add_sync(0xffffffffu, region[bin * 32 + lane]);
-    if (lane == 0) region[bin * 32] = t;
+  {   // bin totals into the inboxes of all CTAs: four threads a bin, each with eight replicas (in turns, so that banks differ)
+    const int bin = tid >> 2, q = tid & 3;
+    unsigned t = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) t += region[bin * 32 + q * 8 + ((i + bin) & 7)];
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    static_assert(CH_CBINS == CH_THREADS / 4 + 1, "four threads a bin, and the last bin");
+    unsigned last = 0;
+    if (warp == 0) last = __reduce_add_sync(0xffffffffu, region[(CH_CBINS - 1) * 32 + lane]);
+#pragma unroll
+    for (int r = 0; r < CS; r += 4)
+      if (r + q < CS) {
+        unsigned* at = inbox + rank * SEL_WORDS;
+        if (CS > 1) at = cluster.map_shared_rank(at, r + q);
+        at[bin] = t;
+        if (tid < 4) at[CH_CBINS - 1] = last;
+      }
   }
-  __syncthreads();
-  if (tid < CH_CBINS) put_everywhere<CS>(cluster, inbox + rank * SEL_BINS + tid, region[tid * 32]);
   sync_cluster<CS>(cluster);
   cluster_threshold<CS, CH_CBINS>(s, inbox, rank, (unsigned)C_want);
   const unsigned T = s.res[0], quota = (unsigned)C_want - s.res[1];
@@ -221,7 +258,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
 
   // ---- final top-K over the cluster ----
   __syncthreads();   // the scores are complete; the level table and the histogram region are free
-  cluster_select<CS, F32Row, false>(
+  cluster_select<CS, F32Row<512>, false>(
       cluster, s, region, inbox, lev2, FR_WORDS, rank, n_list, K_here, p.final_out + bh * p.K,
       [&](int i) -> uint32_t { return __float_as_uint(score_at(i)); }, [&](int i) -> int64_t { return id_at(i); }, kmin, kmax, true);
 }

@@ -29,7 +29,7 @@ struct TopkParams {
   int cache;                 // elements of a slice kept in shared memory: all of them, or 0
 };
 
-template <int CS, class Row>
+template <int CS, template <int> class Row>
 __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char dyn[];
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
   const int64_t slice = ((L + CS - 1) / CS + 31) / 32 * 32, begin = min(L, (int64_t)rank * slice);
   const int n = (int)(min(L, begin + slice) - begin);
   const uint32_t* in = p.in + row * p.row_stride + begin;
-  const bool cached = n <= p.cache;
+  const bool cached = p.cache > 0;   // the same for all CTAs of the row
   unsigned kmin = 0xffffffffu, kmax = 0u;
   int done = 0;
   if (cached && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {   // whole groups of four: up to six such loads in flight per thread
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
 #pragma unroll
       for (int j = 0; j < 6; j++) {   // (past the end: the last group again, which changes nothing)
         reinterpret_cast<uint4*>(cache)[min(base + j * SEL_THREADS, groups - 1)] = u[j];
-        const unsigned k0 = Row::key(u[j].x), k1 = Row::key(u[j].y), k2 = Row::key(u[j].z), k3 = Row::key(u[j].w);
+        const unsigned k0 = Row<512>::key(u[j].x), k1 = Row<512>::key(u[j].y), k2 = Row<512>::key(u[j].z), k3 = Row<512>::key(u[j].w);
         kmin = min(min(kmin, min(k0, k1)), min(k2, k3)), kmax = max(max(kmax, max(k0, k1)), max(k2, k3));
       }
     }
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
       const int i = base + j * SEL_THREADS;
       if (i < n) {
         if (cached) cache[i] = u[j];
-        const unsigned k = Row::key(u[j]);
+        const unsigned k = Row<512>::key(u[j]);
         kmin = min(kmin, k), kmax = max(kmax, k);
       }
     }
@@ -91,14 +91,14 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
   const int64_t* map = p.map ? p.map + row * p.map_stride + begin : nullptr;
   auto out_of = [&](int i) -> int64_t { return map ? map[i] : begin + i; };
   if (cached)
-    cluster_select<CS, Row, true>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
+    cluster_select<CS, Row<512>, true>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
                             [&](int i) -> uint32_t { return cache[i]; }, out_of, kmin, kmax);
   else
-    cluster_select<CS, Row, true>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
+    cluster_select<CS, Row<256>, true>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
                             [&](int i) -> uint32_t { return in[i]; }, out_of, kmin, kmax);
 }
 
-template <int CS, class Row>
+template <int CS, template <int> class Row>
 int topk_active() {   // clusters that fit the device at once; also opts in to the shared memory
   auto kern = topk_kernel<CS, Row>;
   const int smem = tk_fixed(CS) + TK_CACHE * 4;
@@ -119,7 +119,7 @@ int topk_active() {   // clusters that fit the device at once; also opts in to t
 struct TopkCapacity {
   int active[N_CLUSTER_SIZES];
 };
-template <class Row>
+template <template <int> class Row>
 const TopkCapacity* topk_capacity() {
   static TopkCapacity cap[64];
   static PerDevice asked;
@@ -133,7 +133,7 @@ const TopkCapacity* topk_capacity() {
   return &cap[dev];
 }
 
-template <int CS, class Row>
+template <int CS, template <int> class Row>
 cudaError_t launch_topk_cs(int64_t rows, size_t smem, cudaStream_t st, const TopkParams& p) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(CS, (unsigned)rows), cfg.blockDim = dim3(SEL_THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st;
@@ -153,7 +153,7 @@ cudaError_t launch_topk_cs(int64_t rows, size_t smem, cudaStream_t st, const Top
   return cudaLaunchKernelEx(&cfg, topk_kernel<CS, Row>, p);
 }
 
-template <class Row>
+template <template <int> class Row>
 int launch_rows(TopkParams p, int64_t rows, cudaStream_t st) {
   const TopkCapacity* cap = topk_capacity<Row>();
   if (!cap) return fail(PK_ERR_CUDA, "topk: cannot identify the device");
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(1024) sort_by_value_kernel(const uint32_t* in,
     unsigned long long v = 0;
     if (i < k) {
       const int64_t idx = o[i];
-      v = ((unsigned long long)(is_float ? F32Row::key(row[idx]) : I32Row::key(row[idx])) << 32) | (0xffffffffu - (unsigned)idx);
+      v = ((unsigned long long)(is_float ? F32Row<512>::key(row[idx]) : I32Row<512>::key(row[idx])) << 32) | (0xffffffffu - (unsigned)idx);
     }
     sk[i] = v;
   }

@@ -784,3 +784,32 @@ def test_gemv_splits_against_fp64(ops, O, I):
         # two roundings of either factor (gate, silu(gate); up), one of the product; silu's slope is below 1.1
         err = 2.0 ** -8 * (1.1 * gate.abs() * up.abs() + 3 * want.abs()) + I * 2.0 ** -22 * (mag[:, :O // 2] * up.abs() + mag[:, O // 2:] * gate.abs() + 1)
         assert ((act - want).abs() <= err).all()
+
+
+# Slices of the most elements that are kept in shared memory (16-bit counts of 512 bins; all of them in one bin, or nearly) and one
+# group more (32-bit counts of 256 bins), on the largest cluster and on one CTA.
+@pytest.mark.parametrize("rows,L", [(1, 16 * 32768), (1, 16 * 32768 + 1), (150, 32768), (150, 32769), (3, 16 * 511), (2, 5000)])
+@pytest.mark.parametrize("kind", ["equal", "two values", "one off", "wide ints", "floats", "floats with inf and nan"])
+def test_topk_bins_at_the_edges_of_a_slice(ops, rows, L, kind):
+    g = torch.Generator(device=DEV).manual_seed(L + rows)
+    if kind == "equal":
+        x = torch.full((rows, L), 7, dtype=torch.int32, device=DEV)
+    elif kind == "two values":
+        x = torch.randint(0, 2, (rows, L), generator=g, device=DEV, dtype=torch.int32)
+    elif kind == "one off":
+        x = torch.zeros(rows, L, device=DEV)
+        x[:, L // 3] = 1e30
+    elif kind == "wide ints":
+        x = torch.randint(-2 ** 31, 2 ** 31 - 1, (rows, L), generator=g, device=DEV, dtype=torch.int32)
+    else:
+        x = torch.randn(rows, L, generator=g, device=DEV)
+        if "nan" in kind:
+            x[:, L // 2], x[:, L // 5], x[:, 11] = float("inf"), float("nan"), -float("inf")
+    for k in (1, 100, L // 50 + 1):
+        got = ops.topk(x, k)
+        key = x.double() if x.dtype == torch.int32 else torch.where(x.isnan(), torch.full_like(x, float("inf")), x).double()
+        if "nan" in kind:
+            key[:, L // 5] = 3e38 * 10   # above infinity
+            key[:, L // 2] = 3e38 * 5
+        want = torch.sort(key, dim=1, descending=True, stable=True).indices[:, :k].sort(dim=1).values
+        assert torch.equal(got, want), (kind, k)
