@@ -387,8 +387,10 @@ extern "C" int pk_gemv(const pk_tensor* weight, const pk_tensor* x, const pk_ten
   StageTimer timer(ST_GEMV, (cudaStream_t)stream);
   auto launch = [&](auto chunks) {
     constexpr int CH = decltype(chunks)::value;
-    launch_chain(gated ? gemv_kernel<true, CH> : gemv_kernel<false, CH>, dim3(grid), dim3(GV_THREADS), 0, (cudaStream_t)stream,
-                 (const uint16_t*)weight->data, (const uint16_t*)x->data, (uint16_t*)out->data, (int)n_out, (int)I, split.k_log, pdl_early());
+    const uint16_t *w = (const uint16_t*)weight->data, *in = (const uint16_t*)x->data;
+    uint16_t* y = (uint16_t*)out->data;
+    if (gated) launch_chain(gemv_kernel<true, CH>, dim3(grid), dim3(GV_THREADS), 0, (cudaStream_t)stream, w, in, y, (int)n_out, (int)I, split.k_log, pdl_early());
+    else launch_chain(gemv_kernel<false, CH>, dim3(grid), dim3(GV_THREADS), 0, (cudaStream_t)stream, w, in, y, (int)n_out, (int)I, split.k_log, pdl_early());
   };
   switch (split.chunks) {
     case 1: launch(std::integral_constant<int, 1>()); break;
