@@ -28,15 +28,16 @@ namespace {
 
 namespace cg = cooperative_groups;
 
+// Threads of a block: 512, or twice as many for long slices (see topk.cu).
 constexpr int SEL_THREADS = 512;
-constexpr int SEL_WARPS = SEL_THREADS / 32;
+constexpr int SEL_WARPS_MAX = 32;
 constexpr int SEL_WORDS = 256;   // words of a histogram: 512 bins of 16 bits for slices below 65536 elements, 256 of 32 bits for longer ones
 constexpr int SEL_SUB = 64;
 constexpr int SEL_TIES = 1024;
 constexpr int SEL_REGION = 2 * SEL_TIES * 8;   // bytes of dynamic shared memory
 // What the CTAs of a cluster write into each other, at the same offset of dynamic shared memory in every CTA and used by nothing
 // else: histograms [rank][SEL_WORDS], extremes [rank][warp].
-__host__ __device__ constexpr int sel_inbox_bytes(int cs) { return cs * (SEL_WORDS * 4 + SEL_WARPS * 8); }
+__host__ __device__ constexpr int sel_inbox_bytes(int cs, int threads = SEL_THREADS) { return cs * (SEL_WORDS * 4 + threads / 32 * 8); }
 
 // Rows of a type: the ordered key of an element, and the level-0 bins between the extremes of the row's keys.  A bin is
 // monotone in the key; sub() cuts a bin into SEL_SUB parts, monotone as well; single(): a bin holds one value.
@@ -86,7 +87,7 @@ struct SelShared {               // static: small block-wide results
   unsigned thr_key, thr_pos;     // the last element taken from the threshold bin
   unsigned lower_sel;            // elements taken from the threshold bin by lower ranks
   unsigned res[5];               // threshold bin, elements above it, elements in it, the same two of lower ranks
-  unsigned warp_a[SEL_WARPS], warp_b[SEL_WARPS];
+  unsigned warp_a[SEL_WARPS_MAX], warp_b[SEL_WARPS_MAX];
   unsigned sub[SEL_SUB], n_few;
 };
 
@@ -162,11 +163,11 @@ __device__ __forceinline__ void cluster_threshold(SelShared& s, const unsigned* 
 }
 
 // A warp's extremes into the inboxes of all CTAs.
-template <int CS>
+template <int CS, int WARPS>
 __device__ __forceinline__ void publish_range(cg::cluster_group& cluster, unsigned* inbox, unsigned rank, unsigned kmin, unsigned kmax) {
   uint2* extremes = reinterpret_cast<uint2*>(inbox + CS * SEL_WORDS);
   kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
-  put_by_lanes<CS>(cluster, extremes + rank * SEL_WARPS + (threadIdx.x >> 5), make_uint2(kmin, kmax), threadIdx.x & 31);
+  put_by_lanes<CS>(cluster, extremes + rank * WARPS + (threadIdx.x >> 5), make_uint2(kmin, kmax), threadIdx.x & 31);
 }
 
 // n: elements of this slice; at(i): raw 32 bits of element i; out_of(i): the 64-bit value to emit for it.
@@ -179,28 +180,28 @@ __device__ __forceinline__ void publish_range(cg::cluster_group& cluster, unsign
 // K (>= 1, at most the row's length), after a cluster barrier, none of them still using its region for anything else.
 // LISTED: the elements are listed in shared memory before out_of() is asked for them, all at once: for values that have to be
 // fetched from global memory.
-template <int CS, class V, bool LISTED, class At, class OutOf>
+template <int CS, class V, bool LISTED, int THREADS, class At, class OutOf>
 __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelShared& s, unsigned* region, unsigned* inbox,
                                                unsigned* words, int words_cap, unsigned rank, int n, int K, int64_t* __restrict__ out, At at,
                                                OutOf out_of, unsigned kmin, unsigned kmax, bool published = false) {
-  constexpr int BINS = V::BINS;
+  constexpr int BINS = V::BINS, WARPS = THREADS / 32;
   static_assert(BINS == SEL_WORDS || BINS == 2 * SEL_WORDS, "one word or half a word per bin");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned* hists = inbox;
   uint2* extremes = reinterpret_cast<uint2*>(inbox + CS * SEL_WORDS);
   auto exchange_range = [&](bool published) {   // extremes over the cluster, to kmin and kmax of every thread; clears the histogram replicas
-    for (int i = tid; i < 4 * BINS; i += SEL_THREADS) region[i] = 0;
+    for (int i = tid; i < 4 * BINS; i += THREADS) region[i] = 0;
     if (published) {
       if (CS > 1) cluster.barrier_wait();
       __syncthreads();
       kmin = 0xffffffffu, kmax = 0u;
     } else {
-      publish_range<CS>(cluster, inbox, rank, kmin, kmax);
+      publish_range<CS, WARPS>(cluster, inbox, rank, kmin, kmax);
       sync_cluster<CS>(cluster);
     }
 #pragma unroll
-    for (int i = 0; i < (CS * SEL_WARPS + 31) / 32; i++) {
-      const uint2 e = extremes[min(i * 32 + lane, CS * SEL_WARPS - 1)];
+    for (int i = 0; i < (CS * WARPS + 31) / 32; i++) {
+      const uint2 e = extremes[min(i * 32 + lane, CS * WARPS - 1)];
       kmin = min(kmin, e.x), kmax = max(kmax, e.y);
     }
     kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
@@ -228,7 +229,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   const typename V::Bins bins(kmin, kmax);
   auto bin0 = [&](uint32_t u) -> unsigned { return bins.of(u); };
 #pragma unroll 4
-  for (int i = tid; i < n; i += SEL_THREADS) atomicAdd(&my_hist[bin0(at(i))], 1u);
+  for (int i = tid; i < n; i += THREADS) atomicAdd(&my_hist[bin0(at(i))], 1u);
   exchange_hist();
   cluster_threshold<CS, BINS>(s, hists, rank, (unsigned)K);
   const unsigned T0 = s.res[0];
@@ -238,7 +239,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   while (in_bin > (unsigned)SEL_TIES && lo != hi) {
     kmin = 0xffffffffu, kmax = 0u;
 #pragma unroll 1
-    for (int i = tid; i < n; i += SEL_THREADS) {
+    for (int i = tid; i < n; i += THREADS) {
       const uint32_t u = at(i), k = V::key(u);
       if (bin0(u) == T0 && k >= lo && k <= hi) kmin = min(kmin, k), kmax = max(kmax, k);
     }
@@ -251,7 +252,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     }
     const int shift = max(0, (BINS == 512 ? 23 : 24) - __clz(top - base));   // (top - base) >> shift < BINS
 #pragma unroll 1
-    for (int i = tid; i < n; i += SEL_THREADS) {
+    for (int i = tid; i < n; i += THREADS) {
       const uint32_t u = at(i), k = V::key(u);
       if (bin0(u) == T0 && k >= base && k <= top) atomicAdd(&my_hist[(k - base) >> shift], 1u);
     }
@@ -289,7 +290,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   __syncthreads();
   if (kept || !flat) {
 #pragma unroll 2
-    for (int w = warp; w < n_words; w += SEL_WARPS) {   // a warp takes every 16th group of 32 elements
+    for (int w = warp; w < n_words; w += WARPS) {   // a warp takes every 16th group of 32 elements
       const int i = w * 32 + lane;
       bool above = false, member = false;
       const uint32_t u = at(min(i, n - 1));
@@ -308,7 +309,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   if (!flat) {
     sync_cluster<CS>(cluster);
     const unsigned before_me = pre_in, n_all = min(in_bin, (unsigned)SEL_TIES);
-    if (n_all <= SEL_THREADS / 4) {   // four lanes rank a member
+    if (n_all <= THREADS / 4) {   // four lanes rank a member
       const unsigned t = tid >> 2;
       const uint2 me = t < n_all ? all[t] : make_uint2(0u, 0u);
       unsigned rk = 0;
@@ -326,7 +327,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     } else {
       // the members' place within the threshold bin: ranks have to be counted out only in the sub-bin of the last one taken
       auto sub_of = [&](unsigned k) -> unsigned { return level0 ? bins.sub(k, T0) : 0u; };
-      for (unsigned t = tid; t < n_all; t += SEL_THREADS) atomicAdd(&s.sub[sub_of(all[t].x)], 1u);
+      for (unsigned t = tid; t < n_all; t += THREADS) atomicAdd(&s.sub[sub_of(all[t].x)], 1u);
       __syncthreads();
       if (warp == 0) {   // lane l: sub-bins 2l, 2l + 1
         const unsigned c0 = s.sub[2 * lane], c1 = s.sub[2 * lane + 1];
@@ -343,7 +344,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       __syncthreads();
       const unsigned S = s.res[0], need = rem - s.res[1];
       uint2* few = all + SEL_TIES;   // the sub-bin's elements; bit 31 of the position: held by a lower rank
-      for (unsigned t = tid; t < n_all; t += SEL_THREADS) {
+      for (unsigned t = tid; t < n_all; t += THREADS) {
         const uint2 m = all[t];
         const unsigned ms = sub_of(m.x);
         if (ms == S) few[atomicAdd(&s.n_few, 1u)] = make_uint2(m.x, m.y | (t < before_me ? 0x80000000u : 0u));
@@ -352,7 +353,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       __syncthreads();
       const unsigned n_few = s.n_few;
 #pragma unroll 1
-      for (unsigned t = warp; t < n_few; t += SEL_WARPS) {   // a warp ranks an element
+      for (unsigned t = warp; t < n_few; t += WARPS) {   // a warp ranks an element
         const uint2 me = few[t];
         const unsigned pos = me.y & 0x7fffffffu;
         unsigned rk = 0;
@@ -375,7 +376,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   auto taken = [&](unsigned k, unsigned pos) -> bool { return k > thr_key || (k == thr_key && pos <= thr_pos); };
   if (kept && !flat) {   // members that are taken join the elements above
     const unsigned m = min(s.n_members, (unsigned)SEL_TIES - min(pre_in, (unsigned)SEL_TIES));
-    for (unsigned t = tid; t < m; t += SEL_THREADS) {
+    for (unsigned t = tid; t < m; t += THREADS) {
       const uint2 me = own[t];
       const unsigned i = me.y & 0x07ffffffu;
       if (taken(me.x, me.y)) atomicOr(&above_w[i >> 5], 1u << (i & 31));
@@ -390,7 +391,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     const int nw = min(n_words - w0, words_cap);
     if (!kept) {
       __syncthreads();   // the words of the window before have been read
-      for (int w = warp; w < nw; w += SEL_WARPS) {
+      for (int w = warp; w < nw; w += WARPS) {
         const int i = (w0 + w) * 32 + lane;
         bool above = false, member = false;
         const uint32_t u = at(min(i, n - 1));
@@ -401,7 +402,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
       }
     }
     __syncthreads();
-    const int per = (nw + SEL_WARPS - 1) / SEL_WARPS;   // a warp's consecutive words
+    const int per = (nw + WARPS - 1) / WARPS;   // a warp's consecutive words
     const int a0 = min(nw, warp * per), a1 = min(nw, a0 + per);
     unsigned na = 0, nm = 0;
     for (int w = a0 + lane; w < a1; w += 32) na += __popc(above_w[w]), nm += __popc(member_w[w]);
@@ -410,7 +411,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
     __syncthreads();
     unsigned gw, ew;
     {
-      const unsigned x = lane < SEL_WARPS ? s.warp_a[lane] : 0u, y = lane < SEL_WARPS ? s.warp_b[lane] : 0u;
+      const unsigned x = lane < WARPS ? s.warp_a[lane] : 0u, y = lane < WARPS ? s.warp_b[lane] : 0u;
       gw = g + __reduce_add_sync(0xffffffffu, lane < warp ? x : 0u), ew = e + __reduce_add_sync(0xffffffffu, lane < warp ? y : 0u);
       g += __reduce_add_sync(0xffffffffu, x), e += __reduce_add_sync(0xffffffffu, y);
     }
@@ -448,7 +449,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   if (!LISTED) return;
   __syncthreads();
   const unsigned last = min((unsigned)K, g + min(e, room)), n_list = last > pos0 ? min(last - pos0, LIST) : 0u;
-  for (unsigned t = tid; t < n_list; t += SEL_THREADS) out[pos0 + t] = out_of(list[t]);
+  for (unsigned t = tid; t < n_list; t += THREADS) out[pos0 + t] = out_of(list[t]);
 }
 
 }  // namespace

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   auto publish = [&]() {
     if (published) return;
     published = true;
-    publish_range<CS>(cluster, inbox, rank, kmin, kmax);
+    publish_range<CS, CH_WARPS>(cluster, inbox, rank, kmin, kmax);
     if (CS > 1) cluster.barrier_arrive();
   };
   {
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
 
   // ---- final top-K over the cluster ----
   __syncthreads();   // the scores are complete; the level table and the histogram region are free
-  cluster_select<CS, F32Row<512>, false>(
+  cluster_select<CS, F32Row<512>, false, CH_THREADS>(
       cluster, s, region, inbox, lev2, FR_WORDS, rank, n_list, K_here, p.final_out + bh * p.K,
       [&](int i) -> uint32_t { return __float_as_uint(score_at(i)); }, [&](int i) -> int64_t { return id_at(i); }, kmin, kmax, true);
 }

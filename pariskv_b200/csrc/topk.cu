@@ -6,7 +6,9 @@
 // bisected levels and per-thread spans; one CTA per row up to 16384 elements) -> now: 8 rows of 32768 counts, k 4096
 // 16.7 -> 10.0; 8 rows of 4096 scores, k 256 9.6 -> 8.7.  The operators' nine launches, two of them these: 68.1 -> 65.2 us with
 // the exchanges by remote stores.  Rows read four elements a load, six loads in flight: 8 rows of 105K scores, the last launch of
-// a step with 1M keys, 114.2 -> 112.7 us a step.
+// a step with 1M keys, 114.2 -> 112.7 us a step.  Slices of 4096 elements and more take 1024 threads: that step 110.8 -> 107.4, the
+// operators over 8 x 131072 keys with 20000 candidates 151.5 -> 143.6, 32 x 50000 keys 266 -> 260, 8 x 60000 (slices of 6000) 89.4 ->
+// 87; shorter slices (8 x 32768 keys, 3300 a slice) lost 1 us to them, 1250 a slice 3.
 #include "cluster_select.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
@@ -16,7 +18,9 @@ namespace {
 
 constexpr int TK_WORDS = 1024;              // ballots kept per kind: slices of up to 32 K elements
 constexpr int TK_CACHE = 32 * TK_WORDS;     // elements of a slice kept in shared memory; longer ones are read again from L2
-__host__ __device__ constexpr int tk_fixed(int cs) { return SEL_REGION + 2 * TK_WORDS * 4 + sel_inbox_bytes(cs); }
+constexpr int TK_THREADS_LONG = 1024;       // threads of a block for slices of at least TK_LONG elements
+constexpr int TK_LONG = 4096;
+__host__ __device__ constexpr int tk_fixed(int cs, int threads) { return SEL_REGION + 2 * TK_WORDS * 4 + sel_inbox_bytes(cs, threads); }
 
 struct TopkParams {
   const uint32_t* in;
@@ -29,15 +33,15 @@ struct TopkParams {
   int cache;                 // elements of a slice kept in shared memory: all of them, or 0
 };
 
-template <int CS, template <int> class Row>
-__global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
+template <int CS, template <int> class Row, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS) topk_kernel(TopkParams p) {
   cg::cluster_group cluster = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ SelShared s;
   unsigned* region = reinterpret_cast<unsigned*>(dyn);
   unsigned* words = region + SEL_REGION / 4;
   unsigned* inbox = words + 2 * TK_WORDS;
-  uint32_t* cache = inbox + sel_inbox_bytes(CS) / 4;
+  uint32_t* cache = inbox + sel_inbox_bytes(CS, THREADS) / 4;
   const int tid = threadIdx.x;
   const unsigned rank = CS == 1 ? 0u : cluster.block_rank();
   const int64_t row = blockIdx.y;
@@ -60,26 +64,26 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
   if (cached && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {   // whole groups of four: up to six such loads in flight per thread
     const int groups = n >> 2;
     const uint4* in4 = reinterpret_cast<const uint4*>(in);
-    for (int base = tid; base < groups; base += 6 * SEL_THREADS) {
+    for (int base = tid; base < groups; base += 6 * THREADS) {
       uint4 u[6];
 #pragma unroll
-      for (int j = 0; j < 6; j++) u[j] = in4[min(base + j * SEL_THREADS, groups - 1)];
+      for (int j = 0; j < 6; j++) u[j] = in4[min(base + j * THREADS, groups - 1)];
 #pragma unroll
       for (int j = 0; j < 6; j++) {   // (past the end: the last group again, which changes nothing)
-        reinterpret_cast<uint4*>(cache)[min(base + j * SEL_THREADS, groups - 1)] = u[j];
+        reinterpret_cast<uint4*>(cache)[min(base + j * THREADS, groups - 1)] = u[j];
         const unsigned k0 = Row<512>::key(u[j].x), k1 = Row<512>::key(u[j].y), k2 = Row<512>::key(u[j].z), k3 = Row<512>::key(u[j].w);
         kmin = min(min(kmin, min(k0, k1)), min(k2, k3)), kmax = max(max(kmax, max(k0, k1)), max(k2, k3));
       }
     }
     done = groups * 4;
   }
-  for (int base = done + tid; base < n; base += 8 * SEL_THREADS) {   // eight loads in flight per thread
+  for (int base = done + tid; base < n; base += 8 * THREADS) {   // eight loads in flight per thread
     uint32_t u[8];
 #pragma unroll
-    for (int j = 0; j < 8; j++) u[j] = in[min(base + j * SEL_THREADS, n - 1)];
+    for (int j = 0; j < 8; j++) u[j] = in[min(base + j * THREADS, n - 1)];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      const int i = base + j * SEL_THREADS;
+      const int i = base + j * THREADS;
       if (i < n) {
         if (cached) cache[i] = u[j];
         const unsigned k = Row<512>::key(u[j]);
@@ -91,23 +95,23 @@ __global__ void __launch_bounds__(SEL_THREADS, 2) topk_kernel(TopkParams p) {
   const int64_t* map = p.map ? p.map + row * p.map_stride + begin : nullptr;
   auto out_of = [&](int i) -> int64_t { return map ? map[i] : begin + i; };
   if (cached)
-    cluster_select<CS, Row<512>, true>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
+    cluster_select<CS, Row<512>, true, THREADS>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
                             [&](int i) -> uint32_t { return cache[i]; }, out_of, kmin, kmax);
   else
-    cluster_select<CS, Row<256>, true>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
+    cluster_select<CS, Row<256>, true, THREADS>(cluster, s, region, inbox, words, TK_WORDS, rank, n, K, p.out + row * p.k,
                             [&](int i) -> uint32_t { return in[i]; }, out_of, kmin, kmax);
 }
 
-template <int CS, template <int> class Row>
+template <int CS, template <int> class Row, int THREADS>
 int topk_active() {   // clusters that fit the device at once; also opts in to the shared memory
-  auto kern = topk_kernel<CS, Row>;
-  const int smem = tk_fixed(CS) + TK_CACHE * 4;
+  auto kern = topk_kernel<CS, Row, THREADS>;
+  const int smem = tk_fixed(CS, THREADS) + TK_CACHE * 4;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return cudaGetLastError(), 0;
   if (CS > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
     return cudaGetLastError(), 0;
   if (CS == 1) return sm_count();
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CS, 64), cfg.blockDim = dim3(SEL_THREADS), cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.gridDim = dim3(CS, 64), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = (size_t)smem;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = CS, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
@@ -127,16 +131,19 @@ const TopkCapacity* topk_capacity() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
   if (const unsigned long long bit = first_on_device(asked)) {
     for (int i = 0; i < N_CLUSTER_SIZES; i++)   // several threads may ask at the same time: they write the same numbers
-      with_cluster_size(CLUSTER_SIZES[i], [&](auto cs) { cap[dev].active[i] = topk_active<cs.value, Row>(); });
+      with_cluster_size(CLUSTER_SIZES[i], [&](auto cs) {
+        const int a = topk_active<cs.value, Row, SEL_THREADS>(), b = topk_active<cs.value, Row, TK_THREADS_LONG>();
+        cap[dev].active[i] = a < b ? a : b;
+      });
     mark_on_device(asked, bit);
   }
   return &cap[dev];
 }
 
-template <int CS, template <int> class Row>
+template <int CS, template <int> class Row, int THREADS>
 cudaError_t launch_topk_cs(int64_t rows, size_t smem, cudaStream_t st, const TopkParams& p) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(CS, (unsigned)rows), cfg.blockDim = dim3(SEL_THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+  cfg.gridDim = dim3(CS, (unsigned)rows), cfg.blockDim = dim3(THREADS), cfg.dynamicSmemBytes = smem, cfg.stream = st;
   cudaLaunchAttribute attr[2];
   int n = 0;
   if (CS > 1) {
@@ -150,7 +157,7 @@ cudaError_t launch_topk_cs(int64_t rows, size_t smem, cudaStream_t st, const Top
     n++;
   }
   cfg.attrs = attr, cfg.numAttrs = n;
-  return cudaLaunchKernelEx(&cfg, topk_kernel<CS, Row>, p);
+  return cudaLaunchKernelEx(&cfg, topk_kernel<CS, Row, THREADS>, p);
 }
 
 template <template <int> class Row>
@@ -169,7 +176,8 @@ int launch_rows(TopkParams p, int64_t rows, cudaStream_t st) {
   const int64_t slice = ((p.L + best - 1) / best + 31) / 32 * 32;
   if (slice >= (1LL << 27)) return fail(PK_ERR_ARG, "topk: row too long");
   p.cache = slice <= TK_CACHE ? (int)slice : 0;
-  const size_t smem = tk_fixed(best) + (size_t)p.cache * 4;
+  const bool is_long = slice >= TK_LONG;
+  const size_t smem = tk_fixed(best, is_long ? TK_THREADS_LONG : SEL_THREADS) + (size_t)p.cache * 4;
   for (int64_t r0 = 0; r0 < rows; r0 += 65535) {   // grid.y limit
     TopkParams q = p;
     const int64_t nr = rows - r0 < 65535 ? rows - r0 : 65535;
@@ -178,7 +186,9 @@ int launch_rows(TopkParams p, int64_t rows, cudaStream_t st) {
     if (q.n_dev) q.n_dev += r0;
     if (q.n_out) q.n_out += r0;
     cudaError_t e = cudaErrorInvalidValue;
-    with_cluster_size(best, [&](auto c) { e = launch_topk_cs<c.value, Row>(nr, smem, st, q); });
+    with_cluster_size(best, [&](auto c) {
+      e = is_long ? launch_topk_cs<c.value, Row, TK_THREADS_LONG>(nr, smem, st, q) : launch_topk_cs<c.value, Row, SEL_THREADS>(nr, smem, st, q);
+    });
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(PK_ERR_CUDA, "topk: %s", cudaGetErrorString(e));

@@ -787,8 +787,9 @@ def test_gemv_splits_against_fp64(ops, O, I):
 
 
 # Slices of the most elements that are kept in shared memory (16-bit counts of 512 bins; all of them in one bin, or nearly) and one
-# group more (32-bit counts of 256 bins), on the largest cluster and on one CTA.
-@pytest.mark.parametrize("rows,L", [(1, 16 * 32768), (1, 16 * 32768 + 1), (150, 32768), (150, 32769), (3, 16 * 511), (2, 5000)])
+# group more (32-bit counts of 256 bins), on the largest cluster and on one CTA; slices around 4096 (512 and 1024 threads).
+@pytest.mark.parametrize("rows,L", [(1, 16 * 32768), (1, 16 * 32768 + 1), (150, 32768), (150, 32769), (3, 16 * 511), (2, 5000), (1, 16 * 4064),
+                                    (1, 16 * 4064 + 1), (150, 4064), (150, 4065)])
 @pytest.mark.parametrize("kind", ["equal", "two values", "one off", "wide ints", "floats", "floats with inf and nan"])
 def test_topk_bins_at_the_edges_of_a_slice(ops, rows, L, kind):
     g = torch.Generator(device=DEV).manual_seed(L + rows)
