@@ -54,7 +54,7 @@ struct AttParams {
   const int32_t* n_sel;   // [bs*H] or null
   int64_t K, index_offset;
   int H, Hq, G, n_qgroups;
-  int tiles_per_block;    // consecutive tiles of a (batch, KV head) that one block streams; the grid has ceil(tiles / it) groups
+  int tiles_per_block;    // consecutive tiles of a (batch, KV head) that one block streams at most; the grid has ceil(tiles / it) groups
   float scale_log2;
   unsigned* counters;     // [bs*H] arrival counters, zero between calls
   int* status;            // set to 1 if a copy barrier was never completed
@@ -169,8 +169,8 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
   const int tid = threadIdx.x;
   const int h = blockIdx.y, b = blockIdx.z;
   const int64_t bh = (int64_t)b * p.H + h;
-  const int n_groups = (int)gridDim.x, tpb = p.tiles_per_block;
-  const int t_first = (int)blockIdx.x * tpb;
+  const int n_groups = (int)gridDim.x;
+  int tpb = p.tiles_per_block, t_first = (int)blockIdx.x * tpb;
   const unsigned mb0 = (unsigned)__cvta_generic_to_shared(&mbar[0]);
   if (tid == 0) {
 #pragma unroll
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
   __syncthreads();
   // index of this thread's row of tile t: loaded a tile ahead of the copy that needs it, the first with the row counts
   auto index_of = [&](int t) -> int64_t {
-    const int64_t r = (int64_t)t * TILE + (tid >> 1);
+    const int r = t * TILE + (tid >> 1);
     return r < p.K ? p.sel[b * p.sel_b + h * p.sel_h + r] : 0;
   };
   pdl_wait();  // the selected indices and the per-head row counts come from the kernels before this one
@@ -190,16 +190,27 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
   if (CLUSTER)
 #pragma unroll
     for (int i = 0; i < ATT_HEAD_BUFS - 1; i++) later[i] = i + 1 < tpb ? index_of(t_first + i + 1) : 0;
-  const int64_t n_sel = p.n_sel ? min((int64_t)p.n_sel[bh], p.K) : p.K;
-  const int64_t n_window =
-      p.n_window_dev ? min(p.n_window, max((int64_t)0, (int64_t)p.n_window_dev[0] + p.n_window_add)) : p.n_window;
-  const int64_t n_rows = n_window + n_sel;
+  const int n_sel = (int)(p.n_sel ? min((int64_t)p.n_sel[bh], p.K) : p.K);   // (a call has at most 65536 rows)
+  const int n_window = (int)(p.n_window_dev ? min(p.n_window, max((int64_t)0, (int64_t)p.n_window_dev[0] + p.n_window_add)) : p.n_window);
+  const int n_rows = n_window + n_sel;
+  // The launch is sized for the most rows there can be; where a block's share of those that there are is a tile less, they are
+  // spread evenly over all blocks of the head.  (The indices are then asked for again: their first read was for another tile.)
+  // Adaptive budgets select 1024 of the 4096 rows that a launch has room for: two of six blocks a head had all the work.  B200, a
+  // step of two layers: 8 sequences 126.8 -> 122.2 us, 16 of two KV heads 136.7 -> 125.5, one sequence 100.0 -> 91.5.
+  if ((n_rows + TILE - 1) / TILE <= (tpb - 1) * n_groups) {
+    tpb = max(1, (int)((unsigned)((n_rows + TILE - 1) / TILE + n_groups - 1) / (unsigned)n_groups));
+    t_first = (int)blockIdx.x * tpb;
+    ahead = index_of(t_first);
+    if (CLUSTER)
+#pragma unroll
+      for (int i = 0; i < ATT_HEAD_BUFS - 1; i++) later[i] = i + 1 < tpb ? index_of(t_first + i + 1) : 0;
+  }
 
   // ---- stage a tile: thread t copies row t/2, K for even t and V for odd t; where the store keeps the V row of a
   // key right behind its K row, the even thread fetches both with one 512-byte copy (half as many requests on the
   // host link).  Every thread arrives on the tile's barrier exactly once, the copying ones with their byte count ----
   auto tile_rows = [&](int t) -> int {
-    return (int)max((int64_t)0, min((int64_t)TILE, n_rows - (int64_t)t * TILE));
+    return max(0, min(TILE, n_rows - t * TILE));
   };
   auto issue = [&](int t, int buf) {
     const int i = tid >> 1;
@@ -207,7 +218,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
     const uint16_t* src = nullptr;
     bool ok = i < tile_rows(t), paired = false;
     if (ok) {
-      const int64_t r = (int64_t)t * TILE + i;
+      const int r = t * TILE + i;
       if (r >= n_sel) {
         src = (is_v ? p.wv : p.wk) + b * p.w_b + h * p.w_h + (r - n_sel) * p.w_l;
       } else {

@@ -814,3 +814,33 @@ def test_topk_bins_at_the_edges_of_a_slice(ops, rows, L, kind):
             key[:, L // 2] = 3e38 * 5
         want = torch.sort(key, dim=1, descending=True, stable=True).indices[:, :k].sort(dim=1).values
         assert torch.equal(got, want), (kind, k)
+
+
+# Fewer selected rows than the launch is sized for, in the streaming, the cluster and the one-tile form: a head's rows are spread
+# anew over its blocks, at counts around the edges of their shares.
+@pytest.mark.parametrize("bs,H,G,K,n_window", [(8, 8, 4, 4000, 70), (16, 8, 2, 2048, 132), (1, 8, 4, 4096, 20), (3, 2, 5, 2000, 0), (2, 8, 8, 900, 200), (1, 2, 12, 700, 33)])
+@pytest.mark.parametrize("on_device", [False, True])
+def test_attention_spreads_the_rows_that_there_are(ops, bs, H, G, K, n_window, on_device):
+    g = torch.Generator(device=DEV).manual_seed(K)
+    cap, cap_w = K + 500, n_window + 50
+    q = torch.randn(bs, 1, H * G, 128, generator=g, device=DEV).to(torch.bfloat16)
+    wk, wv = (torch.randn(bs, H, cap_w, 128, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+    store = torch.randn(bs, H, cap, 2, 128, generator=g, device=DEV).to(torch.bfloat16)
+    sel = torch.rand(bs, H, cap, generator=g, device=DEV).argsort(-1)[..., :K].sort(-1).values.contiguous()
+    edges = [0, 1, 63, 64, 65, 127, 128, 129, 191, 192, 193, 250, 384, 500, 640, 641, 767, 768, 769, K - 64, K - 1, K]
+    n_sel = torch.tensor([max(0, min(K, edges[i % len(edges)])) for i in range(bs * H)], dtype=torch.int32, device=DEV).view(bs, H)
+    rows_dev = torch.tensor([n_window - 3], dtype=torch.int32, device=DEV)
+    more = dict(n_window_dev=rows_dev, n_window_add=3) if on_device else {}
+    out = ops.sparse_attention(q, wk, wv, cap_w if on_device else n_window, store[..., 0, :], store[..., 1, :], sel, n_sel=n_sel, **more)
+    for b in range(bs):
+        for h in range(H):
+            idx = sel[b, h, :int(n_sel[b, h])]
+            k = torch.cat([store[b, h, idx, 0], wk[b, h, :n_window]]).double()
+            v = torch.cat([store[b, h, idx, 1], wv[b, h, :n_window]]).double()
+            got = out[b, 0, h * G:(h + 1) * G].double()
+            if k.shape[0] == 0:
+                assert not got.any()
+                continue
+            p = torch.softmax(q[b, 0, h * G:(h + 1) * G].double() @ k.t() / 128 ** 0.5, -1)
+            # fp32 sums and probabilities of 17 bits, then one rounding to bf16: 2^-9 of the value, 2^-14 of the weighted magnitudes
+            assert ((got - p @ v).abs() <= 2.0 ** -8 * (p @ v).abs() + 2.0 ** -14 * (p @ v.abs())).all()
