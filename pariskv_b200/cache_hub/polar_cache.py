@@ -162,7 +162,8 @@ class polar_cache(KV_Cache):
         self.current_seq_len = [0] * layer_num      # tokens seen per layer (longest sample)
         self._window_len = [0] * layer_num          # valid rows of the window per layer
         self._sample_window = [[0] * bs for _ in range(layer_num)]   # the same, per sample, while prefill is under way
-        self._all_rows = None
+        self._all_rows = self._zone_rows = None     # index rows of full attention: all of a zone's, the first _all_rows_n
+        self._all_rows_n = 0
         self.device_positions = True                # positions are always read on the device (kept for callers that ask)
         self.context = 0
         self.last_topk_indices = None               # [bs,H,K] of the most recent compute (for inspection)
@@ -339,7 +340,8 @@ class polar_cache(KV_Cache):
         l = layer_idx
         if self._window_len[l] + 1 == self.window_capacity and max(self.zone_len[l]) + self.dynamic_update_interval > self.zone_capacity:
             raise RuntimeError("zone store is full: construct the cache with a larger max_length / max_new_length")
-        self._wait_offload(l)      # the flush writes store rows: stay ordered behind a pending bulk offload
+        if self._offload_event[l] is not None:
+            self._wait_offload(l)  # the flush writes store rows: stay ordered behind a pending bulk offload
         _lib.native().append_encode(
             key_states, value_states, self.srht_diagonal_signs, self.unified_keys_gpu[l], self.unified_values_gpu[l],
             self._win_codes[l], self._win_weight[l], self._win_4bit[l], self._win_vnorm[l], self.codebook_gpu[l],
@@ -388,7 +390,7 @@ class polar_cache(KV_Cache):
     def _full_regime(self, layer_idx):
         """True while the sequence is short enough to attend every zone row (cache_hub/polar_cache.py:1033-1045)."""
         total = self.current_seq_len[layer_idx]
-        return total < max(self.FULL_ATTENTION_THRESHOLD, self.steady_size + 2 * self.final_topk) or self.cpu_valid_end[layer_idx] <= 0
+        return total < self.FULL_ATTENTION_THRESHOLD or total < self.steady_size + 2 * self.final_topk or self.cpu_valid_end[layer_idx] <= 0
 
     def graph_key(self):
         """What a captured decode step depends on besides the device words: which of the two attention regimes the
@@ -397,9 +399,11 @@ class polar_cache(KV_Cache):
 
     def compute(self, queries, layer_idx):
         """Decode attention of one token: queries [bs, 1, num_heads, 128] -> [bs, 1, num_heads, 128]."""
-        queries = queries.contiguous()
-        self._wait_offload(layer_idx)
+        if not queries.is_contiguous():
+            queries = queries.contiguous()
         l = layer_idx
+        if self._offload_event[l] is not None:
+            self._wait_offload(l)
         wk, wv = self.unified_keys_gpu[l], self.unified_values_gpu[l]
         sk, sv = self._store_k[l], self._store_v[l]
         if self._full_regime(l):  # attend everything (eager only: the row count is a host number)
@@ -409,12 +413,15 @@ class polar_cache(KV_Cache):
             if N <= 0:
                 return self._attend(queries, wk, wv, n_win)
             # rows 0 .. N-1 of every head: a view of one index row, made again only when the zone has grown
-            if self._all_rows is None:
-                self._all_rows = torch.arange(self.zone_capacity, device=self.device).expand(self.batch_size, self.kv_head, -1)
-                self._all_rows_n = None
-            if self._all_rows_n is None or self._all_rows_n.shape[2] != N:
-                self._all_rows_n = self._all_rows[:, :, :N]
-            return self._attend(queries, wk, wv, n_win, sk, sv, self._all_rows_n)
+            if N != self._all_rows_n:
+                if self._all_rows is None:
+                    self._all_rows = torch.arange(self.zone_capacity, device=self.device).expand(self.batch_size, self.kv_head, -1)
+                self._zone_rows, self._all_rows_n = self._all_rows[:, :, :N], N
+            if n_win + N > self._attn_rows_max:
+                return self._attend(queries, wk, wv, n_win, sk, sv, self._zone_rows)
+            # A short sequence is bound by the host: no calls and no tensor shapes that this does not need.
+            return _lib.native().sparse_attention(queries, wk, wv, n_win, None, 0, sk, sv, self._zone_rows, None, 0, self._softmax_scale,
+                                                  None, None, self._attn_scratch.buf)
         if self.per_query_head_retrieval:
             return self._compute_per_query_head(queries, l)
         # A caller whose queries are made BEFORE it calls decode_update_kv_cache (one kernel makes q and k) says so with
