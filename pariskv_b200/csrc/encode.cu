@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
 // Tiles of zone rows come by TMA into one of two stages of shared memory and go to the store from there, K and V, four
 // instructions of one thread each way; the warps only read the keys, lane l of a warp 32 dimensions (quarter l / 8) of its key
 // l % 8, so that with the copies' 128-byte swizzle the eight lanes of a quarter-warp read fall into eight different groups of
-// four banks.  Other tiles (window rows; every row where the tensors cannot be described to the TMA unit) are loaded and
-// stored row by row.
+// four banks.  Other tiles (window rows; every row of a short prompt, or where the tensors cannot be described to the TMA unit) are
+// loaded and stored row by row.
 // What bounds it: issue slots of the coding, 70 - 75 % of them taken (integer ALU 60 %, DRAM 67 - 80 %), with 24 warps per SM.
 // 131072 tokens x 8 heads on B200: 2003 us as coding, interleaving and copy launches; 271 as one launch that carried the rows
 // through registers, 126 of them, 16 warps per SM; 226 as this one: 5.3 TB/s of 1136 bytes per key.  A block's tiles are an even
@@ -149,6 +149,7 @@ constexpr int PF_HALF = PF_TILE * 128;            // bytes of 64 dimensions of a
 constexpr int PF_STAGE = 4 * PF_HALF;             // K, V; two halves each
 constexpr int PF_HIST = 16 * 256 * 4;
 constexpr int PF_SMEM = 2 * PF_STAGE + PF_HIST + 256 + 32;
+constexpr int64_t PF_TMA_KEYS = 16 * 1024;        // keys of a prompt (over all heads) above which its rows come by TMA
 constexpr int PF_WAIT_LIMIT = 4000000;            // polls of a barrier before giving up
 
 __device__ __forceinline__ bool pf_wait(unsigned mbar, unsigned parity) {
@@ -808,7 +809,10 @@ extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const p
   p.P = P, p.N = N, p.cap_z = c.cap_z;
   if (N > 0) p.store = (uint16_t*)rows->data, p.store_cap = H == 1 ? rows->shape[1] : rows->stride[0] / 256;
   p.H = (int)H, p.cap_w = (int)c.cap_w, p.sink = (int)sink, p.n_window = (int)(N > 0 ? sink + local : P), p.b = (int)b;
-  p.tma = N > 0 && prefill_maps(p);
+  // Describing the tensors costs the host 1 - 1.5 us; shorter prompts take the device much less time than the host and go row by row
+  // (B200, us a call, row by row | by TMA: four samples of 1000 tokens x 8 heads 86 | 92, 6000 x 8 heads 33.2 | 34.5, where only host
+  // time shows; two layers of two samples of 2477 and 3001 tokens to host memory 843 | 836, 16000 x 8 heads 50 | 43).
+  p.tma = N * H > PF_TMA_KEYS && prefill_maps(p);
   p.zone_tiles = p.tma ? (N + PF_TILE - 1) / PF_TILE : 0;
   p.n_tiles = p.zone_tiles + ((p.tma ? p.n_window : P) + PF_TILE - 1) / PF_TILE;
   // one wave of two blocks per SM, an even share of the tiles for each

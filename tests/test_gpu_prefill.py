@@ -88,11 +88,13 @@ def _prompt(g, layout, bs, P, H):
     return [rows(kind) for kind in (("tokens", "heads") if layout == "mixed" else (layout, layout))]
 
 
-# Zone rows around the edges of a tile of 96, windows of one tile and of two, one tile per block and several (both stages in turn).
+# Row by row (up to 16384 keys): zone rows around the edges of a tile of 96, windows of one tile and of two.  By TMA: the same edges,
+# one tile per block and several (both stages in turn), every layout; K and V in different orders and expanded heads go row by row.
 @pytest.mark.parametrize("P,H,local,layout", [
     (115, 3, 16, "tokens"), (116, 3, 16, "heads"), (117, 3, 16, "mixed"), (211, 2, 16, "slice"), (213, 2, 16, "expanded"),
-    (228, 1, 128, "tokens"), (229, 2, 128, "heads"), (95, 2, 91, "tokens"), (96, 2, 91, "tokens"), (5001, 8, 64, "expanded"),
-    (90001, 1, 64, "slice"), (12900, 5, 100, "heads"), (40000, 2, 64, "tokens")])
+    (228, 1, 128, "tokens"), (95, 2, 91, "tokens"), (96, 2, 91, "tokens"), (2048 + 20, 8, 16, "tokens"),
+    (2049 + 20, 8, 16, "tokens"), (8255 + 20, 8, 16, "heads"), (8256 + 20, 8, 16, "slice"), (8257 + 20, 8, 16, "tokens"),
+    (9001, 8, 64, "expanded"), (9000, 8, 300, "mixed"), (90001, 1, 64, "slice"), (13900, 5, 100, "heads"), (40000, 2, 128, "tokens")])
 def test_prefill_tiles_match_oracle(oracle, P, H, local, layout):
     from pariskv_b200.cache_hub.polar_cache_adaptivek_varlen import polar_cache
     sink, bs = 4, 1
