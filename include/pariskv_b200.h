@@ -104,8 +104,8 @@ int pk_encode_keys(const pk_tensor* keys, const pk_tensor* signs, const pk_tenso
  *   cluster_counts i32 [bs,H,16,256] contiguous; row b is overwritten
  *   rows           bf16 [H,n >= N,2,128], last two dims contiguous, device memory: where zone rows go (row b of the store,
  *                  or a buffer that the caller copies to a host store: pk_copy_rows)
- *   state          i32 [4 + bs]: state[0] = window rows, state[1..3] = 0, state[4 + b] = zone rows; state[3] = 1 if copies of
- *                  the rows never completed
+ *   state          i32 [4 + bs]: state[0] = window rows, state[1..2] = 0, state[4 + b] = zone rows; state[3] = 1 if copies of
+ *                  the rows never completed.  Only sample 0 clears state[3]: what an earlier sample reported stays
  * With N = max(0, P - sink - local): tokens [sink, sink + N) become zone rows 0 .. N - 1, the first `sink` and the last
  * `local` tokens window rows (every token where N == 0; P must then fit the window). */
 int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const pk_tensor* signs, const pk_tensor* window_k,

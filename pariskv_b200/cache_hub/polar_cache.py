@@ -271,7 +271,7 @@ class polar_cache(KV_Cache):
                 self.sink_size, self.local_size)
         else:
             self.cluster_key_counts_gpu[layer][b].zero_()
-            self._layer_state[layer][:4].zero_()
+            self._layer_state[layer][:3 if b else 4].zero_()   # (the error word is sample 0's to clear)
             self._layer_state[layer][4 + b] = 0
         if staged:
             self._offload_rows(layer, b, rows, N, slot)

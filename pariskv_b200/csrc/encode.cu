@@ -152,6 +152,14 @@ constexpr int PF_SMEM = 2 * PF_STAGE + PF_HIST + 256 + 32;
 constexpr int64_t PF_TMA_KEYS = 16 * 1024;        // keys of a prompt (over all heads) above which its rows come by TMA
 constexpr int PF_WAIT_LIMIT = 4000000;            // polls of a barrier before giving up
 
+// Ahead of a prompt: its histogram, and with a layer's first sample the error word that all samples share.  A launch of its own,
+// so that the word is clear before any block may set it; with a later sample it would take the report of an earlier one away.
+// In the place of a memset of the histogram, and as fast.
+__global__ void __launch_bounds__(1024) prefill_clear_kernel(int32_t* counts, int32_t* error) {
+  counts[(int64_t)blockIdx.x * 1024 + threadIdx.x] = 0;
+  if (error && blockIdx.x == 0 && threadIdx.x == 0) *error = 0;
+}
+
 __device__ __forceinline__ bool pf_wait(unsigned mbar, unsigned parity) {
   unsigned done = 0;
   for (int it = 0; it < PF_WAIT_LIMIT && !done; it++)
@@ -186,7 +194,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_con
   for (int i = tid; i < 16 * 256; i += PF_THREADS) hist[i] = 0;
   if (tid < 64) masks[tid] = reinterpret_cast<const uint32_t*>(p.signs)[tid] & 0x80008000u;
   if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) {
-    p.state[0] = p.n_window, p.state[1] = 0, p.state[2] = 0, p.state[3] = 0;
+    p.state[0] = p.n_window, p.state[1] = 0, p.state[2] = 0;   // (state[3]: see prefill_clear_kernel)
     p.state[4 + p.b] = (int32_t)p.N;
   }
   __syncthreads();
@@ -824,7 +832,8 @@ extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const p
     if (cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM) != cudaSuccess) return check_launch("prefill smem", 0);
     mark_on_device(smem_attr, bit);
   }
-  if (cudaMemsetAsync(p.counts, 0, (size_t)(H * 16 * 256 * 4), st) != cudaSuccess) return check_launch("prefill memset", 0);
+  prefill_clear_kernel<<<(unsigned)(H * 4), 1024, 0, st>>>(p.counts, b == 0 ? p.state + 3 : nullptr);
+  if (const int rc_clear = check_launch("prefill clear")) return rc_clear;
   StageTimer tm(ST_ENCODE, st);
   prefill_kernel<<<dim3((unsigned)H, (unsigned)((p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block)), PF_THREADS, PF_SMEM, st>>>(p);
   return check_launch("prefill");

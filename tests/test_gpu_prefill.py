@@ -125,3 +125,26 @@ def test_prefill_tiles_match_oracle(oracle, P, H, local, layout):
     assert torch.equal(cache.cluster_key_counts_gpu[0].cpu(), counts)
     if N:   # rows behind the zone's end are untouched
         assert not cache._store_kv[0][:, :, N:].any() and not cache.codebook_gpu[0][..., N:].any()
+
+
+@pytest.mark.parametrize("P", [700, 9000])     # row by row; by TMA
+@pytest.mark.parametrize("empty", [False, True])
+def test_report_of_one_sample_outlives_the_next(P, empty):
+    """All samples of a layer share one error word: the host sets it, as sample 0 would, and sample 1 leaves it alone, a sample
+    without tokens too.  A new prompt for sample 0 starts clean."""
+    from pariskv_b200.cache_hub.polar_cache import polar_cache
+    g = torch.Generator().manual_seed(P)
+    k, v = _prompt(g, "tokens", 1, P, 2)
+    cache = polar_cache(valid_start=0, layer_num=2, batch_size=2, max_length=P + 32, num_key_value_heads=2, num_heads=2, head_dim=128,
+                        dtype=torch.bfloat16, layer_mapping={"0": DEV, "1": DEV}, max_new_length=32, sink_size=4, local_size=16,
+                        final_topk=16, dynamic_update_interval=8, enable_offload=False)
+    cache._prefill_sample(k[0], v[0], 1, 0, 0)
+    cache.check_status()
+    cache._layer_state[1][3] = 1
+    cache._prefill_sample(k[0], v[0], 1, 1, P if empty else 0)
+    with pytest.raises(RuntimeError, match=r"layers \[1\]"):
+        cache.check_status()
+    cache._prefill_sample(k[0], v[0], 1, 0, P if empty else 0)
+    cache.check_status()
+    cache._prefill_sample(k[0], v[0], 1, 1, 0)
+    cache.check_status()
