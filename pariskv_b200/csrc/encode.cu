@@ -104,21 +104,22 @@ __global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
 // store (K row and V row of a key next to each other), its key is coded into the staging arrays or the zone records, ||v||
 // and the cluster histogram come with it.  A head's tokens are cut into tiles of 96, the zone rows first and the window
 // rows behind them; a block takes consecutive tiles, the heads of a token range side by side in the grid, since they are
-// neighbours in memory.
+// neighbours in memory (prefill_kernel; short prompts, and those that cannot be described to the TMA unit: prefill_rows_kernel).
 // Tiles of zone rows come by TMA into one of two stages of shared memory and go to the store from there, K and V, four
 // instructions of one thread each way; the warps only read the keys, lane l of a warp 32 dimensions (quarter l / 8) of its key
 // l % 8, so that with the copies' 128-byte swizzle the eight lanes of a quarter-warp read fall into eight different groups of
-// four banks.  Other tiles (window rows; every row of a short prompt, or where the tensors cannot be described to the TMA unit) are
-// loaded and stored row by row.
+// four banks.  Window rows are loaded and stored row by row.
 // What bounds it: issue slots of the coding, 70 - 75 % of them taken (integer ALU 60 %, DRAM 67 - 80 %), with 24 warps per SM.
-// 131072 tokens x 8 heads on B200: 2003 us as coding, interleaving and copy launches; 271 as one launch that carried the rows
-// through registers, 126 of them, 16 warps per SM; 226 as this one: 5.3 TB/s of 1136 bytes per key.  A block's tiles are an even
+// 131072 tokens x 8 heads on B200: 2003 us as coding, interleaving and copy launches; 262 as one launch that carries the rows
+// through registers, 16 warps per SM (prefill_rows_kernel); 211 as this one: 5.6 TB/s of 1136 bytes per key.  A block's tiles are an even
 // share of one wave: two waves of half the size take 229.  (Single rows by bulk copies took 450: the copy engine takes a row
 // per instruction no faster than a tile.)
+struct PrefillMaps {
+  CUtensorMap k, v;         // [P][H][128] by 64 dimensions x 1 head x 96 tokens
+  CUtensorMap store;        // [H][N][256] by 64 x 96 rows x 1 head
+  int heads_inner;          // the heads are the middle dimension of k and v, not the outer one
+};
 struct PrefillParams {
-  CUtensorMap map_k, map_v; // [P][H][128] by 64 dimensions x 1 head x 96 tokens
-  CUtensorMap map_store;    // [H][N][256] by 64 x 96 rows x 1 head
-  int tma, heads_inner;     // the maps are there; the heads are the middle dimension of map_k and map_v, not the outer one
   const uint16_t* k;        // [P][H][128] of one sample
   const uint16_t* v;
   int64_t k_l, k_h, v_l, v_h;
@@ -139,7 +140,8 @@ struct PrefillParams {
   uint16_t* store;          // [H][store_cap][2][128]
   int32_t* state;           // the layer's words
   int64_t P, N, cap_z, store_cap;
-  int64_t zone_tiles, n_tiles, tiles_per_block;   // tiles of a head: those by TMA, all
+  int64_t zone_tiles, n_tiles, tiles_per_block;   // prefill_kernel: tiles of a head, those of zone rows and all
+  int64_t chunk;                                  // prefill_rows_kernel: tokens of a block
   int H, cap_w, sink, n_window, b;
 };
 
@@ -154,7 +156,8 @@ constexpr int PF_WAIT_LIMIT = 4000000;            // polls of a barrier before g
 
 // Ahead of a prompt: its histogram, and with a layer's first sample the error word that all samples share.  A launch of its own,
 // so that the word is clear before any block may set it; with a later sample it would take the report of an earlier one away.
-// In the place of a memset of the histogram, and as fast.
+// In the place of a memset of the histogram, and 0.15 us faster; it costs the host 0.6 us more, so that prefill_rows_kernel, which
+// reports nothing, clears the word itself behind a memset.
 __global__ void __launch_bounds__(1024) prefill_clear_kernel(int32_t* counts, int32_t* error) {
   counts[(int64_t)blockIdx.x * 1024 + threadIdx.x] = 0;
   if (error && blockIdx.x == 0 && threadIdx.x == 0) *error = 0;
@@ -173,7 +176,7 @@ __device__ __forceinline__ bool pf_wait(unsigned mbar, unsigned parity) {
   return done != 0;
 }
 
-__global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_constant__ PrefillParams p) {
+__global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_constant__ PrefillMaps m) {
   extern __shared__ __align__(1024) unsigned char pf_smem[];   // (no static shared memory: the stages start on 1024 bytes)
   int* hist = reinterpret_cast<int*>(pf_smem + 2 * PF_STAGE);
   uint32_t* masks = reinterpret_cast<uint32_t*>(pf_smem + 2 * PF_STAGE + PF_HIST);
@@ -200,13 +203,13 @@ __global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_con
   __syncthreads();
   auto load_tile = [&](int j) {   // (thread 0)
     const unsigned dst = smem0 + (j & 1) * PF_STAGE, bar = full0 + 8 * (j & 1);
-    const int t = (int)(p.sink + (first + j) * PF_TILE), c1 = p.heads_inner ? h : t, c2 = p.heads_inner ? t : h;
+    const int t = (int)(p.sink + (first + j) * PF_TILE), c1 = m.heads_inner ? h : t, c2 = m.heads_inner ? t : h;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(PF_STAGE) : "memory");
 #pragma unroll
     for (int i = 0; i < 4; i++)
       asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
                        dst + i * PF_HALF),
-                   "l"(i < 2 ? &p.map_k : &p.map_v), "r"((i & 1) * 64), "r"(c1), "r"(c2), "r"(bar)
+                   "l"(i < 2 ? &m.k : &m.v), "r"((i & 1) * 64), "r"(c1), "r"(c2), "r"(bar)
                    : "memory");
   };
   auto store_tile = [&](int j) {   // (thread 0)
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_con
     const int z = (int)((first + j) * PF_TILE);
 #pragma unroll
     for (int i = 0; i < 4; i++)
-      asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(&p.map_store), "r"(i * 64), "r"(z),
+      asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(&m.store), "r"(i * 64), "r"(z),
                    "r"(h), "r"(src + i * PF_HALF)
                    : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
@@ -250,16 +253,16 @@ __global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_con
                      : "=r"(key[i].x), "=r"(key[i].y), "=r"(key[i].z), "=r"(key[i].w)
                      : "r"(at + ((((s & 1) * 4 + i) ^ (lane & 7)) << 4)));
     } else {
-      const int64_t q = (first + j - p.zone_tiles) * PF_TILE + row;   // counted without the rows that come by TMA
-      t = q < (p.tma ? p.n_window : p.P) ? (p.tma && q >= p.sink ? q + p.N : q) : p.P;
+      const int64_t q = (first + j - p.zone_tiles) * PF_TILE + row;   // window row
+      t = q < p.n_window ? (q >= p.sink ? q + p.N : q) : p.P;
 #pragma unroll
       for (int i = 0; i < 4; i++) key[i] = reinterpret_cast<const uint4*>(kb + min(t, p.P - 1) * p.k_l + 32 * s)[i];
     }
     const int64_t z = t - p.sink;   // zone row, if 0 <= z < N; window row t or t - N otherwise
     const bool zone = z >= 0 && z < p.N;
-    const int64_t wrow = z < p.N || p.N == 0 ? t : t - p.N;
+    const int64_t wrow = z < p.N ? t : t - p.N;
     if (j >= n_tma && t < p.P) {
-      uint4* dst = reinterpret_cast<uint4*>(zone ? p.store + ((int64_t)h * p.store_cap + z) * 256 : p.wk + h * p.w_h + wrow * 128) + 4 * s;
+      uint4* dst = reinterpret_cast<uint4*>(p.wk + h * p.w_h + wrow * 128) + 4 * s;
 #pragma unroll
       for (int i = 0; i < 4; i++) dst[i] = key[i];
     }
@@ -269,7 +272,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_con
 #pragma unroll 1
       for (int i = 0; i < 4; i++) {
         const int64_t tv = __shfl_sync(0xffffffffu, t, 2 * i + (lane >> 4)), zv = tv - p.sink;
-        const int64_t wv = zv < p.N || p.N == 0 ? tv : tv - p.N;
+        const int64_t wv = zv < p.N ? tv : tv - p.N;
         const bool in_zone = zv >= 0 && zv < p.N;
         const int l = lane & 15;
         uint4 raw;
@@ -279,8 +282,7 @@ __global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_con
           asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(raw.x), "=r"(raw.y), "=r"(raw.z), "=r"(raw.w) : "r"(at));
         } else {
           raw = reinterpret_cast<const uint4*>(vb + min(tv, p.P - 1) * p.v_l)[l];
-          if (tv < p.P)
-            (reinterpret_cast<uint4*>(in_zone ? p.store + ((int64_t)h * p.store_cap + zv) * 256 + 128 : p.wv + h * p.w_h + wv * 128))[l] = raw;
+          if (tv < p.P) reinterpret_cast<uint4*>(p.wv + h * p.w_h + wv * 128)[l] = raw;
         }
         const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
         float a = 0.0f;
@@ -320,6 +322,100 @@ __global__ void __launch_bounds__(PF_THREADS, 2) prefill_kernel(const __grid_con
   __syncthreads();
   int32_t* dst = p.counts + (int64_t)h * 16 * 256;
   for (int i = tid; i < 16 * 256; i += PF_THREADS)
+    if (hist[i]) atomicAdd(dst + i, hist[i]);
+}
+
+// The same row by row: the heads of a token range side by side in the grid, block (h, chunk) a head's consecutive tokens, the next
+// round's rows in flight in registers while a round is coded.  Short prompts, which the setup of the other form takes longer than,
+// and whatever cannot be described to the TMA unit (K and V in different orders of tokens and heads, heads that share their rows).
+// What bounds it: issue slots of the coding, with 16 warps per SM.  B200, us, this form | prefill_kernel with all rows loaded where
+// they are used, no round in flight: 300 tokens x 8 heads 7.8 | 10.4, 2000 x 8 11.5 | 16.7, 131072 x 8 with K and V in different
+// orders 261 | 359.
+__global__ void __launch_bounds__(EN_THREADS, 2) prefill_rows_kernel(PrefillParams p) {
+  __shared__ int hist[16 * 256];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, s = tid & 3, grp = tid >> 2;
+  const int h = blockIdx.x;
+  for (int i = tid; i < 16 * 256; i += EN_THREADS) hist[i] = 0;
+  if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) {
+    p.state[0] = p.n_window, p.state[1] = 0, p.state[2] = 0;
+    if (p.b == 0) p.state[3] = 0;   // (a later sample's launch would take the report of an earlier one away)
+    p.state[4 + p.b] = (int32_t)p.N;
+  }
+  __syncthreads();
+  const RotateLane rl(s);
+  uint4 mask[4];
+  load_key32(mask, p.signs, s);
+#pragma unroll
+  for (int i = 0; i < 4; i++) mask[i] = sign_mask(mask[i]);
+  const int64_t begin = (int64_t)blockIdx.y * p.chunk, end = min(p.P, begin + p.chunk);
+  const uint16_t* kb = p.k + h * p.k_h;
+  const uint16_t* vb = p.v + h * p.v_h;
+  // V is only copied: a half warp takes a row (16 bytes per lane), a warp the rows 2i, 2i + 1 of its eight in step i
+  uint4 kr[4], kn[4], vr[4];
+  auto load_v = [&](int64_t t0) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      vr[i] = reinterpret_cast<const uint4*>(vb + min(t0 + warp * 8 + 2 * i + (lane >> 4), end - 1) * p.v_l)[lane & 15];
+  };
+  load_key32(kr, kb + min(begin + grp, end - 1) * p.k_l, s);
+  load_v(begin);
+  for (int64_t t0 = begin; t0 < end; t0 += EN_KEYS) {
+    load_key32(kn, kb + min(t0 + EN_KEYS + grp, end - 1) * p.k_l, s);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int64_t t = t0 + warp * 8 + 2 * i + (lane >> 4), z = t - p.sink;
+      const bool zone = z >= 0 && z < p.N;
+      if (!zone || p.z_vnorm) {   // uniform over the half warp of a row
+        const uint32_t w[4] = {vr[i].x, vr[i].y, vr[i].z, vr[i].w};
+        float a = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; j++) a = fmaf(lo_f(w[j]), lo_f(w[j]), fmaf(hi_f(w[j]), hi_f(w[j]), a));
+        const unsigned half = 0xffffu << (lane & 16);
+#pragma unroll
+        for (int off = 1; off < 16; off <<= 1) a += __shfl_xor_sync(half, a, off);
+        if (t < end && (lane & 15) == 0) {
+          if (zone) p.z_vnorm[(int64_t)h * p.cap_z + z] = sqrtf(a);
+          else p.win_vnorm[(int64_t)h * p.cap_w + (z < p.N || p.N == 0 ? t : t - p.N)] = sqrtf(a);
+        }
+      }
+      if (t < end) {
+        if (zone) __stcs(reinterpret_cast<uint4*>(p.store + ((int64_t)h * p.store_cap + z) * 256 + 128) + (lane & 15), vr[i]);
+        else reinterpret_cast<uint4*>(p.wv + h * p.w_h + (z < p.N || p.N == 0 ? t : t - p.N) * 128)[lane & 15] = vr[i];
+      }
+    }
+    load_v(t0 + EN_KEYS);
+    const int64_t t = t0 + grp, z = t - p.sink;   // zone row, if 0 <= z < N; window row t or t - N otherwise
+    const bool zone = z >= 0 && z < p.N;
+    const int64_t wrow = z < p.N || p.N == 0 ? t : t - p.N;
+    if (t < end) {
+      uint4* dst = reinterpret_cast<uint4*>(zone ? p.store + ((int64_t)h * p.store_cap + z) * 256 : p.wk + h * p.w_h + wrow * 128) + 4 * s;
+#pragma unroll
+      for (int i = 0; i < 4; i++) dst[i] = kr[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) kr[i] = flip(kr[i], mask[i]);
+    const KeyCode kc = code_key<1>(kr, rl);
+    if (t < end) {
+      if (zone) {
+        const int64_t rec = (int64_t)h * p.cap_z + z;
+        *reinterpret_cast<uint32_t*>(p.z_codes + rec * 16 + 4 * s) = kc.codes;
+        *reinterpret_cast<uint2*>(p.z_w + rec * p.z_wl + 4 * s) = kc.weights;
+        *reinterpret_cast<uint4*>(p.z_pk + rec * p.z_pl + 16 * s) = kc.packed;
+#pragma unroll
+        for (int i = 0; i < 4; i++) atomicAdd(&hist[(4 * s + i) * 256 + ((kc.codes >> (8 * i)) & 0xffu)], 1);
+      } else {
+        const int64_t rec = (int64_t)h * p.cap_w + wrow;
+        *reinterpret_cast<uint32_t*>(p.win_codes + rec * 16 + 4 * s) = kc.codes;
+        *reinterpret_cast<uint2*>(p.win_w + rec * 16 + 4 * s) = kc.weights;
+        *reinterpret_cast<uint4*>(p.win_pk + rec * 64 + 16 * s) = kc.packed;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) kr[i] = kn[i];
+  }
+  __syncthreads();
+  int32_t* dst = p.counts + (int64_t)h * 16 * 256;
+  for (int i = tid; i < 16 * 256; i += EN_THREADS)
     if (hist[i]) atomicAdd(dst + i, hist[i]);
 }
 
@@ -688,15 +784,15 @@ static bool row_map(CUtensorMap* m, const void* base, int64_t inner, int64_t d1,
                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 // The maps of a prompt with zone rows; false: the kernel copies row by row.  K and V share the order of their dimensions.
-static bool prefill_maps(PrefillParams& p) {
+static bool prefill_maps(PrefillMaps& m, const PrefillParams& p) {
   const int64_t kh = p.H == 1 ? p.P * p.k_l : p.k_h, vh = p.H == 1 ? p.P * p.v_l : p.v_h;
-  p.heads_inner = p.H > 1 && kh < p.k_l;
-  if (p.heads_inner != (p.H > 1 && vh < p.v_l)) return false;
-  auto prompt = [&](CUtensorMap* m, const uint16_t* x, int64_t sl, int64_t sh) {
-    return p.heads_inner ? row_map(m, x, 128, p.H, sh, p.P, sl, 1, PF_TILE) : row_map(m, x, 128, p.P, sl, p.H, sh, PF_TILE, 1);
+  m.heads_inner = p.H > 1 && kh < p.k_l;
+  if (m.heads_inner != (p.H > 1 && vh < p.v_l)) return false;
+  auto prompt = [&](CUtensorMap* map, const uint16_t* x, int64_t sl, int64_t sh) {
+    return m.heads_inner ? row_map(map, x, 128, p.H, sh, p.P, sl, 1, PF_TILE) : row_map(map, x, 128, p.P, sl, p.H, sh, PF_TILE, 1);
   };
-  return prompt(&p.map_k, p.k, p.k_l, kh) && prompt(&p.map_v, p.v, p.v_l, vh) &&
-         row_map(&p.map_store, p.store, 256, p.N, 256, p.H, p.store_cap * 256, PF_TILE, 1);
+  return prompt(&m.k, p.k, p.k_l, kh) && prompt(&m.v, p.v, p.v_l, vh) &&
+         row_map(&m.store, p.store, 256, p.N, 256, p.H, p.store_cap * 256, PF_TILE, 1);
 }
 
 // The tensors of one cache layer that pk_append_encode and pk_prefill_sample share.
@@ -820,9 +916,16 @@ extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const p
   // Describing the tensors costs the host 1 - 1.5 us; shorter prompts take the device much less time than the host and go row by row
   // (B200, us a call, row by row | by TMA: four samples of 1000 tokens x 8 heads 86 | 92, 6000 x 8 heads 33.2 | 34.5, where only host
   // time shows; two layers of two samples of 2477 and 3001 tokens to host memory 843 | 836, 16000 x 8 heads 50 | 43).
-  p.tma = N * H > PF_TMA_KEYS && prefill_maps(p);
-  p.zone_tiles = p.tma ? (N + PF_TILE - 1) / PF_TILE : 0;
-  p.n_tiles = p.zone_tiles + ((p.tma ? p.n_window : P) + PF_TILE - 1) / PF_TILE;
+  PrefillMaps maps;
+  if (N * H <= PF_TMA_KEYS || !prefill_maps(maps, p)) {
+    p.chunk = encode_chunk(P, H);
+    if (cudaMemsetAsync(p.counts, 0, (size_t)(H * 16 * 256 * 4), st) != cudaSuccess) return check_launch("prefill memset", 0);
+    StageTimer tm(ST_ENCODE, st);
+    prefill_rows_kernel<<<dim3((unsigned)H, (unsigned)((P + p.chunk - 1) / p.chunk)), EN_THREADS, 0, st>>>(p);
+    return check_launch("prefill");
+  }
+  p.zone_tiles = (N + PF_TILE - 1) / PF_TILE;
+  p.n_tiles = p.zone_tiles + (p.n_window + PF_TILE - 1) / PF_TILE;
   // one wave of two blocks per SM, an even share of the tiles for each
   const int64_t fit = 2 * (int64_t)sm_count() / H;
   p.tiles_per_block = fit > 1 ? (p.n_tiles + fit - 1) / fit : p.n_tiles;
@@ -835,7 +938,7 @@ extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const p
   prefill_clear_kernel<<<(unsigned)(H * 4), 1024, 0, st>>>(p.counts, b == 0 ? p.state + 3 : nullptr);
   if (const int rc_clear = check_launch("prefill clear")) return rc_clear;
   StageTimer tm(ST_ENCODE, st);
-  prefill_kernel<<<dim3((unsigned)H, (unsigned)((p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block)), PF_THREADS, PF_SMEM, st>>>(p);
+  prefill_kernel<<<dim3((unsigned)H, (unsigned)((p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block)), PF_THREADS, PF_SMEM, st>>>(p, maps);
   return check_launch("prefill");
 }
 

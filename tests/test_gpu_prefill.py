@@ -127,7 +127,7 @@ def test_prefill_tiles_match_oracle(oracle, P, H, local, layout):
         assert not cache._store_kv[0][:, :, N:].any() and not cache.codebook_gpu[0][..., N:].any()
 
 
-@pytest.mark.parametrize("P", [700, 9000])     # row by row; by TMA
+@pytest.mark.parametrize("P", [700, 12000])    # row by row; by TMA
 @pytest.mark.parametrize("empty", [False, True])
 def test_report_of_one_sample_outlives_the_next(P, empty):
     """All samples of a layer share one error word: the host sets it, as sample 0 would, and sample 1 leaves it alone, a sample
