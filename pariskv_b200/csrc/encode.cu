@@ -151,7 +151,6 @@ constexpr int PF_HALF = PF_TILE * 128;            // bytes of 64 dimensions of a
 constexpr int PF_STAGE = 4 * PF_HALF;             // K, V; two halves each
 constexpr int PF_HIST = 16 * 256 * 4;
 constexpr int PF_SMEM = 2 * PF_STAGE + PF_HIST + 256 + 32;
-constexpr int64_t PF_TMA_KEYS = 16 * 1024;        // keys of a prompt (over all heads) above which its rows come by TMA
 constexpr int PF_WAIT_LIMIT = 4000000;            // polls of a barrier before giving up
 
 // Ahead of a prompt: its histogram, and with a layer's first sample the error word that all samples share.  A launch of its own,
@@ -913,23 +912,26 @@ extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const p
   p.P = P, p.N = N, p.cap_z = c.cap_z;
   if (N > 0) p.store = (uint16_t*)rows->data, p.store_cap = H == 1 ? rows->shape[1] : rows->stride[0] / 256;
   p.H = (int)H, p.cap_w = (int)c.cap_w, p.sink = (int)sink, p.n_window = (int)(N > 0 ? sink + local : P), p.b = (int)b;
-  // Describing the tensors costs the host 1 - 1.5 us; shorter prompts take the device much less time than the host and go row by row
-  // (B200, us a call, row by row | by TMA: four samples of 1000 tokens x 8 heads 86 | 92, 6000 x 8 heads 33.2 | 34.5, where only host
-  // time shows; two layers of two samples of 2477 and 3001 tokens to host memory 843 | 836, 16000 x 8 heads 50 | 43).
+  // By TMA: one wave of two blocks per SM, an even share of the tiles for each; where that makes less than 4/3 of a block per SM (one
+  // or two tiles a block, half the warps that an SM has room for), row by row.  B200, us on the device, row by row | by TMA: 8 heads
+  // of 2000 tokens (176 blocks) 11.2 | 13.3, 2400 (200) 14.5 | 13.4, 3500 (296) 16.6 | 14.1, 4000 (168) 18.1 | 21.2, 4500 (192)
+  // 18.6 | 20.4, 5000 (216) 22.4 | 18.4, 8000 (224) 30.0 | 26.8; 4 heads of 8000 (168) 18.4 | 20.7, of 12000 (252) 24.7 | 20.7; one
+  // head of 16000 (167) 10.8 | 13.4, of 24000 (250) 16.9 | 13.1, of 32768 (171) 17.8 | 20.8, of 48000 (250) 24.3 | 18.9.  The host's
+  // share of a call (three tensors described, one launch more) is 1.5 - 2 us more by TMA, and hidden at these sizes.
+  p.zone_tiles = (N + PF_TILE - 1) / PF_TILE;
+  p.n_tiles = p.zone_tiles + (p.n_window + PF_TILE - 1) / PF_TILE;
+  const int64_t fit = 2 * (int64_t)sm_count() / H;
+  p.tiles_per_block = fit > 1 ? (p.n_tiles + fit - 1) / fit : p.n_tiles;
+  while ((p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block > 65535) p.tiles_per_block *= 2;
+  const int64_t blocks = (p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block;   // of a head
   PrefillMaps maps;
-  if (N * H <= PF_TMA_KEYS || !prefill_maps(maps, p)) {
+  if (N == 0 || 3 * blocks * H < 4 * (int64_t)sm_count() || !prefill_maps(maps, p)) {
     p.chunk = encode_chunk(P, H);
     if (cudaMemsetAsync(p.counts, 0, (size_t)(H * 16 * 256 * 4), st) != cudaSuccess) return check_launch("prefill memset", 0);
     StageTimer tm(ST_ENCODE, st);
     prefill_rows_kernel<<<dim3((unsigned)H, (unsigned)((P + p.chunk - 1) / p.chunk)), EN_THREADS, 0, st>>>(p);
     return check_launch("prefill");
   }
-  p.zone_tiles = (N + PF_TILE - 1) / PF_TILE;
-  p.n_tiles = p.zone_tiles + (p.n_window + PF_TILE - 1) / PF_TILE;
-  // one wave of two blocks per SM, an even share of the tiles for each
-  const int64_t fit = 2 * (int64_t)sm_count() / H;
-  p.tiles_per_block = fit > 1 ? (p.n_tiles + fit - 1) / fit : p.n_tiles;
-  while ((p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block > 65535) p.tiles_per_block *= 2;
   static PerDevice smem_attr;
   if (const unsigned long long bit = first_on_device(smem_attr)) {
     if (cudaFuncSetAttribute(prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM) != cudaSuccess) return check_launch("prefill smem", 0);
@@ -938,7 +940,7 @@ extern "C" int pk_prefill_sample(const pk_tensor* k, const pk_tensor* v, const p
   prefill_clear_kernel<<<(unsigned)(H * 4), 1024, 0, st>>>(p.counts, b == 0 ? p.state + 3 : nullptr);
   if (const int rc_clear = check_launch("prefill clear")) return rc_clear;
   StageTimer tm(ST_ENCODE, st);
-  prefill_kernel<<<dim3((unsigned)H, (unsigned)((p.n_tiles + p.tiles_per_block - 1) / p.tiles_per_block)), PF_THREADS, PF_SMEM, st>>>(p, maps);
+  prefill_kernel<<<dim3((unsigned)H, (unsigned)blocks), PF_THREADS, PF_SMEM, st>>>(p, maps);
   return check_launch("prefill");
 }
 

@@ -148,3 +148,47 @@ def test_report_of_one_sample_outlives_the_next(P, empty):
     cache.check_status()
     cache._prefill_sample(k[0], v[0], 1, 1, 0)
     cache.check_status()
+
+
+# On both sides of the line between the two forms, and of the widths around it: 148 SMs x 4/3 = 198 blocks; one tile a block (25
+# tiles x 8 heads = 200 blocks by TMA, 24 x 8 = 192 row by row), two (4000 x 8: 168 row by row, 5000 x 8: 216 by TMA), three.
+@pytest.mark.parametrize("P,H", [(2300, 8), (2400, 8), (4000, 8), (5000, 8), (12300, 2), (24000, 1), (32768, 1)])
+@pytest.mark.parametrize("cls,offload,record", [("topk", True, 128), ("topk", False, 96), ("adaptive", True, 96), ("adaptive", False, 128)])
+def test_prompts_of_a_batch_match_oracle(oracle, P, H, cls, offload, record):
+    """Two samples of different valid_start, prefilled twice into the same cache: the bases of sample 1, a prompt that starts inside
+    its tensor, the staging rows behind the stores of the launch before, no value norms, both sizes of a key record."""
+    from pariskv_b200.cache_hub import polar_cache_adaptivek_varlen
+    from pariskv_b200.cache_hub.polar_cache import polar_cache
+    make = polar_cache if cls == "topk" else polar_cache_adaptivek_varlen.polar_cache
+    sink, local, starts, g = 4, 64, [3, 90], torch.Generator().manual_seed(P + H)
+    cache = make(valid_start=starts, layer_num=1, batch_size=2, max_length=P + 32, num_key_value_heads=H, num_heads=H, head_dim=128,
+                 dtype=torch.bfloat16, layer_mapping={"0": DEV}, max_new_length=32, sink_size=sink, local_size=local, final_topk=16,
+                 dynamic_update_interval=8, enable_offload=offload, key_record_bytes=record)
+    for _ in range(2):
+        k, v = _prompt(g, "tokens", 2, P, H)
+        cache.prefill_update_kv_cache(None, k, v, 0, 0)
+    cache.sync(0, 0)
+    torch.cuda.synchronize()
+    cache.check_status()
+    for b in range(2):
+        kt, vt = k[b:b + 1, starts[b]:].transpose(1, 2).cpu(), v[b:b + 1, starts[b]:].transpose(1, 2).cpu()
+        n = kt.shape[2]
+        N, one, zone = n - sink - local, slice(b, b + 1), slice(sink, n - local)
+        win = list(range(sink)) + list(range(n - local, n))
+        cb, w, pk = oracle.encode(kt.contiguous(), cache.srht_diagonal_signs.cpu())
+        w_n = sink + local
+        assert cache._layer_state[0].tolist()[:4] == [w_n, 0, 0, 0] and int(cache._layer_state[0][4 + b]) == N
+        for got, want in [(cache.unified_keys_gpu[0][one, :, :w_n], kt[:, :, win]), (cache.unified_values_gpu[0][one, :, :w_n], vt[:, :, win]),
+                          (cache._win_codes[0][one, :, :w_n].permute(0, 1, 3, 2), cb[..., win]),
+                          (cache._win_4bit[0][one, :, :w_n].permute(0, 1, 3, 2, 4), pk[..., win, :]),
+                          (cache.codebook_gpu[0][one, ..., :N], cb[..., zone]), (cache.key_4bit_packed_gpu[0][one, ..., :N, :], pk[..., zone, :]),
+                          (cache._store_k[0][one, :, :N], kt[:, :, zone]), (cache._store_v[0][one, :, :N], vt[:, :, zone])]:
+            assert torch.equal(got.cpu(), want)
+        assert torch.equal(bits_of(cache._win_weight[0][one, :, :w_n].cpu().permute(0, 1, 3, 2)), bits_of(w[..., win]))
+        assert torch.equal(bits_of(cache.key_block_weight_gpu[0][one, ..., :N].cpu()), bits_of(w[..., zone]))
+        # sums of 128 squares in fp32, as above
+        norm = vt.float().norm(dim=-1)
+        assert torch.allclose(cache._win_vnorm[0][one, :, :w_n].cpu(), norm[:, :, win], rtol=1e-5)
+        if cls == "adaptive":
+            assert torch.allclose(cache.value_norm_gpu[0][one, ..., :N].cpu(), norm[..., zone], rtol=1e-5)
+        assert torch.equal(cache.cluster_key_counts_gpu[0][one].cpu(), oracle.cluster_counts(cb[..., zone].contiguous()))
