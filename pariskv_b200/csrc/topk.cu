@@ -8,7 +8,9 @@
 // the exchanges by remote stores.  Rows read four elements a load, six loads in flight: 8 rows of 105K scores, the last launch of
 // a step with 1M keys, 114.2 -> 112.7 us a step.  Slices of 4096 elements and more take 1024 threads: that step 110.8 -> 107.4, the
 // operators over 8 x 131072 keys with 20000 candidates 151.5 -> 143.6, 32 x 50000 keys 266 -> 260, 8 x 60000 (slices of 6000) 89.4 ->
-// 87; shorter slices (8 x 32768 keys, 3300 a slice) lost 1 us to them, 1250 a slice 3.
+// 87; shorter slices (8 x 32768 keys, 3300 a slice) lost 1 us to them, 1250 a slice 3.  (Called one after the other with nothing
+// between, where a block of 512 threads shares an SM with the call before, slices of 4 - 10 K elements lose about 1 us: 8 x 60000
+// 10.5 | 11.5.)  More rows than fit at once keep 512 threads: see launch_rows.
 #include "cluster_select.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
@@ -20,6 +22,8 @@ constexpr int TK_WORDS = 1024;              // ballots kept per kind: slices of 
 constexpr int TK_CACHE = 32 * TK_WORDS;     // elements of a slice kept in shared memory; longer ones are read again from L2
 constexpr int TK_THREADS_LONG = 1024;       // threads of a block for slices of at least TK_LONG elements
 constexpr int TK_LONG = 4096;
+constexpr int64_t SM_SMEM = 228 << 10;      // shared memory of an SM
+constexpr int TK_STATIC = 2048;             // of a block besides the dynamic: SelShared, and 1 KB of the system's
 __host__ __device__ constexpr int tk_fixed(int cs, int threads) { return SEL_REGION + 2 * TK_WORDS * 4 + sel_inbox_bytes(cs, threads); }
 
 struct TopkParams {
@@ -166,17 +170,21 @@ int launch_rows(TopkParams p, int64_t rows, cudaStream_t st) {
   if (!cap) return fail(PK_ERR_CUDA, "topk: cannot identify the device");
   // CTAs per row: as many as are resident at once with at least 512 elements each (less does not pay for the exchanges);
   // a CTA numbers its elements with 27 bits
-  int best = 0;
+  int best = 0, best_i = 0;
   for (int i = 0; i < N_CLUSTER_SIZES; i++) {
     const int cs = CLUSTER_SIZES[i];
     if (cap->active[i] <= 0) continue;
     const bool fits = rows <= cap->active[i] && p.L >= 512LL * cs;
-    if (best == 0 || fits || (p.L + best - 1) / best >= (1LL << 27)) best = cs;
+    if (best == 0 || fits || (p.L + best - 1) / best >= (1LL << 27)) best = cs, best_i = i;
   }
   const int64_t slice = ((p.L + best - 1) / best + 31) / 32 * 32;
   if (slice >= (1LL << 27)) return fail(PK_ERR_ARG, "topk: row too long");
   p.cache = slice <= TK_CACHE ? (int)slice : 0;
-  const bool is_long = slice >= TK_LONG;
+  // 1024 threads, of which an SM takes one block, unless the rows are more than fit at once and two blocks of 512 threads would share
+  // an SM.  B200, us, 512 | 1024 threads: 300 rows of 5000 counts 14.0 | 19.6, of 16384 33.2 | 36.7, of 22000 43.8 | 45.6; of 24000, of
+  // which an SM takes one block either way, 58.6 | 48.6; of 60000, read again from L2, 197 | 170; 128 rows of 16384 15.3 | 13.3.
+  const bool pair = p.cache > 0 && 2 * (tk_fixed(best, SEL_THREADS) + (int64_t)p.cache * 4 + TK_STATIC) <= SM_SMEM;
+  const bool is_long = slice >= TK_LONG && (rows <= cap->active[best_i] || !pair);
   const size_t smem = tk_fixed(best, is_long ? TK_THREADS_LONG : SEL_THREADS) + (size_t)p.cache * 4;
   for (int64_t r0 = 0; r0 < rows; r0 += 65535) {   // grid.y limit
     TopkParams q = p;

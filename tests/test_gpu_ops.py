@@ -844,3 +844,17 @@ def test_attention_spreads_the_rows_that_there_are(ops, bs, H, G, K, n_window, o
             p = torch.softmax(q[b, 0, h * G:(h + 1) * G].double() @ k.t() / 128 ** 0.5, -1)
             # fp32 sums and probabilities of 17 bits, then one rounding to bf16: 2^-9 of the value, 2^-14 of the weighted magnitudes
             assert ((got - p @ v).abs() <= 2.0 ** -8 * (p @ v).abs() + 2.0 ** -14 * (p @ v.abs())).all()
+
+
+# As many rows as SMs (148 on B200) and more, at slices around 4096 elements, around the most of which two blocks share an SM
+# (2 * (16384 + 8192 + 1152 + 4 n + 2048) = 228 KB: n = 22240) and around those kept in shared memory: blocks of 512 and 1024 threads.
+@pytest.mark.parametrize("rows", [148, 149, 300])
+@pytest.mark.parametrize("L", [4064, 4065, 22240, 22241, 32768, 32769])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.float32])
+def test_topk_more_rows_than_fit_at_once(ops, rows, L, dtype):
+    g = torch.Generator(device=DEV).manual_seed(rows + L)
+    x = torch.randint(-40, 40, (rows, L), generator=g, device=DEV, dtype=torch.int32) if dtype is torch.int32 else torch.randn(rows, L, generator=g, device=DEV)
+    x[:, L // 2] = x[:, 3]
+    for k in (1, L // 20, L):
+        want = torch.sort(x.double(), dim=1, descending=True, stable=True).indices[:, :k].sort(dim=1).values
+        assert torch.equal(ops.topk(x, k), want)
