@@ -212,13 +212,19 @@ extern "C" int pk_silu_mul(const pk_tensor* gate_up, const pk_tensor* out, void*
 }
 
 // ---- matrix-vector products of a decode step (one token): y = W x, W bf16 [O, I] row-major, fp32 accumulation ------
-// HBM-bound: the weights are read once.  A block per SM takes an even share of the rows, one range of memory; its warps share the
-// columns (GvSplit::k_warps of them; where rows are short several rows are taken side by side), so that a warp keeps its part
-// of x in registers for all rows, and every lane has two steps of weight loads in flight.
-// What is lost to the copy rate is the start of each launch: its blocks are there while the launch before it still runs, and ask
-// for the first 48 KB of their rows by one prefetch to L2 before they wait.  On B200, a dense pass of two layers: hidden 4096,
-// feed-forward 12288 (770 MB) 148.8 -> 143.1 us against two rows per warp, 256 threads and a grid of 1.2 to 5.2 waves (without
-// the prefetch 146.4; 16, 32, 64, 128 KB 145.1, 143.4, 143.7, 146.4); hidden 2944, 8008: 93.4 -> 83; 5120, 13824: 217 -> 194.5.
+// HBM-bound: the weights are read once.  A block per SM takes an even share of the rows; its warps share the columns
+// (GvSplit::k_warps of them; where rows are short several rows are taken side by side), so that a warp keeps its part
+// of x in registers for all rows, and every lane has two steps of up to ten weight loads in flight, by pointers that move on.
+// What is lost to the copy rate is the start of each launch.  A block takes nearly all registers of an SM: it starts when its SM's
+// block of such a launch before it has ended, beside other kernels at once, and asks for the first 48 KB of its rows by one
+// prefetch to L2 before it waits.
+// B200, us, in a graph: 6144 x 4096 9.5, 4096 x 12288 15.9, gate and up of 12288 x 4096 32.5, 7168 x 5120 12.6 (two rows per warp, 256
+// threads and a grid of 1.2 to 5.2 waves: 10.9, 18.1, 33.7, 15.2; indexes multiplied out for each load and one row of 5120 a step: 9.7,
+// 17.1, 32.8, 13.9).  The prefetch: a dense pass of two layers, hidden 4096, feed-forward 12288, 143.1 with it, 146.4 without (16, 32,
+// 64, 128 KB 145.1, 143.4, 143.7, 146.4).
+// Rows in one range per block up to GV_TURNS steps a block; from there on they are dealt out a step at a time, so that all SMs read one
+// window of memory (a last step that only some blocks have costs less than an eighth).  One range | in turn: 151936 x 4096 176.0 | 174.1,
+// 32768 x 4096 42.0 | 41.1, 10240 x 4096 14.3 | 14.1, 20480 x 8192 52.1 | 50.1, gate and up of 28672 x 8192 135.1 | 132.5.
 // GATED: the rows are (o, o + F) of a stacked [gate; up] matrix and the output is silu(gate) * up, rounded like the
 // separate launches would (bf16 after the product, after silu, after the multiply).
 namespace pk {
@@ -228,6 +234,7 @@ constexpr int GV_THREADS = 512, GV_WARPS = GV_THREADS / 32;
 constexpr int GV_CHUNKS = 6;               // 16-byte pieces of a row that a lane takes at most
 constexpr int GV_PANEL = 128;              // rows whose partial sums are kept at a time
 constexpr unsigned GV_PREFETCH = 48 << 10; // bytes
+constexpr int GV_TURNS = 8;                // steps of a block from which on its rows are dealt out in turn
 
 // How the columns are split: 1 << k_log warps over a row, `chunks` pieces for a lane.
 struct GvSplit {
@@ -266,20 +273,33 @@ __device__ __forceinline__ float warp_sums(float (&v)[N], int lane) {
 template <int N>
 __device__ __forceinline__ int sum_of(int lane) { return lane * N / 32; }
 
+// Outputs of a warp per step, of U rows of CH pieces each: up to ten loads a lane.
+__host__ __device__ constexpr int gv_outputs(int U, int CH) {
+  return CH * U >= 6 || (U == 2 && CH >= 3) ? 1 : CH * U >= 3 ? 2 : 8 / (CH * U);
+}
+
 // CH: pieces of a row per lane
 template <bool GATED, int CH>
-__global__ void __launch_bounds__(GV_THREADS, 1) gemv_kernel(const uint16_t* W, const uint16_t* x, uint16_t* out, int n_out, int I, int k_log, bool early) {
+__global__ void __launch_bounds__(GV_THREADS, 1) gemv_kernel(const uint16_t* W, const uint16_t* x, uint16_t* out, int n_out, int I, int k_log, int share, int extra, bool early) {
   constexpr int U = GATED ? 2 : 1;                                            // rows of W per output
-  constexpr int RB = CH * U >= 5 ? 1 : CH * U >= 3 ? 2 / U + (U == 2 && CH == 2) : 8 / (CH * U);   // outputs of a warp per step
+  constexpr int RB = gv_outputs(U, CH);                                       // outputs of a warp per step
   constexpr int NV = RB * U;
   static_assert(NV == 1 || NV == 2 || NV == 4 || NV == 8, "warp_sums");
   __shared__ float part[GV_PANEL * U][GV_WARPS + 1];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int k_warps = 1 << k_log, kw = warp & (k_warps - 1), side = GV_WARPS >> k_log, group = warp >> k_log;
-  const int first = (int)((int64_t)n_out * blockIdx.x / gridDim.x), rows = (int)((int64_t)n_out * (blockIdx.x + 1) / gridDim.x) - first;
+  static_assert((RB & (RB - 1)) == 0, "shifts");
+  const int step_log = 4 - k_log + (RB >= 8 ? 3 : RB >= 4 ? 2 : RB >= 2 ? 1 : 0), per_step = 1 << step_log;   // RB * side outputs
+  // step s of the block: outputs first + s * stride .. + per_step - 1, those below `end`
+  const bool in_turn = share == 0;
+  const int block = (int)blockIdx.x, first = in_turn ? block * per_step : block * share + min(block, extra);
+  const int end = in_turn ? n_out : first + share + (block < extra);
+  const int stride = in_turn ? (int)gridDim.x * per_step : per_step;
+  int steps = (end - first + per_step - 1) >> step_log;
+  if (in_turn) steps = (int)((unsigned)(steps + (int)gridDim.x - 1) / gridDim.x);
   const int n = I >> 3, c0 = (int)((int64_t)n * kw >> k_log) + lane, c1 = (int)((int64_t)n * (kw + 1) >> k_log);
   if (tid == 0) {   // what this block reads first, on its way to L2 while it waits (a hint: no value is taken before the wait)
-    const int64_t bytes = (int64_t)rows * I * 2;
+    const int64_t bytes = (int64_t)(in_turn ? min(per_step, end - first) : end - first) * I * 2;
     const unsigned size = (unsigned)min(bytes, (int64_t)(GV_PREFETCH / U));
 #pragma unroll
     for (int u = 0; u < U; u++)
@@ -288,30 +308,35 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_kernel(const uint16_t* W, 
   struct Step {
     uint4 w[RB][U][CH];
   };
-  auto load = [&](Step& s, int step) {   // outputs (step * RB + i) * side + group of the block
+  const uint4* at = reinterpret_cast<const uint4*>(W + (int64_t)(first + group) * I) + c0;   // of the step that is loaded next
+  const int64_t next_row = (int64_t)side * n, next_step = (int64_t)stride * n, up = (int64_t)n_out * n;
+  int left = end - first - group;   // rows of the block from that step's first of this group on
+  auto load = [&](Step& s) {
 #pragma unroll
-    for (int i = 0; i < RB; i++) {
-      const int r = (step * RB + i) * side + group;
+    for (int i = 0; i < RB; i++)
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const uint4* row = reinterpret_cast<const uint4*>(W + ((int64_t)first + r + (int64_t)u * n_out) * I);
+      for (int u = 0; u < U; u++)
 #pragma unroll
-        for (int j = 0; j < CH; j++) s.w[i][u][j] = r < rows && c0 + 32 * j < c1 ? __ldcs(row + c0 + 32 * j) : make_uint4(0, 0, 0, 0);
-      }
-    }
+        for (int j = 0; j < CH; j++)
+          s.w[i][u][j] = i * side < left && c0 + 32 * j < c1 ? __ldcs(at + i * next_row + u * up + 32 * j) : make_uint4(0, 0, 0, 0);
+    at += next_step, left -= stride;
   };
   Step a, b;
   if (!early) pdl_wait();
-  load(a, 0);
+  load(a);
   pdl_wait();
   pdl_trigger();
+  constexpr bool KEEP_X = CH * U < 12;   // (otherwise the registers do not hold it beside two steps: from L1 each time)
+  auto load_x = [&](int j) -> uint4 { return c0 + 32 * j < c1 ? reinterpret_cast<const uint4*>(x)[c0 + 32 * j] : make_uint4(0, 0, 0, 0); };
   uint4 xs[CH];
+  if (KEEP_X)
 #pragma unroll
-  for (int j = 0; j < CH; j++) xs[j] = c0 + 32 * j < c1 ? reinterpret_cast<const uint4*>(x)[c0 + 32 * j] : make_uint4(0, 0, 0, 0);
-  const int per_step = RB * side, steps = (rows + per_step - 1) / per_step, panel = GV_PANEL / per_step;
-  auto flush = [&](int p0, int p_rows) {   // the panel's outputs
+    for (int j = 0; j < CH; j++) xs[j] = load_x(j);
+  const int panel = GV_PANEL >> step_log;
+  auto flush = [&](int step, int n_steps) {   // the outputs of a panel of n_steps steps
     __syncthreads();
-    if (tid < p_rows) {
+    const int o = first + (step + (tid >> step_log)) * stride + (tid & (per_step - 1));
+    if (tid < n_steps << step_log && o < end) {
       float y[U];
 #pragma unroll
       for (int u = 0; u < U; u++) {
@@ -320,13 +345,13 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_kernel(const uint16_t* W, 
       }
       if (GATED) {
         const float g = bfround(y[0]), up = bfround(y[U - 1]);
-        out[first + p0 + tid] = f2bf(bfround(g / (1.0f + __expf(-g))) * up);
+        out[o] = f2bf(bfround(g / (1.0f + __expf(-g))) * up);
       } else {
-        out[first + p0 + tid] = f2bf(y[0]);
+        out[o] = f2bf(y[0]);
       }
     }
   };
-  auto use = [&](const Step& s, int step, int in_panel) {
+  auto use = [&](const Step& s, int in_panel) {
     float v[NV];
 #pragma unroll
     for (int i = 0; i < RB; i++)
@@ -335,9 +360,9 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_kernel(const uint16_t* W, 
         float acc = 0.0f;
 #pragma unroll
         for (int j = 0; j < CH; j++) {
-          const uint4 w = s.w[i][u][j];
-          acc = fma_bf16x2(w.x, xs[j].x, acc), acc = fma_bf16x2(w.y, xs[j].y, acc);
-          acc = fma_bf16x2(w.z, xs[j].z, acc), acc = fma_bf16x2(w.w, xs[j].w, acc);
+          const uint4 w = s.w[i][u][j], v8 = KEEP_X ? xs[j] : load_x(j);
+          acc = fma_bf16x2(w.x, v8.x, acc), acc = fma_bf16x2(w.y, v8.y, acc);
+          acc = fma_bf16x2(w.z, v8.z, acc), acc = fma_bf16x2(w.w, v8.w, acc);
         }
         v[i * U + u] = acc;
       }
@@ -345,26 +370,26 @@ __global__ void __launch_bounds__(GV_THREADS, 1) gemv_kernel(const uint16_t* W, 
     const int at = sum_of<NV>(lane), r = (in_panel * RB + at / U) * side + group;
     if (lane % (32 / NV) == 0) part[r * U + at % U][kw] = sum;
   };
-  int in_panel = 0, p0 = 0;
+  int in_panel = 0, panel_first = 0;
   auto step_done = [&]() {
     if (++in_panel == panel) {
-      flush(p0, min(panel * per_step, rows - p0));
+      flush(panel_first, panel);
       __syncthreads();
-      in_panel = 0, p0 += panel * per_step;
+      in_panel = 0, panel_first += panel;
     }
   };
 #pragma unroll 1
   for (int step = 0; step < steps; step += 2) {
-    if (step + 1 < steps) load(b, step + 1);
-    use(a, step, in_panel);
+    if (step + 1 < steps) load(b);
+    use(a, in_panel);
     step_done();
     if (step + 1 < steps) {
-      if (step + 2 < steps) load(a, step + 2);
-      use(b, step + 1, in_panel);
+      if (step + 2 < steps) load(a);
+      use(b, in_panel);
       step_done();
     }
   }
-  if (in_panel) flush(p0, rows - p0);
+  if (in_panel) flush(panel_first, in_panel);
 }
 
 }  // namespace
@@ -389,8 +414,10 @@ extern "C" int pk_gemv(const pk_tensor* weight, const pk_tensor* x, const pk_ten
     constexpr int CH = decltype(chunks)::value;
     const uint16_t *w = (const uint16_t*)weight->data, *in = (const uint16_t*)x->data;
     uint16_t* y = (uint16_t*)out->data;
-    if (gated) launch_chain(gemv_kernel<true, CH>, dim3(grid), dim3(GV_THREADS), 0, (cudaStream_t)stream, w, in, y, (int)n_out, (int)I, split.k_log, pdl_early());
-    else launch_chain(gemv_kernel<false, CH>, dim3(grid), dim3(GV_THREADS), 0, (cudaStream_t)stream, w, in, y, (int)n_out, (int)I, split.k_log, pdl_early());
+    const int per_step = gv_outputs(gated ? 2 : 1, CH) * (GV_WARPS >> split.k_log), in_turn = n_out >= (int64_t)GV_TURNS * per_step * grid;
+    const int share = in_turn ? 0 : (int)(n_out / grid), extra = (int)(n_out % grid);
+    if (gated) launch_chain(gemv_kernel<true, CH>, dim3(grid), dim3(GV_THREADS), 0, (cudaStream_t)stream, w, in, y, (int)n_out, (int)I, split.k_log, share, extra, pdl_early());
+    else launch_chain(gemv_kernel<false, CH>, dim3(grid), dim3(GV_THREADS), 0, (cudaStream_t)stream, w, in, y, (int)n_out, (int)I, split.k_log, share, extra, pdl_early());
   };
   switch (split.chunks) {
     case 1: launch(std::integral_constant<int, 1>()); break;

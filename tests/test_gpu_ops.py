@@ -858,3 +858,26 @@ def test_topk_more_rows_than_fit_at_once(ops, rows, L, dtype):
     for k in (1, L // 20, L):
         want = torch.sort(x.double(), dim=1, descending=True, stable=True).indices[:, :k].sort(dim=1).values
         assert torch.equal(ops.topk(x, k), want)
+
+
+# Rows dealt out a step at a time from 8 steps of 148 blocks on (a step is 16 outputs at 2048 columns, 8 at 4096 and 5120, 2 at 12288
+# and 13824, half of that gated, 1 at 24576 gated): one output fewer, just as many, a last step of one output and of some blocks only.
+@pytest.mark.parametrize("I,step,gated", [(2048, 16, False), (4096, 8, False), (4096, 4, True), (5120, 8, False), (5120, 4, True), (12288, 2, False),
+                                          (13824, 2, False), (13824, 1, True), (24576, 1, True), (24576, 1, False)])
+@pytest.mark.parametrize("more", [-1, 0, 1, 7])
+def test_gemv_rows_in_turn_against_fp64(ops, I, step, gated, more):
+    """The bounds of test_gemv_splits_against_fp64."""
+    n = 8 * 148 * step + (more if more < 7 else 7 + 70 * step)
+    g = torch.Generator(device=DEV).manual_seed(I + n)
+    W = (torch.randn(2 * n if gated else n, I, generator=g, device=DEV) * 0.05).to(torch.bfloat16)
+    x = torch.randn(1, I, generator=g, device=DEV).to(torch.bfloat16)
+    ref = torch.cat([x.double() @ part.double().t() for part in W.split(4096)], 1)
+    mag = torch.cat([x.double().abs() @ part.double().abs().t() for part in W.split(4096)], 1)
+    y = ops.gemv(W, x, gated=gated).double()
+    if gated:
+        gate, up = ref[:, :n], ref[:, n:]
+        want = torch.nn.functional.silu(gate) * up
+        err = 2.0 ** -8 * (1.1 * gate.abs() * up.abs() + 3 * want.abs()) + I * 2.0 ** -22 * (mag[:, :n] * up.abs() + mag[:, n:] * gate.abs() + 1)
+        assert ((y - want).abs() <= err).all()
+    else:
+        assert ((y - ref).abs() <= 2.0 ** -8 * ref.abs() + I * 2.0 ** -24 * mag + 1e-30).all()
