@@ -192,13 +192,14 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
     for (int i = 0; i < ATT_HEAD_BUFS - 1; i++) later[i] = i + 1 < tpb ? index_of(t_first + i + 1) : 0;
   const int n_sel = (int)(p.n_sel ? min((int64_t)p.n_sel[bh], p.K) : p.K);   // (a call has at most 65536 rows)
   const int n_window = (int)(p.n_window_dev ? min(p.n_window, max((int64_t)0, (int64_t)p.n_window_dev[0] + p.n_window_add)) : p.n_window);
-  const int n_rows = n_window + n_sel;
+  const int n_rows = max(0, n_window + n_sel);   // (a count far below zero, which the caller's word may hold, is no row at all)
   // The launch is sized for the most rows there can be; where a block's share of those that there are is a tile less, they are
   // spread evenly over all blocks of the head.  (The indices are then asked for again: their first read was for another tile.)
   // Adaptive budgets select 1024 of the 4096 rows that a launch has room for: two of six blocks a head had all the work.  B200, a
   // step of two layers: 8 sequences 126.8 -> 122.2 us, 16 of two KV heads 136.7 -> 125.5, one sequence 100.0 -> 91.5.
-  if ((n_rows + TILE - 1) / TILE <= (tpb - 1) * n_groups) {
-    tpb = max(1, (int)((unsigned)((n_rows + TILE - 1) / TILE + n_groups - 1) / (unsigned)n_groups));
+  const int n_tiles = (n_rows + TILE - 1) / TILE;
+  if (n_tiles <= (tpb - 1) * n_groups) {
+    tpb = max(1, (int)((unsigned)(n_tiles + n_groups - 1) / (unsigned)n_groups));
     t_first = (int)blockIdx.x * tpb;
     ahead = index_of(t_first);
     if (CLUSTER)

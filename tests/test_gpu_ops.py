@@ -881,3 +881,22 @@ def test_gemv_rows_in_turn_against_fp64(ops, I, step, gated, more):
         assert ((y - want).abs() <= err).all()
     else:
         assert ((y - ref).abs() <= 2.0 ** -8 * ref.abs() + I * 2.0 ** -24 * mag + 1e-30).all()
+
+
+@pytest.mark.parametrize("bs,H,G,K", [(8, 8, 4, 4000), (1, 8, 4, 2048), (2, 2, 8, 900), (1, 2, 12, 700)])
+@pytest.mark.parametrize("count", [-33, -1000, -2 ** 31])
+def test_attention_takes_a_count_below_zero_for_no_rows(ops, bs, H, G, K, count):
+    """The rows of a head are counted from words on the device: one so far below zero that the window rows do not make up for it
+    leaves the head without rows, an output of zeros, in every form; the heads beside it are not touched."""
+    g = torch.Generator(device=DEV).manual_seed(K)
+    q = torch.randn(bs, 1, H * G, 128, generator=g, device=DEV).to(torch.bfloat16)
+    w = torch.randn(bs, H, 40, 128, generator=g, device=DEV).to(torch.bfloat16)
+    store = torch.randn(bs, H, K, 2, 128, generator=g, device=DEV).to(torch.bfloat16)
+    sel = torch.arange(K, device=DEV).expand(bs, H, K).contiguous()
+    n_sel = torch.full((bs, H), K, dtype=torch.int32, device=DEV)
+    want = ops.sparse_attention(q, w, w, 33, store[..., 0, :], store[..., 1, :], sel, n_sel=n_sel)
+    n_sel[0, 1] = count
+    got = ops.sparse_attention(q, w, w, 33, store[..., 0, :], store[..., 1, :], sel, n_sel=n_sel)
+    assert not got[0, 0, G:2 * G].any()
+    got[0, 0, G:2 * G] = want[0, 0, G:2 * G]
+    assert torch.equal(got, want)
