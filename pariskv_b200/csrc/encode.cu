@@ -5,6 +5,8 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "keycode.cuh"
 #include "rotate.cuh"
@@ -760,16 +762,17 @@ extern "C" int pk_encode_keys(const pk_tensor* keys, const pk_tensor* signs, con
 }
 
 // ---- tensor maps of the prompt's copies ----
-// The driver's encoder, asked for once: through the runtime, so that the library does not link to the driver.
+// The driver's encoder, through the runtime, so that the library does not link to the driver.  Asked for until it is found: a lookup
+// that fails once does not keep the process on the other form.
 static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
-      return cudaGetLastError(), (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
-    return (PFN_cuTensorMapEncodeTiled_v12000)f;
-  }();
-  return fn;
+  static std::atomic<PFN_cuTensorMapEncodeTiled_v12000> found{nullptr};
+  if (const auto fn = found.load(std::memory_order_relaxed)) return fn;
+  void* f = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+    return cudaGetLastError(), nullptr;
+  found.store((PFN_cuTensorMapEncodeTiled_v12000)f, std::memory_order_relaxed);
+  return (PFN_cuTensorMapEncodeTiled_v12000)f;
 }
 // 64 elements x box1 x box2 of a bf16 tensor [d2][d1][inner] in device memory; strides in elements, a multiple of 8.
 static bool row_map(CUtensorMap* m, const void* base, int64_t inner, int64_t d1, int64_t s1, int64_t d2, int64_t s2, int box1, int box2) {
