@@ -900,3 +900,33 @@ def test_attention_takes_a_count_below_zero_for_no_rows(ops, bs, H, G, K, count)
     assert not got[0, 0, G:2 * G].any()
     got[0, 0, G:2 * G] = want[0, 0, G:2 * G]
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("hidden,ffn", [(1024, 3072), (4096, 12288)])
+def test_gemv_with_early_loads_gives_the_same_bits(ops, hidden, ffn):
+    """norm -> gate and up -> down, each launch reading what the one before it wrote: with early loads the weights are read before the
+    wait, x never is.  Plain launches give the values."""
+    from pariskv_b200 import _lib
+    g = torch.Generator(device=DEV).manual_seed(hidden)
+    gu, down = ((torch.randn(o, i, generator=g, device=DEV) * 0.03).to(torch.bfloat16) for o, i in ((2 * ffn, hidden), (hidden, ffn)))
+    norm = torch.ones(hidden, dtype=torch.bfloat16, device=DEV)
+    xs = torch.randn(24, 1, hidden, generator=g, device=DEV).to(torch.bfloat16)
+
+    def run():
+        h, out = torch.zeros(1, hidden, dtype=torch.bfloat16, device=DEV), []
+        for x in xs:
+            h, n = ops.add_rmsnorm(x, h, norm)
+            h = ops.gemv(down, ops.gemv(gu, n, gated=True))
+            out.append(h)
+        return torch.cat(out)
+
+    try:
+        _lib.set_dependent_launch(False)
+        want = run()
+        _lib.set_dependent_launch(True)
+        assert torch.equal(run(), want)
+        _lib.set_pdl(True)
+        for _ in range(5):
+            assert torch.equal(run(), want)
+    finally:
+        _lib.set_dependent_launch(True)

@@ -253,3 +253,23 @@ def test_mirror_ops_under_transforms_and_tracing():
     assert not torch_ops.direct(neg) and torch.equal(bucket_topk(neg, 7), bucket_topk(neg.clone(), 7))
     with torch.device("cpu"):
         assert not torch_ops.direct(x)
+
+
+# Heads of which clusters of 10, 6, 5, 4, 3 and 2 blocks are taken (on B200): from four blocks on, the sixteen tier tables are made
+# by the blocks in turn and exchanged, unevenly with 5, 6 and 10; the counting's last round is one of 3 keys, or a whole one.
+@pytest.mark.parametrize("bs,H,N", [(1, 8, 12003), (2, 8, 12003), (1, 20, 12003), (11, 2, 12160), (3, 8, 12003), (13, 2, 12003), (7, 4, 12160), (5, 6, 12003),
+                                    (4, 8, 12003), (33, 1, 12160), (6, 6, 12003), (5, 8, 12003), (9, 6, 12003), (9, 8, 12003)])
+def test_retrieve_on_clusters_of_every_size(oracle, bs, H, N):
+    from pariskv_b200 import ops
+    g = torch.Generator().manual_seed(N + bs * H)
+    keys = synth_keys(g, bs, H, N)
+    q, signs, C, K = synth_queries(g, keys, 2), srht_signs(), 2000, 700
+    _, cen = oracle.constants()
+    counts = torch.zeros(bs, H, 16, 256, dtype=torch.int32, device=DEV)
+    cb, w, pk = ops.encode_keys(keys.to(DEV), signs.to(DEV), cluster_counts=counts)
+    ref = oracle.retrieve(q, signs, cb.cpu(), w.cpu(), pk.cpu(), counts.cpu(), cen, 0.25, C, K)
+    fin, ex = ops.retrieve(q.to(DEV), signs.to(DEV), cen.to(DEV), cb, w, pk, counts, oracle.tier_counts(N, 0.25), C, K,
+                           want=("cand", "scores_f32"))
+    assert torch.equal(ex["cand"].cpu(), ref["cand"])
+    assert torch.equal(ex["scores_f32"].cpu(), ref["score32"])
+    assert torch.equal(fin.cpu(), ref["final"])
