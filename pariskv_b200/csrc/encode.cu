@@ -58,14 +58,14 @@ __global__ void __launch_bounds__(EN_THREADS, 2) encode_kernel(EncodeParams p) {
   const uint16_t* kbase = p.keys + b * p.k_b + h * p.k_h;
   uint4 raw[4], nxt[4];
   load_key32(raw, kbase + min(begin + grp, end - 1) * p.k_l, s);
+#pragma unroll
+  for (int i = 0; i < 4; i++) raw[i] = flip(raw[i], mask[i]);
   for (int64_t k0 = begin; k0 < end; k0 += EN_KEYS) {  // uniform per block: shuffles need whole warps
     const int64_t key = k0 + grp;
     load_key32(nxt, kbase + min(key + EN_KEYS, end - 1) * p.k_l, s);   // in flight during the arithmetic
-#pragma unroll
-    for (int i = 0; i < 4; i++) raw[i] = flip(raw[i], mask[i]);
     const KeyCode kc = code_key<1>(raw, rl);
 #pragma unroll
-    for (int i = 0; i < 4; i++) raw[i] = nxt[i];
+    for (int i = 0; i < 4; i++) raw[i] = flip(nxt[i], mask[i]);   // (behind the coding: 8 heads x 131072 keys 221.1 -> 208.7 us on B200)
     if (key >= end) continue;
     if (KEY_MAJOR) {
       *reinterpret_cast<uint32_t*>(p.codes + b * p.c_b + h * p.c_h + key * 16 + 4 * s) = kc.codes;
