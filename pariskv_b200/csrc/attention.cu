@@ -195,8 +195,9 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS > 4 ? 1 : 3) sparse_attentio
   const int n_rows = max(0, n_window + n_sel);   // (a count far below zero, which the caller's word may hold, is no row at all)
   // The launch is sized for the most rows there can be; where a block's share of those that there are is a tile less, they are
   // spread evenly over all blocks of the head.  (The indices are then asked for again: their first read was for another tile.)
-  // Adaptive budgets select 1024 of the 4096 rows that a launch has room for: two of six blocks a head had all the work.  B200, a
-  // step of two layers: 8 sequences 126.8 -> 122.2 us, 16 of two KV heads 136.7 -> 125.5, one sequence 100.0 -> 91.5.
+  // Adaptive budgets select 1024 of the 4096 rows that a launch has room for: two of six blocks a head had all the work.  B200, the
+  // launch alone, some 1000 of 4096 rows: 64 heads 25.9 -> 13.9 us, 8 heads 10.5 -> 7.3, of 2048 rows: 96 heads 22.0 -> 16.4; with all of 2048 rows the
+  // look at the counts costs 64 heads 0.2 of 17.4, 128 heads 0.5 of 32.9.
   const int n_tiles = (n_rows + TILE - 1) / TILE;
   if (n_tiles <= (tpb - 1) * n_groups) {
     tpb = max(1, (int)((unsigned)(n_tiles + n_groups - 1) / (unsigned)n_groups));

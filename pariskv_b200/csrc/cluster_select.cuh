@@ -175,7 +175,7 @@ __device__ __forceinline__ void publish_range(cg::cluster_group& cluster, unsign
 // called publish_range() with the extremes of some of the slice's elements, and every thread has arrived at a cluster barrier
 // (CS > 1) behind it; the level-0 bins then lie between those extremes, elements outside fall into the first and the last one.
 // V::BINS: 512 where no CTA's slice has more than 65535 elements, otherwise 256.
-// region: SEL_REGION bytes, inbox: sel_inbox_bytes(CS), at the same offsets in all CTAs; words: 2 * words_cap words of this
+// region: SEL_REGION bytes, inbox: sel_inbox_bytes(CS, THREADS), at the same offsets in all CTAs; words: 2 * words_cap words of this
 // CTA's shared memory for ballots (longer slices are evaluated again instead).  All CTAs of the cluster call this with the same
 // K (>= 1, at most the row's length), after a cluster barrier, none of them still using its region for anything else.
 // LISTED: the elements are listed in shared memory before out_of() is asked for them, all at once: for values that have to be
@@ -290,7 +290,7 @@ __device__ __forceinline__ void cluster_select(cg::cluster_group& cluster, SelSh
   __syncthreads();
   if (kept || !flat) {
 #pragma unroll 2
-    for (int w = warp; w < n_words; w += WARPS) {   // a warp takes every 16th group of 32 elements
+    for (int w = warp; w < n_words; w += WARPS) {   // a warp takes every WARPS-th group of 32 elements
       const int i = w * 32 + lane;
       bool above = false, member = false;
       const uint32_t u = at(min(i, n - 1));

@@ -73,6 +73,8 @@ inline int elem_size(int dtype) {
 // Without the launch attribute both instructions do nothing.  The attribute is set unless pk_set_pdl(-1).
 // Only after pk_set_pdl(1) may a kernel load global memory before its wait (pdl_early(): weights, codes), and then only what
 // no launch of the running step writes: a caller who has not asked for it may have written those tensors a launch ago.
+// A prefetch to L2 delivers no value and may be issued before the wait at any time (gemv_kernel: its first rows): L2 is where the
+// writes of other kernels arrive, so that the load behind the wait sees them.
 // EVERY kernel launched through launch_chain() must call pdl_wait() before it reads or writes anything an earlier
 // kernel may touch: a kernel that skipped the wait would break the chain for its successors.
 // Such a kernel is resident while its predecessor still writes, so nothing that it reads is read-only for its lifetime: it

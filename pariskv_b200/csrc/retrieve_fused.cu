@@ -11,7 +11,7 @@
 // Why this split: as two launches (count | select + rerank + final top-K by the last block of a head) the final stage ran
 // on one SM per head, 12 us of 48 at 128K keys, and counts and scores went through L2.  Time line of a CTA on B200
 // (8 heads x 131004 keys, 10 CTAs each; query and ranking, 2.4 us, before the wait): tables 1.9 us, counting 13 K keys 6.8, threshold
-// 1.5, list 2.2, rerank of 1310 candidates 5.9, final selection 6.7.  Graph-replayed layer step, two launches -> one: 16
+// 1.5, list 2.2, rerank of 1310 candidates 5.9, final selection 6.7: 25 behind the wait.  Graph-replayed layer step, two launches -> one: 16
 // sequences of 16 - 32K keys (one CTA per head, no exchange at all) 155 -> 116 us, 8 heads x 128K keys 70 -> 60, 10K keys 27 -> 19
 // for the chain.
 // What bounds it: the serial chain of exchanges for small zones; for long ones instruction issue in the counting (85
@@ -107,11 +107,11 @@ __global__ void __launch_bounds__(CH_THREADS, 1) retrieve_fused_kernel(FusedPara
   };
   // In a large cluster a CTA makes the tables of its share of the subspaces only, a warp each, and writes them into all CTAs:
   // sixteen warps at the tier counts are bound by the integer ALU, and the exchange costs less than that (sort and tables of 10K
-  // keys on 10 CTAs 3.6 -> 2.7 us; on one or two CTAs there is nothing to gain).  With the level table left to the warps that do not
-  // prepare the query, a histogram that four threads a bin add up, and 512 bins in the selection, a step of four layers with
-  // 10K keys in host memory 140.6 -> 133.2 us, with 128K keys 188.5 -> 182.3, one KV head of eight sequences 168.3 -> 162.1; of two
-  // layers with 16 sequences of 16 - 32K keys 195.5 -> 190.8.  All pairs of clusters compared by all threads instead of the sort
-  // took 0.6 us longer: reads of shared memory.
+  // keys on 10 CTAs 3.6 -> 2.7 us; on one or two CTAs there is nothing to gain).  The chain alone in a graph, every CTA all tables |
+  // shared: 16 heads of 12K keys, six CTAs each, 15.3 | 14.5, 32 heads, four each, 16.1 | 15.3, 24 heads of 40K 21.8 | 21.3.  With the
+  // level table left to the warps that do not prepare the query, a histogram that four threads a bin add up, and 512 bins in the
+  // selection: 8 heads of 10K keys 15.4 -> 14.0, of 131K 29.4 -> 28.4, eight sequences of one head of 65K 21.7 -> 20.5, 128 heads of
+  // 33K 49.0 -> 48.2.  All pairs of clusters compared by all threads instead of the sort took longer: reads of shared memory.
   constexpr bool SHARED_TABLES = CS >= 4;
   const int sub = SHARED_TABLES ? (int)rank + CS * warp : warp;
   const bool ranks = sub < 16;
@@ -331,12 +331,14 @@ cudaError_t launch_cs(dim3 grid, size_t smem, cudaStream_t st, const FusedParams
 // candidates.  This one: waves x (16 us + 0.66 ns a key and 3.9 a candidate of a CTA's slice); without the final top-K 11 us,
 // 0.59 and 2.8.  The other: 22 us + 0.74 ns a key and 1.6 a candidate of an SM's share + 2.8 a candidate of a CTA's slice in the
 // top-k launch; without it 13 us.  It uses all SMs, so it wins where a cluster would leave most of them idle (one head) or the
-// heads are more than one wave.  us measured, this form | the other: 8 heads of 131K keys 30.0 | 31.4, of 200K 36.6 | 36.3, of
-// 400K 57.0 | 52.0; one head of 131K 25.7 | 26.4, of 400K 43.9 | 31.5; 16 heads of 262K 85.6 | 58.7; 128 heads of 33K 44.0 | 57.9;
-// without top-K 8 heads of 66K 15.8 | 16.0, of 131K 20.6 | 18.9, one head of 400K 29.8 | 18.2.  The other form has to win by 8 us
+// heads are more than one wave.  (Fitted before the tables were shared and the top-k had 1024 threads; both forms have become up to 2 us
+// faster since, and the rule takes the faster one at all of these but for the margin.)  us measured with the present kernels, alone in a
+// graph, 10 % of candidates, this form | the other: 8 heads of 10K keys 14.0 | 19.1, of 131K 28.4 | 30.7, of 200K 36.8 | 38.6, of
+// 400K 57.4 | 54.7; one head of 131K 22.7 | 23.4, of 400K 41.7 | 28.9; 16 heads of 262K 85.2 | 61.6; 128 heads of 33K 48.3 | 63.3;
+// without top-K 8 heads of 66K 15.5 | 16.1, of 131K 22.7 | 20.1, one head of 400K 34.6 | 18.3.  The other form has to win by 8 us
 // of a full zone: its further launches cost a program that calls eagerly, and is bound by its host, up to 5 (one layer of two heads,
 // adaptive budget, 91K keys 77.3 us a step with this form, 81.5 with the other), and a zone that is nearly empty 4 on the device.
-// A captured call has no such host time and pays the margin all the same: 8 heads of 400K keys take the 57.0 us.
+// A captured call has no such host time and pays the margin all the same: 8 heads of 400K keys take the 57.4 us.
 int fused_cluster_size(const pk_tensor* codebook, const RerankArgs& a, int64_t bs_h, int64_t N, int64_t C, int64_t K) {
   int layout = 0;
   chain_layout(codebook, &layout);

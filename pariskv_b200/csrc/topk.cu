@@ -6,9 +6,9 @@
 // bisected levels and per-thread spans; one CTA per row up to 16384 elements) -> now: 8 rows of 32768 counts, k 4096
 // 16.7 -> 10.0; 8 rows of 4096 scores, k 256 9.6 -> 8.7.  The operators' nine launches, two of them these: 68.1 -> 65.2 us with
 // the exchanges by remote stores.  Rows read four elements a load, six loads in flight: 8 rows of 105K scores, the last launch of
-// a step with 1M keys, 114.2 -> 112.7 us a step.  Slices of 4096 elements and more take 1024 threads: that step 110.8 -> 107.4, the
-// operators over 8 x 131072 keys with 20000 candidates 151.5 -> 143.6, 32 x 50000 keys 266 -> 260, 8 x 60000 (slices of 6000) 89.4 ->
-// 87; shorter slices (8 x 32768 keys, 3300 a slice) lost 1 us to them, 1250 a slice 3.  (Called one after the other with nothing
+// a step with 1M keys, 114.2 -> 112.7 us a step.  Slices of 4096 elements and more take 1024 threads: that step 114.2 -> 109.3, the
+// operators over 8 x 131072 keys with 20000 candidates 243.7 -> 235.3, 32 x 50000 keys 234.0 -> 226.4, 8 x 60000 (slices of 6000) 95.1 ->
+// 92.6; shorter slices (8 x 32768 keys, 3300 a slice) lost 1 us to them, 1250 a slice 3.  (Called one after the other with nothing
 // between, where a block of 512 threads shares an SM with the call before, slices of 4 - 10 K elements lose about 1 us: 8 x 60000
 // 10.5 | 11.5.)  More rows than fit at once keep 512 threads: see launch_rows.
 #include "cluster_select.cuh"
